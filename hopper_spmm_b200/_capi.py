@@ -98,6 +98,7 @@ SIGNATURES = {
     "b200spmm_spmm": (C.c_int, [vp, vp, i64, i64, vp, i64, C.c_int, vp]),
     "b200spmm_fp16_spmm": (C.c_int, [vp, vp, i64, i64, vp, i64, C.c_int, vp]),
     "b200spmm_tf32_spmm": (C.c_int, [vp, vp, i64, i64, vp, i64, C.c_int, vp]),
+    "b200spmm_release_cached_memory": (C.c_int, [C.c_int]),
     "b200spmm_plan_sync": (C.c_int, [vp, vp]),
     "b200spmm_spmm_host": (C.c_int, [vp, vp, i64, vp, C.c_int]),
     "b200spmm_bench": (C.c_int, [vp, vp, i64, i64, vp, i64, C.c_int, C.c_int, C.c_int, vp, C.POINTER(C.c_float)]),

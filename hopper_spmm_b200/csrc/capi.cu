@@ -12,10 +12,12 @@
 #include "../../include/b200_spmm.h"
 #include "common.hpp"
 #include "compress_gpu.hpp"
+#include "device_pool.hpp"
 #include "format.hpp"
 #include "handles.hpp"
 #include "spmm_kernel.cuh"
 #include "spmm_pair_kernel.cuh"
+#include "spmm_rows_kernel.cuh"
 #include "spmm_tall_kernel.cuh"
 #include "tall_gpu.hpp"
 #include "tensormap.hpp"
@@ -83,6 +85,11 @@ struct b200spmm_plan {
     // launches wider than 128 features when doubling the window height again halves the tile count.
     TallFormat pair;
     int pair_clusters = 0;     // two-CTA clusters of that kernel the GPU runs at the same time
+    // ... and as row units for the kernel that loads rows of B entry by entry (spmm_rows_kernel.cuh).  A matrix
+    // whose tiles are nearly empty keeps nothing else (rows_only).
+    RowsFormat rows_fmt;
+    bool rows_only = false;
+    bool has_tile_path = false;  // schedule and tile image of the 16-row kernel are there
     // Most tiles of the super-window format name one aligned group of CW consecutive rows of B: then B
     // is re-laid as shared-memory images at every launch (scratch of the plan, as large as B) and such a
     // tile's operand arrives by one bulk copy.
@@ -216,6 +223,17 @@ int launch_slab(b200spmm_plan *p, SpmmParams &prm, const CUtensorMap &tmap_b, cu
         case 64: return launch_one<kTf32, 64, kTma, kTiles>(p, prm, tmap_b, stream);
         default: return launch_one<kTf32, 128, kTma, kTiles>(p, prm, tmap_b, stream);
     }
+}
+
+// Slots for the pieces of windows or rows that are computed in parts, grown to the largest need seen.
+int grow_partial(b200spmm_plan *p, size_t floats) {
+    if (floats <= p->partial_floats) return B200SPMM_OK;
+    cudaFree(p->d_partial);
+    p->d_partial = nullptr;
+    p->partial_floats = 0;
+    B200_CUDA_TRY(cudaMalloc(&p->d_partial, floats * sizeof(float)));
+    p->partial_floats = floats;
+    return B200SPMM_OK;
 }
 
 // The environment is consulted when a plan is made (and once per process for the plan-less
@@ -381,6 +399,65 @@ int pair_max_clusters(int *out) {
     return B200SPMM_OK;
 }
 
+// ---- row units
+// A tile costs the 16-row kernel its gathered rows and one matrix instruction per 128 features whatever it
+// holds; a row unit costs a row load per entry.
+constexpr double kRowsMaxFill = 0.08;  // share of a tile's slots in use
+
+bool use_rows(const b200spmm_plan *p, int64_t ldb) {
+    return p->rows_only && ldb * p->info.elt_size <= 0xFFFFFFFFll;  // (the kernel's row pitch is 32-bit)
+}
+
+int launch_rows(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
+                cudaStream_t stream, int band) {
+    const RowsFormat &f = p->rows_fmt;
+    if (band >= 0 && (size_t)band + 1 >= f.bands.size()) return B200SPMM_ERR_INVALID_ARG;
+    const RowBand &from = f.bands[band < 0 ? 0 : band], &to = band < 0 ? f.bands.back() : f.bands[band + 1];
+    RowsParams prm{};
+    prm.batches = f.d_batches;
+    prm.units = f.d_units;
+    prm.unit_begin = from.unit;
+    prm.unit_end = to.unit;
+    prm.empty_begin = from.empty;
+    prm.empty_end = to.empty;
+    prm.n_batches = f.n_batches;
+    prm.B = d_B;
+    prm.C = d_C;
+    prm.ldb = ldb;
+    prm.ldc = ldc;
+    prm.n = (uint32_t)n;
+    prm.slab = slab_for(prm.n);
+    prm.c_is_half = c_dtype == B200SPMM_C_F16;
+    if (f.n_slots) {
+        int st = grow_partial(p, (size_t)f.n_slots * (size_t)n);
+        if (st != B200SPMM_OK) return st;
+    }
+    prm.partial = p->d_partial;
+    // a group of lanes for every kRowsGroupBatches batches, but enough of them for one wave where there are units for it
+    const uint32_t vec = 16u / (uint32_t)p->info.elt_size;
+    const uint32_t n_slabs = (prm.n + prm.slab - 1) / prm.slab;
+    const uint32_t groups = 32u / (std::min(prm.slab, prm.n) / vec);
+    const uint32_t n_units = std::max(prm.unit_end - prm.unit_begin, prm.empty_end - prm.empty_begin), per_block = groups * (kRowsThreads / 32);
+    const uint64_t share = (uint64_t)f.n_batches * n_units / f.n_units / kRowsGroupBatches / per_block;
+    const dim3 grid(std::min((n_units + per_block - 1) / per_block, std::max((uint32_t)share, (uint32_t)(p->n_sms * kRowsBlocksPerSm))), n_slabs);
+    p->last.n_ctas = (int)(grid.x * grid.y);
+    p->last.threads = kRowsThreads;
+    p->last.feature_slab = (int)prm.slab;
+    p->last.n_slabs = (int)n_slabs;
+    p->last.row_window = kRowWindow;
+    if (!n_units) return B200SPMM_OK;
+    auto kernel = p->info.dtype == B200SPMM_TF32 ? spmm_rows_kernel<true> : spmm_rows_kernel<false>;
+    kernel<<<grid, kRowsThreads, 0, stream>>>(prm);
+    B200_CUDA_TRY(cudaGetLastError());
+    p->last.kernel_launches = 1;
+    const uint32_t s0 = from.split, s1 = to.split;
+    if (s1 == s0) return B200SPMM_OK;
+    rows_fixup_kernel<<<s1 - s0, 256, 0, stream>>>(f.d_splits + s0, p->d_partial, d_C, ldc, prm.n, prm.c_is_half);
+    B200_CUDA_TRY(cudaGetLastError());
+    p->last.kernel_launches = 2;
+    return B200SPMM_OK;
+}
+
 bool use_pair(const b200spmm_plan *p, int64_t n) {
     if (!p->pair.tiles || p->pair_clusters < 1 || n <= 128) return false;
     if (p->tall_forced) return true;
@@ -526,16 +603,9 @@ int plan_build_tile_image(b200spmm_plan *p) {
     return B200SPMM_OK;
 }
 
-int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h_rowIdx, int n_ctas) {
+// The schedule of the 16-row kernel, on the device.
+int plan_build_schedule(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h_rowIdx, int n_ctas) {
     const auto &info = p->info;
-    if (info.row_window != kRowWindow) return B200SPMM_ERR_UNSUPPORTED;
-    const int cw = info.dtype == B200SPMM_F16 ? 16 : 8;
-    if (info.col_window != cw) return B200SPMM_ERR_UNSUPPORTED;
-    if (info.total_tiles * (uint64_t)kRowWindow >= 0x7FFFFFFFull) return B200SPMM_ERR_UNSUPPORTED;  // TMA row coordinate
-    cudaDeviceProp prop;
-    B200_CUDA_TRY(cudaGetDeviceProperties(&prop, p->device));
-    if (prop.major != 10) return B200SPMM_ERR_NO_DEVICE;
-    p->n_sms = prop.multiProcessorCount;
     auto upload = [](auto **dst, const auto &v) -> int {
         using T = typename std::remove_reference<decltype(v)>::type::value_type;
         B200_CUDA_TRY(cudaMalloc(dst, std::max<size_t>(v.size() * sizeof(T), 16)));
@@ -544,7 +614,7 @@ int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h
     };
     {
         b200spmm_plan::Sched &ps = p->sched;
-        ps.n_ctas = n_ctas > 0 ? n_ctas : prop.multiProcessorCount * kCtasPerSm;
+        ps.n_ctas = n_ctas > 0 ? n_ctas : p->n_sms * kCtasPerSm;
         // Several chunks per CTA, taken from all over the matrix, even out regions whose tiles
         // cost more than the schedule's model says; a chunk stays long enough (512 tiles or
         // more) for the hand-over at its start not to matter.
@@ -571,11 +641,15 @@ int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h
         ps.band_row = bands.row;
         ps.band_split = bands.split;
     }
-    // status word, then the two counters of the chunk hand-out (the kernel leaves them at zero)
-    B200_CUDA_TRY(cudaMalloc(&p->d_status, 4 * sizeof(uint32_t)));
-    B200_CUDA_TRY(cudaMemset(p->d_status, 0, 4 * sizeof(uint32_t)));
+    return B200SPMM_OK;
+}
+
+// What the tile kernels need beside the format: schedule, compressed tiles or super-windows, tile image.
+int plan_build_tile_path(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h_rowIdx, int n_ctas) {
+    const auto &info = p->info;
     {
-        int st = encode_tile_map(p);
+        int st = plan_build_schedule(p, h_rowOffset, h_rowIdx, n_ctas);
+        if (st == B200SPMM_OK) st = encode_tile_map(p);
         if (st != B200SPMM_OK) return st;
     }
     // On request (B200SPMM_TILES=bitmap) the kernels stream the tiles in compressed form - bitmap +
@@ -583,8 +657,6 @@ int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h
     // give the same C bit for bit.  The compressed form moves an eighth of the tile bytes at a
     // few per cent fill but costs the producer warps more instructions per tile than they can
     // spare today, so dense tiles are the default.
-    p->gather_cpasync = env_is("B200SPMM_GATHER", "cpasync");
-    p->host_split = !env_is("B200SPMM_HOST_SPLIT", "0");
     if (info.total_tiles && env_is("B200SPMM_TILES", "bitmap")) {
         int st = compress_tiles_device(p->d_data, info.total_tiles, info.dtype, &p->comp);
         if (st != B200SPMM_OK) return st;
@@ -610,7 +682,37 @@ int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h
         int st = plan_build_tall(p, h_rowOffset, h_rowIdx);
         if (st != B200SPMM_OK) return st;
     }
+    p->has_tile_path = true;
     return plan_build_tile_image(p);
+}
+
+int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h_rowIdx, int n_ctas) {
+    const auto &info = p->info;
+    if (info.row_window != kRowWindow) return B200SPMM_ERR_UNSUPPORTED;
+    const int cw = info.dtype == B200SPMM_F16 ? 16 : 8;
+    if (info.col_window != cw) return B200SPMM_ERR_UNSUPPORTED;
+    if (info.total_tiles * (uint64_t)kRowWindow >= 0x7FFFFFFFull) return B200SPMM_ERR_UNSUPPORTED;  // TMA row coordinate
+    int major = 0;
+    B200_CUDA_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, p->device));
+    if (major != 10) return B200SPMM_ERR_NO_DEVICE;
+    B200_CUDA_TRY(cudaDeviceGetAttribute(&p->n_sms, cudaDevAttrMultiProcessorCount, p->device));
+    // status word, then the two counters of the chunk hand-out (the kernel leaves them at zero)
+    B200_CUDA_TRY(cudaMalloc(&p->d_status, 4 * sizeof(uint32_t)));
+    B200_CUDA_TRY(cudaMemset(p->d_status, 0, 4 * sizeof(uint32_t)));
+    p->gather_cpasync = env_is("B200SPMM_GATHER", "cpasync");
+    p->host_split = !env_is("B200SPMM_HOST_SPLIT", "0");
+    // An explicit CTA count, a way to fetch tiles or rows, or a window height asks for a tile kernel.
+    // B200SPMM_WINDOW=rows asks for the row units whatever the matrix.
+    const bool force_rows = env_is("B200SPMM_WINDOW", "rows");
+    if (n_ctas <= 0 && (force_rows || (!std::getenv("B200SPMM_WINDOW") && !std::getenv("B200SPMM_TILES") && !p->gather_cpasync))) {
+        int st = build_rows_device(info, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, p->n_sms, &p->rows_fmt);
+        if (st != B200SPMM_OK) return st;
+        const double slots = (double)info.total_tiles * kRowWindow * cw;
+        p->rows_only = p->rows_fmt.n_units && (force_rows || (double)p->rows_fmt.nnz <= kRowsMaxFill * slots);
+        if (p->rows_only) return B200SPMM_OK;
+        free_rows(&p->rows_fmt);
+    }
+    return plan_build_tile_path(p, h_rowOffset, h_rowIdx, n_ctas);
 }
 
 }  // namespace
@@ -851,6 +953,7 @@ void b200spmm_plan_destroy(b200spmm_plan_t *p) {
         cudaFree(ps.d_piece_slots);
     }
     free_compressed_tiles(&p->comp);
+    free_rows(&p->rows_fmt);
     cudaFree(p->d_tile_entries);
     free_tall(&p->tall);
     free_tall(&p->pair);
@@ -1025,6 +1128,13 @@ int b200spmm_plan_launch_info(const b200spmm_plan_t *p, b200spmm_launch_info_t *
 
 namespace {
 
+int plan_add_tile_path(b200spmm_plan *p) {
+    std::vector<uint32_t> h_rowOffset(p->info.eff_row_windows + 1), h_rowIdx(p->info.eff_row_windows);
+    B200_CUDA_TRY(cudaMemcpy(h_rowOffset.data(), p->d_rowOffset, h_rowOffset.size() * 4, cudaMemcpyDeviceToHost));
+    B200_CUDA_TRY(cudaMemcpy(h_rowIdx.data(), p->d_rowIdx, h_rowIdx.size() * 4, cudaMemcpyDeviceToHost));
+    return plan_build_tile_path(p, h_rowOffset.data(), h_rowIdx.data(), 0);
+}
+
 // The product, or one band of it (band < 0: every chunk; otherwise the chunks, rows and split
 // windows of that band of the schedule the launch selects - see b200spmm_plan::Sched).
 int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
@@ -1041,6 +1151,11 @@ int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, voi
     if (p->info.eff_row_windows == 0) {  // nothing stored: C is all zeros
         B200_CUDA_TRY(cudaMemset2DAsync(d_C, (size_t)ldc * csz, 0, (size_t)n * csz, p->info.rows, stream));
         return B200SPMM_OK;
+    }
+    if (!p->starve_gathers && use_rows(p, ldb)) return launch_rows(p, d_B, ldb, n, d_C, ldc, c_dtype, stream, band);
+    if (!p->has_tile_path) {  // only row units were kept; the starved test launch and a huge ldb ask for more
+        int st = plan_add_tile_path(p);
+        if (st != B200SPMM_OK) return st;
     }
     if (band < 0 && use_tall(p, n)) return launch_tall(p, d_B, ldb, n, d_C, ldc, c_dtype, stream);
     SpmmParams prm{};
@@ -1061,14 +1176,8 @@ int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, voi
     const uint32_t split_end = band < 0 ? sc.n_splits : sc.band_split[band + 1];
     prm.sched_counter = sc.n_chunks > (uint32_t)sc.n_ctas ? p->d_status + 1 : nullptr;
     if (sc.n_slots) {  // slots for the pieces of windows that span chunks
-        const size_t need = (size_t)sc.n_slots * kRowWindow * (size_t)n;
-        if (need > p->partial_floats) {
-            cudaFree(p->d_partial);
-            p->d_partial = nullptr;
-            p->partial_floats = 0;
-            B200_CUDA_TRY(cudaMalloc(&p->d_partial, need * sizeof(float)));
-            p->partial_floats = need;
-        }
+        int st = grow_partial(p, (size_t)sc.n_slots * kRowWindow * (size_t)n);
+        if (st != B200SPMM_OK) return st;
     }
     prm.partial = p->d_partial;
     prm.tiles_image = static_cast<const uint8_t *>(p->d_tiles_image);
@@ -1156,8 +1265,13 @@ int b200spmm_spmm_host(b200spmm_plan_t *p, const void *h_B, int64_t n, void *h_C
         B200_CUDA_TRY(cudaMalloc(&p->d_C, c_bytes));
         p->d_C_bytes = c_bytes;
     }
-    const b200spmm_plan::Sched &sc = p->sched;
-    const size_t bands = sc.band_chunk.size() > 1 && !use_tall(p, n) ? sc.band_chunk.size() - 1 : 1;
+    const bool rows = use_rows(p, n);
+    std::vector<uint64_t> band_row = p->sched.band_row;
+    if (rows) {
+        band_row.clear();
+        for (const RowBand &b : p->rows_fmt.bands) band_row.push_back(b.row);
+    }
+    const size_t bands = band_row.size() > 1 && (rows || !use_tall(p, n)) ? band_row.size() - 1 : 1;
     if (bands == 1 || p->info.eff_row_windows == 0) {
         B200_CUDA_TRY(cudaMemcpyAsync(p->d_B, h_B, b_bytes, cudaMemcpyHostToDevice, nullptr));
         int st = b200spmm_spmm(p, p->d_B, n, n, p->d_C, n, c_dtype, nullptr);
@@ -1212,7 +1326,7 @@ int b200spmm_spmm_host(b200spmm_plan_t *p, const void *h_B, int64_t n, void *h_C
             cudaEvent_t done = p->band_done[(size_t)part * bands + k];
             B200_CUDA_TRY(cudaEventRecord(done, nullptr));
             B200_CUDA_TRY(cudaStreamWaitEvent(p->copy_stream, done, 0));
-            const uint64_t r0 = sc.band_row[k], r1 = sc.band_row[k + 1];
+            const uint64_t r0 = band_row[k], r1 = band_row[k + 1];
             if (r1 == r0) continue;
             B200_CUDA_TRY(cudaMemcpy2DAsync(static_cast<char *>(h_C) + r0 * c_pitch + (size_t)f0 * csz, c_pitch, c_part + r0 * c_pitch,
                                             c_pitch, (size_t)nf * csz, r1 - r0, cudaMemcpyDeviceToHost, p->copy_stream));

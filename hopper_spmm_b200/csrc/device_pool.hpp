@@ -1,0 +1,50 @@
+// Device memory of formats, plans and their construction.
+//
+// cudaMalloc and cudaFree map and unmap memory and stop the device; a conversion makes two dozen buffers, and a
+// caller with a new matrix per step (a sampled graph) paid ten milliseconds for them.  They come from one CUDA
+// memory pool per device instead, which keeps at most kPoolKeepBytes of freed memory for the next object and
+// gives the rest back to the driver at the next synchronisation; b200spmm_release_cached_memory gives back all
+// of it, and so does an allocation that finds the device full.  The pool is the driver's: it may be used from
+// any thread, and what one stream frees another one gets only when the order of their work allows it.
+#pragma once
+
+#include <algorithm>
+#include <cstddef>
+#include <cuda_runtime.h>
+
+namespace b200spmm {
+
+// Enough for the working set of a matrix of some ten million entries, 0.3 % of the card.
+constexpr size_t kPoolKeepBytes = (size_t)512 << 20;
+
+cudaError_t pool_alloc_bytes(void **out, size_t bytes, cudaStream_t stream);
+void pool_free(void *ptr, cudaStream_t stream = nullptr);
+cudaError_t pool_release(int device);
+
+// Memory of the current device, usable by work that is ordered after `stream`.
+template <typename T>
+cudaError_t pool_alloc(T **out, size_t count, cudaStream_t stream = nullptr) {
+    void *p = nullptr;
+    const cudaError_t e = pool_alloc_bytes(&p, std::max<size_t>(count * sizeof(T), 16), stream);
+    *out = static_cast<T *>(p);
+    return e;
+}
+
+// Buffers that are needed while an object is built, released on every exit path.
+struct PoolScratch {
+    cudaStream_t stream = nullptr;
+    void *ptrs[24] = {};
+    int n = 0;
+    explicit PoolScratch(cudaStream_t s = nullptr) : stream(s) {}
+    PoolScratch(const PoolScratch &) = delete;
+    template <typename T>
+    cudaError_t alloc(T **out, size_t count) {
+        if (n == 24) return cudaErrorMemoryAllocation;
+        const cudaError_t e = pool_alloc(out, count, stream);
+        if (e == cudaSuccess) ptrs[n++] = *out;
+        return e;
+    }
+    ~PoolScratch() { for (int i = 0; i < n; ++i) pool_free(ptrs[i], stream); }
+};
+
+}  // namespace b200spmm

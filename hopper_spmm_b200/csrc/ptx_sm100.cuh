@@ -149,6 +149,16 @@ B200_DEVICE void tma_gather4_2d(uint32_t dst, const void *tmap, int32_t x, int32
         : "memory");
 }
 
+B200_DEVICE uint4 ld_shared_v4(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+B200_DEVICE uint32_t ld_shared_u32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
 B200_DEVICE void st_shared_v4(uint32_t addr, uint4 v) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
@@ -162,6 +172,10 @@ B200_DEVICE void st_shared_u16(uint32_t addr, uint16_t v) {
 // (src_bytes == 0 reads nothing and writes 16 zero bytes).
 B200_DEVICE void cp_async_16(uint32_t dst, const void *src, uint32_t src_bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+}
+// The same for data that is likely to be asked for again by this SM: cached in L1.
+B200_DEVICE void cp_async_ca_16(uint32_t dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 // Copies 4 bytes global -> shared (cached in L1: neighbouring words are fetched next).
 B200_DEVICE void cp_async_4(uint32_t dst, const void *src) {

@@ -1,0 +1,383 @@
+// Condensed tiles -> row units, on the device.
+//
+//   1. the tiles of every window in runs of at most kRunTiles; a warp counts the stored values of each of the
+//      sixteen rows of its run (one 16-byte load per lane is half a tile row)
+//   2. per (window, row): running sums over the window's runs -> row lengths; scans over the rows -> the units,
+//      slots and bands
+//   3. units sorted by (band, length), longest first (CUB radix sort, a few key bits), their batches numbered in
+//      that order
+//   4. the warps of step 1 write (column, value) to the place of their row's unit
+// A stored value is one whose bits are not all zero (an explicit zero adds nothing to a product).
+#include <algorithm>
+#include <cub/cub.cuh>
+
+#include "common.hpp"
+#include "device_pool.hpp"
+#include "rows_gpu.hpp"
+
+namespace b200spmm {
+namespace {
+
+constexpr int kBlock = 256;
+constexpr uint32_t kRunTiles = 256;
+constexpr uint32_t kMaxBands = 8;
+constexpr uint32_t kEmptyKey = kMaxBands << 9;  // sort key: rows without entries last, then the band, then the longest first
+constexpr uint64_t kMinBandedCost = 2000000;  // bands pay where one keeps the GPU busy for tens of microseconds
+// For the bands a row counts as this many entries: its store is 4 bytes a feature where a gathered entry is 2.
+constexpr uint64_t kRowCost = 2;
+
+inline int grid_for(uint64_t n) { return (int)std::max<uint64_t>(1, std::min<uint64_t>((n + kBlock - 1) / kBlock, 148 * 32)); }
+
+__host__ __device__ __forceinline__ uint32_t pieces_of(uint32_t len, uint32_t cap) { return len <= cap ? 1u : (len + cap - 1) / cap; }
+
+__global__ void run_counts_kernel(const uint32_t *__restrict__ rowOffset, uint32_t eff, uint32_t *__restrict__ n_runs) {
+    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w < eff) n_runs[w] = (rowOffset[w + 1] - rowOffset[w] + kRunTiles - 1) / kRunTiles;
+    if (w == eff) n_runs[w] = 0;
+}
+
+__global__ void run_windows_kernel(const uint32_t *__restrict__ run_first, uint32_t eff, uint32_t *__restrict__ run_window) {
+    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w >= eff) return;
+    for (uint32_t r = run_first[w]; r < run_first[w + 1]; ++r) run_window[r] = w;
+}
+
+// The lane's share of a tile: row lane / 2, its left or right half of the columns.
+template <typename T>
+struct Piece {
+    static constexpr int kPer = 16 / (int)sizeof(T);
+    T v[kPer];
+    uint32_t mask;
+    __device__ __forceinline__ void load(const T *__restrict__ data, uint64_t tile, uint32_t lane) {
+        *reinterpret_cast<uint4 *>(v) = __ldcs(reinterpret_cast<const uint4 *>(data + tile * (32 * kPer) + lane * kPer));
+        mask = 0;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) mask |= v[k] != 0 ? 1u << k : 0u;
+    }
+};
+
+// counts[run * 16 + row] = stored values of that row in the run's tiles
+template <typename T>
+__global__ void __launch_bounds__(kBlock)
+run_rows_kernel(const uint32_t *__restrict__ rowOffset, const T *__restrict__ data, const uint32_t *__restrict__ run_first,
+                const uint32_t *__restrict__ run_window, uint32_t eff, uint32_t *__restrict__ counts) {
+    const uint32_t lane = threadIdx.x & 31u, n_runs = run_first[eff];
+    for (uint32_t run = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); run < n_runs; run += gridDim.x * (kBlock / 32)) {
+        const uint32_t w = run_window[run], t0 = rowOffset[w] + (run - run_first[w]) * kRunTiles;
+        const uint32_t t1 = min(t0 + kRunTiles, rowOffset[w + 1]);
+        uint32_t mine = 0;
+#pragma unroll 4
+        for (uint32_t t = t0; t < t1; ++t) {
+            Piece<T> p;
+            p.load(data, t, lane);
+            mine += __popc(p.mask);
+        }
+        mine += __shfl_xor_sync(0xffffffffu, mine, 1);
+        if (!(lane & 1u)) counts[(uint64_t)run * 16 + (lane >> 1)] = mine;
+    }
+}
+
+// thread (window, row of it): counts of its runs become what the earlier runs hold; the sum is the row's length
+__global__ void row_lengths_kernel(const uint32_t *__restrict__ run_first, const uint32_t *__restrict__ rowIdx, uint32_t eff,
+                                   uint32_t rows, uint32_t *__restrict__ counts, uint32_t *__restrict__ row_len) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t w = (uint32_t)(i >> 4), r = (uint32_t)i & 15u;
+    if (w >= eff) return;
+    uint32_t sum = 0;
+    for (uint32_t run = run_first[w]; run < run_first[w + 1]; ++run) {
+        const uint32_t c = counts[(uint64_t)run * 16 + r];
+        counts[(uint64_t)run * 16 + r] = sum;
+        sum += c;
+    }
+    if (rowIdx[w] + r < rows) row_len[rowIdx[w] + r] = sum;
+}
+
+// Inclusive scans follow over both: (entries << 32 | units) and (cut rows << 32 | slots).
+__global__ void row_terms_kernel(const uint32_t *__restrict__ row_len, uint32_t rows, uint32_t cap, unsigned long long *__restrict__ a,
+                                 unsigned long long *__restrict__ b) {
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= rows) return;
+    const uint32_t len = row_len[r], n = pieces_of(len, cap);
+    a[r] = ((unsigned long long)len << 32) | n;
+    b[r] = n > 1 ? (1ull << 32) | n : 0ull;
+}
+
+// totals[0..3]: entries, units, cut rows, slots; then per band its first row and cut row
+__global__ void row_bands_kernel(uint32_t rows, const unsigned long long *__restrict__ a, const unsigned long long *__restrict__ b,
+                                 uint32_t *__restrict__ totals) {
+    const uint32_t k = threadIdx.x;
+    if (k == 0) {
+        totals[0] = (uint32_t)(a[rows - 1] >> 32);
+        totals[1] = (uint32_t)a[rows - 1];
+        totals[2] = (uint32_t)(b[rows - 1] >> 32);
+        totals[3] = (uint32_t)b[rows - 1];
+    }
+    if (k > kMaxBands) return;
+    const uint64_t cost = (a[rows - 1] >> 32) + kRowCost * rows;
+    const uint32_t bands = cost >= kMinBandedCost ? kMaxBands : 1u;
+    uint32_t lo = 0, hi = rows;  // rows before which k / bands of the cost lie
+    const uint64_t want = cost * k / bands;
+    while (k < bands && lo < hi) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        if ((a[mid] >> 32) + kRowCost * (mid + 1) <= want) lo = mid + 1; else hi = mid;
+    }
+    if (k >= bands) lo = rows;
+    totals[4 + k * 2] = lo;
+    totals[5 + k * 2] = lo ? (uint32_t)(b[lo - 1] >> 32) : 0u;
+}
+
+// one thread per row: sort keys of its units, and its line of the split table
+__global__ void unit_keys_kernel(const uint32_t *__restrict__ row_len, uint32_t rows, uint32_t cap, uint32_t bands,
+                                 const unsigned long long *__restrict__ a, const unsigned long long *__restrict__ b,
+                                 const uint32_t *__restrict__ totals, uint32_t *__restrict__ keys, uint32_t *__restrict__ ids,
+                                 uint32_t *__restrict__ unit_row, RowSplit *__restrict__ splits) {
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= rows) return;
+    const uint32_t len = row_len[r], n = pieces_of(len, cap), first = (uint32_t)a[r] - n;
+    uint32_t band = 0;
+    for (uint32_t k = 1; k < bands; ++k) band += r >= totals[4 + k * 2] ? 1u : 0u;
+    for (uint32_t q = 0; q < n; ++q) {
+        const uint32_t part = min(len - q * cap, cap);
+        keys[first + q] = (part ? 0u : kEmptyKey) | (band << 9) | (kMaxUnitEntries - part);
+        ids[first + q] = first + q;
+        unit_row[first + q] = r;
+    }
+    if (n > 1) splits[(uint32_t)(b[r] >> 32) - 1] = RowSplit{r, (uint32_t)b[r] - n, (uint32_t)b[r]};
+}
+
+__device__ __forceinline__ uint32_t batches_of_key(uint32_t key) { return (kMaxUnitEntries - (key & 511u) + kUnitBatch - 1) / kUnitBatch; }
+
+// Four neighbours of the sorted list form a quad and are stored batch by batch side by side (batch k of all four,
+// then batch k + 1): the groups of a warp, which walk neighbours, read their entries from the same lines.
+__global__ void quad_lengths_kernel(const uint32_t *__restrict__ keys, uint32_t n_units, uint32_t n_quads, uint32_t *__restrict__ quads) {
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q > n_quads) return;
+    uint32_t most = 0;
+    for (uint32_t i = 4 * q; i < min(4 * q + 4, n_units); ++i) most = max(most, batches_of_key(keys[i]));
+    quads[q] = most;  // (0 for q == n_quads: its place in the running sum is the total)
+}
+
+// place i of the sorted list: where the unit's batches lie, and the targets in them
+template <bool kTf32>
+__global__ void place_units_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ ids, const uint32_t *__restrict__ quads,
+                                   uint32_t n_units, uint32_t cap, const uint32_t *__restrict__ unit_row, const uint32_t *__restrict__ row_len,
+                                   const unsigned long long *__restrict__ a, const unsigned long long *__restrict__ b,
+                                   uint2 *__restrict__ units, uint32_t *__restrict__ unit_batch, uint32_t *__restrict__ batches) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_units) return;
+    const uint32_t u = ids[i], r = unit_row[u], n = pieces_of(row_len[r], cap), first = quads[i >> 2] * 4 + (i & 3u);
+    const uint32_t q = u - ((uint32_t)a[r] - n);  // which piece of its row
+    const uint32_t n_batches = batches_of_key(keys[i]);
+    units[i] = make_uint2(n_batches ? first : r, n_batches);
+    unit_batch[u] = first;
+    for (uint32_t k = 0; k < n_batches; ++k)
+        batches[(uint64_t)(first + 4 * k) * kBatchWords<kTf32> + kTargetWord<kTf32>] =
+            k + 1 < n_batches ? kNoTarget : n > 1 ? kSlotTarget | ((uint32_t)b[r] - n + q) : r;
+    if (i == n_units - 1) {  // the batch that belongs to nobody
+        uint32_t *w = batches + (uint64_t)quads[(n_units + 3) / 4] * 4 * kBatchWords<kTf32>;
+        for (uint32_t k = 0; k < kBatchWords<kTf32>; ++k) w[k] = k == kTargetWord<kTf32> ? kNoTarget : 0u;
+    }
+}
+
+// band k <= bands: the places of its first unit and of its first row without entries; and the number of batches
+__global__ void band_units_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ quads, uint32_t n_units,
+                                  uint32_t bands, uint32_t *__restrict__ out) {
+    const uint32_t i = threadIdx.x, k = i >> 1;
+    if (k > bands) {
+        if (k == bands + 1 && !(i & 1u)) out[i] = 4 * quads[(n_units + 3) / 4];
+        return;
+    }
+    const uint32_t want = ((i & 1u) ? kEmptyKey : 0u) + (k << 9);
+    uint32_t lo = 0, hi = n_units;
+    while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        if (keys[mid] < want) lo = mid + 1; else hi = mid;
+    }
+    out[i] = lo;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kBlock)
+write_entries_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B, const T *__restrict__ data,
+                     const uint32_t *__restrict__ rowIdx, const uint32_t *__restrict__ run_first,
+                     const uint32_t *__restrict__ run_window, uint32_t eff, uint32_t rows, uint32_t cap, const uint32_t *__restrict__ counts,
+                     const uint32_t *__restrict__ row_len, const unsigned long long *__restrict__ a,
+                     const uint32_t *__restrict__ unit_batch, uint32_t *__restrict__ batches) {
+    constexpr int kPer = Piece<T>::kPer;
+    constexpr uint32_t kWords = kBatchWords<sizeof(T) == 4>;
+    const uint32_t lane = threadIdx.x & 31u, n_runs = run_first[eff];
+    for (uint32_t run = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); run < n_runs; run += gridDim.x * (kBlock / 32)) {
+        const uint32_t w = run_window[run], t0 = rowOffset[w] + (run - run_first[w]) * kRunTiles;
+        const uint32_t t1 = min(t0 + kRunTiles, rowOffset[w + 1]), row = min(rowIdx[w] + (lane >> 1), rows - 1);
+        const uint32_t len = row_len[row];
+        const uint32_t *unit = unit_batch + ((uint32_t)a[row] - pieces_of(len, cap));  // first batches of the row's units
+        uint32_t at = counts[(uint64_t)run * 16 + (lane >> 1)];  // entries of the row so far
+        uint32_t piece = 0xFFFFFFFFu, piece_end = 0;
+        uint32_t *out = batches;
+        auto put = [&](uint32_t e, uint32_t col, T v) {
+            uint32_t *words = out + (e / kUnitBatch) * (4 * kWords);
+            words[e % kUnitBatch] = col;
+            reinterpret_cast<T *>(words + kUnitBatch)[e % kUnitBatch] = sizeof(T) == 2 ? v : (T)((uint32_t)v & 0xFFFFE000u);  // as the tensor core reads it
+        };
+#pragma unroll 2
+        for (uint32_t t = t0; t < t1; ++t) {
+            Piece<T> p;
+            p.load(data, t, lane);
+            const uint32_t mine = (uint32_t)__popc(p.mask), other = __shfl_xor_sync(0xffffffffu, mine, 1);
+            uint32_t k_out = at + ((lane & 1u) ? other : 0u);
+            at += mine + other;
+            const uint32_t *cols = tcA2B + (uint64_t)t * (2 * kPer) + (lane & 1u) * kPer;
+#pragma unroll
+            for (int k = 0; k < kPer; ++k)
+                if (p.mask & (1u << k)) {
+                    if (k_out >= piece_end) {
+                        piece = k_out / cap;
+                        piece_end = (piece + 1) * cap;
+                        out = batches + (uint64_t)unit[piece] * kWords;
+                    }
+                    const uint32_t e = k_out - piece * cap, col = cols[k];
+                    put(e, col, p.v[k]);
+                    if (++k_out == len)  // the row's last entry: fill its batch up
+                        for (uint32_t f = e + 1; f % kUnitBatch; ++f) put(f, col, (T)0);
+                }
+        }
+    }
+}
+
+// Entries of one row that are summed in one go; a longer row is cut.  A piece costs its slot, written and read
+// once - 3 % of the rows of B that 256 entries gather - so large matrices keep to the maximum.  On small ones a
+// warp's whole share is a few hundred entries and a unit of 256 would be the longest thing in the launch; but
+// ordinary rows stay whole (up to twice the mean), because cut rows cost a second launch.
+uint32_t unit_entries_for(uint64_t nnz, uint64_t rows, int n_sms) {
+    const uint64_t share = nnz / ((uint64_t)n_sms * 128), mean = rows ? nnz / rows : 0;
+    uint32_t cap = 64;
+    while (cap < kMaxUnitEntries && (cap < share || cap < 2 * mean)) cap *= 2;
+    return cap;
+}
+
+}  // namespace
+
+void free_rows(RowsFormat *r) {
+    pool_free(r->d_batches);
+    pool_free(r->d_units);
+    pool_free(r->d_splits);
+    *r = RowsFormat();
+}
+
+int build_rows_device(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOffset, const uint32_t *d_tcA2B,
+                      const void *d_data, const uint32_t *d_rowIdx, int n_sms, RowsFormat *out) {
+    *out = RowsFormat();
+    const uint64_t tiles = info.total_tiles;
+    if (!info.eff_row_windows || !tiles || info.rows >= kSlotTarget) return B200SPMM_OK;
+    const uint32_t rows = (uint32_t)info.rows, eff = (uint32_t)info.eff_row_windows;
+    const uint32_t cap = unit_entries_for(info.nnzs, info.rows, n_sms);
+    RowsFormat f;
+    struct Guard {
+        RowsFormat *f;
+        ~Guard() { if (f) free_rows(f); }
+    } guard{&f};
+    PoolScratch tmp;
+    const uint64_t max_runs = eff + tiles / kRunTiles;
+    uint32_t *n_runs = nullptr, *run_first = nullptr, *run_window = nullptr, *counts = nullptr, *row_len = nullptr, *totals = nullptr;
+    unsigned long long *a = nullptr, *b = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&n_runs, eff + 1));
+    B200_CUDA_TRY(tmp.alloc(&run_first, eff + 1));
+    B200_CUDA_TRY(tmp.alloc(&run_window, max_runs));
+    B200_CUDA_TRY(tmp.alloc(&counts, max_runs * 16));
+    B200_CUDA_TRY(tmp.alloc(&row_len, rows));
+    B200_CUDA_TRY(tmp.alloc(&a, rows));
+    B200_CUDA_TRY(tmp.alloc(&b, rows));
+    B200_CUDA_TRY(tmp.alloc(&totals, 4 + 2 * (kMaxBands + 1)));
+    size_t run_bytes = 0, row_bytes = 0;
+    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, run_bytes, n_runs, run_first, (int64_t)eff + 1));
+    B200_CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, row_bytes, a, a, (int64_t)rows));
+    uint8_t *scan_tmp = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&scan_tmp, std::max(run_bytes, row_bytes)));
+
+    run_counts_kernel<<<eff / kBlock + 1, kBlock>>>(d_rowOffset, eff, n_runs);
+    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(scan_tmp, run_bytes, n_runs, run_first, (int64_t)eff + 1));
+    run_windows_kernel<<<(eff + kBlock - 1) / kBlock, kBlock>>>(run_first, eff, run_window);
+    const bool f16 = info.elt_size == 2;
+    const uint16_t *data16 = static_cast<const uint16_t *>(d_data);
+    const uint32_t *data32 = static_cast<const uint32_t *>(d_data);
+    const int run_grid = grid_for(max_runs * 32), row_grid = (int)((rows + kBlock - 1) / kBlock);
+    if (f16) run_rows_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, data16, run_first, run_window, eff, counts);
+    else run_rows_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, data32, run_first, run_window, eff, counts);
+    B200_CUDA_TRY(cudaMemsetAsync(row_len, 0, (size_t)rows * 4));
+    row_lengths_kernel<<<(unsigned)(((uint64_t)eff * 16 + kBlock - 1) / kBlock), kBlock>>>(run_first, d_rowIdx, eff, rows, counts, row_len);
+    row_terms_kernel<<<row_grid, kBlock>>>(row_len, rows, cap, a, b);
+    B200_CUDA_TRY(cub::DeviceScan::InclusiveSum(scan_tmp, row_bytes, a, a, (int64_t)rows));
+    B200_CUDA_TRY(cub::DeviceScan::InclusiveSum(scan_tmp, row_bytes, b, b, (int64_t)rows));
+    row_bands_kernel<<<1, 32>>>(rows, a, b, totals);
+    B200_CUDA_TRY(cudaGetLastError());
+    uint32_t h[4 + 2 * (kMaxBands + 1)];
+    B200_CUDA_TRY(cudaMemcpy(h, totals, sizeof(h), cudaMemcpyDeviceToHost));
+    f.nnz = h[0];
+    f.n_units = h[1];
+    f.n_splits = h[2];
+    f.n_slots = h[3];
+    uint32_t bands = 0;
+    while (h[4 + 2 * bands] != rows) ++bands;
+    for (uint32_t k = 0; k <= bands; ++k) f.bands.push_back(RowBand{0, 0, h[5 + 2 * k], h[4 + 2 * k]});
+
+    // Every unit rounds up to a batch, every quad to its longest unit: up to three longest units for each band,
+    // as its lengths fall from first to last, and three more where a quad holds the end of one and the start of the next.
+    const uint64_t max_batches = f.nnz / kUnitBatch + f.n_units + kMaxBands * 6 * (kMaxUnitEntries / kUnitBatch) + 8;
+    if (max_batches > 0xFFFFFFFFull || f.n_slots >= kSlotTarget - 1) return B200SPMM_OK;
+    const uint32_t words = info.elt_size == 2 ? kBatchWords<false> : kBatchWords<true>;
+    uint32_t *keys[2] = {}, *ids[2] = {}, *unit_row = nullptr;
+    cudaError_t e = pool_alloc(&f.d_batches, max_batches * words);
+    if (e == cudaSuccess) e = pool_alloc(&f.d_units, f.n_units);
+    if (e == cudaSuccess) e = pool_alloc(&f.d_splits, f.n_splits);
+    for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
+        e = tmp.alloc(&keys[k], f.n_units);
+        if (e == cudaSuccess) e = tmp.alloc(&ids[k], f.n_units);
+    }
+    if (e == cudaSuccess) e = tmp.alloc(&unit_row, f.n_units);
+    if (e == cudaErrorMemoryAllocation) {  // no room: the tile kernels still work
+        cudaGetLastError();
+        return B200SPMM_OK;
+    }
+    B200_CUDA_TRY(e);
+    const uint32_t n_quads = (f.n_units + 3) / 4;
+    uint32_t *quads = nullptr, *unit_batch = keys[0];  // (free again once the pairs are sorted)
+    B200_CUDA_TRY(tmp.alloc(&quads, n_quads + 1));
+    const int key_bits = 13;
+    unit_keys_kernel<<<row_grid, kBlock>>>(row_len, rows, cap, bands, a, b, totals, keys[0], ids[0], unit_row, f.d_splits);
+    size_t sort_bytes = 0, batch_bytes = 0;
+    B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, keys[0], keys[1], ids[0], ids[1], (int64_t)f.n_units, 0, key_bits));
+    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, batch_bytes, quads, quads, (int64_t)n_quads + 1));
+    uint8_t *sort_tmp = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&sort_tmp, std::max(sort_bytes, batch_bytes)));
+    B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, keys[0], keys[1], ids[0], ids[1], (int64_t)f.n_units, 0, key_bits));
+    quad_lengths_kernel<<<(int)(n_quads / kBlock + 1), kBlock>>>(keys[1], f.n_units, n_quads, quads);
+    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(sort_tmp, batch_bytes, quads, quads, (int64_t)n_quads + 1));
+    const int unit_grid = (int)((f.n_units + kBlock - 1) / kBlock);
+    if (f16) {
+        place_units_kernel<false><<<unit_grid, kBlock>>>(keys[1], ids[1], quads, f.n_units, cap, unit_row, row_len, a, b, f.d_units,
+                                                         unit_batch, f.d_batches);
+        write_entries_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data16, d_rowIdx, run_first, run_window, eff, rows, cap,
+                                                             counts, row_len, a, unit_batch, f.d_batches);
+    } else {
+        place_units_kernel<true><<<unit_grid, kBlock>>>(keys[1], ids[1], quads, f.n_units, cap, unit_row, row_len, a, b, f.d_units,
+                                                        unit_batch, f.d_batches);
+        write_entries_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data32, d_rowIdx, run_first, run_window, eff, rows, cap,
+                                                             counts, row_len, a, unit_batch, f.d_batches);
+    }
+    band_units_kernel<<<1, 32>>>(keys[1], quads, f.n_units, bands, totals);
+    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(cudaMemcpy(h, totals, (2 * bands + 3) * 4, cudaMemcpyDeviceToHost));
+    for (uint32_t k = 0; k <= bands; ++k) {
+        f.bands[k].unit = h[2 * k];
+        f.bands[k].empty = h[2 * k + 1];
+    }
+    f.bands[bands].unit = f.bands[0].empty;  // (all units, then all rows without entries)
+    f.bands[bands].empty = f.n_units;
+    f.n_batches = h[2 * bands + 2];
+    B200_CUDA_TRY(cudaDeviceSynchronize());
+    *out = f;
+    guard.f = nullptr;
+    return B200SPMM_OK;
+}
+
+}  // namespace b200spmm

@@ -1,0 +1,51 @@
+// The matrix of a plan as row units (see spmm_rows_kernel.cuh), built on the device from the condensed tiles.
+#pragma once
+
+#include <cstdint>
+#include <cuda_runtime.h>
+#include <vector>
+
+#include "../../include/b200_spmm.h"
+#include "format.hpp"
+
+namespace b200spmm {
+
+// A unit is a row, or a piece of a long one.  Its entries lie in consecutive batches of four; the last batch is
+// filled up with its last column and zero values.  A batch is kBatchWords 32-bit words: four columns, four
+// values (fp16: two words, tf32: four, low 13 bits dropped), the target of the unit's sum in the unit's last
+// batch and kNoTarget in the others, padding to 16 bytes.
+constexpr uint32_t kMaxUnitEntries = 256;  // no unit is longer, see unit_entries_for
+constexpr uint32_t kUnitBatch = 4;
+template <bool kTf32>
+constexpr uint32_t kBatchWords = kTf32 ? 12 : 8;
+template <bool kTf32>
+constexpr uint32_t kTargetWord = kTf32 ? 8 : 6;
+constexpr uint32_t kSlotTarget = 0x80000000u, kNoTarget = 0xFFFFFFFFu;  // a row, or kSlotTarget | slot of a piece
+
+// A row that was cut: its pieces lie in slots [slot_begin, slot_end), in entry order.
+struct RowSplit {
+    uint32_t row, slot_begin, slot_end;
+};
+
+// A band of whole rows: where its units (longest first), its rows without entries (behind the units of all
+// bands), its cut rows and its rows begin.
+struct RowBand {
+    uint32_t unit, empty, split;
+    uint64_t row;
+};
+
+struct RowsFormat {
+    uint32_t *d_batches = nullptr;    // [n_batches + 1][kBatchWords], the last one belongs to nobody
+    uint2 *d_units = nullptr;         // [n_units] first batch and number of batches, or (row, 0) for one without entries
+    RowSplit *d_splits = nullptr;     // [n_splits] by row
+    uint64_t nnz = 0;
+    uint32_t n_batches = 0, n_units = 0, n_splits = 0, n_slots = 0;
+    std::vector<RowBand> bands;       // one more than there are bands: the last one holds the totals
+};
+
+// The tiles must be in the reference's layout (row-major 16 x CW).  Leaves *out empty when device memory is short.
+int build_rows_device(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOffset, const uint32_t *d_tcA2B,
+                      const void *d_data, const uint32_t *d_rowIdx, int n_sms, RowsFormat *out);
+void free_rows(RowsFormat *r);
+
+}  // namespace b200spmm

@@ -345,6 +345,13 @@ void b200spmm_plan_destroy(b200spmm_plan_t *p);
 int b200spmm_plan_info(const b200spmm_plan_t *p, b200spmm_btcf_info_t *info);
 
 /*
+ * The library keeps up to 512 MiB of the device memory it has freed per device, so that a caller who converts
+ * and plans a new matrix at every step does not pay for mapping memory each time (the reference allocates and
+ * frees everything on every call, src/fp16.cu:236-279).  This call gives all of it back to the driver.
+ */
+int b200spmm_release_cached_memory(int device);
+
+/*
  * C[rows, n] = A * B[cols, n] on the plan's device; B and C are device pointers, row-major
  * with leading dimensions ldb / ldc in elements.  Asynchronous on `stream` (a cudaStream_t).
  * Replaces the launch of fp16_spmm_kernel inside fp16_spmm (src/fp16.cu:36-175, 255-264)

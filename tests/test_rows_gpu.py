@@ -1,0 +1,57 @@
+"""The row-by-row kernel on the device against the CPU oracle, at the sizes where its cuts and lane groups can go
+wrong.  B200SPMM_WINDOW=rows sends any matrix down this path; nearly empty tiles take it by themselves."""
+import numpy as np
+import pytest
+
+import hopper_spmm_b200 as hs
+import parity
+from cases import dense_b
+
+pytestmark = pytest.mark.gpu
+
+
+def rows_of_lengths(lengths, cols, seed, dt):
+    rng = np.random.default_rng(seed)
+    ci = np.concatenate([np.sort(rng.choice(cols, k, replace=False)) for k in lengths]).astype(np.uint32)
+    v = rng.uniform(-1, 1, ci.size).astype(np.float32).astype(dt)
+    v[v == 0] = 1
+    return len(lengths), cols, np.concatenate([[0], np.cumsum(lengths)]).astype(np.uint32), ci, v
+
+
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+@pytest.mark.parametrize("n", [8, 24, 40, 64, 104, 128, 136, 520])
+def test_batches_units_and_pieces_at_their_edges(dt, n, monkeypatch):
+    # whole and ragged batches of four, rows of one unit, rows cut into two, three and many pieces, empty rows at
+    # both ends and in between; n covers one lane per row up to a full warp, lanes left over, a narrower last pass
+    import torch
+    monkeypatch.setenv("B200SPMM_WINDOW", "rows")
+    lengths = [0, 0, 1, 2, 3, 4, 5, 63, 64, 65, 0, 127, 128, 129, 255, 256, 257, 1000, 0, 7] + [9] * 40 + [0] * 21
+    rows, cols, rp, ci, v = rows_of_lengths(lengths, 1013, 3, dt)
+    Bfull = torch.from_numpy(dense_b(cols, n + 16, 9, dt)).cuda()
+    Bv = Bfull[:, 8:8 + n]
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    try:
+        Cfull = torch.full((rows, n + 24), float("nan"), device="cuda")  # every row must be written, and nothing else
+        plan.spmm(Bv, Cfull[:, 8:8 + n])
+        info = plan.launch_info()
+        assert info.row_window == 16 and info.stages == 0 and info.kernel_launches == 2
+        first = Cfull[:, 8:8 + n].clone()
+        parity.check(first.cpu().numpy(), rows, rp, ci, v, Bv.cpu().numpy())
+        assert torch.isnan(Cfull[:, :8]).all() and torch.isnan(Cfull[:, 8 + n:]).all()
+        plan.spmm(Bv, Cfull[:, 8:8 + n])
+        assert torch.equal(first, Cfull[:, 8:8 + n])
+        assert torch.equal(plan.spmm(Bv, c_half=True), first.half())
+    finally:
+        plan.close()
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 5), (17, 1), (3, 4000)])
+def test_smallest_matrices(rows, cols, monkeypatch):
+    monkeypatch.setenv("B200SPMM_WINDOW", "rows")
+    rows, cols, rp, ci, v = rows_of_lengths([min(cols, 1 + 700 * k) for k in range(rows)], cols, 1, np.float16)
+    B = dense_b(cols, 72, 2)
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    try:
+        parity.check(plan.spmm_host(B), rows, rp, ci, v, B)
+    finally:
+        plan.close()
