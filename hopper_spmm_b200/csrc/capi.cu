@@ -89,6 +89,7 @@ struct b200spmm_plan {
     // whose tiles are nearly empty keeps nothing else (rows_only).
     RowsFormat rows_fmt;
     bool rows_only = false;
+    bool may_time_out = false;   // a kernel with bounded waits was launched since the status word was last read
     bool has_tile_path = false;  // schedule and tile image of the 16-row kernel are there
     // Most tiles of the super-window format name one aligned group of CW consecutive rows of B: then B
     // is re-laid as shared-memory images at every launch (scratch of the plan, as large as B) and such a
@@ -225,15 +226,25 @@ int launch_slab(b200spmm_plan *p, SpmmParams &prm, const CUtensorMap &tmap_b, cu
     }
 }
 
+// A buffer of the plan that launches on any stream may use: what is there is given back once nothing uses it.
+template <typename T>
+int grow_buffer(T **buf, size_t bytes) {
+    if (*buf) B200_CUDA_TRY(cudaDeviceSynchronize());
+    pool_free(*buf);
+    *buf = nullptr;
+    void *ptr = nullptr;
+    B200_CUDA_TRY(pool_alloc_bytes(&ptr, bytes, nullptr));
+    B200_CUDA_TRY(cudaStreamSynchronize(nullptr));  // from here on the memory is there for every stream
+    *buf = static_cast<T *>(ptr);
+    return B200SPMM_OK;
+}
+
 // Slots for the pieces of windows or rows that are computed in parts, grown to the largest need seen.
 int grow_partial(b200spmm_plan *p, size_t floats) {
     if (floats <= p->partial_floats) return B200SPMM_OK;
-    cudaFree(p->d_partial);
-    p->d_partial = nullptr;
-    p->partial_floats = 0;
-    B200_CUDA_TRY(cudaMalloc(&p->d_partial, floats * sizeof(float)));
-    p->partial_floats = floats;
-    return B200SPMM_OK;
+    const int st = grow_buffer(&p->d_partial, floats * sizeof(float));
+    p->partial_floats = st == B200SPMM_OK ? floats : 0;
+    return st;
 }
 
 // The environment is consulted when a plan is made (and once per process for the plan-less
@@ -496,10 +507,9 @@ int launch_tall(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void 
         const uint32_t groups = (uint32_t)((p->info.cols + cw - 1) / cw);
         const size_t need = (size_t)n_slabs * groups * 32u * slab;
         if (need > p->b_packed_bytes) {
-            cudaFree(p->d_b_packed);
-            p->d_b_packed = nullptr;
             p->b_packed_bytes = 0;
-            B200_CUDA_TRY(cudaMalloc(&p->d_b_packed, need));
+            int st = grow_buffer(&p->d_b_packed, need);
+            if (st != B200SPMM_OK) return st;
             p->b_packed_bytes = need;
         }
         const int grid = (int)std::min<size_t>((need / 16 + 255) / 256, (size_t)p->n_sms * 16);
@@ -589,7 +599,7 @@ int plan_build_tile_image(b200spmm_plan *p) {
     if (!n_rows || p->comp.tcBit) return B200SPMM_OK;  // compressed tiles are expanded in the kernel
     void *dst = p->d_data;
     if (!p->owns_format) {
-        if (cudaMalloc(&dst, n_rows * 32) != cudaSuccess) {  // no room for a copy: the tiled loads still work
+        if (pool_alloc_bytes(&dst, n_rows * 32, nullptr) != cudaSuccess) {  // no room for a copy: the tiled loads still work
             cudaGetLastError();
             return B200SPMM_OK;
         }
@@ -608,7 +618,7 @@ int plan_build_schedule(b200spmm_plan *p, const uint32_t *h_rowOffset, const uin
     const auto &info = p->info;
     auto upload = [](auto **dst, const auto &v) -> int {
         using T = typename std::remove_reference<decltype(v)>::type::value_type;
-        B200_CUDA_TRY(cudaMalloc(dst, std::max<size_t>(v.size() * sizeof(T), 16)));
+        B200_CUDA_TRY(pool_alloc(dst, v.size()));
         if (!v.empty()) B200_CUDA_TRY(cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
         return B200SPMM_OK;
     };
@@ -665,7 +675,7 @@ int plan_build_tile_path(b200spmm_plan *p, const uint32_t *h_rowOffset, const ui
     // quarter of the dense bytes - which a producer warp expands with two stores per lane; tiles with more than
     // 32 entries still come from the dense image.  Same C bit for bit.
     if (info.total_tiles && info.dtype == B200SPMM_F16 && env_is("B200SPMM_TILES", "entries")) {
-        B200_CUDA_TRY(cudaMalloc(&p->d_tile_entries, info.total_tiles * 128));
+        B200_CUDA_TRY(pool_alloc(&p->d_tile_entries, info.total_tiles * 32));
         unsigned long long *d_count = nullptr;
         B200_CUDA_TRY(cudaMalloc(&d_count, 8));
         B200_CUDA_TRY(cudaMemset(d_count, 0, 8));
@@ -686,6 +696,15 @@ int plan_build_tile_path(b200spmm_plan *p, const uint32_t *h_rowOffset, const ui
     return plan_build_tile_image(p);
 }
 
+// The window tables on the host, read back where the caller has them on the device only.
+int plan_add_tile_path(b200spmm_plan *p, int n_ctas) {
+    std::vector<uint32_t> h_rowOffset(p->info.eff_row_windows + 1), h_rowIdx(p->info.eff_row_windows);
+    B200_CUDA_TRY(cudaMemcpy(h_rowOffset.data(), p->d_rowOffset, h_rowOffset.size() * 4, cudaMemcpyDeviceToHost));
+    if (!h_rowIdx.empty()) B200_CUDA_TRY(cudaMemcpy(h_rowIdx.data(), p->d_rowIdx, h_rowIdx.size() * 4, cudaMemcpyDeviceToHost));
+    return plan_build_tile_path(p, h_rowOffset.data(), h_rowIdx.data(), n_ctas);
+}
+
+// h_rowOffset and h_rowIdx may be null: they are read back if the plan needs them.
 int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h_rowIdx, int n_ctas) {
     const auto &info = p->info;
     if (info.row_window != kRowWindow) return B200SPMM_ERR_UNSUPPORTED;
@@ -697,7 +716,7 @@ int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h
     if (major != 10) return B200SPMM_ERR_NO_DEVICE;
     B200_CUDA_TRY(cudaDeviceGetAttribute(&p->n_sms, cudaDevAttrMultiProcessorCount, p->device));
     // status word, then the two counters of the chunk hand-out (the kernel leaves them at zero)
-    B200_CUDA_TRY(cudaMalloc(&p->d_status, 4 * sizeof(uint32_t)));
+    B200_CUDA_TRY(pool_alloc(&p->d_status, 4));
     B200_CUDA_TRY(cudaMemset(p->d_status, 0, 4 * sizeof(uint32_t)));
     p->gather_cpasync = env_is("B200SPMM_GATHER", "cpasync");
     p->host_split = !env_is("B200SPMM_HOST_SPLIT", "0");
@@ -712,7 +731,7 @@ int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h
         if (p->rows_only) return B200SPMM_OK;
         free_rows(&p->rows_fmt);
     }
-    return plan_build_tile_path(p, h_rowOffset, h_rowIdx, n_ctas);
+    return h_rowOffset ? plan_build_tile_path(p, h_rowOffset, h_rowIdx, n_ctas) : plan_add_tile_path(p, n_ctas);
 }
 
 }  // namespace
@@ -936,38 +955,39 @@ int b200spmm_build_row_bands(const uint32_t *rowOffset, const uint32_t *rowIdx, 
 void b200spmm_plan_destroy(b200spmm_plan_t *p) {
     if (!p) return;
     cudaSetDevice(p->device);
+    cudaDeviceSynchronize();  // a launch may still be using the plan
     if (p->owns_format) {
-        cudaFree(p->d_rowOffset);
-        cudaFree(p->d_tcA2B);
-        cudaFree(p->d_rowIdx);
-        cudaFree(p->d_data);
+        pool_free(p->d_rowOffset);
+        pool_free(p->d_tcA2B);
+        pool_free(p->d_rowIdx);
+        pool_free(p->d_data);
     }
     {
         auto &ps = p->sched;
-        cudaFree(ps.d_tile);
-        cudaFree(ps.d_wfirst);
-        cudaFree(ps.d_wlast);
-        cudaFree(ps.d_head_slot);
-        cudaFree(ps.d_tail_slot);
-        cudaFree(ps.d_splits);
-        cudaFree(ps.d_piece_slots);
+        pool_free(ps.d_tile);
+        pool_free(ps.d_wfirst);
+        pool_free(ps.d_wlast);
+        pool_free(ps.d_head_slot);
+        pool_free(ps.d_tail_slot);
+        pool_free(ps.d_splits);
+        pool_free(ps.d_piece_slots);
     }
     free_compressed_tiles(&p->comp);
     free_rows(&p->rows_fmt);
-    cudaFree(p->d_tile_entries);
+    pool_free(p->d_tile_entries);
     free_tall(&p->tall);
     free_tall(&p->pair);
-    cudaFree(p->d_b_packed);
-    if (p->image_is_copy) cudaFree(p->d_tiles_image);
+    pool_free(p->d_b_packed);
+    if (p->image_is_copy) pool_free(p->d_tiles_image);
     for (cudaEvent_t e : p->band_done) cudaEventDestroy(e);
     if (p->copy_stream) cudaStreamDestroy(p->copy_stream);
     if (p->upload_stream) cudaStreamDestroy(p->upload_stream);
     for (cudaEvent_t e : p->half_up)
         if (e) cudaEventDestroy(e);
-    cudaFree(p->d_partial);
-    cudaFree(p->d_status);
-    cudaFree(p->d_B);
-    cudaFree(p->d_C);
+    pool_free(p->d_partial);
+    pool_free(p->d_status);
+    pool_free(p->d_B);
+    pool_free(p->d_C);
     delete p;
 }
 
@@ -991,7 +1011,7 @@ int b200spmm_plan_create(const b200spmm_btcf_t *h, int device, int n_ctas, b200s
     b200spmm_btcf_info(h, &p->info);
     const Btcf &f = h->f;
     auto upload = [&](void **dst, const void *src, size_t bytes) -> int {
-        B200_CUDA_TRY(cudaMalloc(dst, std::max<size_t>(bytes, 16)));
+        B200_CUDA_TRY(pool_alloc_bytes(dst, std::max<size_t>(bytes, 16), nullptr));
         if (bytes) B200_CUDA_TRY(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
         return B200SPMM_OK;
     };
@@ -1030,20 +1050,14 @@ int b200spmm_plan_create_device(const b200spmm_btcf_info_t *info, const uint32_t
     p->d_tcA2B = const_cast<uint32_t *>(d_tcA2B);
     p->d_rowIdx = const_cast<uint32_t *>(d_rowIdx);
     p->d_data = const_cast<void *>(d_data);
-    std::vector<uint32_t> h_rowOffset(info->eff_row_windows + 1);
     int st = B200SPMM_OK;
-    if (cudaMemcpy(h_rowOffset.data(), d_rowOffset, h_rowOffset.size() * 4, cudaMemcpyDeviceToHost) != cudaSuccess) {
+    uint32_t tiles = 0;
+    if (cudaMemcpy(&tiles, d_rowOffset + info->eff_row_windows, 4, cudaMemcpyDeviceToHost) != cudaSuccess) {
         record_cuda_error(cudaGetLastError(), "cudaMemcpy(rowOffset)");
         st = B200SPMM_ERR_CUDA;
     }
-    if (st == B200SPMM_OK && h_rowOffset[info->eff_row_windows] != info->total_tiles) st = B200SPMM_ERR_INVALID_ARG;
-    std::vector<uint32_t> h_rowIdx(info->eff_row_windows);
-    if (st == B200SPMM_OK && info->eff_row_windows &&
-        cudaMemcpy(h_rowIdx.data(), d_rowIdx, h_rowIdx.size() * 4, cudaMemcpyDeviceToHost) != cudaSuccess) {
-        record_cuda_error(cudaGetLastError(), "cudaMemcpy(rowIdx)");
-        st = B200SPMM_ERR_CUDA;
-    }
-    if (st == B200SPMM_OK) st = plan_finish(p, h_rowOffset.data(), h_rowIdx.data(), n_ctas);
+    if (st == B200SPMM_OK && tiles != info->total_tiles) st = B200SPMM_ERR_INVALID_ARG;
+    if (st == B200SPMM_OK) st = plan_finish(p, nullptr, nullptr, n_ctas);
     if (st != B200SPMM_OK) {
         b200spmm_plan_destroy(p);
         return st;
@@ -1128,13 +1142,6 @@ int b200spmm_plan_launch_info(const b200spmm_plan_t *p, b200spmm_launch_info_t *
 
 namespace {
 
-int plan_add_tile_path(b200spmm_plan *p) {
-    std::vector<uint32_t> h_rowOffset(p->info.eff_row_windows + 1), h_rowIdx(p->info.eff_row_windows);
-    B200_CUDA_TRY(cudaMemcpy(h_rowOffset.data(), p->d_rowOffset, h_rowOffset.size() * 4, cudaMemcpyDeviceToHost));
-    B200_CUDA_TRY(cudaMemcpy(h_rowIdx.data(), p->d_rowIdx, h_rowIdx.size() * 4, cudaMemcpyDeviceToHost));
-    return plan_build_tile_path(p, h_rowOffset.data(), h_rowIdx.data(), 0);
-}
-
 // The product, or one band of it (band < 0: every chunk; otherwise the chunks, rows and split
 // windows of that band of the schedule the launch selects - see b200spmm_plan::Sched).
 int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
@@ -1154,9 +1161,10 @@ int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, voi
     }
     if (!p->starve_gathers && use_rows(p, ldb)) return launch_rows(p, d_B, ldb, n, d_C, ldc, c_dtype, stream, band);
     if (!p->has_tile_path) {  // only row units were kept; the starved test launch and a huge ldb ask for more
-        int st = plan_add_tile_path(p);
+        int st = plan_add_tile_path(p, 0);
         if (st != B200SPMM_OK) return st;
     }
+    p->may_time_out = true;
     if (band < 0 && use_tall(p, n)) return launch_tall(p, d_B, ldb, n, d_C, ldc, c_dtype, stream);
     SpmmParams prm{};
     prm.rowOffset = p->d_rowOffset;
@@ -1236,8 +1244,10 @@ int b200spmm_plan_sync(b200spmm_plan_t *p, void *stream_v) {
     if (!p) return B200SPMM_ERR_INVALID_ARG;
     B200_CUDA_TRY(cudaSetDevice(p->device));
     B200_CUDA_TRY(cudaStreamSynchronize(static_cast<cudaStream_t>(stream_v)));
+    if (!p->may_time_out) return B200SPMM_OK;  // (row units wait for nothing)
     uint32_t status = 0;
     B200_CUDA_TRY(cudaMemcpy(&status, p->d_status, sizeof(status), cudaMemcpyDeviceToHost));
+    p->may_time_out = false;
     if (status) {
         B200_CUDA_TRY(cudaMemset(p->d_status, 0, 4 * sizeof(uint32_t)));  // status and the hand-out counters
         return B200SPMM_ERR_DEVICE_TIMEOUT;
@@ -1252,17 +1262,15 @@ int b200spmm_spmm_host(b200spmm_plan_t *p, const void *h_B, int64_t n, void *h_C
     const size_t b_bytes = (size_t)p->info.cols * n * p->info.elt_size;
     const size_t c_bytes = (size_t)p->info.rows * n * (c_dtype == B200SPMM_C_F32 ? 4 : 2);
     if (b_bytes > p->d_B_bytes) {
-        cudaFree(p->d_B);
-        p->d_B = nullptr;
         p->d_B_bytes = 0;
-        B200_CUDA_TRY(cudaMalloc(&p->d_B, b_bytes));
+        int st = grow_buffer(&p->d_B, b_bytes);
+        if (st != B200SPMM_OK) return st;
         p->d_B_bytes = b_bytes;
     }
     if (c_bytes > p->d_C_bytes) {
-        cudaFree(p->d_C);
-        p->d_C = nullptr;
         p->d_C_bytes = 0;
-        B200_CUDA_TRY(cudaMalloc(&p->d_C, c_bytes));
+        int st = grow_buffer(&p->d_C, c_bytes);
+        if (st != B200SPMM_OK) return st;
         p->d_C_bytes = c_bytes;
     }
     const bool rows = use_rows(p, n);

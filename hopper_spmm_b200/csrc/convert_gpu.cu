@@ -6,7 +6,8 @@
 // the device.
 //
 // Steps (all integer work, bound by HBM traffic):
-//   1. one key (window << 32 | column) per entry, the entry's row found by binary search in row_ptr
+//   1. one key (window, column) per entry, in as few bits as the matrix needs - 32-bit keys where they fit - since
+//      every eight bits are a pass of the sort; the entry's row is found by binary search in row_ptr
 //   2. radix sort of the keys, then unique -> the sorted distinct columns of every window
 //      (CUB device primitives: sort, select-unique, run-length encode, scans)
 //   3. run lengths per window -> tiles per window -> rowOffset, rowIdx; column lists scattered into
@@ -20,6 +21,7 @@
 
 #include "../../include/b200_spmm.h"
 #include "common.hpp"
+#include "device_pool.hpp"
 #include "format.hpp"
 
 struct b200spmm_dbtcf {
@@ -44,22 +46,25 @@ __device__ __forceinline__ uint32_t row_of_entry(const uint32_t *__restrict__ ro
     return lo;
 }
 
-// keys[p] = window(p) << 32 | col[p]; row_of[p]; flags a column out of range or a row whose
+// keys[p] = window(p) << col_bits | col[p]; row_of[p]; flags a column out of range or a row whose
 // columns are not strictly ascending.
+template <typename K>
 __global__ void make_keys_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ col_idx,
-                                 uint32_t rows, uint32_t cols, uint64_t nnz, uint32_t row_window,
-                                 uint64_t *__restrict__ keys, uint32_t *__restrict__ row_of, uint32_t *__restrict__ bad) {
+                                 uint32_t rows, uint32_t cols, uint64_t nnz, uint32_t row_window, int col_bits,
+                                 K *__restrict__ keys, uint32_t *__restrict__ row_of, uint32_t *__restrict__ bad) {
     for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t r = row_of_entry(row_ptr, rows, (uint32_t)p);
         const uint32_t c = col_idx[p];
         if (c >= cols || (p > row_ptr[r] && col_idx[p - 1] >= c)) atomicOr(bad, 1u);
-        keys[p] = ((uint64_t)(r / row_window) << 32) | c;
+        keys[p] = ((K)(r / row_window) << col_bits) | c;
         row_of[p] = r;
     }
 }
 
+template <typename K>
 struct WindowOfKey {
-    __host__ __device__ uint32_t operator()(uint64_t k) const { return (uint32_t)(k >> 32); }
+    int col_bits;
+    __host__ __device__ uint32_t operator()(K k) const { return (uint32_t)(k >> col_bits); }
 };
 
 // per effective window e: tiles, first row; dense map window -> e
@@ -75,15 +80,16 @@ __global__ void window_tables_kernel(const uint32_t *__restrict__ win_ids, const
 }
 
 // distinct column j (sorted by window, column) -> its place in the window's padded column list
-__global__ void scatter_columns_kernel(const uint64_t *__restrict__ ukeys, uint64_t n_unique,
+template <typename K>
+__global__ void scatter_columns_kernel(const K *__restrict__ ukeys, uint64_t n_unique, int col_bits,
                                        const uint32_t *__restrict__ win2eff, const uint32_t *__restrict__ ubase,
                                        const uint32_t *__restrict__ rowOffset, uint32_t col_window,
                                        uint32_t *__restrict__ tcA2B) {
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n_unique; j += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t k = ukeys[j];
-        const uint32_t e = win2eff[(uint32_t)(k >> 32)];
+        const K k = ukeys[j];
+        const uint32_t e = win2eff[(uint32_t)(k >> col_bits)];
         const uint64_t pos = j - ubase[e];
-        tcA2B[(uint64_t)rowOffset[e] * col_window + pos] = (uint32_t)k;
+        tcA2B[(uint64_t)rowOffset[e] * col_window + pos] = (uint32_t)(k & (((K)1 << col_bits) - 1));
     }
 }
 
@@ -108,21 +114,106 @@ __global__ void scatter_values_kernel(const uint32_t *__restrict__ col_idx, cons
     }
 }
 
-struct Scratch {  // device buffers released on every exit path
-    void *ptrs[16] = {};
-    int n = 0;
-    template <typename T>
-    cudaError_t alloc(T **out, size_t count) {
-        void *p = nullptr;
-        cudaError_t e = cudaMalloc(&p, std::max<size_t>(count * sizeof(T), 16));
-        if (e == cudaSuccess) ptrs[n++] = p;
-        *out = static_cast<T *>(p);
-        return e;
-    }
-    ~Scratch() { for (int i = 0; i < n; ++i) cudaFree(ptrs[i]); }
-};
-
 inline int grid_for(uint64_t n) { return (int)std::min<uint64_t>((n + kBlock - 1) / kBlock, 148 * 32); }
+
+// Steps 1 - 4, with keys of key_bits bits (col_bits of them the column).
+template <typename K>
+int convert_on_device(b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const uint32_t *d_col_idx, const void *d_values, int col_bits,
+                      int key_bits, cudaStream_t stream) {
+    const uint64_t rows = f->info.rows, cols = f->info.cols, nnz = f->info.nnzs, n_windows = f->info.total_row_windows;
+    const uint32_t RW = (uint32_t)f->info.row_window, CW = (uint32_t)f->info.col_window;
+    const int esz = f->info.elt_size;
+    PoolScratch tmp(stream);
+    K *keys = nullptr, *keys_sorted = nullptr, *ukeys = nullptr;
+    uint64_t *n_sel = nullptr;
+    uint32_t *row_of = nullptr, *bad = nullptr, *win_ids = nullptr, *counts = nullptr, *n_runs = nullptr;
+    uint32_t *tiles = nullptr, *ubase = nullptr, *win2eff = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&keys, nnz));
+    B200_CUDA_TRY(tmp.alloc(&keys_sorted, nnz));
+    B200_CUDA_TRY(tmp.alloc(&row_of, nnz));
+    B200_CUDA_TRY(tmp.alloc(&bad, 1));
+    B200_CUDA_TRY(tmp.alloc(&n_sel, 1));
+    B200_CUDA_TRY(tmp.alloc(&n_runs, 1));
+    B200_CUDA_TRY(cudaMemsetAsync(bad, 0, 4, stream));
+
+    // 1. keys
+    make_keys_kernel<<<grid_for(nnz), kBlock, 0, stream>>>(d_row_ptr, d_col_idx, (uint32_t)rows, (uint32_t)cols, nnz, RW,
+                                                           col_bits, keys, row_of, bad);
+    B200_CUDA_TRY(cudaGetLastError());
+
+    // 2. sort, unique
+    size_t sort_bytes = 0, sel_bytes = 0, rle_bytes = 0, scan_bytes = 0;
+    B200_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, keys, keys_sorted, (int64_t)nnz, 0, key_bits, stream));
+    ukeys = keys;  // the unsorted keys are dead once sorted: reuse their buffer for the distinct keys
+    B200_CUDA_TRY(cub::DeviceSelect::Unique(nullptr, sel_bytes, keys_sorted, ukeys, n_sel, (int64_t)nnz, stream));
+    uint8_t *cub_tmp = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&cub_tmp, std::max(sort_bytes, sel_bytes)));
+    B200_CUDA_TRY(cub::DeviceRadixSort::SortKeys(cub_tmp, sort_bytes, keys, keys_sorted, (int64_t)nnz, 0, key_bits, stream));
+    B200_CUDA_TRY(cub::DeviceSelect::Unique(cub_tmp, sel_bytes, keys_sorted, ukeys, n_sel, (int64_t)nnz, stream));
+    uint64_t n_unique = 0;
+    uint32_t bad_h = 0;
+    B200_CUDA_TRY(cudaMemcpyAsync(&n_unique, n_sel, 8, cudaMemcpyDeviceToHost, stream));
+    B200_CUDA_TRY(cudaMemcpyAsync(&bad_h, bad, 4, cudaMemcpyDeviceToHost, stream));
+    B200_CUDA_TRY(cudaStreamSynchronize(stream));
+    if (bad_h) return B200SPMM_ERR_BAD_CSR;
+
+    // 3. windows: run lengths of the window id over the distinct keys
+    B200_CUDA_TRY(tmp.alloc(&win_ids, std::min<uint64_t>(n_windows, n_unique)));
+    B200_CUDA_TRY(tmp.alloc(&counts, std::min<uint64_t>(n_windows, n_unique) + 1));
+    auto win_of = thrust::make_transform_iterator(static_cast<const K *>(ukeys), WindowOfKey<K>{col_bits});
+    B200_CUDA_TRY(cub::DeviceRunLengthEncode::Encode(nullptr, rle_bytes, win_of, win_ids, counts, n_runs, (int64_t)n_unique, stream));
+    uint8_t *rle_tmp = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&rle_tmp, rle_bytes));
+    B200_CUDA_TRY(cub::DeviceRunLengthEncode::Encode(rle_tmp, rle_bytes, win_of, win_ids, counts, n_runs, (int64_t)n_unique, stream));
+    uint32_t eff = 0;
+    B200_CUDA_TRY(cudaMemcpyAsync(&eff, n_runs, 4, cudaMemcpyDeviceToHost, stream));
+    B200_CUDA_TRY(cudaStreamSynchronize(stream));
+
+    B200_CUDA_TRY(tmp.alloc(&tiles, (uint64_t)eff + 1));
+    B200_CUDA_TRY(tmp.alloc(&ubase, (uint64_t)eff + 1));
+    B200_CUDA_TRY(tmp.alloc(&win2eff, n_windows));
+    B200_CUDA_TRY(pool_alloc(&f->d_rowOffset, (uint64_t)eff + 1, stream));
+    B200_CUDA_TRY(pool_alloc(&f->d_rowIdx, eff, stream));
+    B200_CUDA_TRY(cudaMemsetAsync(tiles + eff, 0, 4, stream));
+    B200_CUDA_TRY(cudaMemsetAsync(counts + eff, 0, 4, stream));
+    window_tables_kernel<<<(eff + kBlock - 1) / kBlock, kBlock, 0, stream>>>(win_ids, counts, eff, RW, CW, tiles,
+                                                                             f->d_rowIdx, win2eff);
+    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, tiles, f->d_rowOffset, (int)(eff + 1), stream));
+    uint8_t *scan_tmp = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&scan_tmp, scan_bytes));
+    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, tiles, f->d_rowOffset, (int)(eff + 1), stream));
+    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, counts, ubase, (int)(eff + 1), stream));
+    uint32_t total_tiles = 0;
+    B200_CUDA_TRY(cudaMemcpyAsync(&total_tiles, f->d_rowOffset + eff, 4, cudaMemcpyDeviceToHost, stream));
+    B200_CUDA_TRY(cudaStreamSynchronize(stream));
+    // (a tile count beyond 32 bits would have wrapped in the scan: bound it by the entry count instead)
+    if ((uint64_t)n_unique / CW + eff > 0xFFFFFFFFull) return B200SPMM_ERR_UNSUPPORTED;
+
+    f->info.eff_row_windows = eff;
+    f->info.total_tiles = total_tiles;
+    const uint64_t list_len = (uint64_t)total_tiles * CW, data_len = (uint64_t)total_tiles * RW * CW;
+    B200_CUDA_TRY(pool_alloc(&f->d_tcA2B, list_len, stream));
+    B200_CUDA_TRY(pool_alloc_bytes(&f->d_data, std::max<uint64_t>(data_len * esz, 16), stream));
+    B200_CUDA_TRY(cudaMemsetAsync(f->d_tcA2B, 0xFF, list_len * 4, stream));  // kIdxMax padding
+    B200_CUDA_TRY(cudaMemsetAsync(f->d_data, 0, data_len * esz, stream));
+    scatter_columns_kernel<<<grid_for(n_unique), kBlock, 0, stream>>>(ukeys, n_unique, col_bits, win2eff, ubase, f->d_rowOffset, CW,
+                                                                      f->d_tcA2B);
+    B200_CUDA_TRY(cudaGetLastError());
+
+    // 4. values
+    if (esz == 2)
+        scatter_values_kernel<uint16_t><<<grid_for(nnz), kBlock, 0, stream>>>(
+            d_col_idx, static_cast<const uint16_t *>(d_values), row_of, nnz, win2eff, f->d_rowOffset, counts, f->d_tcA2B,
+            RW, CW, static_cast<uint16_t *>(f->d_data));
+    else
+        scatter_values_kernel<uint32_t><<<grid_for(nnz), kBlock, 0, stream>>>(
+            d_col_idx, static_cast<const uint32_t *>(d_values), row_of, nnz, win2eff, f->d_rowOffset, counts, f->d_tcA2B,
+            RW, CW, static_cast<uint32_t *>(f->d_data));
+    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(cudaStreamSynchronize(stream));
+    return B200SPMM_OK;
+}
 
 }  // namespace gpuconv
 }  // namespace b200spmm
@@ -135,10 +226,11 @@ extern "C" {
 void b200spmm_dbtcf_destroy(b200spmm_dbtcf_t *f) {
     if (!f) return;
     cudaSetDevice(f->device);
-    cudaFree(f->d_rowOffset);
-    cudaFree(f->d_tcA2B);
-    cudaFree(f->d_rowIdx);
-    cudaFree(f->d_data);
+    cudaDeviceSynchronize();  // a product may still be reading the arrays
+    pool_free(f->d_rowOffset);
+    pool_free(f->d_tcA2B);
+    pool_free(f->d_rowIdx);
+    pool_free(f->d_data);
     delete f;
 }
 
@@ -179,7 +271,7 @@ int b200spmm_csr2btcf_nobitmap_device(uint64_t rows, uint64_t cols, uint64_t nnz
     if (rows >= 0xFFFFFFFFull || cols > 0xFFFFFFFFull || nnz > 0xFFFFFFFFull) return B200SPMM_ERR_UNSUPPORTED;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     B200_CUDA_TRY(cudaSetDevice(device));
-    const uint32_t RW = (uint32_t)row_window, CW = (uint32_t)col_window;
+    const uint32_t RW = (uint32_t)row_window;
     const int esz = dtype == B200SPMM_F16 ? 2 : 4;
     const uint64_t n_windows = (rows + RW - 1) / RW;
 
@@ -207,7 +299,7 @@ int b200spmm_csr2btcf_nobitmap_device(uint64_t rows, uint64_t cols, uint64_t nnz
         if (head[0] != 0 || head[1] != nnz) return B200SPMM_ERR_BAD_CSR;
     }
     if (nnz == 0) {
-        B200_CUDA_TRY(cudaMalloc(&f->d_rowOffset, 16));
+        B200_CUDA_TRY(pool_alloc(&f->d_rowOffset, 4, stream));
         B200_CUDA_TRY(cudaMemsetAsync(f->d_rowOffset, 0, 16, stream));
         B200_CUDA_TRY(cudaStreamSynchronize(stream));
         guard.f = nullptr;
@@ -215,96 +307,13 @@ int b200spmm_csr2btcf_nobitmap_device(uint64_t rows, uint64_t cols, uint64_t nnz
         return B200SPMM_OK;
     }
 
-    Scratch tmp;
-    uint64_t *keys = nullptr, *keys_sorted = nullptr, *ukeys = nullptr, *n_sel = nullptr;
-    uint32_t *row_of = nullptr, *bad = nullptr, *win_ids = nullptr, *counts = nullptr, *n_runs = nullptr;
-    uint32_t *tiles = nullptr, *ubase = nullptr, *win2eff = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&keys, nnz));
-    B200_CUDA_TRY(tmp.alloc(&keys_sorted, nnz));
-    B200_CUDA_TRY(tmp.alloc(&row_of, nnz));
-    B200_CUDA_TRY(tmp.alloc(&bad, 1));
-    B200_CUDA_TRY(tmp.alloc(&n_sel, 1));
-    B200_CUDA_TRY(tmp.alloc(&n_runs, 1));
-    B200_CUDA_TRY(cudaMemsetAsync(bad, 0, 4, stream));
-
-    // 1. keys
-    make_keys_kernel<<<grid_for(nnz), kBlock, 0, stream>>>(d_row_ptr, d_col_idx, (uint32_t)rows, (uint32_t)cols, nnz, RW,
-                                                           keys, row_of, bad);
-    B200_CUDA_TRY(cudaGetLastError());
-
-    // 2. sort, unique
-    int win_bits = 1;
+    int win_bits = 1, col_bits = 1;
     while ((1ull << win_bits) < n_windows) ++win_bits;
-    size_t sort_bytes = 0, sel_bytes = 0, rle_bytes = 0, scan_bytes = 0;
-    B200_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, keys, keys_sorted, (int64_t)nnz, 0, 32 + win_bits, stream));
-    ukeys = keys;  // the unsorted keys are dead once sorted: reuse their buffer for the distinct keys
-    B200_CUDA_TRY(cub::DeviceSelect::Unique(nullptr, sel_bytes, keys_sorted, ukeys, n_sel, (int64_t)nnz, stream));
-    uint8_t *cub_tmp = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&cub_tmp, std::max(sort_bytes, sel_bytes)));
-    B200_CUDA_TRY(cub::DeviceRadixSort::SortKeys(cub_tmp, sort_bytes, keys, keys_sorted, (int64_t)nnz, 0, 32 + win_bits, stream));
-    B200_CUDA_TRY(cub::DeviceSelect::Unique(cub_tmp, sel_bytes, keys_sorted, ukeys, n_sel, (int64_t)nnz, stream));
-    uint64_t n_unique = 0;
-    uint32_t bad_h = 0;
-    B200_CUDA_TRY(cudaMemcpyAsync(&n_unique, n_sel, 8, cudaMemcpyDeviceToHost, stream));
-    B200_CUDA_TRY(cudaMemcpyAsync(&bad_h, bad, 4, cudaMemcpyDeviceToHost, stream));
-    B200_CUDA_TRY(cudaStreamSynchronize(stream));
-    if (bad_h) return B200SPMM_ERR_BAD_CSR;
-
-    // 3. windows: run lengths of the window id over the distinct keys
-    B200_CUDA_TRY(tmp.alloc(&win_ids, std::min<uint64_t>(n_windows, n_unique)));
-    B200_CUDA_TRY(tmp.alloc(&counts, std::min<uint64_t>(n_windows, n_unique) + 1));
-    auto win_of = thrust::make_transform_iterator(static_cast<const uint64_t *>(ukeys), WindowOfKey());
-    B200_CUDA_TRY(cub::DeviceRunLengthEncode::Encode(nullptr, rle_bytes, win_of, win_ids, counts, n_runs, (int64_t)n_unique, stream));
-    uint8_t *rle_tmp = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&rle_tmp, rle_bytes));
-    B200_CUDA_TRY(cub::DeviceRunLengthEncode::Encode(rle_tmp, rle_bytes, win_of, win_ids, counts, n_runs, (int64_t)n_unique, stream));
-    uint32_t eff = 0;
-    B200_CUDA_TRY(cudaMemcpyAsync(&eff, n_runs, 4, cudaMemcpyDeviceToHost, stream));
-    B200_CUDA_TRY(cudaStreamSynchronize(stream));
-
-    B200_CUDA_TRY(tmp.alloc(&tiles, (uint64_t)eff + 1));
-    B200_CUDA_TRY(tmp.alloc(&ubase, (uint64_t)eff + 1));
-    B200_CUDA_TRY(tmp.alloc(&win2eff, n_windows));
-    B200_CUDA_TRY(cudaMalloc(&f->d_rowOffset, ((uint64_t)eff + 1) * 4));
-    B200_CUDA_TRY(cudaMalloc(&f->d_rowIdx, std::max<uint64_t>((uint64_t)eff * 4, 16)));
-    B200_CUDA_TRY(cudaMemsetAsync(tiles + eff, 0, 4, stream));
-    B200_CUDA_TRY(cudaMemsetAsync(counts + eff, 0, 4, stream));
-    window_tables_kernel<<<(eff + kBlock - 1) / kBlock, kBlock, 0, stream>>>(win_ids, counts, eff, RW, CW, tiles,
-                                                                             f->d_rowIdx, win2eff);
-    B200_CUDA_TRY(cudaGetLastError());
-    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, tiles, f->d_rowOffset, (int)(eff + 1), stream));
-    uint8_t *scan_tmp = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&scan_tmp, scan_bytes));
-    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, tiles, f->d_rowOffset, (int)(eff + 1), stream));
-    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, counts, ubase, (int)(eff + 1), stream));
-    uint32_t total_tiles = 0;
-    B200_CUDA_TRY(cudaMemcpyAsync(&total_tiles, f->d_rowOffset + eff, 4, cudaMemcpyDeviceToHost, stream));
-    B200_CUDA_TRY(cudaStreamSynchronize(stream));
-    // (a tile count beyond 32 bits would have wrapped in the scan: bound it by the entry count instead)
-    if ((uint64_t)n_unique / CW + eff > 0xFFFFFFFFull) return B200SPMM_ERR_UNSUPPORTED;
-
-    f->info.eff_row_windows = eff;
-    f->info.total_tiles = total_tiles;
-    const uint64_t list_len = (uint64_t)total_tiles * CW, data_len = (uint64_t)total_tiles * RW * CW;
-    B200_CUDA_TRY(cudaMalloc(&f->d_tcA2B, std::max<uint64_t>(list_len * 4, 16)));
-    B200_CUDA_TRY(cudaMalloc(&f->d_data, std::max<uint64_t>(data_len * esz, 16)));
-    B200_CUDA_TRY(cudaMemsetAsync(f->d_tcA2B, 0xFF, list_len * 4, stream));  // kIdxMax padding
-    B200_CUDA_TRY(cudaMemsetAsync(f->d_data, 0, data_len * esz, stream));
-    scatter_columns_kernel<<<grid_for(n_unique), kBlock, 0, stream>>>(ukeys, n_unique, win2eff, ubase, f->d_rowOffset, CW,
-                                                                      f->d_tcA2B);
-    B200_CUDA_TRY(cudaGetLastError());
-
-    // 4. values
-    if (esz == 2)
-        scatter_values_kernel<uint16_t><<<grid_for(nnz), kBlock, 0, stream>>>(
-            d_col_idx, static_cast<const uint16_t *>(d_values), row_of, nnz, win2eff, f->d_rowOffset, counts, f->d_tcA2B,
-            RW, CW, static_cast<uint16_t *>(f->d_data));
-    else
-        scatter_values_kernel<uint32_t><<<grid_for(nnz), kBlock, 0, stream>>>(
-            d_col_idx, static_cast<const uint32_t *>(d_values), row_of, nnz, win2eff, f->d_rowOffset, counts, f->d_tcA2B,
-            RW, CW, static_cast<uint32_t *>(f->d_data));
-    B200_CUDA_TRY(cudaGetLastError());
-    B200_CUDA_TRY(cudaStreamSynchronize(stream));
+    while ((1ull << col_bits) < cols) ++col_bits;
+    const int st = win_bits + col_bits <= 32
+                       ? convert_on_device<uint32_t>(f, d_row_ptr, d_col_idx, d_values, col_bits, win_bits + col_bits, stream)
+                       : convert_on_device<uint64_t>(f, d_row_ptr, d_col_idx, d_values, col_bits, win_bits + col_bits, stream);
+    if (st != B200SPMM_OK) return st;
     guard.f = nullptr;
     *out = f;
     return B200SPMM_OK;

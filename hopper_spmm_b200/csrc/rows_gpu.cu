@@ -19,7 +19,9 @@ namespace b200spmm {
 namespace {
 
 constexpr int kBlock = 256;
-constexpr uint32_t kRunTiles = 256;
+// A hub window has thousands of tiles: short runs, or its warps are what everybody waits for (60,000 nodes, hub
+// row of 10,000 entries: 419 us for write_entries_kernel with runs of 256 tiles).
+constexpr uint32_t kRunTiles = 16;
 constexpr uint32_t kMaxBands = 8;
 constexpr uint32_t kEmptyKey = kMaxBands << 9;  // sort key: rows without entries last, then the band, then the longest first
 constexpr uint64_t kMinBandedCost = 2000000;  // bands pay where one keeps the GPU busy for tens of microseconds
@@ -84,10 +86,16 @@ __global__ void row_lengths_kernel(const uint32_t *__restrict__ run_first, const
     const uint32_t w = (uint32_t)(i >> 4), r = (uint32_t)i & 15u;
     if (w >= eff) return;
     uint32_t sum = 0;
-    for (uint32_t run = run_first[w]; run < run_first[w + 1]; ++run) {
-        const uint32_t c = counts[(uint64_t)run * 16 + r];
-        counts[(uint64_t)run * 16 + r] = sum;
-        sum += c;
+    const uint32_t end = run_first[w + 1];
+    for (uint32_t run = run_first[w]; run < end; run += 8) {
+        uint32_t c[8];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) c[k] = run + k < end ? counts[(uint64_t)(run + k) * 16 + r] : 0u;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            if (run + k < end) counts[(uint64_t)(run + k) * 16 + r] = sum;
+            sum += c[k];
+        }
     }
     if (rowIdx[w] + r < rows) row_len[rowIdx[w] + r] = sum;
 }

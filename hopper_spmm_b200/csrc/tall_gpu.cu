@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "common.hpp"
+#include "device_pool.hpp"
 #include "format.hpp"
 #include "tall_gpu.hpp"
 
@@ -23,20 +24,6 @@ namespace {
 
 constexpr int kBlock = 256;
 constexpr uint32_t kShort = 16;
-
-struct Scratch {  // device buffers released on every exit path
-    void *ptrs[16] = {};
-    int n = 0;
-    template <typename T>
-    cudaError_t alloc(T **out, size_t count) {
-        void *p = nullptr;
-        cudaError_t e = cudaMalloc(&p, std::max<size_t>(count * sizeof(T), 16));
-        if (e == cudaSuccess) ptrs[n++] = p;
-        *out = static_cast<T *>(p);
-        return e;
-    }
-    ~Scratch() { for (int i = 0; i < n; ++i) cudaFree(ptrs[i]); }
-};
 
 inline int grid_for(uint64_t n) { return (int)std::max<uint64_t>(1, std::min<uint64_t>((n + kBlock - 1) / kBlock, 148 * 32)); }
 
@@ -170,10 +157,10 @@ int estimate_tall_tile_ratio(const b200spmm_btcf_info_t &info, const uint32_t *h
 }
 
 void free_tall(TallFormat *t) {
-    cudaFree(t->d_rowOffset);
-    cudaFree(t->d_tcA2B);
-    cudaFree(t->d_rowIdx);
-    cudaFree(t->d_data);
+    pool_free(t->d_rowOffset);
+    pool_free(t->d_tcA2B);
+    pool_free(t->d_rowIdx);
+    pool_free(t->d_data);
     *t = TallFormat();
 }
 
@@ -193,7 +180,7 @@ int build_tall_device(const b200spmm_btcf_info_t &info, const uint32_t *h_rowOff
     std::vector<uint32_t> h_t_rowIdx(n_groups);
     for (uint64_t g = 0; g < n_groups; ++g) h_t_rowIdx[g] = h_rowIdx[group_first[g]] / kTall * kTall;
 
-    Scratch tmp;
+    PoolScratch tmp;
     uint32_t *d_group = nullptr, *d_ubase = nullptr;
     uint64_t *keys = nullptr, *keys_sorted = nullptr, *n_sel = nullptr;
     B200_CUDA_TRY(tmp.alloc(&d_group, eff));
@@ -237,10 +224,10 @@ int build_tall_device(const b200spmm_btcf_info_t &info, const uint32_t *h_rowOff
         ~Guard() { if (t) free_tall(t); }
     } guard{&t};
     const uint64_t list_len = t_tiles * cw, data_len = t_tiles * kTall * cw;
-    B200_CUDA_TRY(cudaMalloc(&t.d_rowOffset, (n_groups + 1) * 4));
-    B200_CUDA_TRY(cudaMalloc(&t.d_rowIdx, n_groups * 4));
-    B200_CUDA_TRY(cudaMalloc(&t.d_tcA2B, list_len * 4));
-    B200_CUDA_TRY(cudaMalloc(&t.d_data, data_len * info.elt_size));
+    B200_CUDA_TRY(pool_alloc(&t.d_rowOffset, n_groups + 1));
+    B200_CUDA_TRY(pool_alloc(&t.d_rowIdx, n_groups));
+    B200_CUDA_TRY(pool_alloc(&t.d_tcA2B, list_len));
+    B200_CUDA_TRY(pool_alloc_bytes(&t.d_data, data_len * info.elt_size, nullptr));
     B200_CUDA_TRY(cudaMemcpy(t.d_rowOffset, t_rowOffset.data(), (n_groups + 1) * 4, cudaMemcpyHostToDevice));
     B200_CUDA_TRY(cudaMemcpy(t.d_rowIdx, h_t_rowIdx.data(), n_groups * 4, cudaMemcpyHostToDevice));
     B200_CUDA_TRY(cudaMemset(t.d_tcA2B, 0xFF, list_len * 4));
