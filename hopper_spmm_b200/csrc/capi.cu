@@ -1012,7 +1012,7 @@ int b200spmm_plan_create(const b200spmm_btcf_t *h, int device, int n_ctas, b200s
     const Btcf &f = h->f;
     auto upload = [&](void **dst, const void *src, size_t bytes) -> int {
         B200_CUDA_TRY(pool_alloc_bytes(dst, std::max<size_t>(bytes, 16), nullptr));
-        if (bytes) B200_CUDA_TRY(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
+        if (bytes) B200_CUDA_TRY(upload_pageable(*dst, src, bytes));
         return B200SPMM_OK;
     };
     int st = upload((void **)&p->d_rowOffset, f.rowOffset.data(), f.rowOffset.size() * 4);

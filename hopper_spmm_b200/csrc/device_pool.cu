@@ -1,7 +1,11 @@
 #include "device_pool.hpp"
 
+#include <atomic>
 #include <cstdint>
+#include <cstring>
 #include <mutex>
+#include <thread>
+#include <vector>
 
 #include "../../include/b200_spmm.h"
 #include "common.hpp"
@@ -36,7 +40,57 @@ cudaError_t pool_of(int device, cudaMemPool_t *out) {
     return cudaSuccess;
 }
 
+std::mutex g_staging_lock;
+void *g_staging = nullptr;  // [kUploadThreads][2][kUploadChunk] pinned bytes
+
 }  // namespace
+
+cudaError_t upload_pageable(void *dst, const void *src, size_t bytes) {
+    std::unique_lock<std::mutex> guard(g_staging_lock, std::defer_lock);
+    if (bytes < 4 * kUploadChunk || !guard.try_lock()) return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    if (!g_staging && cudaHostAlloc(&g_staging, kUploadThreads * 2 * kUploadChunk, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        g_staging = nullptr;
+        return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    }
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // whatever was queued before the copy is done before it
+    if (e != cudaSuccess) return e;
+    std::atomic<size_t> next{0};
+    std::atomic<int> failed{(int)cudaSuccess};
+    auto worker = [&](int t) {
+        cudaStream_t stream = nullptr;
+        cudaEvent_t done[2] = {nullptr, nullptr};
+        auto ok = [&](cudaError_t r) {
+            if (r != cudaSuccess) failed = (int)r;
+            return r == cudaSuccess;
+        };
+        if (ok(cudaSetDevice(device)) && ok(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking)) &&
+            ok(cudaEventCreateWithFlags(&done[0], cudaEventDisableTiming)) && ok(cudaEventCreateWithFlags(&done[1], cudaEventDisableTiming))) {
+            for (int k = 0; failed == (int)cudaSuccess; k ^= 1) {
+                const size_t at = next.fetch_add(kUploadChunk);
+                if (at >= bytes) break;
+                const size_t n = std::min(kUploadChunk, bytes - at);
+                char *buf = static_cast<char *>(g_staging) + (size_t)(2 * t + k) * kUploadChunk;
+                if (!ok(cudaEventSynchronize(done[k]))) break;  // (at once for an event never recorded)
+                std::memcpy(buf, static_cast<const char *>(src) + at, n);
+                if (!ok(cudaMemcpyAsync(static_cast<char *>(dst) + at, buf, n, cudaMemcpyHostToDevice, stream)) ||
+                    !ok(cudaEventRecord(done[k], stream)))
+                    break;
+            }
+            ok(cudaStreamSynchronize(stream));
+        }
+        for (cudaEvent_t d : done)
+            if (d) cudaEventDestroy(d);
+        if (stream) cudaStreamDestroy(stream);
+    };
+    std::vector<std::thread> pool;
+    for (int t = 1; t < kUploadThreads; ++t) pool.emplace_back(worker, t);
+    worker(0);
+    for (auto &th : pool) th.join();
+    return (cudaError_t)failed.load();
+}
 
 cudaError_t pool_alloc_bytes(void **out, size_t bytes, cudaStream_t stream) {
     *out = nullptr;
@@ -60,6 +114,11 @@ void pool_free(void *ptr, cudaStream_t stream) {
 }
 
 cudaError_t pool_release(int device) {
+    {
+        std::lock_guard<std::mutex> guard(g_staging_lock);
+        if (g_staging) cudaFreeHost(g_staging);
+        g_staging = nullptr;
+    }
     cudaMemPool_t pool = nullptr;
     {
         std::lock_guard<std::mutex> guard(g_lock);

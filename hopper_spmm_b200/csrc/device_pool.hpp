@@ -30,6 +30,14 @@ cudaError_t pool_alloc(T **out, size_t count, cudaStream_t stream = nullptr) {
     return e;
 }
 
+// Copies `bytes` from pageable host memory to the current device and waits for it.  The driver's own copy moves 11
+// GB/s, one thread filling its staging buffer; here kUploadThreads threads fill pinned buffers of their own (16 MB
+// in all, kept for the next upload until b200spmm_release_cached_memory), which keeps the link at 40-50 GB/s.
+// Small copies, and uploads while another one holds the buffers, go the driver's way.
+constexpr int kUploadThreads = 4;
+constexpr size_t kUploadChunk = (size_t)2 << 20;
+cudaError_t upload_pageable(void *dst, const void *src, size_t bytes);
+
 // Buffers that are needed while an object is built, released on every exit path.
 struct PoolScratch {
     cudaStream_t stream = nullptr;

@@ -14,10 +14,19 @@ namespace b200spmm {
 
 namespace {
 
+int thread_count(int n_threads) {
+    if (n_threads <= 0) n_threads = (int)std::thread::hardware_concurrency();
+    return n_threads <= 0 ? 1 : n_threads;
+}
+
+// Items a worker takes at a time: enough chunks for the workers to even out.
+uint64_t chunk_for(uint64_t n_items, int n_threads) {
+    return std::max<uint64_t>(1, std::min<uint64_t>(256, n_items / ((uint64_t)thread_count(n_threads) * 8)));
+}
+
 template <class Fn>
 void parallel_chunks(uint64_t n_items, uint64_t chunk, int n_threads, Fn fn) {
-    if (n_threads <= 0) n_threads = (int)std::thread::hardware_concurrency();
-    if (n_threads <= 0) n_threads = 1;
+    n_threads = thread_count(n_threads);
     uint64_t n_chunks = (n_items + chunk - 1) / chunk;
     if ((uint64_t)n_threads > n_chunks) n_threads = (int)std::max<uint64_t>(1, n_chunks);
     std::atomic<uint64_t> next{0};
@@ -38,13 +47,60 @@ void parallel_chunks(uint64_t n_items, uint64_t chunk, int n_threads, Fn fn) {
     for (auto &t : pool) t.join();
 }
 
-// Sorted distinct columns of rows [first, last).
-void window_columns(const uint32_t *row_ptr, const uint32_t *col_idx, uint64_t first, uint64_t last,
-                    std::vector<uint32_t> *cols) {
-    cols->assign(col_idx + row_ptr[first], col_idx + row_ptr[last]);
-    std::sort(cols->begin(), cols->end());
-    cols->erase(std::unique(cols->begin(), cols->end()), cols->end());
-}
+// The sorted distinct columns of a window, and the place of a column among them.  Where the window's entries are
+// dense in the columns (a pruned weight matrix: a sixth of them) a bit set does both in one step per entry;
+// otherwise the columns are sorted and searched.
+class WindowColumns {
+public:
+    explicit WindowColumns(uint64_t cols) : words_((cols + 63) / 64) {}
+
+    // Appends the columns of col_idx[0, n) to *out and returns how many there are.
+    size_t collect(const uint32_t *col_idx, size_t n, std::vector<uint32_t> *out) {
+        const size_t begin = out->size();
+        if (!use_bits(n)) {
+            out->insert(out->end(), col_idx, col_idx + n);
+            std::sort(out->begin() + begin, out->end());
+            out->erase(std::unique(out->begin() + begin, out->end()), out->end());
+            return out->size() - begin;
+        }
+        bits_.resize(words_);
+        for (size_t i = 0; i < n; ++i) bits_[col_idx[i] >> 6] |= 1ull << (col_idx[i] & 63u);
+        for (size_t w = 0; w < words_; ++w) {
+            for (uint64_t b = bits_[w]; b; b &= b - 1) out->push_back((uint32_t)(w * 64 + (size_t)__builtin_ctzll(b)));
+            bits_[w] = 0;
+        }
+        return out->size() - begin;
+    }
+
+    // place(c) is valid for the columns list[0, n) until the next open().
+    void open(const uint32_t *list, size_t n, size_t entries) {
+        list_ = list;
+        n_ = n;
+        by_bits_ = use_bits(entries);
+        if (!by_bits_) return;
+        bits_.assign(words_, 0);
+        before_.resize(words_);
+        for (size_t i = 0; i < n; ++i) bits_[list[i] >> 6] |= 1ull << (list[i] & 63u);
+        uint32_t sum = 0;
+        for (size_t w = 0; w < words_; ++w) {
+            before_[w] = sum;
+            sum += (uint32_t)__builtin_popcountll(bits_[w]);
+        }
+    }
+    uint64_t place(uint32_t c) const {
+        if (by_bits_) return before_[c >> 6] + (uint64_t)__builtin_popcountll(bits_[c >> 6] & ((1ull << (c & 63u)) - 1));
+        return (uint64_t)(std::lower_bound(list_, list_ + n_, c) - list_);
+    }
+
+private:
+    // a pass over the words costs about what a few steps per entry do
+    bool use_bits(size_t entries) const { return words_ <= 4 * entries; }
+    size_t words_, n_ = 0;
+    const uint32_t *list_ = nullptr;
+    bool by_bits_ = false;
+    std::vector<uint64_t> bits_;
+    std::vector<uint32_t> before_;
+};
 
 }  // namespace
 
@@ -53,7 +109,7 @@ int validate_csr(uint64_t rows, uint64_t cols, uint64_t nnz, const uint32_t *row
     if (rows >= 0xFFFFFFFFull || cols > 0xFFFFFFFFull || nnz > 0xFFFFFFFFull) return B200SPMM_ERR_UNSUPPORTED;
     if (row_ptr[0] != 0 || row_ptr[rows] != nnz) return B200SPMM_ERR_BAD_CSR;
     std::atomic<int> bad{0};
-    parallel_chunks(rows, 1 << 16, 0, [&](uint64_t lo, uint64_t hi) {
+    parallel_chunks(rows, std::max<uint64_t>(64, std::min<uint64_t>(1 << 16, rows / 256)), 0, [&](uint64_t lo, uint64_t hi) {
         for (uint64_t r = lo; r < hi; ++r) {
             if (row_ptr[r + 1] < row_ptr[r] || row_ptr[r + 1] > nnz) {
                 bad = 1;
@@ -84,18 +140,17 @@ int convert_csr_to_btcf(uint64_t rows, uint64_t cols, uint64_t nnz, const uint32
     const int esz = dtype == B200SPMM_F16 ? 2 : 4;
     const uint64_t n_windows = (rows + RW - 1) / RW;
 
-    // Pass 1: tiles per window (0 marks an empty window, which the format omits, convert.h:162).
-    std::vector<uint32_t> window_tiles(n_windows);
-    parallel_chunks(n_windows, 256, n_threads, [&](uint64_t lo, uint64_t hi) {
-        std::vector<uint32_t> cols_w;
+    // Pass 1: column lists and tiles per window (0 marks an empty window, which the format omits, convert.h:162).
+    const uint64_t chunk = chunk_for(n_windows, n_threads);
+    std::vector<uint32_t> window_tiles(n_windows), window_cols(n_windows);
+    std::vector<std::vector<uint32_t>> lists((n_windows + chunk - 1) / chunk);  // of a chunk's windows, one after the other
+    parallel_chunks(n_windows, chunk, n_threads, [&](uint64_t lo, uint64_t hi) {
+        WindowColumns set(cols);
+        std::vector<uint32_t> &list = lists[lo / chunk];
         for (uint64_t w = lo; w < hi; ++w) {
-            uint64_t first = w * RW, last = std::min(rows, first + RW);
-            if (row_ptr[first] == row_ptr[last]) {
-                window_tiles[w] = 0;
-                continue;
-            }
-            window_columns(row_ptr, col_idx, first, last, &cols_w);
-            window_tiles[w] = (uint32_t)((cols_w.size() + CW - 1) / CW);
+            const uint64_t first = w * RW, last = std::min(rows, first + RW);
+            window_cols[w] = (uint32_t)set.collect(col_idx + row_ptr[first], row_ptr[last] - row_ptr[first], &list);
+            window_tiles[w] = (uint32_t)((window_cols[w] + CW - 1) / CW);
         }
     });
 
@@ -127,33 +182,40 @@ int convert_csr_to_btcf(uint64_t rows, uint64_t cols, uint64_t nnz, const uint32
     try {
         f.rowOffset.assign(eff + 1, 0);
         f.rowIdx.assign(eff, 0);
-        f.tcA2B.assign(tiles * CW, kIdxMax);
-        f.data.assign(tiles * RW * CW * esz, 0);
+        f.tcA2B.resize(tiles * CW);
+        f.data.resize(tiles * RW * CW * esz);
     } catch (const std::bad_alloc &) {
         return B200SPMM_ERR_NO_MEMORY;
     }
 
-    // Pass 2: column lists and tile values.
+    // Pass 2: padded column lists and tile values; the threads also touch the memory they fill for the first time.
     const uint8_t *vals = static_cast<const uint8_t *>(values);
-    parallel_chunks(n_windows, 256, n_threads, [&](uint64_t lo, uint64_t hi) {
-        std::vector<uint32_t> cols_w;
-        for (uint64_t w = lo; w < hi; ++w) {
+    parallel_chunks(n_windows, chunk, n_threads, [&](uint64_t lo, uint64_t hi) {
+        WindowColumns set(cols);
+        const uint32_t *list = lists[lo / chunk].data();
+        for (uint64_t w = lo; w < hi; list += window_cols[w], ++w) {
             if (!window_tiles[w]) continue;
-            uint64_t first = w * RW, last = std::min(rows, first + RW);
-            window_columns(row_ptr, col_idx, first, last, &cols_w);
-            uint64_t e = eff_base[w], t0 = tile_base[w];
+            const uint64_t first = w * RW, last = std::min(rows, first + RW), n = window_cols[w];
+            const uint64_t e = eff_base[w], t0 = tile_base[w], slots = (uint64_t)window_tiles[w] * CW;
             f.rowOffset[e + 1] = (uint32_t)(t0 + window_tiles[w]);
             f.rowIdx[e] = (uint32_t)first;
-            std::memcpy(&f.tcA2B[t0 * CW], cols_w.data(), cols_w.size() * sizeof(uint32_t));
+            uint32_t *wlist = &f.tcA2B[t0 * CW];
+            std::memcpy(wlist, list, n * sizeof(uint32_t));
+            std::fill(wlist + n, wlist + slots, kIdxMax);
             uint8_t *wdata = f.data.data() + t0 * RW * CW * esz;
-            for (uint64_t r = first; r < last; ++r) {
-                const uint64_t lr = r % RW;
-                for (uint64_t p = row_ptr[r]; p < row_ptr[r + 1]; ++p) {
-                    uint64_t slot = std::lower_bound(cols_w.begin(), cols_w.end(), col_idx[p]) - cols_w.begin();
-                    uint64_t off = (slot / CW) * RW * CW + lr * CW + slot % CW;  // row-major tile
-                    std::memcpy(wdata + off * esz, vals + p * esz, esz);  // repeated (r,c): last one stays
+            std::memset(wdata, 0, slots * RW * esz);
+            set.open(list, n, row_ptr[last] - row_ptr[first]);
+            auto scatter = [&](auto *tiles_out, const auto *in) {
+                for (uint64_t r = first; r < last; ++r) {
+                    const uint64_t lr = r % RW;
+                    for (uint64_t p = row_ptr[r]; p < row_ptr[r + 1]; ++p) {
+                        const uint64_t slot = set.place(col_idx[p]);
+                        tiles_out[(slot / CW) * RW * CW + lr * CW + slot % CW] = in[p];  // row-major tile; repeated (r,c): last one stays
+                    }
                 }
-            }
+            };
+            if (esz == 2) scatter(reinterpret_cast<uint16_t *>(wdata), reinterpret_cast<const uint16_t *>(vals));
+            else scatter(reinterpret_cast<uint32_t *>(wdata), reinterpret_cast<const uint32_t *>(vals));
         }
     });
     return B200SPMM_OK;
@@ -205,7 +267,7 @@ int rewindow_btcf(uint64_t rows, uint64_t cols, uint64_t nnz, int dtype, int rw_
     };
 
     std::vector<uint32_t> group_tiles(eff);
-    parallel_chunks(eff, 256, n_threads, [&](uint64_t lo, uint64_t hi) {
+    parallel_chunks(eff, chunk_for(eff, n_threads), n_threads, [&](uint64_t lo, uint64_t hi) {
         std::vector<uint32_t> u;
         for (uint64_t g = lo; g < hi; ++g) {
             group_columns(g, &u);
@@ -242,7 +304,7 @@ int rewindow_btcf(uint64_t rows, uint64_t cols, uint64_t nnz, int dtype, int rw_
         f.rowIdx[g] = (uint32_t)(in_rowIdx[group_first[g]] / RWO * RWO);
     }
     const uint8_t *src = static_cast<const uint8_t *>(in_data);
-    parallel_chunks(eff, 256, n_threads, [&](uint64_t lo, uint64_t hi) {
+    parallel_chunks(eff, chunk_for(eff, n_threads), n_threads, [&](uint64_t lo, uint64_t hi) {
         std::vector<uint32_t> u;
         for (uint64_t g = lo; g < hi; ++g) {
             group_columns(g, &u);

@@ -4,6 +4,10 @@
 #pragma once
 
 #include <cstdint>
+#include <cstdlib>
+#include <new>
+#include <sys/mman.h>
+#include <utility>
 #include <vector>
 
 namespace b200spmm {
@@ -16,6 +20,39 @@ constexpr uint32_t kIdxMax = 0xFFFFFFFFu;  // IDX_MAX, src/common.h:47
 // tile count alone.
 constexpr uint64_t kWindowCharge = 12;
 
+// Vectors that do not clear what they allocate, on huge pages when large: the converter writes every byte of its
+// arrays anyway, from many threads, and clearing a hundred megabytes first costs one thread (and a page fault per
+// 4 KB) more than the rest of the conversion.
+template <typename T>
+struct RawAllocator {
+    using value_type = T;
+    RawAllocator() = default;
+    template <typename U>
+    RawAllocator(const RawAllocator<U> &) {}
+    static constexpr size_t kHuge = (size_t)2 << 20;
+    T *allocate(size_t n) {
+        const size_t bytes = n * sizeof(T);
+        void *p = nullptr;
+        if (bytes >= 2 * kHuge) {
+            p = std::aligned_alloc(kHuge, (bytes + kHuge - 1) / kHuge * kHuge);
+            if (p) madvise(p, bytes, MADV_HUGEPAGE);
+        } else {
+            p = std::malloc(bytes ? bytes : 1);
+        }
+        if (!p) throw std::bad_alloc();
+        return static_cast<T *>(p);
+    }
+    void deallocate(T *p, size_t) { std::free(p); }
+    template <typename U>
+    void construct(U *p) { ::new (static_cast<void *>(p)) U; }
+    template <typename U, typename... A>
+    void construct(U *p, A &&...a) { ::new (static_cast<void *>(p)) U(std::forward<A>(a)...); }
+    bool operator==(const RawAllocator &) const { return true; }
+    bool operator!=(const RawAllocator &) const { return false; }
+};
+template <typename T>
+using RawVector = std::vector<T, RawAllocator<T>>;
+
 struct Btcf {
     uint64_t rows = 0, cols = 0, nnzs = 0;
     uint64_t total_row_windows = 0, eff_row_windows = 0, total_tiles = 0;
@@ -23,8 +60,8 @@ struct Btcf {
     int dtype = 0;     // B200SPMM_F16 / B200SPMM_TF32
     int elt_size = 2;  // bytes per value
     std::vector<uint32_t> rowOffset;  // [eff+1], in tiles
-    std::vector<uint32_t> tcA2B;      // [tiles*CW], padded with kIdxMax
-    std::vector<uint8_t> data;        // [tiles*RW*CW*elt_size]
+    RawVector<uint32_t> tcA2B;        // [tiles*CW], padded with kIdxMax
+    RawVector<uint8_t> data;          // [tiles*RW*CW*elt_size]
     std::vector<uint32_t> rowIdx;     // [eff], first row of each non-empty window
     bool col_major_tiles = false;     // tiles stored column by column (the reference's SPARSE_A_TRANSPOSE build)
 };

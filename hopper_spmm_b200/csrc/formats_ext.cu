@@ -121,7 +121,7 @@ int expand_bitmap(const BtcfBitmap &in, Btcf *out) {
     const uint64_t slots = (uint64_t)in.row_window * in.col_window, esz = (uint64_t)in.elt_size;
     try {
         f.rowOffset = in.rowOffset;
-        f.tcA2B = in.tcA2B;
+        f.tcA2B.assign(in.tcA2B.begin(), in.tcA2B.end());
         f.rowIdx = in.rowIdx;
         f.data.assign(in.total_tiles * slots * esz, 0);
     } catch (const std::bad_alloc &) {

@@ -112,6 +112,24 @@ __global__ void tall_scatter_values_kernel(const uint32_t *__restrict__ rowOffse
     }
 }
 
+// Distinct columns in the lists of a run of 16-row tiles, one block per run.
+__global__ void __launch_bounds__(1024)
+distinct_columns_kernel(const uint32_t *__restrict__ tcA2B, const uint2 *__restrict__ ranges, uint32_t cw, uint64_t words,
+                        uint32_t *__restrict__ bits, uint32_t *__restrict__ distinct) {
+    __shared__ uint32_t total;
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    const uint64_t end = (uint64_t)ranges[blockIdx.x].y * cw;
+    uint32_t *mine = bits + blockIdx.x * words, n = 0;
+    for (uint64_t e = (uint64_t)ranges[blockIdx.x].x * cw + threadIdx.x; e < end; e += 1024) {
+        const uint32_t c = tcA2B[e];
+        if (c != kIdxMax && !(atomicOr(mine + (c >> 5), 1u << (c & 31u)) & (1u << (c & 31u)))) ++n;
+    }
+    atomicAdd(&total, n);
+    __syncthreads();
+    if (threadIdx.x == 0) distinct[blockIdx.x] = total;
+}
+
 // Runs of 16-row windows that fall into the same 128-row window.
 void group_windows(const uint32_t *h_rowIdx, uint64_t eff, uint32_t kTall, std::vector<uint32_t> *win_group,
                    std::vector<uint64_t> *group_first) {
@@ -137,21 +155,29 @@ int estimate_tall_tile_ratio(const b200spmm_btcf_info_t &info, const uint32_t *h
     *n_super_windows = n_groups;
     *ratio = 1.0;
     if (!n_groups || max_samples < 1) return B200SPMM_OK;
-    const uint64_t step = std::max<uint64_t>(1, n_groups / (uint64_t)max_samples);
-    uint64_t short_tiles = 0, tall_tiles = 0, copied = 0;
-    std::vector<uint32_t> list;
-    for (uint64_t g = step / 2; g < n_groups; g += step) {
-        const uint64_t t0 = h_rowOffset[group_first[g]], t1 = h_rowOffset[group_first[g + 1]];
-        if ((t1 - t0) * cw * 4 > (64u << 20) || copied > (256u << 20)) continue;  // keep the probe small
-        list.resize((t1 - t0) * cw);
-        B200_CUDA_TRY(cudaMemcpy(list.data(), d_tcA2B + t0 * cw, list.size() * 4, cudaMemcpyDeviceToHost));
-        copied += list.size() * 4;
-        std::sort(list.begin(), list.end());
-        list.erase(std::unique(list.begin(), list.end()), list.end());
-        while (!list.empty() && list.back() == kIdxMax) list.pop_back();
-        short_tiles += t1 - t0;
-        tall_tiles += (list.size() + cw - 1) / cw;
+    // one bit per column and sampled super-window, at most 64 MB of them
+    const uint64_t words = (info.cols + 31) / 32;
+    const uint64_t n_samples = std::max<uint64_t>(1, std::min({(uint64_t)max_samples, n_groups, ((uint64_t)16 << 20) / words}));
+    std::vector<uint2> ranges;
+    uint64_t short_tiles = 0, tall_tiles = 0;
+    for (uint64_t k = 0; k < n_samples; ++k) {
+        const uint64_t g = (2 * k + 1) * n_groups / (2 * n_samples);
+        ranges.push_back(make_uint2(h_rowOffset[group_first[g]], h_rowOffset[group_first[g + 1]]));
+        short_tiles += ranges.back().y - ranges.back().x;
     }
+    PoolScratch tmp;
+    uint2 *d_ranges = nullptr;
+    uint32_t *bits = nullptr, *d_distinct = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&d_ranges, n_samples));
+    B200_CUDA_TRY(tmp.alloc(&d_distinct, n_samples));
+    B200_CUDA_TRY(tmp.alloc(&bits, n_samples * words));
+    B200_CUDA_TRY(cudaMemsetAsync(bits, 0, n_samples * words * 4));
+    B200_CUDA_TRY(cudaMemcpy(d_ranges, ranges.data(), n_samples * sizeof(uint2), cudaMemcpyHostToDevice));
+    distinct_columns_kernel<<<(unsigned)n_samples, 1024>>>(d_tcA2B, d_ranges, (uint32_t)cw, words, bits, d_distinct);
+    B200_CUDA_TRY(cudaGetLastError());
+    std::vector<uint32_t> distinct(n_samples);
+    B200_CUDA_TRY(cudaMemcpy(distinct.data(), d_distinct, n_samples * 4, cudaMemcpyDeviceToHost));
+    for (uint32_t d : distinct) tall_tiles += (d + cw - 1) / cw;
     if (short_tiles) *ratio = (double)tall_tiles / (double)short_tiles;
     return B200SPMM_OK;
 }
