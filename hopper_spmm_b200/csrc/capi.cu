@@ -16,6 +16,7 @@
 #include "format.hpp"
 #include "handles.hpp"
 #include "spmm_kernel.cuh"
+#include "spmm_narrow_kernel.cuh"
 #include "spmm_pair_kernel.cuh"
 #include "spmm_rows_kernel.cuh"
 #include "spmm_tall_kernel.cuh"
@@ -89,6 +90,7 @@ struct b200spmm_plan {
     // whose tiles are nearly empty keeps nothing else (rows_only).
     RowsFormat rows_fmt;
     bool rows_only = false;
+    NarrowFormat narrow;       // the entries once more for narrow B (spmm_narrow_kernel.cuh), or empty
     bool may_time_out = false;   // a kernel with bounded waits was launched since the status word was last read
     bool has_tile_path = false;  // schedule and tile image of the 16-row kernel are there
     // Most tiles of the super-window format name one aligned group of CW consecutive rows of B: then B
@@ -469,6 +471,65 @@ int launch_rows(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void 
     return B200SPMM_OK;
 }
 
+// ---- narrow B
+template <bool kTf32>
+int launch_narrow_vecs(const NarrowParams &prm, int vecs, unsigned n_ctas, size_t smem, cudaStream_t stream) {
+    using Kernel = void (*)(const NarrowParams);
+    constexpr Kernel kernels[kNarrowMaxVecs] = {spmm_narrow_kernel<kTf32, 1>, spmm_narrow_kernel<kTf32, 2>, spmm_narrow_kernel<kTf32, 3>,
+                                                spmm_narrow_kernel<kTf32, 4>, spmm_narrow_kernel<kTf32, 5>, spmm_narrow_kernel<kTf32, 6>};
+    static thread_local int configured_device = -1;
+    int device = 0;
+    B200_CUDA_TRY(cudaGetDevice(&device));
+    if (configured_device != device) {
+        for (Kernel k : kernels) B200_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNarrowSmemMax));
+        configured_device = device;
+    }
+    kernels[vecs - 1]<<<n_ctas, kNarrowThreads, smem, stream>>>(prm);
+    B200_CUDA_TRY(cudaGetLastError());
+    return B200SPMM_OK;
+}
+
+// Column blocks per group for B of width n: as many as fit shared memory, 0 if the kernel does not take it.
+uint32_t narrow_group_blocks(const b200spmm_plan *p, int64_t n) {
+    const NarrowFormat &f = p->narrow;
+    const int64_t vecs = n * p->info.elt_size / 16;
+    if (!f.n_ctas || vecs > kNarrowMaxVecs) return 0;
+    uint32_t g = f.n_blocks;
+    while (g && narrow_smem_bytes((uint32_t)vecs, (uint32_t)p->info.cols, g, f.n_blocks, f.max_rows, (uint32_t)n) > kNarrowSmemMax) --g;
+    return g;
+}
+
+int launch_narrow(b200spmm_plan *p, uint32_t group_blocks, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
+                  cudaStream_t stream) {
+    const NarrowFormat &f = p->narrow;
+    NarrowParams prm{};
+    prm.entries = f.d_entries;
+    prm.seg = f.d_seg;
+    prm.cut = f.d_cut;
+    prm.n_blocks = f.n_blocks;
+    prm.group_blocks = group_blocks;
+    prm.B = d_B;
+    prm.C = d_C;
+    prm.ldb = ldb;
+    prm.ldc = ldc;
+    prm.cols = (uint32_t)p->info.cols;
+    prm.n = (uint32_t)n;
+    prm.c_is_half = c_dtype == B200SPMM_C_F16;
+    const int vecs = (int)(n * p->info.elt_size / 16);
+    const size_t smem = narrow_smem_bytes((uint32_t)vecs, prm.cols, group_blocks, f.n_blocks, f.max_rows, prm.n);
+    const int st = p->info.dtype == B200SPMM_TF32 ? launch_narrow_vecs<true>(prm, vecs, f.n_ctas, smem, stream)
+                                                  : launch_narrow_vecs<false>(prm, vecs, f.n_ctas, smem, stream);
+    if (st != B200SPMM_OK) return st;
+    p->last.n_ctas = (int)f.n_ctas;
+    p->last.threads = kNarrowThreads;
+    p->last.feature_slab = 64;
+    p->last.n_slabs = 1;
+    p->last.smem_bytes = (int64_t)smem;
+    p->last.kernel_launches = 1;
+    p->last.row_window = kRowWindow;
+    return B200SPMM_OK;
+}
+
 bool use_pair(const b200spmm_plan *p, int64_t n) {
     if (!p->pair.tiles || p->pair_clusters < 1 || n <= 128) return false;
     if (p->tall_forced) return true;
@@ -724,12 +785,11 @@ int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h
     // B200SPMM_WINDOW=rows asks for the row units whatever the matrix.
     const bool force_rows = env_is("B200SPMM_WINDOW", "rows");
     if (n_ctas <= 0 && (force_rows || (!std::getenv("B200SPMM_WINDOW") && !std::getenv("B200SPMM_TILES") && !p->gather_cpasync))) {
-        int st = build_rows_device(info, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, p->n_sms, &p->rows_fmt);
+        int st = build_row_formats(info, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, p->n_sms, kRowsMaxFill, force_rows,
+                                   &p->rows_fmt, &p->narrow);
         if (st != B200SPMM_OK) return st;
-        const double slots = (double)info.total_tiles * kRowWindow * cw;
-        p->rows_only = p->rows_fmt.n_units && (force_rows || (double)p->rows_fmt.nnz <= kRowsMaxFill * slots);
+        p->rows_only = p->rows_fmt.n_units > 0;
         if (p->rows_only) return B200SPMM_OK;
-        free_rows(&p->rows_fmt);
     }
     return h_rowOffset ? plan_build_tile_path(p, h_rowOffset, h_rowIdx, n_ctas) : plan_add_tile_path(p, n_ctas);
 }
@@ -974,6 +1034,7 @@ void b200spmm_plan_destroy(b200spmm_plan_t *p) {
     }
     free_compressed_tiles(&p->comp);
     free_rows(&p->rows_fmt);
+    free_narrow(&p->narrow);
     pool_free(p->d_tile_entries);
     free_tall(&p->tall);
     free_tall(&p->pair);
@@ -1160,6 +1221,8 @@ int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, voi
         return B200SPMM_OK;
     }
     if (!p->starve_gathers && use_rows(p, ldb)) return launch_rows(p, d_B, ldb, n, d_C, ldc, c_dtype, stream, band);
+    if (const uint32_t g = p->starve_gathers || band >= 0 ? 0u : narrow_group_blocks(p, n))
+        return launch_narrow(p, g, d_B, ldb, n, d_C, ldc, c_dtype, stream);
     if (!p->has_tile_path) {  // only row units were kept; the starved test launch and a huge ldb ask for more
         int st = plan_add_tile_path(p, 0);
         if (st != B200SPMM_OK) return st;
@@ -1279,7 +1342,7 @@ int b200spmm_spmm_host(b200spmm_plan_t *p, const void *h_B, int64_t n, void *h_C
         band_row.clear();
         for (const RowBand &b : p->rows_fmt.bands) band_row.push_back(b.row);
     }
-    const size_t bands = band_row.size() > 1 && (rows || !use_tall(p, n)) ? band_row.size() - 1 : 1;
+    const size_t bands = band_row.size() > 1 && (rows || !(use_tall(p, n) || narrow_group_blocks(p, n))) ? band_row.size() - 1 : 1;
     if (bands == 1 || p->info.eff_row_windows == 0) {
         B200_CUDA_TRY(cudaMemcpyAsync(p->d_B, h_B, b_bytes, cudaMemcpyHostToDevice, nullptr));
         int st = b200spmm_spmm(p, p->d_B, n, n, p->d_C, n, c_dtype, nullptr);

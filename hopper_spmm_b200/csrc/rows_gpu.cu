@@ -24,9 +24,12 @@ constexpr int kBlock = 256;
 constexpr uint32_t kRunTiles = 16;
 constexpr uint32_t kMaxBands = 8;
 constexpr uint32_t kEmptyKey = kMaxBands << 9;  // sort key: rows without entries last, then the band, then the longest first
+constexpr uint32_t kMaxLenAt = 4 + 2 * (kMaxBands + 1);  // in the table of totals: the longest row
 constexpr uint64_t kMinBandedCost = 2000000;  // bands pay where one keeps the GPU busy for tens of microseconds
 // For the bands a row counts as this many entries: its store is 4 bytes a feature where a gathered entry is 2.
 constexpr uint64_t kRowCost = 2;
+// Starting and reducing a row costs a warp of the narrow kernel about what 64 entries do.
+constexpr uint64_t kNarrowRowCost = 64;
 
 inline int grid_for(uint64_t n) { return (int)std::max<uint64_t>(1, std::min<uint64_t>((n + kBlock - 1) / kBlock, 148 * 32)); }
 
@@ -81,7 +84,8 @@ run_rows_kernel(const uint32_t *__restrict__ rowOffset, const T *__restrict__ da
 
 // thread (window, row of it): counts of its runs become what the earlier runs hold; the sum is the row's length
 __global__ void row_lengths_kernel(const uint32_t *__restrict__ run_first, const uint32_t *__restrict__ rowIdx, uint32_t eff,
-                                   uint32_t rows, uint32_t *__restrict__ counts, uint32_t *__restrict__ row_len) {
+                                   uint32_t rows, uint32_t *__restrict__ counts, uint32_t *__restrict__ row_len,
+                                   uint32_t *__restrict__ max_len) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t w = (uint32_t)(i >> 4), r = (uint32_t)i & 15u;
     if (w >= eff) return;
@@ -98,6 +102,7 @@ __global__ void row_lengths_kernel(const uint32_t *__restrict__ run_first, const
         }
     }
     if (rowIdx[w] + r < rows) row_len[rowIdx[w] + r] = sum;
+    if (sum > *max_len) atomicMax(max_len, sum);
 }
 
 // Inclusive scans follow over both: (entries << 32 | units) and (cut rows << 32 | slots).
@@ -263,7 +268,108 @@ uint32_t unit_entries_for(uint64_t nnz, uint64_t rows, int n_sms) {
     return cap;
 }
 
+// ---- entries for narrow B
+
+// columns and values of the rows one after the other, in column order
+template <typename T>
+__global__ void __launch_bounds__(kBlock)
+write_csr_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B, const T *__restrict__ data,
+                 const uint32_t *__restrict__ rowIdx, const uint32_t *__restrict__ run_first, const uint32_t *__restrict__ run_window,
+                 uint32_t eff, uint32_t rows, const uint32_t *__restrict__ counts, const unsigned long long *__restrict__ a,
+                 uint32_t *__restrict__ cols_out, T *__restrict__ vals_out) {
+    constexpr int kPer = Piece<T>::kPer;
+    const uint32_t lane = threadIdx.x & 31u, n_runs = run_first[eff];
+    for (uint32_t run = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); run < n_runs; run += gridDim.x * (kBlock / 32)) {
+        const uint32_t w = run_window[run], t0 = rowOffset[w] + (run - run_first[w]) * kRunTiles;
+        const uint32_t t1 = min(t0 + kRunTiles, rowOffset[w + 1]), row = min(rowIdx[w] + (lane >> 1), rows - 1);
+        uint32_t at = (row ? (uint32_t)(a[row - 1] >> 32) : 0u) + counts[(uint64_t)run * 16 + (lane >> 1)];
+#pragma unroll 2
+        for (uint32_t t = t0; t < t1; ++t) {
+            Piece<T> p;
+            p.load(data, t, lane);
+            const uint32_t mine = (uint32_t)__popc(p.mask), other = __shfl_xor_sync(0xffffffffu, mine, 1);
+            uint32_t k_out = at + ((lane & 1u) ? other : 0u);
+            at += mine + other;
+            const uint32_t *cols = tcA2B + (uint64_t)t * (2 * kPer) + (lane & 1u) * kPer;
+#pragma unroll
+            for (int k = 0; k < kPer; ++k)
+                if (p.mask & (1u << k)) {
+                    cols_out[k_out] = cols[k];
+                    vals_out[k_out++] = p.v[k];
+                }
+        }
+    }
+}
+
+// One warp per row.  The kernel reads shared memory at 16 bytes x (column mod 8) for eight neighbouring entries at a
+// time, so inside a block the entries are dealt out by column mod 8: first the first column of every class, then the
+// second of every class, and so on.  Entry of rank r in class c comes behind min(count, r) entries of every class
+// and one more of the classes below c that have it.
+template <typename T>
+__global__ void __launch_bounds__(kBlock)
+narrow_entries_kernel(const uint32_t *__restrict__ cols, const T *__restrict__ vals, const unsigned long long *__restrict__ a, uint32_t rows,
+                      uint32_t n_blocks, uint32_t *__restrict__ seg, uint32_t *__restrict__ entries) {
+    extern __shared__ uint32_t narrow_smem[];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, row = blockIdx.x * (kBlock / 32) + warp;
+    uint32_t *count = narrow_smem + warp * (2 * n_blocks * 8), *run = count + n_blocks * 8;
+    if (row >= rows) return;
+    for (uint32_t k = lane; k < 2 * n_blocks * 8; k += 32) count[k] = 0;
+    __syncwarp();
+    const uint32_t begin = row ? (uint32_t)(a[row - 1] >> 32) : 0u, end = (uint32_t)(a[row] >> 32);
+    for (uint32_t e = begin + lane; e < end; e += 32) atomicAdd(&count[(cols[e] / kNarrowCols) * 8 + (cols[e] & 7u)], 1u);
+    __syncwarp();
+    uint32_t *my_seg = seg + (uint64_t)row * (n_blocks + 1);
+    if (lane == 0) {
+        uint32_t at = begin;
+        for (uint32_t b = 0; b < n_blocks; ++b) {
+            my_seg[b] = at;
+            for (uint32_t c = 0; c < 8; ++c) at += count[b * 8 + c];
+        }
+        my_seg[n_blocks] = at;
+    }
+    __syncwarp();
+    for (uint32_t e0 = begin; e0 < end; e0 += 32) {
+        const bool live = e0 + lane < end;
+        const uint32_t col = live ? cols[e0 + lane] : 0xFFFFFFFFu, c = col & 7u, b = col / kNarrowCols;
+        const uint32_t same = __match_any_sync(0xffffffffu, live ? b * 8 + c : 0xFFFFFFFFu);
+        if (live) {
+            const uint32_t rank = run[b * 8 + c] + (uint32_t)__popc(same & ((1u << lane) - 1u));
+            uint32_t at = my_seg[b];
+#pragma unroll
+            for (uint32_t k = 0; k < 8; ++k) {
+                const uint32_t n = count[b * 8 + k];
+                at += min(n, rank) + (k < c && n > rank ? 1u : 0u);
+            }
+            if constexpr (sizeof(T) == 2) entries[at] = ((uint32_t)vals[e0 + lane] << 16) | (col & 0xFFFFu);
+            else reinterpret_cast<uint2 *>(entries)[at] = make_uint2(col, (uint32_t)vals[e0 + lane] & 0xFFFFE000u);
+        }
+        __syncwarp();
+        if (live && (same >> lane) == 1u) run[b * 8 + c] += (uint32_t)__popc(same);  // the last lane of the class
+        __syncwarp();
+    }
+}
+
+// CTA k: rows from the first one whose cost reaches k / n_ctas of the total on
+__global__ void narrow_cuts_kernel(const unsigned long long *__restrict__ a, uint32_t rows, uint32_t n_ctas, uint32_t *__restrict__ cut) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k > n_ctas) return;
+    const uint64_t total = (a[rows - 1] >> 32) + kNarrowRowCost * rows, want = total * k / n_ctas;
+    uint32_t lo = 0, hi = rows;
+    while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        if ((a[mid] >> 32) + kNarrowRowCost * (mid + 1ull) <= want) lo = mid + 1; else hi = mid;
+    }
+    cut[k] = k == n_ctas ? rows : lo;
+}
+
 }  // namespace
+
+void free_narrow(NarrowFormat *f) {
+    pool_free(f->d_entries);
+    pool_free(f->d_seg);
+    pool_free(f->d_cut);
+    *f = NarrowFormat();
+}
 
 void free_rows(RowsFormat *r) {
     pool_free(r->d_batches);
@@ -272,9 +378,67 @@ void free_rows(RowsFormat *r) {
     *r = RowsFormat();
 }
 
-int build_rows_device(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOffset, const uint32_t *d_tcA2B,
-                      const void *d_data, const uint32_t *d_rowIdx, int n_sms, RowsFormat *out) {
+namespace {
+
+// CTAs hold whole rows and a row is a warp's work: rows of a few steps of 32 lanes at least on average, and none
+// longer than a quarter of a CTA's share.
+bool narrow_pays(uint64_t nnz, uint64_t rows, uint64_t cols, uint64_t max_len, int n_sms) {
+    return cols <= 65536 && nnz >= 48 * rows && max_len * (uint64_t)n_sms <= 4 * nnz + 32 * (uint64_t)n_sms * 32;
+}
+
+int build_narrow(const b200spmm_btcf_info_t &info, uint64_t nnz, const uint32_t *d_rowOffset, const uint32_t *d_tcA2B, const void *d_data,
+                 const uint32_t *d_rowIdx, int n_sms, const uint32_t *run_first, const uint32_t *run_window, int run_grid,
+                 const uint32_t *counts, const unsigned long long *a, NarrowFormat *out) {
+    const uint32_t rows = (uint32_t)info.rows, eff = (uint32_t)info.eff_row_windows, words = (uint32_t)info.elt_size / 2;
+    NarrowFormat f;
+    struct Guard {
+        NarrowFormat *f;
+        ~Guard() { if (f) free_narrow(f); }
+    } guard{&f};
+    PoolScratch tmp;
+    f.n_blocks = (uint32_t)((info.cols + kNarrowCols - 1) / kNarrowCols);
+    f.n_ctas = (uint32_t)std::min<uint64_t>((uint64_t)n_sms, rows);
+    uint32_t *cols = nullptr;
+    void *vals = nullptr;
+    cudaError_t e = pool_alloc(&f.d_entries, nnz * words);
+    if (e == cudaSuccess) e = pool_alloc(&f.d_seg, (uint64_t)rows * (f.n_blocks + 1));
+    if (e == cudaSuccess) e = pool_alloc(&f.d_cut, f.n_ctas + 1);
+    if (e == cudaSuccess) e = tmp.alloc(&cols, nnz);
+    if (e == cudaSuccess) e = tmp.alloc(reinterpret_cast<uint16_t **>(&vals), nnz * words);
+    if (e == cudaErrorMemoryAllocation) {  // no room: the tile kernels still work
+        cudaGetLastError();
+        return B200SPMM_OK;
+    }
+    B200_CUDA_TRY(e);
+    const int grid = (int)((rows + kBlock / 32 - 1) / (kBlock / 32));
+    const size_t smem = (size_t)(kBlock / 32) * 2 * f.n_blocks * 8 * 4;
+    if (info.elt_size == 2) {
+        write_csr_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, static_cast<const uint16_t *>(d_data), d_rowIdx, run_first,
+                                                         run_window, eff, rows, counts, a, cols, static_cast<uint16_t *>(vals));
+        narrow_entries_kernel<uint16_t><<<grid, kBlock, smem>>>(cols, static_cast<const uint16_t *>(vals), a, rows, f.n_blocks, f.d_seg, f.d_entries);
+    } else {
+        write_csr_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, static_cast<const uint32_t *>(d_data), d_rowIdx, run_first,
+                                                         run_window, eff, rows, counts, a, cols, static_cast<uint32_t *>(vals));
+        narrow_entries_kernel<uint32_t><<<grid, kBlock, smem>>>(cols, static_cast<const uint32_t *>(vals), a, rows, f.n_blocks, f.d_seg, f.d_entries);
+    }
+    narrow_cuts_kernel<<<(int)(f.n_ctas / kBlock + 1), kBlock>>>(a, rows, f.n_ctas, f.d_cut);
+    B200_CUDA_TRY(cudaGetLastError());
+    std::vector<uint32_t> cut(f.n_ctas + 1);
+    B200_CUDA_TRY(cudaMemcpy(cut.data(), f.d_cut, cut.size() * 4, cudaMemcpyDeviceToHost));
+    for (uint32_t k = 0; k < f.n_ctas; ++k) f.max_rows = std::max(f.max_rows, cut[k + 1] - cut[k]);
+    B200_CUDA_TRY(cudaDeviceSynchronize());
+    *out = f;
+    guard.f = nullptr;
+    return B200SPMM_OK;
+}
+
+}  // namespace
+
+int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOffset, const uint32_t *d_tcA2B,
+                      const void *d_data, const uint32_t *d_rowIdx, int n_sms, double max_fill, bool force_rows,
+                      RowsFormat *out, NarrowFormat *narrow) {
     *out = RowsFormat();
+    *narrow = NarrowFormat();
     const uint64_t tiles = info.total_tiles;
     if (!info.eff_row_windows || !tiles || info.rows >= kSlotTarget) return B200SPMM_OK;
     const uint32_t rows = (uint32_t)info.rows, eff = (uint32_t)info.eff_row_windows;
@@ -295,7 +459,7 @@ int build_rows_device(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
     B200_CUDA_TRY(tmp.alloc(&row_len, rows));
     B200_CUDA_TRY(tmp.alloc(&a, rows));
     B200_CUDA_TRY(tmp.alloc(&b, rows));
-    B200_CUDA_TRY(tmp.alloc(&totals, 4 + 2 * (kMaxBands + 1)));
+    B200_CUDA_TRY(tmp.alloc(&totals, kMaxLenAt + 1));
     size_t run_bytes = 0, row_bytes = 0;
     B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, run_bytes, n_runs, run_first, (int64_t)eff + 1));
     B200_CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, row_bytes, a, a, (int64_t)rows));
@@ -311,15 +475,22 @@ int build_rows_device(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
     const int run_grid = grid_for(max_runs * 32), row_grid = (int)((rows + kBlock - 1) / kBlock);
     if (f16) run_rows_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, data16, run_first, run_window, eff, counts);
     else run_rows_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, data32, run_first, run_window, eff, counts);
+    uint32_t *max_len = totals + kMaxLenAt;
     B200_CUDA_TRY(cudaMemsetAsync(row_len, 0, (size_t)rows * 4));
-    row_lengths_kernel<<<(unsigned)(((uint64_t)eff * 16 + kBlock - 1) / kBlock), kBlock>>>(run_first, d_rowIdx, eff, rows, counts, row_len);
+    B200_CUDA_TRY(cudaMemsetAsync(max_len, 0, 4));
+    row_lengths_kernel<<<(unsigned)(((uint64_t)eff * 16 + kBlock - 1) / kBlock), kBlock>>>(run_first, d_rowIdx, eff, rows, counts, row_len, max_len);
     row_terms_kernel<<<row_grid, kBlock>>>(row_len, rows, cap, a, b);
     B200_CUDA_TRY(cub::DeviceScan::InclusiveSum(scan_tmp, row_bytes, a, a, (int64_t)rows));
     B200_CUDA_TRY(cub::DeviceScan::InclusiveSum(scan_tmp, row_bytes, b, b, (int64_t)rows));
     row_bands_kernel<<<1, 32>>>(rows, a, b, totals);
     B200_CUDA_TRY(cudaGetLastError());
-    uint32_t h[4 + 2 * (kMaxBands + 1)];
+    uint32_t h[kMaxLenAt + 1];
     B200_CUDA_TRY(cudaMemcpy(h, totals, sizeof(h), cudaMemcpyDeviceToHost));
+    if (!force_rows && (double)h[0] > max_fill * (double)tiles * 16.0 * info.col_window) {
+        if (narrow_pays(h[0], rows, info.cols, h[kMaxLenAt], n_sms))
+            return build_narrow(info, h[0], d_rowOffset, d_tcA2B, d_data, d_rowIdx, n_sms, run_first, run_window, run_grid, counts, a, narrow);
+        return B200SPMM_OK;
+    }
     f.nnz = h[0];
     f.n_units = h[1];
     f.n_splits = h[2];

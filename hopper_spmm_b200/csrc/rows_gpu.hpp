@@ -43,9 +43,24 @@ struct RowsFormat {
     std::vector<RowBand> bands;       // one more than there are bands: the last one holds the totals
 };
 
-// The tiles must be in the reference's layout (row-major 16 x CW).  Leaves *out empty when device memory is short.
-int build_rows_device(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOffset, const uint32_t *d_tcA2B,
-                      const void *d_data, const uint32_t *d_rowIdx, int n_sms, RowsFormat *out);
+// The same entries for narrow B (see spmm_narrow_kernel.cuh): row after row, and inside a row column block after
+// column block of kNarrowCols columns.  fp16: (value << 16) | low half of the column; tf32: (column, value bits).
+constexpr uint32_t kNarrowCols = 2048;
+struct NarrowFormat {
+    uint32_t *d_entries = nullptr;    // [nnz] words (fp16) or pairs of words (tf32)
+    uint32_t *d_seg = nullptr;        // [rows][n_blocks + 1] first entry of every (row, block), and the row's end
+    uint32_t *d_cut = nullptr;        // [n_ctas + 1] rows of every CTA
+    uint32_t n_blocks = 0, n_ctas = 0, max_rows = 0;  // max_rows: of one CTA
+};
+
+// Builds what the kernels outside the tile path want from a matrix: row units alone when `force_rows` or when at
+// most max_fill of the tiles' slots are in use, else the format for narrow B where it fits (at most 65,536 columns,
+// no row so long that CTAs of whole rows could not be balanced).  The tiles must be in the reference's layout
+// (row-major 16 x CW).  A format stays empty when device memory is short.
+int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOffset, const uint32_t *d_tcA2B,
+                      const void *d_data, const uint32_t *d_rowIdx, int n_sms, double max_fill, bool force_rows,
+                      RowsFormat *rows, NarrowFormat *narrow);
 void free_rows(RowsFormat *r);
+void free_narrow(NarrowFormat *f);
 
 }  // namespace b200spmm

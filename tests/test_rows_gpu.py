@@ -55,3 +55,28 @@ def test_smallest_matrices(rows, cols, monkeypatch):
         parity.check(plan.spmm_host(B), rows, rp, ci, v, B)
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+@pytest.mark.parametrize("n", [8, 16, 24, 40, 48])
+@pytest.mark.parametrize("rows,cols", [(700, 6001), (149, 2048), (3, 700), (1200, 16500)])
+def test_narrow_b_at_the_edges_of_its_column_blocks(dt, n, rows, cols):
+    # one column block and several, all in shared memory at once and group by group; CTAs with one row, several rows
+    # and none; rows of a few entries, empty ones and rows of many steps
+    import torch
+    rng = np.random.default_rng(rows + n)
+    lengths = rng.integers(cols // 12, cols // 5, rows)
+    lengths[[0, rows // 2, rows - 1]] = [0, 5, 33]
+    rows, cols, rp, ci, v = rows_of_lengths(lengths, cols, 7, dt)
+    Bfull = torch.from_numpy(dense_b(cols, n + 16, 4, dt)).cuda()
+    Bv = Bfull[:, 8:8 + n]
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    try:
+        Cfull = torch.full((rows, n + 8), float("nan"), device="cuda")
+        plan.spmm(Bv, Cfull[:, 4:4 + n])
+        got = Cfull[:, 4:4 + n].clone()
+        assert torch.isnan(Cfull[:, :4]).all() and torch.isnan(Cfull[:, 4 + n:]).all()
+        parity.check(got.cpu().numpy(), rows, rp, ci, v, Bv.cpu().numpy())
+        assert torch.equal(plan.spmm(Bv, c_half=True), got.half()) and torch.equal(plan.spmm(Bv), got)
+    finally:
+        plan.close()
