@@ -283,12 +283,12 @@ int b_tensor_map(b200spmm_plan *p, const void *B, int64_t ldb, uint32_t n, uint3
     return B200SPMM_OK;
 }
 
-// How the rows of B are gathered: TMA tile::gather4 unless the plan was made with
-// B200SPMM_GATHER=cpasync or B is narrower than one 128-byte TMA box.
+// How the rows of B are gathered: TMA tile::gather4 unless the plan was made with B200SPMM_GATHER=cpasync.  The
+// features a 128-byte box has beyond n arrive as zeros; a narrow row costs a whole box of shared memory, but the
+// cp.async copies cost the producer warps far more (pruned 28672 x 8192 weight, 8 columns: 306 us).
 template <bool kTf32>
 int launch_dtype(b200spmm_plan *p, SpmmParams &prm, cudaStream_t stream) {
-    constexpr uint32_t esz = kTf32 ? 4 : 2, box = 128 / esz;
-    if (p->gather_cpasync || prm.n < box) return launch_slab<kTf32, false, 0>(p, prm, p->tmap_b, stream);
+    if (p->gather_cpasync) return launch_slab<kTf32, false, 0>(p, prm, p->tmap_b, stream);
     {
         int st = b_tensor_map(p, prm.B, prm.ldb, prm.n, prm.cols, kTf32);
         if (st != B200SPMM_OK) return st;
@@ -476,7 +476,7 @@ template <bool kTf32>
 int launch_narrow_vecs(const NarrowParams &prm, int vecs, unsigned n_ctas, size_t smem, cudaStream_t stream) {
     using Kernel = void (*)(const NarrowParams);
     constexpr Kernel kernels[kNarrowMaxVecs] = {spmm_narrow_kernel<kTf32, 1>, spmm_narrow_kernel<kTf32, 2>, spmm_narrow_kernel<kTf32, 3>,
-                                                spmm_narrow_kernel<kTf32, 4>, spmm_narrow_kernel<kTf32, 5>, spmm_narrow_kernel<kTf32, 6>};
+                                                spmm_narrow_kernel<kTf32, 4>};
     static thread_local int configured_device = -1;
     int device = 0;
     B200_CUDA_TRY(cudaGetDevice(&device));
@@ -489,11 +489,14 @@ int launch_narrow_vecs(const NarrowParams &prm, int vecs, unsigned n_ctas, size_
     return B200SPMM_OK;
 }
 
-// Column blocks per group for B of width n: as many as fit shared memory, 0 if the kernel does not take it.
+// Column blocks per group for B of width n: as many as fit shared memory, 0 if the kernel does not take it.  Every
+// 16-byte word of a row of B adds to it - pruned 28672 x 8192 weight, fp16: 35, 68, 89, 146 us for 8, 16, 24, 32
+// columns - while the tile kernels take the same time up to 64 features (98 us; tf32: 86 and 133 us for 8 and 16
+// columns against 186), so it ends at 24 fp16 or 16 tf32 columns.
 uint32_t narrow_group_blocks(const b200spmm_plan *p, int64_t n) {
     const NarrowFormat &f = p->narrow;
     const int64_t vecs = n * p->info.elt_size / 16;
-    if (!f.n_ctas || vecs > kNarrowMaxVecs) return 0;
+    if (!f.n_ctas || vecs > (p->info.dtype == B200SPMM_TF32 ? kNarrowMaxVecs : kNarrowMaxVecs - 1)) return 0;
     uint32_t g = f.n_blocks;
     while (g && narrow_smem_bytes((uint32_t)vecs, (uint32_t)p->info.cols, g, f.n_blocks, f.max_rows, (uint32_t)n) > kNarrowSmemMax) --g;
     return g;
@@ -536,13 +539,11 @@ bool use_pair(const b200spmm_plan *p, int64_t n) {
     return (int64_t)p->pair.eff * ((n + 255) / 256) >= p->pair_clusters;
 }
 
-// Does this launch go to the super-window kernel?  Only with the TMA gathers (B at least one
-// 128-byte box wide), and - unless forced - only when there are enough (window, slab) items to
-// occupy every SM.
+// Does this launch go to the super-window kernel?  Only with the TMA gathers, and - unless forced, for B at
+// least one 128-byte box wide - only when there are enough (window, slab) items to occupy every SM.
 bool use_tall(const b200spmm_plan *p, int64_t n) {
     if (!p->tall.tiles || p->gather_cpasync) return false;
-    if (n * p->info.elt_size < 128) return false;
-    if (p->tall_forced) return true;
+    if (p->tall_forced) return n * p->info.elt_size >= 128;
     const int64_t slab = n <= 128 ? 128 : 256;
     return (int64_t)p->tall.eff * ((n + slab - 1) / slab) >= p->n_sms;
 }
@@ -1438,7 +1439,7 @@ int b200spmm_bench(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, 
 int b200spmm_kat_spmm_starved(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc,
                               unsigned long long limit_ns, void *stream) {
     if (!p || limit_ns == 0 || limit_ns > kDeviceWaitLimitNs) return B200SPMM_ERR_INVALID_ARG;
-    if (p->gather_cpasync || n * p->info.elt_size < 128) return B200SPMM_ERR_UNSUPPORTED;  // needs the TMA gathers
+    if (p->gather_cpasync || n * p->info.elt_size < 128) return B200SPMM_ERR_UNSUPPORTED;  // needs whole TMA boxes
     p->starve_gathers = true;
     p->wait_limit_ns = limit_ns;
     p->tmap_b_ptr = nullptr;  // a map encoded for a normal launch must not be reused, nor this one later

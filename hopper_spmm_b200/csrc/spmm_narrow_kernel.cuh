@@ -31,7 +31,7 @@ struct NarrowParams {
 
 constexpr int kNarrowThreads = 1024;
 constexpr int kNarrowSteps = 8;        // steps whose entries are loaded at one time, and again one ahead
-constexpr int kNarrowMaxVecs = 6;      // 16-byte words of a row of B
+constexpr int kNarrowMaxVecs = 4;      // 16-byte words of a row of B
 constexpr size_t kNarrowSmemMax = 232448;
 
 // Columns of B and (with several groups) fp32 sums in shared memory.

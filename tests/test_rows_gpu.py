@@ -80,3 +80,18 @@ def test_narrow_b_at_the_edges_of_its_column_blocks(dt, n, rows, cols):
         assert torch.equal(plan.spmm(Bv, c_half=True), got.half()) and torch.equal(plan.spmm(Bv), got)
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+@pytest.mark.parametrize("n", [8, 24, 56])
+def test_tma_boxes_wider_than_b(dt, n, monkeypatch):
+    # the 16-row tile kernel with B narrower than one 128-byte box: the features beyond n arrive as zeros
+    monkeypatch.setenv("B200SPMM_WINDOW", "16")
+    rows, cols, rp, ci, v = rows_of_lengths([40, 0, 7, 300] * 30 + [1], 500, 5, dt)
+    B = dense_b(cols, n, 6, dt)
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    try:
+        parity.check(plan.spmm_host(B), rows, rp, ci, v, B)
+        assert plan.launch_info().tma_gather == 1
+    finally:
+        plan.close()
