@@ -1204,6 +1204,13 @@ int b200spmm_plan_launch_info(const b200spmm_plan_t *p, b200spmm_launch_info_t *
 
 namespace {
 
+// cudaSetDevice costs a launch-bound call more than asking.
+cudaError_t make_current(int device) {
+    int now = -1;
+    const cudaError_t e = cudaGetDevice(&now);
+    return e == cudaSuccess && now != device ? cudaSetDevice(device) : e;
+}
+
 // The product, or one band of it (band < 0: every chunk; otherwise the chunks, rows and split
 // windows of that band of the schedule the launch selects - see b200spmm_plan::Sched).
 int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
@@ -1215,7 +1222,7 @@ int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, voi
     if ((reinterpret_cast<uintptr_t>(d_B) & 15u) || (reinterpret_cast<uintptr_t>(d_C) & 15u)) return B200SPMM_ERR_UNSUPPORTED;
     if ((ldb * esz) % 16 || (ldc * csz) % 16) return B200SPMM_ERR_UNSUPPORTED;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-    B200_CUDA_TRY(cudaSetDevice(p->device));
+    B200_CUDA_TRY(make_current(p->device));
     p->last = b200spmm_launch_info_t{};
     if (p->info.eff_row_windows == 0) {  // nothing stored: C is all zeros
         B200_CUDA_TRY(cudaMemset2DAsync(d_C, (size_t)ldc * csz, 0, (size_t)n * csz, p->info.rows, stream));

@@ -233,6 +233,24 @@ def shard_rows(rows: int, row_ptr, parts: int, row_window: int = ROW_WINDOW, row
     return cuts
 
 
+_native = None
+
+
+def _native_spmm():
+    """The native half of SpmmPlan.spmm; like the library itself it has no fallback."""
+    global _native
+    if _native is None:
+        import torch  # noqa: F401  (the module links against torch's libraries)
+        capi.lib()
+        try:
+            from ._torch_binding import spmm
+        except ImportError as e:
+            raise RuntimeError("hopper_spmm_b200/_torch_binding.so is missing or unusable: build it with "
+                               "`python -m hopper_spmm_b200.build`") from e
+        _native = spmm
+    return _native
+
+
 class SpmmPlan:
     """Device-resident matrix + persistent schedule (b200spmm_plan_*).  Replaces the
     allocate / copy / build-descriptor prologue of fp16_spmm (src/fp16.cu:236-252)."""
@@ -276,22 +294,15 @@ class SpmmPlan:
     # -- device tensors (torch) ------------------------------------------------------------
     def spmm(self, B, C_out=None, c_half: bool = False, stream=None, sync: bool = True):
         """C = A @ B for a torch CUDA tensor B [cols, n]; returns C [rows, n] (fp32, or fp16)."""
-        import torch
-        want = torch.float16 if self.is_f16 else torch.float32
-        if not B.is_cuda or B.dtype != want or B.dim() != 2 or B.stride(1) != 1 or B.shape[0] != self.cols:
-            raise ValueError(f"B must be a CUDA {want} tensor of shape [{self.cols}, n] with unit column stride")
-        n = B.shape[1]
-        cdt = torch.float16 if c_half else torch.float32
-        if C_out is None:
-            C_out = torch.empty((self.rows, n), dtype=cdt, device=B.device)
-        elif (not C_out.is_cuda or C_out.dtype != cdt or C_out.shape != (self.rows, n) or C_out.stride(1) != 1):
-            raise ValueError("C has the wrong shape, dtype or layout")
-        s = (stream or torch.cuda.current_stream(B.device)).cuda_stream
-        fn = capi.lib().b200spmm_fp16_spmm if self.is_f16 else capi.lib().b200spmm_tf32_spmm
-        capi.check(fn(self._p, B.data_ptr(), B.stride(0), n, C_out.data_ptr(), C_out.stride(0),
-                      capi.C_F16 if c_half else capi.C_F32, s), "b200spmm_spmm")
+        C_out = _native_spmm()(self._p.value or 0, self.is_f16, self.rows, self.cols, B, C_out, c_half,
+                               None if stream is None else stream.cuda_stream)
+        if type(C_out) is int:
+            raise capi.SpmmError(C_out, "b200spmm_spmm")
         if sync:
-            capi.check(capi.lib().b200spmm_plan_sync(self._p, s), "b200spmm_plan_sync")
+            if stream is None:
+                import torch
+                stream = torch.cuda.current_stream(B.device)
+            capi.check(capi.lib().b200spmm_plan_sync(self._p, stream.cuda_stream), "b200spmm_plan_sync")
         return C_out
 
     def sync(self, stream=None):
