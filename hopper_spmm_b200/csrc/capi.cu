@@ -416,6 +416,13 @@ int pair_max_clusters(int *out) {
 // A tile costs the 16-row kernel its gathered rows and one matrix instruction per 128 features whatever it
 // holds; a row unit costs a row load per entry.
 constexpr double kRowsMaxFill = 0.08;  // share of a tile's slots in use
+// Up to this fill the row units still win over 16-row tiles (128 fp16 features: graph of 10,000 nodes, degree 40, 15.0
+// against 21.7 us; 3000 x 3000 at 7 %, 10 % fill, 25.2 against 25.1 us), but not where super-windows do: those take a
+// matrix whose merged tiles are at least kTallMinFill full (pruned at 5 %) and that has enough windows for the SMs.  A
+// graph of 20,000 nodes merges well too, and waits for its hub window: 148 us against 35.  Matrices of fewer tiles
+// than two a CTA take the same few microseconds either way and stay with their tiles.
+constexpr double kRowsMaxFillWide = 0.11, kTallMinFill = 0.03;
+constexpr uint64_t kRowsWideMinTiles = 592;
 
 bool use_rows(const b200spmm_plan *p, int64_t ldb) {
     return p->rows_only && ldb * p->info.elt_size <= 0xFFFFFFFFll;  // (the kernel's row pitch is 32-bit)
@@ -758,11 +765,19 @@ int plan_build_tile_path(b200spmm_plan *p, const uint32_t *h_rowOffset, const ui
     return plan_build_tile_image(p);
 }
 
-// The window tables on the host, read back where the caller has them on the device only.
+// The window tables on the host, where the caller has them on the device only.
+int read_window_tables(b200spmm_plan *p, std::vector<uint32_t> *rowOffset, std::vector<uint32_t> *rowIdx) {
+    rowOffset->resize(p->info.eff_row_windows + 1);
+    rowIdx->resize(p->info.eff_row_windows);
+    B200_CUDA_TRY(cudaMemcpy(rowOffset->data(), p->d_rowOffset, rowOffset->size() * 4, cudaMemcpyDeviceToHost));
+    if (!rowIdx->empty()) B200_CUDA_TRY(cudaMemcpy(rowIdx->data(), p->d_rowIdx, rowIdx->size() * 4, cudaMemcpyDeviceToHost));
+    return B200SPMM_OK;
+}
+
 int plan_add_tile_path(b200spmm_plan *p, int n_ctas) {
-    std::vector<uint32_t> h_rowOffset(p->info.eff_row_windows + 1), h_rowIdx(p->info.eff_row_windows);
-    B200_CUDA_TRY(cudaMemcpy(h_rowOffset.data(), p->d_rowOffset, h_rowOffset.size() * 4, cudaMemcpyDeviceToHost));
-    if (!h_rowIdx.empty()) B200_CUDA_TRY(cudaMemcpy(h_rowIdx.data(), p->d_rowIdx, h_rowIdx.size() * 4, cudaMemcpyDeviceToHost));
+    std::vector<uint32_t> h_rowOffset, h_rowIdx;
+    const int st = read_window_tables(p, &h_rowOffset, &h_rowIdx);
+    if (st != B200SPMM_OK) return st;
     return plan_build_tile_path(p, h_rowOffset.data(), h_rowIdx.data(), n_ctas);
 }
 
@@ -786,7 +801,23 @@ int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h
     // B200SPMM_WINDOW=rows asks for the row units whatever the matrix.
     const bool force_rows = env_is("B200SPMM_WINDOW", "rows");
     if (n_ctas <= 0 && (force_rows || (!std::getenv("B200SPMM_WINDOW") && !std::getenv("B200SPMM_TILES") && !p->gather_cpasync))) {
-        int st = build_row_formats(info, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, p->n_sms, kRowsMaxFill, force_rows,
+        const double fill = info.total_tiles ? (double)info.nnzs / ((double)info.total_tiles * kRowWindow * cw) : 0.0;
+        double max_fill = kRowsMaxFill;
+        if (fill > kRowsMaxFill && fill <= kRowsMaxFillWide && info.total_tiles >= kRowsWideMinTiles && !force_rows) {
+            std::vector<uint32_t> tables[2];
+            if (!h_rowOffset) {
+                int st = read_window_tables(p, &tables[0], &tables[1]);
+                if (st != B200SPMM_OK) return st;
+            }
+            double ratio = 1.0;
+            uint64_t n_super = 0;
+            int st = estimate_tall_tile_ratio(info, h_rowOffset ? h_rowOffset : tables[0].data(), h_rowOffset ? h_rowIdx : tables[1].data(),
+                                              p->d_tcA2B, kTallRows, 48, &ratio, &n_super);
+            if (st != B200SPMM_OK) return st;
+            // (an eighth of the short tiles is the least that merging eight windows can leave)
+            if (fill / (8.0 * ratio) < kTallMinFill || n_super * 4 < (uint64_t)p->n_sms) max_fill = kRowsMaxFillWide;
+        }
+        int st = build_row_formats(info, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, p->n_sms, max_fill, force_rows,
                                    &p->rows_fmt, &p->narrow);
         if (st != B200SPMM_OK) return st;
         p->rows_only = p->rows_fmt.n_units > 0;
@@ -1228,9 +1259,9 @@ int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, voi
         B200_CUDA_TRY(cudaMemset2DAsync(d_C, (size_t)ldc * csz, 0, (size_t)n * csz, p->info.rows, stream));
         return B200SPMM_OK;
     }
-    if (!p->starve_gathers && use_rows(p, ldb)) return launch_rows(p, d_B, ldb, n, d_C, ldc, c_dtype, stream, band);
     if (const uint32_t g = p->starve_gathers || band >= 0 ? 0u : narrow_group_blocks(p, n))
         return launch_narrow(p, g, d_B, ldb, n, d_C, ldc, c_dtype, stream);
+    if (!p->starve_gathers && use_rows(p, ldb)) return launch_rows(p, d_B, ldb, n, d_C, ldc, c_dtype, stream, band);
     if (!p->has_tile_path) {  // only row units were kept; the starved test launch and a huge ldb ask for more
         int st = plan_add_tile_path(p, 0);
         if (st != B200SPMM_OK) return st;
@@ -1350,7 +1381,7 @@ int b200spmm_spmm_host(b200spmm_plan_t *p, const void *h_B, int64_t n, void *h_C
         band_row.clear();
         for (const RowBand &b : p->rows_fmt.bands) band_row.push_back(b.row);
     }
-    const size_t bands = band_row.size() > 1 && (rows || !(use_tall(p, n) || narrow_group_blocks(p, n))) ? band_row.size() - 1 : 1;
+    const size_t bands = band_row.size() > 1 && !narrow_group_blocks(p, n) && (rows || !use_tall(p, n)) ? band_row.size() - 1 : 1;
     if (bands == 1 || p->info.eff_row_windows == 0) {
         B200_CUDA_TRY(cudaMemcpyAsync(p->d_B, h_B, b_bytes, cudaMemcpyHostToDevice, nullptr));
         int st = b200spmm_spmm(p, p->d_B, n, n, p->d_C, n, c_dtype, nullptr);

@@ -491,6 +491,7 @@ int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
             return build_narrow(info, h[0], d_rowOffset, d_tcA2B, d_data, d_rowIdx, n_sms, run_first, run_window, run_grid, counts, a, narrow);
         return B200SPMM_OK;
     }
+    const uint32_t h_max_len = h[kMaxLenAt];
     f.nnz = h[0];
     f.n_units = h[1];
     f.n_splits = h[2];
@@ -554,6 +555,10 @@ int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
     f.bands[bands].empty = f.n_units;
     f.n_batches = h[2 * bands + 2];
     B200_CUDA_TRY(cudaDeviceSynchronize());
+    if (!force_rows && narrow_pays(f.nnz, rows, info.cols, h_max_len, n_sms)) {
+        const int st = build_narrow(info, f.nnz, d_rowOffset, d_tcA2B, d_data, d_rowIdx, n_sms, run_first, run_window, run_grid, counts, a, narrow);
+        if (st != B200SPMM_OK) return st;
+    }
     *out = f;
     guard.f = nullptr;
     return B200SPMM_OK;

@@ -95,3 +95,20 @@ def test_tma_boxes_wider_than_b(dt, n, monkeypatch):
         assert plan.launch_info().tma_gather == 1
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("density,rows_kernel", [(0.04, True), (0.07, True), (0.11, False)])
+def test_fill_of_the_tiles_decides_between_units_and_tiles(density, rows_kernel):
+    # 0.04: 7 % of a tile's slots in use, 0.07: 10 %, and super-windows would wait for too few tiles; 0.11: 13 %
+    import torch
+    rng = np.random.default_rng(2)
+    lengths = rng.binomial(700, density, 600)
+    rows, cols, rp, ci, v = rows_of_lengths(lengths, 700, 7, np.float16)
+    B = dense_b(cols, 96, 2)
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    try:
+        got = plan.spmm(torch.from_numpy(B).cuda())
+        assert (plan.launch_info().stages == 0) == rows_kernel
+        parity.check(got.cpu().numpy(), rows, rp, ci, v, B)
+    finally:
+        plan.close()
