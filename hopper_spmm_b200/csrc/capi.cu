@@ -115,6 +115,7 @@ struct b200spmm_plan {
     const void *tmap_b_ptr = nullptr;
     int64_t tmap_b_ldb = 0;
     uint32_t tmap_b_n = 0;
+    bool row_boxes = false;       // keep tmap_bt (the allocation-free call encodes one map only)
     bool gather_cpasync = false;  // B200SPMM_GATHER=cpasync, read when the plan is made
     unsigned long long wait_limit_ns = kDeviceWaitLimitNs;  // how long a wait inside the kernel may last
     bool starve_gathers = false;  // b200spmm_kat_spmm_starved only: B's tensor map delivers half the bytes
@@ -194,7 +195,7 @@ int launch_one(b200spmm_plan *p, const SpmmParams &prm, const CUtensorMap &tmap_
         B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         configured_device = p->device;
     }
-    kernel<<<p->launch_sched->n_ctas, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(p->tmap_a, tmap_b, prm);
+    kernel<<<p->launch_sched->n_ctas, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(p->tmap_a, tmap_b, p->tmap_bt, prm);
     B200_CUDA_TRY(cudaGetLastError());
     p->last.n_ctas = p->launch_sched->n_ctas;
     p->last.threads = Cfg::kThreads;
@@ -270,9 +271,9 @@ int b_tensor_map(b200spmm_plan *p, const void *B, int64_t ldb, uint32_t n, uint3
         set_last_error_static("cuTensorMapEncodeTiled failed for B");
         return B200SPMM_ERR_CUDA;
     }
-    if (p->tall.tiles &&
+    if (p->row_boxes &&
         !encode_2d(&p->tmap_bt, tf32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, B, n, cols,
-                   (uint64_t)ldb * esz, 128 / esz, std::min<uint32_t>((uint32_t)p->info.col_window, cols),
+                   (uint64_t)ldb * esz, box, std::min<uint32_t>((uint32_t)p->info.col_window, cols),
                    tf32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B)) {
         set_last_error_static("cuTensorMapEncodeTiled failed for B (row boxes)");
         return B200SPMM_ERR_CUDA;
@@ -294,6 +295,7 @@ int launch_dtype(b200spmm_plan *p, SpmmParams &prm, cudaStream_t stream) {
         if (st != B200SPMM_OK) return st;
     }
     const CUtensorMap &tmap_b = p->tmap_b;
+    prm.row_boxes = p->row_boxes ? 1u : 0u;
     if (p->comp.tcBit) {  // stream the compressed tiles
         prm.tcBit = p->comp.tcBit;
         prm.nnzOffset = p->comp.nnzOffset;
@@ -797,6 +799,7 @@ int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h
     B200_CUDA_TRY(cudaMemset(p->d_status, 0, 4 * sizeof(uint32_t)));
     p->gather_cpasync = env_is("B200SPMM_GATHER", "cpasync");
     p->host_split = !env_is("B200SPMM_HOST_SPLIT", "0");
+    p->row_boxes = true;
     // An explicit CTA count, a way to fetch tiles or rows, or a window height asks for a tile kernel.
     // B200SPMM_WINDOW=rows asks for the row units whatever the matrix.
     const bool force_rows = env_is("B200SPMM_WINDOW", "rows");

@@ -118,6 +118,7 @@ struct SpmmParams {
     uint32_t eff_row_windows;
     uint32_t n_slabs;            // ceil(n / kNs)
     uint32_t c_is_half;          // 0: fp32 C, 1: fp16 C
+    uint32_t row_boxes;          // 1: tiles whose columns are neighbours fetch their rows of B as boxes (tmap_bt)
     uint32_t *status;            // device status word
     unsigned long long wait_limit_ns;
 #ifdef B200SPMM_PROFILE
@@ -169,7 +170,9 @@ struct SpmmCfg {
     // that box for four of the tile's rows.
     static constexpr int kBoxFeatures = 128 / kEsz;
     static constexpr int kRowQuads = kCW / 4;
-    static constexpr int kGatherOps = kRowQuads * (kNs / kBoxFeatures);  // per tile, at most 16
+    static constexpr int kBoxes = kNs / kBoxFeatures;      // 128-byte column blocks of a slab
+    static constexpr int kBoxBytes = kCW * 128;            // CW neighbouring rows of B, one column block
+    static constexpr int kGatherOps = kRowQuads * kBoxes;  // per tile, at most 16
     static constexpr int kWinAhead = 16;   // windows whose tile counts the MMA issuer prefetches
     static constexpr int kWinSlots = 32;
     // Each producer warp keeps the column lists of its next kIdxAhead tiles in a private ring of
@@ -197,7 +200,7 @@ struct SpmmCfg {
 template <bool kTf32, int kNs, bool kTma, int kTiles>
 __global__ void __launch_bounds__((SpmmCfg<kTf32, kNs, kTma, kTiles>::kThreads), (SpmmCfg<kTf32, kNs, kTma, kTiles>::kCtasPerSm))
 spmm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                  const SpmmParams p) {
+                  const __grid_constant__ CUtensorMap tmap_bt, const SpmmParams p) {
     using Cfg = SpmmCfg<kTf32, kNs, kTma, kTiles>;
     constexpr bool kBitmap = Cfg::kBitmap, kEntries = Cfg::kEntries;
     constexpr int kStages = Cfg::kStages;
@@ -294,6 +297,7 @@ spmm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         ptx::fence_mbar_init();
         if (kTiles == 0) ptx::prefetch_tensormap(&tmap_a);
         if (kTma) ptx::prefetch_tensormap(&tmap_b);
+        if (kTma && p.row_boxes) ptx::prefetch_tensormap(&tmap_bt);
     }
     if (warp == kMmaWarp) {
         ptx::tmem_alloc(ptx::smem_u32(tmem_slot), kTmemCols);
@@ -735,8 +739,17 @@ spmm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             }
             if (kTma) {
                 B200_PROF_T0();
-                if (half < gather_here && hl < (uint32_t)Cfg::kGatherOps) {
-                    const uint4 rows4 = *reinterpret_cast<const uint4 *>(slot_words + half * Cfg::kCW + op_quad * 4);
+                // A list is ascending and distinct (padding 0xFFFFFFFF at its end): when its last entry is CW - 1 past
+                // its first, the tile's rows of B are neighbours (a matrix of aligned blocks has no others) and come
+                // as boxes of CW rows, half or a quarter of the instructions and none of the gather's rate limit.
+                const uint32_t *list = slot_words + half * Cfg::kCW;
+                const uint32_t list0 = list[0];
+                if (p.row_boxes && list[Cfg::kCW - 1] - list0 == (uint32_t)Cfg::kCW - 1u) {
+                    if (half < gather_here && hl < (uint32_t)Cfg::kBoxes)
+                        ptx::tma_load_2d(gather_addr + (first_slot + half) * Cfg::kGatherBytes + hl * Cfg::kBoxBytes, &tmap_bt,
+                                         (int32_t)(slab * kNs + hl * Cfg::kBoxFeatures), (int32_t)list0, full_bar(s));
+                } else if (half < gather_here && hl < (uint32_t)Cfg::kGatherOps) {
+                    const uint4 rows4 = *reinterpret_cast<const uint4 *>(list + op_quad * 4);
                     // padded slots hold 0xFFFFFFFF: clamp to the first row past the end, which reads zeros
                     ptx::tma_gather4_2d(gather_addr + (first_slot + half) * Cfg::kGatherBytes + op_dst, &tmap_b,
                                         (int32_t)(slab * kNs + op_x),

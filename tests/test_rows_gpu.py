@@ -112,3 +112,26 @@ def test_fill_of_the_tiles_decides_between_units_and_tiles(density, rows_kernel)
         parity.check(got.cpu().numpy(), rows, rp, ci, v, B)
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+@pytest.mark.parametrize("n", [16, 64, 136, 320])
+def test_tiles_of_consecutive_columns_read_b_in_boxes(dt, n):
+    # dense blocks: B's rows arrive in one box per tile, past its last row in the ragged one; mixed tiles in between
+    import torch
+    rng = np.random.default_rng(1)
+    cols = 1045
+    blocks = [np.arange(b, min(b + 29, cols)) for b in (0, 131, 640, cols - 29, cols - 5)]
+    per_row = [np.unique(np.concatenate([blocks[(r // 16) % 5], blocks[(r // 48 + 2) % 5], rng.choice(cols, 3)])) for r in range(400)]
+    ci = np.concatenate(per_row).astype(np.uint32)
+    rp = np.concatenate([[0], np.cumsum([c.size for c in per_row])]).astype(np.uint32)
+    v = rng.uniform(0.1, 1, ci.size).astype(np.float32).astype(dt)
+    B = dense_b(cols, n, 8, dt)
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(400, cols, rp, ci, v)))
+    try:
+        dC = torch.full((400, n), float("nan"), device="cuda")
+        plan.spmm(torch.from_numpy(B).cuda(), dC)
+        assert plan.launch_info().stages > 0
+        parity.check(dC.cpu().numpy(), 400, rp, ci, v, B)
+    finally:
+        plan.close()
