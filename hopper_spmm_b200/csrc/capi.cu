@@ -420,11 +420,12 @@ int pair_max_clusters(int *out) {
 constexpr double kRowsMaxFill = 0.08;  // share of a tile's slots in use
 // Up to this fill the row units still win over 16-row tiles (128 fp16 features: graph of 10,000 nodes, degree 40, 15.0
 // against 21.7 us; 3000 x 3000 at 7 %, 10 % fill, 25.2 against 25.1 us), but not where super-windows do: those take a
-// matrix whose merged tiles are at least kTallMinFill full (pruned at 5 %) and that has enough windows for the SMs.  A
+// matrix whose merged tiles are at least kTallMinFill full (pruned at 5 %) and that has enough of them for the SMs.  A
 // graph of 20,000 nodes merges well too, and waits for its hub window: 148 us against 35.  Matrices of fewer tiles
 // than two a CTA take the same few microseconds either way and stay with their tiles.
 constexpr double kRowsMaxFillWide = 0.11, kTallMinFill = 0.03;
 constexpr uint64_t kRowsWideMinTiles = 592;
+constexpr uint64_t kTallMinShortTiles = 16384;  // 19 us with 16 rows at 64 columns: nothing to gain with 128
 
 bool use_rows(const b200spmm_plan *p, int64_t ldb) {
     return p->rows_only && ldb * p->info.elt_size <= 0xFFFFFFFFll;  // (the kernel's row pitch is 32-bit)
@@ -542,19 +543,32 @@ int launch_narrow(b200spmm_plan *p, uint32_t group_blocks, const void *d_B, int6
     return B200SPMM_OK;
 }
 
+// How long a launch takes, in microseconds, to choose between the tile kernels.  A super-window launch lasts as many
+// rounds of its CTAs or pairs as its items need, each as long as the longest window, so a matrix with one heavy window
+// stays with 16 rows; the 16-row kernel spreads its tiles evenly over all CTAs.  It pays long before every SM has an
+// item: pruned 14336 x 4096, 10 %, fp16, 64 / 128 / 192 columns 33 / 36 / 43 us (56 windows of 256 rows for 74 pairs)
+// against 62 / 79 / 146 with 16 rows; 3000 x 3000, 12 %, 192 columns 33 against 45, but at 64 columns 25 against 23.
+double tall_micros(const TallFormat &f, int units, int64_t n, int64_t slab) {
+    const int64_t items = (int64_t)f.eff * ((n + slab - 1) / slab);
+    return 12.0 + (double)((items + units - 1) / units) * (double)f.max_window_tiles * (slab > 128 ? 0.11 : 0.085);
+}
+double short_micros(const b200spmm_plan *p, int64_t n) {
+    return 14.0 + (double)p->info.total_tiles * (n <= 64 ? 0.28e-3 : 0.4e-3 * (double)((n + 127) / 128));
+}
+
 bool use_pair(const b200spmm_plan *p, int64_t n) {
     if (!p->pair.tiles || p->pair_clusters < 1 || n <= 128) return false;
     if (p->tall_forced) return true;
-    return (int64_t)p->pair.eff * ((n + 255) / 256) >= p->pair_clusters;
+    return tall_micros(p->pair, p->pair_clusters, n, 256) < short_micros(p, n);
 }
 
 // Does this launch go to the super-window kernel?  Only with the TMA gathers, and - unless forced, for B at
-// least one 128-byte box wide - only when there are enough (window, slab) items to occupy every SM.
+// least one 128-byte box wide - only when it is expected to be faster.
 bool use_tall(const b200spmm_plan *p, int64_t n) {
     if (!p->tall.tiles || p->gather_cpasync) return false;
     if (p->tall_forced) return n * p->info.elt_size >= 128;
     const int64_t slab = n <= 128 ? 128 : 256;
-    return (int64_t)p->tall.eff * ((n + slab - 1) / slab) >= p->n_sms;
+    return use_pair(p, n) || tall_micros(p->tall, p->n_sms, n, slab) < short_micros(p, n);
 }
 
 int launch_tall(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
@@ -632,7 +646,7 @@ int plan_build_tall(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_
         int st = estimate_tall_tile_ratio(info, h_rowOffset, h_rowIdx, p->d_tcA2B, kTallRows, 48, &ratio, &n_super);
         if (st != B200SPMM_OK) return st;
         // fewer super-windows than SMs / 16 can never fill the GPU, however wide B is
-        if (ratio > 0.7 || n_super * 16 < (uint64_t)p->n_sms) return B200SPMM_OK;
+        if (ratio > 0.7 || n_super * 16 < (uint64_t)p->n_sms || info.total_tiles < kTallMinShortTiles) return B200SPMM_OK;
     }
     int st = build_tall_device(info, h_rowOffset, h_rowIdx, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, kTallRows, &p->tall);
     if (st == B200SPMM_ERR_UNSUPPORTED) return B200SPMM_OK;  // too many tiles for 32-bit offsets: 16-row kernel
@@ -818,7 +832,7 @@ int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h
                                               p->d_tcA2B, kTallRows, 48, &ratio, &n_super);
             if (st != B200SPMM_OK) return st;
             // (an eighth of the short tiles is the least that merging eight windows can leave)
-            if (fill / (8.0 * ratio) < kTallMinFill || n_super * 4 < (uint64_t)p->n_sms) max_fill = kRowsMaxFillWide;
+            if (fill / (8.0 * ratio) < kTallMinFill || info.total_tiles < kTallMinShortTiles) max_fill = kRowsMaxFillWide;
         }
         int st = build_row_formats(info, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, p->n_sms, max_fill, force_rows,
                                    &p->rows_fmt, &p->narrow);

@@ -182,3 +182,20 @@ def test_starved_pipeline_times_out_and_the_plan_recovers(dt, tall):
             parity.check(dC.cpu().numpy(), rows, rp, ci, v, B.cpu().numpy())
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("dt,n,window", [(np.float16, 64, 16), (np.float16, 136, 256), (np.float16, 256, 256), (np.float32, 64, 16),
+                                         (np.float32, 200, 256)])
+def test_fewer_windows_than_sms_take_the_kernel_expected_to_be_faster(dt, n, window):
+    # twelve windows of 256 rows: most pairs of SMs stay idle, and from two slabs of 128 on they are still the faster ones
+    import torch
+    rows, cols, rp, ci, v = random_csr(2990, 3001, 0.12, 5, dt, empty_rows=[(512, 640)])
+    B = dense_b(cols, n, 3, dt)
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    try:
+        dC = torch.full((rows, n), float("nan"), device="cuda")
+        plan.spmm(torch.from_numpy(B).cuda(), dC)
+        assert plan.launch_info().row_window == window
+        parity.check(dC.cpu().numpy(), rows, rp, ci, v, B)
+    finally:
+        plan.close()
