@@ -9,13 +9,17 @@
 //   1. one key (window, column) per entry, in as few bits as the matrix needs - 32-bit keys where they fit - since
 //      every eight bits are a pass of the sort; the entry's row is found by binary search in row_ptr
 //   2. radix sort of the keys, then unique -> the sorted distinct columns of every window
-//      (CUB device primitives: sort, select-unique, run-length encode, scans)
-//   3. run lengths per window -> tiles per window -> rowOffset, rowIdx; column lists scattered into
-//      tcA2B (pre-filled with 0xFFFFFFFF padding)
-//   4. every entry finds its slot by binary search in its window's column list and is written into
+//      (CUB device primitives: sort, select-unique, scan)
+//   3. every window finds its range of them by binary search; one scan of (holds entries, tiles) gives
+//      rowOffset, rowIdx and all sizes.  The host waits for the device once on the way, for those sizes: a
+//      wait in each step (entries, distinct columns, windows, tiles) left the device idle for 80 of 290 us on
+//      a matrix of 700,000 entries.
+//   4. column lists scattered into tcA2B (pre-filled with 0xFFFFFFFF padding); every entry finds its slot by binary search in its window's column list and is written into
 //      the zero-filled tile array
+#include <algorithm>
 #include <cstdint>
 #include <cub/cub.cuh>
+#include <thrust/iterator/counting_iterator.h>
 #include <thrust/iterator/transform_iterator.h>
 #include <new>
 
@@ -36,9 +40,10 @@ namespace gpuconv {
 
 constexpr int kBlock = 256;
 
-__device__ __forceinline__ uint32_t row_of_entry(const uint32_t *__restrict__ row_ptr, uint32_t rows, uint32_t p) {
-    // last row r with row_ptr[r] <= p
-    uint32_t lo = 0, hi = rows;
+constexpr uint32_t kKeyEntries = 4 * kBlock;  // entries a block takes at a time in make_keys_kernel
+
+// last row r in [lo, hi) with row_ptr[r] <= p, or lo
+__device__ __forceinline__ uint32_t row_of_entry(const uint32_t *__restrict__ row_ptr, uint32_t lo, uint32_t hi, uint32_t p) {
     while (hi - lo > 1) {
         const uint32_t mid = lo + (hi - lo) / 2;
         if (row_ptr[mid] <= p) lo = mid; else hi = mid;
@@ -46,70 +51,105 @@ __device__ __forceinline__ uint32_t row_of_entry(const uint32_t *__restrict__ ro
     return lo;
 }
 
-// keys[p] = window(p) << col_bits | col[p]; row_of[p]; flags a column out of range or a row whose
-// columns are not strictly ascending.
+struct Totals {
+    uint64_t n_unique;
+    unsigned long long windows_tiles;  // windows that hold entries << 32 | their tiles
+    uint32_t bad;
+};
+
+// keys[p] = window(p) << col_bits | col[p]; row_of[p]; flags row pointers that do not run from 0 to nnz, a column out
+// of range or a row whose columns are not strictly ascending.  Neighbouring entries lie in few rows: a block searches
+// the whole of row_ptr for its first and last entry only.
 template <typename K>
-__global__ void make_keys_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ col_idx,
-                                 uint32_t rows, uint32_t cols, uint64_t nnz, uint32_t row_window, int col_bits,
-                                 K *__restrict__ keys, uint32_t *__restrict__ row_of, uint32_t *__restrict__ bad) {
-    for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t r = row_of_entry(row_ptr, rows, (uint32_t)p);
-        const uint32_t c = col_idx[p];
-        if (c >= cols || (p > row_ptr[r] && col_idx[p - 1] >= c)) atomicOr(bad, 1u);
-        keys[p] = ((K)(r / row_window) << col_bits) | c;
-        row_of[p] = r;
+__global__ void __launch_bounds__(kBlock)
+make_keys_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ col_idx, uint32_t rows, uint32_t cols, uint64_t nnz,
+                 uint32_t row_window, int col_bits, K *__restrict__ keys, uint32_t *__restrict__ row_of, Totals *__restrict__ totals) {
+    __shared__ uint32_t range[2];
+    if (blockIdx.x == 0 && threadIdx.x == 0 && (row_ptr[0] != 0 || row_ptr[rows] != nnz)) atomicOr(&totals->bad, 1u);
+    for (uint64_t p0 = (uint64_t)blockIdx.x * kKeyEntries; p0 < nnz; p0 += (uint64_t)gridDim.x * kKeyEntries) {
+        const uint64_t p1 = min(p0 + kKeyEntries, nnz);
+        __syncthreads();
+        if (threadIdx.x < 2) range[threadIdx.x] = row_of_entry(row_ptr, 0, rows, (uint32_t)(threadIdx.x ? p1 - 1 : p0));
+        __syncthreads();
+        const uint32_t first = range[0], end = max(range[1], first) + 1;
+        for (uint64_t p = p0 + threadIdx.x; p < p1; p += kBlock) {
+            const uint32_t r = row_of_entry(row_ptr, first, end, (uint32_t)p), c = col_idx[p], start = row_ptr[r];
+            if (c >= cols || p < start || p >= row_ptr[r + 1] || (p > start && col_idx[p - 1] >= c)) atomicOr(&totals->bad, 1u);
+            keys[p] = ((K)(r / row_window) << col_bits) | c;
+            row_of[p] = r;
+        }
     }
 }
 
+// first[w] = distinct (window, column) pairs of the windows before w
 template <typename K>
-struct WindowOfKey {
-    int col_bits;
-    __host__ __device__ uint32_t operator()(K k) const { return (uint32_t)(k >> col_bits); }
+__global__ void window_bounds_kernel(const K *__restrict__ ukeys, const Totals *__restrict__ totals, uint32_t n_windows, int col_bits,
+                                     uint32_t *__restrict__ first) {
+    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w > n_windows) return;
+    uint32_t lo = 0, hi = totals->bad ? 0u : (uint32_t)totals->n_unique;  // (the keys of a bad matrix need not be sorted)
+    if (w == n_windows) lo = hi;
+    while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        if (ukeys[mid] < (K)w << col_bits) lo = mid + 1; else hi = mid;
+    }
+    first[w] = lo;
+}
+
+// The window's terms of the scan.  Fewer than 2^32 entries make fewer than 2^30 full tiles, 2^29 windows as many more.
+struct WindowTerms {
+    const uint32_t *first;
+    uint32_t n_windows, col_window;
+    __host__ __device__ unsigned long long operator()(uint32_t w) const {
+        if (w >= n_windows) return 0;
+        const uint32_t n = first[w + 1] - first[w];
+        return (unsigned long long)(n != 0) << 32 | ((unsigned long long)n + col_window - 1) / col_window;
+    }
 };
 
-// per effective window e: tiles, first row; dense map window -> e
-__global__ void window_tables_kernel(const uint32_t *__restrict__ win_ids, const uint32_t *__restrict__ counts,
-                                     uint32_t eff, uint32_t row_window, uint32_t col_window,
-                                     uint32_t *__restrict__ tiles, uint32_t *__restrict__ rowIdx,
-                                     uint32_t *__restrict__ win2eff) {
-    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= eff) return;
-    tiles[e] = (counts[e] + col_window - 1) / col_window;
-    rowIdx[e] = win_ids[e] * row_window;
-    win2eff[win_ids[e]] = e;
+__global__ void window_tables_kernel(const uint32_t *__restrict__ first, const unsigned long long *__restrict__ before, uint32_t n_windows,
+                                     uint32_t row_window, uint32_t *__restrict__ rowOffset, uint32_t *__restrict__ rowIdx,
+                                     uint32_t *__restrict__ tile_of, Totals *__restrict__ totals) {
+    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w > n_windows) return;
+    const uint32_t e = (uint32_t)(before[w] >> 32), tile = (uint32_t)before[w];
+    if (w == n_windows) {
+        rowOffset[e] = tile;
+        totals->windows_tiles = before[w];
+        return;
+    }
+    tile_of[w] = tile;
+    if (first[w + 1] == first[w]) return;
+    rowOffset[e] = tile;
+    rowIdx[e] = w * row_window;
 }
 
 // distinct column j (sorted by window, column) -> its place in the window's padded column list
 template <typename K>
-__global__ void scatter_columns_kernel(const K *__restrict__ ukeys, uint64_t n_unique, int col_bits,
-                                       const uint32_t *__restrict__ win2eff, const uint32_t *__restrict__ ubase,
-                                       const uint32_t *__restrict__ rowOffset, uint32_t col_window,
-                                       uint32_t *__restrict__ tcA2B) {
+__global__ void scatter_columns_kernel(const K *__restrict__ ukeys, uint64_t n_unique, int col_bits, const uint32_t *__restrict__ first,
+                                       const uint32_t *__restrict__ tile_of, uint32_t col_window, uint32_t *__restrict__ tcA2B) {
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n_unique; j += (uint64_t)gridDim.x * blockDim.x) {
         const K k = ukeys[j];
-        const uint32_t e = win2eff[(uint32_t)(k >> col_bits)];
-        const uint64_t pos = j - ubase[e];
-        tcA2B[(uint64_t)rowOffset[e] * col_window + pos] = (uint32_t)(k & (((K)1 << col_bits) - 1));
+        const uint32_t w = (uint32_t)(k >> col_bits);
+        tcA2B[(uint64_t)tile_of[w] * col_window + (j - first[w])] = (uint32_t)(k & (((K)1 << col_bits) - 1));
     }
 }
 
-// entry p -> data[(rowOffset[e] + slot / CW) * RW * CW + (r % RW) * CW + slot % CW]
+// entry p -> its slot in the zero-filled tile array
 template <typename T>
 __global__ void scatter_values_kernel(const uint32_t *__restrict__ col_idx, const T *__restrict__ values,
-                                      const uint32_t *__restrict__ row_of, uint64_t nnz,
-                                      const uint32_t *__restrict__ win2eff, const uint32_t *__restrict__ rowOffset,
-                                      const uint32_t *__restrict__ counts, const uint32_t *__restrict__ tcA2B,
-                                      uint32_t row_window, uint32_t col_window, T *__restrict__ data) {
+                                      const uint32_t *__restrict__ row_of, uint64_t nnz, const uint32_t *__restrict__ first,
+                                      const uint32_t *__restrict__ tile_of, const uint32_t *__restrict__ tcA2B, uint32_t row_window,
+                                      uint32_t col_window, T *__restrict__ data) {
     for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t r = row_of[p], c = col_idx[p];
-        const uint32_t e = win2eff[r / row_window];
-        const uint32_t *list = tcA2B + (uint64_t)rowOffset[e] * col_window;
-        uint32_t lo = 0, hi = counts[e];  // the window's real columns are ascending; padding follows them
+        const uint32_t r = row_of[p], c = col_idx[p], w = r / row_window, tile0 = tile_of[w];
+        const uint32_t *list = tcA2B + (uint64_t)tile0 * col_window;
+        uint32_t lo = 0, hi = first[w + 1] - first[w];  // the window's real columns are ascending; padding follows them
         while (lo < hi) {
             const uint32_t mid = lo + (hi - lo) / 2;
             if (list[mid] < c) lo = mid + 1; else hi = mid;
         }
-        const uint64_t tile = (uint64_t)rowOffset[e] + lo / col_window;
+        const uint64_t tile = (uint64_t)tile0 + lo / col_window;
         data[tile * row_window * col_window + (uint64_t)(r % row_window) * col_window + lo % col_window] = values[p];
     }
 }
@@ -125,91 +165,70 @@ int convert_on_device(b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const uint32
     const int esz = f->info.elt_size;
     PoolScratch tmp(stream);
     K *keys = nullptr, *keys_sorted = nullptr, *ukeys = nullptr;
-    uint64_t *n_sel = nullptr;
-    uint32_t *row_of = nullptr, *bad = nullptr, *win_ids = nullptr, *counts = nullptr, *n_runs = nullptr;
-    uint32_t *tiles = nullptr, *ubase = nullptr, *win2eff = nullptr;
+    Totals *totals = nullptr;
+    uint32_t *row_of = nullptr, *first = nullptr, *tile_of = nullptr;
+    unsigned long long *before = nullptr;
     B200_CUDA_TRY(tmp.alloc(&keys, nnz));
     B200_CUDA_TRY(tmp.alloc(&keys_sorted, nnz));
     B200_CUDA_TRY(tmp.alloc(&row_of, nnz));
-    B200_CUDA_TRY(tmp.alloc(&bad, 1));
-    B200_CUDA_TRY(tmp.alloc(&n_sel, 1));
-    B200_CUDA_TRY(tmp.alloc(&n_runs, 1));
-    B200_CUDA_TRY(cudaMemsetAsync(bad, 0, 4, stream));
+    B200_CUDA_TRY(tmp.alloc(&totals, 1));
+    B200_CUDA_TRY(tmp.alloc(&first, n_windows + 1));
+    B200_CUDA_TRY(tmp.alloc(&tile_of, n_windows));
+    B200_CUDA_TRY(tmp.alloc(&before, n_windows + 1));
+    ukeys = keys;  // the unsorted keys are dead once sorted: reuse their buffer for the distinct keys
+    auto terms = thrust::make_transform_iterator(thrust::make_counting_iterator<uint32_t>(0), WindowTerms{first, (uint32_t)n_windows, CW});
+    size_t sort_bytes = 0, sel_bytes = 0, scan_bytes = 0;
+    B200_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, keys, keys_sorted, (int64_t)nnz, 0, key_bits, stream));
+    B200_CUDA_TRY(cub::DeviceSelect::Unique(nullptr, sel_bytes, keys_sorted, ukeys, &totals->n_unique, (int64_t)nnz, stream));
+    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, terms, before, (int64_t)n_windows + 1, stream));
+    uint8_t *cub_tmp = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&cub_tmp, std::max({sort_bytes, sel_bytes, scan_bytes})));
+    B200_CUDA_TRY(pool_alloc(&f->d_rowOffset, n_windows + 1, stream));
+    B200_CUDA_TRY(pool_alloc(&f->d_rowIdx, n_windows, stream));
 
     // 1. keys
-    make_keys_kernel<<<grid_for(nnz), kBlock, 0, stream>>>(d_row_ptr, d_col_idx, (uint32_t)rows, (uint32_t)cols, nnz, RW,
-                                                           col_bits, keys, row_of, bad);
+    B200_CUDA_TRY(cudaMemsetAsync(totals, 0, sizeof(Totals), stream));
+    const int key_grid = (int)std::min<uint64_t>((nnz + kKeyEntries - 1) / kKeyEntries, 148 * 8);
+    make_keys_kernel<<<key_grid, kBlock, 0, stream>>>(d_row_ptr, d_col_idx, (uint32_t)rows, (uint32_t)cols, nnz, RW, col_bits, keys, row_of,
+                                                      totals);
     B200_CUDA_TRY(cudaGetLastError());
 
     // 2. sort, unique
-    size_t sort_bytes = 0, sel_bytes = 0, rle_bytes = 0, scan_bytes = 0;
-    B200_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, keys, keys_sorted, (int64_t)nnz, 0, key_bits, stream));
-    ukeys = keys;  // the unsorted keys are dead once sorted: reuse their buffer for the distinct keys
-    B200_CUDA_TRY(cub::DeviceSelect::Unique(nullptr, sel_bytes, keys_sorted, ukeys, n_sel, (int64_t)nnz, stream));
-    uint8_t *cub_tmp = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&cub_tmp, std::max(sort_bytes, sel_bytes)));
     B200_CUDA_TRY(cub::DeviceRadixSort::SortKeys(cub_tmp, sort_bytes, keys, keys_sorted, (int64_t)nnz, 0, key_bits, stream));
-    B200_CUDA_TRY(cub::DeviceSelect::Unique(cub_tmp, sel_bytes, keys_sorted, ukeys, n_sel, (int64_t)nnz, stream));
-    uint64_t n_unique = 0;
-    uint32_t bad_h = 0;
-    B200_CUDA_TRY(cudaMemcpyAsync(&n_unique, n_sel, 8, cudaMemcpyDeviceToHost, stream));
-    B200_CUDA_TRY(cudaMemcpyAsync(&bad_h, bad, 4, cudaMemcpyDeviceToHost, stream));
-    B200_CUDA_TRY(cudaStreamSynchronize(stream));
-    if (bad_h) return B200SPMM_ERR_BAD_CSR;
+    B200_CUDA_TRY(cub::DeviceSelect::Unique(cub_tmp, sel_bytes, keys_sorted, ukeys, &totals->n_unique, (int64_t)nnz, stream));
 
-    // 3. windows: run lengths of the window id over the distinct keys
-    B200_CUDA_TRY(tmp.alloc(&win_ids, std::min<uint64_t>(n_windows, n_unique)));
-    B200_CUDA_TRY(tmp.alloc(&counts, std::min<uint64_t>(n_windows, n_unique) + 1));
-    auto win_of = thrust::make_transform_iterator(static_cast<const K *>(ukeys), WindowOfKey<K>{col_bits});
-    B200_CUDA_TRY(cub::DeviceRunLengthEncode::Encode(nullptr, rle_bytes, win_of, win_ids, counts, n_runs, (int64_t)n_unique, stream));
-    uint8_t *rle_tmp = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&rle_tmp, rle_bytes));
-    B200_CUDA_TRY(cub::DeviceRunLengthEncode::Encode(rle_tmp, rle_bytes, win_of, win_ids, counts, n_runs, (int64_t)n_unique, stream));
-    uint32_t eff = 0;
-    B200_CUDA_TRY(cudaMemcpyAsync(&eff, n_runs, 4, cudaMemcpyDeviceToHost, stream));
-    B200_CUDA_TRY(cudaStreamSynchronize(stream));
-
-    B200_CUDA_TRY(tmp.alloc(&tiles, (uint64_t)eff + 1));
-    B200_CUDA_TRY(tmp.alloc(&ubase, (uint64_t)eff + 1));
-    B200_CUDA_TRY(tmp.alloc(&win2eff, n_windows));
-    B200_CUDA_TRY(pool_alloc(&f->d_rowOffset, (uint64_t)eff + 1, stream));
-    B200_CUDA_TRY(pool_alloc(&f->d_rowIdx, eff, stream));
-    B200_CUDA_TRY(cudaMemsetAsync(tiles + eff, 0, 4, stream));
-    B200_CUDA_TRY(cudaMemsetAsync(counts + eff, 0, 4, stream));
-    window_tables_kernel<<<(eff + kBlock - 1) / kBlock, kBlock, 0, stream>>>(win_ids, counts, eff, RW, CW, tiles,
-                                                                             f->d_rowIdx, win2eff);
+    // 3. windows
+    const unsigned window_grid = (unsigned)(n_windows / kBlock + 1);
+    window_bounds_kernel<<<window_grid, kBlock, 0, stream>>>(ukeys, totals, (uint32_t)n_windows, col_bits, first);
+    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, scan_bytes, terms, before, (int64_t)n_windows + 1, stream));
+    window_tables_kernel<<<window_grid, kBlock, 0, stream>>>(first, before, (uint32_t)n_windows, RW, f->d_rowOffset, f->d_rowIdx, tile_of,
+                                                             totals);
     B200_CUDA_TRY(cudaGetLastError());
-    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, tiles, f->d_rowOffset, (int)(eff + 1), stream));
-    uint8_t *scan_tmp = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&scan_tmp, scan_bytes));
-    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, tiles, f->d_rowOffset, (int)(eff + 1), stream));
-    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, counts, ubase, (int)(eff + 1), stream));
-    uint32_t total_tiles = 0;
-    B200_CUDA_TRY(cudaMemcpyAsync(&total_tiles, f->d_rowOffset + eff, 4, cudaMemcpyDeviceToHost, stream));
+    Totals h;
+    B200_CUDA_TRY(cudaMemcpyAsync(&h, totals, sizeof(h), cudaMemcpyDeviceToHost, stream));
     B200_CUDA_TRY(cudaStreamSynchronize(stream));
-    // (a tile count beyond 32 bits would have wrapped in the scan: bound it by the entry count instead)
-    if ((uint64_t)n_unique / CW + eff > 0xFFFFFFFFull) return B200SPMM_ERR_UNSUPPORTED;
-
+    if (h.bad) return B200SPMM_ERR_BAD_CSR;
+    const uint64_t n_unique = h.n_unique;
+    const uint32_t eff = (uint32_t)(h.windows_tiles >> 32), total_tiles = (uint32_t)h.windows_tiles;
     f->info.eff_row_windows = eff;
     f->info.total_tiles = total_tiles;
+
+    // 4. column lists and values
     const uint64_t list_len = (uint64_t)total_tiles * CW, data_len = (uint64_t)total_tiles * RW * CW;
     B200_CUDA_TRY(pool_alloc(&f->d_tcA2B, list_len, stream));
     B200_CUDA_TRY(pool_alloc_bytes(&f->d_data, std::max<uint64_t>(data_len * esz, 16), stream));
     B200_CUDA_TRY(cudaMemsetAsync(f->d_tcA2B, 0xFF, list_len * 4, stream));  // kIdxMax padding
     B200_CUDA_TRY(cudaMemsetAsync(f->d_data, 0, data_len * esz, stream));
-    scatter_columns_kernel<<<grid_for(n_unique), kBlock, 0, stream>>>(ukeys, n_unique, col_bits, win2eff, ubase, f->d_rowOffset, CW,
-                                                                      f->d_tcA2B);
+    scatter_columns_kernel<<<grid_for(n_unique), kBlock, 0, stream>>>(ukeys, n_unique, col_bits, first, tile_of, CW, f->d_tcA2B);
     B200_CUDA_TRY(cudaGetLastError());
-
-    // 4. values
     if (esz == 2)
         scatter_values_kernel<uint16_t><<<grid_for(nnz), kBlock, 0, stream>>>(
-            d_col_idx, static_cast<const uint16_t *>(d_values), row_of, nnz, win2eff, f->d_rowOffset, counts, f->d_tcA2B,
-            RW, CW, static_cast<uint16_t *>(f->d_data));
+            d_col_idx, static_cast<const uint16_t *>(d_values), row_of, nnz, first, tile_of, f->d_tcA2B, RW, CW,
+            static_cast<uint16_t *>(f->d_data));
     else
         scatter_values_kernel<uint32_t><<<grid_for(nnz), kBlock, 0, stream>>>(
-            d_col_idx, static_cast<const uint32_t *>(d_values), row_of, nnz, win2eff, f->d_rowOffset, counts, f->d_tcA2B,
-            RW, CW, static_cast<uint32_t *>(f->d_data));
+            d_col_idx, static_cast<const uint32_t *>(d_values), row_of, nnz, first, tile_of, f->d_tcA2B, RW, CW,
+            static_cast<uint32_t *>(f->d_data));
     B200_CUDA_TRY(cudaGetLastError());
     B200_CUDA_TRY(cudaStreamSynchronize(stream));
     return B200SPMM_OK;
@@ -291,14 +310,12 @@ int b200spmm_csr2btcf_nobitmap_device(uint64_t rows, uint64_t cols, uint64_t nnz
         ~Guard() { if (f) b200spmm_dbtcf_destroy(f); }
     } guard{f};
 
-    uint32_t head[2] = {0, 0};
-    {   // row_ptr must start at 0 and end at nnz
+    if (nnz == 0) {
+        uint32_t head[2] = {0, 0};  // (with entries make_keys_kernel looks at them)
         B200_CUDA_TRY(cudaMemcpyAsync(&head[0], d_row_ptr, 4, cudaMemcpyDeviceToHost, stream));
         B200_CUDA_TRY(cudaMemcpyAsync(&head[1], d_row_ptr + rows, 4, cudaMemcpyDeviceToHost, stream));
         B200_CUDA_TRY(cudaStreamSynchronize(stream));
-        if (head[0] != 0 || head[1] != nnz) return B200SPMM_ERR_BAD_CSR;
-    }
-    if (nnz == 0) {
+        if (head[0] != 0 || head[1] != 0) return B200SPMM_ERR_BAD_CSR;
         B200_CUDA_TRY(pool_alloc(&f->d_rowOffset, 4, stream));
         B200_CUDA_TRY(cudaMemsetAsync(f->d_rowOffset, 0, 16, stream));
         B200_CUDA_TRY(cudaStreamSynchronize(stream));

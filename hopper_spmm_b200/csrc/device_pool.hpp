@@ -38,19 +38,39 @@ constexpr int kUploadThreads = 4;
 constexpr size_t kUploadChunk = (size_t)2 << 20;
 cudaError_t upload_pageable(void *dst, const void *src, size_t bytes);
 
-// Buffers that are needed while an object is built, released on every exit path.
+// Buffers that are needed while an object is built, released on every exit path.  Small ones share blocks of
+// kBlockBytes: two dozen calls of the driver, each way, were a tenth of a small conversion.
 struct PoolScratch {
+    static constexpr size_t kBlockBytes = (size_t)8 << 20;
     cudaStream_t stream = nullptr;
     void *ptrs[24] = {};
     int n = 0;
+    char *block = nullptr;  // the current block's free part
+    size_t left = 0;
     explicit PoolScratch(cudaStream_t s = nullptr) : stream(s) {}
     PoolScratch(const PoolScratch &) = delete;
     template <typename T>
     cudaError_t alloc(T **out, size_t count) {
-        if (n == 24) return cudaErrorMemoryAllocation;
-        const cudaError_t e = pool_alloc(out, count, stream);
-        if (e == cudaSuccess) ptrs[n++] = *out;
-        return e;
+        const size_t bytes = (std::max<size_t>(count * sizeof(T), 16) + 255) & ~(size_t)255;
+        *out = nullptr;
+        const bool shared = bytes <= kBlockBytes / 2;
+        if (!shared || left < bytes) {
+            if (n == 24) return cudaErrorMemoryAllocation;
+            void *p = nullptr;
+            const cudaError_t e = pool_alloc_bytes(&p, shared ? kBlockBytes : bytes, stream);
+            if (e != cudaSuccess) return e;
+            ptrs[n++] = p;
+            if (!shared) {
+                *out = static_cast<T *>(p);
+                return e;
+            }
+            block = static_cast<char *>(p);
+            left = kBlockBytes;
+        }
+        *out = reinterpret_cast<T *>(block);
+        block += bytes;
+        left -= bytes;
+        return cudaSuccess;
     }
     ~PoolScratch() { for (int i = 0; i < n; ++i) pool_free(ptrs[i], stream); }
 };
