@@ -5,7 +5,11 @@
 // benchmark matrix (5.2e8 entries) takes ten seconds on sixteen host cores and well under one on
 // the device.
 //
-// Steps (all integer work, bound by HBM traffic):
+// A matrix whose windows are not too empty for it (see window_bits_pay) is converted window by window: a block marks
+// the window's columns in a bit set in shared memory and lists them in order; after one scan over the windows the lists
+// move to their places.  60,000 nodes, 700,000 entries: X us where the sort and what belongs to it took 90.
+//
+// Steps otherwise (all integer work, bound by HBM traffic):
 //   1. one key (window, column) per entry, in as few bits as the matrix needs - 32-bit keys where they fit - since
 //      every eight bits are a pass of the sort; the entry's row is found by binary search in row_ptr
 //   2. radix sort of the keys, then unique -> the sorted distinct columns of every window
@@ -57,13 +61,13 @@ struct Totals {
     uint32_t bad;
 };
 
-// keys[p] = window(p) << col_bits | col[p]; row_of[p]; flags row pointers that do not run from 0 to nnz, a column out
+// keys[p] = window(p) << col_bits | col[p]; flags row pointers that do not run from 0 to nnz, a column out
 // of range or a row whose columns are not strictly ascending.  Neighbouring entries lie in few rows: a block searches
 // the whole of row_ptr for its first and last entry only.
 template <typename K>
 __global__ void __launch_bounds__(kBlock)
 make_keys_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ col_idx, uint32_t rows, uint32_t cols, uint64_t nnz,
-                 uint32_t row_window, int col_bits, K *__restrict__ keys, uint32_t *__restrict__ row_of, Totals *__restrict__ totals) {
+                 uint32_t row_window, int col_bits, K *__restrict__ keys, Totals *__restrict__ totals) {
     __shared__ uint32_t range[2];
     if (blockIdx.x == 0 && threadIdx.x == 0 && (row_ptr[0] != 0 || row_ptr[rows] != nnz)) atomicOr(&totals->bad, 1u);
     for (uint64_t p0 = (uint64_t)blockIdx.x * kKeyEntries; p0 < nnz; p0 += (uint64_t)gridDim.x * kKeyEntries) {
@@ -76,7 +80,6 @@ make_keys_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restric
             const uint32_t r = row_of_entry(row_ptr, first, end, (uint32_t)p), c = col_idx[p], start = row_ptr[r];
             if (c >= cols || p < start || p >= row_ptr[r + 1] || (p > start && col_idx[p - 1] >= c)) atomicOr(&totals->bad, 1u);
             keys[p] = ((K)(r / row_window) << col_bits) | c;
-            row_of[p] = r;
         }
     }
 }
@@ -96,18 +99,136 @@ __global__ void window_bounds_kernel(const K *__restrict__ ukeys, const Totals *
     first[w] = lo;
 }
 
+constexpr int kBitsBlock = 256;
+constexpr size_t kBitsSmemMax = 100 * 1024;
+constexpr uint32_t kGroupWords = 8;  // words of the bit set that share a rank
+
+inline uint32_t bit_words(uint64_t cols) { return (uint32_t)((cols + 32 * kGroupWords - 1) / (32 * kGroupWords)) * kGroupWords; }
+inline size_t bits_smem(uint64_t cols) { return (size_t)bit_words(cols) * 4 + (size_t)(bit_words(cols) / kGroupWords) * 4; }
+
+// A pass over the bit set costs a window its words, four at a time, where the sort costs an entry four or more passes
+// of ~20 bytes each.  The two meet at some forty words an entry; the set has to leave room for two blocks an SM.
+inline bool window_bits_pay(uint64_t n_windows, uint64_t cols, uint64_t nnz) {
+    return bits_smem(cols) <= kBitsSmemMax && n_windows * bit_words(cols) <= 32 * nnz;
+}
+
+// The distinct columns of every window in order, at columns[first entry of the window ..], and how many they are.
+template <int kUnroll>
+__global__ void __launch_bounds__(kBitsBlock)
+window_columns_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ col_idx, uint32_t rows, uint32_t cols, uint32_t nnz,
+                      uint32_t row_window, uint32_t n_windows, uint32_t words, uint32_t *__restrict__ columns, uint32_t *__restrict__ count,
+                      Totals *__restrict__ totals) {
+    extern __shared__ __align__(16) uint32_t bits[];
+    __shared__ uint32_t start[32], sums[kBitsBlock / 32];
+    const uint32_t groups = words / kGroupWords, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t *rank = bits + words;  // columns in the groups before
+    if (blockIdx.x == 0 && threadIdx.x == 0 && (row_ptr[0] != 0 || row_ptr[rows] != nnz)) atomicOr(&totals->bad, 1u);
+    for (uint32_t w = blockIdx.x; w < n_windows; w += gridDim.x) {
+        bool ok = true;
+        if (threadIdx.x <= row_window) {
+            const uint64_t r = (uint64_t)w * row_window + threadIdx.x;
+            const uint32_t s = row_ptr[min(r, (uint64_t)rows)], prev = threadIdx.x ? row_ptr[min(r - 1, (uint64_t)rows)] : 0u;
+            start[threadIdx.x] = s;
+            ok = s <= nnz && prev <= s;
+        }
+        for (uint32_t k = threadIdx.x; k < words / 4; k += kBitsBlock) reinterpret_cast<uint4 *>(bits)[k] = make_uint4(0, 0, 0, 0);
+        ok = __syncthreads_and(ok);
+        const uint32_t p0 = start[0], p1 = start[row_window];
+        if (!ok || p0 == p1) {
+            if (threadIdx.x == 0) {
+                count[w] = 0;
+                if (!ok) atomicOr(&totals->bad, 1u);
+            }
+            __syncthreads();
+            continue;
+        }
+        for (uint32_t q = p0 + threadIdx.x; q < p1; q += kUnroll * kBitsBlock) {  // (no overflow: p1 <= 2^32 - 1 is checked by the host)
+            uint32_t c[kUnroll], left[kUnroll];
+#pragma unroll
+            for (int k = 0; k < kUnroll; ++k) {
+                const uint64_t p = (uint64_t)q + (uint32_t)k * kBitsBlock;
+                c[k] = p < p1 ? col_idx[p] : 0u;
+                left[k] = p < p1 && p > p0 ? col_idx[p - 1] : 0u;
+            }
+#pragma unroll
+            for (int k = 0; k < kUnroll; ++k) {
+                const uint64_t p = (uint64_t)q + (uint32_t)k * kBitsBlock;
+                if (p >= p1) break;
+                if (p > p0 && left[k] >= c[k]) {  // only where a row starts
+                    bool row_start = false;
+                    for (uint32_t r = 1; r < row_window; ++r) row_start |= start[r] == p;
+                    if (!row_start) atomicOr(&totals->bad, 1u);
+                }
+                if (c[k] < cols) atomicOr(bits + (c[k] >> 5), 1u << (c[k] & 31u));
+                else atomicOr(&totals->bad, 1u);
+            }
+            if (p1 - q <= kUnroll * kBitsBlock) break;
+        }
+        __syncthreads();
+        uint32_t base = 0;
+        for (uint32_t g0 = 0; g0 < groups; g0 += kBitsBlock) {  // one group a thread
+            const uint32_t g = g0 + threadIdx.x;
+            uint32_t mine = 0;
+            if (g < groups)
+#pragma unroll
+                for (uint32_t k = 0; k < kGroupWords; ++k) mine += __popc(bits[g * kGroupWords + k]);
+            uint32_t upto = mine;
+#pragma unroll
+            for (int d = 1; d < 32; d *= 2) {
+                const uint32_t x = __shfl_up_sync(0xffffffffu, upto, d);
+                if (lane >= (uint32_t)d) upto += x;
+            }
+            __syncthreads();  // `sums` of the round before has been read
+            if (lane == 31) sums[warp] = upto;
+            __syncthreads();
+            uint32_t before = base;
+            for (uint32_t k = 0; k < kBitsBlock / 32; ++k) {
+                if (k < warp) before += sums[k];
+                base += sums[k];
+            }
+            if (g < groups) rank[g] = before + upto - mine;
+        }
+        __syncthreads();
+        for (uint32_t k = threadIdx.x; k < words; k += kBitsBlock) {
+            uint32_t b = bits[k];
+            if (!b) continue;
+            uint32_t at = p0 + rank[k / kGroupWords];
+            for (uint32_t j = k / kGroupWords * kGroupWords; j < k; ++j) at += __popc(bits[j]);
+            for (; b; b &= b - 1u) columns[at++] = k * 32u + (uint32_t)__ffs((int)b) - 1u;
+        }
+        if (threadIdx.x == 0) count[w] = base;
+        __syncthreads();  // the next window clears the set
+    }
+}
+
+// The lists at their places, padded to whole tiles.
+__global__ void __launch_bounds__(kBitsBlock)
+place_columns_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ columns, const uint32_t *__restrict__ count,
+                     const uint32_t *__restrict__ tile_of, uint32_t n_windows, uint32_t row_window, uint32_t col_window,
+                     uint32_t *__restrict__ tcA2B) {
+    for (uint32_t w = blockIdx.x; w < n_windows; w += gridDim.x) {
+        const uint32_t n = count[w], padded = (n + col_window - 1) / col_window * col_window;
+        if (!n) continue;
+        const uint32_t *from = columns + row_ptr[w * row_window];
+        uint32_t *list = tcA2B + (uint64_t)tile_of[w] * col_window;
+#pragma unroll 4
+        for (uint32_t k = threadIdx.x; k < padded; k += kBitsBlock) list[k] = k < n ? from[k] : 0xFFFFFFFFu;
+    }
+}
+
 // The window's terms of the scan.  Fewer than 2^32 entries make fewer than 2^30 full tiles, 2^29 windows as many more.
 struct WindowTerms {
-    const uint32_t *first;
+    const uint32_t *first, *count;  // one of the two
     uint32_t n_windows, col_window;
+    __host__ __device__ uint32_t columns_of(uint32_t w) const { return count ? count[w] : first[w + 1] - first[w]; }
     __host__ __device__ unsigned long long operator()(uint32_t w) const {
         if (w >= n_windows) return 0;
-        const uint32_t n = first[w + 1] - first[w];
+        const uint32_t n = columns_of(w);
         return (unsigned long long)(n != 0) << 32 | ((unsigned long long)n + col_window - 1) / col_window;
     }
 };
 
-__global__ void window_tables_kernel(const uint32_t *__restrict__ first, const unsigned long long *__restrict__ before, uint32_t n_windows,
+__global__ void window_tables_kernel(const unsigned long long *__restrict__ before, uint32_t n_windows,
                                      uint32_t row_window, uint32_t *__restrict__ rowOffset, uint32_t *__restrict__ rowIdx,
                                      uint32_t *__restrict__ tile_of, Totals *__restrict__ totals) {
     const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
@@ -119,7 +240,7 @@ __global__ void window_tables_kernel(const uint32_t *__restrict__ first, const u
         return;
     }
     tile_of[w] = tile;
-    if (first[w + 1] == first[w]) return;
+    if ((uint32_t)(before[w + 1] >> 32) == e) return;
     rowOffset[e] = tile;
     rowIdx[e] = w * row_window;
 }
@@ -137,24 +258,96 @@ __global__ void scatter_columns_kernel(const K *__restrict__ ukeys, uint64_t n_u
 
 // entry p -> its slot in the zero-filled tile array
 template <typename T>
-__global__ void scatter_values_kernel(const uint32_t *__restrict__ col_idx, const T *__restrict__ values,
-                                      const uint32_t *__restrict__ row_of, uint64_t nnz, const uint32_t *__restrict__ first,
-                                      const uint32_t *__restrict__ tile_of, const uint32_t *__restrict__ tcA2B, uint32_t row_window,
-                                      uint32_t col_window, T *__restrict__ data) {
-    for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t r = row_of[p], c = col_idx[p], w = r / row_window, tile0 = tile_of[w];
-        const uint32_t *list = tcA2B + (uint64_t)tile0 * col_window;
-        uint32_t lo = 0, hi = first[w + 1] - first[w];  // the window's real columns are ascending; padding follows them
-        while (lo < hi) {
-            const uint32_t mid = lo + (hi - lo) / 2;
-            if (list[mid] < c) lo = mid + 1; else hi = mid;
+__global__ void __launch_bounds__(kBlock)
+scatter_values_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ col_idx, const T *__restrict__ values, uint32_t rows,
+                      uint64_t nnz, WindowTerms windows, const uint32_t *__restrict__ tile_of, const uint32_t *__restrict__ tcA2B,
+                      uint32_t row_window, uint32_t col_window, T *__restrict__ data) {
+    __shared__ uint32_t range[2];
+    for (uint64_t p0 = (uint64_t)blockIdx.x * kKeyEntries; p0 < nnz; p0 += (uint64_t)gridDim.x * kKeyEntries) {
+        const uint64_t p1 = min(p0 + kKeyEntries, nnz);
+        __syncthreads();
+        if (threadIdx.x < 2) range[threadIdx.x] = row_of_entry(row_ptr, 0, rows, (uint32_t)(threadIdx.x ? p1 - 1 : p0));
+        __syncthreads();
+        const uint32_t first = range[0], end = range[1] + 1;
+        for (uint64_t p = p0 + threadIdx.x; p < p1; p += kBlock) {
+            const uint32_t r = row_of_entry(row_ptr, first, end, (uint32_t)p), c = col_idx[p], w = r / row_window, tile0 = tile_of[w];
+            const uint32_t *list = tcA2B + (uint64_t)tile0 * col_window;
+            uint32_t lo = 0, hi = windows.columns_of(w);  // the window's real columns are ascending; padding follows them
+            while (lo < hi) {
+                const uint32_t mid = lo + (hi - lo) / 2;
+                if (list[mid] < c) lo = mid + 1; else hi = mid;
+            }
+            const uint64_t tile = (uint64_t)tile0 + lo / col_window;
+            data[tile * row_window * col_window + (uint64_t)(r % row_window) * col_window + lo % col_window] = values[p];
         }
-        const uint64_t tile = (uint64_t)tile0 + lo / col_window;
-        data[tile * row_window * col_window + (uint64_t)(r % row_window) * col_window + lo % col_window] = values[p];
     }
 }
 
 inline int grid_for(uint64_t n) { return (int)std::min<uint64_t>((n + kBlock - 1) / kBlock, 148 * 32); }
+
+void scatter_values(const b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const uint32_t *d_col_idx, const void *d_values,
+                    const WindowTerms &windows, const uint32_t *tile_of, cudaStream_t stream) {
+    const auto &i = f->info;
+    const int grid = (int)std::min<uint64_t>((i.nnzs + kKeyEntries - 1) / kKeyEntries, 148 * 32);
+    if (i.elt_size == 2)
+        scatter_values_kernel<uint16_t><<<grid, kBlock, 0, stream>>>(d_row_ptr, d_col_idx, static_cast<const uint16_t *>(d_values),
+                                                                     (uint32_t)i.rows, i.nnzs, windows, tile_of, f->d_tcA2B,
+                                                                     (uint32_t)i.row_window, (uint32_t)i.col_window, static_cast<uint16_t *>(f->d_data));
+    else
+        scatter_values_kernel<uint32_t><<<grid, kBlock, 0, stream>>>(d_row_ptr, d_col_idx, static_cast<const uint32_t *>(d_values),
+                                                                     (uint32_t)i.rows, i.nnzs, windows, tile_of, f->d_tcA2B,
+                                                                     (uint32_t)i.row_window, (uint32_t)i.col_window, static_cast<uint32_t *>(f->d_data));
+}
+
+int convert_by_windows(b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const uint32_t *d_col_idx, const void *d_values, cudaStream_t stream) {
+    const uint32_t rows = (uint32_t)f->info.rows, cols = (uint32_t)f->info.cols, nnz = (uint32_t)f->info.nnzs;
+    const uint32_t n_windows = (uint32_t)f->info.total_row_windows, RW = (uint32_t)f->info.row_window, CW = (uint32_t)f->info.col_window;
+    const uint32_t words = bit_words(f->info.cols);
+    const size_t smem = bits_smem(f->info.cols);
+    const int esz = f->info.elt_size;
+    PoolScratch tmp(stream);
+    Totals *totals = nullptr;
+    uint32_t *columns = nullptr, *count = nullptr, *tile_of = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&columns, nnz));
+    unsigned long long *before = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&totals, 1));
+    B200_CUDA_TRY(tmp.alloc(&count, n_windows));
+    B200_CUDA_TRY(tmp.alloc(&tile_of, n_windows));
+    B200_CUDA_TRY(tmp.alloc(&before, (size_t)n_windows + 1));
+    const WindowTerms windows{nullptr, count, n_windows, CW};
+    auto terms = thrust::make_transform_iterator(thrust::make_counting_iterator<uint32_t>(0), windows);
+    size_t scan_bytes = 0;
+    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, terms, before, (int64_t)n_windows + 1, stream));
+    uint8_t *scan_tmp = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&scan_tmp, scan_bytes));
+    B200_CUDA_TRY(pool_alloc(&f->d_rowOffset, (size_t)n_windows + 1, stream));
+    B200_CUDA_TRY(pool_alloc(&f->d_rowIdx, n_windows, stream));
+    if (smem > 48 * 1024)
+        B200_CUDA_TRY(cudaFuncSetAttribute(window_columns_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBitsSmemMax));
+    const unsigned grid = std::min<uint32_t>(n_windows, 148 * 64), table_grid = n_windows / kBlock + 1;
+    B200_CUDA_TRY(cudaMemsetAsync(totals, 0, sizeof(Totals), stream));
+    window_columns_kernel<8><<<grid, kBitsBlock, smem, stream>>>(d_row_ptr, d_col_idx, rows, cols, nnz, RW, n_windows, words, columns, count,
+                                                                 totals);
+    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, terms, before, (int64_t)n_windows + 1, stream));
+    window_tables_kernel<<<table_grid, kBlock, 0, stream>>>(before, n_windows, RW, f->d_rowOffset, f->d_rowIdx, tile_of, totals);
+    B200_CUDA_TRY(cudaGetLastError());
+    Totals h;
+    B200_CUDA_TRY(cudaMemcpyAsync(&h, totals, sizeof(h), cudaMemcpyDeviceToHost, stream));
+    B200_CUDA_TRY(cudaStreamSynchronize(stream));
+    if (h.bad) return B200SPMM_ERR_BAD_CSR;
+    f->info.eff_row_windows = h.windows_tiles >> 32;
+    f->info.total_tiles = (uint32_t)h.windows_tiles;
+    const uint64_t data_bytes = f->info.total_tiles * RW * CW * esz;
+    B200_CUDA_TRY(pool_alloc(&f->d_tcA2B, f->info.total_tiles * CW, stream));
+    B200_CUDA_TRY(pool_alloc_bytes(&f->d_data, std::max<uint64_t>(data_bytes, 16), stream));
+    B200_CUDA_TRY(cudaMemsetAsync(f->d_data, 0, data_bytes, stream));
+    place_columns_kernel<<<grid, kBitsBlock, 0, stream>>>(d_row_ptr, columns, count, tile_of, n_windows, RW, CW, f->d_tcA2B);
+    scatter_values(f, d_row_ptr, d_col_idx, d_values, windows, tile_of, stream);
+    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(cudaStreamSynchronize(stream));
+    return B200SPMM_OK;
+}
 
 // Steps 1 - 4, with keys of key_bits bits (col_bits of them the column).
 template <typename K>
@@ -166,17 +359,17 @@ int convert_on_device(b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const uint32
     PoolScratch tmp(stream);
     K *keys = nullptr, *keys_sorted = nullptr, *ukeys = nullptr;
     Totals *totals = nullptr;
-    uint32_t *row_of = nullptr, *first = nullptr, *tile_of = nullptr;
+    uint32_t *first = nullptr, *tile_of = nullptr;
     unsigned long long *before = nullptr;
     B200_CUDA_TRY(tmp.alloc(&keys, nnz));
     B200_CUDA_TRY(tmp.alloc(&keys_sorted, nnz));
-    B200_CUDA_TRY(tmp.alloc(&row_of, nnz));
     B200_CUDA_TRY(tmp.alloc(&totals, 1));
     B200_CUDA_TRY(tmp.alloc(&first, n_windows + 1));
     B200_CUDA_TRY(tmp.alloc(&tile_of, n_windows));
     B200_CUDA_TRY(tmp.alloc(&before, n_windows + 1));
     ukeys = keys;  // the unsorted keys are dead once sorted: reuse their buffer for the distinct keys
-    auto terms = thrust::make_transform_iterator(thrust::make_counting_iterator<uint32_t>(0), WindowTerms{first, (uint32_t)n_windows, CW});
+    const WindowTerms windows{first, nullptr, (uint32_t)n_windows, CW};
+    auto terms = thrust::make_transform_iterator(thrust::make_counting_iterator<uint32_t>(0), windows);
     size_t sort_bytes = 0, sel_bytes = 0, scan_bytes = 0;
     B200_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, keys, keys_sorted, (int64_t)nnz, 0, key_bits, stream));
     B200_CUDA_TRY(cub::DeviceSelect::Unique(nullptr, sel_bytes, keys_sorted, ukeys, &totals->n_unique, (int64_t)nnz, stream));
@@ -189,7 +382,7 @@ int convert_on_device(b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const uint32
     // 1. keys
     B200_CUDA_TRY(cudaMemsetAsync(totals, 0, sizeof(Totals), stream));
     const int key_grid = (int)std::min<uint64_t>((nnz + kKeyEntries - 1) / kKeyEntries, 148 * 8);
-    make_keys_kernel<<<key_grid, kBlock, 0, stream>>>(d_row_ptr, d_col_idx, (uint32_t)rows, (uint32_t)cols, nnz, RW, col_bits, keys, row_of,
+    make_keys_kernel<<<key_grid, kBlock, 0, stream>>>(d_row_ptr, d_col_idx, (uint32_t)rows, (uint32_t)cols, nnz, RW, col_bits, keys,
                                                       totals);
     B200_CUDA_TRY(cudaGetLastError());
 
@@ -201,7 +394,7 @@ int convert_on_device(b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const uint32
     const unsigned window_grid = (unsigned)(n_windows / kBlock + 1);
     window_bounds_kernel<<<window_grid, kBlock, 0, stream>>>(ukeys, totals, (uint32_t)n_windows, col_bits, first);
     B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, scan_bytes, terms, before, (int64_t)n_windows + 1, stream));
-    window_tables_kernel<<<window_grid, kBlock, 0, stream>>>(first, before, (uint32_t)n_windows, RW, f->d_rowOffset, f->d_rowIdx, tile_of,
+    window_tables_kernel<<<window_grid, kBlock, 0, stream>>>(before, (uint32_t)n_windows, RW, f->d_rowOffset, f->d_rowIdx, tile_of,
                                                              totals);
     B200_CUDA_TRY(cudaGetLastError());
     Totals h;
@@ -221,14 +414,7 @@ int convert_on_device(b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const uint32
     B200_CUDA_TRY(cudaMemsetAsync(f->d_data, 0, data_len * esz, stream));
     scatter_columns_kernel<<<grid_for(n_unique), kBlock, 0, stream>>>(ukeys, n_unique, col_bits, first, tile_of, CW, f->d_tcA2B);
     B200_CUDA_TRY(cudaGetLastError());
-    if (esz == 2)
-        scatter_values_kernel<uint16_t><<<grid_for(nnz), kBlock, 0, stream>>>(
-            d_col_idx, static_cast<const uint16_t *>(d_values), row_of, nnz, first, tile_of, f->d_tcA2B, RW, CW,
-            static_cast<uint16_t *>(f->d_data));
-    else
-        scatter_values_kernel<uint32_t><<<grid_for(nnz), kBlock, 0, stream>>>(
-            d_col_idx, static_cast<const uint32_t *>(d_values), row_of, nnz, first, tile_of, f->d_tcA2B, RW, CW,
-            static_cast<uint32_t *>(f->d_data));
+    scatter_values(f, d_row_ptr, d_col_idx, d_values, windows, tile_of, stream);
     B200_CUDA_TRY(cudaGetLastError());
     B200_CUDA_TRY(cudaStreamSynchronize(stream));
     return B200SPMM_OK;
@@ -324,6 +510,13 @@ int b200spmm_csr2btcf_nobitmap_device(uint64_t rows, uint64_t cols, uint64_t nnz
         return B200SPMM_OK;
     }
 
+    if (window_bits_pay(n_windows, cols, nnz)) {
+        const int st = convert_by_windows(f, d_row_ptr, d_col_idx, d_values, stream);
+        if (st != B200SPMM_OK) return st;
+        guard.f = nullptr;
+        *out = f;
+        return B200SPMM_OK;
+    }
     int win_bits = 1, col_bits = 1;
     while ((1ull << win_bits) < n_windows) ++win_bits;
     while ((1ull << col_bits) < cols) ++col_bits;

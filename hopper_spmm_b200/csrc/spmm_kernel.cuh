@@ -30,7 +30,7 @@
 //              warp of the group brings the stage's eight 512-byte A tiles with one TMA load; every
 //              half-warp fetches the CW rows of B its tile selects with TMA tile::gather4 (four rows
 //              per instruction, one instruction per lane, landing in the swizzled operand layout;
-//              a cp.async variant exists for comparison and for very narrow B).  Column lists are
+//              a cp.async variant exists for comparison).  Column lists are
 //              fetched a few iterations ahead into a per-warp ring.  Two tiles per warp and
 //              iteration halve the producers' instructions per tile; eight tiles per stage halve
 //              the barrier round trips of the MMA issuer.

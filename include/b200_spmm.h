@@ -435,8 +435,8 @@ int b200spmm_spmm_noalloc_status(int device, void *stream);
  * converter's algorithm (src/utils/convert.h:146-225) at ROW_WINDOW = 128 - and multiplies it with a
  * kernel whose MMA is 128 window rows x 128/256 features instead of 128 features x 16 rows.  The choice
  * is made when the plan is created (the merge must leave fewer than ~0.7 of the tiles, estimated on a
- * sample of windows; B200SPMM_WINDOW=16 or =128 in the environment overrides it) and per launch (B at
- * least 128 bytes wide, enough windows x feature slabs to occupy every SM).  The format handed to
+ * sample of windows; B200SPMM_WINDOW=16 or =128 in the environment overrides it) and per launch (the
+ * expected time: rounds of windows x feature slabs against 16-row tiles spread evenly).  The format handed to
  * callers is unchanged.  b200spmm_plan_tall_info reports the merged format (row_window 128, or 0 when
  * the plan has none); b200spmm_plan_tall_copy_to_host copies its four arrays out (buffers sized from
  * that info) so that it can be compared with a conversion at 128 rows.  No counterpart in the
@@ -467,7 +467,8 @@ typedef struct {
     int32_t tma_gather;      /* 1: rows of B fetched by TMA tile::gather4, 0: by cp.async copies */
     int32_t bitmap_tiles;    /* 0: dense tiles; 1: tiles streamed as bitmap + stored values and expanded in the kernel;
                                 2: tiles streamed as records of 32 (position, value) words (B200SPMM_TILES=entries) */
-    int32_t row_window;      /* rows per window the launched kernel consumed: 16, or 128 (super-windows) */
+    int32_t row_window;      /* rows per window the launched kernel consumed: 16, or 128 / 256 (super-windows); 16 and
+                                stages == 0 for the kernels that read entries instead of tiles (row units, narrow B) */
 } b200spmm_launch_info_t;
 int b200spmm_plan_launch_info(const b200spmm_plan_t *p, b200spmm_launch_info_t *info);
 

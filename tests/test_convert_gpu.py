@@ -71,3 +71,32 @@ def test_product_from_a_matrix_that_stayed_on_the_gpu():
     rp, ci, v = csr.numpy()
     parity.check(C_dev.cpu().numpy(), csr.rows, rp, ci, v, B.cpu().numpy())
     plan.close()
+
+
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+@pytest.mark.parametrize("rows,cols,per_row", [(50, 255, 40), (50, 256, 40), (50, 257, 40), (33, 66000, 900), (40, 520001, 3000),
+                                               (3001, 300000, 3), (700, 900001, 2000)])
+def test_window_by_window_and_through_the_sort(dt, rows, cols, per_row):
+    # a bit set of one group, its edges, several groups a thread, a set above 48 KB; windows too empty for a set and
+    # rows too long for one.  Rows of very different length, empty ones in between
+    rng = np.random.default_rng(cols)
+    lengths = np.minimum(rng.integers(0, 2 * per_row + 1, rows), cols)
+    lengths[rows // 2] = min(cols, 40 * per_row)
+    ci = np.concatenate([np.sort(rng.choice(cols, k, replace=False)) for k in lengths]).astype(np.uint32)
+    rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.uint32)
+    v = rng.uniform(0.5, 1, ci.size).astype(np.float32).astype(dt)
+    dev = device_convert(rows, cols, rp, ci, v)
+    assert_same(dev, hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    dev.close()
+    bad = []
+    for at in (rp[rows // 2], rp[rows // 2] + 1):  # a column out of range, two columns out of order
+        c = ci.copy()
+        c[at] = cols if at == rp[rows // 2] else c[at - 1]
+        bad.append((rp, c))
+    r = rp.copy()
+    r[rows // 2] += 1 + r[rows // 2 + 1] - r[rows // 2]  # row pointers that fall
+    bad += [(r, ci), (np.concatenate([rp[:-1], [rp[-1] - 1]]).astype(np.uint32), ci), (np.concatenate([[1], rp[1:]]).astype(np.uint32), ci)]
+    for r, c in bad:
+        with pytest.raises(capi.SpmmError) as e:
+            device_convert(rows, cols, r, c, v)
+        assert e.value.status == capi.ERR_BAD_CSR
