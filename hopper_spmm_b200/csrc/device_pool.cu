@@ -5,6 +5,7 @@
 #include <cstring>
 #include <mutex>
 #include <thread>
+#include <unordered_set>
 #include <vector>
 
 #include "../../include/b200_spmm.h"
@@ -39,6 +40,9 @@ cudaError_t pool_of(int device, cudaMemPool_t *out) {
     *out = g_pool[device];
     return cudaSuccess;
 }
+
+std::mutex g_large_lock;
+std::unordered_set<void *> g_large;  // buffers of kPoolMaxBytes and more
 
 std::mutex g_staging_lock;
 void *g_staging = nullptr;  // [kUploadThreads][2][kUploadChunk] pinned bytes
@@ -99,18 +103,30 @@ cudaError_t pool_alloc_bytes(void **out, size_t bytes, cudaStream_t stream) {
     cudaMemPool_t pool = nullptr;
     if (e == cudaSuccess) e = pool_of(device, &pool);
     if (e != cudaSuccess) return e;
-    e = cudaMallocFromPoolAsync(out, bytes, pool, stream);
+    auto allocate = [&]() { return bytes >= kPoolMaxBytes ? cudaMalloc(out, bytes) : cudaMallocFromPoolAsync(out, bytes, pool, stream); };
+    e = allocate();
     if (e == cudaErrorMemoryAllocation) {  // what was freed may still be waiting for its stream, or be kept
         cudaGetLastError();
         cudaDeviceSynchronize();
         cudaMemPoolTrimTo(pool, 0);
-        e = cudaMallocFromPoolAsync(out, bytes, pool, stream);
+        e = allocate();
+    }
+    if (e == cudaSuccess && bytes >= kPoolMaxBytes) {
+        std::lock_guard<std::mutex> guard(g_large_lock);
+        g_large.insert(*out);
     }
     return e;
 }
 
 void pool_free(void *ptr, cudaStream_t stream) {
-    if (ptr) cudaFreeAsync(ptr, stream);
+    if (!ptr) return;
+    bool large;
+    {
+        std::lock_guard<std::mutex> guard(g_large_lock);
+        large = g_large.erase(ptr) != 0;
+    }
+    if (large) cudaFree(ptr);  // (waits for the device)
+    else cudaFreeAsync(ptr, stream);
 }
 
 cudaError_t pool_release(int device) {
