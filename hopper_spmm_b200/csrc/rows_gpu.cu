@@ -47,12 +47,27 @@ __global__ void run_windows_kernel(const uint32_t *__restrict__ run_first, uint3
     for (uint32_t r = run_first[w]; r < run_first[w + 1]; ++r) run_window[r] = w;
 }
 
+// a[k] of registers, by halves: two predicates less a register than comparing k with every index
+template <int kN>
+__device__ __forceinline__ uint32_t pick(const uint32_t (&a)[kN], int k) {
+    const uint32_t lo = (k & 2) ? ((k & 1) ? a[3] : a[2]) : ((k & 1) ? a[1] : a[0]);
+    if (kN == 4) return lo;
+    const uint32_t hi = (k & 2) ? ((k & 1) ? a[kN - 1] : a[kN - 2]) : ((k & 1) ? a[kN - 3] : a[kN - 4]);
+    return (k & 4) ? hi : lo;
+}
+
 // The lane's share of a tile: row lane / 2, its left or right half of the columns.
 template <typename T>
 struct Piece {
     static constexpr int kPer = 16 / (int)sizeof(T);
-    T v[kPer];
+    alignas(16) T v[kPer];
     uint32_t mask;
+    __device__ __forceinline__ T pick(int k) const {  // v[k]
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(v);
+        const int i = sizeof(T) == 2 ? k >> 1 : k;
+        const uint32_t word = (i & 2) ? ((i & 1) ? w[3] : w[2]) : ((i & 1) ? w[1] : w[0]);
+        return sizeof(T) == 2 ? (T)(word >> ((k & 1) * 16)) : (T)word;
+    }
     __device__ __forceinline__ void load(const T *__restrict__ data, uint64_t tile, uint32_t lane) {
         *reinterpret_cast<uint4 *>(v) = __ldcs(reinterpret_cast<const uint4 *>(data + tile * (32 * kPer) + lane * kPer));
         mask = 0;
@@ -255,13 +270,8 @@ write_entries_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__r
             at += mine + other;
             for (uint32_t m = p.mask; m; m &= m - 1u) {  // (two or three steps a warp; one per column would be eight)
                 const int k = __ffs((int)m) - 1;
-                uint32_t col = cols[0];
-                T v = p.v[0];
-#pragma unroll
-                for (int j = 1; j < kPer; ++j) {
-                    col = k == j ? cols[j] : col;
-                    v = k == j ? p.v[j] : v;
-                }
+                const uint32_t col = pick(cols, k);
+                const T v = p.pick(k);
                 if (k_out >= piece_end) {
                     piece = k_out / cap;
                     piece_end = (piece + 1) * cap;
