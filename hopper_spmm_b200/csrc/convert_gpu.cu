@@ -7,7 +7,8 @@
 //
 // A matrix whose windows are not too empty for it (see window_bits_pay) is converted window by window: a block marks
 // the window's columns in a bit set in shared memory and lists them in order; after one scan over the windows the lists
-// move to their places.  60,000 nodes, 700,000 entries: X us where the sort and what belongs to it took 90.
+// move to their places.  60,000 nodes, 700,000 entries: 67 us with the values, where the sort took 101.  A block of 512 or 1024
+// threads is slower (conversion 140 us a call with 256, 164 with 512): most windows have a few hundred entries.
 //
 // Steps otherwise (all integer work, bound by HBM traffic):
 //   1. one key (window, column) per entry, in as few bits as the matrix needs - 32-bit keys where they fit - since
@@ -107,9 +108,10 @@ inline uint32_t bit_words(uint64_t cols) { return (uint32_t)((cols + 32 * kGroup
 inline size_t bits_smem(uint64_t cols) { return (size_t)bit_words(cols) * 4 + (size_t)(bit_words(cols) / kGroupWords) * 4; }
 
 // A pass over the bit set costs a window its words, four at a time, where the sort costs an entry four or more passes
-// of ~20 bytes each.  The two meet at some forty words an entry; the set has to leave room for two blocks an SM.
+// of ~20 bytes each.  Conversion of graphs in us, sets against sort, at words of the sets per entry: 133 / 212 at 10,
+// 151 / 218 at 23, 3,930 / 5,208 at 36, 272 / 268 at 58, 705 / 490 at 90.  The set has to leave room for two blocks an SM.
 inline bool window_bits_pay(uint64_t n_windows, uint64_t cols, uint64_t nnz) {
-    return bits_smem(cols) <= kBitsSmemMax && n_windows * bit_words(cols) <= 32 * nnz;
+    return bits_smem(cols) <= kBitsSmemMax && n_windows * bit_words(cols) <= 40 * nnz;
 }
 
 // The distinct columns of every window in order, at columns[first entry of the window ..], and how many they are.

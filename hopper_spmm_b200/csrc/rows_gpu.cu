@@ -242,7 +242,7 @@ write_entries_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__r
         uint32_t at = counts[(uint64_t)run * 16 + (lane >> 1)];  // entries of the row so far
         // Everything a lane reads comes ahead of its stores and for all lanes at once - the unit it starts in, a tile's
         // columns and values while the tile before is written: fetched at its first entry, one by one, they cost the warp
-        // a round trip to L2 per entry (43 us of a matrix of 700,000 entries, 60,000 rows; now 34).
+        // a round trip to L2 per entry (43 us of a matrix of 700,000 entries, 60,000 rows; now 32).
         uint32_t piece = min(at / cap, pieces_of(len, cap) - 1u), piece_end = (piece + 1) * cap;
         uint32_t *out = batches + (uint64_t)unit[piece] * kWords;
         auto put = [&](uint32_t e, uint32_t col, T v) {
