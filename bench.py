@@ -336,8 +336,8 @@ def run_other_workload(name, dev, steps, warmup, hbm_gbs, f16_tflops, tf32_tflop
            "graph_replay_ms": graph_replay_ms(plan, B, C_dev, steps) if ms_hot < 0.2 else None}
     # executed MMA work: every tile of the kernel that ran is a dense (window rows x CW) block times all features
     win = rec["kernel"]["row_window"]
-    if win == 16:
-        ex_tiles = int(btcf.total_tiles)
+    if win == 16:  # (row units and narrow B read entries, not tiles: stages == 0)
+        ex_tiles = int(btcf.total_tiles) if info.stages else 0
     else:
         lib = capi_mod().lib()
         tinfo = capi_mod().BtcfInfo()
@@ -610,8 +610,9 @@ def main():
     roofline = roofline_record(nnz_local, rows_local, cols, n_feat, esz, kernel_ms, hbm_gbs,
                                f16_tflops if dtype_name == "f16" else tf32_tflops, peak_kind,
                                "" if dtype_name == "f16" else "tf32 matmul measured in this run")
-    roofline["kernel"] = "spmm_sm100_kernel"
-    roofline["traffic"] = dram_traffic(args.workload, tiles_local, info.n_slabs)
+    by_tiles = info.stages != 0  # else row units; their DRAM traffic was not captured at full size
+    roofline["kernel"] = "spmm_sm100_kernel" if by_tiles else "spmm_rows_kernel"
+    roofline["traffic"] = dram_traffic(args.workload, tiles_local, info.n_slabs) if by_tiles else None
     # whole job: every rank's A and C bytes once, B once (it is replicated, not re-read by the algorithm),
     # against N GPUs' bandwidth
     alg_job = algorithmic_bytes(total_nnz, total_rows, cols, n_feat, esz, esz, 4)
@@ -667,7 +668,7 @@ def main():
         details = dict(tiles_rank0=int(tiles_local), fill_rank0=fill, n_ctas=info.n_ctas, feature_slab=info.feature_slab,
                        stages=info.stages, convert_s_rank0=t_conv, rank_ms=[round(x, 4) for x in rank_ms],
                        # what the tensor cores execute: every tile is a dense 16 x CW x n product
-                       executed_mma_gflop_rank0=2.0 * tiles_local * 16 * btcf.col_window * n_feat / 1e9,
+                       executed_mma_gflop_rank0=2.0 * tiles_local * 16 * btcf.col_window * n_feat / 1e9 if info.stages else 0.0,
                        graph_replay_ms_per_step=graph_ms, allgather_c_ms=allgather_ms, allgather_c_bytes=allgather_bytes,
                        tf32_tflops_measured=tf32_tflops, host_cores=host_cores())
         line = {"metric": "SpMM effective GFLOP/s (2*nnz*N)", "value": value, "unit": "GFLOP/s", "n_gpus": world,
