@@ -6,6 +6,7 @@
 
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/b200_spmm.h"
@@ -18,7 +19,10 @@ PyObject *refuse(const char *what) {
 }
 
 // spmm(plan, is_f16, rows, cols, B, C or None, c_half, stream or None) -> C, or a status code that is not 0
+// Any tensor accessor may throw: a sparse tensor has no strides, a tensor subclass may answer for sizes and strides in
+// Python.  The macros turn whatever comes (a Python error among it) into the exception the caller sees.
 PyObject *spmm(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
+    HANDLE_TH_ERRORS
     if (n_args != 8) {
         PyErr_SetString(PyExc_TypeError, "spmm takes 8 arguments");
         return nullptr;
@@ -47,13 +51,8 @@ PyObject *spmm(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
         stream = PyLong_AsVoidPtr(args[7]);
         if (PyErr_Occurred()) return nullptr;
     }
-    try {
-        if (args[5] == Py_None) C = at::empty({rows, n}, B.options().dtype(c_type).requires_grad(false));
-        if (args[7] == Py_None) stream = c10::cuda::getCurrentCUDAStream(B.get_device()).stream();
-    } catch (const std::exception &e) {
-        PyErr_SetString(PyExc_RuntimeError, e.what());
-        return nullptr;
-    }
+    if (args[5] == Py_None) C = at::empty({rows, n}, B.options().dtype(c_type).requires_grad(false));
+    if (args[7] == Py_None) stream = c10::cuda::getCurrentCUDAStream(B.get_device()).stream();
     const int st = b200spmm_spmm(plan, B.data_ptr(), B.stride(0), n, C.data_ptr(), C.stride(0), c_half ? B200SPMM_C_F16 : B200SPMM_C_F32, stream);
     if (st != B200SPMM_OK) return PyLong_FromLong(st);
     if (args[5] != Py_None) {
@@ -61,6 +60,7 @@ PyObject *spmm(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
         return args[5];
     }
     return THPVariable_Wrap(std::move(C));
+    END_HANDLE_TH_ERRORS
 }
 
 PyMethodDef methods[] = {{"spmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(spmm)), METH_FASTCALL, nullptr}, {nullptr, nullptr, 0, nullptr}};

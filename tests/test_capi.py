@@ -2,6 +2,8 @@
 import ctypes as C
 import os
 import re
+import subprocess
+import sys
 
 import numpy as np
 
@@ -142,3 +144,27 @@ def test_allgather_plan_moves_every_byte_to_every_device():
         for d in range(n):
             assert have[d].all(), (cut, part)
     assert 0 < two_step < len(cases)
+
+
+@pytest.mark.parametrize("policy", ["strides", "sizes"])
+def test_an_argument_whose_accessors_raise_is_an_exception(policy):
+    # a CUDA tensor (in name only) that raises when it is asked for its strides or sizes, as a sparse tensor does; in a
+    # process of its own, which a C++ exception that leaves the native function would abort
+    code = """
+import torch
+from hopper_spmm_b200.spmm import _native_spmm
+class Odd(torch.Tensor):
+    @staticmethod
+    def __new__(cls, dtype):
+        return torch.Tensor._make_wrapper_subclass(cls, (16, 8), dtype=dtype, device="cuda", dispatch_sizes_strides_policy="%s")
+    @classmethod
+    def __torch_dispatch__(cls, func, types, args=(), kwargs=None):
+        raise KeyError("asked")
+for B, C_out in ((Odd(torch.float16), None), (Odd(torch.float16), Odd(torch.float32))):
+    try:
+        _native_spmm()(0, True, 16, 16, B, C_out, False, 0)
+    except KeyError:
+        print("raised")
+""" % policy
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.count("raised") == 2, r.stderr
