@@ -18,6 +18,12 @@ PyObject *refuse(const char *what) {
     return nullptr;
 }
 
+// Other Python threads run while this exists.
+struct ThreadsAllowed {
+    PyThreadState *state = PyEval_SaveThread();
+    ~ThreadsAllowed() { PyEval_RestoreThread(state); }
+};
+
 // spmm(plan, is_f16, rows, cols, B, C or None, c_half, stream or None) -> C, or a status code that is not 0
 // Any tensor accessor may throw: a sparse tensor has no strides, a tensor subclass may answer for sizes and strides in
 // Python.  The macros turn whatever comes (a Python error among it) into the exception the caller sees.
@@ -53,7 +59,14 @@ PyObject *spmm(PyObject *, PyObject *const *args, Py_ssize_t n_args) {
     }
     if (args[5] == Py_None) C = at::empty({rows, n}, B.options().dtype(c_type).requires_grad(false));
     if (args[7] == Py_None) stream = c10::cuda::getCurrentCUDAStream(B.get_device()).stream();
-    const int st = b200spmm_spmm(plan, B.data_ptr(), B.stride(0), n, C.data_ptr(), C.stride(0), c_half ? B200SPMM_C_F16 : B200SPMM_C_F32, stream);
+    const void *b = B.data_ptr();
+    void *c = C.data_ptr();
+    const int64_t ldb = B.stride(0), ldc = C.stride(0);
+    int st;
+    {  // the call waits for the device when a buffer of the plan grows, and for room when the stream's queue is full
+        const ThreadsAllowed threads;
+        st = b200spmm_spmm(plan, b, ldb, n, c, ldc, c_half ? B200SPMM_C_F16 : B200SPMM_C_F32, stream);
+    }
     if (st != B200SPMM_OK) return PyLong_FromLong(st);
     if (args[5] != Py_None) {
         Py_INCREF(args[5]);

@@ -141,6 +141,41 @@ def test_starved_pipeline_times_out_and_the_plan_recovers(case):
         plan.close()
 
 
+def test_other_threads_run_while_a_launch_waits():
+    # A wider B lets a buffer of the plan (pieces of cut rows) grow, which waits for the device, here for some 0.2 s of
+    # queued work: another Python thread has to go on meanwhile.
+    import threading
+    import time
+    import torch
+    rows, cols, rp, ci, v = random_csr(2000, 2000, 0.002, 3, dense_rows=[7])
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    ticks, done = [], threading.Event()
+
+    def tick():
+        while not done.wait(0.002):
+            ticks.append(time.perf_counter())
+
+    other = threading.Thread(target=tick)
+    try:
+        B = torch.from_numpy(dense_b(cols, 192, 3)).cuda()
+        plan.spmm(B[:, :64])
+        assert plan.launch_info().kernel_launches == 2  # there are cut rows
+        other.start()
+        torch.cuda._sleep(400_000_000)
+        t0 = time.perf_counter()
+        got = plan.spmm(B, sync=False)
+        t1 = time.perf_counter()
+        plan.sync()
+        parity.check(got.cpu().numpy(), rows, rp, ci, v, B.cpu().numpy())
+    finally:
+        done.set()
+        if other.ident:
+            other.join()
+        plan.close()
+    assert t1 - t0 > 0.05, "the launch did not wait"
+    assert sum(t0 < t < t1 for t in ticks) >= 5
+
+
 def test_more_ctas_than_windows_and_one_cta():
     rows, cols, rp, ci, v = random_csr(96, 300, 0.1, 8)
     B = dense_b(cols, 64, 4)
