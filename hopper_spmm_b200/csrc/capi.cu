@@ -91,8 +91,7 @@ struct b200spmm_plan {
     RowsFormat rows_fmt;
     bool rows_only = false;
     NarrowFormat narrow;       // the entries once more for narrow B (spmm_narrow_kernel.cuh), or empty
-    bool may_time_out = false;   // a kernel with bounded waits was launched since the status word was last read
-    bool has_tile_path = false;  // schedule and tile image of the 16-row kernel are there
+    bool has_tile_path = false;  // schedule and tile image of the 16-row kernel are there, so kernels with bounded waits may run
     // Most tiles of the super-window format name one aligned group of CW consecutive rows of B: then B
     // is re-laid as shared-memory images at every launch (scratch of the plan, as large as B) and such a
     // tile's operand arrives by one bulk copy.
@@ -1283,7 +1282,6 @@ int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, voi
         int st = plan_add_tile_path(p, 0);
         if (st != B200SPMM_OK) return st;
     }
-    p->may_time_out = true;
     if (band < 0 && use_tall(p, n)) return launch_tall(p, d_B, ldb, n, d_C, ldc, c_dtype, stream);
     SpmmParams prm{};
     prm.rowOffset = p->d_rowOffset;
@@ -1363,12 +1361,15 @@ int b200spmm_plan_sync(b200spmm_plan_t *p, void *stream_v) {
     if (!p) return B200SPMM_ERR_INVALID_ARG;
     B200_CUDA_TRY(cudaSetDevice(p->device));
     B200_CUDA_TRY(cudaStreamSynchronize(static_cast<cudaStream_t>(stream_v)));
-    if (!p->may_time_out) return B200SPMM_OK;  // (row units wait for nothing)
+    // Row units wait for nothing.  Any other plan's word is read at every call: a captured launch runs again without
+    // passing here, and one on another stream may raise it after this call.
+    if (!p->has_tile_path) return B200SPMM_OK;
     uint32_t status = 0;
     B200_CUDA_TRY(cudaMemcpy(&status, p->d_status, sizeof(status), cudaMemcpyDeviceToHost));
-    p->may_time_out = false;
     if (status) {
-        B200_CUDA_TRY(cudaMemset(p->d_status, 0, 4 * sizeof(uint32_t)));  // status and the hand-out counters
+        // status and the hand-out counters, cleared before the caller can launch again (on any stream)
+        B200_CUDA_TRY(cudaMemset(p->d_status, 0, 4 * sizeof(uint32_t)));
+        B200_CUDA_TRY(cudaStreamSynchronize(nullptr));
         return B200SPMM_ERR_DEVICE_TIMEOUT;
     }
     return B200SPMM_OK;

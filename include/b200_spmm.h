@@ -368,8 +368,9 @@ int b200spmm_tf32_spmm(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t
                        int c_dtype, void *stream);
 
 /*
- * Blocks until `stream` is idle, then returns the kernel-side status of the plan's last
- * launch (B200SPMM_ERR_DEVICE_TIMEOUT if a bounded wait gave up).
+ * Blocks until `stream` is idle, then returns the kernel-side status of the plan's launches
+ * (B200SPMM_ERR_DEVICE_TIMEOUT if a bounded wait of one of them gave up and no earlier call
+ * has said so; replays of a captured launch count).
  */
 int b200spmm_plan_sync(b200spmm_plan_t *p, void *stream);
 

@@ -141,6 +141,46 @@ def test_starved_pipeline_times_out_and_the_plan_recovers(case):
         plan.close()
 
 
+@pytest.mark.parametrize("how", ["graph", "streams"])
+def test_a_time_out_is_reported_after_an_earlier_sync(how, monkeypatch):
+    # The launch of the test above, seen by a later sync than the first one: every replay of a captured product that
+    # times out is reported, and a sync on another stream than the launch's does not hide it.
+    import torch
+    monkeypatch.setenv("B200SPMM_WINDOW", "16")
+    rows, cols, rp, ci, v = random_csr(203, 517, 0.03, 11, dense_rows=[7])
+    n = 128
+    B = torch.from_numpy(dense_b(cols, n, 3)).cuda()
+    dC = torch.zeros((rows, n), device="cuda")
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    lib = capi.lib()
+
+    def starve(stream, limit_ns):
+        return lib.b200spmm_kat_spmm_starved(plan._p, B.data_ptr(), n, n, dC.data_ptr(), n, limit_ns, stream.cuda_stream)
+
+    try:
+        plan.spmm(B, dC)  # (buffers are grown before a capture)
+        launch, other = torch.cuda.Stream(), torch.cuda.Stream()
+        torch.cuda.synchronize()
+        if how == "graph":
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=launch):
+                assert starve(launch, 5_000_000) == 0
+            for _ in range(3):
+                with torch.cuda.stream(launch):
+                    graph.replay()
+                assert lib.b200spmm_plan_sync(plan._p, launch.cuda_stream) == capi.ERR_DEVICE_TIMEOUT
+            del graph
+        else:
+            assert starve(launch, 200_000_000) == 0
+            assert lib.b200spmm_plan_sync(plan._p, other.cuda_stream) == 0  # still waiting
+            assert lib.b200spmm_plan_sync(plan._p, launch.cuda_stream) == capi.ERR_DEVICE_TIMEOUT
+        assert lib.b200spmm_plan_sync(plan._p, launch.cuda_stream) == 0  # reported once
+        plan.spmm(B, dC)
+        parity.check(dC.cpu().numpy(), rows, rp, ci, v, B.cpu().numpy())
+    finally:
+        plan.close()
+
+
 def test_other_threads_run_while_a_launch_waits():
     # A wider B lets a buffer of the plan (pieces of cut rows) grow, which waits for the device, here for some 0.2 s of
     # queued work: another Python thread has to go on meanwhile.
