@@ -91,6 +91,9 @@ struct b200spmm_plan {
     RowsFormat rows_fmt;
     bool rows_only = false;
     NarrowFormat narrow;       // the entries once more for narrow B (spmm_narrow_kernel.cuh), or empty
+    // A caller's column lists that are not as the converter makes them: only what takes any list may run, the 16-row
+    // kernel without row boxes and the kernels that go by entries.
+    bool loose_lists = false;
     bool has_tile_path = false;  // schedule and tile image of the 16-row kernel are there, so kernels with bounded waits may run
     // Most tiles of the super-window format name one aligned group of CW consecutive rows of B: then B
     // is re-laid as shared-memory images at every launch (scratch of the plan, as large as B) and such a
@@ -180,6 +183,60 @@ tile_entries_kernel(const uint16_t *__restrict__ data, uint64_t tiles, uint32_t 
 }
 
 }  // namespace tileimage
+
+namespace formatcheck {
+
+enum : uint32_t { kBadTables = 1u, kLooseLists = 2u };
+
+struct Found {
+    uint32_t flags;
+    int32_t falls;  // places where a column is not above the one before it, less those where a window starts
+};
+
+// Looks over the tables of a caller's format.  Bad tables: window offsets that do not rise from 0 to the number of tiles,
+// window rows that are past the end or closer than a window; nothing can run on them.  Loose lists: a window's columns are
+// not ascending and distinct with less than a tile of padding behind them, one is past the end, or a window starts off the
+// 16-row grid.  A column that does not rise is right where a window starts and nowhere else, so the lists are read once, four
+// entries a thread, and the windows take their own falls off the count (searching the window of every fall: 8 us for
+// 60,000 nodes and 700,000 entries, now 5).  Reads inside [eff + 1], [eff] and [tiles * cw] whatever the tables hold.
+__global__ void __launch_bounds__(256)
+tables_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B, const uint32_t *__restrict__ rowIdx, uint32_t eff,
+              uint32_t tiles, uint64_t rows, uint64_t cols, uint32_t cw, Found *__restrict__ found) {
+    uint32_t flags = 0;
+    int32_t falls = 0;
+    const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    if (first == 0 && (rowOffset[0] != 0 || rowOffset[eff] != tiles)) flags |= kBadTables;
+    auto fall = [](uint32_t before, uint32_t c) { return c != kIdxMax && before >= c; };
+    for (uint64_t w = first; w < eff; w += step) {
+        const uint32_t t = rowOffset[w], row = rowIdx[w];
+        if (rowOffset[w + 1] <= t || row >= rows) flags |= kBadTables;
+        if (row % kRowWindow) flags |= kLooseLists;
+        if (!w) continue;
+        const uint32_t row_before = rowIdx[w - 1];
+        if (row < row_before || row - row_before < (uint32_t)kRowWindow) flags |= kBadTables;
+        if (t && t < tiles && fall(tcA2B[(uint64_t)t * cw - 1], tcA2B[(uint64_t)t * cw])) --falls;
+    }
+    for (uint64_t q = first; q < (uint64_t)tiles * cw / 4; q += step) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(tcA2B) + q);
+        const uint32_t c[4] = {v.x, v.y, v.z, v.w};
+        uint32_t before = q ? __ldg(tcA2B + q * 4 - 1) : 0u;
+        if (q * 4 % cw == 0 && c[0] == kIdxMax) flags |= kLooseLists;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (c[k] != kIdxMax && c[k] >= cols) flags |= kLooseLists;
+            if ((q || k) && fall(before, c[k])) ++falls;
+            before = c[k];
+        }
+    }
+    falls = __reduce_add_sync(0xffffffffu, falls);
+    flags = __reduce_or_sync(0xffffffffu, flags);
+    if ((threadIdx.x & 31u) == 0) {
+        if (falls) atomicAdd(&found->falls, falls);
+        if (flags) atomicOr(&found->flags, flags);
+    }
+}
+
+}  // namespace formatcheck
 
 namespace {
 
@@ -772,7 +829,8 @@ int plan_build_tile_path(b200spmm_plan *p, const uint32_t *h_rowOffset, const ui
         B200_CUDA_TRY(e);
         p->entry_dense_tiles = n_dense;
     }
-    if (n_ctas <= 0 && !p->comp.tcBit) {  // an explicit CTA count or compressed tiles ask for the 16-row kernel
+    // an explicit CTA count or compressed tiles ask for the 16-row kernel, and loose lists cannot be merged
+    if (n_ctas <= 0 && !p->comp.tcBit && !p->loose_lists) {
         int st = plan_build_tall(p, h_rowOffset, h_rowIdx);
         if (st != B200SPMM_OK) return st;
     }
@@ -796,8 +854,8 @@ int plan_add_tile_path(b200spmm_plan *p, int n_ctas) {
     return plan_build_tile_path(p, h_rowOffset.data(), h_rowIdx.data(), n_ctas);
 }
 
-// h_rowOffset and h_rowIdx may be null: they are read back if the plan needs them.
-int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h_rowIdx, int n_ctas) {
+// What every plan starts with: a format and a device the kernels take, and the status word.
+int plan_start(b200spmm_plan *p) {
     const auto &info = p->info;
     if (info.row_window != kRowWindow) return B200SPMM_ERR_UNSUPPORTED;
     const int cw = info.dtype == B200SPMM_F16 ? 16 : 8;
@@ -807,12 +865,39 @@ int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h
     B200_CUDA_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, p->device));
     if (major != 10) return B200SPMM_ERR_NO_DEVICE;
     B200_CUDA_TRY(cudaDeviceGetAttribute(&p->n_sms, cudaDevAttrMultiProcessorCount, p->device));
-    // status word, then the two counters of the chunk hand-out (the kernel leaves them at zero)
-    B200_CUDA_TRY(pool_alloc(&p->d_status, 4));
-    B200_CUDA_TRY(cudaMemset(p->d_status, 0, 4 * sizeof(uint32_t)));
+    // status word, then the two counters of the chunk hand-out (the kernel leaves them at zero), then plan_check_tables' two
+    B200_CUDA_TRY(pool_alloc(&p->d_status, 6));
+    B200_CUDA_TRY(cudaMemset(p->d_status, 0, 6 * sizeof(uint32_t)));
+    return B200SPMM_OK;
+}
+
+// A caller's device arrays: refused, or marked as loose (see formatcheck::tables_kernel).
+int plan_check_tables(b200spmm_plan *p) {
+    const auto &info = p->info;
+    if (info.eff_row_windows > info.total_tiles) return B200SPMM_ERR_INVALID_ARG;  // every window holds a tile
+    auto *d_found = reinterpret_cast<formatcheck::Found *>(p->d_status + 4);
+    formatcheck::Found found{};
+    const uint64_t n = std::max<uint64_t>(info.eff_row_windows, info.total_tiles * (uint64_t)info.col_window / 4);
+    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)p->n_sms * 8));
+    formatcheck::tables_kernel<<<grid, 256>>>(p->d_rowOffset, p->d_tcA2B, p->d_rowIdx, (uint32_t)info.eff_row_windows, (uint32_t)info.total_tiles,
+                                              info.rows, info.cols, (uint32_t)info.col_window, d_found);
+    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(cudaMemcpy(&found, d_found, sizeof(found), cudaMemcpyDeviceToHost));
+    if (found.flags & formatcheck::kBadTables) {
+        set_last_error_static("rowOffset or rowIdx does not describe windows of the matrix");
+        return B200SPMM_ERR_INVALID_ARG;
+    }
+    p->loose_lists = found.flags || found.falls;
+    return B200SPMM_OK;
+}
+
+// h_rowOffset and h_rowIdx may be null: they are read back if the plan needs them.
+int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h_rowIdx, int n_ctas) {
+    const auto &info = p->info;
+    const int cw = info.col_window;
     p->gather_cpasync = env_is("B200SPMM_GATHER", "cpasync");
     p->host_split = !env_is("B200SPMM_HOST_SPLIT", "0");
-    p->row_boxes = true;
+    p->row_boxes = !p->loose_lists;
     // An explicit CTA count, a way to fetch tiles or rows, or a window height asks for a tile kernel.
     // B200SPMM_WINDOW=rows asks for the row units whatever the matrix.
     const bool force_rows = env_is("B200SPMM_WINDOW", "rows");
@@ -833,7 +918,7 @@ int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h
             // (an eighth of the short tiles is the least that merging eight windows can leave)
             if (fill / (8.0 * ratio) < kTallMinFill || info.total_tiles < kTallMinShortTiles) max_fill = kRowsMaxFillWide;
         }
-        int st = build_row_formats(info, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, p->n_sms, max_fill, force_rows,
+        int st = build_row_formats(info, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, p->loose_lists, p->n_sms, max_fill, force_rows,
                                    &p->rows_fmt, &p->narrow);
         if (st != B200SPMM_OK) return st;
         p->rows_only = p->rows_fmt.n_units > 0;
@@ -1128,6 +1213,7 @@ int b200spmm_plan_create(const b200spmm_btcf_t *h, int device, int n_ctas, b200s
     if (st == B200SPMM_OK) st = upload((void **)&p->d_tcA2B, f.tcA2B.data(), f.tcA2B.size() * 4);
     if (st == B200SPMM_OK) st = upload((void **)&p->d_rowIdx, f.rowIdx.data(), f.rowIdx.size() * 4);
     if (st == B200SPMM_OK) st = upload(&p->d_data, f.data.data(), f.data.size());
+    if (st == B200SPMM_OK) st = plan_start(p);
     if (st == B200SPMM_OK) st = plan_finish(p, f.rowOffset.data(), f.rowIdx.data(), n_ctas);
     if (st != B200SPMM_OK) {
         b200spmm_plan_destroy(p);
@@ -1142,7 +1228,7 @@ int b200spmm_plan_create_device(const b200spmm_btcf_info_t *info, const uint32_t
                                 b200spmm_plan_t **out) {
     if (!info || !out || !d_rowOffset) return B200SPMM_ERR_INVALID_ARG;
     if (info->total_tiles && (!d_tcA2B || !d_data || !d_rowIdx)) return B200SPMM_ERR_INVALID_ARG;
-    if ((reinterpret_cast<uintptr_t>(d_data) & 15u) != 0) return B200SPMM_ERR_UNSUPPORTED;
+    if (((reinterpret_cast<uintptr_t>(d_data) | reinterpret_cast<uintptr_t>(d_tcA2B)) & 15u) != 0) return B200SPMM_ERR_UNSUPPORTED;
     *out = nullptr;
     int n_dev = 0;
     if (cudaGetDeviceCount(&n_dev) != cudaSuccess || device < 0 || device >= n_dev) {
@@ -1159,13 +1245,9 @@ int b200spmm_plan_create_device(const b200spmm_btcf_info_t *info, const uint32_t
     p->d_tcA2B = const_cast<uint32_t *>(d_tcA2B);
     p->d_rowIdx = const_cast<uint32_t *>(d_rowIdx);
     p->d_data = const_cast<void *>(d_data);
-    int st = B200SPMM_OK;
-    uint32_t tiles = 0;
-    if (cudaMemcpy(&tiles, d_rowOffset + info->eff_row_windows, 4, cudaMemcpyDeviceToHost) != cudaSuccess) {
-        record_cuda_error(cudaGetLastError(), "cudaMemcpy(rowOffset)");
-        st = B200SPMM_ERR_CUDA;
-    }
-    if (st == B200SPMM_OK && tiles != info->total_tiles) st = B200SPMM_ERR_INVALID_ARG;
+    p->info.elt_size = info->dtype == B200SPMM_F16 ? 2 : 4;
+    int st = plan_start(p);
+    if (st == B200SPMM_OK) st = plan_check_tables(p);
     if (st == B200SPMM_OK) st = plan_finish(p, nullptr, nullptr, n_ctas);
     if (st != B200SPMM_OK) {
         b200spmm_plan_destroy(p);

@@ -7,7 +7,8 @@
 //   3. units sorted by (band, length), longest first (CUB radix sort, a few key bits), their batches numbered in
 //      that order
 //   4. the warps of step 1 write (column, value) to the place of their row's unit
-// A stored value is one whose bits are not all zero (an explicit zero adds nothing to a product).
+// A stored value is one whose bits are not all zero (an explicit zero adds nothing to a product), in a row and a column
+// of the matrix: the arrays may be a caller's, and what lies in a padded slot or below the last row multiplies nothing.
 #include <algorithm>
 #include <cub/cub.cuh>
 
@@ -74,24 +75,56 @@ struct Piece {
 #pragma unroll
         for (int k = 0; k < kPer; ++k) mask |= v[k] != 0 ? 1u << k : 0u;
     }
+    // Leaves the values that count.  `cols`: of the lane's half, `n_cols`: 0 for a row below the last one.  Unless the lists
+    // are loose, only the last tile of a window has slots without a column.
+    __device__ __forceinline__ void keep(const uint32_t (&cols)[kPer], uint32_t n_cols) {
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) mask &= cols[k] < n_cols ? 0xFFFFFFFFu : ~(1u << k);
+    }
 };
+
+// The columns of the lane's half of a tile.
+template <int kPer>
+__device__ __forceinline__ void load_columns(uint32_t (&cols)[kPer], const uint32_t *__restrict__ tcA2B, uint64_t tile, uint32_t lane) {
+#pragma unroll
+    for (int k = 0; k < kPer / 4; ++k)
+        reinterpret_cast<uint4 *>(cols)[k] = __ldg(reinterpret_cast<const uint4 *>(tcA2B + tile * (2 * kPer) + (lane & 1u) * kPer) + k);
+}
 
 // counts[run * 16 + row] = stored values of that row in the run's tiles
 template <typename T>
 __global__ void __launch_bounds__(kBlock)
-run_rows_kernel(const uint32_t *__restrict__ rowOffset, const T *__restrict__ data, const uint32_t *__restrict__ run_first,
-                const uint32_t *__restrict__ run_window, uint32_t eff, uint32_t *__restrict__ counts) {
+run_rows_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B, const T *__restrict__ data,
+                const uint32_t *__restrict__ rowIdx, const uint32_t *__restrict__ run_first, const uint32_t *__restrict__ run_window,
+                uint32_t eff, uint32_t rows, uint32_t cols, bool loose, uint32_t *__restrict__ counts) {
     const uint32_t lane = threadIdx.x & 31u, n_runs = run_first[eff];
     for (uint32_t run = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); run < n_runs; run += gridDim.x * (kBlock / 32)) {
         const uint32_t w = run_window[run], t0 = rowOffset[w] + (run - run_first[w]) * kRunTiles;
-        const uint32_t t1 = min(t0 + kRunTiles, rowOffset[w + 1]);
+        const uint32_t end = rowOffset[w + 1], t1 = min(t0 + kRunTiles, end);
+        alignas(16) uint32_t of[Piece<T>::kPer];
+        load_columns(of, tcA2B, t1 - 1, lane);
         uint32_t mine = 0;
+        Piece<T> p;
+        if (loose) {
+            for (uint32_t t = t0; t < t1; ++t) {
+                p.load(data, t, lane);
+                load_columns(of, tcA2B, t, lane);
+                p.keep(of, cols);
+                mine += __popc(p.mask);
+            }
+        } else {
 #pragma unroll 4
-        for (uint32_t t = t0; t < t1; ++t) {
-            Piece<T> p;
-            p.load(data, t, lane);
-            mine += __popc(p.mask);
+            for (uint32_t t = t0; t < t1; ++t) {
+                p.load(data, t, lane);
+                mine += __popc(p.mask);
+            }
+            if (t1 == end) {
+                mine -= __popc(p.mask);
+                p.keep(of, cols);
+                mine += __popc(p.mask);
+            }
         }
+        if (rowIdx[w] + (lane >> 1) >= rows) mine = 0;
         mine += __shfl_xor_sync(0xffffffffu, mine, 1);
         if (!(lane & 1u)) counts[(uint64_t)run * 16 + (lane >> 1)] = mine;
     }
@@ -228,7 +261,8 @@ template <typename T>
 __global__ void __launch_bounds__(kBlock)
 write_entries_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B, const T *__restrict__ data,
                      const uint32_t *__restrict__ rowIdx, const uint32_t *__restrict__ run_first,
-                     const uint32_t *__restrict__ run_window, uint32_t eff, uint32_t rows, uint32_t cap, const uint32_t *__restrict__ counts,
+                     const uint32_t *__restrict__ run_window, uint32_t eff, uint32_t rows, uint32_t n_cols, bool loose, uint32_t cap,
+                     const uint32_t *__restrict__ counts,
                      const uint32_t *__restrict__ row_len, const unsigned long long *__restrict__ a,
                      const uint32_t *__restrict__ unit_batch, uint32_t *__restrict__ batches) {
     constexpr int kPer = Piece<T>::kPer;
@@ -236,8 +270,8 @@ write_entries_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__r
     const uint32_t lane = threadIdx.x & 31u, n_runs = run_first[eff];
     for (uint32_t run = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); run < n_runs; run += gridDim.x * (kBlock / 32)) {
         const uint32_t w = run_window[run], t0 = rowOffset[w] + (run - run_first[w]) * kRunTiles;
-        const uint32_t t1 = min(t0 + kRunTiles, rowOffset[w + 1]), row = min(rowIdx[w] + (lane >> 1), rows - 1);
-        const uint32_t len = row_len[row];
+        const uint32_t w_end = rowOffset[w + 1], t1 = min(t0 + kRunTiles, w_end), row = min(rowIdx[w] + (lane >> 1), rows - 1);
+        const uint32_t len = row_len[row], limit = rowIdx[w] + (lane >> 1) < rows ? n_cols : 0u;
         const uint32_t *unit = unit_batch + ((uint32_t)a[row] - pieces_of(len, cap));  // first batches of the row's units
         uint32_t at = counts[(uint64_t)run * 16 + (lane >> 1)];  // entries of the row so far
         // Everything a lane reads comes ahead of its stores and for all lanes at once - the unit it starts in, a tile's
@@ -251,19 +285,18 @@ write_entries_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__r
             reinterpret_cast<T *>(words + kUnitBatch)[e % kUnitBatch] = sizeof(T) == 2 ? v : (T)((uint32_t)v & 0xFFFFE000u);  // as the tensor core reads it
         };
         Piece<T> next;
-        uint32_t next_cols[kPer];
+        alignas(16) uint32_t next_cols[kPer];
         auto fetch = [&](uint32_t t) {
             next.load(data, t, lane);
-#pragma unroll
-            for (int k = 0; k < kPer / 4; ++k)
-                reinterpret_cast<uint4 *>(next_cols)[k] = __ldg(reinterpret_cast<const uint4 *>(tcA2B + (uint64_t)t * (2 * kPer) + (lane & 1u) * kPer) + k);
+            load_columns(next_cols, tcA2B, t, lane);
         };
         fetch(t0);
         for (uint32_t t = t0; t < t1; ++t) {
-            const Piece<T> p = next;
+            Piece<T> p = next;
             uint32_t cols[kPer];
 #pragma unroll
             for (int k = 0; k < kPer; ++k) cols[k] = next_cols[k];
+            if (loose || t + 1 == w_end || limit == 0) p.keep(cols, limit);
             if (t + 1 < t1) fetch(t + 1);
             const uint32_t mine = (uint32_t)__popc(p.mask), other = __shfl_xor_sync(0xffffffffu, mine, 1);
             uint32_t k_out = at + ((lane & 1u) ? other : 0u);
@@ -304,25 +337,25 @@ template <typename T>
 __global__ void __launch_bounds__(kBlock)
 write_csr_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B, const T *__restrict__ data,
                  const uint32_t *__restrict__ rowIdx, const uint32_t *__restrict__ run_first, const uint32_t *__restrict__ run_window,
-                 uint32_t eff, uint32_t rows, const uint32_t *__restrict__ counts, const unsigned long long *__restrict__ a,
-                 uint32_t *__restrict__ cols_out, T *__restrict__ vals_out) {
+                 uint32_t eff, uint32_t rows, uint32_t n_cols, const uint32_t *__restrict__ counts,
+                 const unsigned long long *__restrict__ a, uint32_t *__restrict__ cols_out, T *__restrict__ vals_out) {
     constexpr int kPer = Piece<T>::kPer;
     const uint32_t lane = threadIdx.x & 31u, n_runs = run_first[eff];
     for (uint32_t run = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); run < n_runs; run += gridDim.x * (kBlock / 32)) {
         const uint32_t w = run_window[run], t0 = rowOffset[w] + (run - run_first[w]) * kRunTiles;
         const uint32_t t1 = min(t0 + kRunTiles, rowOffset[w + 1]), row = min(rowIdx[w] + (lane >> 1), rows - 1);
+        const uint32_t limit = rowIdx[w] + (lane >> 1) < rows ? n_cols : 0u;
         uint32_t at = (row ? (uint32_t)(a[row - 1] >> 32) : 0u) + counts[(uint64_t)run * 16 + (lane >> 1)];
 #pragma unroll 2
         for (uint32_t t = t0; t < t1; ++t) {
             Piece<T> p;
+            alignas(16) uint32_t cols[kPer];
             p.load(data, t, lane);
+            load_columns(cols, tcA2B, t, lane);
+            p.keep(cols, limit);
             const uint32_t mine = (uint32_t)__popc(p.mask), other = __shfl_xor_sync(0xffffffffu, mine, 1);
             uint32_t k_out = at + ((lane & 1u) ? other : 0u);
             at += mine + other;
-            uint32_t cols[kPer];
-#pragma unroll
-            for (int k = 0; k < kPer / 4; ++k)
-                reinterpret_cast<uint4 *>(cols)[k] = __ldg(reinterpret_cast<const uint4 *>(tcA2B + (uint64_t)t * (2 * kPer) + (lane & 1u) * kPer) + k);
 #pragma unroll
             for (int k = 0; k < kPer; ++k)
                 if (p.mask & (1u << k)) {
@@ -422,6 +455,7 @@ int build_narrow(const b200spmm_btcf_info_t &info, uint64_t nnz, const uint32_t 
                  const uint32_t *d_rowIdx, int n_sms, const uint32_t *run_first, const uint32_t *run_window, int run_grid,
                  const uint32_t *counts, const unsigned long long *a, NarrowFormat *out) {
     const uint32_t rows = (uint32_t)info.rows, eff = (uint32_t)info.eff_row_windows, words = (uint32_t)info.elt_size / 2;
+    const uint32_t n_cols = (uint32_t)info.cols;
     NarrowFormat f;
     struct Guard {
         NarrowFormat *f;
@@ -446,11 +480,11 @@ int build_narrow(const b200spmm_btcf_info_t &info, uint64_t nnz, const uint32_t 
     const size_t smem = (size_t)(kBlock / 32) * 2 * f.n_blocks * 8 * 4;
     if (info.elt_size == 2) {
         write_csr_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, static_cast<const uint16_t *>(d_data), d_rowIdx, run_first,
-                                                         run_window, eff, rows, counts, a, cols, static_cast<uint16_t *>(vals));
+                                                         run_window, eff, rows, n_cols, counts, a, cols, static_cast<uint16_t *>(vals));
         narrow_entries_kernel<uint16_t><<<grid, kBlock, smem>>>(cols, static_cast<const uint16_t *>(vals), a, rows, f.n_blocks, f.d_seg, f.d_entries);
     } else {
         write_csr_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, static_cast<const uint32_t *>(d_data), d_rowIdx, run_first,
-                                                         run_window, eff, rows, counts, a, cols, static_cast<uint32_t *>(vals));
+                                                         run_window, eff, rows, n_cols, counts, a, cols, static_cast<uint32_t *>(vals));
         narrow_entries_kernel<uint32_t><<<grid, kBlock, smem>>>(cols, static_cast<const uint32_t *>(vals), a, rows, f.n_blocks, f.d_seg, f.d_entries);
     }
     narrow_cuts_kernel<<<(int)(f.n_ctas / kBlock + 1), kBlock>>>(a, rows, f.n_ctas, f.d_cut);
@@ -467,13 +501,14 @@ int build_narrow(const b200spmm_btcf_info_t &info, uint64_t nnz, const uint32_t 
 }  // namespace
 
 int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOffset, const uint32_t *d_tcA2B,
-                      const void *d_data, const uint32_t *d_rowIdx, int n_sms, double max_fill, bool force_rows,
+                      const void *d_data, const uint32_t *d_rowIdx, bool loose, int n_sms, double max_fill, bool force_rows,
                       RowsFormat *out, NarrowFormat *narrow) {
     *out = RowsFormat();
     *narrow = NarrowFormat();
     const uint64_t tiles = info.total_tiles;
-    if (!info.eff_row_windows || !tiles || info.rows >= kSlotTarget) return B200SPMM_OK;
-    const uint32_t rows = (uint32_t)info.rows, eff = (uint32_t)info.eff_row_windows;
+    // (the product is refused for more columns, and the running sums of entries are 32-bit)
+    if (!info.eff_row_windows || !tiles || info.rows >= kSlotTarget || info.cols > 0x7FFFFFFFull || info.nnzs > 0xFFFFFFFFull) return B200SPMM_OK;
+    const uint32_t rows = (uint32_t)info.rows, cols = (uint32_t)info.cols, eff = (uint32_t)info.eff_row_windows;
     const uint32_t cap = unit_entries_for(info.nnzs, info.rows, n_sms);
     RowsFormat f;
     struct Guard {
@@ -505,8 +540,8 @@ int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
     const uint16_t *data16 = static_cast<const uint16_t *>(d_data);
     const uint32_t *data32 = static_cast<const uint32_t *>(d_data);
     const int run_grid = grid_for(max_runs * 32), row_grid = (int)((rows + kBlock - 1) / kBlock);
-    if (f16) run_rows_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, data16, run_first, run_window, eff, counts);
-    else run_rows_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, data32, run_first, run_window, eff, counts);
+    if (f16) run_rows_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data16, d_rowIdx, run_first, run_window, eff, rows, cols, loose, counts);
+    else run_rows_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data32, d_rowIdx, run_first, run_window, eff, rows, cols, loose, counts);
     uint32_t *max_len = totals + kMaxLenAt;
     B200_CUDA_TRY(cudaMemsetAsync(row_len, 0, (size_t)rows * 4));
     B200_CUDA_TRY(cudaMemsetAsync(max_len, 0, 4));
@@ -568,12 +603,12 @@ int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
     if (f16) {
         place_units_kernel<false><<<unit_grid, kBlock>>>(keys[1], ids[1], quads, f.n_units, cap, unit_row, row_len, a, b, f.d_units,
                                                          unit_batch, f.d_batches);
-        write_entries_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data16, d_rowIdx, run_first, run_window, eff, rows, cap,
+        write_entries_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data16, d_rowIdx, run_first, run_window, eff, rows, cols, loose, cap,
                                                              counts, row_len, a, unit_batch, f.d_batches);
     } else {
         place_units_kernel<true><<<unit_grid, kBlock>>>(keys[1], ids[1], quads, f.n_units, cap, unit_row, row_len, a, b, f.d_units,
                                                         unit_batch, f.d_batches);
-        write_entries_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data32, d_rowIdx, run_first, run_window, eff, rows, cap,
+        write_entries_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data32, d_rowIdx, run_first, run_window, eff, rows, cols, loose, cap,
                                                              counts, row_len, a, unit_batch, f.d_batches);
     }
     band_units_kernel<<<1, 32>>>(keys[1], quads, f.n_units, bands, totals);

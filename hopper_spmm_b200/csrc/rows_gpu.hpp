@@ -56,9 +56,9 @@ struct NarrowFormat {
 // Builds what the kernels outside the tile path want from a matrix: row units when `force_rows` or when at most
 // max_fill of the tiles' slots are in use, and the format for narrow B where it fits (at most 65,536 columns, rows
 // of some length, none so long that CTAs of whole rows could not be balanced).  The tiles must be in the reference's layout
-// (row-major 16 x CW).  A format stays empty when device memory is short.
+// (row-major 16 x CW); `loose`: slots without a column may lie anywhere in a window, and not only in its last tile.  A format stays empty when device memory is short.
 int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOffset, const uint32_t *d_tcA2B,
-                      const void *d_data, const uint32_t *d_rowIdx, int n_sms, double max_fill, bool force_rows,
+                      const void *d_data, const uint32_t *d_rowIdx, bool loose, int n_sms, double max_fill, bool force_rows,
                       RowsFormat *rows, NarrowFormat *narrow);
 void free_rows(RowsFormat *r);
 void free_narrow(NarrowFormat *f);

@@ -114,7 +114,7 @@ __global__ void tall_scatter_values_kernel(const uint32_t *__restrict__ rowOffse
 
 // Distinct columns in the lists of a run of 16-row tiles, one block per run.
 __global__ void __launch_bounds__(1024)
-distinct_columns_kernel(const uint32_t *__restrict__ tcA2B, const uint2 *__restrict__ ranges, uint32_t cw, uint64_t words,
+distinct_columns_kernel(const uint32_t *__restrict__ tcA2B, const uint2 *__restrict__ ranges, uint32_t cw, uint64_t cols, uint64_t words,
                         uint32_t *__restrict__ bits, uint32_t *__restrict__ distinct) {
     __shared__ uint32_t total;
     if (threadIdx.x == 0) total = 0;
@@ -123,7 +123,7 @@ distinct_columns_kernel(const uint32_t *__restrict__ tcA2B, const uint2 *__restr
     uint32_t *mine = bits + blockIdx.x * words, n = 0;
     for (uint64_t e = (uint64_t)ranges[blockIdx.x].x * cw + threadIdx.x; e < end; e += 1024) {
         const uint32_t c = tcA2B[e];
-        if (c != kIdxMax && !(atomicOr(mine + (c >> 5), 1u << (c & 31u)) & (1u << (c & 31u)))) ++n;
+        if (c < cols && c != kIdxMax && !(atomicOr(mine + (c >> 5), 1u << (c & 31u)) & (1u << (c & 31u)))) ++n;
     }
     atomicAdd(&total, n);
     __syncthreads();
@@ -156,7 +156,7 @@ int estimate_tall_tile_ratio(const b200spmm_btcf_info_t &info, const uint32_t *h
     *ratio = 1.0;
     if (!n_groups || max_samples < 1) return B200SPMM_OK;
     // one bit per column and sampled super-window, at most 64 MB of them
-    const uint64_t words = (info.cols + 31) / 32;
+    const uint64_t words = info.cols / 32 + 1;
     const uint64_t n_samples = std::max<uint64_t>(1, std::min({(uint64_t)max_samples, n_groups, ((uint64_t)16 << 20) / words}));
     std::vector<uint2> ranges;
     uint64_t short_tiles = 0, tall_tiles = 0;
@@ -173,7 +173,7 @@ int estimate_tall_tile_ratio(const b200spmm_btcf_info_t &info, const uint32_t *h
     B200_CUDA_TRY(tmp.alloc(&bits, n_samples * words));
     B200_CUDA_TRY(cudaMemsetAsync(bits, 0, n_samples * words * 4));
     B200_CUDA_TRY(cudaMemcpy(d_ranges, ranges.data(), n_samples * sizeof(uint2), cudaMemcpyHostToDevice));
-    distinct_columns_kernel<<<(unsigned)n_samples, 1024>>>(d_tcA2B, d_ranges, (uint32_t)cw, words, bits, d_distinct);
+    distinct_columns_kernel<<<(unsigned)n_samples, 1024>>>(d_tcA2B, d_ranges, (uint32_t)cw, info.cols, words, bits, d_distinct);
     B200_CUDA_TRY(cudaGetLastError());
     std::vector<uint32_t> distinct(n_samples);
     B200_CUDA_TRY(cudaMemcpy(distinct.data(), d_distinct, n_samples * 4, cudaMemcpyDeviceToHost));

@@ -336,7 +336,15 @@ int b200spmm_plan_create(const b200spmm_btcf_t *f, int device, int n_ctas, b200s
 /*
  * Same, from format arrays that already live on `device` (for a GPU-side converter or a
  * caller that keeps the format resident).  The plan borrows the four arrays; they must
- * outlive it.  rowOffset is read back once to build the schedule.
+ * outlive it.  d_tcA2B and d_data are 16-byte aligned; info->nnzs is at least the number of values
+ * that are not zero.  The tables are looked over on the device:
+ *   rowOffset rises from 0 to total_tiles, rowIdx lies inside the matrix in steps of at least
+ *   row_window: else B200SPMM_ERR_INVALID_ARG;
+ *   tcA2B as the converter makes it (ascending and distinct columns per window, 0xFFFFFFFF behind
+ *   them) and rowIdx in multiples of row_window: otherwise the product is the same, but the faster
+ *   kernels that rely on it stay out.
+ * A value in a padded slot, in a column past the end or in a row past the end multiplies nothing.
+ * The arrays must not change while the plan is in use.
  */
 int b200spmm_plan_create_device(const b200spmm_btcf_info_t *info, const uint32_t *d_rowOffset,
                                 const uint32_t *d_tcA2B, const void *d_data, const uint32_t *d_rowIdx,
@@ -422,6 +430,7 @@ int b200spmm_bench(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, 
  *     B200SPMM_ERR_DEVICE_TIMEOUT if a bounded wait inside the last allocation-free launch on that
  *     device gave up (it allocates nothing either).
  * Same requirements on shapes and alignment as b200spmm_spmm; d_tcA2B and d_data 16-byte aligned.
+ * rowOffset and rowIdx must be as b200spmm_plan_create_device wants them: nothing is looked over here.
  * Asynchronous on `stream`.
  */
 int b200spmm_spmm_noalloc(const b200spmm_btcf_info_t *info, const uint32_t *d_rowOffset, const uint32_t *d_tcA2B,
