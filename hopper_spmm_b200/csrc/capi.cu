@@ -481,7 +481,10 @@ constexpr double kRowsMaxFill = 0.08;  // share of a tile's slots in use
 // than two a CTA take the same few microseconds either way and stay with their tiles.
 constexpr double kRowsMaxFillWide = 0.11, kTallMinFill = 0.03;
 constexpr uint64_t kRowsWideMinTiles = 592;
-constexpr uint64_t kTallMinShortTiles = 16384;  // 19 us with 16 rows at 64 columns: nothing to gain with 128
+// Fewer tiles keep to 16 rows: the plan is made in 290 us instead of 660, and up to 128 columns the product takes the same
+// (1500 x 1500 at 25 %, 8,758 tiles: 17 and 19 us for 64 and 128 columns against 19 and 20 with 128 rows).  A wide B pays
+// for that: 28 against 25 us for 256 columns, 82 against 26 for 1,024, 298 against 43 for 4,096.
+constexpr uint64_t kTallMinShortTiles = 16384;
 
 bool use_rows(const b200spmm_plan *p, int64_t ldb) {
     return p->rows_only && ldb * p->info.elt_size <= 0xFFFFFFFFll;  // (the kernel's row pitch is 32-bit)
@@ -604,12 +607,16 @@ int launch_narrow(b200spmm_plan *p, uint32_t group_blocks, const void *d_B, int6
 // stays with 16 rows; the 16-row kernel spreads its tiles evenly over all CTAs.  It pays long before every SM has an
 // item: pruned 14336 x 4096, 10 %, fp16, 64 / 128 / 192 columns 33 / 36 / 43 us (56 windows of 256 rows for 74 pairs)
 // against 62 / 79 / 146 with 16 rows; 3000 x 3000, 12 %, 192 columns 33 against 45, but at 64 columns 25 against 23.
+// A tf32 tile takes what an fp16 one does, eight rows of B of twice the bytes.  Pruned, uniform and block matrices and
+// graphs of at least kTallMinShortTiles tiles, 32 to 1,024 columns, against the best of the three kernels when forced: the
+// choice is 0.3 % slower on average in tf32 (84 products, at most 7 %), and in fp16 as fast on average (77 products, at
+// most 15 % slower: 3000 x 3000 with 128 columns, 29 us against 25).
 double tall_micros(const TallFormat &f, int units, int64_t n, int64_t slab) {
     const int64_t items = (int64_t)f.eff * ((n + slab - 1) / slab);
     return 12.0 + (double)((items + units - 1) / units) * (double)f.max_window_tiles * (slab > 128 ? 0.11 : 0.085);
 }
-double short_micros(const b200spmm_plan *p, int64_t n) {
-    return 14.0 + (double)p->info.total_tiles * (n <= 64 ? 0.28e-3 : 0.4e-3 * (double)((n + 127) / 128));
+double short_micros(const b200spmm_plan *p, int64_t n) {  // (tiles over 148 SMs)
+    return 14.0 + (double)p->info.total_tiles * (148.0 / p->n_sms) * (n <= 64 ? 0.28e-3 : 0.4e-3 * (double)((n + 127) / 128));
 }
 
 bool use_pair(const b200spmm_plan *p, int64_t n) {
