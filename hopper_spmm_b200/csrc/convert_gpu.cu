@@ -115,11 +115,11 @@ inline bool window_bits_pay(uint64_t n_windows, uint64_t cols, uint64_t nnz) {
 }
 
 // The distinct columns of every window in order, at columns[first entry of the window ..], and how many they are.
-template <int kUnroll>
 __global__ void __launch_bounds__(kBitsBlock)
 window_columns_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ col_idx, uint32_t rows, uint32_t cols, uint32_t nnz,
                       uint32_t row_window, uint32_t n_windows, uint32_t words, uint32_t *__restrict__ columns, uint32_t *__restrict__ count,
                       Totals *__restrict__ totals) {
+    constexpr int kUnroll = 8;  // columns of a thread in flight
     extern __shared__ __align__(16) uint32_t bits[];
     __shared__ uint32_t start[32], sums[kBitsBlock / 32];
     const uint32_t groups = words / kGroupWords, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -325,10 +325,10 @@ int convert_by_windows(b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const uint3
     B200_CUDA_TRY(pool_alloc(&f->d_rowOffset, (size_t)n_windows + 1, stream));
     B200_CUDA_TRY(pool_alloc(&f->d_rowIdx, n_windows, stream));
     if (smem > 48 * 1024)
-        B200_CUDA_TRY(cudaFuncSetAttribute(window_columns_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBitsSmemMax));
+        B200_CUDA_TRY(cudaFuncSetAttribute(window_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBitsSmemMax));
     const unsigned grid = std::min<uint32_t>(n_windows, 148 * 64), table_grid = n_windows / kBlock + 1;
     B200_CUDA_TRY(cudaMemsetAsync(totals, 0, sizeof(Totals), stream));
-    window_columns_kernel<8><<<grid, kBitsBlock, smem, stream>>>(d_row_ptr, d_col_idx, rows, cols, nnz, RW, n_windows, words, columns, count,
+    window_columns_kernel<<<grid, kBitsBlock, smem, stream>>>(d_row_ptr, d_col_idx, rows, cols, nnz, RW, n_windows, words, columns, count,
                                                                  totals);
     B200_CUDA_TRY(cudaGetLastError());
     B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, terms, before, (int64_t)n_windows + 1, stream));

@@ -25,17 +25,6 @@ B200_DEVICE uint64_t global_timer_ns() {
     return t;
 }
 
-B200_DEVICE bool elect_one() {
-    uint32_t pred;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "elect.sync _|p, 0xffffffff;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(pred));
-    return pred != 0;
-}
 
 // ------------------------------------------------------------------ mbarrier
 
@@ -110,9 +99,6 @@ B200_DEVICE void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shar
 B200_DEVICE void tcgen05_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 B200_DEVICE void tcgen05_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-B200_DEVICE void named_barrier_sync(uint32_t id, uint32_t n_threads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n_threads) : "memory");
-}
 
 // ------------------------------------------------------------------ TMA loads (own HBM only)
 
@@ -154,11 +140,6 @@ B200_DEVICE uint4 ld_shared_v4(uint32_t addr) {
     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
     return v;
 }
-B200_DEVICE uint32_t ld_shared_u32(uint32_t addr) {
-    uint32_t v;
-    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-    return v;
-}
 B200_DEVICE void st_shared_v4(uint32_t addr, uint4 v) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
@@ -173,20 +154,11 @@ B200_DEVICE void st_shared_u16(uint32_t addr, uint16_t v) {
 B200_DEVICE void cp_async_16(uint32_t dst, const void *src, uint32_t src_bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
-// The same for data that is likely to be asked for again by this SM: cached in L1.
-B200_DEVICE void cp_async_ca_16(uint32_t dst, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
 // Copies 4 bytes global -> shared (cached in L1: neighbouring words are fetched next).
 B200_DEVICE void cp_async_4(uint32_t dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 B200_DEVICE void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// Makes `bar` receive one arrival (counted among the expected ones) once every cp.async this
-// thread has issued so far has completed.
-B200_DEVICE void cp_async_mbar_arrive_noinc(uint32_t bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
 template <int N>
 B200_DEVICE void cp_async_wait_group() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
