@@ -22,9 +22,9 @@ _p = C.c_void_p
 
 
 def reference_dir() -> str:
-    """Where the reference project's sources are mounted: $HOPPER_SPMM_REFERENCE, else the default
-    mount point.  Only the build of the harness reads it; nothing needs it at run time."""
-    return os.environ.get("HOPPER_SPMM_REFERENCE", "/root/reference")
+    """Where the reference project's sources are: $HOPPER_SPMM_REFERENCE, or empty.  Only the build of the
+    harness reads it; nothing needs it at run time."""
+    return os.environ.get("HOPPER_SPMM_REFERENCE", "")
 
 
 def build(with_ref: bool = False) -> None:
