@@ -33,8 +33,12 @@ thread_local const char *g_last_static_error = nullptr;
 }
 
 void record_cuda_error(cudaError_t e, const char *what) {
-    g_last_static_error = nullptr;
-    g_last_cuda_error = std::string(what) + ": " + cudaGetErrorString(e);
+    try {
+        g_last_cuda_error = std::string(what) + ": " + cudaGetErrorString(e);
+        g_last_static_error = nullptr;
+    } catch (const std::exception &) {  // no room for the text
+        g_last_static_error = cudaGetErrorString(e);
+    }
     cudaGetLastError();  // clear the sticky-free error so later calls start clean
 }
 
@@ -1032,7 +1036,7 @@ int b200spmm_csr2btcf_nobitmap(uint64_t rows, uint64_t cols, uint64_t nnz, const
     *out = nullptr;
     b200spmm_btcf *h = new (std::nothrow) b200spmm_btcf();
     if (!h) return B200SPMM_ERR_NO_MEMORY;
-    int st = convert_csr_to_btcf(rows, cols, nnz, row_ptr, col_idx, values, dtype, row_window, col_window, n_threads, &h->f);
+    int st = guarded([&]() { return convert_csr_to_btcf(rows, cols, nnz, row_ptr, col_idx, values, dtype, row_window, col_window, n_threads, &h->f); });
     if (st != B200SPMM_OK) {
         delete h;
         return st;
@@ -1043,8 +1047,10 @@ int b200spmm_csr2btcf_nobitmap(uint64_t rows, uint64_t cols, uint64_t nnz, const
 
 int b200spmm_btcf_transpose_tiles(b200spmm_btcf_t *f) {
     if (!f) return B200SPMM_ERR_INVALID_ARG;
-    transpose_tiles(&f->f);
-    return B200SPMM_OK;
+    return guarded([&]() -> int {
+        transpose_tiles(&f->f);
+        return B200SPMM_OK;
+    });
 }
 
 int b200spmm_btcf_tiles_col_major(const b200spmm_btcf_t *f) { return f && f->f.col_major_tiles ? 1 : 0; }
@@ -1058,8 +1064,10 @@ int b200spmm_btcf_rewindow(const b200spmm_btcf_info_t *info, const uint32_t *row
     if (rowOffset[info->eff_row_windows] != info->total_tiles) return B200SPMM_ERR_INVALID_ARG;
     b200spmm_btcf *h = new (std::nothrow) b200spmm_btcf();
     if (!h) return B200SPMM_ERR_NO_MEMORY;
-    int st = rewindow_btcf(info->rows, info->cols, info->nnzs, info->dtype, info->row_window, info->col_window,
-                           info->eff_row_windows, rowOffset, tcA2B, data, rowIdx, row_window, n_threads, &h->f);
+    int st = guarded([&]() {
+        return rewindow_btcf(info->rows, info->cols, info->nnzs, info->dtype, info->row_window, info->col_window,
+                             info->eff_row_windows, rowOffset, tcA2B, data, rowIdx, row_window, n_threads, &h->f);
+    });
     if (st != B200SPMM_OK) {
         delete h;
         return st;
@@ -1116,40 +1124,46 @@ int b200spmm_allgather_plan(const uint64_t *cut, int n_parts, uint64_t *even_par
 }
 
 int b200spmm_build_schedule(const uint32_t *rowOffset, uint64_t eff_row_windows, int n_ctas, uint32_t *cta_window) {
-    if (!rowOffset || !cta_window || n_ctas < 1) return B200SPMM_ERR_INVALID_ARG;
-    std::vector<uint32_t> cuts;
-    build_cta_schedule(rowOffset, eff_row_windows, n_ctas, &cuts);
-    std::memcpy(cta_window, cuts.data(), cuts.size() * sizeof(uint32_t));
-    return B200SPMM_OK;
+    return guarded([&]() -> int {
+        if (!rowOffset || !cta_window || n_ctas < 1) return B200SPMM_ERR_INVALID_ARG;
+        std::vector<uint32_t> cuts;
+        build_cta_schedule(rowOffset, eff_row_windows, n_ctas, &cuts);
+        std::memcpy(cta_window, cuts.data(), cuts.size() * sizeof(uint32_t));
+        return B200SPMM_OK;
+    });
 }
 
 int b200spmm_build_tile_schedule(const uint32_t *rowOffset, uint64_t eff_row_windows, int n_ctas, uint32_t *cta_tile,
                                  uint32_t *cta_wfirst, uint32_t *cta_wlast, uint32_t *slot_window) {
-    if (!rowOffset || !cta_tile || !cta_wfirst || !cta_wlast || !slot_window || n_ctas < 1) return B200SPMM_ERR_INVALID_ARG;
-    TileSchedule sc;
-    build_tile_schedule(rowOffset, eff_row_windows, n_ctas, /*allow_split=*/true, &sc);
-    std::memcpy(cta_tile, sc.tile.data(), sc.tile.size() * sizeof(uint32_t));
-    std::memcpy(cta_wfirst, sc.wfirst.data(), sc.wfirst.size() * sizeof(uint32_t));
-    std::memcpy(cta_wlast, sc.wlast.data(), sc.wlast.size() * sizeof(uint32_t));
-    for (int c = 0; c < n_ctas; ++c) {
-        slot_window[2 * c] = sc.head_slot[c] != kNoSlot ? sc.wfirst[c] : 0xFFFFFFFFu;
-        slot_window[2 * c + 1] = sc.tail_slot[c] != kNoSlot ? sc.wlast[c] : 0xFFFFFFFFu;
-    }
-    return B200SPMM_OK;
+    return guarded([&]() -> int {
+        if (!rowOffset || !cta_tile || !cta_wfirst || !cta_wlast || !slot_window || n_ctas < 1) return B200SPMM_ERR_INVALID_ARG;
+        TileSchedule sc;
+        build_tile_schedule(rowOffset, eff_row_windows, n_ctas, /*allow_split=*/true, &sc);
+        std::memcpy(cta_tile, sc.tile.data(), sc.tile.size() * sizeof(uint32_t));
+        std::memcpy(cta_wfirst, sc.wfirst.data(), sc.wfirst.size() * sizeof(uint32_t));
+        std::memcpy(cta_wlast, sc.wlast.data(), sc.wlast.size() * sizeof(uint32_t));
+        for (int c = 0; c < n_ctas; ++c) {
+            slot_window[2 * c] = sc.head_slot[c] != kNoSlot ? sc.wfirst[c] : 0xFFFFFFFFu;
+            slot_window[2 * c + 1] = sc.tail_slot[c] != kNoSlot ? sc.wlast[c] : 0xFFFFFFFFu;
+        }
+        return B200SPMM_OK;
+    });
 }
 
 int b200spmm_build_row_bands(const uint32_t *rowOffset, const uint32_t *rowIdx, uint64_t eff_row_windows, uint64_t rows,
                              int n_parts, int max_bands, uint32_t *band_chunk, uint64_t *band_row, int *n_bands) {
-    if (!rowOffset || !band_chunk || !band_row || !n_bands || n_parts < 1 || max_bands < 1 || (eff_row_windows && !rowIdx))
-        return B200SPMM_ERR_INVALID_ARG;
-    TileSchedule sc;
-    build_tile_schedule(rowOffset, eff_row_windows, n_parts, /*allow_split=*/true, &sc);
-    RowBands bands;
-    build_row_bands(sc, rowIdx, rows, (uint32_t)max_bands, &bands);
-    *n_bands = (int)bands.chunk.size() - 1;
-    std::memcpy(band_chunk, bands.chunk.data(), bands.chunk.size() * sizeof(uint32_t));
-    std::memcpy(band_row, bands.row.data(), bands.row.size() * sizeof(uint64_t));
-    return B200SPMM_OK;
+    return guarded([&]() -> int {
+        if (!rowOffset || !band_chunk || !band_row || !n_bands || n_parts < 1 || max_bands < 1 || (eff_row_windows && !rowIdx))
+            return B200SPMM_ERR_INVALID_ARG;
+        TileSchedule sc;
+        build_tile_schedule(rowOffset, eff_row_windows, n_parts, /*allow_split=*/true, &sc);
+        RowBands bands;
+        build_row_bands(sc, rowIdx, rows, (uint32_t)max_bands, &bands);
+        *n_bands = (int)bands.chunk.size() - 1;
+        std::memcpy(band_chunk, bands.chunk.data(), bands.chunk.size() * sizeof(uint32_t));
+        std::memcpy(band_row, bands.row.data(), bands.row.size() * sizeof(uint64_t));
+        return B200SPMM_OK;
+    });
 }
 
 void b200spmm_plan_destroy(b200spmm_plan_t *p) {
@@ -1213,7 +1227,11 @@ int b200spmm_plan_create(const b200spmm_btcf_t *h, int device, int n_ctas, b200s
     const Btcf &f = h->f;
     auto upload = [&](void **dst, const void *src, size_t bytes) -> int {
         B200_CUDA_TRY(pool_alloc_bytes(dst, std::max<size_t>(bytes, 16), nullptr));
-        if (bytes) B200_CUDA_TRY(upload_pageable(*dst, src, bytes));
+        if (bytes)
+            return guarded([&]() -> int {
+                B200_CUDA_TRY(upload_pageable(*dst, src, bytes));
+                return B200SPMM_OK;
+            });
         return B200SPMM_OK;
     };
     int st = upload((void **)&p->d_rowOffset, f.rowOffset.data(), f.rowOffset.size() * 4);
@@ -1221,7 +1239,7 @@ int b200spmm_plan_create(const b200spmm_btcf_t *h, int device, int n_ctas, b200s
     if (st == B200SPMM_OK) st = upload((void **)&p->d_rowIdx, f.rowIdx.data(), f.rowIdx.size() * 4);
     if (st == B200SPMM_OK) st = upload(&p->d_data, f.data.data(), f.data.size());
     if (st == B200SPMM_OK) st = plan_start(p);
-    if (st == B200SPMM_OK) st = plan_finish(p, f.rowOffset.data(), f.rowIdx.data(), n_ctas);
+    if (st == B200SPMM_OK) st = guarded([&]() { return plan_finish(p, f.rowOffset.data(), f.rowIdx.data(), n_ctas); });
     if (st != B200SPMM_OK) {
         b200spmm_plan_destroy(p);
         return st;
@@ -1255,7 +1273,7 @@ int b200spmm_plan_create_device(const b200spmm_btcf_info_t *info, const uint32_t
     p->info.elt_size = info->dtype == B200SPMM_F16 ? 2 : 4;
     int st = plan_start(p);
     if (st == B200SPMM_OK) st = plan_check_tables(p);
-    if (st == B200SPMM_OK) st = plan_finish(p, nullptr, nullptr, n_ctas);
+    if (st == B200SPMM_OK) st = guarded([&]() { return plan_finish(p, nullptr, nullptr, n_ctas); });
     if (st != B200SPMM_OK) {
         b200spmm_plan_destroy(p);
         return st;
@@ -1282,33 +1300,35 @@ static int super_window_info(const b200spmm_plan_t *p, const TallFormat &f, int 
 
 static int super_window_copy_to_host(const b200spmm_plan_t *p, const TallFormat &f, uint32_t *rowOffset, uint32_t *tcA2B,
                                      void *data, uint32_t *rowIdx) {
-    if (!p || !rowOffset || !tcA2B || !data || !rowIdx) return B200SPMM_ERR_INVALID_ARG;
-    if (!f.tiles) return B200SPMM_ERR_UNSUPPORTED;
-    B200_CUDA_TRY(cudaSetDevice(p->device));
-    const uint64_t cw = (uint64_t)p->info.col_window, parts = f.rows / 128u;
-    B200_CUDA_TRY(cudaMemcpy(rowOffset, f.d_rowOffset, (f.eff + 1) * 4, cudaMemcpyDeviceToHost));
-    B200_CUDA_TRY(cudaMemcpy(rowIdx, f.d_rowIdx, f.eff * 4, cudaMemcpyDeviceToHost));
-    B200_CUDA_TRY(cudaMemcpy(tcA2B, f.d_tcA2B, f.tiles * cw * 4, cudaMemcpyDeviceToHost));
-    // The device copy holds 128-row images as they lie in shared memory (the halves of a row swapped when
-    // row / 4 is odd), for 256-row windows per window first rows 0-127 of all its tiles, then rows 128-255:
-    // put the halves back and the images where the converter would have them.
-    std::vector<uint8_t> img(f.tiles * parts * 4096);
-    B200_CUDA_TRY(cudaMemcpy(img.data(), f.d_data, img.size(), cudaMemcpyDeviceToHost));
-    uint8_t *bytes = static_cast<uint8_t *>(data);
-    for (uint64_t g = 0; g < f.eff; ++g) {
-        const uint64_t first = rowOffset[g], n_tiles = rowOffset[g + 1] - first;
-        for (uint64_t part = 0; part < parts; ++part)
-            for (uint64_t t = 0; t < n_tiles; ++t) {
-                const uint8_t *src = img.data() + (first * parts + part * n_tiles + t) * 4096;
-                uint8_t *dst = bytes + ((first + t) * parts + part) * 4096;
-                for (uint32_t r = 0; r < 128; ++r) {
-                    const uint32_t flip = (r >> 2) & 1u;
-                    std::memcpy(dst + r * 32, src + r * 32 + (flip ? 16 : 0), 16);
-                    std::memcpy(dst + r * 32 + 16, src + r * 32 + (flip ? 0 : 16), 16);
+    return guarded([&]() -> int {
+        if (!p || !rowOffset || !tcA2B || !data || !rowIdx) return B200SPMM_ERR_INVALID_ARG;
+        if (!f.tiles) return B200SPMM_ERR_UNSUPPORTED;
+        B200_CUDA_TRY(cudaSetDevice(p->device));
+        const uint64_t cw = (uint64_t)p->info.col_window, parts = f.rows / 128u;
+        B200_CUDA_TRY(cudaMemcpy(rowOffset, f.d_rowOffset, (f.eff + 1) * 4, cudaMemcpyDeviceToHost));
+        B200_CUDA_TRY(cudaMemcpy(rowIdx, f.d_rowIdx, f.eff * 4, cudaMemcpyDeviceToHost));
+        B200_CUDA_TRY(cudaMemcpy(tcA2B, f.d_tcA2B, f.tiles * cw * 4, cudaMemcpyDeviceToHost));
+        // The device copy holds 128-row images as they lie in shared memory (the halves of a row swapped when
+        // row / 4 is odd), for 256-row windows per window first rows 0-127 of all its tiles, then rows 128-255:
+        // put the halves back and the images where the converter would have them.
+        std::vector<uint8_t> img(f.tiles * parts * 4096);
+        B200_CUDA_TRY(cudaMemcpy(img.data(), f.d_data, img.size(), cudaMemcpyDeviceToHost));
+        uint8_t *bytes = static_cast<uint8_t *>(data);
+        for (uint64_t g = 0; g < f.eff; ++g) {
+            const uint64_t first = rowOffset[g], n_tiles = rowOffset[g + 1] - first;
+            for (uint64_t part = 0; part < parts; ++part)
+                for (uint64_t t = 0; t < n_tiles; ++t) {
+                    const uint8_t *src = img.data() + (first * parts + part * n_tiles + t) * 4096;
+                    uint8_t *dst = bytes + ((first + t) * parts + part) * 4096;
+                    for (uint32_t r = 0; r < 128; ++r) {
+                        const uint32_t flip = (r >> 2) & 1u;
+                        std::memcpy(dst + r * 32, src + r * 32 + (flip ? 16 : 0), 16);
+                        std::memcpy(dst + r * 32 + 16, src + r * 32 + (flip ? 0 : 16), 16);
+                    }
                 }
-            }
-    }
-    return B200SPMM_OK;
+        }
+        return B200SPMM_OK;
+    });
 }
 
 int b200spmm_plan_tall_info(const b200spmm_plan_t *p, b200spmm_btcf_info_t *info) {
@@ -1429,7 +1449,7 @@ extern "C" {
 
 int b200spmm_spmm(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
                   void *stream_v) {
-    return spmm_launch(p, d_B, ldb, n, d_C, ldc, c_dtype, stream_v, -1);
+    return guarded([&]() { return spmm_launch(p, d_B, ldb, n, d_C, ldc, c_dtype, stream_v, -1); });
 }
 
 int b200spmm_fp16_spmm(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
@@ -1464,7 +1484,7 @@ int b200spmm_plan_sync(b200spmm_plan_t *p, void *stream_v) {
     return B200SPMM_OK;
 }
 
-int b200spmm_spmm_host(b200spmm_plan_t *p, const void *h_B, int64_t n, void *h_C, int c_dtype) {
+static int run_host(b200spmm_plan_t *p, const void *h_B, int64_t n, void *h_C, int c_dtype) {
     if (!p || !h_B || !h_C || n <= 0) return B200SPMM_ERR_INVALID_ARG;
     if (c_dtype != B200SPMM_C_F32 && c_dtype != B200SPMM_C_F16) return B200SPMM_ERR_INVALID_ARG;
     B200_CUDA_TRY(cudaSetDevice(p->device));
@@ -1554,6 +1574,10 @@ int b200spmm_spmm_host(b200spmm_plan_t *p, const void *h_B, int64_t n, void *h_C
     return b200spmm_plan_sync(p, nullptr);
 }
 
+int b200spmm_spmm_host(b200spmm_plan_t *p, const void *h_B, int64_t n, void *h_C, int c_dtype) {
+    return guarded([&]() { return run_host(p, h_B, n, h_C, c_dtype); });
+}
+
 int b200spmm_bench(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
                    int warmup, int runs, void *stream_v, float *total_ms) {
     if (!p || !total_ms || warmup < 0 || runs < 1) return B200SPMM_ERR_INVALID_ARG;
@@ -1588,7 +1612,7 @@ int b200spmm_kat_spmm_starved(b200spmm_plan_t *p, const void *d_B, int64_t ldb, 
     p->starve_gathers = true;
     p->wait_limit_ns = limit_ns;
     p->tmap_b_ptr = nullptr;  // a map encoded for a normal launch must not be reused, nor this one later
-    const int st = spmm_launch(p, d_B, ldb, n, d_C, ldc, B200SPMM_C_F32, stream, -1);
+    const int st = guarded([&]() { return spmm_launch(p, d_B, ldb, n, d_C, ldc, B200SPMM_C_F32, stream, -1); });
     p->starve_gathers = false;
     p->wait_limit_ns = kDeviceWaitLimitNs;
     p->tmap_b_ptr = nullptr;

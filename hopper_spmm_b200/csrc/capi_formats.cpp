@@ -3,6 +3,7 @@
 #include <new>
 
 #include "../../include/b200_spmm.h"
+#include "common.hpp"
 #include "handles.hpp"
 
 using namespace b200spmm;
@@ -16,8 +17,9 @@ int b200spmm_csr2btcf(uint64_t rows, uint64_t cols, uint64_t nnz, const uint32_t
     *out = nullptr;
     b200spmm_btcfb *h = new (std::nothrow) b200spmm_btcfb();
     if (!h) return B200SPMM_ERR_NO_MEMORY;
-    int st = convert_csr_to_btcf_bitmap(rows, cols, nnz, row_ptr, col_idx, values, dtype, row_window, col_window,
-                                        n_threads, &h->f);
+    int st = guarded([&]() {
+        return convert_csr_to_btcf_bitmap(rows, cols, nnz, row_ptr, col_idx, values, dtype, row_window, col_window, n_threads, &h->f);
+    });
     if (st != B200SPMM_OK) {
         delete h;
         return st;
@@ -56,7 +58,7 @@ int b200spmm_btcfb_expand(const b200spmm_btcfb_t *in, b200spmm_btcf_t **out) {
     *out = nullptr;
     b200spmm_btcf *h = new (std::nothrow) b200spmm_btcf();
     if (!h) return B200SPMM_ERR_NO_MEMORY;
-    int st = expand_bitmap(in->f, &h->f);
+    int st = guarded([&]() { return expand_bitmap(in->f, &h->f); });
     if (st != B200SPMM_OK) {
         delete h;
         return st;
@@ -117,7 +119,7 @@ int b200spmm_load_matrix(const char *path, int dtype, b200spmm_csr_t **out) {
     *out = nullptr;
     b200spmm_csr *h = new (std::nothrow) b200spmm_csr();
     if (!h) return B200SPMM_ERR_NO_MEMORY;
-    int st = load_matrix_market(path, dtype, &h->m);
+    int st = guarded([&]() { return load_matrix_market(path, dtype, &h->m); });
     if (st != B200SPMM_OK) {
         delete h;
         return st;

@@ -5,6 +5,8 @@
 
 #include <cuda_runtime.h>
 
+#include <exception>
+
 #include "../../include/b200_spmm.h"
 
 namespace b200spmm {
@@ -13,6 +15,17 @@ namespace b200spmm {
 void record_cuda_error(cudaError_t e, const char *what);
 // Same, for a fixed message: keeps the pointer, allocates nothing.
 void set_last_error_static(const char *message);
+
+// Runs the body of a C entry point.  What it throws - host memory or a thread that is not to be had - becomes a status:
+// an exception that leaves a C function ends the process.
+template <class Fn>
+int guarded(Fn &&body) noexcept {
+    try {
+        return body();
+    } catch (const std::exception &) {
+        return B200SPMM_ERR_NO_MEMORY;
+    }
+}
 
 // How long a device-side wait may spin before the kernel gives up (nanoseconds).
 constexpr unsigned long long kDeviceWaitLimitNs = 2000000000ull;

@@ -4,6 +4,7 @@
 #include <cstdint>
 #include <cstring>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <unordered_set>
 #include <vector>
@@ -90,7 +91,11 @@ cudaError_t upload_pageable(void *dst, const void *src, size_t bytes) {
         if (stream) cudaStreamDestroy(stream);
     };
     std::vector<std::thread> pool;
-    for (int t = 1; t < kUploadThreads; ++t) pool.emplace_back(worker, t);
+    pool.reserve(kUploadThreads);
+    try {
+        for (int t = 1; t < kUploadThreads; ++t) pool.emplace_back(worker, t);
+    } catch (const std::system_error &) {  // no more threads to be had: those there are move all of it
+    }
     worker(0);
     for (auto &th : pool) th.join();
     return (cudaError_t)failed.load();

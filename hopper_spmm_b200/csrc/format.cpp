@@ -6,6 +6,8 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <exception>
+#include <system_error>
 #include <thread>
 
 #include "../../include/b200_spmm.h"
@@ -30,21 +32,29 @@ void parallel_chunks(uint64_t n_items, uint64_t chunk, int n_threads, Fn fn) {
     uint64_t n_chunks = (n_items + chunk - 1) / chunk;
     if ((uint64_t)n_threads > n_chunks) n_threads = (int)std::max<uint64_t>(1, n_chunks);
     std::atomic<uint64_t> next{0};
+    std::atomic<bool> failed{false};
+    std::exception_ptr first;  // what a worker threw; an exception that leaves a thread ends the process
     auto worker = [&]() {
-        for (;;) {
-            uint64_t c = next.fetch_add(1);
-            if (c >= n_chunks) break;
-            fn(c * chunk, std::min(n_items, (c + 1) * chunk));
+        try {
+            for (;;) {
+                uint64_t c = next.fetch_add(1);
+                if (c >= n_chunks) break;
+                fn(c * chunk, std::min(n_items, (c + 1) * chunk));
+            }
+        } catch (...) {
+            if (!failed.exchange(true)) first = std::current_exception();
+            next = n_chunks;
         }
     };
-    if (n_threads == 1) {
-        worker();
-        return;
-    }
     std::vector<std::thread> pool;
     pool.reserve(n_threads);
-    for (int t = 0; t < n_threads; ++t) pool.emplace_back(worker);
+    try {
+        for (int t = 1; t < n_threads; ++t) pool.emplace_back(worker);
+    } catch (const std::system_error &) {  // no more threads to be had: those there are do the work
+    }
+    worker();
     for (auto &t : pool) t.join();
+    if (first) std::rethrow_exception(first);
 }
 
 // The sorted distinct columns of a window, and the place of a column among them.  Where the window's entries are

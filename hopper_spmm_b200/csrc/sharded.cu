@@ -203,9 +203,9 @@ void b200spmm_sharded_destroy(b200spmm_sharded_t *s) {
     delete s;
 }
 
-int b200spmm_sharded_create(uint64_t rows, uint64_t cols, uint64_t nnz, const uint32_t *row_ptr, const uint32_t *col_idx,
-                            const void *values, int dtype, const int *devices, int n_devices, uint64_t row_charge,
-                            b200spmm_sharded_t **out) {
+static int create_sharded(uint64_t rows, uint64_t cols, uint64_t nnz, const uint32_t *row_ptr, const uint32_t *col_idx,
+                          const void *values, int dtype, const int *devices, int n_devices, uint64_t row_charge,
+                          b200spmm_sharded_t **out) {
     if (!out) return B200SPMM_ERR_INVALID_ARG;
     *out = nullptr;
     if (!devices || n_devices < 1 || n_devices > 64 || !row_ptr || (nnz && (!col_idx || !values))) return B200SPMM_ERR_INVALID_ARG;
@@ -288,6 +288,12 @@ int b200spmm_sharded_create(uint64_t rows, uint64_t cols, uint64_t nnz, const ui
     return B200SPMM_OK;
 }
 
+int b200spmm_sharded_create(uint64_t rows, uint64_t cols, uint64_t nnz, const uint32_t *row_ptr, const uint32_t *col_idx,
+                            const void *values, int dtype, const int *devices, int n_devices, uint64_t row_charge,
+                            b200spmm_sharded_t **out) {
+    return guarded([&]() { return create_sharded(rows, cols, nnz, row_ptr, col_idx, values, dtype, devices, n_devices, row_charge, out); });
+}
+
 int b200spmm_sharded_info(const b200spmm_sharded_t *s, int *n_devices, uint64_t *row_begin) {
     if (!s) return B200SPMM_ERR_INVALID_ARG;
     if (n_devices) *n_devices = s->n_dev;
@@ -324,12 +330,14 @@ int b200spmm_allgather_c(b200spmm_sharded_t *s, void *const *d_C_full, int64_t n
     if (!s || !d_C_full || n <= 0) return B200SPMM_ERR_INVALID_ARG;
     if (c_dtype != B200SPMM_C_F32 && c_dtype != B200SPMM_C_F16) return B200SPMM_ERR_INVALID_ARG;
     const uint64_t row_bytes = (uint64_t)n * (c_dtype == B200SPMM_C_F32 ? 4 : 2);
-    std::vector<uint64_t> cut(s->row_begin);
-    for (auto &c : cut) c *= row_bytes;
-    return exchange_ranges(s, d_C_full, cut);
+    return guarded([&]() {
+        std::vector<uint64_t> cut(s->row_begin);
+        for (auto &c : cut) c *= row_bytes;
+        return exchange_ranges(s, d_C_full, cut);
+    });
 }
 
-int b200spmm_spmm_sharded_host(b200spmm_sharded_t *s, const void *h_B, int64_t n, void *h_C, int c_dtype) {
+static int run_sharded_host(b200spmm_sharded_t *s, const void *h_B, int64_t n, void *h_C, int c_dtype) {
     if (!s || !h_B || !h_C || n <= 0) return B200SPMM_ERR_INVALID_ARG;
     if (c_dtype != B200SPMM_C_F32 && c_dtype != B200SPMM_C_F16) return B200SPMM_ERR_INVALID_ARG;
     const uint64_t b_row = (uint64_t)n * s->elt_size, c_row = (uint64_t)n * (c_dtype == B200SPMM_C_F32 ? 4 : 2);
@@ -358,6 +366,10 @@ int b200spmm_spmm_sharded_host(b200spmm_sharded_t *s, const void *h_B, int64_t n
                                       s->streams[d]));
     }
     return b200spmm_sharded_sync(s);
+}
+
+int b200spmm_spmm_sharded_host(b200spmm_sharded_t *s, const void *h_B, int64_t n, void *h_C, int c_dtype) {
+    return guarded([&]() { return run_sharded_host(s, h_B, n, h_C, c_dtype); });
 }
 
 }  // extern "C"

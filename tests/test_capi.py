@@ -168,3 +168,34 @@ for B, C_out in ((Odd(torch.float16), None), (Odd(torch.float16), Odd(torch.floa
 """ % policy
     r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.count("raised") == 2, r.stderr
+
+
+def test_a_conversion_without_memory_or_threads_is_a_status():
+    # room for no thread's stack, for some of the threads, for their stacks but not for the column lists: whatever a
+    # worker throws comes back as a status, in a process that an exception leaving a thread or a C function would abort
+    code = """
+import resource
+import numpy as np
+import hopper_spmm_b200 as hs
+from hopper_spmm_b200 import _capi as capi
+capi.lib()
+rows, cols, per = 100000, 1000003, 40
+ci = np.arange(per, dtype=np.uint64) * 104729 + np.arange(rows, dtype=np.uint64)[:, None] * 7919
+ci = np.sort(ci % cols, axis=1).astype(np.uint32).ravel()
+m = hs.CSR_MTX(rows, cols, np.arange(rows + 1, dtype=np.uint32) * per, ci, np.ones(ci.size, np.float16))
+used = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+hard = resource.getrlimit(resource.RLIMIT_AS)[1]
+for mb in (1, 6, 20, 60, 100):
+    resource.setrlimit(resource.RLIMIT_AS, (used + (mb << 20), hard))
+    try:
+        hs.CSR2BTCFNOBITMAP(m, n_threads=8)
+        print("converted")
+    except capi.SpmmError as e:
+        print("status", e.status)
+resource.setrlimit(resource.RLIMIT_AS, (hard, hard))
+print("tiles", hs.CSR2BTCFNOBITMAP(m, n_threads=8).total_tiles > 0)
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    lines = r.stdout.split("\n")[:-1]
+    assert r.returncode == 0 and lines[0] == "status %d" % capi.ERR_NO_MEMORY and lines[-1] == "tiles True", r.stderr + r.stdout
+    assert set(lines[:-1]) <= {"status %d" % capi.ERR_NO_MEMORY, "converted"} and len(lines) == 6
