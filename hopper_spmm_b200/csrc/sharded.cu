@@ -267,6 +267,8 @@ static int create_sharded(uint64_t rows, uint64_t cols, uint64_t nnz, const uint
         if (e == cudaSuccess && part_nnz) e = cudaMemcpy(d_ci, col_idx + lo, part_nnz * 4, cudaMemcpyHostToDevice);
         if (e == cudaSuccess && part_nnz)
             e = cudaMemcpy(d_v, static_cast<const char *>(values) + lo * s->elt_size, part_nnz * s->elt_size, cudaMemcpyHostToDevice);
+        // a copy from pageable memory may return before it has arrived, and the conversion's stream does not wait for this one
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
         if (e != cudaSuccess) {
             drop();
             record_cuda_error(e, "uploading a shard's CSR");
