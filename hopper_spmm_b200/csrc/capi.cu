@@ -1575,7 +1575,13 @@ static int run_host(b200spmm_plan_t *p, const void *h_B, int64_t n, void *h_C, i
 }
 
 int b200spmm_spmm_host(b200spmm_plan_t *p, const void *h_B, int64_t n, void *h_C, int c_dtype) {
-    return guarded([&]() { return run_host(p, h_B, n, h_C, c_dtype); });
+    const int st = guarded([&]() { return run_host(p, h_B, n, h_C, c_dtype); });
+    if (st != B200SPMM_OK && p) {  // copies may have been started: they must not outlive the call, nor the caller's buffers
+        cudaStreamSynchronize(nullptr);
+        if (p->upload_stream) cudaStreamSynchronize(p->upload_stream);
+        if (p->copy_stream) cudaStreamSynchronize(p->copy_stream);
+    }
+    return st;
 }
 
 int b200spmm_bench(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,

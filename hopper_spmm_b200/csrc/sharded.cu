@@ -371,7 +371,11 @@ static int run_sharded_host(b200spmm_sharded_t *s, const void *h_B, int64_t n, v
 }
 
 int b200spmm_spmm_sharded_host(b200spmm_sharded_t *s, const void *h_B, int64_t n, void *h_C, int c_dtype) {
-    return guarded([&]() { return run_sharded_host(s, h_B, n, h_C, c_dtype); });
+    const int st = guarded([&]() { return run_sharded_host(s, h_B, n, h_C, c_dtype); });
+    if (st != B200SPMM_OK && s)  // copies may have been started: they must not outlive the call, nor the caller's buffers
+        for (int d = 0; d < s->n_dev; ++d)
+            if (cudaSetDevice(s->devices[d]) == cudaSuccess) cudaStreamSynchronize(s->streams[d]);
+    return st;
 }
 
 }  // extern "C"

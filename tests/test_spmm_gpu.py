@@ -216,6 +216,24 @@ def test_other_threads_run_while_a_launch_waits():
     assert sum(t0 < t < t1 for t in ticks) >= 5
 
 
+@pytest.mark.parametrize("rows", [300, 300_000])  # one product; bands of rows
+def test_a_refused_host_call_leaves_no_copy_behind(rows):
+    import torch
+    rng = np.random.default_rng(2)
+    cols, per = 3_000_000, 10
+    ci = np.sort(rng.integers(0, cols // per, (rows, per)) + np.arange(per) * (cols // per), axis=1).astype(np.uint32).ravel()
+    rp = (np.arange(rows + 1) * per).astype(np.uint32)
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, np.ones(ci.size, np.float16))))
+    try:
+        B = torch.zeros((cols, 36), dtype=torch.float16).pin_memory()  # 216 MB: the copy takes 4 ms; and 36 is no multiple of 8
+        with pytest.raises(capi.SpmmError) as e:
+            plan.spmm_host(B.numpy())
+        assert torch.cuda.default_stream().query()
+        assert e.value.status == capi.ERR_UNSUPPORTED
+    finally:
+        plan.close()
+
+
 def test_more_ctas_than_windows_and_one_cta():
     rows, cols, rp, ci, v = random_csr(96, 300, 0.1, 8)
     B = dense_b(cols, 64, 4)
