@@ -11,6 +11,7 @@
 // of the matrix: the arrays may be a caller's, and what lies in a padded slot or below the last row multiplies nothing.
 #include <algorithm>
 #include <cub/cub.cuh>
+#include <cuda_fp16.h>
 
 #include "common.hpp"
 #include "device_pool.hpp"
@@ -257,6 +258,37 @@ __global__ void band_units_kernel(const uint32_t *__restrict__ keys, const uint3
     out[i] = lo;
 }
 
+// v as first + n * unit, all three of v's sign, for the slots that fill a batch up: v's significand less n, and ones of its
+// last place.  Times a value of B and added one after the other, first to nothing, every partial sum has the 22 bits of a
+// product at most: the sum of the parts is the product, bit for bit, and infinite where it is.  (Zeros as fillers would make
+// zero times infinity of it.)  A subnormal of n units and less has no such parts: it is followed by zeros.
+__device__ __forceinline__ void split_value(uint16_t v, uint32_t n, uint16_t *first, uint16_t *unit) {
+    const uint32_t exp = (v >> 10) & 31u, sign = v & 0x8000u, m = (v & 1023u) | (exp ? 1024u : 0u);
+    *first = *unit = v;
+    if (exp == 31u || m == 0) return;
+    if (m <= n) {
+        *unit = 0;
+        return;
+    }
+    const float one = __uint_as_float((sign << 16) | ((max(exp, 1u) - 25u + 127u) << 23));
+    *first = __half_as_ushort(__float2half_rn(__half2float(__ushort_as_half(v)) - (float)n * one));
+    *unit = __half_as_ushort(__float2half_rn(one));
+}
+// the same for what a tf32 value has: ten bits behind the leading one
+__device__ __forceinline__ void split_value(uint32_t v, uint32_t n, uint32_t *first, uint32_t *unit) {
+    const uint32_t exp = (v >> 23) & 255u, sign = v & 0x80000000u, m = ((v >> 13) & 1023u) | (exp ? 1024u : 0u);
+    *first = *unit = v;
+    if (exp == 255u || m == 0) return;
+    if (m <= n) {
+        *unit = 0;
+        return;
+    }
+    const uint32_t e = max(exp, 1u);
+    const float one = __uint_as_float(sign | (e > 10u ? (e - 10u) << 23 : 1u << (e + 12u)));
+    *first = __float_as_uint(__uint_as_float(v) - (float)n * one);
+    *unit = __float_as_uint(one);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kBlock)
 write_entries_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B, const T *__restrict__ data,
@@ -278,11 +310,12 @@ write_entries_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__r
         // columns and values while the tile before is written: fetched at its first entry, one by one, they cost the warp
         // a round trip to L2 per entry (43 us of a matrix of 700,000 entries, 60,000 rows; now 32).
         uint32_t piece = min(at / cap, pieces_of(len, cap) - 1u), piece_end = (piece + 1) * cap;
+        uint32_t fill = (0u - min(len - piece * cap, cap)) % kUnitBatch;  // slots before the second entry of the unit
         uint32_t *out = batches + (uint64_t)unit[piece] * kWords;
         auto put = [&](uint32_t e, uint32_t col, T v) {
             uint32_t *words = out + (e / kUnitBatch) * (4 * kWords);
             words[e % kUnitBatch] = col;
-            reinterpret_cast<T *>(words + kUnitBatch)[e % kUnitBatch] = sizeof(T) == 2 ? v : (T)((uint32_t)v & 0xFFFFE000u);  // as the tensor core reads it
+            reinterpret_cast<T *>(words + kUnitBatch)[e % kUnitBatch] = v;
         };
         Piece<T> next;
         alignas(16) uint32_t next_cols[kPer];
@@ -304,16 +337,23 @@ write_entries_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__r
             for (uint32_t m = p.mask; m; m &= m - 1u) {  // (two or three steps a warp; one per column would be eight)
                 const int k = __ffs((int)m) - 1;
                 const uint32_t col = pick(cols, k);
-                const T v = p.pick(k);
+                const T v = sizeof(T) == 2 ? p.pick(k) : (T)((uint32_t)p.pick(k) & 0xFFFFE000u);  // as the tensor core reads it
                 if (k_out >= piece_end) {
                     piece = k_out / cap;
                     piece_end = (piece + 1) * cap;
                     out = batches + (uint64_t)unit[piece] * kWords;
+                    fill = (0u - min(len - piece * cap, cap)) % kUnitBatch;
                 }
                 const uint32_t e = k_out - piece * cap;
-                put(e, col, v);
-                if (++k_out == len)  // the row's last entry: fill its batch up
-                    for (uint32_t f = e + 1; f % kUnitBatch; ++f) put(f, col, (T)0);
+                ++k_out;
+                if (e || !fill) {
+                    put(e + fill, col, v);
+                    continue;
+                }
+                T first, one;
+                split_value(v, fill, &first, &one);
+                put(0, col, first);
+                for (uint32_t f = 1; f <= fill; ++f) put(f, col, one);
             }
         }
     }

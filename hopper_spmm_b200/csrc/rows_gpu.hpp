@@ -10,8 +10,8 @@
 
 namespace b200spmm {
 
-// A unit is a row, or a piece of a long one.  Its entries lie in consecutive batches of four; the last batch is
-// filled up with its last column and zero values.  A batch is kBatchWords 32-bit words: four columns, four
+// A unit is a row, or a piece of a long one.  Its entries lie in consecutive batches of four; the first batch is
+// filled up with parts of the unit's first value (split_value in rows_gpu.cu).  A batch is kBatchWords 32-bit words: four columns, four
 // values (fp16: two words, tf32: four, low 13 bits dropped), the target of the unit's sum in the unit's last
 // batch and kNoTarget in the others, padding to 16 bytes.
 constexpr uint32_t kMaxUnitEntries = 256;  // no unit is longer, see unit_entries_for

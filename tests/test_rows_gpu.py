@@ -45,6 +45,33 @@ def test_batches_units_and_pieces_at_their_edges(dt, n, monkeypatch):
         plan.close()
 
 
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+def test_infinities_in_b_reach_the_rows_that_meet_them(dt, monkeypatch):
+    # rows with every remainder of a batch, whole and cut (units of 64 entries); every column of B but the last few has
+    # an infinity in a row of its own: a row of C is infinite exactly where it has an entry there, and nowhere NaN
+    import torch
+    monkeypatch.setenv("B200SPMM_WINDOW", "rows")
+    cols, n = 200, 136
+    lengths = list(range(1, 14)) + [61, 62, 63, 64, 65, 66, 67, 129, 130, 131] + [3, 6, 1] * 9
+    rows, cols, rp, ci, v = rows_of_lengths(lengths, cols, 8, dt)
+    B = dense_b(cols, n, 4, dt)
+    hit = np.random.default_rng(5).permutation(cols)[:n - 4]
+    B[hit, np.arange(n - 4)] = np.where(np.arange(n - 4) % 2, np.inf, -np.inf).astype(dt)
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    try:
+        got = plan.spmm(torch.from_numpy(B).cuda()).cpu().numpy()
+    finally:
+        plan.close()
+    bits = (lambda x: x) if dt == np.float16 else (lambda x: (x.view(np.uint32) & np.uint32(0xFFFFE000)).view(np.float32))
+    for r in range(rows):
+        at = slice(rp[r], rp[r + 1])
+        terms = bits(v[at]).astype(np.float64)[:, None] * bits(B[ci[at]]).astype(np.float64)
+        want = terms.sum(0)
+        assert np.array_equal(got[r][np.isinf(want)], want[np.isinf(want)]), r
+        fin = np.isfinite(want)
+        assert (np.abs(got[r][fin] - want[fin]) <= len(terms) * 2.0 ** -23 * np.abs(terms).sum(0)[fin]).all(), r  # fp32 sums
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 5), (17, 1), (3, 4000)])
 def test_smallest_matrices(rows, cols, monkeypatch):
     monkeypatch.setenv("B200SPMM_WINDOW", "rows")
