@@ -98,7 +98,11 @@ struct b200spmm_plan {
     // A caller's column lists that are not as the converter makes them: only what takes any list may run, the 16-row
     // kernel without row boxes and the kernels that go by entries.
     bool loose_lists = false;
-    bool has_tile_path = false;  // schedule and tile image of the 16-row kernel are there, so kernels with bounded waits may run
+    bool has_tile_path = false;  // schedule and tile image of the 16-row kernel are there
+    // Launches of kernels with bounded waits whose status word no sync has read yet: of one stream, or more than that can
+    // be said about (a captured launch runs again without passing through the host).
+    enum class Unread { none, one_stream, any } unread = Unread::none;
+    unsigned long long unread_stream = 0;  // its id (a handle may come back as another stream)
     // Most tiles of the super-window format name one aligned group of CW consecutive rows of B: then B
     // is re-laid as shared-memory images at every launch (scratch of the plan, as large as B) and such a
     // tile's operand arrives by one bulk copy.
@@ -1367,6 +1371,25 @@ cudaError_t make_current(int device) {
     return e == cudaSuccess && now != device ? cudaSetDevice(device) : e;
 }
 
+// A kernel that may raise the status word goes to `stream`.
+void note_bounded_waits(b200spmm_plan_t *p, cudaStream_t stream) {
+    using Unread = b200spmm_plan::Unread;
+    if (p->unread == Unread::any) return;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    // (the default stream does not answer while another one is being captured: the launch will say so; and asking a stream
+    // for its id ends its capture)
+    const bool known = cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone &&
+                       cudaStreamGetId(stream, &id) == cudaSuccess;
+    if (!known) cudaGetLastError();
+    if (!known || (p->unread == Unread::one_stream && p->unread_stream != id)) {
+        p->unread = Unread::any;
+        return;
+    }
+    p->unread = Unread::one_stream;
+    p->unread_stream = id;
+}
+
 // The product, or one band of it (band < 0: every chunk; otherwise the chunks, rows and split
 // windows of that band of the schedule the launch selects - see b200spmm_plan::Sched).
 int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
@@ -1391,6 +1414,7 @@ int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, voi
         int st = plan_add_tile_path(p, 0);
         if (st != B200SPMM_OK) return st;
     }
+    note_bounded_waits(p, stream);
     if (band < 0 && use_tall(p, n)) return launch_tall(p, d_B, ldb, n, d_C, ldc, c_dtype, stream);
     SpmmParams prm{};
     prm.rowOffset = p->d_rowOffset;
@@ -1470,11 +1494,13 @@ int b200spmm_plan_sync(b200spmm_plan_t *p, void *stream_v) {
     if (!p) return B200SPMM_ERR_INVALID_ARG;
     B200_CUDA_TRY(cudaSetDevice(p->device));
     B200_CUDA_TRY(cudaStreamSynchronize(static_cast<cudaStream_t>(stream_v)));
-    // Row units wait for nothing.  Any other plan's word is read at every call: a captured launch runs again without
-    // passing here, and one on another stream may raise it after this call.
-    if (!p->has_tile_path) return B200SPMM_OK;
+    using Unread = b200spmm_plan::Unread;
+    if (p->unread == Unread::none) return B200SPMM_OK;  // (row units and the narrow kernel wait for nothing)
     uint32_t status = 0;
     B200_CUDA_TRY(cudaMemcpy(&status, p->d_status, sizeof(status), cudaMemcpyDeviceToHost));
+    unsigned long long id = 0;
+    if (p->unread == Unread::one_stream && cudaStreamGetId(static_cast<cudaStream_t>(stream_v), &id) == cudaSuccess && id == p->unread_stream)
+        p->unread = Unread::none;  // what was launched there is done, and read
     if (status) {
         // status and the hand-out counters, cleared before the caller can launch again (on any stream)
         B200_CUDA_TRY(cudaMemset(p->d_status, 0, 4 * sizeof(uint32_t)));

@@ -174,6 +174,10 @@ def test_a_time_out_is_reported_after_an_earlier_sync(how, monkeypatch):
             assert starve(launch, 200_000_000) == 0
             assert lib.b200spmm_plan_sync(plan._p, other.cuda_stream) == 0  # still waiting
             assert lib.b200spmm_plan_sync(plan._p, launch.cuda_stream) == capi.ERR_DEVICE_TIMEOUT
+            assert starve(launch, 5_000_000) == 0
+            torch.cuda.synchronize()
+            plan.spmm(B, dC, stream=other, sync=False)  # a launch on another stream in between
+            assert lib.b200spmm_plan_sync(plan._p, other.cuda_stream) == capi.ERR_DEVICE_TIMEOUT
         assert lib.b200spmm_plan_sync(plan._p, launch.cuda_stream) == 0  # reported once
         plan.spmm(B, dC)
         parity.check(dC.cpu().numpy(), rows, rp, ci, v, B.cpu().numpy())
