@@ -1549,6 +1549,9 @@ static int run_host(b200spmm_plan_t *p, const void *h_B, int64_t n, void *h_C, i
     // features: with the features cut in two halves, the first half of C goes out while the second
     // half of B comes in, and the host link carries both directions at once for the middle third of
     // the step.  Each half is a product of its own (B and C as views with the full leading dimension).
+    // The copy engines move a piece of a row at a time: 55 + 57 GB/s (in, out; 50 each way at once) for 256 bytes and whole
+    // rows, 51 + 53 (36) for 128 and 40 + 43 (20) for 64.  Halves of H bytes take H / in + H / both + H / out against 2 H / in +
+    // 2 H / out in one piece: 0.066 against 0.072 ns a byte for pieces of 128 bytes, 0.099 for 64.  So the line is at 128.
     const size_t esz = (size_t)p->info.elt_size, csz = c_dtype == B200SPMM_C_F32 ? 4 : 2;
     const int64_t n_first = n / 2;
     const bool halves = p->host_split && n % 16 == 0 && (size_t)n_first * esz >= 128;

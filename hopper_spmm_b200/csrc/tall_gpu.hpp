@@ -19,8 +19,8 @@ struct TallFormat {
 };
 
 // How many tiles the matrix would have with 128-row windows, as a fraction of its 16-row tiles,
-// estimated from up to `max_samples` super-windows spread over the matrix (their column lists are
-// copied from the device and merged on the host).  1/8 means every merged window kept the column
+// estimated from up to `max_samples` super-windows spread over the matrix (their distinct columns are
+// counted on the device, a bit per column).  1/8 means every merged window kept the column
 // list of its fullest part (executed work unchanged); 1 means nothing was shared (work x 8).
 // h_rowOffset / h_rowIdx are host copies of the 16-row arrays.  Returns a B200SPMM status.
 int estimate_tall_tile_ratio(const b200spmm_btcf_info_t &info, const uint32_t *h_rowOffset, const uint32_t *h_rowIdx,
