@@ -11,7 +11,6 @@
 // of the matrix: the arrays may be a caller's, and what lies in a padded slot or below the last row multiplies nothing.
 #include <algorithm>
 #include <cub/cub.cuh>
-#include <cuda_fp16.h>
 
 #include "common.hpp"
 #include "device_pool.hpp"
@@ -103,7 +102,7 @@ run_rows_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restri
         const uint32_t w = run_window[run], t0 = rowOffset[w] + (run - run_first[w]) * kRunTiles;
         const uint32_t end = rowOffset[w + 1], t1 = min(t0 + kRunTiles, end);
         alignas(16) uint32_t of[Piece<T>::kPer];
-        load_columns(of, tcA2B, t1 - 1, lane);
+        if (t1 == end) load_columns(of, tcA2B, end - 1, lane);
         uint32_t mine = 0;
         Piece<T> p;
         if (loose) {
@@ -259,34 +258,24 @@ __global__ void band_units_kernel(const uint32_t *__restrict__ keys, const uint3
 }
 
 // v as first + n * unit, all three of v's sign, for the slots that fill a batch up: v's significand less n, and ones of its
-// last place.  Times a value of B and added one after the other, first to nothing, every partial sum has the 22 bits of a
-// product at most: the sum of the parts is the product, bit for bit, and infinite where it is.  (Zeros as fillers would make
-// zero times infinity of it.)  A subnormal of n units and less has no such parts: it is followed by zeros.
-__device__ __forceinline__ void split_value(uint16_t v, uint32_t n, uint16_t *first, uint16_t *unit) {
-    const uint32_t exp = (v >> 10) & 31u, sign = v & 0x8000u, m = (v & 1023u) | (exp ? 1024u : 0u);
+// last place (tf32 has the same ten bits of it as fp16, thirteen places further up).  Times a value of B and added one after
+// the other, first to nothing, every partial sum has the 22 bits of a product at most: the sum of the parts is the product,
+// bit for bit, and infinite where it is.  (Zeros as fillers would make zero times infinity of it.)  A subnormal of n units
+// and less has no such parts: it is followed by zeros.
+template <typename T>
+__device__ __forceinline__ void split_value(T v, uint32_t n, T *first, T *unit) {
+    constexpr uint32_t kLow = sizeof(T) == 2 ? 0 : 13, kExp = sizeof(T) == 2 ? 31u : 255u;
+    const uint32_t exp = ((uint32_t)v >> (10 + kLow)) & kExp, sign = (uint32_t)v & ((kExp + 1) << (10 + kLow));
+    const uint32_t below = ((uint32_t)v >> kLow) & 1023u, m = below | (exp ? 1024u : 0u);
     *first = *unit = v;
-    if (exp == 31u || m == 0) return;
+    if (exp == kExp || m == 0) return;
     if (m <= n) {
         *unit = 0;
         return;
     }
-    const float one = __uint_as_float((sign << 16) | ((max(exp, 1u) - 25u + 127u) << 23));
-    *first = __half_as_ushort(__float2half_rn(__half2float(__ushort_as_half(v)) - (float)n * one));
-    *unit = __half_as_ushort(__float2half_rn(one));
-}
-// the same for what a tf32 value has: ten bits behind the leading one
-__device__ __forceinline__ void split_value(uint32_t v, uint32_t n, uint32_t *first, uint32_t *unit) {
-    const uint32_t exp = (v >> 23) & 255u, sign = v & 0x80000000u, m = ((v >> 13) & 1023u) | (exp ? 1024u : 0u);
-    *first = *unit = v;
-    if (exp == 255u || m == 0) return;
-    if (m <= n) {
-        *unit = 0;
-        return;
-    }
-    const uint32_t e = max(exp, 1u);
-    const float one = __uint_as_float(sign | (e > 10u ? (e - 10u) << 23 : 1u << (e + 12u)));
-    *first = __float_as_uint(__uint_as_float(v) - (float)n * one);
-    *unit = __float_as_uint(one);
+    // under a power of two the places are half as wide
+    *first = (T)((uint32_t)v - ((below >= n || exp <= 1 ? n : 2 * n - below) << kLow));
+    *unit = (T)(sign | (exp > 10 ? (exp - 10) << (10 + kLow) : 1u << (max(exp, 1u) - 1 + kLow)));
 }
 
 template <typename T>
@@ -346,14 +335,12 @@ write_entries_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__r
                 }
                 const uint32_t e = k_out - piece * cap;
                 ++k_out;
-                if (e || !fill) {
-                    put(e + fill, col, v);
-                    continue;
+                T value = v, one;
+                if (!e && fill) {
+                    split_value(v, fill, &value, &one);
+                    for (uint32_t f = 1; f <= fill; ++f) put(f, col, one);
                 }
-                T first, one;
-                split_value(v, fill, &first, &one);
-                put(0, col, first);
-                for (uint32_t f = 1; f <= fill; ++f) put(f, col, one);
+                put(e ? e + fill : 0u, col, value);
             }
         }
     }

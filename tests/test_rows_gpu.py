@@ -72,6 +72,34 @@ def test_infinities_in_b_reach_the_rows_that_meet_them(dt, monkeypatch):
         assert (np.abs(got[r][fin] - want[fin]) <= len(terms) * 2.0 ** -23 * np.abs(terms).sum(0)[fin]).all(), r  # fp32 sums
 
 
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+def test_a_row_of_one_entry_is_one_exact_product(dt, monkeypatch):
+    # its batch is filled up with parts of the value: every finite fp16 value; tf32 values of every exponent, about the
+    # powers of two.  Products of 11 bits by 11 are exact in fp32 (those of tf32 that stay normal are compared).
+    import torch
+    monkeypatch.setenv("B200SPMM_WINDOW", "rows")
+    if dt == np.float16:
+        v = np.arange(1, 65536, dtype=np.uint16).view(np.float16)
+    else:
+        low = np.array([0, 1, 2, 3, 4, 511, 512, 1022, 1023], np.uint32)
+        v = ((np.arange(255, dtype=np.uint32)[:, None] << 10 | low).ravel() << 13).view(np.float32)
+        v = np.concatenate([v, -v])
+    v = v[np.isfinite(v)]
+    rows, cols, n = v.size, 8, 16
+    ci = (np.arange(rows) % cols).astype(np.uint32)
+    B = dense_b(cols, n, 6, dt)
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, np.arange(rows + 1, dtype=np.uint32), ci, v)))
+    try:
+        got = plan.spmm(torch.from_numpy(B).cuda()).cpu().numpy()
+        assert plan.launch_info().stages == 0
+    finally:
+        plan.close()
+    b = B if dt == np.float16 else (B.view(np.uint32) & np.uint32(0xFFFFE000)).view(np.float32)
+    want = v.astype(np.float64)[:, None] * b[ci].astype(np.float64)
+    normal = (np.abs(want) >= 2.0 ** -104) & (np.abs(want) < 2.0 ** 127) | (dt == np.float16)  # (the last part's product too)
+    assert np.array_equal(got[normal], want[normal])
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 5), (17, 1), (3, 4000)])
 def test_smallest_matrices(rows, cols, monkeypatch):
     monkeypatch.setenv("B200SPMM_WINDOW", "rows")
