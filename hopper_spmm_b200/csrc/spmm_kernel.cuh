@@ -739,7 +739,7 @@ spmm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             }
             if (kTma) {
                 B200_PROF_T0();
-                // A list is ascending and distinct (padding 0xFFFFFFFF at its end): when its last entry is CW - 1 past
+                // Where row_boxes is set a list is ascending and distinct (padding 0xFFFFFFFF at its end): with its last entry CW - 1 past
                 // its first, the tile's rows of B are neighbours (a matrix of aligned blocks has no others) and come
                 // as boxes of CW rows, half or a quarter of the instructions and none of the gather's rate limit.
                 const uint32_t *list = slot_words + half * Cfg::kCW;
