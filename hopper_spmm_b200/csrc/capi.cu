@@ -505,7 +505,7 @@ int launch_rows(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void 
     const RowBand &from = f.bands[band < 0 ? 0 : band], &to = band < 0 ? f.bands.back() : f.bands[band + 1];
     RowsParams prm{};
     prm.batches = f.d_batches;
-    prm.units = f.d_units;
+    prm.units = band >= 0 && f.d_band_units ? f.d_band_units : f.d_units;
     prm.unit_begin = from.unit;
     prm.unit_end = to.unit;
     prm.empty_begin = from.empty;

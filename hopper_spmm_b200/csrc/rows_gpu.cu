@@ -4,8 +4,8 @@
 //      sixteen rows of its run (one 16-byte load per lane is half a tile row)
 //   2. per (window, row): running sums over the window's runs -> row lengths; scans over the rows -> the units,
 //      slots and bands
-//   3. units sorted by (band, length), longest first (CUB radix sort, a few key bits), their batches numbered in
-//      that order
+//   3. units sorted by length, longest first (CUB radix sort, a few key bits), their batches numbered in that order;
+//      where there are bands, the list once more with the bands apart
 //   4. the warps of step 1 write (column, value) to the place of their row's unit
 // A stored value is one whose bits are not all zero (an explicit zero adds nothing to a product), in a row and a column
 // of the matrix: the arrays may be a caller's, and what lies in a padded slot or below the last row multiplies nothing.
@@ -24,7 +24,10 @@ constexpr int kBlock = 256;
 // row of 10,000 entries: 419 us for write_entries_kernel with runs of 256 tiles).
 constexpr uint32_t kRunTiles = 16;
 constexpr uint32_t kMaxBands = 8;
-constexpr uint32_t kEmptyKey = kMaxBands << 9;  // sort key: rows without entries last, then the band, then the longest first
+constexpr uint32_t kEmptyKey = 512;  // sort key of the units: longest first, rows without entries last
+constexpr int kUnitKeyBits = 10;
+constexpr uint32_t kEmptyBandKey = kMaxBands;  // sort key of the bands: their units, then their rows without entries
+constexpr int kBandKeyBits = 4;
 constexpr uint32_t kMaxLenAt = 4 + 2 * (kMaxBands + 1);  // in the table of totals: the longest row
 constexpr uint64_t kMinBandedCost = 2000000;  // bands pay where one keeps the GPU busy for tens of microseconds
 // For the bands a row counts as this many entries: its store is 4 bytes a feature where a gathered entry is 2.
@@ -188,25 +191,25 @@ __global__ void row_bands_kernel(uint32_t rows, const unsigned long long *__rest
 }
 
 // one thread per row: sort keys of its units, and its line of the split table
-__global__ void unit_keys_kernel(const uint32_t *__restrict__ row_len, uint32_t rows, uint32_t cap, uint32_t bands,
+__global__ void unit_keys_kernel(const uint32_t *__restrict__ row_len, uint32_t rows, uint32_t cap,
                                  const unsigned long long *__restrict__ a, const unsigned long long *__restrict__ b,
-                                 const uint32_t *__restrict__ totals, uint32_t *__restrict__ keys, uint32_t *__restrict__ ids,
+                                 uint32_t *__restrict__ keys, uint32_t *__restrict__ ids,
                                  uint32_t *__restrict__ unit_row, RowSplit *__restrict__ splits) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= rows) return;
     const uint32_t len = row_len[r], n = pieces_of(len, cap), first = (uint32_t)a[r] - n;
-    uint32_t band = 0;
-    for (uint32_t k = 1; k < bands; ++k) band += r >= totals[4 + k * 2] ? 1u : 0u;
     for (uint32_t q = 0; q < n; ++q) {
         const uint32_t part = min(len - q * cap, cap);
-        keys[first + q] = (part ? 0u : kEmptyKey) | (band << 9) | (kMaxUnitEntries - part);
+        keys[first + q] = part ? kMaxUnitEntries - part : kEmptyKey;
         ids[first + q] = first + q;
         unit_row[first + q] = r;
     }
     if (n > 1) splits[(uint32_t)(b[r] >> 32) - 1] = RowSplit{r, (uint32_t)b[r] - n, (uint32_t)b[r]};
 }
 
-__device__ __forceinline__ uint32_t batches_of_key(uint32_t key) { return (kMaxUnitEntries - (key & 511u) + kUnitBatch - 1) / kUnitBatch; }
+__device__ __forceinline__ uint32_t batches_of_key(uint32_t key) {
+    return key == kEmptyKey ? 0u : (kMaxUnitEntries - key + kUnitBatch - 1) / kUnitBatch;
+}
 
 // Four neighbours of the sorted list form a quad and are stored batch by batch side by side (batch k of all four,
 // then batch k + 1): the groups of a warp, which walk neighbours, read their entries from the same lines.
@@ -218,12 +221,13 @@ __global__ void quad_lengths_kernel(const uint32_t *__restrict__ keys, uint32_t 
     quads[q] = most;  // (0 for q == n_quads: its place in the running sum is the total)
 }
 
-// place i of the sorted list: where the unit's batches lie, and the targets in them
+// place i of the sorted list: where the unit's batches lie, the targets in them, and the key of its band
 template <bool kTf32>
 __global__ void place_units_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ ids, const uint32_t *__restrict__ quads,
                                    uint32_t n_units, uint32_t cap, const uint32_t *__restrict__ unit_row, const uint32_t *__restrict__ row_len,
                                    const unsigned long long *__restrict__ a, const unsigned long long *__restrict__ b,
-                                   uint2 *__restrict__ units, uint32_t *__restrict__ unit_batch, uint32_t *__restrict__ batches) {
+                                   uint2 *__restrict__ units, uint32_t *__restrict__ unit_batch, uint32_t *__restrict__ batches,
+                                   uint32_t bands, const uint32_t *__restrict__ totals, uint32_t *__restrict__ band_keys) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_units) return;
     const uint32_t u = ids[i], r = unit_row[u], n = pieces_of(row_len[r], cap), first = quads[i >> 2] * 4 + (i & 3u);
@@ -231,6 +235,11 @@ __global__ void place_units_kernel(const uint32_t *__restrict__ keys, const uint
     const uint32_t n_batches = batches_of_key(keys[i]);
     units[i] = make_uint2(n_batches ? first : r, n_batches);
     unit_batch[u] = first;
+    if (bands > 1) {
+        uint32_t band = 0;
+        for (uint32_t k = 1; k < bands; ++k) band += r >= totals[4 + k * 2] ? 1u : 0u;
+        band_keys[i] = (n_batches ? 0u : kEmptyBandKey) | band;
+    }
     for (uint32_t k = 0; k < n_batches; ++k)
         batches[(uint64_t)(first + 4 * k) * kBatchWords<kTf32> + kTargetWord<kTf32>] =
             k + 1 < n_batches ? kNoTarget : n > 1 ? kSlotTarget | ((uint32_t)b[r] - n + q) : r;
@@ -240,7 +249,8 @@ __global__ void place_units_kernel(const uint32_t *__restrict__ keys, const uint
     }
 }
 
-// band k <= bands: the places of its first unit and of its first row without entries; and the number of batches
+// band k <= bands: the places of its first unit and of its first row without entries (keys: of the bands, or of the units
+// where there is one band); and the number of batches
 __global__ void band_units_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ quads, uint32_t n_units,
                                   uint32_t bands, uint32_t *__restrict__ out) {
     const uint32_t i = threadIdx.x, k = i >> 1;
@@ -248,7 +258,7 @@ __global__ void band_units_kernel(const uint32_t *__restrict__ keys, const uint3
         if (k == bands + 1 && !(i & 1u)) out[i] = 4 * quads[(n_units + 3) / 4];
         return;
     }
-    const uint32_t want = ((i & 1u) ? kEmptyKey : 0u) + (k << 9);
+    const uint32_t want = ((i & 1u) ? (bands > 1 ? kEmptyBandKey : kEmptyKey) : 0u) + k;
     uint32_t lo = 0, hi = n_units;
     while (lo < hi) {
         const uint32_t mid = lo + (hi - lo) / 2;
@@ -466,6 +476,7 @@ void free_narrow(NarrowFormat *f) {
 void free_rows(RowsFormat *r) {
     pool_free(r->d_batches);
     pool_free(r->d_units);
+    pool_free(r->d_band_units);
     pool_free(r->d_splits);
     *r = RowsFormat();
 }
@@ -594,14 +605,15 @@ int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
     while (h[4 + 2 * bands] != rows) ++bands;
     for (uint32_t k = 0; k <= bands; ++k) f.bands.push_back(RowBand{0, 0, h[5 + 2 * k], h[4 + 2 * k]});
 
-    // Every unit rounds up to a batch, every quad to its longest unit: up to three longest units for each band,
-    // as its lengths fall from first to last, and three more where a quad holds the end of one and the start of the next.
-    const uint64_t max_batches = f.nnz / kUnitBatch + f.n_units + kMaxBands * 6 * (kMaxUnitEntries / kUnitBatch) + 8;
+    // Every unit rounds up to a batch, every quad to its longest unit: up to three longest units in all, as the lengths
+    // fall from first to last, and three more where a quad holds the last units.
+    const uint64_t max_batches = f.nnz / kUnitBatch + f.n_units + 6 * (kMaxUnitEntries / kUnitBatch) + 8;
     if (max_batches > 0xFFFFFFFFull || f.n_slots >= kSlotTarget - 1) return B200SPMM_OK;
     const uint32_t words = info.elt_size == 2 ? kBatchWords<false> : kBatchWords<true>;
     uint32_t *keys[2] = {}, *ids[2] = {}, *unit_row = nullptr;
     cudaError_t e = pool_alloc(&f.d_batches, max_batches * words);
     if (e == cudaSuccess) e = pool_alloc(&f.d_units, f.n_units);
+    if (e == cudaSuccess && bands > 1) e = pool_alloc(&f.d_band_units, f.n_units);
     if (e == cudaSuccess) e = pool_alloc(&f.d_splits, f.n_splits);
     for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
         e = tmp.alloc(&keys[k], f.n_units);
@@ -614,31 +626,37 @@ int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
     }
     B200_CUDA_TRY(e);
     const uint32_t n_quads = (f.n_units + 3) / 4;
-    uint32_t *quads = nullptr, *unit_batch = keys[0];  // (free again once the pairs are sorted)
+    uint32_t *quads = nullptr, *unit_batch = keys[0], *band_keys = ids[0];  // (free again once the pairs are sorted)
     B200_CUDA_TRY(tmp.alloc(&quads, n_quads + 1));
-    const int key_bits = 13;
-    unit_keys_kernel<<<row_grid, kBlock>>>(row_len, rows, cap, bands, a, b, totals, keys[0], ids[0], unit_row, f.d_splits);
-    size_t sort_bytes = 0, batch_bytes = 0;
-    B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, keys[0], keys[1], ids[0], ids[1], (int64_t)f.n_units, 0, key_bits));
+    unit_keys_kernel<<<row_grid, kBlock>>>(row_len, rows, cap, a, b, keys[0], ids[0], unit_row, f.d_splits);
+    size_t sort_bytes = 0, batch_bytes = 0, band_bytes = 0;
+    B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, keys[0], keys[1], ids[0], ids[1], (int64_t)f.n_units, 0, kUnitKeyBits));
     B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, batch_bytes, quads, quads, (int64_t)n_quads + 1));
+    if (bands > 1)
+        B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, band_bytes, band_keys, unit_row, f.d_units, f.d_band_units, (int64_t)f.n_units, 0, kBandKeyBits));
     uint8_t *sort_tmp = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&sort_tmp, std::max(sort_bytes, batch_bytes)));
-    B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, keys[0], keys[1], ids[0], ids[1], (int64_t)f.n_units, 0, key_bits));
+    B200_CUDA_TRY(tmp.alloc(&sort_tmp, std::max({sort_bytes, batch_bytes, band_bytes})));
+    B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, keys[0], keys[1], ids[0], ids[1], (int64_t)f.n_units, 0, kUnitKeyBits));
     quad_lengths_kernel<<<(int)(n_quads / kBlock + 1), kBlock>>>(keys[1], f.n_units, n_quads, quads);
     B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(sort_tmp, batch_bytes, quads, quads, (int64_t)n_quads + 1));
     const int unit_grid = (int)((f.n_units + kBlock - 1) / kBlock);
     if (f16) {
         place_units_kernel<false><<<unit_grid, kBlock>>>(keys[1], ids[1], quads, f.n_units, cap, unit_row, row_len, a, b, f.d_units,
-                                                         unit_batch, f.d_batches);
+                                                         unit_batch, f.d_batches, bands, totals, band_keys);
         write_entries_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data16, d_rowIdx, run_first, run_window, eff, rows, cols, loose, cap,
                                                              counts, row_len, a, unit_batch, f.d_batches);
     } else {
         place_units_kernel<true><<<unit_grid, kBlock>>>(keys[1], ids[1], quads, f.n_units, cap, unit_row, row_len, a, b, f.d_units,
-                                                        unit_batch, f.d_batches);
+                                                        unit_batch, f.d_batches, bands, totals, band_keys);
         write_entries_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data32, d_rowIdx, run_first, run_window, eff, rows, cols, loose, cap,
                                                              counts, row_len, a, unit_batch, f.d_batches);
     }
-    band_units_kernel<<<1, 32>>>(keys[1], quads, f.n_units, bands, totals);
+    const uint32_t *sorted_bands = keys[1];
+    if (bands > 1) {  // (the units of a band keep their order)
+        B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sort_tmp, band_bytes, band_keys, unit_row, f.d_units, f.d_band_units, (int64_t)f.n_units, 0, kBandKeyBits));
+        sorted_bands = unit_row;
+    }
+    band_units_kernel<<<1, 32>>>(sorted_bands, quads, f.n_units, bands, totals);
     B200_CUDA_TRY(cudaGetLastError());
     B200_CUDA_TRY(cudaMemcpy(h, totals, (2 * bands + 3) * 4, cudaMemcpyDeviceToHost));
     for (uint32_t k = 0; k <= bands; ++k) {

@@ -27,8 +27,8 @@ struct RowSplit {
     uint32_t row, slot_begin, slot_end;
 };
 
-// A band of whole rows: where its units (longest first), its rows without entries (behind the units of all
-// bands), its cut rows and its rows begin.
+// A band of whole rows: where in the list of bands its units (longest first) and its rows without entries (behind
+// the units of all bands) begin, its cut rows and its rows.
 struct RowBand {
     uint32_t unit, empty, split;
     uint64_t row;
@@ -36,7 +36,8 @@ struct RowBand {
 
 struct RowsFormat {
     uint32_t *d_batches = nullptr;    // [n_batches + 1][kBatchWords], the last one belongs to nobody
-    uint2 *d_units = nullptr;         // [n_units] first batch and number of batches, or (row, 0) for one without entries
+    uint2 *d_units = nullptr;         // [n_units] first batch and number of batches, longest first, then (row, 0) for rows without entries
+    uint2 *d_band_units = nullptr;    // the same band by band, or null where there is one band
     RowSplit *d_splits = nullptr;     // [n_splits] by row
     uint64_t nnz = 0;
     uint32_t n_batches = 0, n_units = 0, n_splits = 0, n_slots = 0;

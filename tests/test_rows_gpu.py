@@ -100,6 +100,35 @@ def test_a_row_of_one_entry_is_one_exact_product(dt, monkeypatch):
     assert np.array_equal(got[normal], want[normal])
 
 
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+def test_bands_and_the_whole_walk_the_same_units(dt, monkeypatch):
+    # large enough for bands: the host call goes band by band through a list of its own, the device call through the list
+    # of all units; rows without entries in every band, hub rows cut into many pieces, a run of them at one end
+    import torch
+    monkeypatch.setenv("B200SPMM_WINDOW", "rows")
+    rng = np.random.default_rng(12)
+    lengths = rng.integers(0, 40, 130_007)
+    lengths[rng.random(lengths.size) < 0.1] = 0
+    lengths[rng.integers(0, lengths.size, 40)] = rng.integers(250, 1100, 40)
+    lengths[-5:] = 1001  # (2.5 million entries and rows: bands start at two)
+    cols, rp = 1201, np.concatenate([[0], np.cumsum(lengths)]).astype(np.uint32)
+    start = rng.integers(0, cols - lengths)
+    ci = (np.repeat(start - rp[:-1].astype(np.int64), lengths) + np.arange(rp[-1])).astype(np.uint32)  # neighbours: distinct, ascending
+    v = rng.uniform(0.1, 1, ci.size).astype(dt)
+    B = dense_b(cols, 24, 3, dt)
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(lengths.size, cols, rp, ci, v)))
+    try:
+        host = plan.spmm_host(B, np.full((lengths.size, 24), np.nan, np.float32))
+        assert plan.launch_info().kernel_launches > 2 and plan.launch_info().stages == 0  # bands
+        dC = torch.full((lengths.size, 24), float("nan"), device="cuda")
+        plan.spmm(torch.from_numpy(B).cuda(), dC)
+        assert plan.launch_info().kernel_launches == 2
+        assert np.array_equal(host, dC.cpu().numpy())
+        parity.check(host, lengths.size, rp, ci, v, B)
+    finally:
+        plan.close()
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 5), (17, 1), (3, 4000)])
 def test_smallest_matrices(rows, cols, monkeypatch):
     monkeypatch.setenv("B200SPMM_WINDOW", "rows")
