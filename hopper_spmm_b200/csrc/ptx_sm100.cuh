@@ -25,6 +25,19 @@ B200_DEVICE uint64_t global_timer_ns() {
     return t;
 }
 
+// The kernels of a product are launched with programmatic stream serialization (launch_after in capi.cu): a grid may
+// start once every block of the grid before it in the stream has ended, while that one's results are still on their way.
+// From this wait on they are visible.  Before it a kernel may read what the plan holds - made, and waited for, when
+// the plan was - and nothing else; and it writes nothing.  Every thread waits, so that a grid that has ended means that those
+// before it have too.
+B200_DEVICE void wait_for_grids_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// A load that may not go through the read-only path: what it reads may have been written since this grid started.
+B200_DEVICE uint4 ld_global_v4(const void *p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
 
 // ------------------------------------------------------------------ mbarrier
 

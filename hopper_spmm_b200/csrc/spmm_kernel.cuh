@@ -303,6 +303,7 @@ spmm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         ptx::tmem_alloc(ptx::smem_u32(tmem_slot), kTmemCols);
         ptx::tmem_relinquish_alloc_permit();
     }
+    ptx::wait_for_grids_before();
     ptx::tcgen05_fence_before_sync();
     __syncthreads();
     ptx::tcgen05_fence_after_sync();
@@ -1131,11 +1132,12 @@ struct SplitWindow {
 // One CTA per split window; thread t handles four consecutive features of one row at a time.
 __global__ void __launch_bounds__(256)
 spmm_fixup_kernel(const SplitWindow *__restrict__ splits, const uint32_t *__restrict__ piece_slots,
-                  const float *__restrict__ partial, const uint32_t *__restrict__ rowIdx, void *__restrict__ C,
+                  const float *partial, const uint32_t *__restrict__ rowIdx, void *C,
                   int64_t ldc, uint32_t rows, uint32_t n, uint32_t c_is_half) {
     const SplitWindow sp = splits[blockIdx.x];
     const uint32_t row0 = rowIdx[sp.window];
     const uint32_t vec_per_row = n / 4;
+    ptx::wait_for_grids_before();
     for (uint32_t idx = threadIdx.x; idx < kRowWindow * vec_per_row; idx += blockDim.x) {
         const uint32_t r = idx / vec_per_row, c4 = idx % vec_per_row;
         if (row0 + r >= rows) continue;

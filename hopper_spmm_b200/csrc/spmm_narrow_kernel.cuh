@@ -59,13 +59,6 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) spmm_narrow_kernel(const Na
 
     for (uint32_t g0 = 0; g0 < p.n_blocks; g0 += p.group_blocks) {
         const uint32_t g1 = min(g0 + p.group_blocks, p.n_blocks), col0 = g0 * kNarrowCols, n_cols = min(p.cols - col0, max_cols);
-        if (g0) __syncthreads();  // everybody is through with the group before
-        for (uint32_t i = threadIdx.x; i < n_cols * kVecs; i += kNarrowThreads) {
-            const uint32_t c = i / kVecs, v = i % kVecs;
-            ptx::cp_async_16(b_addr + v * plane + c * 16u,
-                             static_cast<const uint8_t *>(p.B) + (uint64_t)(col0 + c) * ((uint64_t)p.ldb * kEsz) + v * 16u, 16u);
-        }
-        ptx::cp_async_commit();
         uint32_t row = row0 + warp;
         uint32_t e = 0, end = 0, next_e = 0, next_end = 0;
         auto segment = [&](uint32_t r, uint32_t &lo, uint32_t &hi) {
@@ -88,6 +81,14 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) spmm_narrow_kernel(const Na
         segment(row, e, end);
         segment(row + kNarrowThreads / 32, next_e, next_end);
         load(w, e, end);
+        if (g0) __syncthreads();  // everybody is through with the group before
+        else ptx::wait_for_grids_before();
+        for (uint32_t i = threadIdx.x; i < n_cols * kVecs; i += kNarrowThreads) {
+            const uint32_t c = i / kVecs, v = i % kVecs;
+            ptx::cp_async_16(b_addr + v * plane + c * 16u,
+                             static_cast<const uint8_t *>(p.B) + (uint64_t)(col0 + c) * ((uint64_t)p.ldb * kEsz) + v * 16u, 16u);
+        }
+        ptx::cp_async_commit();
         ptx::cp_async_wait_group<0>();
         __syncthreads();
         for (; row < row1; row += kNarrowThreads / 32) {

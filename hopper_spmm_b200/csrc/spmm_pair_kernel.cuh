@@ -143,6 +143,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
         ptx::tmem_alloc_pair(ptx::smem_u32(tmem_slot), Cfg::kTmemCols);
         ptx::tmem_relinquish_alloc_permit_pair();
     }
+    ptx::wait_for_grids_before();
     ptx::tcgen05_fence_before_sync();
     __syncthreads();
     ptx::cluster_arrive();  // the other CTA's barriers exist before anything arrives on them

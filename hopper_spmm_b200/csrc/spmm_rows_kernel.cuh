@@ -20,6 +20,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include "ptx_sm100.cuh"
 #include "rows_gpu.hpp"
 
 namespace b200spmm {
@@ -110,8 +111,6 @@ __global__ void __launch_bounds__(kRowsThreads, kRowsBlocksPerSm) spmm_rows_kern
         else if (p.c_is_half) rowsdev::store_f16(static_cast<__half *>(p.C) + (int64_t)to * p.ldc + feat, acc);
         else rowsdev::store_f32(static_cast<float *>(p.C) + (int64_t)to * p.ldc + feat, acc);
     };
-    for (uint32_t k = p.empty_begin + first; k < p.empty_end; k += stride) store_row(__ldg(p.units + k).x);
-
     uint32_t u = p.unit_begin + first;
     auto load_unit = [&](uint32_t k) { return k < p.unit_end ? __ldg(p.units + k) : make_uint2(p.n_batches, 0xFFFFFFFFu); };
     const uint4 *batches = reinterpret_cast<const uint4 *>(p.batches);
@@ -123,11 +122,13 @@ __global__ void __launch_bounds__(kRowsThreads, kRowsBlocksPerSm) spmm_rows_kern
     };
     u += stride;
     fetch(unit.x);
+    ptx::wait_for_grids_before();
+    for (uint32_t k = p.empty_begin + first; k < p.empty_end; k += stride) store_row(__ldg(p.units + k).x);
     while (!__all_sync(0xffffffffu, unit.x == p.n_batches)) {  // a group that is through stays at the spare batch
         uint4 b[kUnitBatch];
         const uint32_t col[4] = {e[0].x, e[0].y, e[0].z, e[0].w};
 #pragma unroll
-        for (uint32_t k = 0; k < kUnitBatch; ++k) b[k] = __ldg(reinterpret_cast<const uint4 *>(Bf + (uint64_t)col[k] * pitch));
+        for (uint32_t k = 0; k < kUnitBatch; ++k) b[k] = ptx::ld_global_v4(Bf + (uint64_t)col[k] * pitch);
         uint32_t val[4], to;
         if constexpr (kTf32) {
             val[0] = e[1].x; val[1] = e[1].y; val[2] = e[1].z; val[3] = e[1].w;
@@ -159,11 +160,12 @@ __global__ void __launch_bounds__(kRowsThreads, kRowsBlocksPerSm) spmm_rows_kern
 // Adds the pieces of every cut row and writes the row of C.  One block per row: 8 runs of pieces (piece k
 // belongs to run k mod 8, whatever the width) times 32 lanes of four features.
 __global__ void __launch_bounds__(256)
-rows_fixup_kernel(const RowSplit *__restrict__ splits, const float *__restrict__ partial, void *__restrict__ C, int64_t ldc,
+rows_fixup_kernel(const RowSplit *__restrict__ splits, const float *partial, void *C, int64_t ldc,
                   uint32_t n, uint32_t c_is_half) {
     __shared__ float4 part[8][32];
     const RowSplit sp = splits[blockIdx.x];
     const uint32_t lane = threadIdx.x & 31u, run = threadIdx.x >> 5;
+    ptx::wait_for_grids_before();
     for (uint32_t f0 = 0; f0 < n; f0 += 128) {
         const uint32_t feat = f0 + lane * 4;
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);

@@ -223,6 +223,7 @@ spmm_tall_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
         ptx::tmem_alloc(ptx::smem_u32(tmem_slot), Cfg::kTmemCols);
         ptx::tmem_relinquish_alloc_permit();
     }
+    ptx::wait_for_grids_before();
     ptx::tcgen05_fence_before_sync();
     __syncthreads();
     ptx::tcgen05_fence_after_sync();
@@ -568,11 +569,12 @@ spmm_tall_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
 // zeros.  One thread per 16-byte piece.
 template <bool kTf32>
 __global__ void __launch_bounds__(256)
-pack_b_kernel(const uint8_t *__restrict__ B, int64_t ldb_bytes, uint32_t cols, uint32_t n, uint32_t kNs, uint32_t n_slabs,
-              uint32_t n_groups, uint8_t *__restrict__ packed) {
+pack_b_kernel(const uint8_t *B, int64_t ldb_bytes, uint32_t cols, uint32_t n, uint32_t kNs, uint32_t n_slabs,
+              uint32_t n_groups, uint8_t *packed) {
     constexpr uint32_t kCW = kTf32 ? 8 : 16, kEsz = kTf32 ? 4 : 2;
     const uint32_t row_pieces = kNs * kEsz / 16;                       // 16-byte pieces of one row of a slab
     const uint64_t total = (uint64_t)n_slabs * n_groups * kCW * row_pieces;
+    ptx::wait_for_grids_before();
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t piece = (uint32_t)(i % row_pieces);             // consecutive threads: consecutive pieces of a row
         uint64_t rest = i / row_pieces;
@@ -582,7 +584,7 @@ pack_b_kernel(const uint8_t *__restrict__ B, int64_t ldb_bytes, uint32_t cols, u
         const uint32_t row = group * kCW + k;
         const uint32_t feat_byte = (slab * kNs * kEsz) + piece * 16;   // byte offset inside the row of B
         uint4 v = make_uint4(0, 0, 0, 0);
-        if (row < cols && feat_byte < n * kEsz) v = *reinterpret_cast<const uint4 *>(B + (uint64_t)row * ldb_bytes + feat_byte);
+        if (row < cols && feat_byte < n * kEsz) v = ptx::ld_global_v4(B + (uint64_t)row * ldb_bytes + feat_byte);
         const uint32_t h = piece >> 3, cc = piece & 7u;                // 128-byte column block, piece inside it
         uint32_t off;
         if (kTf32) {

@@ -238,6 +238,50 @@ def test_a_refused_host_call_leaves_no_copy_behind(rows):
         plan.close()
 
 
+@pytest.mark.parametrize("how,n", [("rows", 40), ("16", 72), ("128", 128), ("256", 320), ("256", 72), (None, 8)])
+def test_each_product_of_a_chain_sees_the_one_before(how, n, monkeypatch):
+    # a launch may start before the one ahead of it in the stream has delivered: its B is that one's C here, with a kernel of
+    # torch's in between now and then, in a stream and in a graph; hub rows, so that some sums come from a second launch
+    import torch
+    if how:
+        monkeypatch.setenv("B200SPMM_WINDOW", how)
+    rng = np.random.default_rng(3)
+    size = 1500
+    lengths = rng.binomial(size, 0.12, size) if how != "rows" else rng.integers(1, 9, size)
+    lengths[[3, 700, 701]] = [size, size - 7, 900] if how else lengths[[3, 700, 701]]
+    ci = np.concatenate([np.sort(rng.choice(size, k, replace=False)) for k in lengths]).astype(np.uint32)
+    rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.uint32)
+    v = (rng.choice([-1, 1], ci.size) / np.repeat(np.sqrt(lengths), lengths)).astype(np.float16)
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(size, size, rp, ci, v)))
+    start = torch.from_numpy(dense_b(size, n, 4)).cuda()
+    steps = 24
+
+    def chain(out, wait):
+        x = start
+        for k in range(steps):
+            plan.spmm(x, out[k], c_half=True, sync=False)
+            if wait:
+                plan.sync()
+            x = out[k] if k % 5 else out[k] * 0.5
+        return out
+
+    try:
+        one_by_one = chain(torch.zeros(steps, size, n, dtype=torch.float16, device="cuda"), True)
+        assert one_by_one.isfinite().all() and one_by_one[-1].abs().max() > 0
+        for _ in range(5):
+            assert torch.equal(chain(torch.zeros_like(one_by_one), False), one_by_one)
+        g, out = torch.cuda.CUDAGraph(), torch.zeros_like(one_by_one)
+        with torch.cuda.graph(g):
+            chain(out, False)
+        for _ in range(3):
+            out.zero_()
+            g.replay()
+            assert torch.equal(out, one_by_one)
+        plan.sync()
+    finally:
+        plan.close()
+
+
 def test_more_ctas_than_windows_and_one_cta():
     rows, cols, rp, ci, v = random_csr(96, 300, 0.1, 8)
     B = dense_b(cols, 64, 4)
