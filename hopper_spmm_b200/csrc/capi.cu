@@ -507,6 +507,39 @@ bool use_rows(const b200spmm_plan *p, int64_t ldb) {
     return p->rows_only && ldb * p->info.elt_size <= 0xFFFFFFFFll;  // (the kernel's row pitch is 32-bit)
 }
 
+// How many of the longest units of a launch are walked by whole warps (spmm_rows_kernel<., true>).  They pay where the
+// longest unit would take longer than all the work does: a batch is a round trip to L2 of about 0.35 us, and an SM gets through
+// a warp's four entries a group in 0.025, so where the longest unit has a sixteenth of an SM's steps.  Then the units of
+// at least 2, 4, 8 ... batches, as many as half as many warps again as are resident allow: with twice that the blocks'
+// starts cost more than the chains.  4096 x 4096 at 1 %, 32 / 128 columns 4.9 -> 4.0 / 6.0 -> 5.2 us; 600 x 8000 at 2 %,
+// 128 columns (passes of 32) 12.8 -> 4.4; graphs of 2,000 nodes, 64 columns 7.3 -> 4.4 and of 10,000, 128 columns 9.5 -> 7.9;
+// but 8000 x 3000 at 1 %, 128 columns 6.5 -> 8.0 and 6000 x 6000 at 1 %, tf32, 64 columns 8.9 -> 10.2.
+// (Rows without entries are only stored, but by all warps; where they alone would fill the GPU, the launch has to.)
+uint32_t team_units(const b200spmm_plan *p, uint32_t n_units, uint32_t n_empty, uint32_t groups, uint32_t n_slabs) {
+    const RowsFormat &f = p->rows_fmt;
+    const uint64_t resident = (uint64_t)p->n_sms * kRowsWarpsPerSm, steps = (uint64_t)f.n_batches * n_slabs / groups / p->n_sms;
+    if (groups < 2 || 16ull * f.most_batches < steps || (uint64_t)n_empty / groups * n_slabs > resident) return 0;
+    for (uint32_t longest : f.long_units)
+        if (longest && 2 * ((uint64_t)longest + (n_units - longest) / groups) * n_slabs <= 3 * resident) return longest;
+    return 0;
+}
+
+int launch_rows_grid(b200spmm_plan *p, const RowsParams &prm, dim3 grid, void (*kernel)(const RowsParams), uint32_t s0, uint32_t s1,
+                     cudaStream_t stream) {
+    B200_CUDA_TRY(launch_after(kernel, grid, kRowsThreads, 0, 1, stream, prm));
+    p->last.n_ctas = (int)(grid.x * grid.y);
+    p->last.threads = kRowsThreads;
+    p->last.feature_slab = (int)slab_for(prm.n);  // (what a pass covers; teams share a pass out by features, too)
+    p->last.n_slabs = (int)((prm.n + slab_for(prm.n) - 1) / slab_for(prm.n));
+    p->last.row_window = kRowWindow;
+    p->last.kernel_launches = 1;
+    if (s1 == s0) return B200SPMM_OK;
+    B200_CUDA_TRY(launch_after(rows_fixup_kernel, dim3(s1 - s0), 256, 0, 1, stream, p->rows_fmt.d_splits + s0, (const float *)p->d_partial, prm.C,
+                               prm.ldc, prm.n, prm.c_is_half));
+    p->last.kernel_launches = 2;
+    return B200SPMM_OK;
+}
+
 int launch_rows(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
                 cudaStream_t stream, int band) {
     const RowsFormat &f = p->rows_fmt;
@@ -525,34 +558,45 @@ int launch_rows(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void 
     prm.ldb = ldb;
     prm.ldc = ldc;
     prm.n = (uint32_t)n;
-    prm.slab = slab_for(prm.n);
     prm.c_is_half = c_dtype == B200SPMM_C_F16;
     if (f.n_slots) {
         int st = grow_partial(p, (size_t)f.n_slots * (size_t)n);
         if (st != B200SPMM_OK) return st;
     }
     prm.partial = p->d_partial;
-    // a group of lanes for every kRowsGroupBatches batches, but enough of them for one wave where there are units for it
     const uint32_t vec = 16u / (uint32_t)p->info.elt_size;
-    const uint32_t n_slabs = (prm.n + prm.slab - 1) / prm.slab;
-    const uint32_t groups = 32u / (std::min(prm.slab, prm.n) / vec);
-    const uint32_t n_units = std::max(prm.unit_end - prm.unit_begin, prm.empty_end - prm.empty_begin), per_block = groups * (kRowsThreads / 32);
+    uint32_t n_slabs = 0, groups = 0;
+    auto set_slab = [&](uint32_t slab) {
+        prm.slab = slab;
+        n_slabs = (prm.n + slab - 1) / slab;
+        groups = 32u / (std::min(slab, prm.n) / vec);
+    };
+    const uint32_t whole = slab_for(prm.n), all_units = to.unit - from.unit, n_empty = prm.empty_end - prm.empty_begin;
+    uint32_t n_team = 0;
+    if (band < 0 && f.bands.size() == 2) {
+        set_slab(whole);
+        if (groups < 2) set_slab(whole / 2);  // (128 tf32 features take all lanes)
+        n_team = team_units(p, all_units, n_empty, groups, n_slabs);
+    }
+    if (n_team) {
+        // a pass shared out by features gives more groups a warp, down to 64 bytes of a row, while all warps are resident
+        while (n_team == all_units && prm.slab > 4 * vec && (uint64_t)all_units * n_slabs * 2 <= (uint64_t)p->n_sms * kRowsWarpsPerSm)
+            set_slab(prm.slab / 2);
+        const uint32_t warps = kRowsThreads / 32, rest = all_units - n_team;
+        prm.team_end = prm.unit_begin + n_team;
+        prm.team_blocks = (n_team + warps - 1) / warps;
+        const dim3 grid(prm.team_blocks + (rest + groups * warps - 1) / (groups * warps), n_slabs);
+        return launch_rows_grid(p, prm, grid, p->info.dtype == B200SPMM_TF32 ? spmm_rows_kernel<true, true> : spmm_rows_kernel<false, true>,
+                                from.split, to.split, stream);
+    }
+    set_slab(whole);
+    // a group of lanes for every kRowsGroupBatches batches, but enough of them for one wave where there are units for it
+    const uint32_t n_units = std::max(all_units, n_empty), per_block = groups * (kRowsThreads / 32);
     const uint64_t share = (uint64_t)f.n_batches * n_units / f.n_units / kRowsGroupBatches / per_block;
     const dim3 grid(std::min((n_units + per_block - 1) / per_block, std::max((uint32_t)share, (uint32_t)(p->n_sms * kRowsBlocksPerSm))), n_slabs);
-    p->last.n_ctas = (int)(grid.x * grid.y);
-    p->last.threads = kRowsThreads;
-    p->last.feature_slab = (int)prm.slab;
-    p->last.n_slabs = (int)n_slabs;
-    p->last.row_window = kRowWindow;
     if (!n_units) return B200SPMM_OK;
-    auto kernel = p->info.dtype == B200SPMM_TF32 ? spmm_rows_kernel<true> : spmm_rows_kernel<false>;
-    B200_CUDA_TRY(launch_after(kernel, grid, kRowsThreads, 0, 1, stream, prm));
-    p->last.kernel_launches = 1;
-    const uint32_t s0 = from.split, s1 = to.split;
-    if (s1 == s0) return B200SPMM_OK;
-    B200_CUDA_TRY(launch_after(rows_fixup_kernel, dim3(s1 - s0), 256, 0, 1, stream, f.d_splits + s0, p->d_partial, d_C, ldc, prm.n, prm.c_is_half));
-    p->last.kernel_launches = 2;
-    return B200SPMM_OK;
+    return launch_rows_grid(p, prm, grid, p->info.dtype == B200SPMM_TF32 ? spmm_rows_kernel<true, false> : spmm_rows_kernel<false, false>,
+                            from.split, to.split, stream);
 }
 
 // ---- narrow B

@@ -28,7 +28,7 @@ constexpr uint32_t kEmptyKey = 512;  // sort key of the units: longest first, ro
 constexpr int kUnitKeyBits = 10;
 constexpr uint32_t kEmptyBandKey = kMaxBands;  // sort key of the bands: their units, then their rows without entries
 constexpr int kBandKeyBits = 4;
-constexpr uint32_t kMaxLenAt = 4 + 2 * (kMaxBands + 1);  // in the table of totals: the longest row
+constexpr uint32_t kMaxLenAt = 4 + 2 * (kMaxBands + 1) + kLongUnits;  // in the table of totals: the longest row
 constexpr uint64_t kMinBandedCost = 2000000;  // bands pay where one keeps the GPU busy for tens of microseconds
 // For the bands a row counts as this many entries: its store is 4 bytes a feature where a gathered entry is 2.
 constexpr uint64_t kRowCost = 2;
@@ -250,15 +250,20 @@ __global__ void place_units_kernel(const uint32_t *__restrict__ keys, const uint
 }
 
 // band k <= bands: the places of its first unit and of its first row without entries (keys: of the bands, or of the units
-// where there is one band); and the number of batches
-__global__ void band_units_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ quads, uint32_t n_units,
-                                  uint32_t bands, uint32_t *__restrict__ out) {
-    const uint32_t i = threadIdx.x, k = i >> 1;
-    if (k > bands) {
-        if (k == bands + 1 && !(i & 1u)) out[i] = 4 * quads[(n_units + 3) / 4];
+// where there is one band); the number of batches; and how many units have at least 2 << j batches (unit_keys)
+__global__ void band_units_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ unit_keys, const uint32_t *__restrict__ quads,
+                                  uint32_t n_units, uint32_t bands, uint32_t *__restrict__ out) {
+    const uint32_t i = threadIdx.x, k = i >> 1, n_bounds = 2 * bands + 2;
+    if (i > n_bounds + kLongUnits) return;
+    if (i == n_bounds) {
+        out[i] = 4 * quads[(n_units + 3) / 4];
         return;
     }
-    const uint32_t want = ((i & 1u) ? (bands > 1 ? kEmptyBandKey : kEmptyKey) : 0u) + k;
+    uint32_t want = ((i & 1u) ? (bands > 1 ? kEmptyBandKey : kEmptyKey) : 0u) + k;
+    if (i > n_bounds) {  // the first key that stands for fewer batches
+        keys = unit_keys;
+        want = kMaxUnitEntries - kUnitBatch * ((2u << (i - n_bounds - 1)) - 1u);
+    }
     uint32_t lo = 0, hi = n_units;
     while (lo < hi) {
         const uint32_t mid = lo + (hi - lo) / 2;
@@ -656,9 +661,9 @@ int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
         B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sort_tmp, band_bytes, band_keys, unit_row, f.d_units, f.d_band_units, (int64_t)f.n_units, 0, kBandKeyBits));
         sorted_bands = unit_row;
     }
-    band_units_kernel<<<1, 32>>>(sorted_bands, quads, f.n_units, bands, totals);
+    band_units_kernel<<<1, 32>>>(sorted_bands, keys[1], quads, f.n_units, bands, totals);
     B200_CUDA_TRY(cudaGetLastError());
-    B200_CUDA_TRY(cudaMemcpy(h, totals, (2 * bands + 3) * 4, cudaMemcpyDeviceToHost));
+    B200_CUDA_TRY(cudaMemcpy(h, totals, (2 * bands + 3 + kLongUnits) * 4, cudaMemcpyDeviceToHost));
     for (uint32_t k = 0; k <= bands; ++k) {
         f.bands[k].unit = h[2 * k];
         f.bands[k].empty = h[2 * k + 1];
@@ -666,6 +671,8 @@ int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
     f.bands[bands].unit = f.bands[0].empty;  // (all units, then all rows without entries)
     f.bands[bands].empty = f.n_units;
     f.n_batches = h[2 * bands + 2];
+    f.most_batches = (std::min(h_max_len, cap) + kUnitBatch - 1) / kUnitBatch;
+    for (uint32_t k = 0; k < kLongUnits; ++k) f.long_units[k] = h[2 * bands + 3 + k];
     if (!force_rows && narrow_pays(f.nnz, rows, info.cols, h_max_len, n_sms)) {
         const int st = build_narrow(info, f.nnz, d_rowOffset, d_tcA2B, d_data, d_rowIdx, n_sms, run_first, run_window, run_grid, counts, a, narrow);
         if (st != B200SPMM_OK) return st;

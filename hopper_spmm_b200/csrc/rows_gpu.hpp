@@ -20,6 +20,7 @@ template <bool kTf32>
 constexpr uint32_t kBatchWords = kTf32 ? 12 : 8;
 template <bool kTf32>
 constexpr uint32_t kTargetWord = kTf32 ? 8 : 6;
+constexpr uint32_t kLongUnits = 5;
 constexpr uint32_t kSlotTarget = 0x80000000u, kNoTarget = 0xFFFFFFFFu;  // a row, or kSlotTarget | slot of a piece
 
 // A row that was cut: its pieces lie in slots [slot_begin, slot_end), in entry order.
@@ -41,6 +42,8 @@ struct RowsFormat {
     RowSplit *d_splits = nullptr;     // [n_splits] by row
     uint64_t nnz = 0;
     uint32_t n_batches = 0, n_units = 0, n_splits = 0, n_slots = 0;
+    uint32_t most_batches = 0;             // of a unit
+    uint32_t long_units[kLongUnits] = {};  // units of at least 2 << i batches
     std::vector<RowBand> bands;       // one more than there are bands: the last one holds the totals
 };
 

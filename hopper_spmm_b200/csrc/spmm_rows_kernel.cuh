@@ -30,6 +30,7 @@ struct RowsParams {
     const uint2 *units;               // first batch and number of batches, or a row without entries
     uint32_t unit_begin, unit_end;    // units with entries: their first batches
     uint32_t empty_begin, empty_end;  // rows without entries
+    uint32_t team_end, team_blocks;   // kTeams: units before team_end are walked by whole warps, of the first team_blocks blocks
     uint32_t n_batches;
     const void *B;              // [cols, n] row-major
     void *C;                    // [rows, n] row-major
@@ -47,6 +48,7 @@ struct RowsParams {
 constexpr int kRowsThreads = 64;
 constexpr int kRowsBlocksPerSm = 16;
 constexpr uint64_t kRowsGroupBatches = 16;
+constexpr uint32_t kRowsWarpsPerSm = kRowsBlocksPerSm * kRowsThreads / 32;
 
 namespace rowsdev {
 
@@ -88,7 +90,11 @@ __device__ __forceinline__ void store_f16(__half *dst, const float (&acc)[kN]) {
 
 }  // namespace rowsdev
 
-template <bool kTf32>
+// kTeams: in launches that leave the GPU half empty a unit is a chain of batches, each a round trip to L2, that too few
+// others hide.  There all groups of a warp share a unit - group t takes every groups-th batch from t on - and are summed
+// by shuffles (always in the same order).  It costs the loop registers and instructions, 8 % of a large launch, so it is a
+// kernel of its own; launch_rows has the rule and what it gives.
+template <bool kTf32, bool kTeams>
 __global__ void __launch_bounds__(kRowsThreads, kRowsBlocksPerSm) spmm_rows_kernel(const RowsParams p) {
     constexpr uint32_t kVec = kTf32 ? 4 : 8;  // features per lane: 16 bytes
     constexpr uint32_t kEsz = kTf32 ? 4 : 2;
@@ -101,30 +107,41 @@ __global__ void __launch_bounds__(kRowsThreads, kRowsBlocksPerSm) spmm_rows_kern
     const uint32_t feat = f0 + (live ? pos : 0u) * kVec;
     const uint8_t *Bf = static_cast<const uint8_t *>(p.B) + (size_t)feat * kEsz;
     const uint32_t pitch = (uint32_t)p.ldb * kEsz;
-    const uint32_t stride = gridDim.x * (kRowsThreads / 32) * groups;
-    const uint32_t first = (blockIdx.x * (kRowsThreads / 32) + warp) * groups + g;
+    const uint32_t everyone = gridDim.x * (kRowsThreads / 32) * groups;
+    const uint32_t me = (blockIdx.x * (kRowsThreads / 32) + warp) * groups + g;
+    const bool team = kTeams && blockIdx.x < p.team_blocks;
+    const uint32_t step = team ? groups : 1u, t = team ? g : 0u;  // groups that share a unit, and which of them this one is
+    uint32_t stride = everyone, first = p.unit_begin + me, end = p.unit_end;
+    if (kTeams) {
+        const uint32_t warps = kRowsThreads / 32, block = team ? blockIdx.x : blockIdx.x - p.team_blocks;
+        stride = (team ? p.team_blocks : (gridDim.x - p.team_blocks) * groups) * warps;
+        first = team ? p.unit_begin + block * warps + warp : p.team_end + (block * warps + warp) * groups + g;
+        if (team) end = p.team_end;
+    }
 
     float acc[kVec] = {};
     auto store_row = [&](uint32_t to) {
-        if (!live) return;
+        if (!live || (kTeams && to == kNoTarget)) return;
         if (to & kSlotTarget) rowsdev::store_f32(p.partial + (size_t)(to & ~kSlotTarget) * p.n + feat, acc);
         else if (p.c_is_half) rowsdev::store_f16(static_cast<__half *>(p.C) + (int64_t)to * p.ldc + feat, acc);
         else rowsdev::store_f32(static_cast<float *>(p.C) + (int64_t)to * p.ldc + feat, acc);
     };
-    uint32_t u = p.unit_begin + first;
-    auto load_unit = [&](uint32_t k) { return k < p.unit_end ? __ldg(p.units + k) : make_uint2(p.n_batches, 0xFFFFFFFFu); };
+    uint32_t u = first;
+    auto load_unit = [&](uint32_t k) { return k < end ? __ldg(p.units + k) : make_uint2(p.n_batches, kTeams ? 0u : 0xFFFFFFFFu); };
     const uint4 *batches = reinterpret_cast<const uint4 *>(p.batches);
     uint2 unit = load_unit(u), next = load_unit(u + stride);
     uint4 e[kQ];  // entries of the next batch
-    auto fetch = [&](uint32_t at) {
+    auto fetch = [&]() {
+        // (a group of a team has nothing to fetch where fewer batches than groups are left)
+        const uint32_t at = !kTeams ? unit.x : t < unit.y ? unit.x + 4u * t : p.n_batches;
 #pragma unroll
         for (uint32_t k = 0; k < kQ; ++k) e[k] = __ldg(batches + (uint64_t)at * kQ + k);
     };
     u += stride;
-    fetch(unit.x);
+    fetch();
     ptx::wait_for_grids_before();
-    for (uint32_t k = p.empty_begin + first; k < p.empty_end; k += stride) store_row(__ldg(p.units + k).x);
-    while (!__all_sync(0xffffffffu, unit.x == p.n_batches)) {  // a group that is through stays at the spare batch
+    for (uint32_t k = p.empty_begin + me; k < p.empty_end; k += everyone) store_row(__ldg(p.units + k).x);
+    while (!__all_sync(0xffffffffu, kTeams ? unit.y == 0 : unit.x == p.n_batches)) {  // a group that is through stays at the spare batch
         uint4 b[kUnitBatch];
         const uint32_t col[4] = {e[0].x, e[0].y, e[0].z, e[0].w};
 #pragma unroll
@@ -138,18 +155,47 @@ __global__ void __launch_bounds__(kRowsThreads, kRowsBlocksPerSm) spmm_rows_kern
             to = e[1].z;
         }
         // the batch behind this one, or the first one of the next unit
-        const bool last = --unit.y == 0;
+        const uint32_t left = unit.y;  // batches of the unit, this one and those of the other groups of a team among them
+        bool last;
+        if (kTeams) {
+            last = left <= step;
+            unit.x += 4u * step;
+            unit.y -= step;
+        } else {
+            last = --unit.y == 0;
+        }
         if (last) {
             unit = next;
             u += stride;
             next = load_unit(u);
-        } else if (unit.x != p.n_batches) {
+        } else if (!kTeams && unit.x != p.n_batches) {
             unit.x += 4;
         }
-        fetch(unit.x);
+        fetch();
+        if (!kTeams || t < left) {
 #pragma unroll
-        for (uint32_t k = 0; k < kUnitBatch; ++k) rowsdev::accumulate<kTf32>(acc, b[k], val[k]);
+            for (uint32_t k = 0; k < kUnitBatch; ++k) rowsdev::accumulate<kTf32>(acc, b[k], val[k]);
+        }
         if (last) {
+            if (kTeams && left == 0) to = kNoTarget;  // (through)
+            if (team) {
+                to = __shfl_sync(0xffffffffu, to, (left - 1) * lanes);  // the group of the last batch knows the target
+                if ((lanes & (lanes - 1)) == 0) {
+                    for (uint32_t o = lanes; o < 32; o *= 2) {
+#pragma unroll
+                        for (uint32_t k = 0; k < kVec; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+                    }
+                } else {
+                    float sum[kVec] = {};
+                    for (uint32_t j = 0; j < groups; ++j) {
+#pragma unroll
+                        for (uint32_t k = 0; k < kVec; ++k) sum[k] += __shfl_sync(0xffffffffu, acc[k], j * lanes + pos);
+                    }
+#pragma unroll
+                    for (uint32_t k = 0; k < kVec; ++k) acc[k] = sum[k];
+                }
+                if (g != 0) to = kNoTarget;
+            }
             store_row(to);
 #pragma unroll
             for (uint32_t k = 0; k < kVec; ++k) acc[k] = 0.f;

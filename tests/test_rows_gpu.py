@@ -46,6 +46,36 @@ def test_batches_units_and_pieces_at_their_edges(dt, n, monkeypatch):
 
 
 @pytest.mark.parametrize("dt", [np.float16, np.float32])
+@pytest.mark.parametrize("n", [8, 40, 72, 128, 136])
+@pytest.mark.parametrize("fill", [0, 0.7, 1.1])
+def test_units_walked_by_warps_and_by_groups(dt, n, fill, monkeypatch):
+    # long rows of every remainder of a batch and of a warp's groups, among so many short ones that whole warps take all units,
+    # the long ones, or none: short rows of up to two batches, `fill` times as many as the GPU's resident warps hold
+    import torch
+    monkeypatch.setenv("B200SPMM_WINDOW", "rows")
+    lanes = min(n, 128, 256 // np.dtype(dt).itemsize) * np.dtype(dt).itemsize // 16  # (of a pass: at least two groups a warp)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n_short = int(fill * sms * 32 * (32 // lanes) / -(-n // 128))
+    lengths = np.concatenate([[0, 200, 0], np.arange(9, 45), [61, 64, 65, 100, 129, 255, 256, 0], np.arange(n_short) % 8 + 1])
+    cols = 1013
+    rng = np.random.default_rng(n)
+    rp = np.concatenate([[0], np.cumsum(lengths)])
+    ci = (np.repeat(rng.integers(0, cols - lengths) - rp[:-1], lengths) + np.arange(rp[-1])).astype(np.uint32)
+    v = (rng.choice([-1, 1], ci.size) * rng.uniform(0.1, 1, ci.size)).astype(dt)
+    rp = rp.astype(np.uint32)
+    B = dense_b(cols, n, 9, dt)
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(lengths.size, cols, rp, ci, v)))
+    try:
+        dC = torch.full((lengths.size, n), float("nan"), device="cuda")
+        plan.spmm(torch.from_numpy(B).cuda(), dC)
+        assert plan.launch_info().stages == 0
+        parity.check(dC.cpu().numpy(), lengths.size, rp, ci, v, B)
+        assert torch.equal(plan.spmm(torch.from_numpy(B).cuda()), dC)
+    finally:
+        plan.close()
+
+
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
 def test_infinities_in_b_reach_the_rows_that_meet_them(dt, monkeypatch):
     # rows with every remainder of a batch, whole and cut (units of 64 entries); every column of B but the last few has
     # an infinity in a row of its own: a row of C is infinite exactly where it has an entry there, and nowhere NaN
