@@ -324,7 +324,7 @@ int convert_by_windows(b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const uint3
     B200_CUDA_TRY(tmp.alloc(&scan_tmp, scan_bytes));
     B200_CUDA_TRY(pool_alloc(&f->d_rowOffset, (size_t)n_windows + 1, stream));
     B200_CUDA_TRY(pool_alloc(&f->d_rowIdx, n_windows, stream));
-    if (smem > 48 * 1024)
+    if (smem > 47 * 1024)  // (48 KB hold the kernel's own shared variables, too)
         B200_CUDA_TRY(cudaFuncSetAttribute(window_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBitsSmemMax));
     const unsigned grid = std::min<uint32_t>(n_windows, 148 * 64), table_grid = n_windows / kBlock + 1;
     B200_CUDA_TRY(cudaMemsetAsync(totals, 0, sizeof(Totals), stream));

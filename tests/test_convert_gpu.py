@@ -100,3 +100,18 @@ def test_window_by_window_and_through_the_sort(dt, rows, cols, per_row):
         with pytest.raises(capi.SpmmError) as e:
             device_convert(rows, cols, r, c, v)
         assert e.value.status == capi.ERR_BAD_CSR
+
+
+def test_bit_set_that_just_fits_48_kb():
+    # with the kernel's own shared variables it does not: in a process where no larger set has run before
+    import subprocess
+    import sys
+    code = """if True:
+        import numpy as np, torch, hopper_spmm_b200 as hs
+        cols, ci = 348_519, np.arange(17, 348_519, 500, dtype=np.int32)
+        d = lambda a: torch.from_numpy(a).cuda()
+        dev = hs.DeviceBtcf(1, cols, d(np.array([0, ci.size], np.int32)), d(ci), d(np.ones(ci.size, np.float16)))
+        got = dev.to_host()["tcA2B"]
+        assert np.array_equal(got[:ci.size], ci.view(np.uint32)) and (got[ci.size:] == 0xFFFFFFFF).all()
+    """
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300)
