@@ -510,8 +510,9 @@ bool use_rows(const b200spmm_plan *p, int64_t ldb) {
 // How many of the longest units of a launch are walked by whole warps (spmm_rows_kernel<., true>).  They pay where the
 // longest unit would take longer than all the work does: a batch is a round trip to L2 of about 0.35 us, and an SM gets through
 // a warp's four entries a group in 0.025, so where the longest unit has a sixteenth of an SM's steps.  Then the units of
-// at least 2, 4, 8 ... batches, as many as half as many warps again as are resident allow: with twice that the blocks'
-// starts cost more than the chains.  4096 x 4096 at 1 %, 32 / 128 columns 4.9 -> 4.0 / 6.0 -> 5.2 us; 600 x 8000 at 2 %,
+// at least 2, 4, 8 ... batches, as many as are resident at one time and leave the launch with at most half as many warps
+// again: where all are teams and start in two waves, the starts cost more than the chains (6578 x 2298 at 2.5 %, 80 columns
+// 8.5 -> 9.4).  4096 x 4096 at 1 %, 32 / 128 columns 4.9 -> 4.0 / 6.0 -> 5.2 us; 600 x 8000 at 2 %,
 // 128 columns (passes of 32) 12.8 -> 4.4; graphs of 2,000 nodes, 64 columns 7.3 -> 4.4 and of 10,000, 128 columns 9.5 -> 7.9;
 // but 8000 x 3000 at 1 %, 128 columns 6.5 -> 8.0 and 6000 x 6000 at 1 %, tf32, 64 columns 8.9 -> 10.2.
 // (Rows without entries are only stored, but by all warps; where they alone would fill the GPU, the launch has to.)
@@ -520,7 +521,8 @@ uint32_t team_units(const b200spmm_plan *p, uint32_t n_units, uint32_t n_empty, 
     const uint64_t resident = (uint64_t)p->n_sms * kRowsWarpsPerSm, steps = (uint64_t)f.n_batches * n_slabs / groups / p->n_sms;
     if (groups < 2 || 16ull * f.most_batches < steps || (uint64_t)n_empty / groups * n_slabs > resident) return 0;
     for (uint32_t longest : f.long_units)
-        if (longest && 2 * ((uint64_t)longest + (n_units - longest) / groups) * n_slabs <= 3 * resident) return longest;
+        if (longest && (uint64_t)longest * n_slabs <= resident && 2 * ((uint64_t)longest + (n_units - longest) / groups) * n_slabs <= 3 * resident)
+            return longest;
     return 0;
 }
 

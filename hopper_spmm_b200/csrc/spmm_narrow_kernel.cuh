@@ -80,7 +80,6 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) spmm_narrow_kernel(const Na
         };
         segment(row, e, end);
         segment(row + kNarrowThreads / 32, next_e, next_end);
-        load(w, e, end);
         if (g0) __syncthreads();  // everybody is through with the group before
         else ptx::wait_for_grids_before();
         for (uint32_t i = threadIdx.x; i < n_cols * kVecs; i += kNarrowThreads) {
@@ -89,6 +88,7 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) spmm_narrow_kernel(const Na
                              static_cast<const uint8_t *>(p.B) + (uint64_t)(col0 + c) * ((uint64_t)p.ldb * kEsz) + v * 16u, 16u);
         }
         ptx::cp_async_commit();
+        load(w, e, end);
         ptx::cp_async_wait_group<0>();
         __syncthreads();
         for (; row < row1; row += kNarrowThreads / 32) {
