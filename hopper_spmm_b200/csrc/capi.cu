@@ -427,7 +427,7 @@ int launch_tall_one(b200spmm_plan *p, TallParams &prm, cudaStream_t stream) {
         configured_device = p->device;
     }
     prm.n_slabs = (prm.n + kNs - 1) / kNs;
-    prm.n_items = prm.eff_row_windows * prm.n_slabs;
+    prm.n_items = prm.eff_row_windows * prm.n_slabs * prm.parts;
     const int n_ctas = (int)std::min<uint32_t>(prm.n_items, (uint32_t)p->n_sms);
     B200_CUDA_TRY(launch_after(kernel, dim3(n_ctas), Cfg::kThreads, Cfg::kSmemBytes, 1, stream, p->tmap_b, p->tmap_bt, prm));
     p->last.n_ctas = n_ctas;
@@ -448,7 +448,7 @@ int launch_pair_one(b200spmm_plan *p, TallParams &prm, cudaStream_t stream) {
     using Cfg = PairCfg<kTf32>;
     auto kernel = spmm_pair_kernel<kTf32>;
     prm.n_slabs = (prm.n + Cfg::kNs - 1) / Cfg::kNs;
-    prm.n_items = prm.eff_row_windows * prm.n_slabs;
+    prm.n_items = prm.eff_row_windows * prm.n_slabs * prm.parts;
     const int n_pairs = (int)std::min<uint32_t>(prm.n_items, (uint32_t)p->pair_clusters);
     B200_CUDA_TRY(launch_after(kernel, dim3(2 * n_pairs), Cfg::kThreads, Cfg::kSmemBytes, 2, stream, p->tmap_b, p->tmap_bt, prm));
     p->last.n_ctas = 2 * n_pairs;
@@ -671,9 +671,36 @@ int launch_narrow(b200spmm_plan *p, uint32_t group_blocks, const void *d_B, int6
 // graphs of at least kTallMinShortTiles tiles, 32 to 1,024 columns, against the best of the three kernels when forced: the
 // choice is 0.3 % slower on average in tf32 (84 products, at most 7 %), and in fp16 as fast on average (77 products, at
 // most 15 % slower: 3000 x 3000 with 128 columns, 29 us against 25).
-double tall_micros(const TallFormat &f, int units, int64_t n, int64_t slab) {
-    const int64_t items = (int64_t)f.eff * ((n + slab - 1) / slab);
-    return 12.0 + (double)((items + units - 1) / units) * (double)f.max_window_tiles * (slab > 128 ? 0.11 : 0.085);
+//
+// With fewer items than CTAs or pairs the windows are cut into parts, as many as fit in one round: a tile takes the time it
+// takes a CTA by itself then, and the sums go through L2 twice, where a launch of their own adds them up.  Parts in us,
+// whole / 2 / 4 / 8 (16-row kernel): 1777 x 7404 at 15 %, fp16, 104 columns 38.6 / 26.2 / 19.1 / 15.9 (43); 1668 x 5737 at
+// 28 %, tf32, 392 columns 67 / 46 / 35 / - (114); 1682 x 1536 at 11 %, fp16, 816 columns 28 / 21.5 / - / - (78); more than one
+// round of parts is slower again (2000 x 8000 at 10 %, 1,024 columns 56 / 45 / 55 / 81).
+// Up to 64 columns a matrix of fewer than kSplitMinShortTiles tiles keeps to whole windows, and so mostly to the 16-row
+// kernel, a choice that is held to elsewhere: 3000 x 3000 at 12 %, 64 columns 19 us where six parts would take 12.5.
+struct TallLaunch {
+    double micros;
+    uint32_t parts;
+};
+constexpr uint64_t kSplitMinShortTiles = 80000;
+TallLaunch tall_launch(const b200spmm_plan *p, const TallFormat &f, int64_t n) {
+    const bool pair = f.rows == (uint32_t)kPairRows;
+    const int64_t slab = pair || n > 128 ? 256 : 128, units = pair ? p->pair_clusters : p->n_sms, items = (int64_t)f.eff * ((n + slab - 1) / slab);
+    const double longest = (double)f.max_window_tiles, alone = pair ? 0.088 : slab > 128 ? 0.105 : 0.068;
+    TallLaunch best{12.0 + (double)((items + units - 1) / units) * longest * (slab > 128 ? 0.11 : 0.085), 1};
+    if (p->tall_forced || (n <= 64 && p->info.total_tiles < kSplitMinShortTiles)) return best;
+    double least = 12.0 + longest * alone;
+    const uint64_t stages = (f.min_window_tiles + kTallStageTiles - 1) / kTallStageTiles;
+    for (uint32_t parts = 2; parts <= 16 && parts <= stages && items * parts <= units; ++parts) {
+        const double sums = (double)parts * (double)f.eff * f.rows * (double)n * 4.0;
+        const double micros = 12.0 + longest / parts * alone + 1.5 + 2.0 * sums * 0.22e-6;
+        if (micros < least) {
+            least = micros;
+            best = {micros, parts};
+        }
+    }
+    return best;
 }
 double short_micros(const b200spmm_plan *p, int64_t n) {  // (tiles over 148 SMs)
     return 14.0 + (double)p->info.total_tiles * (148.0 / p->n_sms) * (n <= 64 ? 0.28e-3 : 0.4e-3 * (double)((n + 127) / 128));
@@ -682,7 +709,7 @@ double short_micros(const b200spmm_plan *p, int64_t n) {  // (tiles over 148 SMs
 bool use_pair(const b200spmm_plan *p, int64_t n) {
     if (!p->pair.tiles || p->pair_clusters < 1 || n <= 128) return false;
     if (p->tall_forced) return true;
-    return tall_micros(p->pair, p->pair_clusters, n, 256) < short_micros(p, n);
+    return tall_launch(p, p->pair, n).micros < short_micros(p, n);
 }
 
 // Does this launch go to the super-window kernel?  Only with the TMA gathers, and - unless forced, for B at
@@ -690,8 +717,38 @@ bool use_pair(const b200spmm_plan *p, int64_t n) {
 bool use_tall(const b200spmm_plan *p, int64_t n) {
     if (!p->tall.tiles || p->gather_cpasync) return false;
     if (p->tall_forced) return n * p->info.elt_size >= 128;
-    const int64_t slab = n <= 128 ? 128 : 256;
-    return use_pair(p, n) || tall_micros(p->tall, p->n_sms, n, slab) < short_micros(p, n);
+    return use_pair(p, n) || tall_launch(p, p->tall, n).micros < short_micros(p, n);
+}
+
+// What a super-window launch needs of the plan's scratch.
+struct TallScratch {
+    uint32_t parts;
+    size_t partial_floats, packed_bytes;
+};
+TallScratch tall_scratch(const b200spmm_plan *p, int64_t n) {
+    const bool pair = use_pair(p, n);
+    TallScratch s{};
+    s.parts = tall_launch(p, pair ? p->pair : p->tall, n).parts;
+    if (s.parts > 1) s.partial_floats = (size_t)s.parts * (size_t)p->info.rows * (size_t)n;
+    if (p->tall_pack_b) {
+        // the pair kernel's CTAs fetch 128-feature halves of a 256-feature slab: both halves of the last slab must
+        // exist in the packed copy (as zeros past n), so an even number of 128-feature blocks
+        const size_t features = pair || n > 128 ? (size_t)(n + 255) / 256 * 256 : 128;
+        s.packed_bytes = features * 32u * (size_t)((p->info.cols + p->info.col_window - 1) / p->info.col_window);
+    }
+    return s;
+}
+
+// While a stream is being captured no scratch can be had; the 16-row kernel may do without.
+bool tall_can_launch(const b200spmm_plan *p, int64_t n, cudaStream_t stream) {
+    const TallScratch s = tall_scratch(p, n);
+    if (s.partial_floats <= p->partial_floats && s.packed_bytes <= p->b_packed_bytes) return true;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
+        cudaGetLastError();
+        return true;  // (the launch will say what is wrong)
+    }
+    return capture == cudaStreamCaptureStatusNone;
 }
 
 int launch_tall(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
@@ -701,6 +758,7 @@ int launch_tall(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void 
     if (st != B200SPMM_OK) return st;
     const bool pair = use_pair(p, n);
     const TallFormat &fmt = pair ? p->pair : p->tall;
+    const TallScratch scratch = tall_scratch(p, n);
     TallParams prm{};
     prm.rowOffset = fmt.d_rowOffset;
     prm.tcA2B = fmt.d_tcA2B;
@@ -708,12 +766,10 @@ int launch_tall(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void 
     prm.data = static_cast<const uint8_t *>(fmt.d_data);
     if (p->tall_pack_b) {
         const uint32_t cw = (uint32_t)p->info.col_window, esz = (uint32_t)p->info.elt_size;
-        // the pair kernel's CTAs fetch 128-feature halves of a 256-feature slab: both halves of the last slab must
-        // exist in the packed copy (as zeros past n), so an even number of 128-feature blocks
         const uint32_t slab = (n <= 128 || pair) ? 128u : 256u;
         const uint32_t n_slabs = pair ? 2u * (uint32_t)((n + 255) / 256) : (uint32_t)((n + slab - 1) / slab);
         const uint32_t groups = (uint32_t)((p->info.cols + cw - 1) / cw);
-        const size_t need = (size_t)n_slabs * groups * 32u * slab;
+        const size_t need = scratch.packed_bytes;  // n_slabs * groups * 32 * slab
         if (need > p->b_packed_bytes) {
             p->b_packed_bytes = 0;
             int st = grow_buffer(&p->d_b_packed, need);
@@ -726,6 +782,10 @@ int launch_tall(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void 
         prm.b_packed = static_cast<const uint8_t *>(p->d_b_packed);
         prm.b_groups = groups;
     }
+    prm.parts = scratch.parts;
+    st = grow_partial(p, scratch.partial_floats);
+    if (st != B200SPMM_OK) return st;
+    prm.partial = p->d_partial;
     prm.sched_counter = p->d_status + 1;
     prm.C = d_C;
     prm.ldc = ldc;
@@ -743,9 +803,15 @@ int launch_tall(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void 
     cudaMemsetAsync(g_prof, 0, 1024 * 32 * 8, stream);
     prm.prof = g_prof;
 #endif
-    if (pair) return tf32 ? launch_pair_one<true>(p, prm, stream) : launch_pair_one<false>(p, prm, stream);
-    if (n <= 128) return tf32 ? launch_tall_one<true, 128>(p, prm, stream) : launch_tall_one<false, 128>(p, prm, stream);
-    return tf32 ? launch_tall_one<true, 256>(p, prm, stream) : launch_tall_one<false, 256>(p, prm, stream);
+    if (pair) st = tf32 ? launch_pair_one<true>(p, prm, stream) : launch_pair_one<false>(p, prm, stream);
+    else if (n <= 128) st = tf32 ? launch_tall_one<true, 128>(p, prm, stream) : launch_tall_one<false, 128>(p, prm, stream);
+    else st = tf32 ? launch_tall_one<true, 256>(p, prm, stream) : launch_tall_one<false, 256>(p, prm, stream);
+    if (st != B200SPMM_OK || prm.parts == 1) return st;
+    const uint64_t sums = (uint64_t)fmt.eff * fmt.rows * (prm.n / 4);
+    B200_CUDA_TRY(launch_after(tall_sum_parts_kernel, dim3((unsigned)((sums + 255) / 256)), 256, 0, 1, stream, (const float *)prm.partial, prm.parts,
+                               fmt.d_rowIdx, prm.eff_row_windows, fmt.rows, d_C, ldc, prm.rows, prm.n, prm.c_is_half));
+    ++p->last.kernel_launches;
+    return B200SPMM_OK;
 }
 
 // Builds the super-window copy of the matrix when it pays.  The 16-row kernel spends about 100 SM
@@ -763,8 +829,8 @@ int plan_build_tall(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_
         uint64_t n_super = 0;
         int st = estimate_tall_tile_ratio(info, h_rowOffset, h_rowIdx, p->d_tcA2B, kTallRows, 48, &ratio, &n_super);
         if (st != B200SPMM_OK) return st;
-        // fewer super-windows than SMs / 16 can never fill the GPU, however wide B is
-        if (ratio > 0.7 || n_super * 16 < (uint64_t)p->n_sms || info.total_tiles < kTallMinShortTiles) return B200SPMM_OK;
+        // fewer super-windows than SMs / 32 leave the GPU half empty even in sixteen parts each
+        if (ratio > 0.7 || n_super * 32 < (uint64_t)p->n_sms || info.total_tiles < kTallMinShortTiles) return B200SPMM_OK;
     }
     int st = build_tall_device(info, h_rowOffset, h_rowIdx, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, kTallRows, &p->tall);
     if (st == B200SPMM_ERR_UNSUPPORTED) return B200SPMM_OK;  // too many tiles for 32-bit offsets: 16-row kernel
@@ -1462,7 +1528,7 @@ int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, voi
         if (st != B200SPMM_OK) return st;
     }
     note_bounded_waits(p, stream);
-    if (band < 0 && use_tall(p, n)) return launch_tall(p, d_B, ldb, n, d_C, ldc, c_dtype, stream);
+    if (band < 0 && use_tall(p, n) && tall_can_launch(p, n, stream)) return launch_tall(p, d_B, ldb, n, d_C, ldc, c_dtype, stream);
     SpmmParams prm{};
     prm.rowOffset = p->d_rowOffset;
     prm.tcA2B = p->d_tcA2B;

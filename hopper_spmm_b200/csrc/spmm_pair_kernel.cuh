@@ -8,7 +8,7 @@
 // 128-row kernel on a pruned weight matrix.  The reference's kernel keeps a window inside one SM
 // (src/fp16.cu:147); it has no counterpart of this pairing.
 //
-// A work item is (256-row super-window, 256-feature slab); pair k starts with item k, the even CTA
+// A work item is (256-row super-window, 256-feature slab, part of its tiles); pair k starts with item k, the even CTA
 // claims further items from a global counter and writes them into both CTAs' item lists.
 //
 // Roles in a CTA of 416 threads, one CTA per SM:
@@ -38,7 +38,7 @@ struct PairCfg {
     static constexpr int kNc = 128;                         // ... of which one CTA fetches
     static constexpr int kCW = kTf32 ? 8 : 16;
     static constexpr int kEsz = kTf32 ? 4 : 2;
-    static constexpr int kTps = 4;                          // tiles per ring stage (6 and 8 were slower: 711 / 729 us against 678)
+    static constexpr int kTps = kTallStageTiles;                          // tiles per ring stage (6 and 8 were slower: 711 / 729 us against 678)
     static constexpr int kGatherBytes = 32 * kNc;           // CW rows x 128 features
     static constexpr int kStageBytes = kTps * (kGatherBytes + kTallTileBytes);
     static constexpr int kStages = 24 / kTps;               // 192 KB of operands in flight per CTA
@@ -161,7 +161,8 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
         for (uint32_t round = 0; epi_alive; ++round) {
             const uint32_t item = item_id(round);
             if (item == kNoItem) break;
-            const uint32_t w = item / p.n_slabs, slab = item - w * p.n_slabs;
+            const TallItem t = tall_item<kTps>(p, item);
+            const uint32_t w = t.w, slab = t.slab;
             const uint32_t row0 = p.rowIdx[w];
             const uint32_t gap_hi = w + 1 < p.eff_row_windows ? p.rowIdx[w + 1] : p.rows;
             const uint32_t a = round & 1u;
@@ -184,13 +185,13 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
                     if (lane == 0) ptx::mbar_arrive_cluster(a ? leader_acc_empty1 : leader_acc_empty0);
                 }
                 const uint32_t feat0 = f_slab + col0;
-                tall_store_row32(p, row, feat0, r);
+                tall_store_row32(p, t.part, row, feat0, r);
             }
             // Rows of super-windows without entries are absent from the format: clear the gap after this
             // window (and the rows before the very first one), this slab's features.  The sixteen epilogue
             // warps of the pair take every sixteenth row each.
             const bool lead = w == 0 && row0 > 0;
-            if (gap_hi > row0 + kPairRows || lead) {
+            if (t.part == 0 && (gap_hi > row0 + kPairRows || lead)) {
                 const uint32_t slab_feats = min((uint32_t)kNs, p.n - f_slab);
                 const uint32_t who = rank * Cfg::kEpilogueWarps + (uint32_t)warp, of = 2 * Cfg::kEpilogueWarps;
                 tall_clear_rows(p, row0 + kPairRows, min(gap_hi, p.rows), who, of, f_slab, slab_feats, lane);
@@ -212,6 +213,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
 
         struct Cursor {
             uint32_t round, sp, tile_begin, n_tiles, stages, slab, done;
+            uint64_t image;  // this CTA's first tile image of the item
         };
         uint32_t grabbed = 1;
         auto open_item = [&](Cursor &c) {
@@ -233,11 +235,12 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
                 c.done = 1;
                 return;
             }
-            const uint32_t w = item / p.n_slabs;
-            c.slab = item - w * p.n_slabs;
-            const uint32_t t0 = p.rowOffset[w];
-            c.n_tiles = p.rowOffset[w + 1] - t0;
-            c.tile_begin = t0;
+            const TallItem t = tall_item<kTps>(p, item);
+            const uint32_t t0 = p.rowOffset[t.w];
+            c.slab = t.slab;
+            c.n_tiles = t.n_tiles;
+            c.tile_begin = t0 + t.first;
+            c.image = (uint64_t)t0 * 2u + (rank ? p.rowOffset[t.w + 1] - t0 : 0u) + t.first;
             c.stages = (c.n_tiles + kTps - 1) / kTps;
         };
         auto normalise = [&](Cursor &c) {
@@ -247,7 +250,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
                 open_item(c);
             }
         };
-        Cursor cur{0, pid, 0, 0, 0, 0, 0};
+        Cursor cur{0, pid, 0, 0, 0, 0, 0, 0};
         open_item(cur);
         normalise(cur);
         Cursor fc = cur;
@@ -298,7 +301,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
                     // this CTA's halves of the stage's tiles are neighbours in memory and in the ring: one copy
                     if (tile_bytes)
                         ptx::bulk_load(atile_addr + s * kTps * kTallTileBytes,
-                                       p.data + ((uint64_t)cur.tile_begin * 2u + (uint64_t)rank * cur.n_tiles + tpos0) * kTallTileBytes,
+                                       p.data + (cur.image + tpos0) * kTallTileBytes,
                                        here * kTallTileBytes, full_bar(s));
                     B200_PROF_ADD(prof_a_issue);
                 }
@@ -409,8 +412,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
         for (uint32_t round = 0; alive; ++round) {
             const uint32_t item = item_id(round);
             if (item == kNoItem) break;
-            const uint32_t w = item / p.n_slabs;
-            uint32_t nt = p.rowOffset[w + 1] - p.rowOffset[w];
+            uint32_t nt = tall_item<kTps>(p, item).n_tiles;
             const uint32_t a = round & 1u;
             {
                 B200_PROF_T0();
@@ -489,8 +491,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
         for (uint32_t round = 0; alive; ++round) {
             const uint32_t item = item_id(round);
             if (item == kNoItem) break;
-            const uint32_t w = item / p.n_slabs;
-            const uint32_t nt = p.rowOffset[w + 1] - p.rowOffset[w];
+            const uint32_t nt = tall_item<kTps>(p, item).n_tiles;
             for (uint32_t st = 0; st < (nt + kTps - 1) / kTps && alive; ++st) {
                 {
                     B200_PROF_T0();

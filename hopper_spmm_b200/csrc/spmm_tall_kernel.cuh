@@ -16,9 +16,11 @@
 // 128 x kNs x CW multiply-adds at the pipe's full rate, and the accumulator's lane is the window row,
 // so an epilogue thread holds consecutive features of one row and stores them as 16-byte vectors.
 //
-// A work item is (super-window, feature slab); items are numbered window-major, so the CTAs that
-// run at the same time work on the slabs of the same few windows and share their tiles in L2.  CTA b
-// starts with item b and claims further items from a global counter.
+// A work item is (super-window, feature slab, part of the window's tiles); items are numbered window-major, so the
+// CTAs that run at the same time work on the slabs of the same few windows and share their tiles in L2.  CTA b
+// starts with item b and claims further items from a global counter.  Where there are too few windows and slabs
+// for the SMs a window's tiles are cut into several parts (tall_launch in capi.cu has the rule); their sums go to
+// scratch and tall_sum_parts_kernel adds them up, always in the same order.
 //
 // Roles in a CTA of 416 threads, one CTA per SM:
 //   warps 0-7   epilogue: warp w drains TMEM lanes 32 (w % 4) .. +31 (32 window rows), columns half
@@ -39,6 +41,7 @@ namespace b200spmm {
 
 constexpr int kTallRows = 128;                  // rows of a super-window
 constexpr int kTallTileBytes = kTallRows * 32;  // one tile of it: 128 rows x 32 bytes
+constexpr int kTallStageTiles = 4;                    // tiles per ring stage of the super-window kernels
 
 struct TallParams {
     const uint32_t *rowOffset;  // [eff+1] tiles
@@ -57,7 +60,9 @@ struct TallParams {
     uint32_t rows, cols, n;
     uint32_t eff_row_windows;
     uint32_t n_slabs;           // ceil(n / kNs)
-    uint32_t n_items;           // eff_row_windows * n_slabs
+    uint32_t parts;             // of a window's stages; no window has fewer stages than parts
+    float *partial;             // [parts][rows][n] fp32, where there are several
+    uint32_t n_items;           // eff_row_windows * n_slabs * parts
     uint32_t c_is_half;
     uint32_t *status;
     unsigned long long wait_limit_ns;
@@ -69,11 +74,37 @@ struct TallParams {
 #endif
 };
 
+struct TallItem {
+    uint32_t w, slab, part, first, n_tiles;  // first: tile inside the window
+};
+template <uint32_t kTps>  // tiles per stage
+B200_DEVICE TallItem tall_item(const TallParams &p, uint32_t item) {
+    TallItem t;
+    const uint32_t rest = item / p.parts;
+    t.part = item - rest * p.parts;
+    t.w = rest / p.n_slabs;
+    t.slab = rest - t.w * p.n_slabs;
+    t.n_tiles = p.rowOffset[t.w + 1] - p.rowOffset[t.w];
+    t.first = 0;
+    if (p.parts > 1) {
+        const uint32_t stages = (t.n_tiles + kTps - 1) / kTps;
+        t.first = stages * t.part / p.parts * kTps;
+        t.n_tiles = min(stages * (t.part + 1) / p.parts * kTps, t.n_tiles) - t.first;
+    }
+    return t;
+}
+
 // A thread's 32 consecutive features (fp32 bits, feat0 ..) of row `row` -> C, as 16-byte vectors: 8 features per
 // store for fp16 C, 4 for fp32 C (n is a multiple of 8).  Rows past the end and features past n are dropped.
-B200_DEVICE void tall_store_row32(const TallParams &p, uint32_t row, uint32_t feat0, const uint32_t (&r)[32]) {
+B200_DEVICE void tall_store_row32(const TallParams &p, uint32_t part, uint32_t row, uint32_t feat0, const uint32_t (&r)[32]) {
     if (row >= p.rows || feat0 >= p.n) return;
-    if (p.c_is_half) {
+    if (p.parts > 1) {
+        float *dst = p.partial + ((uint64_t)part * p.rows + row) * p.n + feat0;
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+            if (feat0 + v * 4 < p.n)
+                *reinterpret_cast<uint4 *>(dst + v * 4) = make_uint4(r[v * 4], r[v * 4 + 1], r[v * 4 + 2], r[v * 4 + 3]);
+    } else if (p.c_is_half) {
         __half *dst = static_cast<__half *>(p.C) + (int64_t)row * p.ldc + feat0;
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
@@ -122,7 +153,7 @@ struct TallCfg {
     // Four tiles per ring stage: the MMA-issuing thread pays its wait, its commit and its ring
     // bookkeeping (about 330 SM clocks, measured) once per stage, and four MMAs keep the tensor pipe
     // busy for 512 clocks.  With two tiles per stage that thread, not the pipe, set the pace.
-    static constexpr int kTps = 4;                          // tiles per ring stage
+    static constexpr int kTps = kTallStageTiles;                          // tiles per ring stage
     static constexpr int kGatherBytes = 32 * kNs;           // CW rows x kNs features
     static constexpr int kStageBytes = kTps * (kGatherBytes + kTallTileBytes);
     static constexpr int kProducerWarps = 4;
@@ -238,7 +269,8 @@ spmm_tall_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
         for (uint32_t round = 0; epi_alive; ++round) {
             const uint32_t item = item_id(round);
             if (item == kNoItem) break;
-            const uint32_t w = item / p.n_slabs, slab = item - w * p.n_slabs;
+            const TallItem t = tall_item<kTps>(p, item);
+            const uint32_t w = t.w, slab = t.slab;
             const uint32_t row0 = p.rowIdx[w];
             const uint32_t gap_hi = w + 1 < p.eff_row_windows ? p.rowIdx[w + 1] : p.rows;
             const uint32_t a = round & 1u;
@@ -261,13 +293,13 @@ spmm_tall_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
                     if (lane == 0) ptx::mbar_arrive(acc_empty_bar(a));
                 }
                 const uint32_t feat0 = f_slab + col0;  // this thread: features feat0 .. feat0 + 31 of its row
-                tall_store_row32(p, row, feat0, r);
+                tall_store_row32(p, t.part, row, feat0, r);
             }
             // Rows of super-windows without entries are absent from the format: clear the gap after this
             // window (and the rows before the very first one), this slab's features.  Warp w takes every
             // eighth row.
             const bool lead = w == 0 && row0 > 0;
-            if (gap_hi > row0 + kTallRows || lead) {
+            if (t.part == 0 && (gap_hi > row0 + kTallRows || lead)) {
                 const uint32_t slab_feats = min((uint32_t)kNs, p.n - f_slab);
                 tall_clear_rows(p, row0 + kTallRows, min(gap_hi, p.rows), (uint32_t)warp, Cfg::kEpilogueWarps, f_slab, slab_feats, lane);
                 if (lead) tall_clear_rows(p, 0u, row0, (uint32_t)warp, Cfg::kEpilogueWarps, f_slab, slab_feats, lane);
@@ -309,10 +341,10 @@ spmm_tall_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
                 c.done = 1;
                 return;
             }
-            const uint32_t w = item / p.n_slabs;
-            c.slab = item - w * p.n_slabs;
-            c.tile_begin = p.rowOffset[w];
-            c.n_tiles = p.rowOffset[w + 1] - c.tile_begin;
+            const TallItem t = tall_item<kTps>(p, item);
+            c.slab = t.slab;
+            c.tile_begin = p.rowOffset[t.w] + t.first;
+            c.n_tiles = t.n_tiles;
             c.stages = (c.n_tiles + kTps - 1) / kTps;
         };
         auto normalise = [&](Cursor &c) {  // stage cursor past the end of an item: next item
@@ -478,8 +510,7 @@ spmm_tall_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
         for (uint32_t round = 0; alive; ++round) {
             const uint32_t item = item_id(round);
             if (item == kNoItem) break;
-            const uint32_t w = item / p.n_slabs;
-            uint32_t nt = p.rowOffset[w + 1] - p.rowOffset[w];
+            uint32_t nt = tall_item<kTps>(p, item).n_tiles;
             const uint32_t a = round & 1u;
             {
                 B200_PROF_T0();
@@ -558,6 +589,38 @@ spmm_tall_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
             p.sched_counter[0] = 0;
             p.sched_counter[1] = 0;
         }
+    }
+}
+
+// Adds the parts of the windows' rows up and writes them to C: four features a thread, the parts in order.  They lie in L2
+// (a launch has parts for one round of CTAs, 128 KB each).
+__global__ void __launch_bounds__(256)
+tall_sum_parts_kernel(const float *partial, uint32_t parts, const uint32_t *__restrict__ rowIdx, uint32_t eff, uint32_t window_rows, void *C,
+                      int64_t ldc, uint32_t rows, uint32_t n, uint32_t c_is_half) {
+    const uint32_t vec_per_row = n / 4, per_window = window_rows * vec_per_row;
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, w = i / per_window;
+    if (w >= eff) {
+        ptx::wait_for_grids_before();
+        return;
+    }
+    const uint32_t at = (uint32_t)(i - w * per_window), r = rowIdx[w] + at / vec_per_row, feat = at % vec_per_row * 4;
+    ptx::wait_for_grids_before();
+    if (r >= rows) return;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float *src = partial + (uint64_t)r * n + feat;
+#pragma unroll 4
+    for (uint32_t k = 0; k < parts; ++k) {
+        const float4 v = __ldcs(reinterpret_cast<const float4 *>(src + (uint64_t)k * rows * n));
+        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+    }
+    if (c_is_half) {
+        const __half2 lo = __floats2half2_rn(acc.x, acc.y), hi = __floats2half2_rn(acc.z, acc.w);
+        uint2 packed;
+        packed.x = *reinterpret_cast<const uint32_t *>(&lo);
+        packed.y = *reinterpret_cast<const uint32_t *>(&hi);
+        *reinterpret_cast<uint2 *>(static_cast<__half *>(C) + (int64_t)r * ldc + feat) = packed;
+    } else {
+        *reinterpret_cast<float4 *>(static_cast<float *>(C) + (int64_t)r * ldc + feat) = acc;
     }
 }
 

@@ -245,7 +245,11 @@ int build_tall_device(const b200spmm_btcf_info_t &info, const uint32_t *h_rowOff
     t.rows = kTall;
     t.eff = n_groups;
     t.tiles = t_tiles;
-    for (uint64_t g = 0; g < n_groups; ++g) t.max_window_tiles = std::max<uint64_t>(t.max_window_tiles, t_rowOffset[g + 1] - t_rowOffset[g]);
+    t.min_window_tiles = t_tiles;
+    for (uint64_t g = 0; g < n_groups; ++g) {
+        t.max_window_tiles = std::max<uint64_t>(t.max_window_tiles, t_rowOffset[g + 1] - t_rowOffset[g]);
+        t.min_window_tiles = std::min<uint64_t>(t.min_window_tiles, t_rowOffset[g + 1] - t_rowOffset[g]);
+    }
     struct Guard {
         TallFormat *t;
         ~Guard() { if (t) free_tall(t); }

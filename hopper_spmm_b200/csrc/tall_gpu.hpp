@@ -11,7 +11,7 @@ namespace b200spmm {
 struct TallFormat {
     uint32_t rows = 128;          // rows of a super-window: 128, or 256 for the CTA-pair kernel
     uint64_t eff = 0, tiles = 0;  // super-windows holding entries, their tiles (rows x CW each)
-    uint64_t max_window_tiles = 0;
+    uint64_t max_window_tiles = 0, min_window_tiles = 0;
     uint32_t *d_rowOffset = nullptr, *d_tcA2B = nullptr, *d_rowIdx = nullptr;
     void *d_data = nullptr;  // tiles in the kernel's shared-memory image, 128 rows each: row r of an image has its
                              // two 16-byte halves swapped when (r / 4) is odd.  rows == 256: per window the

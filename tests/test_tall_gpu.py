@@ -199,3 +199,31 @@ def test_fewer_windows_than_sms_take_the_kernel_expected_to_be_faster(dt, n, win
         parity.check(dC.cpu().numpy(), rows, rp, ci, v, B)
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("dt,rows,n,window", [(np.float16, 1300, 72, 128), (np.float16, 1800, 128, 128), (np.float16, 1800, 328, 256),
+                                              (np.float32, 1300, 104, 128), (np.float32, 1800, 264, 256)])
+def test_few_windows_are_cut_into_parts(dt, rows, n, window):
+    # fewer windows than SMs or pairs, of unequal length and one gap: their tiles are shared out and the sums added up by a
+    # launch of their own; every row written, nothing beside them, same bits again, in fp16 the rounded sums; in a graph
+    import torch
+    rows, cols, rp, ci, v = random_csr(rows, 6003, 0.14, 5, dt, empty_rows=[(512, 768)])
+    Bfull = torch.from_numpy(dense_b(cols, n + 16, 3, dt)).cuda()
+    Bv = Bfull[:, 8:8 + n]
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    try:
+        Cfull = torch.full((rows, n + 16), float("nan"), device="cuda")
+        plan.spmm(Bv, Cfull[:, 8:8 + n])
+        info = plan.launch_info()
+        assert info.row_window == window and info.kernel_launches == 3  # B re-laid, products, sums
+        got = Cfull[:, 8:8 + n].clone()
+        parity.check(got.cpu().numpy(), rows, rp, ci, v, Bv.cpu().numpy())
+        assert torch.isnan(Cfull[:, :8]).all() and torch.isnan(Cfull[:, 8 + n:]).all()
+        assert torch.equal(plan.spmm(Bv), got) and torch.equal(plan.spmm(Bv, c_half=True), got.half())
+        g, out = torch.cuda.CUDAGraph(), torch.full((rows, n), float("nan"), device="cuda")
+        with torch.cuda.graph(g):
+            plan.spmm(Bv, out, sync=False)
+        g.replay()
+        assert torch.equal(out, got)
+    finally:
+        plan.close()
