@@ -61,6 +61,7 @@ struct b200spmm_plan {
     struct Sched {
         int n_ctas = 0;
         uint32_t n_chunks = 0;
+        uint32_t *d_tables = nullptr;  // holds all that follow
         uint32_t *d_tile = nullptr, *d_wfirst = nullptr, *d_wlast = nullptr, *d_head_slot = nullptr, *d_tail_slot = nullptr;
         SplitWindow *d_splits = nullptr;
         uint32_t *d_piece_slots = nullptr;
@@ -497,11 +498,14 @@ constexpr double kRowsMaxFill = 0.08;  // share of a tile's slots in use
 // graph of 20,000 nodes merges well too, and waits for its hub window: 148 us against 35.  Matrices of fewer tiles
 // than two a CTA take the same few microseconds either way and stay with their tiles.
 constexpr double kRowsMaxFillWide = 0.11, kTallMinFill = 0.03;
-constexpr uint64_t kRowsWideMinTiles = 592;
-// Fewer tiles keep to 16 rows: the plan is made in 290 us instead of 660, and up to 128 columns the product takes the same
-// (1500 x 1500 at 25 %, 8,758 tiles: 17 and 19 us for 64 and 128 columns against 19 and 20 with 128 rows).  A wide B pays
-// for that: 28 against 25 us for 256 columns, 82 against 26 for 1,024, 298 against 43 for 4,096.
-constexpr uint64_t kTallMinShortTiles = 16384;
+constexpr uint64_t kRowsWideMinTiles = 592, kRowsWideAnyTiles = 16384;  // (below the second, whatever super-windows would do)
+// Super-windows are made from this many short tiles on: 1100 x 1100 at 20 % (4,638), fp16, 72 / 200 / 512 / 2,048 columns 15.7
+// / 24.5 / 37.8 / 134 us with 16 rows, 10.9 / 14.9 / 17.1 / 20.2 with them; the plan takes 285 us instead of 276.  Those of
+// 256 rows from the second number on: in parts the two heights take the same (1682 x 1536 at 11 %, 8,614 tiles, 816 columns
+// 21.5 and 22.5 us), and the plan takes 50 us less with one of them.  Below it whole windows of 128 rows do not pay up to 128
+// columns (3000 x 1100 at 10 %, 128 columns 12.4 us with 16 rows, 13.4 with 128).
+constexpr uint64_t kTallMinShortTiles = 2048, kPairMinShortTiles = 16384;
+constexpr uint64_t kTallMaxCounted = 1 << 25, kTallMaxCountedCols = 393216;  // entries of lists; columns of one bit set
 
 bool use_rows(const b200spmm_plan *p, int64_t ldb) {
     return p->rows_only && ldb * p->info.elt_size <= 0xFFFFFFFFll;  // (the kernel's row pitch is 32-bit)
@@ -668,7 +672,7 @@ int launch_narrow(b200spmm_plan *p, uint32_t group_blocks, const void *d_B, int6
 // item: pruned 14336 x 4096, 10 %, fp16, 64 / 128 / 192 columns 33 / 36 / 43 us (56 windows of 256 rows for 74 pairs)
 // against 62 / 79 / 146 with 16 rows; 3000 x 3000, 12 %, 192 columns 33 against 45, but at 64 columns 25 against 23.
 // A tf32 tile takes what an fp16 one does, eight rows of B of twice the bytes.  Pruned, uniform and block matrices and
-// graphs of at least kTallMinShortTiles tiles, 32 to 1,024 columns, against the best of the three kernels when forced: the
+// graphs of at least 16,384 tiles, 32 to 1,024 columns, against the best of the three kernels when forced: the
 // choice is 0.3 % slower on average in tf32 (84 products, at most 7 %), and in fp16 as fast on average (77 products, at
 // most 15 % slower: 3000 x 3000 with 128 columns, 29 us against 25).
 //
@@ -717,7 +721,10 @@ bool use_pair(const b200spmm_plan *p, int64_t n) {
 bool use_tall(const b200spmm_plan *p, int64_t n) {
     if (!p->tall.tiles || p->gather_cpasync) return false;
     if (p->tall_forced) return n * p->info.elt_size >= 128;
-    return use_pair(p, n) || tall_launch(p, p->tall, n).micros < short_micros(p, n);
+    if (use_pair(p, n)) return true;
+    const TallLaunch t = tall_launch(p, p->tall, n);
+    if (t.parts == 1 && n <= 128 && p->info.total_tiles < kPairMinShortTiles) return false;
+    return t.micros < short_micros(p, n);
 }
 
 // What a super-window launch needs of the plan's scratch.
@@ -824,15 +831,29 @@ int plan_build_tall(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_
     if (!info.total_tiles || env_is("B200SPMM_WINDOW", "16")) return B200SPMM_OK;
     const bool want_pair = env_is("B200SPMM_WINDOW", "256");
     p->tall_forced = env_is("B200SPMM_WINDOW", "128") || want_pair;
+    SuperCounts counts;
+    bool counted = false;
     if (!p->tall_forced) {
+        if (info.total_tiles < kTallMinShortTiles) return B200SPMM_OK;
         double ratio = 1.0;
         uint64_t n_super = 0;
-        int st = estimate_tall_tile_ratio(info, h_rowOffset, h_rowIdx, p->d_tcA2B, kTallRows, 48, &ratio, &n_super);
+        // counting all windows takes a look at every list, several where the columns are many: large graphs are sampled first
+        counted = info.total_tiles * (uint64_t)info.col_window <= kTallMaxCounted && info.cols <= kTallMaxCountedCols;
+        int st;
+        if (counted) {
+            st = count_super_windows(info, h_rowOffset, h_rowIdx, p->d_tcA2B, &counts);
+            ratio = (double)counts.tall_tiles / (double)info.total_tiles;
+            n_super = counts.tall_windows;
+        } else {
+            st = estimate_tall_tile_ratio(info, h_rowOffset, h_rowIdx, p->d_tcA2B, kTallRows, 48, &ratio, &n_super);
+        }
         if (st != B200SPMM_OK) return st;
         // fewer super-windows than SMs / 32 leave the GPU half empty even in sixteen parts each
-        if (ratio > 0.7 || n_super * 32 < (uint64_t)p->n_sms || info.total_tiles < kTallMinShortTiles) return B200SPMM_OK;
+        if (ratio > 0.7 || n_super * 32 < (uint64_t)p->n_sms) return B200SPMM_OK;
     }
-    int st = build_tall_device(info, h_rowOffset, h_rowIdx, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, kTallRows, &p->tall);
+    int st = counted ? B200SPMM_OK : count_super_windows(info, h_rowOffset, h_rowIdx, p->d_tcA2B, &counts);
+    if (st != B200SPMM_OK) return st;
+    st = build_tall_device(info, counts, h_rowOffset, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, kTallRows, &p->tall);
     if (st == B200SPMM_ERR_UNSUPPORTED) return B200SPMM_OK;  // too many tiles for 32-bit offsets: 16-row kernel
     if (st != B200SPMM_OK || !p->tall.tiles) return st;
     // The pair kernel does twice the work per tile: it pays when a 256-row window has (about) the column
@@ -840,24 +861,15 @@ int plan_build_tall(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_
     if (!env_is("B200SPMM_WINDOW", "128")) {
         st = info.dtype == B200SPMM_TF32 ? pair_max_clusters<true>(&p->pair_clusters) : pair_max_clusters<false>(&p->pair_clusters);
         if (st != B200SPMM_OK) return st;
-        if (p->pair_clusters > 0) {
-            st = build_tall_device(info, h_rowOffset, h_rowIdx, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, kPairRows, &p->pair);
+        if (p->pair_clusters > 0 && (want_pair || ((double)counts.pair_tiles <= 0.55 * (double)counts.tall_tiles && info.total_tiles >= kPairMinShortTiles))) {
+            st = build_tall_device(info, counts, h_rowOffset, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, kPairRows, &p->pair);
             if (st != B200SPMM_OK && st != B200SPMM_ERR_UNSUPPORTED) return st;
-            if (!want_pair && (double)p->pair.tiles > 0.55 * (double)p->tall.tiles) free_tall(&p->pair);
         }
     }
-    // how many tiles name one aligned row group of B (sampled on the host: every 16th tile's list ends)
-    {
-        const uint64_t cw = (uint64_t)info.col_window, step = 16, n_probe = (p->tall.tiles + step - 1) / step;
-        std::vector<uint32_t> probe(n_probe * 2);
-        // first and last entry of every 16th tile's column list: two strided copies
-        B200_CUDA_TRY(cudaMemcpy2D(probe.data(), 8, p->tall.d_tcA2B, step * cw * 4, 4, n_probe, cudaMemcpyDeviceToHost));
-        B200_CUDA_TRY(cudaMemcpy2D(probe.data() + 1, 8, p->tall.d_tcA2B + (cw - 1), step * cw * 4, 4, n_probe, cudaMemcpyDeviceToHost));
-        uint64_t aligned = 0;
-        for (uint64_t i = 0; i < n_probe; ++i)
-            aligned += (probe[2 * i] % cw == 0 && probe[2 * i + 1] - probe[2 * i] == cw - 1) ? 1 : 0;
-        p->tall_pack_b = aligned * 2 >= n_probe && !env_is("B200SPMM_PACK_B", "0");
-    }
+    uint32_t aligned = 0;
+    B200_CUDA_TRY(cudaMemcpy(&aligned, p->tall.d_aligned, 4, cudaMemcpyDeviceToHost));
+    p->tall_pack_b = (uint64_t)aligned * 2 >= p->tall.tiles && !env_is("B200SPMM_PACK_B", "0");
+    B200_CUDA_TRY(cudaDeviceSynchronize());
     return B200SPMM_OK;
 }
 
@@ -885,12 +897,6 @@ int plan_build_tile_image(b200spmm_plan *p) {
 // The schedule of the 16-row kernel, on the device.
 int plan_build_schedule(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h_rowIdx, int n_ctas) {
     const auto &info = p->info;
-    auto upload = [](auto **dst, const auto &v) -> int {
-        using T = typename std::remove_reference<decltype(v)>::type::value_type;
-        B200_CUDA_TRY(pool_alloc(dst, v.size()));
-        if (!v.empty()) B200_CUDA_TRY(cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
-        return B200SPMM_OK;
-    };
     {
         b200spmm_plan::Sched &ps = p->sched;
         ps.n_ctas = n_ctas > 0 ? n_ctas : p->n_sms * kCtasPerSm;
@@ -904,14 +910,25 @@ int plan_build_schedule(b200spmm_plan *p, const uint32_t *h_rowOffset, const uin
         build_tile_schedule(h_rowOffset, info.eff_row_windows, (int)ps.n_chunks, /*allow_split=*/true, &sc);
         std::vector<SplitWindow> splits;
         for (const auto &sp : sc.splits) splits.push_back(SplitWindow{sp.window, sp.piece_begin, sp.piece_end});
-        int st_up = upload(&ps.d_tile, sc.tile);
-        if (st_up == B200SPMM_OK) st_up = upload(&ps.d_wfirst, sc.wfirst);
-        if (st_up == B200SPMM_OK) st_up = upload(&ps.d_wlast, sc.wlast);
-        if (st_up == B200SPMM_OK) st_up = upload(&ps.d_head_slot, sc.head_slot);
-        if (st_up == B200SPMM_OK) st_up = upload(&ps.d_tail_slot, sc.tail_slot);
-        if (st_up == B200SPMM_OK) st_up = upload(&ps.d_splits, splits);
-        if (st_up == B200SPMM_OK) st_up = upload(&ps.d_piece_slots, sc.piece_slots);
-        if (st_up != B200SPMM_OK) return st_up;
+        // one copy brings all tables
+        std::vector<uint32_t> tables;
+        auto append = [&](const auto &v) {
+            const size_t at = tables.size();
+            tables.resize(at + v.size() * sizeof(v[0]) / 4);
+            std::memcpy(tables.data() + at, v.data(), v.size() * sizeof(v[0]));
+            return at;
+        };
+        const size_t tile = append(sc.tile), wfirst = append(sc.wfirst), wlast = append(sc.wlast), head = append(sc.head_slot),
+                     tail = append(sc.tail_slot), split = append(splits), pieces = append(sc.piece_slots);
+        B200_CUDA_TRY(pool_alloc(&ps.d_tables, tables.size()));
+        B200_CUDA_TRY(cudaMemcpy(ps.d_tables, tables.data(), tables.size() * 4, cudaMemcpyHostToDevice));
+        ps.d_tile = ps.d_tables + tile;
+        ps.d_wfirst = ps.d_tables + wfirst;
+        ps.d_wlast = ps.d_tables + wlast;
+        ps.d_head_slot = ps.d_tables + head;
+        ps.d_tail_slot = ps.d_tables + tail;
+        ps.d_splits = reinterpret_cast<SplitWindow *>(ps.d_tables + split);
+        ps.d_piece_slots = ps.d_tables + pieces;
         ps.n_splits = (uint32_t)splits.size();
         ps.n_slots = sc.n_slots;
         RowBands bands;  // only schedules with many chunks are worth launching in bands
@@ -1044,7 +1061,7 @@ int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h
                                               p->d_tcA2B, kTallRows, 48, &ratio, &n_super);
             if (st != B200SPMM_OK) return st;
             // (an eighth of the short tiles is the least that merging eight windows can leave)
-            if (fill / (8.0 * ratio) < kTallMinFill || info.total_tiles < kTallMinShortTiles) max_fill = kRowsMaxFillWide;
+            if (fill / (8.0 * ratio) < kTallMinFill || info.total_tiles < kRowsWideAnyTiles) max_fill = kRowsMaxFillWide;
         }
         int st = build_row_formats(info, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, p->loose_lists, p->n_sms, max_fill, force_rows,
                                    &p->rows_fmt, &p->narrow);
@@ -1295,13 +1312,7 @@ void b200spmm_plan_destroy(b200spmm_plan_t *p) {
     }
     {
         auto &ps = p->sched;
-        pool_free(ps.d_tile);
-        pool_free(ps.d_wfirst);
-        pool_free(ps.d_wlast);
-        pool_free(ps.d_head_slot);
-        pool_free(ps.d_tail_slot);
-        pool_free(ps.d_splits);
-        pool_free(ps.d_piece_slots);
+        pool_free(ps.d_tables);
     }
     free_compressed_tiles(&p->comp);
     free_rows(&p->rows_fmt);

@@ -2,16 +2,18 @@
 // matrix at that window height with the reference's algorithm (src/utils/convert.h:146-225):
 // sorted distinct columns per window, padded to whole tiles; entries at (row % 128, column slot).
 //
-// Steps (integer work, bound by HBM traffic):
-//   1. one key (super-window << 32 | column) per column-list entry of the 16-row format
-//   2. radix sort + unique (CUB): the sorted distinct columns of every super-window
-//   3. per super-window: first distinct key and count (binary search) -> tiles -> rowOffset
-//   4. column lists scattered into tcA2B (pre-filled with 0xFFFFFFFF)
-//   5. every (16-row tile, column slot) finds its slot in the super-window's list and its sixteen
-//      values move into the zero-filled 128-row tiles, which are stored as the kernel's shared-memory
-//      image (the two 16-byte halves of a tile row swapped when row / 4 is odd: the 32-byte swizzle)
+//   1. count_kernel: a block marks the columns of a 256-row window and of its two halves in bit sets in shared memory and
+//      counts them.  The host makes the tile offsets of both heights from that, its one wait.
+//   2. lists_kernel: the same bit set once more per window; the rank of a word gives its columns their places
+//   3. tiles_kernel: a block makes kRunTiles neighbouring tiles of 128 rows in shared memory - each warp takes a
+//      16-row tile that has columns there, eight values a lane, and looks their slots up in the run's list - and writes them
+//      in one piece, as the product kernel's shared-memory image (the two 16-byte halves of a tile row swapped when
+//      row / 4 is odd: the 32-byte swizzle)
+// Large matrices are bound by the bytes of both formats and the driver's memory, small ones by the copies and waits around
+// three launches.  A whole plan, in us, with a sort of all columns and a scatter of single values into cleared tiles, and so:
+// pruned 28672 x 8192 at 10 % 5,270 and 3,190, 14336 x 4096 2,300 and 730, 1777 x 7404 at 15 % 870 and 445.
 #include <algorithm>
-#include <cub/cub.cuh>
+#include <cstring>
 #include <vector>
 
 #include "common.hpp"
@@ -22,94 +24,198 @@
 namespace b200spmm {
 namespace {
 
-constexpr int kBlock = 256;
 constexpr uint32_t kShort = 16;
+constexpr int kMergeBlock = 512;
+constexpr uint32_t kChunkWords = 12288;  // words of a bit set: wider matrices go through chunks of columns
+constexpr uint32_t kRunTiles = 8;        // 32 KB of tiles a block: six of them an SM
+constexpr int kTilesBlock = 256;
 
-inline int grid_for(uint64_t n) { return (int)std::max<uint64_t>(1, std::min<uint64_t>((n + kBlock - 1) / kBlock, 148 * 32)); }
+inline uint32_t chunk_words(uint64_t cols) { return (uint32_t)std::min<uint64_t>((cols + 127) / 128 * 4, kChunkWords); }
 
-// window holding tile t: last i with rowOffset[i] <= t
-__device__ __forceinline__ uint32_t window_of_tile(const uint32_t *__restrict__ rowOffset, uint32_t eff, uint32_t t) {
-    uint32_t lo = 0, hi = eff;
-    while (hi - lo > 1) {
-        const uint32_t mid = lo + (hi - lo) / 2;
-        if (rowOffset[mid] <= t) lo = mid; else hi = mid;
+// Marks the columns [col0, col0 + 32 * words) of the lists in tiles [t0, t1).
+__device__ __forceinline__ void mark_columns(uint32_t *bits, uint32_t words, const uint32_t *__restrict__ tcA2B, uint32_t t0, uint32_t t1, uint32_t cw,
+                                             uint32_t col0) {
+    const uint4 *lists = reinterpret_cast<const uint4 *>(tcA2B + (uint64_t)t0 * cw);
+    const uint32_t n = (t1 - t0) * (cw / 4);
+#pragma unroll 4
+    for (uint32_t q = threadIdx.x; q < n; q += kMergeBlock) {
+        const uint4 v = __ldg(lists + q);
+        const uint32_t c[4] = {v.x - col0, v.y - col0, v.z - col0, v.w - col0};
+#pragma unroll
+        for (int k = 0; k < 4; ++k)  // (no column: past every word)
+            if ((c[k] >> 5) < words) atomicOr(bits + (c[k] >> 5), 1u << (c[k] & 31u));
     }
-    return lo;
 }
 
-// keys[e] = group(window of entry e) << 32 | column; padding entries get the key of a group past the end
-__global__ void tall_keys_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B,
-                                 const uint32_t *__restrict__ win_group, uint32_t eff, uint32_t n_groups, uint32_t cw,
-                                 uint64_t n_entries, uint64_t *__restrict__ keys) {
-    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n_entries; e += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t c = tcA2B[e];
-        if (c == kIdxMax) {
-            keys[e] = ((uint64_t)n_groups << 32) | kIdxMax;
-        } else {
-            const uint32_t i = window_of_tile(rowOffset, eff, (uint32_t)(e / cw));
-            keys[e] = ((uint64_t)win_group[i] << 32) | c;
+// One block per 256-row window: distinct columns of its upper half, its lower half, and both.
+struct WindowPair {
+    uint32_t t0, t_mid, t1;  // 16-row tiles of the two halves
+};
+__global__ void __launch_bounds__(kMergeBlock)
+count_kernel(const WindowPair *__restrict__ pairs, const uint32_t *__restrict__ tcA2B, uint32_t cw, uint64_t cols, uint32_t words,
+             uint32_t *__restrict__ counts) {
+    extern __shared__ __align__(16) uint32_t merge_smem[];
+    __shared__ uint32_t total[3];
+    uint32_t *upper = merge_smem, *lower = merge_smem + words;
+    const WindowPair p = pairs[blockIdx.x];
+    if (threadIdx.x < 3) total[threadIdx.x] = 0;
+    for (uint64_t col0 = 0; col0 < cols; col0 += 32ull * words) {
+        __syncthreads();
+        for (uint32_t k = threadIdx.x; k < 2 * words; k += kMergeBlock) merge_smem[k] = 0;
+        __syncthreads();
+        mark_columns(upper, words, tcA2B, p.t0, p.t_mid, cw, (uint32_t)col0);
+        mark_columns(lower, words, tcA2B, p.t_mid, p.t1, cw, (uint32_t)col0);
+        __syncthreads();
+        uint32_t n[3] = {};
+        for (uint32_t k = threadIdx.x; k < words; k += kMergeBlock) {
+            const uint32_t a = upper[k], b = lower[k];
+            n[0] += __popc(a);
+            n[1] += __popc(b);
+            n[2] += __popc(a | b);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            n[k] = __reduce_add_sync(0xffffffffu, n[k]);
+            if ((threadIdx.x & 31u) == 0 && n[k]) atomicAdd(&total[k], n[k]);
         }
     }
+    __syncthreads();
+    if (threadIdx.x < 3) counts[blockIdx.x * 3 + threadIdx.x] = total[threadIdx.x];
 }
 
-// ubase[g] = index of the first distinct key of group g (g = n_groups: the end of the real keys)
-__global__ void tall_group_base_kernel(const uint64_t *__restrict__ ukeys, uint64_t n_unique, uint32_t n_groups,
-                                       uint32_t *__restrict__ ubase) {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g > n_groups) return;
-    const uint64_t want = (uint64_t)g << 32;
-    uint64_t lo = 0, hi = n_unique;
-    while (lo < hi) {
-        const uint64_t mid = lo + (hi - lo) / 2;
-        if (ukeys[mid] < want) lo = mid + 1; else hi = mid;
+// One block per super-window: its sorted distinct columns, padded to whole tiles; and how many of the tiles name one aligned
+// group of rows of B (added to *aligned).
+struct WindowLists {
+    uint32_t t0, t1, out, n_tiles;  // 16-row tiles, first tile of the list, tiles
+};
+__global__ void __launch_bounds__(kMergeBlock)
+lists_kernel(const WindowLists *__restrict__ windows, const uint32_t *__restrict__ tcA2B, uint32_t cw, uint64_t cols, uint32_t words,
+             uint32_t *__restrict__ lists, uint32_t *__restrict__ aligned) {
+    extern __shared__ __align__(16) uint32_t merge_smem[];
+    __shared__ uint32_t sums[kMergeBlock / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const WindowLists w = windows[blockIdx.x];
+    uint32_t *out = lists + (uint64_t)w.out * cw, base = 0;
+    for (uint64_t col0 = 0; col0 < cols; col0 += 32ull * words) {
+        __syncthreads();
+        for (uint32_t k = threadIdx.x; k < words; k += kMergeBlock) merge_smem[k] = 0;
+        __syncthreads();
+        mark_columns(merge_smem, words, tcA2B, w.t0, w.t1, cw, (uint32_t)col0);
+        __syncthreads();
+        for (uint32_t k0 = 0; k0 < words; k0 += kMergeBlock) {  // one word a thread
+            const uint32_t k = k0 + threadIdx.x;
+            uint32_t b = k < words ? merge_smem[k] : 0u;
+            const uint32_t mine = __popc(b);
+            uint32_t upto = mine;
+#pragma unroll
+            for (int d = 1; d < 32; d *= 2) {
+                const uint32_t x = __shfl_up_sync(0xffffffffu, upto, d);
+                if (lane >= (uint32_t)d) upto += x;
+            }
+            __syncthreads();  // `sums` of the round before has been read
+            if (lane == 31) sums[warp] = upto;
+            __syncthreads();
+            uint32_t at = base + upto - mine;
+            for (uint32_t i = 0; i < kMergeBlock / 32; ++i) {
+                if (i < warp) at += sums[i];
+                base += sums[i];
+            }
+            for (; b; b &= b - 1u) out[at++] = (uint32_t)col0 + k * 32u + (uint32_t)__ffs((int)b) - 1u;
+        }
     }
-    ubase[g] = (uint32_t)lo;
-}
-
-__global__ void tall_scatter_columns_kernel(const uint64_t *__restrict__ ukeys, uint64_t n_real,
-                                            const uint32_t *__restrict__ ubase, const uint32_t *__restrict__ t_rowOffset,
-                                            uint32_t cw, uint32_t *__restrict__ t_tcA2B) {
-    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n_real; j += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t k = ukeys[j];
-        const uint32_t g = (uint32_t)(k >> 32);
-        t_tcA2B[(uint64_t)t_rowOffset[g] * cw + (j - ubase[g])] = (uint32_t)k;
+    for (uint32_t k = base + threadIdx.x; k < w.n_tiles * cw; k += kMergeBlock) out[k] = kIdxMax;
+    __syncthreads();
+    uint32_t n = 0;
+    for (uint32_t t = threadIdx.x; t < w.n_tiles; t += kMergeBlock) {
+        const uint32_t from = out[t * cw];
+        n += from % cw == 0 && out[t * cw + cw - 1] - from == cw - 1;
     }
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (lane == 0 && n) atomicAdd(aligned, n);
 }
 
-// one thread per (16-row tile, column slot): its sixteen values go to the super-window's tile
+// One block per run of tiles of 128 rows.
+struct TileRun {
+    uint32_t w0, w1, row0;          // 16-row windows of the 128 rows, and the first of these
+    uint32_t list, n_tiles, image;  // first tile of the run in the lists, its tiles, and its first image
+};
 template <typename T>
-__global__ void tall_scatter_values_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B,
-                                           const T *__restrict__ data, const uint32_t *__restrict__ rowIdx,
-                                           const uint32_t *__restrict__ win_group, uint32_t eff, uint32_t cw,
-                                           uint64_t n_entries, const uint32_t *__restrict__ ubase,
-                                           const uint32_t *__restrict__ t_rowOffset, const uint32_t *__restrict__ t_tcA2B,
-                                           const uint32_t *__restrict__ t_rowIdx, uint32_t tall_rows, T *__restrict__ t_data) {
-    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n_entries; e += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t c = tcA2B[e];
-        if (c == kIdxMax) continue;
-        const uint32_t t = (uint32_t)(e / cw), lc = (uint32_t)(e % cw);
-        const uint32_t i = window_of_tile(rowOffset, eff, t);
-        const uint32_t g = win_group[i];
-        const uint32_t *list = t_tcA2B + (uint64_t)t_rowOffset[g] * cw;
-        uint32_t lo = 0, hi = ubase[g + 1] - ubase[g];  // the group's real columns, ascending
+__global__ void __launch_bounds__(kTilesBlock)
+tiles_kernel(const TileRun *__restrict__ runs, const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B,
+             const T *__restrict__ data, const uint32_t *__restrict__ rowIdx, const uint32_t *__restrict__ lists, uint8_t *__restrict__ images) {
+    constexpr uint32_t kPer = 16 / sizeof(T), kCW = 2 * kPer, kWindows = 128 / kShort;  // kPer: values of a lane, half a tile row
+    __shared__ __align__(16) uint8_t image[kRunTiles * 4096];
+    __shared__ uint32_t list[kRunTiles * kCW], first[kWindows], tiles_before[kWindows + 1], bound[2 * kWindows];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const TileRun r = runs[blockIdx.x];
+    const uint32_t n_windows = r.w1 - r.w0, n_list = r.n_tiles * kCW;
+    for (uint32_t k = threadIdx.x; k < n_list; k += kTilesBlock) list[k] = __ldg(lists + (uint64_t)r.list * kCW + k);
+    for (uint32_t k = threadIdx.x; k < r.n_tiles * 256; k += kTilesBlock) reinterpret_cast<uint4 *>(image)[k] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    const uint32_t lowest = list[0];
+    uint32_t n_real = n_list;  // the padding is at the end
+    while (list[n_real - 1] == kIdxMax) --n_real;
+    const uint32_t highest = list[n_real - 1];
+    if (threadIdx.x < 2 * n_windows) {  // where the run's columns begin and end in the windows' lists
+        const uint32_t w = r.w0 + threadIdx.x / 2, t0 = rowOffset[w];
+        const uint32_t *own = tcA2B + (uint64_t)t0 * kCW;
+        uint32_t lo = 0, hi = (rowOffset[w + 1] - t0) * kCW;
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo) / 2, c = own[mid];
+            if ((threadIdx.x & 1u) ? c <= highest : c < lowest) lo = mid + 1; else hi = mid;
+        }
+        bound[threadIdx.x] = lo;
+        if (!(threadIdx.x & 1u)) first[threadIdx.x / 2] = t0;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t sum = 0;
+        for (uint32_t k = 0; k < n_windows; ++k) {
+            const uint32_t begin = bound[2 * k], end = bound[2 * k + 1];
+            tiles_before[k] = sum;
+            first[k] += begin / kCW;
+            if (end > begin) sum += (end - 1) / kCW + 1 - begin / kCW;
+        }
+        tiles_before[n_windows] = sum;
+    }
+    __syncthreads();
+    const uint32_t n_tiles = tiles_before[n_windows];
+    struct Source {
+        uint32_t column, row;
+        alignas(16) T v[kPer];
+    };
+    auto load = [&](uint32_t i, Source &s) {
+        uint32_t k = 0;
+        while (i >= tiles_before[k + 1]) ++k;
+        const uint64_t t = first[k] + (i - tiles_before[k]);
+        s.column = __ldg(tcA2B + t * kCW + lane % kCW);
+        *reinterpret_cast<uint4 *>(s.v) = __ldcs(reinterpret_cast<const uint4 *>(data + (t * 32 + lane) * kPer));
+        s.row = __ldg(rowIdx + r.w0 + k) - r.row0 + (lane >> 1);
+    };
+    Source now, next;
+    if (warp < n_tiles) load(warp, next);
+    for (uint32_t i = warp; i < n_tiles; i += kTilesBlock / 32) {
+        now = next;
+        if (i + kTilesBlock / 32 < n_tiles) load(i + kTilesBlock / 32, next);
+        uint32_t lo = 0, hi = n_real;  // the slot of the lane's column
         while (lo < hi) {
             const uint32_t mid = lo + (hi - lo) / 2;
-            if (list[mid] < c) lo = mid + 1; else hi = mid;
+            if (list[mid] < now.column) lo = mid + 1; else hi = mid;
         }
-        // A tile image is 128 rows.  Windows of 256 rows keep, per window, the images of rows 0-127 of all
-        // its tiles and then those of rows 128-255 (each CTA of a pair reads its own run).
-        const uint32_t olc = lo % cw, shift = rowIdx[i] - t_rowIdx[g], part = shift / 128u, row_shift = shift % 128u;
-        const uint64_t g_first = t_rowOffset[g], g_tiles = t_rowOffset[g + 1] - g_first;
-        const uint64_t ot = g_first * (tall_rows / 128u) + part * g_tiles + lo / cw;
-        const T *src = data + ((uint64_t)t * kShort) * cw + lc;
-        T *dst = t_data + (ot * 128u + row_shift) * cw;
-        const uint32_t half = cw / 2;  // elements per 16-byte half of a tile row
-#pragma unroll 4
-        for (uint32_t lr = 0; lr < kShort; ++lr) {
-            const uint32_t flip = ((row_shift + lr) >> 2) & 1u;  // the 32-byte swizzle of the shared-memory image
-            dst[(uint64_t)lr * cw + (((olc / half) ^ flip) * half + olc % half)] = src[(uint64_t)lr * cw];
+        const uint32_t slot = lo < n_real && list[lo] == now.column ? lo : kIdxMax;
+        uint8_t *row = image + now.row * 32u;
+        const uint32_t flip = (now.row >> 2) & 1u;
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; ++k) {
+            const uint32_t at = __shfl_sync(0xffffffffu, slot, (lane & 1u) * kPer + k);
+            if (at == kIdxMax) continue;
+            const uint32_t in_tile = at % kCW;
+            *reinterpret_cast<T *>(row + at / kCW * 4096u + ((in_tile / kPer) ^ flip) * 16u + in_tile % kPer * sizeof(T)) = now.v[k];
         }
     }
+    __syncthreads();
+    uint4 *out = reinterpret_cast<uint4 *>(images + (uint64_t)r.image * 4096u);
+    for (uint32_t k = threadIdx.x; k < r.n_tiles * 256; k += kTilesBlock) __stcs(out + k, reinterpret_cast<const uint4 *>(image)[k]);
 }
 
 // Distinct columns in the lists of a run of 16-row tiles, one block per run.
@@ -140,6 +246,13 @@ void group_windows(const uint32_t *h_rowIdx, uint64_t eff, uint32_t kTall, std::
         (*win_group)[i] = (uint32_t)(group_first->size() - 1);
     }
     group_first->push_back(eff);
+}
+
+// (always the same limit, whoever else is about to launch)
+template <typename K>
+int allow_bit_sets(K kernel, int sets) {
+    B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sets * (int)kChunkWords * 4));
+    return B200SPMM_OK;
 }
 
 }  // namespace
@@ -182,100 +295,124 @@ int estimate_tall_tile_ratio(const b200spmm_btcf_info_t &info, const uint32_t *h
     return B200SPMM_OK;
 }
 
+int count_super_windows(const b200spmm_btcf_info_t &info, const uint32_t *h_rowOffset, const uint32_t *h_rowIdx, const uint32_t *d_tcA2B,
+                        SuperCounts *out) {
+    *out = SuperCounts();
+    const uint64_t eff = info.eff_row_windows;
+    std::vector<WindowPair> pairs;
+    for (uint64_t i = 0; i < eff;) {
+        SuperCounts::Pair w{(uint32_t)(h_rowIdx[i] / 256u * 256u), (uint32_t)i, (uint32_t)i, (uint32_t)i, {}};
+        while (w.mid < eff && h_rowIdx[w.mid] - w.row0 < 128u) ++w.mid;
+        w.end = w.mid;
+        while (w.end < eff && h_rowIdx[w.end] - w.row0 < 256u) ++w.end;
+        pairs.push_back(WindowPair{h_rowOffset[w.begin], h_rowOffset[w.mid], h_rowOffset[w.end]});
+        out->pairs.push_back(w);
+        i = w.end;
+    }
+    if (pairs.empty()) return B200SPMM_OK;
+    PoolScratch tmp;
+    WindowPair *d_pairs = nullptr;
+    uint32_t *d_counts = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&d_pairs, pairs.size()));
+    B200_CUDA_TRY(tmp.alloc(&d_counts, 3 * pairs.size()));
+    B200_CUDA_TRY(cudaMemcpy(d_pairs, pairs.data(), pairs.size() * sizeof(WindowPair), cudaMemcpyHostToDevice));
+    const uint32_t words = chunk_words(info.cols);
+    const int st = allow_bit_sets(count_kernel, 2);
+    if (st != B200SPMM_OK) return st;
+    count_kernel<<<(unsigned)pairs.size(), kMergeBlock, 2 * words * 4>>>(d_pairs, d_tcA2B, (uint32_t)info.col_window, info.cols, words, d_counts);
+    B200_CUDA_TRY(cudaGetLastError());
+    std::vector<uint32_t> counts(3 * pairs.size());
+    B200_CUDA_TRY(cudaMemcpy(counts.data(), d_counts, counts.size() * 4, cudaMemcpyDeviceToHost));
+    const uint32_t cw = (uint32_t)info.col_window;
+    for (size_t k = 0; k < pairs.size(); ++k) {
+        for (int j = 0; j < 3; ++j) out->pairs[k].tiles[j] = (counts[3 * k + j] + cw - 1) / cw;
+        out->tall_tiles += (uint64_t)out->pairs[k].tiles[0] + out->pairs[k].tiles[1];
+        out->pair_tiles += out->pairs[k].tiles[2];
+        out->tall_windows += (out->pairs[k].tiles[0] != 0) + (out->pairs[k].tiles[1] != 0);
+    }
+    return B200SPMM_OK;
+}
+
 void free_tall(TallFormat *t) {
-    pool_free(t->d_rowOffset);
+    pool_free(t->d_rowOffset);  // (d_rowIdx is behind it)
     pool_free(t->d_tcA2B);
-    pool_free(t->d_rowIdx);
     pool_free(t->d_data);
     *t = TallFormat();
 }
 
-int build_tall_device(const b200spmm_btcf_info_t &info, const uint32_t *h_rowOffset, const uint32_t *h_rowIdx,
-                      const uint32_t *d_rowOffset, const uint32_t *d_tcA2B, const void *d_data, const uint32_t *d_rowIdx,
-                      uint32_t tall_rows, TallFormat *out) {
+int build_tall_device(const b200spmm_btcf_info_t &info, const SuperCounts &counts, const uint32_t *h_rowOffset, const uint32_t *d_rowOffset,
+                      const uint32_t *d_tcA2B, const void *d_data, const uint32_t *d_rowIdx, uint32_t tall_rows, TallFormat *out) {
     *out = TallFormat();
     if (info.row_window != (int)kShort || (tall_rows != 128 && tall_rows != 256)) return B200SPMM_ERR_UNSUPPORTED;
-    const uint32_t kTall = tall_rows;
-    const uint64_t eff = info.eff_row_windows, cw = (uint64_t)info.col_window, tiles = info.total_tiles;
-    if (!eff || !tiles) return B200SPMM_OK;
-    const uint64_t n_entries = tiles * cw;
-    std::vector<uint32_t> win_group;
-    std::vector<uint64_t> group_first;
-    group_windows(h_rowIdx, eff, tall_rows, &win_group, &group_first);
-    const uint64_t n_groups = group_first.size() - 1;
-    std::vector<uint32_t> h_t_rowIdx(n_groups);
-    for (uint64_t g = 0; g < n_groups; ++g) h_t_rowIdx[g] = h_rowIdx[group_first[g]] / kTall * kTall;
-
-    PoolScratch tmp;
-    uint32_t *d_group = nullptr, *d_ubase = nullptr;
-    uint64_t *keys = nullptr, *keys_sorted = nullptr, *n_sel = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&d_group, eff));
-    B200_CUDA_TRY(tmp.alloc(&d_ubase, n_groups + 2));
-    B200_CUDA_TRY(tmp.alloc(&keys, n_entries));
-    B200_CUDA_TRY(tmp.alloc(&keys_sorted, n_entries));
-    B200_CUDA_TRY(tmp.alloc(&n_sel, 1));
-    B200_CUDA_TRY(cudaMemcpy(d_group, win_group.data(), eff * 4, cudaMemcpyHostToDevice));
-    tall_keys_kernel<<<grid_for(n_entries), kBlock>>>(d_rowOffset, d_tcA2B, d_group, (uint32_t)eff, (uint32_t)n_groups,
-                                                      (uint32_t)cw, n_entries, keys);
-    B200_CUDA_TRY(cudaGetLastError());
-    int group_bits = 1;
-    while ((1ull << group_bits) < n_groups + 1) ++group_bits;
-    size_t sort_bytes = 0, sel_bytes = 0;
-    B200_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, keys, keys_sorted, (int64_t)n_entries, 0, 32 + group_bits));
-    uint64_t *ukeys = keys;  // the unsorted keys are dead once sorted
-    B200_CUDA_TRY(cub::DeviceSelect::Unique(nullptr, sel_bytes, keys_sorted, ukeys, n_sel, (int64_t)n_entries));
-    uint8_t *cub_tmp = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&cub_tmp, std::max(sort_bytes, sel_bytes)));
-    B200_CUDA_TRY(cub::DeviceRadixSort::SortKeys(cub_tmp, sort_bytes, keys, keys_sorted, (int64_t)n_entries, 0, 32 + group_bits));
-    B200_CUDA_TRY(cub::DeviceSelect::Unique(cub_tmp, sel_bytes, keys_sorted, ukeys, n_sel, (int64_t)n_entries));
-    uint64_t n_unique = 0;
-    B200_CUDA_TRY(cudaMemcpy(&n_unique, n_sel, 8, cudaMemcpyDeviceToHost));
-    tall_group_base_kernel<<<(unsigned)((n_groups + 1 + kBlock - 1) / kBlock), kBlock>>>(ukeys, n_unique, (uint32_t)n_groups, d_ubase);
-    B200_CUDA_TRY(cudaGetLastError());
-    std::vector<uint32_t> ubase(n_groups + 1), t_rowOffset(n_groups + 1, 0);
-    B200_CUDA_TRY(cudaMemcpy(ubase.data(), d_ubase, (n_groups + 1) * 4, cudaMemcpyDeviceToHost));
-    uint64_t t_tiles = 0;
-    for (uint64_t g = 0; g < n_groups; ++g) {
-        t_tiles += ((uint64_t)(ubase[g + 1] - ubase[g]) + cw - 1) / cw;
-        t_rowOffset[g + 1] = (uint32_t)t_tiles;
-    }
-    if (t_tiles > 0xFFFFFFFFull) return B200SPMM_ERR_UNSUPPORTED;  // rowOffset is 32-bit
-
+    const uint32_t cw = (uint32_t)info.col_window, parts = tall_rows / 128;
+    // (images are numbered in 32 bits here, and rowOffset is 32-bit)
+    if ((tall_rows == 256 ? 2 * counts.pair_tiles : counts.tall_tiles) > 0xFFFFFFFFull) return B200SPMM_ERR_UNSUPPORTED;
+    std::vector<uint32_t> rowOffset{0}, rowIdx;
+    std::vector<WindowLists> windows;
+    std::vector<TileRun> runs;
     TallFormat t;
-    t.rows = kTall;
-    t.eff = n_groups;
-    t.tiles = t_tiles;
-    t.min_window_tiles = t_tiles;
-    for (uint64_t g = 0; g < n_groups; ++g) {
-        t.max_window_tiles = std::max<uint64_t>(t.max_window_tiles, t_rowOffset[g + 1] - t_rowOffset[g]);
-        t.min_window_tiles = std::min<uint64_t>(t.min_window_tiles, t_rowOffset[g + 1] - t_rowOffset[g]);
+    t.rows = tall_rows;
+    // windows [begin, end) of 16 rows with `n` tiles when merged; half j of a 256-row window has images [j n, j n + n)
+    auto add = [&](const SuperCounts::Pair &w, uint32_t begin, uint32_t end, uint32_t row0, uint32_t n) {
+        if (!n) return;
+        const uint32_t list = rowOffset.back();
+        windows.push_back(WindowLists{h_rowOffset[begin], h_rowOffset[end], list, n});
+        rowIdx.push_back(row0);
+        rowOffset.push_back(list + n);
+        t.max_window_tiles = std::max<uint64_t>(t.max_window_tiles, n);
+        t.min_window_tiles = windows.size() == 1 ? n : std::min<uint64_t>(t.min_window_tiles, n);
+        for (uint32_t j = 0; j < parts; ++j) {
+            const uint32_t b = parts == 1 ? begin : j ? w.mid : w.begin, e = parts == 1 ? end : j ? w.end : w.mid;
+            for (uint32_t k = 0; k < n; k += kRunTiles)
+                runs.push_back(TileRun{b, e, row0 + j * 128u, list + k, std::min(kRunTiles, n - k), list * parts + j * n + k});
+        }
+    };
+    for (const SuperCounts::Pair &w : counts.pairs) {
+        if (parts == 2) {
+            add(w, w.begin, w.end, w.row0, w.tiles[2]);
+        } else {
+            add(w, w.begin, w.mid, w.row0, w.tiles[0]);
+            add(w, w.mid, w.end, w.row0 + 128u, w.tiles[1]);
+        }
     }
+    t.eff = windows.size();
+    t.tiles = rowOffset.back();
+    if (!t.tiles) return B200SPMM_OK;
     struct Guard {
         TallFormat *t;
         ~Guard() { if (t) free_tall(t); }
     } guard{&t};
-    const uint64_t list_len = t_tiles * cw, data_len = t_tiles * kTall * cw;
-    B200_CUDA_TRY(pool_alloc(&t.d_rowOffset, n_groups + 1));
-    B200_CUDA_TRY(pool_alloc(&t.d_rowIdx, n_groups));
-    B200_CUDA_TRY(pool_alloc(&t.d_tcA2B, list_len));
-    B200_CUDA_TRY(pool_alloc_bytes(&t.d_data, data_len * info.elt_size, nullptr));
-    B200_CUDA_TRY(cudaMemcpy(t.d_rowOffset, t_rowOffset.data(), (n_groups + 1) * 4, cudaMemcpyHostToDevice));
-    B200_CUDA_TRY(cudaMemcpy(t.d_rowIdx, h_t_rowIdx.data(), n_groups * 4, cudaMemcpyHostToDevice));
-    B200_CUDA_TRY(cudaMemset(t.d_tcA2B, 0xFF, list_len * 4));
-    B200_CUDA_TRY(cudaMemset(t.d_data, 0, data_len * info.elt_size));
-    const uint64_t n_real = ubase[n_groups];
-    tall_scatter_columns_kernel<<<grid_for(n_real), kBlock>>>(ukeys, n_real, d_ubase, t.d_rowOffset, (uint32_t)cw, t.d_tcA2B);
+    // one copy brings all tables (a copy is 8 us, whatever it holds): rowOffset, the aligned tiles, rowIdx, windows, runs
+    std::vector<uint32_t> tables(rowOffset);
+    auto append = [&](const void *from, size_t bytes) {
+        const size_t at = tables.size();
+        tables.resize(at + bytes / 4);
+        std::memcpy(tables.data() + at, from, bytes);
+        return at;
+    };
+    const uint32_t none = 0;
+    const size_t aligned_at = append(&none, 4), rowIdx_at = append(rowIdx.data(), rowIdx.size() * 4),
+                 windows_at = append(windows.data(), windows.size() * sizeof(WindowLists)), runs_at = append(runs.data(), runs.size() * sizeof(TileRun));
+    B200_CUDA_TRY(pool_alloc(&t.d_rowOffset, tables.size()));
+    B200_CUDA_TRY(cudaMemcpy(t.d_rowOffset, tables.data(), tables.size() * 4, cudaMemcpyHostToDevice));
+    t.d_rowIdx = t.d_rowOffset + rowIdx_at;
+    t.d_aligned = t.d_rowOffset + aligned_at;
+    const auto *d_windows = reinterpret_cast<const WindowLists *>(t.d_rowOffset + windows_at);
+    const auto *d_runs = reinterpret_cast<const TileRun *>(t.d_rowOffset + runs_at);
+    B200_CUDA_TRY(pool_alloc(&t.d_tcA2B, t.tiles * cw));
+    B200_CUDA_TRY(pool_alloc_bytes(&t.d_data, t.tiles * parts * 4096, nullptr));
+    const uint32_t words = chunk_words(info.cols);
+    const int st = allow_bit_sets(lists_kernel, 1);
+    if (st != B200SPMM_OK) return st;
+    lists_kernel<<<(unsigned)windows.size(), kMergeBlock, words * 4>>>(d_windows, d_tcA2B, cw, info.cols, words, t.d_tcA2B, t.d_aligned);
     B200_CUDA_TRY(cudaGetLastError());
     if (info.elt_size == 2)
-        tall_scatter_values_kernel<uint16_t><<<grid_for(n_entries), kBlock>>>(
-            d_rowOffset, d_tcA2B, static_cast<const uint16_t *>(d_data), d_rowIdx, d_group, (uint32_t)eff, (uint32_t)cw,
-            n_entries, d_ubase, t.d_rowOffset, t.d_tcA2B, t.d_rowIdx, kTall, static_cast<uint16_t *>(t.d_data));
+        tiles_kernel<uint16_t><<<(unsigned)runs.size(), kTilesBlock>>>(d_runs, d_rowOffset, d_tcA2B, static_cast<const uint16_t *>(d_data), d_rowIdx,
+                                                                       t.d_tcA2B, static_cast<uint8_t *>(t.d_data));
     else
-        tall_scatter_values_kernel<uint32_t><<<grid_for(n_entries), kBlock>>>(
-            d_rowOffset, d_tcA2B, static_cast<const uint32_t *>(d_data), d_rowIdx, d_group, (uint32_t)eff, (uint32_t)cw,
-            n_entries, d_ubase, t.d_rowOffset, t.d_tcA2B, t.d_rowIdx, kTall, static_cast<uint32_t *>(t.d_data));
+        tiles_kernel<uint32_t><<<(unsigned)runs.size(), kTilesBlock>>>(d_runs, d_rowOffset, d_tcA2B, static_cast<const uint32_t *>(d_data), d_rowIdx,
+                                                                       t.d_tcA2B, static_cast<uint8_t *>(t.d_data));
     B200_CUDA_TRY(cudaGetLastError());
-    B200_CUDA_TRY(cudaDeviceSynchronize());
     *out = t;
     guard.t = nullptr;
     return B200SPMM_OK;

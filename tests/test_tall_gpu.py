@@ -227,3 +227,49 @@ def test_few_windows_are_cut_into_parts(dt, rows, n, window):
         assert torch.equal(out, got)
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("dt,rows,cols,n", [(np.float16, 1290, 777, 200), (np.float32, 1100, 900, 72)])
+def test_small_matrices_have_super_windows_too(dt, rows, cols, n):
+    # from a few thousand 16-row tiles on; a window of its own at the end, and one half without entries
+    import torch
+    rows, cols, rp, ci, v = random_csr(rows, cols, 0.2, 9, dt, empty_rows=[(384, 512)])
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    try:
+        B = dense_b(cols, n, 3, dt)
+        dC = torch.full((rows, n), float("nan"), device="cuda")
+        plan.spmm(torch.from_numpy(B).cuda(), dC)
+        assert plan.launch_info().row_window == 128 and plan.tall_format(256) is None
+        parity.check(dC.cpu().numpy(), rows, rp, ci, v, B)
+        want = oracle.csr2btcf_nobitmap(rows, cols, rp, ci, v, 128, 16 if dt == np.float16 else 8)
+        got = plan.tall_format()
+        for k in ("rowOffset", "tcA2B", "rowIdx"):
+            assert np.array_equal(got[k], getattr(want, k)), k
+        assert np.array_equal(got["data"].view(np.uint8), np.ascontiguousarray(want.data).view(np.uint8))
+    finally:
+        plan.close()
+
+
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+def test_merging_more_columns_than_a_bit_set_holds(dt, tall):
+    # lists that reach over two and three chunks of 393,216 columns, at their edges too; several runs of tiles a window
+    edge = 393216
+    near = np.concatenate([np.arange(k * edge - 3, k * edge + 3) for k in (1, 2)])
+    rng = np.random.default_rng(4)
+    cols, rows = 2 * edge + 70_000, 300
+    per_row = [np.unique(np.concatenate([near[r % 4:: 1 + r % 3], rng.integers(0, cols, 40)])) for r in range(rows)]
+    ci = np.concatenate(per_row).astype(np.uint32)
+    rp = np.concatenate([[0], np.cumsum([c.size for c in per_row])]).astype(np.uint32)
+    v = rng.uniform(0.1, 1, ci.size).astype(np.float32).astype(dt)
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    try:
+        for height in (128, 256):
+            got = plan.tall_format(height)
+            if got is None:  # (this plan was asked for 128 rows)
+                continue
+            want = oracle.csr2btcf_nobitmap(rows, cols, rp, ci, v, height, 16 if dt == np.float16 else 8)
+            for k in ("rowOffset", "tcA2B", "rowIdx"):
+                assert np.array_equal(got[k], getattr(want, k)), k
+            assert np.array_equal(got["data"].view(np.uint8), np.ascontiguousarray(want.data).view(np.uint8))
+    finally:
+        plan.close()
