@@ -1,16 +1,21 @@
 // Condensed tiles -> row units, on the device.
 //
-//   1. the tiles of every window in runs of at most kRunTiles; a warp counts the stored values of each of the
-//      sixteen rows of its run (one 16-byte load per lane is half a tile row)
-//   2. per (window, row): running sums over the window's runs -> row lengths; scans over the rows -> the units,
-//      slots and bands
-//   3. units sorted by length, longest first (CUB radix sort, a few key bits), their batches numbered in that order;
-//      where there are bands, the list once more with the bands apart
+//   1. the tile stream in runs of kRunTiles, and a run cut where a window ends; a warp counts the stored values of each of
+//      the sixteen rows of its run (one 16-byte load per lane is half a tile row)
+//   2. per (window, row): running sums over the window's runs -> row lengths, and how many units there are of every length;
+//      one scan over the rows -> the units, slots and bands.  The longest come first, so the lengths alone say where every
+//      unit of a length lies and where its batches do: the host's one wait
+//   3. every row puts its units into the list; where there are bands, the list once more with the bands apart (CUB radix
+//      sort, four key bits)
 //   4. the warps of step 1 write (column, value) to the place of their row's unit
+// Eight launches and one wait before the last.  With the units sorted (CUB), three scans and a launch for each small step there
+// were 26; the plan of a graph of 60,000 nodes and 700,000 entries took 232 us instead of 158, of 10,000 nodes 200 instead of 123.
 // A stored value is one whose bits are not all zero (an explicit zero adds nothing to a product), in a row and a column
 // of the matrix: the arrays may be a caller's, and what lies in a padded slot or below the last row multiplies nothing.
 #include <algorithm>
 #include <cub/cub.cuh>
+#include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
 
 #include "common.hpp"
 #include "device_pool.hpp"
@@ -24,11 +29,10 @@ constexpr int kBlock = 256;
 // row of 10,000 entries: 419 us for write_entries_kernel with runs of 256 tiles).
 constexpr uint32_t kRunTiles = 16;
 constexpr uint32_t kMaxBands = 8;
-constexpr uint32_t kEmptyKey = 512;  // sort key of the units: longest first, rows without entries last
-constexpr int kUnitKeyBits = 10;
+// The lengths of the units: kMaxUnitEntries - entries, so the longest come first; rows without entries are behind all of them.
+constexpr uint32_t kLengths = kMaxUnitEntries, kEmpty = kLengths;
 constexpr uint32_t kEmptyBandKey = kMaxBands;  // sort key of the bands: their units, then their rows without entries
 constexpr int kBandKeyBits = 4;
-constexpr uint32_t kMaxLenAt = 4 + 2 * (kMaxBands + 1) + kLongUnits;  // in the table of totals: the longest row
 constexpr uint64_t kMinBandedCost = 2000000;  // bands pay where one keeps the GPU busy for tens of microseconds
 // For the bands a row counts as this many entries: its store is 4 bytes a feature where a gathered entry is 2.
 constexpr uint64_t kRowCost = 2;
@@ -39,17 +43,66 @@ inline int grid_for(uint64_t n) { return (int)std::max<uint64_t>(1, std::min<uin
 
 __host__ __device__ __forceinline__ uint32_t pieces_of(uint32_t len, uint32_t cap) { return len <= cap ? 1u : (len + cap - 1) / cap; }
 
-__global__ void run_counts_kernel(const uint32_t *__restrict__ rowOffset, uint32_t eff, uint32_t *__restrict__ n_runs) {
-    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w < eff) n_runs[w] = (rowOffset[w + 1] - rowOffset[w] + kRunTiles - 1) / kRunTiles;
-    if (w == eff) n_runs[w] = 0;
+// Running sums over the rows, this one included: (entries << 32 | units) and (cut rows << 32 | slots).
+struct RowSums {
+    unsigned long long a, b;
+};
+struct AddSums {
+    __host__ __device__ RowSums operator()(const RowSums &x, const RowSums &y) const { return {x.a + y.a, x.b + y.b}; }
+};
+struct RowTerms {
+    const uint32_t *row_len;
+    uint32_t cap;
+    __host__ __device__ RowSums operator()(uint32_t r) const {
+        const uint32_t len = row_len[r], n = pieces_of(len, cap);
+        return {((unsigned long long)len << 32) | n, n > 1 ? (1ull << 32) | n : 0ull};
+    }
+};
+
+// What the host waits for.
+struct RowTotals {
+    uint32_t entries, units, cut_rows, slots;
+    uint32_t with_entries, n_batches, long_units[kLongUnits];  // units that have entries; and see RowsFormat
+    uint32_t max_len;
+    uint32_t band_row[kMaxBands + 1], band_cut[kMaxBands + 1];  // the bands' first rows and cut rows
+};
+
+// Where the units of a length lie in the list, and the four neighbours' batches (quads) in front of theirs.
+struct LengthTables {
+    uint32_t count[kLengths];         // units of every length
+    uint32_t start[kLengths + 1];     // place of the first one; of the first row without entries
+    uint32_t quad_steps[kLengths];    // steps of the quads that begin before it
+    uint32_t cursor[kLengths + 1];    // places taken so far
+};
+
+// Run `id` of window w (tiles chunk * kRunTiles .. of the stream, as far as they are the window's; none where a window ends
+// with a chunk) has the number chunk + w.
+__host__ __device__ __forceinline__ uint32_t first_run(uint32_t tile, uint32_t w) { return tile / kRunTiles + w; }
+
+// run -> window; clears what the kernels behind it count in
+__global__ void run_windows_kernel(const uint32_t *__restrict__ rowOffset, uint32_t eff, uint32_t rows, uint32_t *__restrict__ run_window,
+                                   uint32_t *__restrict__ row_len, LengthTables *__restrict__ tables, RowTotals *__restrict__ totals) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < eff)
+        for (uint32_t r = first_run(rowOffset[i], i), end = first_run(rowOffset[i + 1], i + 1); r < end; ++r) run_window[r] = i;
+    if (i < rows) row_len[i] = 0;
+    if (blockIdx.x == 0) {
+        for (uint32_t k = threadIdx.x; k < kLengths; k += blockDim.x) tables->count[k] = 0;
+        if (threadIdx.x == 0) totals->max_len = 0;
+    }
 }
 
-__global__ void run_windows_kernel(const uint32_t *__restrict__ run_first, uint32_t eff, uint32_t *__restrict__ run_window) {
-    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= eff) return;
-    for (uint32_t r = run_first[w]; r < run_first[w + 1]; ++r) run_window[r] = w;
-}
+// The tiles of a run.
+struct RunTiles {
+    uint32_t w, t0, t1, end;  // window, tiles [t0, t1), end of the window
+    __device__ __forceinline__ RunTiles(uint32_t run, const uint32_t *__restrict__ run_window, const uint32_t *__restrict__ rowOffset) {
+        w = run_window[run];
+        const uint32_t chunk = (run - w) * kRunTiles;
+        end = rowOffset[w + 1];
+        t0 = max(chunk, rowOffset[w]);
+        t1 = min(chunk + kRunTiles, end);
+    }
+};
 
 // a[k] of registers, by halves: two predicates less a register than comparing k with every index
 template <int kN>
@@ -98,12 +151,16 @@ __device__ __forceinline__ void load_columns(uint32_t (&cols)[kPer], const uint3
 template <typename T>
 __global__ void __launch_bounds__(kBlock)
 run_rows_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B, const T *__restrict__ data,
-                const uint32_t *__restrict__ rowIdx, const uint32_t *__restrict__ run_first, const uint32_t *__restrict__ run_window,
-                uint32_t eff, uint32_t rows, uint32_t cols, bool loose, uint32_t *__restrict__ counts) {
-    const uint32_t lane = threadIdx.x & 31u, n_runs = run_first[eff];
+                const uint32_t *__restrict__ rowIdx, const uint32_t *__restrict__ run_window,
+                uint32_t n_runs, uint32_t rows, uint32_t cols, bool loose, uint32_t *__restrict__ counts) {
+    const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t run = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); run < n_runs; run += gridDim.x * (kBlock / 32)) {
-        const uint32_t w = run_window[run], t0 = rowOffset[w] + (run - run_first[w]) * kRunTiles;
-        const uint32_t end = rowOffset[w + 1], t1 = min(t0 + kRunTiles, end);
+        const RunTiles tiles(run, run_window, rowOffset);
+        const uint32_t w = tiles.w, t0 = tiles.t0, t1 = tiles.t1, end = tiles.end;
+        if (t0 >= t1) {
+            if (lane < 16) counts[(uint64_t)run * 16 + lane] = 0;
+            continue;
+        }
         alignas(16) uint32_t of[Piece<T>::kPer];
         if (t1 == end) load_columns(of, tcA2B, end - 1, lane);
         uint32_t mine = 0;
@@ -134,136 +191,153 @@ run_rows_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restri
 }
 
 // thread (window, row of it): counts of its runs become what the earlier runs hold; the sum is the row's length
-__global__ void row_lengths_kernel(const uint32_t *__restrict__ run_first, const uint32_t *__restrict__ rowIdx, uint32_t eff,
-                                   uint32_t rows, uint32_t *__restrict__ counts, uint32_t *__restrict__ row_len,
-                                   uint32_t *__restrict__ max_len) {
+__global__ void __launch_bounds__(kBlock)
+row_lengths_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ rowIdx, uint32_t eff, uint32_t rows, uint32_t cap,
+                   uint32_t *__restrict__ counts, uint32_t *__restrict__ row_len, LengthTables *__restrict__ tables,
+                   RowTotals *__restrict__ totals) {
+    __shared__ uint32_t here[kLengths];
+    for (uint32_t k = threadIdx.x; k < kLengths; k += kBlock) here[k] = 0;
+    __syncthreads();
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t w = (uint32_t)(i >> 4), r = (uint32_t)i & 15u;
-    if (w >= eff) return;
     uint32_t sum = 0;
-    const uint32_t end = run_first[w + 1];
-    for (uint32_t run = run_first[w]; run < end; run += 8) {
-        uint32_t c[8];
+    if (w < eff) {
+        const uint32_t end = first_run(rowOffset[w + 1], w + 1);
+        for (uint32_t run = first_run(rowOffset[w], w); run < end; run += 8) {
+            uint32_t c[8];
 #pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) c[k] = run + k < end ? counts[(uint64_t)(run + k) * 16 + r] : 0u;
+            for (uint32_t k = 0; k < 8; ++k) c[k] = run + k < end ? counts[(uint64_t)(run + k) * 16 + r] : 0u;
 #pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) {
-            if (run + k < end) counts[(uint64_t)(run + k) * 16 + r] = sum;
-            sum += c[k];
+            for (uint32_t k = 0; k < 8; ++k) {
+                if (run + k < end) counts[(uint64_t)(run + k) * 16 + r] = sum;
+                sum += c[k];
+            }
         }
+        if (rowIdx[w] + r < rows) row_len[rowIdx[w] + r] = sum;
     }
-    if (rowIdx[w] + r < rows) row_len[rowIdx[w] + r] = sum;
-    if (sum > *max_len) atomicMax(max_len, sum);
+    if (sum) {  // (none below the last row)
+        const uint32_t n = pieces_of(sum, cap);
+        if (n > 1) atomicAdd(&here[kMaxUnitEntries - cap], n - 1);
+        atomicAdd(&here[kMaxUnitEntries - (sum - (n - 1) * cap)], 1u);
+    }
+    const uint32_t most = __reduce_max_sync(0xffffffffu, sum);
+    if ((threadIdx.x & 31u) == 0 && most > totals->max_len) atomicMax(&totals->max_len, most);
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < kLengths; k += kBlock)
+        if (here[k]) atomicAdd(&tables->count[k], here[k]);
 }
 
-// Inclusive scans follow over both: (entries << 32 | units) and (cut rows << 32 | slots).
-__global__ void row_terms_kernel(const uint32_t *__restrict__ row_len, uint32_t rows, uint32_t cap, unsigned long long *__restrict__ a,
-                                 unsigned long long *__restrict__ b) {
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    const uint32_t len = row_len[r], n = pieces_of(len, cap);
-    a[r] = ((unsigned long long)len << 32) | n;
-    b[r] = n > 1 ? (1ull << 32) | n : 0ull;
+__device__ __forceinline__ uint32_t batches_of_length(uint32_t key) { return (kMaxUnitEntries - key + kUnitBatch - 1) / kUnitBatch; }
+__device__ __forceinline__ uint32_t quads_before(uint32_t place) { return (place + 3) / 4; }
+
+// Sum over the threads before this one.
+__device__ __forceinline__ uint32_t block_exclusive_sum(uint32_t mine, uint32_t *warp_sums) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t upto = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, upto, d);
+        if (lane >= (uint32_t)d) upto += x;
+    }
+    __syncthreads();
+    if (lane == 31) warp_sums[warp] = upto;
+    __syncthreads();
+    uint32_t before = upto - mine;
+    for (uint32_t k = 0; k < warp; ++k) before += warp_sums[k];
+    return before;
 }
 
-// totals[0..3]: entries, units, cut rows, slots; then per band its first row and cut row
-__global__ void row_bands_kernel(uint32_t rows, const unsigned long long *__restrict__ a, const unsigned long long *__restrict__ b,
-                                 uint32_t *__restrict__ totals) {
-    const uint32_t k = threadIdx.x;
+// One block of a thread per length.  Four neighbours of the list form a quad and are stored batch by batch side by side (batch
+// k of all four, then batch k + 1): the groups of a warp, which walk neighbours, read their entries from the same lines.  A
+// quad takes the steps of its first unit, which is its longest.
+static_assert(kLengths == kBlock, "a thread for every length");
+__global__ void __launch_bounds__(kBlock)
+row_totals_kernel(uint32_t rows, const RowSums *__restrict__ sums, LengthTables *__restrict__ tables, RowTotals *__restrict__ totals) {
+    __shared__ uint32_t warp_sums[kBlock / 32];
+    const uint32_t k = threadIdx.x, count = tables->count[k], start = block_exclusive_sum(count, warp_sums);
+    const uint32_t steps = (quads_before(start + count) - quads_before(start)) * batches_of_length(k);  // of the quads that begin here
+    const uint32_t steps_before = block_exclusive_sum(steps, warp_sums);
+    tables->start[k] = tables->cursor[k] = start;
+    tables->quad_steps[k] = steps_before;
+    // units of at least 2 << j batches: those of at most this key
+    for (uint32_t j = 0; j < kLongUnits; ++j)
+        if (k == kMaxUnitEntries - kUnitBatch * ((2u << j) - 1u) - 1u) totals->long_units[j] = start + count;
+    if (k == kLengths - 1) {
+        tables->start[kEmpty] = tables->cursor[kEmpty] = totals->with_entries = start + count;
+        totals->n_batches = 4 * (steps_before + steps);
+    }
+    const RowSums all = sums[rows - 1];
     if (k == 0) {
-        totals[0] = (uint32_t)(a[rows - 1] >> 32);
-        totals[1] = (uint32_t)a[rows - 1];
-        totals[2] = (uint32_t)(b[rows - 1] >> 32);
-        totals[3] = (uint32_t)b[rows - 1];
+        totals->entries = (uint32_t)(all.a >> 32);
+        totals->units = (uint32_t)all.a;
+        totals->cut_rows = (uint32_t)(all.b >> 32);
+        totals->slots = (uint32_t)all.b;
     }
     if (k > kMaxBands) return;
-    const uint64_t cost = (a[rows - 1] >> 32) + kRowCost * rows;
+    const uint64_t cost = (all.a >> 32) + kRowCost * rows;
     const uint32_t bands = cost >= kMinBandedCost ? kMaxBands : 1u;
     uint32_t lo = 0, hi = rows;  // rows before which k / bands of the cost lie
     const uint64_t want = cost * k / bands;
     while (k < bands && lo < hi) {
         const uint32_t mid = lo + (hi - lo) / 2;
-        if ((a[mid] >> 32) + kRowCost * (mid + 1) <= want) lo = mid + 1; else hi = mid;
+        if ((sums[mid].a >> 32) + kRowCost * (mid + 1) <= want) lo = mid + 1; else hi = mid;
     }
     if (k >= bands) lo = rows;
-    totals[4 + k * 2] = lo;
-    totals[5 + k * 2] = lo ? (uint32_t)(b[lo - 1] >> 32) : 0u;
+    totals->band_row[k] = lo;
+    totals->band_cut[k] = lo ? (uint32_t)(sums[lo - 1].b >> 32) : 0u;
 }
 
-// one thread per row: sort keys of its units, and its line of the split table
-__global__ void unit_keys_kernel(const uint32_t *__restrict__ row_len, uint32_t rows, uint32_t cap,
-                                 const unsigned long long *__restrict__ a, const unsigned long long *__restrict__ b,
-                                 uint32_t *__restrict__ keys, uint32_t *__restrict__ ids,
-                                 uint32_t *__restrict__ unit_row, RowSplit *__restrict__ splits) {
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+// Thread r: the units of row r take places among those of their length (in the order in which blocks of rows ask), and its
+// line of the split table.
+__global__ void __launch_bounds__(kBlock)
+place_units_kernel(const uint32_t *__restrict__ row_len, uint32_t rows, uint32_t cap, const RowSums *__restrict__ sums, LengthTables *__restrict__ tables,
+                   const RowTotals *__restrict__ totals, uint32_t bands, uint2 *__restrict__ units, uint32_t *__restrict__ unit_batch,
+                   RowSplit *__restrict__ splits, uint32_t *__restrict__ band_keys, uint32_t *__restrict__ batches, uint32_t batch_words) {
+    __shared__ uint32_t base[kLengths + 1];
+    for (uint32_t k = threadIdx.x; k <= kLengths; k += kBlock) base[k] = 0;
+    __syncthreads();
+    const uint32_t r = blockIdx.x * kBlock + threadIdx.x;
+    uint32_t n = 0, full = 0, last_key = 0, rank_full = 0, rank_last = 0;
+    const uint32_t full_key = kMaxUnitEntries - cap;
+    if (r < rows) {
+        const uint32_t len = row_len[r];
+        n = pieces_of(len, cap);
+        full = n - 1;
+        last_key = len ? kMaxUnitEntries - (len - full * cap) : kEmpty;
+        if (full) rank_full = atomicAdd(&base[full_key], full);
+        rank_last = atomicAdd(&base[last_key], 1u);
+    }
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k <= kLengths; k += kBlock)
+        if (base[k]) base[k] = atomicAdd(&tables->cursor[k], base[k]);
+    __syncthreads();
+    if (blockIdx.x == 0 && threadIdx.x < batch_words)  // the batch that belongs to nobody
+        batches[(uint64_t)totals->n_batches * batch_words + threadIdx.x] = batch_words == kBatchWords<true> ? (threadIdx.x == kTargetWord<true> ? kNoTarget : 0u)
+                                                                                                 : (threadIdx.x == kTargetWord<false> ? kNoTarget : 0u);
     if (r >= rows) return;
-    const uint32_t len = row_len[r], n = pieces_of(len, cap), first = (uint32_t)a[r] - n;
+    uint32_t band = 0;
+    for (uint32_t k = 1; k < bands; ++k) band += r >= totals->band_row[k] ? 1u : 0u;
+    const uint32_t first_unit = (uint32_t)sums[r].a - n;
     for (uint32_t q = 0; q < n; ++q) {
-        const uint32_t part = min(len - q * cap, cap);
-        keys[first + q] = part ? kMaxUnitEntries - part : kEmptyKey;
-        ids[first + q] = first + q;
-        unit_row[first + q] = r;
+        const uint32_t key = q < full ? full_key : last_key, place = q < full ? base[full_key] + rank_full + q : base[last_key] + rank_last;
+        uint32_t first = 0;
+        if (key != kEmpty) {
+            uint32_t of = key;  // the length of the quad's first unit
+            while (tables->start[of] > (place & ~3u)) --of;
+            first = 4 * (tables->quad_steps[of] + (place / 4 - quads_before(tables->start[of])) * batches_of_length(of)) + (place & 3u);
+            unit_batch[first_unit + q] = first;
+        }
+        units[place] = key != kEmpty ? make_uint2(first, batches_of_length(key)) : make_uint2(r, 0u);
+        if (bands > 1) band_keys[place] = (key != kEmpty ? 0u : kEmptyBandKey) | band;
     }
-    if (n > 1) splits[(uint32_t)(b[r] >> 32) - 1] = RowSplit{r, (uint32_t)b[r] - n, (uint32_t)b[r]};
+    if (n > 1) splits[(uint32_t)(sums[r].b >> 32) - 1] = RowSplit{r, (uint32_t)sums[r].b - n, (uint32_t)sums[r].b};
 }
 
-__device__ __forceinline__ uint32_t batches_of_key(uint32_t key) {
-    return key == kEmptyKey ? 0u : (kMaxUnitEntries - key + kUnitBatch - 1) / kUnitBatch;
-}
-
-// Four neighbours of the sorted list form a quad and are stored batch by batch side by side (batch k of all four,
-// then batch k + 1): the groups of a warp, which walk neighbours, read their entries from the same lines.
-__global__ void quad_lengths_kernel(const uint32_t *__restrict__ keys, uint32_t n_units, uint32_t n_quads, uint32_t *__restrict__ quads) {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q > n_quads) return;
-    uint32_t most = 0;
-    for (uint32_t i = 4 * q; i < min(4 * q + 4, n_units); ++i) most = max(most, batches_of_key(keys[i]));
-    quads[q] = most;  // (0 for q == n_quads: its place in the running sum is the total)
-}
-
-// place i of the sorted list: where the unit's batches lie, the targets in them, and the key of its band
-template <bool kTf32>
-__global__ void place_units_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ ids, const uint32_t *__restrict__ quads,
-                                   uint32_t n_units, uint32_t cap, const uint32_t *__restrict__ unit_row, const uint32_t *__restrict__ row_len,
-                                   const unsigned long long *__restrict__ a, const unsigned long long *__restrict__ b,
-                                   uint2 *__restrict__ units, uint32_t *__restrict__ unit_batch, uint32_t *__restrict__ batches,
-                                   uint32_t bands, const uint32_t *__restrict__ totals, uint32_t *__restrict__ band_keys) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_units) return;
-    const uint32_t u = ids[i], r = unit_row[u], n = pieces_of(row_len[r], cap), first = quads[i >> 2] * 4 + (i & 3u);
-    const uint32_t q = u - ((uint32_t)a[r] - n);  // which piece of its row
-    const uint32_t n_batches = batches_of_key(keys[i]);
-    units[i] = make_uint2(n_batches ? first : r, n_batches);
-    unit_batch[u] = first;
-    if (bands > 1) {
-        uint32_t band = 0;
-        for (uint32_t k = 1; k < bands; ++k) band += r >= totals[4 + k * 2] ? 1u : 0u;
-        band_keys[i] = (n_batches ? 0u : kEmptyBandKey) | band;
-    }
-    for (uint32_t k = 0; k < n_batches; ++k)
-        batches[(uint64_t)(first + 4 * k) * kBatchWords<kTf32> + kTargetWord<kTf32>] =
-            k + 1 < n_batches ? kNoTarget : n > 1 ? kSlotTarget | ((uint32_t)b[r] - n + q) : r;
-    if (i == n_units - 1) {  // the batch that belongs to nobody
-        uint32_t *w = batches + (uint64_t)quads[(n_units + 3) / 4] * 4 * kBatchWords<kTf32>;
-        for (uint32_t k = 0; k < kBatchWords<kTf32>; ++k) w[k] = k == kTargetWord<kTf32> ? kNoTarget : 0u;
-    }
-}
-
-// band k <= bands: the places of its first unit and of its first row without entries (keys: of the bands, or of the units
-// where there is one band); the number of batches; and how many units have at least 2 << j batches (unit_keys)
-__global__ void band_units_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ unit_keys, const uint32_t *__restrict__ quads,
-                                  uint32_t n_units, uint32_t bands, uint32_t *__restrict__ out) {
-    const uint32_t i = threadIdx.x, k = i >> 1, n_bounds = 2 * bands + 2;
-    if (i > n_bounds + kLongUnits) return;
-    if (i == n_bounds) {
-        out[i] = 4 * quads[(n_units + 3) / 4];
-        return;
-    }
-    uint32_t want = ((i & 1u) ? (bands > 1 ? kEmptyBandKey : kEmptyKey) : 0u) + k;
-    if (i > n_bounds) {  // the first key that stands for fewer batches
-        keys = unit_keys;
-        want = kMaxUnitEntries - kUnitBatch * ((2u << (i - n_bounds - 1)) - 1u);
-    }
+// band k <= bands: the places of its first unit and of its first row without entries in the list of the bands
+__global__ void band_units_kernel(const uint32_t *__restrict__ keys, uint32_t n_units, uint32_t bands, uint32_t *__restrict__ out) {
+    const uint32_t i = threadIdx.x, k = i >> 1;
+    if (k > bands) return;
+    const uint32_t want = ((i & 1u) ? kEmptyBandKey : 0u) + k;
     uint32_t lo = 0, hi = n_units;
     while (lo < hi) {
         const uint32_t mid = lo + (hi - lo) / 2;
@@ -296,29 +370,36 @@ __device__ __forceinline__ void split_value(T v, uint32_t n, T *first, T *unit) 
 template <typename T>
 __global__ void __launch_bounds__(kBlock)
 write_entries_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B, const T *__restrict__ data,
-                     const uint32_t *__restrict__ rowIdx, const uint32_t *__restrict__ run_first,
-                     const uint32_t *__restrict__ run_window, uint32_t eff, uint32_t rows, uint32_t n_cols, bool loose, uint32_t cap,
-                     const uint32_t *__restrict__ counts,
-                     const uint32_t *__restrict__ row_len, const unsigned long long *__restrict__ a,
-                     const uint32_t *__restrict__ unit_batch, uint32_t *__restrict__ batches) {
+                     const uint32_t *__restrict__ rowIdx, const uint32_t *__restrict__ run_window, uint32_t n_runs, uint32_t rows, uint32_t n_cols,
+                     bool loose, uint32_t cap, const uint32_t *__restrict__ counts, const uint32_t *__restrict__ row_len,
+                     const RowSums *__restrict__ sums, const uint32_t *__restrict__ unit_batch, uint32_t *__restrict__ batches) {
     constexpr int kPer = Piece<T>::kPer;
-    constexpr uint32_t kWords = kBatchWords<sizeof(T) == 4>;
-    const uint32_t lane = threadIdx.x & 31u, n_runs = run_first[eff];
+    constexpr uint32_t kWords = kBatchWords<sizeof(T) == 4>, kTo = kTargetWord<sizeof(T) == 4>;
+    const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t run = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); run < n_runs; run += gridDim.x * (kBlock / 32)) {
-        const uint32_t w = run_window[run], t0 = rowOffset[w] + (run - run_first[w]) * kRunTiles;
-        const uint32_t w_end = rowOffset[w + 1], t1 = min(t0 + kRunTiles, w_end), row = min(rowIdx[w] + (lane >> 1), rows - 1);
-        const uint32_t len = row_len[row], limit = rowIdx[w] + (lane >> 1) < rows ? n_cols : 0u;
-        const uint32_t *unit = unit_batch + ((uint32_t)a[row] - pieces_of(len, cap));  // first batches of the row's units
+        const RunTiles tiles(run, run_window, rowOffset);
+        const uint32_t w = tiles.w, t0 = tiles.t0, t1 = tiles.t1, w_end = tiles.end, row = min(rowIdx[w] + (lane >> 1), rows - 1);
+        if (t0 >= t1) continue;
+        const uint32_t len = row_len[row], limit = rowIdx[w] + (lane >> 1) < rows ? n_cols : 0u, n_pieces = pieces_of(len, cap);
+        const RowSums sum = sums[row];
+        const uint32_t *unit = unit_batch + ((uint32_t)sum.a - n_pieces);  // first batches of the row's units
         uint32_t at = counts[(uint64_t)run * 16 + (lane >> 1)];  // entries of the row so far
         // Everything a lane reads comes ahead of its stores and for all lanes at once - the unit it starts in, a tile's
         // columns and values while the tile before is written: fetched at its first entry, one by one, they cost the warp
         // a round trip to L2 per entry (43 us of a matrix of 700,000 entries, 60,000 rows; now 32).
-        uint32_t piece = min(at / cap, pieces_of(len, cap) - 1u), piece_end = (piece + 1) * cap;
+        uint32_t piece = min(at / cap, n_pieces - 1u), piece_end = (piece + 1) * cap;
         uint32_t fill = (0u - min(len - piece * cap, cap)) % kUnitBatch;  // slots before the second entry of the unit
-        uint32_t *out = batches + (uint64_t)unit[piece] * kWords;
+        uint32_t *out = batches + (uint64_t)(len ? unit[piece] : 0u) * kWords;
+        // the unit's last batch holds its target, the others none; a batch's first entry writes it
+        auto target = [&](uint32_t e) {
+            const uint32_t entries = min(len - piece * cap, cap);
+            if (e / kUnitBatch + 1 < (entries + kUnitBatch - 1) / kUnitBatch) return kNoTarget;
+            return n_pieces > 1 ? kSlotTarget | ((uint32_t)sum.b - n_pieces + piece) : row;
+        };
         auto put = [&](uint32_t e, uint32_t col, T v) {
             uint32_t *words = out + (e / kUnitBatch) * (4 * kWords);
             words[e % kUnitBatch] = col;
+            if (e % kUnitBatch == 0) words[kTo] = target(e);
             reinterpret_cast<T *>(words + kUnitBatch)[e % kUnitBatch] = v;
         };
         Piece<T> next;
@@ -378,16 +459,16 @@ uint32_t unit_entries_for(uint64_t nnz, uint64_t rows, int n_sms) {
 template <typename T>
 __global__ void __launch_bounds__(kBlock)
 write_csr_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B, const T *__restrict__ data,
-                 const uint32_t *__restrict__ rowIdx, const uint32_t *__restrict__ run_first, const uint32_t *__restrict__ run_window,
-                 uint32_t eff, uint32_t rows, uint32_t n_cols, const uint32_t *__restrict__ counts,
-                 const unsigned long long *__restrict__ a, uint32_t *__restrict__ cols_out, T *__restrict__ vals_out) {
+                 const uint32_t *__restrict__ rowIdx, const uint32_t *__restrict__ run_window,
+                 uint32_t n_runs, uint32_t rows, uint32_t n_cols, const uint32_t *__restrict__ counts,
+                 const RowSums *__restrict__ sums, uint32_t *__restrict__ cols_out, T *__restrict__ vals_out) {
     constexpr int kPer = Piece<T>::kPer;
-    const uint32_t lane = threadIdx.x & 31u, n_runs = run_first[eff];
+    const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t run = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); run < n_runs; run += gridDim.x * (kBlock / 32)) {
-        const uint32_t w = run_window[run], t0 = rowOffset[w] + (run - run_first[w]) * kRunTiles;
-        const uint32_t t1 = min(t0 + kRunTiles, rowOffset[w + 1]), row = min(rowIdx[w] + (lane >> 1), rows - 1);
+        const RunTiles tiles(run, run_window, rowOffset);
+        const uint32_t w = tiles.w, t0 = tiles.t0, t1 = tiles.t1, row = min(rowIdx[w] + (lane >> 1), rows - 1);
         const uint32_t limit = rowIdx[w] + (lane >> 1) < rows ? n_cols : 0u;
-        uint32_t at = (row ? (uint32_t)(a[row - 1] >> 32) : 0u) + counts[(uint64_t)run * 16 + (lane >> 1)];
+        uint32_t at = (row ? (uint32_t)(sums[row - 1].a >> 32) : 0u) + counts[(uint64_t)run * 16 + (lane >> 1)];
 #pragma unroll 2
         for (uint32_t t = t0; t < t1; ++t) {
             Piece<T> p;
@@ -414,7 +495,7 @@ write_csr_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restr
 // and one more of the classes below c that have it.
 template <typename T>
 __global__ void __launch_bounds__(kBlock)
-narrow_entries_kernel(const uint32_t *__restrict__ cols, const T *__restrict__ vals, const unsigned long long *__restrict__ a, uint32_t rows,
+narrow_entries_kernel(const uint32_t *__restrict__ cols, const T *__restrict__ vals, const RowSums *__restrict__ sums, uint32_t rows,
                       uint32_t n_blocks, uint32_t *__restrict__ seg, uint32_t *__restrict__ entries) {
     extern __shared__ uint32_t narrow_smem[];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, row = blockIdx.x * (kBlock / 32) + warp;
@@ -422,7 +503,7 @@ narrow_entries_kernel(const uint32_t *__restrict__ cols, const T *__restrict__ v
     if (row >= rows) return;
     for (uint32_t k = lane; k < 2 * n_blocks * 8; k += 32) count[k] = 0;
     __syncwarp();
-    const uint32_t begin = row ? (uint32_t)(a[row - 1] >> 32) : 0u, end = (uint32_t)(a[row] >> 32);
+    const uint32_t begin = row ? (uint32_t)(sums[row - 1].a >> 32) : 0u, end = (uint32_t)(sums[row].a >> 32);
     for (uint32_t e = begin + lane; e < end; e += 32) atomicAdd(&count[(cols[e] / kNarrowCols) * 8 + (cols[e] & 7u)], 1u);
     __syncwarp();
     uint32_t *my_seg = seg + (uint64_t)row * (n_blocks + 1);
@@ -457,14 +538,14 @@ narrow_entries_kernel(const uint32_t *__restrict__ cols, const T *__restrict__ v
 }
 
 // CTA k: rows from the first one whose cost reaches k / n_ctas of the total on
-__global__ void narrow_cuts_kernel(const unsigned long long *__restrict__ a, uint32_t rows, uint32_t n_ctas, uint32_t *__restrict__ cut) {
+__global__ void narrow_cuts_kernel(const RowSums *__restrict__ sums, uint32_t rows, uint32_t n_ctas, uint32_t *__restrict__ cut) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k > n_ctas) return;
-    const uint64_t total = (a[rows - 1] >> 32) + kNarrowRowCost * rows, want = total * k / n_ctas;
+    const uint64_t total = (sums[rows - 1].a >> 32) + kNarrowRowCost * rows, want = total * k / n_ctas;
     uint32_t lo = 0, hi = rows;
     while (lo < hi) {
         const uint32_t mid = lo + (hi - lo) / 2;
-        if ((a[mid] >> 32) + kNarrowRowCost * (mid + 1ull) <= want) lo = mid + 1; else hi = mid;
+        if ((sums[mid].a >> 32) + kNarrowRowCost * (mid + 1ull) <= want) lo = mid + 1; else hi = mid;
     }
     cut[k] = k == n_ctas ? rows : lo;
 }
@@ -495,9 +576,9 @@ bool narrow_pays(uint64_t nnz, uint64_t rows, uint64_t cols, uint64_t max_len, i
 }
 
 int build_narrow(const b200spmm_btcf_info_t &info, uint64_t nnz, const uint32_t *d_rowOffset, const uint32_t *d_tcA2B, const void *d_data,
-                 const uint32_t *d_rowIdx, int n_sms, const uint32_t *run_first, const uint32_t *run_window, int run_grid,
-                 const uint32_t *counts, const unsigned long long *a, NarrowFormat *out) {
-    const uint32_t rows = (uint32_t)info.rows, eff = (uint32_t)info.eff_row_windows, words = (uint32_t)info.elt_size / 2;
+                 const uint32_t *d_rowIdx, int n_sms, const uint32_t *run_window, uint32_t n_runs, int run_grid,
+                 const uint32_t *counts, const RowSums *sums, NarrowFormat *out) {
+    const uint32_t rows = (uint32_t)info.rows, words = (uint32_t)info.elt_size / 2;
     const uint32_t n_cols = (uint32_t)info.cols;
     NarrowFormat f;
     struct Guard {
@@ -522,15 +603,15 @@ int build_narrow(const b200spmm_btcf_info_t &info, uint64_t nnz, const uint32_t 
     const int grid = (int)((rows + kBlock / 32 - 1) / (kBlock / 32));
     const size_t smem = (size_t)(kBlock / 32) * 2 * f.n_blocks * 8 * 4;
     if (info.elt_size == 2) {
-        write_csr_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, static_cast<const uint16_t *>(d_data), d_rowIdx, run_first,
-                                                         run_window, eff, rows, n_cols, counts, a, cols, static_cast<uint16_t *>(vals));
-        narrow_entries_kernel<uint16_t><<<grid, kBlock, smem>>>(cols, static_cast<const uint16_t *>(vals), a, rows, f.n_blocks, f.d_seg, f.d_entries);
+        write_csr_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, static_cast<const uint16_t *>(d_data), d_rowIdx,
+                                                         run_window, n_runs, rows, n_cols, counts, sums, cols, static_cast<uint16_t *>(vals));
+        narrow_entries_kernel<uint16_t><<<grid, kBlock, smem>>>(cols, static_cast<const uint16_t *>(vals), sums, rows, f.n_blocks, f.d_seg, f.d_entries);
     } else {
-        write_csr_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, static_cast<const uint32_t *>(d_data), d_rowIdx, run_first,
-                                                         run_window, eff, rows, n_cols, counts, a, cols, static_cast<uint32_t *>(vals));
-        narrow_entries_kernel<uint32_t><<<grid, kBlock, smem>>>(cols, static_cast<const uint32_t *>(vals), a, rows, f.n_blocks, f.d_seg, f.d_entries);
+        write_csr_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, static_cast<const uint32_t *>(d_data), d_rowIdx,
+                                                         run_window, n_runs, rows, n_cols, counts, sums, cols, static_cast<uint32_t *>(vals));
+        narrow_entries_kernel<uint32_t><<<grid, kBlock, smem>>>(cols, static_cast<const uint32_t *>(vals), sums, rows, f.n_blocks, f.d_seg, f.d_entries);
     }
-    narrow_cuts_kernel<<<(int)(f.n_ctas / kBlock + 1), kBlock>>>(a, rows, f.n_ctas, f.d_cut);
+    narrow_cuts_kernel<<<(int)(f.n_ctas / kBlock + 1), kBlock>>>(sums, rows, f.n_ctas, f.d_cut);
     B200_CUDA_TRY(cudaGetLastError());
     std::vector<uint32_t> cut(f.n_ctas + 1);
     B200_CUDA_TRY(cudaMemcpy(cut.data(), f.d_cut, cut.size() * 4, cudaMemcpyDeviceToHost));
@@ -559,122 +640,99 @@ int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
         ~Guard() { if (f) free_rows(f); }
     } guard{&f};
     PoolScratch tmp;
-    const uint64_t max_runs = eff + tiles / kRunTiles;
-    uint32_t *n_runs = nullptr, *run_first = nullptr, *run_window = nullptr, *counts = nullptr, *row_len = nullptr, *totals = nullptr;
-    unsigned long long *a = nullptr, *b = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&n_runs, eff + 1));
-    B200_CUDA_TRY(tmp.alloc(&run_first, eff + 1));
-    B200_CUDA_TRY(tmp.alloc(&run_window, max_runs));
-    B200_CUDA_TRY(tmp.alloc(&counts, max_runs * 16));
+    const uint64_t n_runs64 = tiles / kRunTiles + eff;  // first_run behind the last window
+    if (n_runs64 > 0xFFFFFFFFull) return B200SPMM_OK;
+    const uint32_t n_runs = (uint32_t)n_runs64;
+    uint32_t *run_window = nullptr, *counts = nullptr, *row_len = nullptr;
+    RowSums *sums = nullptr;
+    LengthTables *tables = nullptr;
+    RowTotals *totals = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&run_window, n_runs));
+    B200_CUDA_TRY(tmp.alloc(&counts, n_runs64 * 16));
     B200_CUDA_TRY(tmp.alloc(&row_len, rows));
-    B200_CUDA_TRY(tmp.alloc(&a, rows));
-    B200_CUDA_TRY(tmp.alloc(&b, rows));
-    B200_CUDA_TRY(tmp.alloc(&totals, kMaxLenAt + 1));
-    size_t run_bytes = 0, row_bytes = 0;
-    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, run_bytes, n_runs, run_first, (int64_t)eff + 1));
-    B200_CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, row_bytes, a, a, (int64_t)rows));
+    B200_CUDA_TRY(tmp.alloc(&sums, rows));
+    B200_CUDA_TRY(tmp.alloc(&tables, 1));
+    B200_CUDA_TRY(tmp.alloc(&totals, 1));
+    auto terms = thrust::make_transform_iterator(thrust::make_counting_iterator<uint32_t>(0), RowTerms{row_len, cap});
+    size_t scan_bytes = 0;
+    B200_CUDA_TRY(cub::DeviceScan::InclusiveScan(nullptr, scan_bytes, terms, sums, AddSums{}, (int64_t)rows));
     uint8_t *scan_tmp = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&scan_tmp, std::max(run_bytes, row_bytes)));
+    B200_CUDA_TRY(tmp.alloc(&scan_tmp, scan_bytes));
 
-    run_counts_kernel<<<eff / kBlock + 1, kBlock>>>(d_rowOffset, eff, n_runs);
-    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(scan_tmp, run_bytes, n_runs, run_first, (int64_t)eff + 1));
-    run_windows_kernel<<<(eff + kBlock - 1) / kBlock, kBlock>>>(run_first, eff, run_window);
     const bool f16 = info.elt_size == 2;
     const uint16_t *data16 = static_cast<const uint16_t *>(d_data);
     const uint32_t *data32 = static_cast<const uint32_t *>(d_data);
-    const int run_grid = grid_for(max_runs * 32), row_grid = (int)((rows + kBlock - 1) / kBlock);
-    if (f16) run_rows_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data16, d_rowIdx, run_first, run_window, eff, rows, cols, loose, counts);
-    else run_rows_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data32, d_rowIdx, run_first, run_window, eff, rows, cols, loose, counts);
-    uint32_t *max_len = totals + kMaxLenAt;
-    B200_CUDA_TRY(cudaMemsetAsync(row_len, 0, (size_t)rows * 4));
-    B200_CUDA_TRY(cudaMemsetAsync(max_len, 0, 4));
-    row_lengths_kernel<<<(unsigned)(((uint64_t)eff * 16 + kBlock - 1) / kBlock), kBlock>>>(run_first, d_rowIdx, eff, rows, counts, row_len, max_len);
-    row_terms_kernel<<<row_grid, kBlock>>>(row_len, rows, cap, a, b);
-    B200_CUDA_TRY(cub::DeviceScan::InclusiveSum(scan_tmp, row_bytes, a, a, (int64_t)rows));
-    B200_CUDA_TRY(cub::DeviceScan::InclusiveSum(scan_tmp, row_bytes, b, b, (int64_t)rows));
-    row_bands_kernel<<<1, 32>>>(rows, a, b, totals);
+    const int run_grid = grid_for(n_runs64 * 32), row_grid = (int)(((uint64_t)rows + kBlock - 1) / kBlock);
+    run_windows_kernel<<<(unsigned)((std::max<uint64_t>(eff, rows) + kBlock - 1) / kBlock), kBlock>>>(d_rowOffset, eff, rows, run_window, row_len, tables, totals);
+    if (f16) run_rows_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data16, d_rowIdx, run_window, n_runs, rows, cols, loose, counts);
+    else run_rows_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data32, d_rowIdx, run_window, n_runs, rows, cols, loose, counts);
+    row_lengths_kernel<<<(unsigned)(((uint64_t)eff * 16 + kBlock - 1) / kBlock), kBlock>>>(d_rowOffset, d_rowIdx, eff, rows, cap, counts, row_len, tables, totals);
+    B200_CUDA_TRY(cub::DeviceScan::InclusiveScan(scan_tmp, scan_bytes, terms, sums, AddSums{}, (int64_t)rows));
+    row_totals_kernel<<<1, kBlock>>>(rows, sums, tables, totals);
     B200_CUDA_TRY(cudaGetLastError());
-    uint32_t h[kMaxLenAt + 1];
-    B200_CUDA_TRY(cudaMemcpy(h, totals, sizeof(h), cudaMemcpyDeviceToHost));
-    if (!force_rows && (double)h[0] > max_fill * (double)tiles * 16.0 * info.col_window) {
-        if (narrow_pays(h[0], rows, info.cols, h[kMaxLenAt], n_sms))
-            return build_narrow(info, h[0], d_rowOffset, d_tcA2B, d_data, d_rowIdx, n_sms, run_first, run_window, run_grid, counts, a, narrow);
+    RowTotals h;
+    B200_CUDA_TRY(cudaMemcpy(&h, totals, sizeof(h), cudaMemcpyDeviceToHost));
+    if (!force_rows && (double)h.entries > max_fill * (double)tiles * 16.0 * info.col_window) {
+        if (narrow_pays(h.entries, rows, info.cols, h.max_len, n_sms))
+            return build_narrow(info, h.entries, d_rowOffset, d_tcA2B, d_data, d_rowIdx, n_sms, run_window, n_runs, run_grid, counts, sums, narrow);
         return B200SPMM_OK;
     }
-    const uint32_t h_max_len = h[kMaxLenAt];
-    f.nnz = h[0];
-    f.n_units = h[1];
-    f.n_splits = h[2];
-    f.n_slots = h[3];
+    f.nnz = h.entries;
+    f.n_units = h.units;
+    f.n_splits = h.cut_rows;
+    f.n_slots = h.slots;
+    f.n_batches = h.n_batches;
+    f.most_batches = (std::min(h.max_len, cap) + kUnitBatch - 1) / kUnitBatch;
+    std::copy(h.long_units, h.long_units + kLongUnits, f.long_units);
     uint32_t bands = 0;
-    while (h[4 + 2 * bands] != rows) ++bands;
-    for (uint32_t k = 0; k <= bands; ++k) f.bands.push_back(RowBand{0, 0, h[5 + 2 * k], h[4 + 2 * k]});
+    while (h.band_row[bands] != rows) ++bands;
+    for (uint32_t k = 0; k <= bands; ++k) f.bands.push_back(RowBand{0, h.with_entries, h.band_cut[k], h.band_row[k]});
+    f.bands[bands].unit = h.with_entries;  // (all units, then all rows without entries)
+    f.bands[bands].empty = f.n_units;
 
-    // Every unit rounds up to a batch, every quad to its longest unit: up to three longest units in all, as the lengths
-    // fall from first to last, and three more where a quad holds the last units.
-    const uint64_t max_batches = f.nnz / kUnitBatch + f.n_units + 6 * (kMaxUnitEntries / kUnitBatch) + 8;
-    if (max_batches > 0xFFFFFFFFull || f.n_slots >= kSlotTarget - 1) return B200SPMM_OK;
+    // (the last batch belongs to nobody)
+    const uint64_t n_batches = (uint64_t)f.nnz / kUnitBatch + f.n_units + 6 * (kMaxUnitEntries / kUnitBatch) + 8;
+    if (n_batches > 0xFFFFFFFFull || f.n_slots >= kSlotTarget - 1) return B200SPMM_OK;
     const uint32_t words = info.elt_size == 2 ? kBatchWords<false> : kBatchWords<true>;
-    uint32_t *keys[2] = {}, *ids[2] = {}, *unit_row = nullptr;
-    cudaError_t e = pool_alloc(&f.d_batches, max_batches * words);
+    uint32_t *unit_batch = nullptr, *band_keys[2] = {}, *band_places = nullptr;
+    cudaError_t e = pool_alloc(&f.d_batches, ((uint64_t)f.n_batches + 1) * words);
     if (e == cudaSuccess) e = pool_alloc(&f.d_units, f.n_units);
     if (e == cudaSuccess && bands > 1) e = pool_alloc(&f.d_band_units, f.n_units);
     if (e == cudaSuccess) e = pool_alloc(&f.d_splits, f.n_splits);
-    for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
-        e = tmp.alloc(&keys[k], f.n_units);
-        if (e == cudaSuccess) e = tmp.alloc(&ids[k], f.n_units);
-    }
-    if (e == cudaSuccess) e = tmp.alloc(&unit_row, f.n_units);
+    if (e == cudaSuccess) e = tmp.alloc(&unit_batch, f.n_units);
+    for (int k = 0; k < 2 && e == cudaSuccess && bands > 1; ++k) e = tmp.alloc(&band_keys[k], f.n_units);
+    if (e == cudaSuccess && bands > 1) e = tmp.alloc(&band_places, 2 * bands + 2);
     if (e == cudaErrorMemoryAllocation) {  // no room: the tile kernels still work
         cudaGetLastError();
         return B200SPMM_OK;
     }
     B200_CUDA_TRY(e);
-    const uint32_t n_quads = (f.n_units + 3) / 4;
-    uint32_t *quads = nullptr, *unit_batch = keys[0], *band_keys = ids[0];  // (free again once the pairs are sorted)
-    B200_CUDA_TRY(tmp.alloc(&quads, n_quads + 1));
-    unit_keys_kernel<<<row_grid, kBlock>>>(row_len, rows, cap, a, b, keys[0], ids[0], unit_row, f.d_splits);
-    size_t sort_bytes = 0, batch_bytes = 0, band_bytes = 0;
-    B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, keys[0], keys[1], ids[0], ids[1], (int64_t)f.n_units, 0, kUnitKeyBits));
-    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, batch_bytes, quads, quads, (int64_t)n_quads + 1));
-    if (bands > 1)
-        B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, band_bytes, band_keys, unit_row, f.d_units, f.d_band_units, (int64_t)f.n_units, 0, kBandKeyBits));
-    uint8_t *sort_tmp = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&sort_tmp, std::max({sort_bytes, batch_bytes, band_bytes})));
-    B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, keys[0], keys[1], ids[0], ids[1], (int64_t)f.n_units, 0, kUnitKeyBits));
-    quad_lengths_kernel<<<(int)(n_quads / kBlock + 1), kBlock>>>(keys[1], f.n_units, n_quads, quads);
-    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(sort_tmp, batch_bytes, quads, quads, (int64_t)n_quads + 1));
-    const int unit_grid = (int)((f.n_units + kBlock - 1) / kBlock);
-    if (f16) {
-        place_units_kernel<false><<<unit_grid, kBlock>>>(keys[1], ids[1], quads, f.n_units, cap, unit_row, row_len, a, b, f.d_units,
-                                                         unit_batch, f.d_batches, bands, totals, band_keys);
-        write_entries_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data16, d_rowIdx, run_first, run_window, eff, rows, cols, loose, cap,
-                                                             counts, row_len, a, unit_batch, f.d_batches);
-    } else {
-        place_units_kernel<true><<<unit_grid, kBlock>>>(keys[1], ids[1], quads, f.n_units, cap, unit_row, row_len, a, b, f.d_units,
-                                                        unit_batch, f.d_batches, bands, totals, band_keys);
-        write_entries_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data32, d_rowIdx, run_first, run_window, eff, rows, cols, loose, cap,
-                                                             counts, row_len, a, unit_batch, f.d_batches);
-    }
-    const uint32_t *sorted_bands = keys[1];
-    if (bands > 1) {  // (the units of a band keep their order)
-        B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sort_tmp, band_bytes, band_keys, unit_row, f.d_units, f.d_band_units, (int64_t)f.n_units, 0, kBandKeyBits));
-        sorted_bands = unit_row;
-    }
-    band_units_kernel<<<1, 32>>>(sorted_bands, keys[1], quads, f.n_units, bands, totals);
+    place_units_kernel<<<row_grid, kBlock>>>(row_len, rows, cap, sums, tables, totals, bands, f.d_units, unit_batch, f.d_splits, band_keys[0], f.d_batches, words);
+    if (f16)
+        write_entries_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data16, d_rowIdx, run_window, n_runs, rows, cols, loose, cap, counts,
+                                                             row_len, sums, unit_batch, f.d_batches);
+    else
+        write_entries_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data32, d_rowIdx, run_window, n_runs, rows, cols, loose, cap, counts,
+                                                             row_len, sums, unit_batch, f.d_batches);
     B200_CUDA_TRY(cudaGetLastError());
-    B200_CUDA_TRY(cudaMemcpy(h, totals, (2 * bands + 3 + kLongUnits) * 4, cudaMemcpyDeviceToHost));
-    for (uint32_t k = 0; k <= bands; ++k) {
-        f.bands[k].unit = h[2 * k];
-        f.bands[k].empty = h[2 * k + 1];
+    if (bands > 1) {  // (the units of a band keep their order)
+        size_t sort_bytes = 0;
+        B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, band_keys[0], band_keys[1], f.d_units, f.d_band_units, (int64_t)f.n_units, 0, kBandKeyBits));
+        uint8_t *sort_tmp = nullptr;
+        B200_CUDA_TRY(tmp.alloc(&sort_tmp, sort_bytes));
+        B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, band_keys[0], band_keys[1], f.d_units, f.d_band_units, (int64_t)f.n_units, 0, kBandKeyBits));
+        band_units_kernel<<<1, 32>>>(band_keys[1], f.n_units, bands, band_places);
+        B200_CUDA_TRY(cudaGetLastError());
+        uint32_t places[2 * kMaxBands + 2];
+        B200_CUDA_TRY(cudaMemcpy(places, band_places, (2 * bands + 2) * 4, cudaMemcpyDeviceToHost));
+        for (uint32_t k = 0; k < bands; ++k) {
+            f.bands[k].unit = places[2 * k];
+            f.bands[k].empty = places[2 * k + 1];
+        }
     }
-    f.bands[bands].unit = f.bands[0].empty;  // (all units, then all rows without entries)
-    f.bands[bands].empty = f.n_units;
-    f.n_batches = h[2 * bands + 2];
-    f.most_batches = (std::min(h_max_len, cap) + kUnitBatch - 1) / kUnitBatch;
-    for (uint32_t k = 0; k < kLongUnits; ++k) f.long_units[k] = h[2 * bands + 3 + k];
-    if (!force_rows && narrow_pays(f.nnz, rows, info.cols, h_max_len, n_sms)) {
-        const int st = build_narrow(info, f.nnz, d_rowOffset, d_tcA2B, d_data, d_rowIdx, n_sms, run_first, run_window, run_grid, counts, a, narrow);
+    B200_CUDA_TRY(cudaDeviceSynchronize());
+    if (!force_rows && narrow_pays(f.nnz, rows, info.cols, h.max_len, n_sms)) {
+        const int st = build_narrow(info, f.nnz, d_rowOffset, d_tcA2B, d_data, d_rowIdx, n_sms, run_window, n_runs, run_grid, counts, sums, narrow);
         if (st != B200SPMM_OK) return st;
     }
     *out = f;
