@@ -26,8 +26,9 @@ namespace {
 
 constexpr int kBlock = 256;
 // A hub window has thousands of tiles: short runs, or its warps are what everybody waits for (60,000 nodes, hub
-// row of 10,000 entries: 419 us for write_entries_kernel with runs of 256 tiles).
-constexpr uint32_t kRunTiles = 16;
+// row of 10,000 entries: 419 us for write_entries_kernel with runs of 256 tiles).  A plan, in us, with runs of 16 / 8 / 4:
+// 60,000 nodes 147 / 138 / 136, 10,000 nodes 122 / 99 / 91, 150,001 nodes, tf32 276 / 280 / 300.
+constexpr uint32_t kRunTiles = 8;
 constexpr uint32_t kMaxBands = 8;
 // The lengths of the units: kMaxUnitEntries - entries, so the longest come first; rows without entries are behind all of them.
 constexpr uint32_t kLengths = kMaxUnitEntries, kEmpty = kLengths;
@@ -278,11 +279,11 @@ row_totals_kernel(uint32_t rows, const RowSums *__restrict__ sums, LengthTables 
     const uint32_t bands = cost >= kMinBandedCost ? kMaxBands : 1u;
     uint32_t lo = 0, hi = rows;  // rows before which k / bands of the cost lie
     const uint64_t want = cost * k / bands;
-    while (k < bands && lo < hi) {
+    while (k && k < bands && lo < hi) {
         const uint32_t mid = lo + (hi - lo) / 2;
         if ((sums[mid].a >> 32) + kRowCost * (mid + 1) <= want) lo = mid + 1; else hi = mid;
     }
-    if (k >= bands) lo = rows;
+    if (!k || k >= bands) lo = k ? rows : 0u;
     totals->band_row[k] = lo;
     totals->band_cut[k] = lo ? (uint32_t)(sums[lo - 1].b >> 32) : 0u;
 }
