@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kRowsThreads, kRowsBlocksPerSm) spmm_rows_kern
         // (a group of a team has nothing to fetch where fewer batches than groups are left)
         const uint32_t at = !kTeams ? unit.x : t < unit.y ? unit.x + 4u * t : p.n_batches;
 #pragma unroll
-        for (uint32_t k = 0; k < kQ; ++k) e[k] = __ldg(batches + (uint64_t)at * kQ + k);
+        for (uint32_t k = 0; k < kQ; ++k) e[k] = ptx::ld_global_nc_v4_ahead(batches + (uint64_t)at * kQ + k);
     };
     u += stride;
     fetch();
