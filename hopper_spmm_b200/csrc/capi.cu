@@ -1,6 +1,7 @@
 // C ABI of the library (include/b200_spmm.h): format handles, device plans, launches.
 // Replaces the host side of the reference's operator, fp16_spmm (src/fp16.cu:221-281).
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -622,50 +623,6 @@ int launch_narrow_vecs(const NarrowParams &prm, int vecs, unsigned n_ctas, size_
     return B200SPMM_OK;
 }
 
-// Column blocks per group for B of width n: as many as fit shared memory, 0 if the kernel does not take it.  Every
-// 16-byte word of a row of B adds to it - pruned 28672 x 8192 weight, fp16: 35, 68, 89, 146 us for 8, 16, 24, 32
-// columns - while the tile kernels take the same time up to 64 features (98 us; tf32: 86 and 133 us for 8 and 16
-// columns against 186), so it ends at 24 fp16 or 16 tf32 columns.
-uint32_t narrow_group_blocks(const b200spmm_plan *p, int64_t n) {
-    const NarrowFormat &f = p->narrow;
-    const int64_t vecs = n * p->info.elt_size / 16;
-    if (!f.n_ctas || vecs > (p->info.dtype == B200SPMM_TF32 ? kNarrowMaxVecs : kNarrowMaxVecs - 1)) return 0;
-    uint32_t g = f.n_blocks;
-    while (g && narrow_smem_bytes((uint32_t)vecs, (uint32_t)p->info.cols, g, f.n_blocks, f.max_rows, (uint32_t)n) > kNarrowSmemMax) --g;
-    return g;
-}
-
-int launch_narrow(b200spmm_plan *p, uint32_t group_blocks, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
-                  cudaStream_t stream) {
-    const NarrowFormat &f = p->narrow;
-    NarrowParams prm{};
-    prm.entries = f.d_entries;
-    prm.seg = f.d_seg;
-    prm.cut = f.d_cut;
-    prm.n_blocks = f.n_blocks;
-    prm.group_blocks = group_blocks;
-    prm.B = d_B;
-    prm.C = d_C;
-    prm.ldb = ldb;
-    prm.ldc = ldc;
-    prm.cols = (uint32_t)p->info.cols;
-    prm.n = (uint32_t)n;
-    prm.c_is_half = c_dtype == B200SPMM_C_F16;
-    const int vecs = (int)(n * p->info.elt_size / 16);
-    const size_t smem = narrow_smem_bytes((uint32_t)vecs, prm.cols, group_blocks, f.n_blocks, f.max_rows, prm.n);
-    const int st = p->info.dtype == B200SPMM_TF32 ? launch_narrow_vecs<true>(prm, vecs, f.n_ctas, smem, stream)
-                                                  : launch_narrow_vecs<false>(prm, vecs, f.n_ctas, smem, stream);
-    if (st != B200SPMM_OK) return st;
-    p->last.n_ctas = (int)f.n_ctas;
-    p->last.threads = kNarrowThreads;
-    p->last.feature_slab = 64;
-    p->last.n_slabs = 1;
-    p->last.smem_bytes = (int64_t)smem;
-    p->last.kernel_launches = 1;
-    p->last.row_window = kRowWindow;
-    return B200SPMM_OK;
-}
-
 // How long a launch takes, in microseconds, to choose between the tile kernels.  A super-window launch lasts as many
 // rounds of its CTAs or pairs as its items need, each as long as the longest window, so a matrix with one heavy window
 // stays with 16 rows; the 16-row kernel spreads its tiles evenly over all CTAs.  It pays long before every SM has an
@@ -725,6 +682,59 @@ bool use_tall(const b200spmm_plan *p, int64_t n) {
     const TallLaunch t = tall_launch(p, p->tall, n);
     if (t.parts == 1 && n <= 128 && p->info.total_tiles < kPairMinShortTiles) return false;
     return t.micros < short_micros(p, n);
+}
+
+// Column blocks per group for B of width n: as many as fit shared memory, 0 if the kernel does not take it.  Every
+// 16-byte word of a row of B adds to its time - pruned 28672 x 8192 weight, fp16: 33, 64, 84, 123 us for 8, 16, 24, 32
+// columns; a warp has a row, so 33 rows a CTA take as long as 64 - while the tile kernels take the same up to 64 features (89
+// us; tf32: 98 us for 8 and 16 columns).  Up to 24 fp16 and 16 tf32 columns it is left for super-windows only, where these
+// are expected to be faster (24 columns: 4904 x 6773 at 13 % 33 us against 21, 12000 x 5000 at 20 % 44 against 32); 32 fp16
+// columns go to it where it is expected to be faster than all tiles (1100 x 1100 at 20 % 11.6 -> 7.5 us, 1682 x 1536 at 11 % 13.5 -> 10.0, 3000 x 3000 at 12 %
+// 19.2 -> 17.0), if all of B fits shared memory (2000 x 8000 at 6 %, in two halves, 36 us against 20).
+uint32_t narrow_group_blocks(const b200spmm_plan *p, int64_t n) {
+    const NarrowFormat &f = p->narrow;
+    const int64_t vecs = n * p->info.elt_size / 16;
+    const bool tf32 = p->info.dtype == B200SPMM_TF32;
+    if (!f.n_ctas || vecs > kNarrowMaxVecs) return 0;
+    uint32_t g = f.n_blocks;
+    while (g && narrow_smem_bytes((uint32_t)vecs, (uint32_t)p->info.cols, g, f.n_blocks, f.max_rows, (uint32_t)n) > kNarrowSmemMax) --g;
+    if (!g || p->rows_only) return vecs < kNarrowMaxVecs || tf32 ? g : 0;
+    const double rows = (double)p->info.rows / f.n_ctas, rounds = std::ceil(rows / 32.0) * 32.0 / rows;
+    const double micros = 4.0 + (double)p->info.nnzs * (double)vecs * 1.05e-6 * (148.0 / p->n_sms) * rounds * (g == f.n_blocks ? 1.0 : tf32 || vecs == kNarrowMaxVecs ? 1.5 : 1.05);
+    const TallLaunch tall = p->tall.tiles && !p->gather_cpasync ? tall_launch(p, p->tall, n) : TallLaunch{1e30, 1};
+    if (vecs < kNarrowMaxVecs || tf32) return tall.micros < micros ? 0 : g;
+    return g == f.n_blocks && micros < tall.micros && micros < short_micros(p, n) ? g : 0;
+}
+
+int launch_narrow(b200spmm_plan *p, uint32_t group_blocks, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
+                  cudaStream_t stream) {
+    const NarrowFormat &f = p->narrow;
+    NarrowParams prm{};
+    prm.entries = f.d_entries;
+    prm.seg = f.d_seg;
+    prm.cut = f.d_cut;
+    prm.n_blocks = f.n_blocks;
+    prm.group_blocks = group_blocks;
+    prm.B = d_B;
+    prm.C = d_C;
+    prm.ldb = ldb;
+    prm.ldc = ldc;
+    prm.cols = (uint32_t)p->info.cols;
+    prm.n = (uint32_t)n;
+    prm.c_is_half = c_dtype == B200SPMM_C_F16;
+    const int vecs = (int)(n * p->info.elt_size / 16);
+    const size_t smem = narrow_smem_bytes((uint32_t)vecs, prm.cols, group_blocks, f.n_blocks, f.max_rows, prm.n);
+    const int st = p->info.dtype == B200SPMM_TF32 ? launch_narrow_vecs<true>(prm, vecs, f.n_ctas, smem, stream)
+                                                  : launch_narrow_vecs<false>(prm, vecs, f.n_ctas, smem, stream);
+    if (st != B200SPMM_OK) return st;
+    p->last.n_ctas = (int)f.n_ctas;
+    p->last.threads = kNarrowThreads;
+    p->last.feature_slab = 64;
+    p->last.n_slabs = 1;
+    p->last.smem_bytes = (int64_t)smem;
+    p->last.kernel_launches = 1;
+    p->last.row_window = kRowWindow;
+    return B200SPMM_OK;
 }
 
 // What a super-window launch needs of the plan's scratch.

@@ -30,7 +30,11 @@ struct NarrowParams {
 };
 
 constexpr int kNarrowThreads = 1024;
-constexpr int kNarrowSteps = 8;        // steps whose entries are loaded at one time, and again one ahead
+// Steps whose entries are loaded at one time, and again one ahead.  With one word of B a step is short and eight of them hide
+// the stream's latency (28672 x 8192 at 10 %, 8 columns 33.1 us, with four 35.2); with more, the idle steps at the end of a
+// row cost more than that (16 columns 68.9 with eight, 63.5 with four; tf32 14000 x 8192, 8 columns 49.2 and 39.2).
+template <int kVecs>
+constexpr int kNarrowSteps = kVecs == 1 ? 8 : 4;
 constexpr int kNarrowMaxVecs = 4;      // 16-byte words of a row of B
 constexpr size_t kNarrowSmemMax = 232448;
 
@@ -45,6 +49,7 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) spmm_narrow_kernel(const Na
     constexpr int kPer = kTf32 ? 4 : 8;  // features of a 16-byte word
     constexpr int kW = kVecs * kPer <= 8 ? 8 : kVecs * kPer <= 16 ? 16 : kVecs * kPer <= 32 ? 32 : 64;
     constexpr uint32_t kEsz = kTf32 ? 4 : 2;
+    constexpr int kSteps = kNarrowSteps<kVecs>;
     extern __shared__ __align__(16) uint8_t narrow_b[];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t row0 = p.cut[blockIdx.x], row1 = p.cut[blockIdx.x + 1], stride = p.n_blocks + 1;
@@ -67,10 +72,10 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) spmm_narrow_kernel(const Na
                 hi = __ldg(p.seg + (uint64_t)r * stride + g1);
             }
         };
-        uint2 w[kNarrowSteps];
-        auto load = [&](uint2 (&to)[kNarrowSteps], uint32_t from, uint32_t limit) {
+        uint2 w[kSteps];
+        auto load = [&](uint2 (&to)[kSteps], uint32_t from, uint32_t limit) {
 #pragma unroll
-            for (int k = 0; k < kNarrowSteps; ++k) {
+            for (int k = 0; k < kSteps; ++k) {
                 const uint32_t i = from + k * 32 + lane;
                 if (i < limit) {
                     if (kTf32) to[k] = __ldcs(reinterpret_cast<const uint2 *>(p.entries) + i);
@@ -96,12 +101,12 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) spmm_narrow_kernel(const Na
             uint32_t after_e = 0, after_end = 0;
             segment(row + 2 * (kNarrowThreads / 32), after_e, after_end);
             for (bool last = false; !last;) {
-                last = e + kNarrowSteps * 32 >= end;
-                uint2 ahead[kNarrowSteps];
+                last = e + kSteps * 32 >= end;
+                uint2 ahead[kSteps];
                 if (last) load(ahead, next_e, next_end);
-                else load(ahead, e + kNarrowSteps * 32, end);
+                else load(ahead, e + kSteps * 32, end);
 #pragma unroll
-                for (int k = 0; k < kNarrowSteps; ++k) {
+                for (int k = 0; k < kSteps; ++k) {
                     if (e + k * 32 + lane < end) {
                         const uint32_t c = kTf32 ? w[k].x - col0 : (w[k].x - col0) & 0xFFFFu, a = kTf32 ? w[k].y : w[k].x >> 16;
 #pragma unroll
@@ -110,9 +115,9 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) spmm_narrow_kernel(const Na
                                                        ptx::ld_shared_v4(b_addr + v * plane + c * 16u), a);
                     }
                 }
-                e += kNarrowSteps * 32;
+                e += kSteps * 32;
 #pragma unroll
-                for (int k = 0; k < kNarrowSteps; ++k) w[k] = ahead[k];
+                for (int k = 0; k < kSteps; ++k) w[k] = ahead[k];
             }
             // Sum over the lanes: every step halves the features a lane holds while there are several.
 #pragma unroll

@@ -196,6 +196,23 @@ def test_narrow_b_at_the_edges_of_its_column_blocks(dt, n, rows, cols):
         plan.close()
 
 
+@pytest.mark.parametrize("rows,cols,density,n,narrow", [(1290, 777, 0.2, 32, True), (1290, 777, 0.2, 40, False), (2100, 5000, 0.3, 16, True),
+                                                        (4900, 6773, 0.14, 24, False), (1300, 8000, 0.14, 32, False)])
+def test_narrow_kernel_only_where_it_is_expected_to_be_faster(rows, cols, density, n, narrow):
+    # four words a row of B where all of B fits; super-windows in parts where the rows are few and long
+    import torch
+    rng = np.random.default_rng(rows)
+    rows, cols, rp, ci, v = rows_of_lengths(rng.binomial(cols, density, rows), cols, 7, np.float16)
+    B = dense_b(cols, n, 2)
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    try:
+        got = plan.spmm(torch.from_numpy(B).cuda())
+        assert (plan.launch_info().threads == 1024) == narrow
+        parity.check(got.cpu().numpy(), rows, rp, ci, v, B)
+    finally:
+        plan.close()
+
+
 @pytest.mark.parametrize("dt", [np.float16, np.float32])
 @pytest.mark.parametrize("n", [8, 24, 56])
 def test_tma_boxes_wider_than_b(dt, n, monkeypatch):
