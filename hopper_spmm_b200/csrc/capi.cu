@@ -745,8 +745,9 @@ struct TallScratch {
 TallScratch tall_scratch(const b200spmm_plan *p, int64_t n) {
     const bool pair = use_pair(p, n);
     TallScratch s{};
-    s.parts = tall_launch(p, pair ? p->pair : p->tall, n).parts;
-    if (s.parts > 1) s.partial_floats = (size_t)s.parts * (size_t)p->info.rows * (size_t)n;
+    const TallFormat &f = pair ? p->pair : p->tall;
+    s.parts = tall_launch(p, f, n).parts;
+    if (s.parts > 1) s.partial_floats = (size_t)s.parts * (size_t)f.eff * f.rows * (size_t)n;  // one round of CTAs: 20 MB and less
     if (p->tall_pack_b) {
         // the pair kernel's CTAs fetch 128-feature halves of a 256-feature slab: both halves of the last slab must
         // exist in the packed copy (as zeros past n), so an even number of 128-feature blocks
@@ -799,10 +800,9 @@ int launch_tall(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void 
         prm.b_packed = static_cast<const uint8_t *>(p->d_b_packed);
         prm.b_groups = groups;
     }
-    prm.parts = scratch.parts;
-    st = grow_partial(p, scratch.partial_floats);
-    if (st != B200SPMM_OK) return st;
+    prm.parts = grow_partial(p, scratch.partial_floats) == B200SPMM_OK ? scratch.parts : 1u;  // no room: whole windows
     prm.partial = p->d_partial;
+    prm.partial_rows = (uint32_t)(fmt.eff * fmt.rows);
     prm.sched_counter = p->d_status + 1;
     prm.C = d_C;
     prm.ldc = ldc;

@@ -185,7 +185,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
                     if (lane == 0) ptx::mbar_arrive_cluster(a ? leader_acc_empty1 : leader_acc_empty0);
                 }
                 const uint32_t feat0 = f_slab + col0;
-                tall_store_row32(p, t.part, row, feat0, r);
+                tall_store_row32(p, t.part, w * kPairRows + (row - row0), row, feat0, r);
             }
             // Rows of super-windows without entries are absent from the format: clear the gap after this
             // window (and the rows before the very first one), this slab's features.  The sixteen epilogue

@@ -3,14 +3,14 @@
 // A tile of the condensed format costs the tile kernels its CW gathered rows of B whatever it holds.  On a
 // power-law graph (17 entries per 256-slot tile: about one per gathered row) the matrix instruction has
 // nothing to share, and what remains is the traffic of the gathered rows, which TMA's gather4 delivers at ~39
-// bytes per clock and SM (11 TB/s).  16-byte loads by the lanes of a warp reach 16-20 TB/s as long as B lies in
-// L2, and they need no tiles (512 bytes for 17 entries), so here every entry is one coalesced row load and one
+// bytes per clock and SM (11 TB/s).  16-byte loads by the lanes of a warp reach 17 TB/s as long as B lies in
+// L2 (10 on a graph of 2^20 nodes, where it does not), and they need no tiles (512 bytes for 17 entries), so here every entry is one coalesced row load and one
 // FMA per feature.
 //
 // A unit (a row, or a piece of a long one, see rows_gpu.hpp) is walked by the group of lanes that covers the
 // features of a pass at 16 bytes per lane - 8 lanes for 64 fp16 features, 10 for 40 tf32 ones - so a warp walks
 // 32 / lanes units side by side.  A group that is through with a unit goes on with the next of its share, every
-// n-th unit of a list sorted by length, which gives all groups the same mixture.
+// n-th unit of a list in order of length, longest first: the last blocks have the shortest units.
 //
 // A long row leaves pieces in fp32 slots that rows_fixup_kernel adds in order: C does not depend on timing,
 // bands or feature halves.
@@ -41,10 +41,10 @@ struct RowsParams {
 };
 
 // Two warps a block and 16 blocks an SM: the SM favours its older warps, so equal shares end at very different
-// times, and the shares are handed out by the hardware as small blocks instead (2^20-node R-MAT graph, 64 fp16
-// features: 249 us, against 294-395 us for one resident wave with fixed shares).  A share of 16 batches still
-// hides its start, three dependent loads; with 8 the start shows (277 us), with 64 the last wave does (259 us).
-// The bound of 64 registers lets the compiler keep all four rows of a batch in flight; at 48 it does not (325 us).
+// times, and the shares are handed out by the hardware as small blocks instead, the longest units first (2^20-node R-MAT
+// graph, 64 fp16 features, 220 us now: 15 to 35 % faster than one resident wave with fixed shares).  A share of 16
+// batches still hides its start, three dependent loads; with 8 the start shows (7 %), with 32 nothing changes.
+// The bound of 64 registers lets the compiler keep all four rows of a batch in flight; at 48 it does not (30 % slower).
 constexpr int kRowsThreads = 64;
 constexpr int kRowsBlocksPerSm = 16;
 constexpr uint64_t kRowsGroupBatches = 16;

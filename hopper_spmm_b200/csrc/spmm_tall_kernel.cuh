@@ -61,7 +61,8 @@ struct TallParams {
     uint32_t eff_row_windows;
     uint32_t n_slabs;           // ceil(n / kNs)
     uint32_t parts;             // of a window's stages; no window has fewer stages than parts
-    float *partial;             // [parts][rows][n] fp32, where there are several
+    float *partial;             // [parts][rows of all windows][n] fp32, where there are several
+    uint32_t partial_rows;      // eff_row_windows times the rows of a window
     uint32_t n_items;           // eff_row_windows * n_slabs * parts
     uint32_t c_is_half;
     uint32_t *status;
@@ -96,10 +97,11 @@ B200_DEVICE TallItem tall_item(const TallParams &p, uint32_t item) {
 
 // A thread's 32 consecutive features (fp32 bits, feat0 ..) of row `row` -> C, as 16-byte vectors: 8 features per
 // store for fp16 C, 4 for fp32 C (n is a multiple of 8).  Rows past the end and features past n are dropped.
-B200_DEVICE void tall_store_row32(const TallParams &p, uint32_t part, uint32_t row, uint32_t feat0, const uint32_t (&r)[32]) {
+// With several parts: row `at` of part's sums instead.
+B200_DEVICE void tall_store_row32(const TallParams &p, uint32_t part, uint32_t at, uint32_t row, uint32_t feat0, const uint32_t (&r)[32]) {
     if (row >= p.rows || feat0 >= p.n) return;
     if (p.parts > 1) {
-        float *dst = p.partial + ((uint64_t)part * p.rows + row) * p.n + feat0;
+        float *dst = p.partial + ((uint64_t)part * p.partial_rows + at) * p.n + feat0;
 #pragma unroll
         for (int v = 0; v < 8; ++v)
             if (feat0 + v * 4 < p.n)
@@ -293,7 +295,7 @@ spmm_tall_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
                     if (lane == 0) ptx::mbar_arrive(acc_empty_bar(a));
                 }
                 const uint32_t feat0 = f_slab + col0;  // this thread: features feat0 .. feat0 + 31 of its row
-                tall_store_row32(p, t.part, row, feat0, r);
+                tall_store_row32(p, t.part, w * kTallRows + (row - row0), row, feat0, r);
             }
             // Rows of super-windows without entries are absent from the format: clear the gap after this
             // window (and the rows before the very first one), this slab's features.  Warp w takes every
@@ -603,14 +605,15 @@ tall_sum_parts_kernel(const float *partial, uint32_t parts, const uint32_t *__re
         ptx::wait_for_grids_before();
         return;
     }
-    const uint32_t at = (uint32_t)(i - w * per_window), r = rowIdx[w] + at / vec_per_row, feat = at % vec_per_row * 4;
+    const uint32_t at = (uint32_t)(i - w * per_window), in_window = at / vec_per_row, r = rowIdx[w] + in_window, feat = at % vec_per_row * 4;
     ptx::wait_for_grids_before();
     if (r >= rows) return;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float *src = partial + (uint64_t)r * n + feat;
+    const uint64_t part_floats = (uint64_t)eff * window_rows * n;
+    const float *src = partial + (w * window_rows + in_window) * n + feat;
 #pragma unroll 4
     for (uint32_t k = 0; k < parts; ++k) {
-        const float4 v = __ldcs(reinterpret_cast<const float4 *>(src + (uint64_t)k * rows * n));
+        const float4 v = __ldcs(reinterpret_cast<const float4 *>(src + k * part_floats));
         acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
     if (c_is_half) {
