@@ -45,7 +45,7 @@ def build_binding() -> str:
     from torch.utils import cpp_extension
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-o", BINDING, "torch_binding.cpp"]
     cmd += ["-isystem" + p for p in cpp_extension.include_paths("cuda") + [sysconfig.get_paths()["include"]]]
-    cmd += ["-L" + p for p in cpp_extension.library_paths("cuda")] + ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    cmd += ["-L" + p for p in cpp_extension.library_paths("cuda")] + ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
     cmd += ["-L" + HERE, "-lb200spmm", "-Wl,-rpath,$ORIGIN"]
     subprocess.run(cmd, cwd=CSRC, check=True)
     return BINDING

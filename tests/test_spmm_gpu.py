@@ -494,3 +494,38 @@ def test_tf32_product_against_the_oracle_on_truncated_inputs(window, monkeypatch
     loose = float((np.abs(got - oracle.spmm_csr(rows, rp, ci, v, B))[live] / mag[live]).max())
     print(f"window {window}: error relative to the magnitude sum {tight:.2e} against truncated inputs, {loose:.2e} against fp32 inputs")
     assert tight < 1e-5 < loose < 5e-3
+
+
+@pytest.mark.parametrize("c_half", [False, True])
+def test_the_result_is_made_where_torch_looks_for_it(c_half):
+    # the same tensor whether it comes from the allocator directly or through the dispatcher, which a mode hears
+    import torch
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Heard(TorchDispatchMode):
+        def __init__(self):
+            super().__init__()
+            self.names = []
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.names.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    rows, cols, rp, ci, v = random_csr(203, 517, 0.03, 11)
+    B = torch.from_numpy(dense_b(cols, 40, 3)).cuda()
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    try:
+        first = plan.spmm(B, c_half=c_half)
+        with Heard() as heard:
+            second = plan.spmm(B, c_half=c_half)
+        assert any("empty" in name for name in heard.names)
+        with torch.inference_mode():
+            third = plan.spmm(B, c_half=c_half)
+        assert third.is_inference() and not first.is_inference()
+        for c in (first, second, third):
+            assert c.shape == (rows, 40) and c.is_contiguous() and not c.requires_grad and c.device == B.device
+            assert c.dtype == (torch.float16 if c_half else torch.float32) and torch.equal(c, first)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            assert torch.equal(plan.spmm(B, c_half=c_half), first)
+    finally:
+        plan.close()
