@@ -500,11 +500,10 @@ constexpr double kRowsMaxFill = 0.08;  // share of a tile's slots in use
 // than two a CTA take the same few microseconds either way and stay with their tiles.
 constexpr double kRowsMaxFillWide = 0.11, kTallMinFill = 0.03;
 constexpr uint64_t kRowsWideMinTiles = 592, kRowsWideAnyTiles = 16384;  // (below the second, whatever super-windows would do)
-// Super-windows are made from this many short tiles on: 1100 x 1100 at 20 % (4,638), fp16, 72 / 200 / 512 / 2,048 columns 15.7
-// / 24.5 / 37.8 / 134 us with 16 rows, 10.9 / 14.9 / 17.1 / 20.2 with them; the plan takes 285 us instead of 276.  Those of
+// Super-windows are made from this many short tiles on: 1100 x 1100 at 20 % (4,638), fp16, 72 / 256 / 512 / 2,048 columns 16.4
+// / 22.5 / 38.5 / 135 us with 16 rows, 10.9 / 15.7 / 16.7 / 35.7 with them; the plan takes 285 us instead of 276.  Those of
 // 256 rows from the second number on: in parts the two heights take the same (1682 x 1536 at 11 %, 8,614 tiles, 816 columns
-// 21.5 and 22.5 us), and the plan takes 50 us less with one of them.  Below it whole windows of 128 rows do not pay up to 128
-// columns (3000 x 1100 at 10 %, 128 columns 12.4 us with 16 rows, 13.4 with 128).
+// 21.5 and 22.5 us), and the plan takes 50 us less with one of them.
 constexpr uint64_t kTallMinShortTiles = 2048, kPairMinShortTiles = 16384;
 constexpr uint64_t kTallMaxCounted = 1 << 25, kTallMaxCountedCols = 393216;  // entries of lists; columns of one bit set
 
@@ -640,33 +639,65 @@ int launch_narrow_vecs(const NarrowParams &prm, int vecs, unsigned n_ctas, size_
 // round of parts is slower again (2000 x 8000 at 10 %, 1,024 columns 56 / 45 / 55 / 81).
 // Up to 64 columns a matrix of fewer than kSplitMinShortTiles tiles keeps to whole windows, and so mostly to the 16-row
 // kernel, a choice that is held to elsewhere: 3000 x 3000 at 12 %, 64 columns 19 us where six parts would take 12.5.
+//
+// The tensor core cuts what it adds, so the error of a sum grows with the tiles it runs through: 1.4e-8 a tile here, and with 16
+// rows 1.6e-8 and more in fp16, 1.1e-8 in tf32, over the tiles of a piece of a window.  Where whole super-windows are not
+// expected to be faster than 16 rows, or the matrix is small, the windows are cut so far that the sums are no less exact than
+// those of the 16-row kernel's pieces (tall_least_parts), in more than one round if it takes that; or that kernel stays.
 struct TallLaunch {
     double micros;
     uint32_t parts;
 };
 constexpr uint64_t kSplitMinShortTiles = 80000;
+constexpr double kTallMaxSums = 128e6;  // bytes
+double short_micros(const b200spmm_plan *p, int64_t n) {  // (tiles over 148 SMs)
+    return 14.0 + (double)p->info.total_tiles * (148.0 / p->n_sms) * (n <= 64 ? 0.28e-3 : 0.4e-3 * (double)((n + 127) / 128));
+}
+
+
+bool tall_is_pair(const TallFormat &f) { return f.rows == (uint32_t)kPairRows; }
+int64_t tall_items(const TallFormat &f, int64_t n) {
+    const int64_t slab = tall_is_pair(f) || n > 128 ? 256 : 128;
+    return (int64_t)f.eff * ((n + slab - 1) / slab);
+}
+double tall_whole_micros(const b200spmm_plan *p, const TallFormat &f, int64_t n) {
+    const int64_t units = tall_is_pair(f) ? p->pair_clusters : p->n_sms;
+    return 12.0 + (double)((tall_items(f, n) + units - 1) / units) * (double)f.max_window_tiles * (n > 128 ? 0.11 : 0.085);
+}
+
+uint32_t tall_least_parts(const b200spmm_plan *p, int64_t n) {
+    const bool pair = p->pair.tiles && p->pair_clusters > 0 && n > 128;
+    if (p->info.total_tiles >= kPairMinShortTiles && p->tall.eff * 16 >= (uint64_t)p->n_sms &&
+        ((pair && tall_whole_micros(p, p->pair, n) < short_micros(p, n)) || tall_whole_micros(p, p->tall, n) < short_micros(p, n)))
+        return 1;
+    const double pieces = (double)std::max<uint64_t>(p->info.eff_row_windows, (uint64_t)p->n_sms * kCtasPerSm);
+    const double tiles = (double)p->info.total_tiles / pieces * (p->info.dtype == B200SPMM_TF32 ? 0.65 : 1.0);
+    return (uint32_t)std::ceil((double)p->tall.max_window_tiles / std::max(tiles, 1.0));
+}
+
 TallLaunch tall_launch(const b200spmm_plan *p, const TallFormat &f, int64_t n) {
-    const bool pair = f.rows == (uint32_t)kPairRows;
-    const int64_t slab = pair || n > 128 ? 256 : 128, units = pair ? p->pair_clusters : p->n_sms, items = (int64_t)f.eff * ((n + slab - 1) / slab);
-    const double longest = (double)f.max_window_tiles, alone = pair ? 0.088 : slab > 128 ? 0.105 : 0.068;
-    TallLaunch best{12.0 + (double)((items + units - 1) / units) * longest * (slab > 128 ? 0.11 : 0.085), 1};
-    if (p->tall_forced || (n <= 64 && p->info.total_tiles < kSplitMinShortTiles)) return best;
-    double least = 12.0 + longest * alone;
+    const double whole = tall_whole_micros(p, f, n);
+    if (p->tall_forced) return {whole, 1};
+    const uint32_t least = tall_least_parts(p, n);
+    TallLaunch best{least > 1 ? 1e30 : whole, 1};
+    if (n <= 64 && p->info.total_tiles < kSplitMinShortTiles) return best;
+    const bool pair = tall_is_pair(f);
+    const int64_t units = pair ? p->pair_clusters : p->n_sms, items = tall_items(f, n);
+    const double longest = (double)f.max_window_tiles, alone = pair ? 0.088 : n > 128 ? 0.105 : 0.068;
+    double lowest = least > 1 ? 1e30 : 12.0 + longest * alone;
     const uint64_t stages = (f.min_window_tiles + kTallStageTiles - 1) / kTallStageTiles;
-    for (uint32_t parts = 2; parts <= 16 && parts <= stages && items * parts <= units; ++parts) {
+    for (uint32_t parts = std::max(2u, least); parts <= 16 && parts <= stages; ++parts) {
+        const int64_t rounds = (items * parts + units - 1) / units;
         const double sums = (double)parts * (double)f.eff * f.rows * (double)n * 4.0;
-        const double micros = 12.0 + longest / parts * alone + 1.5 + 2.0 * sums * 0.22e-6;
-        if (micros < least) {
-            least = micros;
+        if ((rounds > 1 && parts > least) || sums > kTallMaxSums) break;
+        const double micros = 12.0 + (double)rounds * longest / parts * (rounds > 1 ? (n > 128 ? 0.11 : 0.085) : alone) + 1.5 + 2.0 * sums * 0.22e-6;
+        if (micros < lowest) {
+            lowest = micros;
             best = {micros, parts};
         }
     }
     return best;
 }
-double short_micros(const b200spmm_plan *p, int64_t n) {  // (tiles over 148 SMs)
-    return 14.0 + (double)p->info.total_tiles * (148.0 / p->n_sms) * (n <= 64 ? 0.28e-3 : 0.4e-3 * (double)((n + 127) / 128));
-}
-
 bool use_pair(const b200spmm_plan *p, int64_t n) {
     if (!p->pair.tiles || p->pair_clusters < 1 || n <= 128) return false;
     if (p->tall_forced) return true;
@@ -679,18 +710,19 @@ bool use_tall(const b200spmm_plan *p, int64_t n) {
     if (!p->tall.tiles || p->gather_cpasync) return false;
     if (p->tall_forced) return n * p->info.elt_size >= 128;
     if (use_pair(p, n)) return true;
-    const TallLaunch t = tall_launch(p, p->tall, n);
-    if (t.parts == 1 && n <= 128 && p->info.total_tiles < kPairMinShortTiles) return false;
-    return t.micros < short_micros(p, n);
+    // (the 16-row kernel is better than its estimate where every SM has a window: 3000 x 1100 at 10 %, 128 columns 12.4 us against 13.3)
+    const double margin = p->info.total_tiles < kPairMinShortTiles && p->info.eff_row_windows >= (uint64_t)p->n_sms ? 1.1 : 1.0;
+    return tall_launch(p, p->tall, n).micros * margin < short_micros(p, n);
 }
 
 // Column blocks per group for B of width n: as many as fit shared memory, 0 if the kernel does not take it.  Every
 // 16-byte word of a row of B adds to its time - pruned 28672 x 8192 weight, fp16: 33, 64, 84, 123 us for 8, 16, 24, 32
 // columns; a warp has a row, so 33 rows a CTA take as long as 64 - while the tile kernels take the same up to 64 features (89
-// us; tf32: 98 us for 8 and 16 columns).  Up to 24 fp16 and 16 tf32 columns it is left for super-windows only, where these
-// are expected to be faster (24 columns: 4904 x 6773 at 13 % 33 us against 21, 12000 x 5000 at 20 % 44 against 32); 32 fp16
-// columns go to it where it is expected to be faster than all tiles (1100 x 1100 at 20 % 11.6 -> 7.5 us, 1682 x 1536 at 11 % 13.5 -> 10.0, 3000 x 3000 at 12 %
-// 19.2 -> 17.0), if all of B fits shared memory (2000 x 8000 at 6 %, in two halves, 36 us against 20).
+// us; tf32: 98 us for 8 and 16 columns).  Up to 24 fp16 and 16 tf32 columns it is taken all the same, also where super-windows
+// would be faster (6000 x 8192 at 20 %, 24 columns 49.6 us against 23.4): its fp32 sums are thirty times as exact as the
+// tensor core's.  32 fp16 columns go to it where all of B fits shared memory and it is expected to be faster than the tiles (1100 x
+// 1100 at 20 % 11.6 -> 7.5 us, 1682 x 1536 at 11 % 13.5 -> 10.0, 3000 x 3000 at 12 % 19.2 -> 17.0; 2000 x 8000 at 6 %, in two
+// halves, 36 against 20).
 uint32_t narrow_group_blocks(const b200spmm_plan *p, int64_t n) {
     const NarrowFormat &f = p->narrow;
     const int64_t vecs = n * p->info.elt_size / 16;
@@ -698,12 +730,12 @@ uint32_t narrow_group_blocks(const b200spmm_plan *p, int64_t n) {
     if (!f.n_ctas || vecs > kNarrowMaxVecs) return 0;
     uint32_t g = f.n_blocks;
     while (g && narrow_smem_bytes((uint32_t)vecs, (uint32_t)p->info.cols, g, f.n_blocks, f.max_rows, (uint32_t)n) > kNarrowSmemMax) --g;
-    if (!g || p->rows_only) return vecs < kNarrowMaxVecs || tf32 ? g : 0;
+    if (!g || vecs < kNarrowMaxVecs || tf32) return g;
+    if (p->rows_only || g < f.n_blocks) return 0;
     const double rows = (double)p->info.rows / f.n_ctas, rounds = std::ceil(rows / 32.0) * 32.0 / rows;
-    const double micros = 4.0 + (double)p->info.nnzs * (double)vecs * 1.05e-6 * (148.0 / p->n_sms) * rounds * (g == f.n_blocks ? 1.0 : tf32 || vecs == kNarrowMaxVecs ? 1.5 : 1.05);
+    const double micros = 4.0 + (double)p->info.nnzs * (double)vecs * 1.05e-6 * (148.0 / p->n_sms) * rounds;
     const TallLaunch tall = p->tall.tiles && !p->gather_cpasync ? tall_launch(p, p->tall, n) : TallLaunch{1e30, 1};
-    if (vecs < kNarrowMaxVecs || tf32) return tall.micros < micros ? 0 : g;
-    return g == f.n_blocks && micros < tall.micros && micros < short_micros(p, n) ? g : 0;
+    return micros < tall.micros && micros < short_micros(p, n) ? g : 0;
 }
 
 int launch_narrow(b200spmm_plan *p, uint32_t group_blocks, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
@@ -747,7 +779,7 @@ TallScratch tall_scratch(const b200spmm_plan *p, int64_t n) {
     TallScratch s{};
     const TallFormat &f = pair ? p->pair : p->tall;
     s.parts = tall_launch(p, f, n).parts;
-    if (s.parts > 1) s.partial_floats = (size_t)s.parts * (size_t)f.eff * f.rows * (size_t)n;  // one round of CTAs: 20 MB and less
+    if (s.parts > 1) s.partial_floats = (size_t)s.parts * (size_t)f.eff * f.rows * (size_t)n;  // kTallMaxSums
     if (p->tall_pack_b) {
         // the pair kernel's CTAs fetch 128-feature halves of a 256-feature slab: both halves of the last slab must
         // exist in the packed copy (as zeros past n), so an even number of 128-feature blocks

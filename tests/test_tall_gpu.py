@@ -275,3 +275,28 @@ def test_merging_more_columns_than_a_bit_set_holds(dt, tall):
             assert np.array_equal(got["data"].view(np.uint8), np.ascontiguousarray(want.data).view(np.uint8))
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("dt,rows,cols,n", [(np.float16, 1682, 1536, 816), (np.float16, 1100, 2400, 512), (np.float16, 1300, 6003, 104),
+                                            (np.float32, 1100, 1100, 512), (np.float32, 1100, 2400, 512), (np.float32, 1300, 6003, 104)])
+def test_sums_are_as_exact_as_those_of_the_16_row_kernel(dt, rows, cols, n, monkeypatch):
+    # against 64 bits, from the values as the tensor core reads them: super-windows that take what 16 rows would otherwise
+    # are cut into parts short enough.  (5 %: the errors are those of some thousand sums cut at 24 bits)
+    import torch
+    rows, cols, rp, ci, v = random_csr(rows, cols, 0.14, 9, dt)
+    cut = (lambda x: x) if dt == np.float16 else (lambda x: (x.view(np.uint32) & np.uint32(0xFFFFE000)).view(np.float32))
+    v, B = cut(np.abs(v) + dt(0.1)), cut(np.abs(dense_b(cols, n, 3, dt)))  # of one sign: what is cut off adds up
+    A = torch.sparse_csr_tensor(torch.from_numpy(rp.astype(np.int64)), torch.from_numpy(ci.astype(np.int64)), torch.from_numpy(v.astype(np.float64)), (rows, cols))
+    want = (A.cuda() @ torch.from_numpy(B.astype(np.float64)).cuda())
+    off, window = {}, {}
+    for how in (None, "16"):
+        if how:
+            monkeypatch.setenv("B200SPMM_WINDOW", how)
+        plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+        try:
+            off[how] = float((plan.spmm(torch.from_numpy(B).cuda()).double() - want).norm() / want.norm())
+            window[how] = plan.launch_info().row_window
+        finally:
+            plan.close()
+    assert window == {None: 128, "16": 16}
+    assert off[None] <= 1.05 * off["16"]
