@@ -109,15 +109,21 @@ struct b200spmm_plan {
     // is re-laid as shared-memory images at every launch (scratch of the plan, as large as B) and such a
     // tile's operand arrives by one bulk copy.
     bool tall_pack_b = false;
-    void *d_b_packed = nullptr;
-    size_t b_packed_bytes = 0;
+    // Scratch of launches, grown to the largest need seen (take_scratch).  A graph runs at the addresses its launches were
+    // captured with: memory that one of them was given is not freed when it is outgrown, but with the plan.
+    struct Scratch {
+        void *ptr = nullptr;
+        size_t bytes = 0;
+        bool in_graph = false;
+    };
+    Scratch b_packed;
+    Scratch partial;  // fp32: pieces of windows or rows that are computed in parts, parts of super-windows
+    std::vector<void *> outgrown;
     int n_sms = 0;
     // The tiles as the kernel's shared-memory image (spmm_kernel.cuh, SpmmParams::tiles_image): the plan's own
     // array swizzled in place when it owns the format, a swizzled copy when the arrays are the caller's.
     void *d_tiles_image = nullptr;
     bool image_is_copy = false;
-    float *d_partial = nullptr;  // [n_slots][16][n] fp32, grown to the largest need seen
-    size_t partial_floats = 0;
     uint32_t *d_status = nullptr;
     CUtensorMap tmap_a{};
     // Tensor map over B, kept between launches: B's address, pitch and width rarely change from call
@@ -330,12 +336,29 @@ int grow_buffer(T **buf, size_t bytes) {
     return B200SPMM_OK;
 }
 
-// Slots for the pieces of windows or rows that are computed in parts, grown to the largest need seen.
-int grow_partial(b200spmm_plan *p, size_t floats) {
-    if (floats <= p->partial_floats) return B200SPMM_OK;
-    const int st = grow_buffer(&p->d_partial, floats * sizeof(float));
-    p->partial_floats = st == B200SPMM_OK ? floats : 0;
-    return st;
+// (The default stream does not answer while another one is being captured; a launch there will say so.)
+bool is_captured(cudaStream_t stream) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) == cudaSuccess) return capture != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
+// Scratch for a launch on `stream`.
+int take_scratch(b200spmm_plan *p, b200spmm_plan::Scratch *s, size_t bytes, cudaStream_t stream) {
+    if (bytes > s->bytes) {
+        if (s->in_graph) {
+            p->outgrown.push_back(s->ptr);
+            s->ptr = nullptr;
+            s->in_graph = false;
+        }
+        s->bytes = 0;
+        const int st = grow_buffer(&s->ptr, bytes);
+        if (st != B200SPMM_OK) return st;
+        s->bytes = bytes;
+    }
+    if (bytes && !s->in_graph) s->in_graph = is_captured(stream);
+    return B200SPMM_OK;
 }
 
 // The environment is consulted when a plan is made (and once per process for the plan-less
@@ -540,7 +563,7 @@ int launch_rows_grid(b200spmm_plan *p, const RowsParams &prm, dim3 grid, void (*
     p->last.row_window = kRowWindow;
     p->last.kernel_launches = 1;
     if (s1 == s0) return B200SPMM_OK;
-    B200_CUDA_TRY(launch_after(rows_fixup_kernel, dim3(s1 - s0), 256, 0, 1, stream, p->rows_fmt.d_splits + s0, (const float *)p->d_partial, prm.C,
+    B200_CUDA_TRY(launch_after(rows_fixup_kernel, dim3(s1 - s0), 256, 0, 1, stream, p->rows_fmt.d_splits + s0, (const float *)prm.partial, prm.C,
                                prm.ldc, prm.n, prm.c_is_half));
     p->last.kernel_launches = 2;
     return B200SPMM_OK;
@@ -566,10 +589,10 @@ int launch_rows(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void 
     prm.n = (uint32_t)n;
     prm.c_is_half = c_dtype == B200SPMM_C_F16;
     if (f.n_slots) {
-        int st = grow_partial(p, (size_t)f.n_slots * (size_t)n);
+        int st = take_scratch(p, &p->partial, (size_t)f.n_slots * (size_t)n * 4, stream);
         if (st != B200SPMM_OK) return st;
     }
-    prm.partial = p->d_partial;
+    prm.partial = static_cast<float *>(p->partial.ptr);
     const uint32_t vec = 16u / (uint32_t)p->info.elt_size;
     uint32_t n_slabs = 0, groups = 0;
     auto set_slab = [&](uint32_t slab) {
@@ -772,14 +795,14 @@ int launch_narrow(b200spmm_plan *p, uint32_t group_blocks, const void *d_B, int6
 // What a super-window launch needs of the plan's scratch.
 struct TallScratch {
     uint32_t parts;
-    size_t partial_floats, packed_bytes;
+    size_t partial_bytes, packed_bytes;
 };
 TallScratch tall_scratch(const b200spmm_plan *p, int64_t n) {
     const bool pair = use_pair(p, n);
     TallScratch s{};
     const TallFormat &f = pair ? p->pair : p->tall;
     s.parts = tall_launch(p, f, n).parts;
-    if (s.parts > 1) s.partial_floats = (size_t)s.parts * (size_t)f.eff * f.rows * (size_t)n;  // kTallMaxSums
+    if (s.parts > 1) s.partial_bytes = (size_t)s.parts * (size_t)f.eff * f.rows * (size_t)n * 4;  // kTallMaxSums
     if (p->tall_pack_b) {
         // the pair kernel's CTAs fetch 128-feature halves of a 256-feature slab: both halves of the last slab must
         // exist in the packed copy (as zeros past n), so an even number of 128-feature blocks
@@ -792,13 +815,8 @@ TallScratch tall_scratch(const b200spmm_plan *p, int64_t n) {
 // While a stream is being captured no scratch can be had; the 16-row kernel may do without.
 bool tall_can_launch(const b200spmm_plan *p, int64_t n, cudaStream_t stream) {
     const TallScratch s = tall_scratch(p, n);
-    if (s.partial_floats <= p->partial_floats && s.packed_bytes <= p->b_packed_bytes) return true;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
-        cudaGetLastError();
-        return true;  // (the launch will say what is wrong)
-    }
-    return capture == cudaStreamCaptureStatusNone;
+    if (s.partial_bytes <= p->partial.bytes && s.packed_bytes <= p->b_packed.bytes) return true;
+    return !is_captured(stream);
 }
 
 int launch_tall(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
@@ -820,20 +838,16 @@ int launch_tall(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void 
         const uint32_t n_slabs = pair ? 2u * (uint32_t)((n + 255) / 256) : (uint32_t)((n + slab - 1) / slab);
         const uint32_t groups = (uint32_t)((p->info.cols + cw - 1) / cw);
         const size_t need = scratch.packed_bytes;  // n_slabs * groups * 32 * slab
-        if (need > p->b_packed_bytes) {
-            p->b_packed_bytes = 0;
-            int st = grow_buffer(&p->d_b_packed, need);
-            if (st != B200SPMM_OK) return st;
-            p->b_packed_bytes = need;
-        }
+        st = take_scratch(p, &p->b_packed, need, stream);
+        if (st != B200SPMM_OK) return st;
         const int grid = (int)std::min<size_t>((need / 16 + 255) / 256, (size_t)p->n_sms * 16);
         B200_CUDA_TRY(launch_after(tf32 ? pack_b_kernel<true> : pack_b_kernel<false>, dim3(grid), 256, 0, 1, stream, static_cast<const uint8_t *>(d_B),
-                                   ldb * esz, (uint32_t)p->info.cols, (uint32_t)n, slab, n_slabs, groups, static_cast<uint8_t *>(p->d_b_packed)));
-        prm.b_packed = static_cast<const uint8_t *>(p->d_b_packed);
+                                   ldb * esz, (uint32_t)p->info.cols, (uint32_t)n, slab, n_slabs, groups, static_cast<uint8_t *>(p->b_packed.ptr)));
+        prm.b_packed = static_cast<const uint8_t *>(p->b_packed.ptr);
         prm.b_groups = groups;
     }
-    prm.parts = grow_partial(p, scratch.partial_floats) == B200SPMM_OK ? scratch.parts : 1u;  // no room: whole windows
-    prm.partial = p->d_partial;
+    prm.parts = take_scratch(p, &p->partial, scratch.partial_bytes, stream) == B200SPMM_OK ? scratch.parts : 1u;  // no room: whole windows
+    prm.partial = static_cast<float *>(p->partial.ptr);
     prm.partial_rows = (uint32_t)(fmt.eff * fmt.rows);
     prm.sched_counter = p->d_status + 1;
     prm.C = d_C;
@@ -1362,14 +1376,15 @@ void b200spmm_plan_destroy(b200spmm_plan_t *p) {
     pool_free(p->d_tile_entries);
     free_tall(&p->tall);
     free_tall(&p->pair);
-    pool_free(p->d_b_packed);
+    pool_free(p->b_packed.ptr);
+    pool_free(p->partial.ptr);
+    for (void *old : p->outgrown) pool_free(old);
     if (p->image_is_copy) pool_free(p->d_tiles_image);
     for (cudaEvent_t e : p->band_done) cudaEventDestroy(e);
     if (p->copy_stream) cudaStreamDestroy(p->copy_stream);
     if (p->upload_stream) cudaStreamDestroy(p->upload_stream);
     for (cudaEvent_t e : p->half_up)
         if (e) cudaEventDestroy(e);
-    pool_free(p->d_partial);
     pool_free(p->d_status);
     pool_free(p->d_B);
     pool_free(p->d_C);
@@ -1541,12 +1556,8 @@ cudaError_t make_current(int device) {
 void note_bounded_waits(b200spmm_plan_t *p, cudaStream_t stream) {
     using Unread = b200spmm_plan::Unread;
     if (p->unread == Unread::any) return;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     unsigned long long id = 0;
-    // (the default stream does not answer while another one is being captured: the launch will say so; and asking a stream
-    // for its id ends its capture)
-    const bool known = cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone &&
-                       cudaStreamGetId(stream, &id) == cudaSuccess;
+    const bool known = !is_captured(stream) && cudaStreamGetId(stream, &id) == cudaSuccess;  // (asking a stream for its id ends its capture)
     if (!known) cudaGetLastError();
     if (!known || (p->unread == Unread::one_stream && p->unread_stream != id)) {
         p->unread = Unread::any;
@@ -1600,10 +1611,10 @@ int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, voi
     const uint32_t split_end = band < 0 ? sc.n_splits : sc.band_split[band + 1];
     prm.sched_counter = sc.n_chunks > (uint32_t)sc.n_ctas ? p->d_status + 1 : nullptr;
     if (sc.n_slots) {  // slots for the pieces of windows that span chunks
-        int st = grow_partial(p, (size_t)sc.n_slots * kRowWindow * (size_t)n);
+        int st = take_scratch(p, &p->partial, (size_t)sc.n_slots * kRowWindow * (size_t)n * 4, stream);
         if (st != B200SPMM_OK) return st;
     }
-    prm.partial = p->d_partial;
+    prm.partial = static_cast<float *>(p->partial.ptr);
     prm.tiles_image = static_cast<const uint8_t *>(p->d_tiles_image);
     prm.total_tiles = (uint32_t)p->info.total_tiles;
     prm.B = d_B;
@@ -1627,7 +1638,7 @@ int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, voi
     if (st != B200SPMM_OK || split_end == split_begin) return st;
     // windows shared out over several CTAs: sum their pieces
     B200_CUDA_TRY(launch_after(spmm_fixup_kernel, dim3(split_end - split_begin), 256, 0, 1, stream, sc.d_splits + split_begin, sc.d_piece_slots,
-                               p->d_partial, p->d_rowIdx, d_C, ldc, prm.rows, prm.n, prm.c_is_half));
+                               (const float *)prm.partial, p->d_rowIdx, d_C, ldc, prm.rows, prm.n, prm.c_is_half));
     p->last.kernel_launches = 2;
     return B200SPMM_OK;
 }
