@@ -344,17 +344,23 @@ bool is_captured(cudaStream_t stream) {
     return true;
 }
 
-// Scratch for a launch on `stream`.
+// Scratch for a launch on `stream`.  A captured launch has it like any other, so that a graph holds the kernels that the call
+// would run; but a capture allows no wait for the device, and what is outgrown then may be in use.
 int take_scratch(b200spmm_plan *p, b200spmm_plan::Scratch *s, size_t bytes, cudaStream_t stream) {
     if (bytes > s->bytes) {
-        if (s->in_graph) {
+        const bool captured = is_captured(stream);
+        if (s->ptr && (captured || s->in_graph)) {
             p->outgrown.push_back(s->ptr);
             s->ptr = nullptr;
-            s->in_graph = false;
         }
+        s->in_graph = false;
         s->bytes = 0;
-        const int st = grow_buffer(&s->ptr, bytes);
-        if (st != B200SPMM_OK) return st;
+        if (captured) {
+            B200_CUDA_TRY(pool_alloc_under_capture(&s->ptr, bytes));
+        } else {
+            const int st = grow_buffer(&s->ptr, bytes);
+            if (st != B200SPMM_OK) return st;
+        }
         s->bytes = bytes;
     }
     if (bytes && !s->in_graph) s->in_graph = is_captured(stream);
@@ -810,13 +816,6 @@ TallScratch tall_scratch(const b200spmm_plan *p, int64_t n) {
         s.packed_bytes = features * 32u * (size_t)((p->info.cols + p->info.col_window - 1) / p->info.col_window);
     }
     return s;
-}
-
-// While a stream is being captured no scratch can be had; the 16-row kernel may do without.
-bool tall_can_launch(const b200spmm_plan *p, int64_t n, cudaStream_t stream) {
-    const TallScratch s = tall_scratch(p, n);
-    if (s.partial_bytes <= p->partial.bytes && s.packed_bytes <= p->b_packed.bytes) return true;
-    return !is_captured(stream);
 }
 
 int launch_tall(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
@@ -1592,7 +1591,7 @@ int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, voi
         if (st != B200SPMM_OK) return st;
     }
     note_bounded_waits(p, stream);
-    if (band < 0 && use_tall(p, n) && tall_can_launch(p, n, stream)) return launch_tall(p, d_B, ldb, n, d_C, ldc, c_dtype, stream);
+    if (band < 0 && use_tall(p, n)) return launch_tall(p, d_B, ldb, n, d_C, ldc, c_dtype, stream);
     SpmmParams prm{};
     prm.rowOffset = p->d_rowOffset;
     prm.tcA2B = p->d_tcA2B;

@@ -43,7 +43,7 @@ cudaError_t pool_of(int device, cudaMemPool_t *out) {
 }
 
 std::mutex g_large_lock;
-std::unordered_set<void *> g_large;  // buffers of kPoolMaxBytes and more
+std::unordered_set<void *> g_large;  // the driver's own buffers: of kPoolMaxBytes and more, or allocated under a capture
 
 std::mutex g_staging_lock;
 void *g_staging = nullptr;  // [kUploadThreads][2][kUploadChunk] pinned bytes
@@ -117,6 +117,20 @@ cudaError_t pool_alloc_bytes(void **out, size_t bytes, cudaStream_t stream) {
         e = allocate();
     }
     if (e == cudaSuccess && bytes >= kPoolMaxBytes) {
+        std::lock_guard<std::mutex> guard(g_large_lock);
+        g_large.insert(*out);
+    }
+    return e;
+}
+
+cudaError_t pool_alloc_under_capture(void **out, size_t bytes) {
+    *out = nullptr;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // cudaMalloc is refused in the other modes; it is no part of the graph
+    cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return e;
+    e = cudaMalloc(out, bytes);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e == cudaSuccess) {
         std::lock_guard<std::mutex> guard(g_large_lock);
         g_large.insert(*out);
     }

@@ -22,6 +22,8 @@ constexpr size_t kPoolMaxBytes = (size_t)128 << 20;
 constexpr size_t kPoolKeepBytes = (size_t)512 << 20;
 
 cudaError_t pool_alloc_bytes(void **out, size_t bytes, cudaStream_t stream);
+// Memory that is there at once, while a stream is being captured too: the driver's own, whatever its size.
+cudaError_t pool_alloc_under_capture(void **out, size_t bytes);
 // What was queued on `stream` may still use the memory; a large buffer is given back when the device is idle.
 void pool_free(void *ptr, cudaStream_t stream = nullptr);
 cudaError_t pool_release(int device);

@@ -365,6 +365,8 @@ int b200spmm_release_cached_memory(int device);
  * Replaces the launch of fp16_spmm_kernel inside fp16_spmm (src/fp16.cu:36-175, 255-264)
  * for both element types (the reference's tf32.cu has no kernel).
  * Rows of windows with no entries are written as zeros, so C needs no prior clearing.
+ * The call may be captured into a CUDA graph, also as the plan's first one: the graph holds the kernels that the
+ * call would run, and the plan must outlive it.  Scratch that a graph uses is kept until the plan is destroyed.
  *   B, C 16-byte aligned; ldb*sizeof(b) and ldc*sizeof(c) multiples of 16; n a multiple of 8.
  */
 int b200spmm_spmm(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc,
