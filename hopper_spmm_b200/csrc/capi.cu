@@ -704,10 +704,9 @@ uint32_t tall_least_parts(const b200spmm_plan *p, int64_t n) {
     return (uint32_t)std::ceil((double)p->tall.max_window_tiles / std::max(tiles, 1.0));
 }
 
-TallLaunch tall_launch(const b200spmm_plan *p, const TallFormat &f, int64_t n) {
+TallLaunch tall_launch(const b200spmm_plan *p, const TallFormat &f, int64_t n, uint32_t least) {
     const double whole = tall_whole_micros(p, f, n);
     if (p->tall_forced) return {whole, 1};
-    const uint32_t least = tall_least_parts(p, n);
     TallLaunch best{least > 1 ? 1e30 : whole, 1};
     if (n <= 64 && p->info.total_tiles < kSplitMinShortTiles) return best;
     const bool pair = tall_is_pair(f);
@@ -727,21 +726,45 @@ TallLaunch tall_launch(const b200spmm_plan *p, const TallFormat &f, int64_t n) {
     }
     return best;
 }
-bool use_pair(const b200spmm_plan *p, int64_t n) {
-    if (!p->pair.tiles || p->pair_clusters < 1 || n <= 128) return false;
-    if (p->tall_forced) return true;
-    return tall_launch(p, p->pair, n).micros < short_micros(p, n);
-}
 
-// Does this launch go to the super-window kernel?  Only with the TMA gathers, and - unless forced, for B at
-// least one 128-byte box wide - only when it is expected to be faster.
-bool use_tall(const b200spmm_plan *p, int64_t n) {
-    if (!p->tall.tiles || p->gather_cpasync) return false;
-    if (p->tall_forced) return n * p->info.elt_size >= 128;
-    if (use_pair(p, n)) return true;
-    // (the 16-row kernel is better than its estimate where every SM has a window: 3000 x 1100 at 10 %, 128 columns 12.4 us against 13.3)
-    const double margin = p->info.total_tiles < kPairMinShortTiles && p->info.eff_row_windows >= (uint64_t)p->n_sms ? 1.1 : 1.0;
-    return tall_launch(p, p->tall, n).micros * margin < short_micros(p, n);
+// Whether a launch goes to the super-window kernels, how, and what it needs of the plan's scratch.  Worked out once a launch.
+// Only with the TMA gathers, and - unless forced, for B at least one 128-byte box wide - only when it is expected to be faster.
+struct TallChoice {
+    bool use, pair;
+    uint32_t parts;
+    size_t partial_bytes, packed_bytes;
+};
+TallChoice choose_tall(const b200spmm_plan *p, int64_t n) {
+    TallChoice c{};
+    if (!p->tall.tiles || p->gather_cpasync) return c;
+    const bool can_pair = p->pair.tiles && p->pair_clusters > 0 && n > 128;
+    if (p->tall_forced) {
+        c.use = n * p->info.elt_size >= 128;
+        c.pair = can_pair;
+        c.parts = 1;
+    } else {
+        const uint32_t least = tall_least_parts(p, n);
+        const double short_time = short_micros(p, n);
+        TallLaunch l{};
+        if (can_pair) l = tall_launch(p, p->pair, n, least);
+        c.use = c.pair = can_pair && l.micros < short_time;
+        if (!c.pair) {
+            // (the 16-row kernel is better than its estimate where every SM has a window: 3000 x 1100 at 10 %, 128 columns 12.4 us against 13.3)
+            const double margin = p->info.total_tiles < kPairMinShortTiles && p->info.eff_row_windows >= (uint64_t)p->n_sms ? 1.1 : 1.0;
+            l = tall_launch(p, p->tall, n, least);
+            c.use = l.micros * margin < short_time;
+        }
+        c.parts = l.parts;
+    }
+    const TallFormat &f = c.pair ? p->pair : p->tall;
+    if (c.parts > 1) c.partial_bytes = (size_t)c.parts * (size_t)f.eff * f.rows * (size_t)n * 4;  // kTallMaxSums
+    if (p->tall_pack_b) {
+        // the pair kernel's CTAs fetch 128-feature halves of a 256-feature slab: both halves of the last slab must
+        // exist in the packed copy (as zeros past n), so an even number of 128-feature blocks
+        const size_t features = c.pair || n > 128 ? (size_t)(n + 255) / 256 * 256 : 128;
+        c.packed_bytes = features * 32u * (size_t)((p->info.cols + p->info.col_window - 1) / p->info.col_window);
+    }
+    return c;
 }
 
 // Column blocks per group for B of width n: as many as fit shared memory, 0 if the kernel does not take it.  Every
@@ -763,7 +786,7 @@ uint32_t narrow_group_blocks(const b200spmm_plan *p, int64_t n) {
     if (p->rows_only || g < f.n_blocks) return 0;
     const double rows = (double)p->info.rows / f.n_ctas, rounds = std::ceil(rows / 32.0) * 32.0 / rows;
     const double micros = 4.0 + (double)p->info.nnzs * (double)vecs * 1.05e-6 * (148.0 / p->n_sms) * rounds;
-    const TallLaunch tall = p->tall.tiles && !p->gather_cpasync ? tall_launch(p, p->tall, n) : TallLaunch{1e30, 1};
+    const TallLaunch tall = p->tall.tiles && !p->gather_cpasync ? tall_launch(p, p->tall, n, tall_least_parts(p, n)) : TallLaunch{1e30, 1};
     return micros < tall.micros && micros < short_micros(p, n) ? g : 0;
 }
 
@@ -798,34 +821,13 @@ int launch_narrow(b200spmm_plan *p, uint32_t group_blocks, const void *d_B, int6
     return B200SPMM_OK;
 }
 
-// What a super-window launch needs of the plan's scratch.
-struct TallScratch {
-    uint32_t parts;
-    size_t partial_bytes, packed_bytes;
-};
-TallScratch tall_scratch(const b200spmm_plan *p, int64_t n) {
-    const bool pair = use_pair(p, n);
-    TallScratch s{};
-    const TallFormat &f = pair ? p->pair : p->tall;
-    s.parts = tall_launch(p, f, n).parts;
-    if (s.parts > 1) s.partial_bytes = (size_t)s.parts * (size_t)f.eff * f.rows * (size_t)n * 4;  // kTallMaxSums
-    if (p->tall_pack_b) {
-        // the pair kernel's CTAs fetch 128-feature halves of a 256-feature slab: both halves of the last slab must
-        // exist in the packed copy (as zeros past n), so an even number of 128-feature blocks
-        const size_t features = pair || n > 128 ? (size_t)(n + 255) / 256 * 256 : 128;
-        s.packed_bytes = features * 32u * (size_t)((p->info.cols + p->info.col_window - 1) / p->info.col_window);
-    }
-    return s;
-}
-
-int launch_tall(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
+int launch_tall(b200spmm_plan *p, const TallChoice &choice, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
                 cudaStream_t stream) {
     const bool tf32 = p->info.dtype == B200SPMM_TF32;
     int st = b_tensor_map(p, d_B, ldb, (uint32_t)n, (uint32_t)p->info.cols, tf32);
     if (st != B200SPMM_OK) return st;
-    const bool pair = use_pair(p, n);
+    const bool pair = choice.pair;
     const TallFormat &fmt = pair ? p->pair : p->tall;
-    const TallScratch scratch = tall_scratch(p, n);
     TallParams prm{};
     prm.rowOffset = fmt.d_rowOffset;
     prm.tcA2B = fmt.d_tcA2B;
@@ -836,7 +838,7 @@ int launch_tall(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void 
         const uint32_t slab = (n <= 128 || pair) ? 128u : 256u;
         const uint32_t n_slabs = pair ? 2u * (uint32_t)((n + 255) / 256) : (uint32_t)((n + slab - 1) / slab);
         const uint32_t groups = (uint32_t)((p->info.cols + cw - 1) / cw);
-        const size_t need = scratch.packed_bytes;  // n_slabs * groups * 32 * slab
+        const size_t need = choice.packed_bytes;  // n_slabs * groups * 32 * slab
         st = take_scratch(p, &p->b_packed, need, stream);
         if (st != B200SPMM_OK) return st;
         const int grid = (int)std::min<size_t>((need / 16 + 255) / 256, (size_t)p->n_sms * 16);
@@ -845,7 +847,7 @@ int launch_tall(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void 
         prm.b_packed = static_cast<const uint8_t *>(p->b_packed.ptr);
         prm.b_groups = groups;
     }
-    prm.parts = take_scratch(p, &p->partial, scratch.partial_bytes, stream) == B200SPMM_OK ? scratch.parts : 1u;  // no room: whole windows
+    prm.parts = take_scratch(p, &p->partial, choice.partial_bytes, stream) == B200SPMM_OK ? choice.parts : 1u;  // no room: whole windows
     prm.partial = static_cast<float *>(p->partial.ptr);
     prm.partial_rows = (uint32_t)(fmt.eff * fmt.rows);
     prm.sched_counter = p->d_status + 1;
@@ -1591,7 +1593,8 @@ int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, voi
         if (st != B200SPMM_OK) return st;
     }
     note_bounded_waits(p, stream);
-    if (band < 0 && use_tall(p, n)) return launch_tall(p, d_B, ldb, n, d_C, ldc, c_dtype, stream);
+    const TallChoice tall = band < 0 ? choose_tall(p, n) : TallChoice{};
+    if (tall.use) return launch_tall(p, tall, d_B, ldb, n, d_C, ldc, c_dtype, stream);
     SpmmParams prm{};
     prm.rowOffset = p->d_rowOffset;
     prm.tcA2B = p->d_tcA2B;
@@ -1709,7 +1712,7 @@ static int run_host(b200spmm_plan_t *p, const void *h_B, int64_t n, void *h_C, i
         band_row.clear();
         for (const RowBand &b : p->rows_fmt.bands) band_row.push_back(b.row);
     }
-    const size_t bands = band_row.size() > 1 && !narrow_group_blocks(p, n) && (rows || !use_tall(p, n)) ? band_row.size() - 1 : 1;
+    const size_t bands = band_row.size() > 1 && !narrow_group_blocks(p, n) && (rows || !choose_tall(p, n).use) ? band_row.size() - 1 : 1;
     if (bands == 1 || p->info.eff_row_windows == 0) {
         B200_CUDA_TRY(cudaMemcpyAsync(p->d_B, h_B, b_bytes, cudaMemcpyHostToDevice, nullptr));
         int st = b200spmm_spmm(p, p->d_B, n, n, p->d_C, n, c_dtype, nullptr);
