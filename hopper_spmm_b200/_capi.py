@@ -117,6 +117,7 @@ SIGNATURES = {
     "b200spmm_kat_umma_pair": (C.c_int, [vp, u32, C.POINTER(KatMma), C.c_int, C.c_int, vp, C.c_int]),
     "b200spmm_kat_wait_limit": (C.c_uint64, [C.c_uint64]),
     "b200spmm_kat_spmm_starved": (C.c_int, [vp, vp, i64, i64, vp, i64, C.c_uint64, vp]),
+    "b200spmm_kat_scratch_limit": (C.c_int, [vp, C.c_uint64]),
     "b200spmm_kat_instr_desc": (u32, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]),
     "b200spmm_kat_tma": (C.c_int, [vp, u64, u64, u64, C.c_int, u32, u32, C.c_int, vp, C.c_int, u32, vp, u32,
                                     C.c_int]),

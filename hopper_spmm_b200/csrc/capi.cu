@@ -135,6 +135,7 @@ struct b200spmm_plan {
     uint32_t tmap_b_n = 0;
     bool row_boxes = false;       // keep tmap_bt (the allocation-free call encodes one map only)
     bool gather_cpasync = false;  // B200SPMM_GATHER=cpasync, read when the plan is made
+    size_t scratch_limit = ~(size_t)0;  // b200spmm_kat_scratch_limit only: who needs more asks for more than there is
     unsigned long long wait_limit_ns = kDeviceWaitLimitNs;  // how long a wait inside the kernel may last
     bool starve_gathers = false;  // b200spmm_kat_spmm_starved only: B's tensor map delivers half the bytes
     // buffers of the host-pointer entry point, grown on demand
@@ -355,10 +356,11 @@ int take_scratch(b200spmm_plan *p, b200spmm_plan::Scratch *s, size_t bytes, cuda
         }
         s->in_graph = false;
         s->bytes = 0;
+        const size_t ask = bytes <= p->scratch_limit ? bytes : (size_t)1 << 60;
         if (captured) {
-            B200_CUDA_TRY(pool_alloc_under_capture(&s->ptr, bytes));
+            B200_CUDA_TRY(pool_alloc_under_capture(&s->ptr, ask));
         } else {
-            const int st = grow_buffer(&s->ptr, bytes);
+            const int st = grow_buffer(&s->ptr, ask);
             if (st != B200SPMM_OK) return st;
         }
         s->bytes = bytes;
@@ -731,7 +733,7 @@ TallLaunch tall_launch(const b200spmm_plan *p, const TallFormat &f, int64_t n, u
 // Only with the TMA gathers, and - unless forced, for B at least one 128-byte box wide - only when it is expected to be faster.
 struct TallChoice {
     bool use, pair;
-    uint32_t parts;
+    uint32_t parts, least_parts;  // with fewer than the second the sums would be less exact than those of 16 rows
     size_t partial_bytes, packed_bytes;
 };
 TallChoice choose_tall(const b200spmm_plan *p, int64_t n) {
@@ -741,9 +743,9 @@ TallChoice choose_tall(const b200spmm_plan *p, int64_t n) {
     if (p->tall_forced) {
         c.use = n * p->info.elt_size >= 128;
         c.pair = can_pair;
-        c.parts = 1;
+        c.parts = c.least_parts = 1;
     } else {
-        const uint32_t least = tall_least_parts(p, n);
+        const uint32_t least = c.least_parts = tall_least_parts(p, n);
         const double short_time = short_micros(p, n);
         TallLaunch l{};
         if (can_pair) l = tall_launch(p, p->pair, n, least);
@@ -847,7 +849,7 @@ int launch_tall(b200spmm_plan *p, const TallChoice &choice, const void *d_B, int
         prm.b_packed = static_cast<const uint8_t *>(p->b_packed.ptr);
         prm.b_groups = groups;
     }
-    prm.parts = take_scratch(p, &p->partial, choice.partial_bytes, stream) == B200SPMM_OK ? choice.parts : 1u;  // no room: whole windows
+    prm.parts = choice.parts;
     prm.partial = static_cast<float *>(p->partial.ptr);
     prm.partial_rows = (uint32_t)(fmt.eff * fmt.rows);
     prm.sched_counter = p->d_status + 1;
@@ -1593,7 +1595,12 @@ int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, voi
         if (st != B200SPMM_OK) return st;
     }
     note_bounded_waits(p, stream);
-    const TallChoice tall = band < 0 ? choose_tall(p, n) : TallChoice{};
+    TallChoice tall = band < 0 ? choose_tall(p, n) : TallChoice{};
+    if (tall.parts > 1 && tall.use && take_scratch(p, &p->partial, tall.partial_bytes, stream) != B200SPMM_OK) {
+        // no room for the parts' sums: whole windows where they are as exact, else the 16-row kernel
+        tall.use = tall.least_parts <= 1;
+        tall.parts = 1;
+    }
     if (tall.use) return launch_tall(p, tall, d_B, ldb, n, d_C, ldc, c_dtype, stream);
     SpmmParams prm{};
     prm.rowOffset = p->d_rowOffset;
@@ -1830,6 +1837,13 @@ int b200spmm_kat_spmm_starved(b200spmm_plan_t *p, const void *d_B, int64_t ldb, 
     p->wait_limit_ns = kDeviceWaitLimitNs;
     p->tmap_b_ptr = nullptr;
     return st;
+}
+
+/* Declared in b200_spmm_kat.h: a device without room for more scratch. */
+int b200spmm_kat_scratch_limit(b200spmm_plan_t *p, uint64_t bytes) {
+    if (!p) return B200SPMM_ERR_INVALID_ARG;
+    p->scratch_limit = (size_t)bytes;
+    return B200SPMM_OK;
 }
 
 int b200spmm_spmm_noalloc_status(int device, void *stream_v) {

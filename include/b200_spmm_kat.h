@@ -73,6 +73,12 @@ struct b200spmm_plan;
 int b200spmm_kat_spmm_starved(struct b200spmm_plan *plan, const void *d_B, int64_t ldb, int64_t n, void *d_C,
                               int64_t ldc, unsigned long long limit_ns, void *stream);
 
+/*
+ * From here on a launch of `plan` that needs a scratch buffer of more than `bytes` asks for more memory than any device
+ * has, and finds none, as where others hold it.  A buffer that is there and large enough serves on.
+ */
+int b200spmm_kat_scratch_limit(struct b200spmm_plan *plan, uint64_t bytes);
+
 /* Builds an instruction descriptor: fmt 0 = f16, 1 = bf16, 2 = tf32; fp32 accumulate. */
 uint32_t b200spmm_kat_instr_desc(int fmt, int m, int n, int a_mn_major, int b_mn_major);
 

@@ -300,3 +300,45 @@ def test_sums_are_as_exact_as_those_of_the_16_row_kernel(dt, rows, cols, n, monk
             plan.close()
     assert window == {None: 128, "16": 16}
     assert off[None] <= 1.05 * off["16"]
+
+
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("dt,rows,cols,n,window", [(np.float16, 1300, 6003, 104, 16), (np.float32, 1300, 6003, 104, 16), (np.float16, 6000, 3000, 192, 256)])
+def test_no_room_for_the_sums_of_parts(dt, rows, cols, n, window, captured, monkeypatch):
+    # the kernel of 16 rows takes over where whole windows would be less exact than it, bit for bit; else whole windows do
+    import torch
+    from hopper_spmm_b200 import _capi as capi
+    rows, cols, rp, ci, v = random_csr(rows, cols, 0.15, 9, dt)
+    B = torch.from_numpy(dense_b(cols, n, 3, dt)).cuda()
+    f = hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v))
+    plan = hs.SpmmPlan(f)
+    monkeypatch.setenv("B200SPMM_WINDOW", str(window))
+    same = hs.SpmmPlan(f)
+    try:
+        want = same.spmm(B).clone()
+        info = same.launch_info()
+        assert info.row_window == window
+        # room for B re-laid, or for the pieces of the 16-row kernel: two CTAs an SM have at most 296 more than there are windows
+        assert capi.lib().b200spmm_kat_scratch_limit(plan._p, 400 * 16 * n * 4) == 0
+        got = torch.full((rows, n), float("nan"), device="cuda")
+        if captured:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g):
+                plan.spmm(B, got, sync=False)
+            g.replay()
+        else:
+            plan.spmm(B, got)
+        now = plan.launch_info()
+        assert (now.row_window, now.kernel_launches) == (window, info.kernel_launches)
+        assert torch.equal(got, want)
+        assert capi.lib().b200spmm_kat_scratch_limit(plan._p, 2**63) == 0
+        parts = plan.spmm(B)
+        assert plan.launch_info().row_window > 16 and plan.launch_info().kernel_launches == 3
+        parity.check(parts.cpu().numpy(), rows, rp, ci, v, B.cpu().numpy())
+        if captured:
+            got.fill_(float("nan"))
+            g.replay()
+            assert torch.equal(got, want)
+    finally:
+        plan.close()
+        same.close()
