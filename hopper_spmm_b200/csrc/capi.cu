@@ -668,8 +668,10 @@ int launch_narrow_vecs(const NarrowParams &prm, int vecs, unsigned n_ctas, size_
 // whole / 2 / 4 / 8 (16-row kernel): 1777 x 7404 at 15 %, fp16, 104 columns 38.6 / 26.2 / 19.1 / 15.9 (43); 1668 x 5737 at
 // 28 %, tf32, 392 columns 67 / 46 / 35 / - (114); 1682 x 1536 at 11 %, fp16, 816 columns 28 / 21.5 / - / - (78); more than one
 // round of parts is slower again (2000 x 8000 at 10 %, 1,024 columns 56 / 45 / 55 / 81).
-// Up to 64 columns a matrix of fewer than kSplitMinShortTiles tiles keeps to whole windows, and so mostly to the 16-row
-// kernel, a choice that is held to elsewhere: 3000 x 3000 at 12 %, 64 columns 19 us where six parts would take 12.5.
+// Up to 64 columns a matrix whose 16-row schedule cuts no window keeps to whole windows or to that kernel, which then is one
+// launch and not two: 1024 x 1024 / 1300 x 1024 / 2048 x 1024 at 30 %, fp16, 64 columns 8.6 / 8.7 / 8.8 us, in parts 10.9 / 10.8 / 10.5.
+// Where it cuts some, parts are as fast from the smallest on (1040 x 1040 at 30 %, tf32, 40 columns 11.3 and 11.5; 1024 x 1700, 64
+// columns 12.4 and 12.4; 3000 x 3000 at 12 %, fp16 19.1 -> 13.2, tf32 24.7 -> 16.3; 2001 x 6167 at 28 %, 40 columns 33.2 -> 13.6).
 //
 // The tensor core cuts what it adds, so the error of a sum grows with the tiles it runs through: 1.4e-8 a tile here, and with 16
 // rows 1.6e-8 and more in fp16, 1.1e-8 in tf32, over the tiles of a piece of a window.  Where whole super-windows are not
@@ -679,7 +681,6 @@ struct TallLaunch {
     double micros;
     uint32_t parts;
 };
-constexpr uint64_t kSplitMinShortTiles = 80000;
 constexpr double kTallMaxSums = 128e6;  // bytes
 double short_micros(const b200spmm_plan *p, int64_t n) {  // (tiles over 148 SMs)
     return 14.0 + (double)p->info.total_tiles * (148.0 / p->n_sms) * (n <= 64 ? 0.28e-3 : 0.4e-3 * (double)((n + 127) / 128));
@@ -710,7 +711,7 @@ TallLaunch tall_launch(const b200spmm_plan *p, const TallFormat &f, int64_t n, u
     const double whole = tall_whole_micros(p, f, n);
     if (p->tall_forced) return {whole, 1};
     TallLaunch best{least > 1 ? 1e30 : whole, 1};
-    if (n <= 64 && p->info.total_tiles < kSplitMinShortTiles) return best;
+    if (n <= 64 && p->sched.n_splits == 0) return best;
     const bool pair = tall_is_pair(f);
     const int64_t units = pair ? p->pair_clusters : p->n_sms, items = tall_items(f, n);
     const double longest = (double)f.max_window_tiles, alone = pair ? 0.088 : n > 128 ? 0.105 : 0.068;
@@ -776,7 +777,10 @@ TallChoice choose_tall(const b200spmm_plan *p, int64_t n) {
 // would be faster (6000 x 8192 at 20 %, 24 columns 49.6 us against 23.4): its fp32 sums are thirty times as exact as the
 // tensor core's.  32 fp16 columns go to it where all of B fits shared memory and it is expected to be faster than the tiles (1100 x
 // 1100 at 20 % 11.6 -> 7.5 us, 1682 x 1536 at 11 % 13.5 -> 10.0, 3000 x 3000 at 12 % 19.2 -> 17.0; 2000 x 8000 at 6 %, in two
-// halves, 36 against 20).
+// halves, 36 against 20).  Below kNarrowPartsTiles tiles than 16 rows or whole windows: windows in parts would be faster (4885 x
+// 1335 at 25 % 15.4 and 12.4 us, 3513 x 3235 at 26 % 23.4 and 12.6), and here too its sums are what it is kept for; above, it
+// would take twice the time of the parts (8221 x 3229 at 25 % 33.4 and 17.0; 16972 x 2328 at 28 % 43.1 and 18.2).
+constexpr uint64_t kNarrowPartsTiles = 80000;
 uint32_t narrow_group_blocks(const b200spmm_plan *p, int64_t n) {
     const NarrowFormat &f = p->narrow;
     const int64_t vecs = n * p->info.elt_size / 16;
@@ -788,8 +792,13 @@ uint32_t narrow_group_blocks(const b200spmm_plan *p, int64_t n) {
     if (p->rows_only || g < f.n_blocks) return 0;
     const double rows = (double)p->info.rows / f.n_ctas, rounds = std::ceil(rows / 32.0) * 32.0 / rows;
     const double micros = 4.0 + (double)p->info.nnzs * (double)vecs * 1.05e-6 * (148.0 / p->n_sms) * rounds;
-    const TallLaunch tall = p->tall.tiles && !p->gather_cpasync ? tall_launch(p, p->tall, n, tall_least_parts(p, n)) : TallLaunch{1e30, 1};
-    return micros < tall.micros && micros < short_micros(p, n) ? g : 0;
+    double tall = 1e30;
+    if (p->tall.tiles && !p->gather_cpasync) {
+        const uint32_t least = p->tall_forced ? 1 : tall_least_parts(p, n);
+        if (p->info.total_tiles >= kNarrowPartsTiles) tall = tall_launch(p, p->tall, n, least).micros;
+        else if (least <= 1) tall = tall_whole_micros(p, p->tall, n);
+    }
+    return micros < tall && micros < short_micros(p, n) ? g : 0;
 }
 
 int launch_narrow(b200spmm_plan *p, uint32_t group_blocks, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,

@@ -184,10 +184,11 @@ def test_starved_pipeline_times_out_and_the_plan_recovers(dt, tall):
         plan.close()
 
 
-@pytest.mark.parametrize("dt,n,window", [(np.float16, 64, 16), (np.float16, 136, 256), (np.float16, 256, 256), (np.float32, 64, 16),
+@pytest.mark.parametrize("dt,n,window", [(np.float16, 64, 128), (np.float16, 136, 256), (np.float16, 256, 256), (np.float32, 64, 128),
                                          (np.float32, 200, 256)])
 def test_fewer_windows_than_sms_take_the_kernel_expected_to_be_faster(dt, n, window):
-    # twelve windows of 256 rows: most pairs of SMs stay idle, and from two slabs of 128 on they are still the faster ones
+    # twelve windows of 256 rows: most pairs of SMs stay idle, and in parts they are still the faster ones, as are those of 128
+    # rows (64 columns in us, 16 rows and parts: fp16 19.1 and 13.2, tf32 24.7 and 16.3)
     import torch
     rows, cols, rp, ci, v = random_csr(2990, 3001, 0.12, 5, dt, empty_rows=[(512, 640)])
     B = dense_b(cols, n, 3, dt)
@@ -227,6 +228,24 @@ def test_few_windows_are_cut_into_parts(dt, rows, n, window):
             plan.spmm(Bv, out, sync=False)
         g.replay()
         assert torch.equal(out, got)
+    finally:
+        plan.close()
+
+
+@pytest.mark.parametrize("dt,rows,cols,n,window", [(np.float16, 1024, 1024, 64, 16), (np.float16, 1024, 1700, 64, 128), (np.float32, 1040, 1040, 40, 128),
+                                                   (np.float16, 3513, 3235, 32, 16), (np.float16, 3513, 3235, 40, 128)])
+def test_up_to_64_columns_parts_are_for_schedules_that_cut_windows(dt, rows, cols, n, window):
+    # where the 16-row kernel needs no second launch it is the faster one; 32 fp16 columns keep the exacter sums of the narrow kernel
+    import torch
+    rows, cols, rp, ci, v = random_csr(rows, cols, 0.3, 5, dt)
+    B = dense_b(cols, n, 3, dt)
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    try:
+        C = plan.spmm(torch.from_numpy(B).cuda())
+        info = plan.launch_info()
+        assert info.row_window == window and info.kernel_launches == (3 if window == 128 else 1)
+        assert (info.stages == 0) == (n == 32)  # the narrow kernel
+        parity.check(C.cpu().numpy(), rows, rp, ci, v, B)
     finally:
         plan.close()
 
@@ -278,7 +297,8 @@ def test_merging_more_columns_than_a_bit_set_holds(dt, tall):
 
 
 @pytest.mark.parametrize("dt,rows,cols,n", [(np.float16, 1682, 1536, 816), (np.float16, 1100, 2400, 512), (np.float16, 1300, 6003, 104),
-                                            (np.float32, 1100, 1100, 512), (np.float32, 1100, 2400, 512), (np.float32, 1300, 6003, 104)])
+                                            (np.float32, 1100, 1100, 512), (np.float32, 1100, 2400, 512), (np.float32, 1300, 6003, 104),
+                                            (np.float16, 1300, 6003, 64), (np.float16, 1830, 1326, 40), (np.float32, 1300, 1024, 24), (np.float32, 1124, 5185, 64)])
 def test_sums_are_as_exact_as_those_of_the_16_row_kernel(dt, rows, cols, n, monkeypatch):
     # against 64 bits, from the values as the tensor core reads them: super-windows that take what 16 rows would otherwise
     # are cut into parts short enough.  (5 %: the errors are those of some thousand sums cut at 24 bits)
