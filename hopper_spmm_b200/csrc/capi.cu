@@ -668,9 +668,10 @@ int launch_narrow_vecs(const NarrowParams &prm, int vecs, unsigned n_ctas, size_
 // whole / 2 / 4 / 8 (16-row kernel): 1777 x 7404 at 15 %, fp16, 104 columns 38.6 / 26.2 / 19.1 / 15.9 (43); 1668 x 5737 at
 // 28 %, tf32, 392 columns 67 / 46 / 35 / - (114); 1682 x 1536 at 11 %, fp16, 816 columns 28 / 21.5 / - / - (78); more than one
 // round of parts is slower again (2000 x 8000 at 10 %, 1,024 columns 56 / 45 / 55 / 81).
-// Up to 64 columns a matrix whose 16-row schedule cuts no window keeps to whole windows or to that kernel, which then is one
-// launch and not two: 1024 x 1024 / 1300 x 1024 / 2048 x 1024 at 30 %, fp16, 64 columns 8.6 / 8.7 / 8.8 us, in parts 10.9 / 10.8 / 10.5.
-// Where it cuts some, parts are as fast from the smallest on (1040 x 1040 at 30 %, tf32, 40 columns 11.3 and 11.5; 1024 x 1700, 64
+// Up to 64 columns a matrix of fewer than kOneLaunchTiles tiles whose 16-row schedule cuts no window keeps to whole windows or to
+// that kernel, which then is one launch and not two: 1024 x 1024 / 2048 x 1024 / 4096 x 1024 at 25 %, fp16, 64 columns 8.9 / 9.2 /
+// 9.3 us, in parts 11.0 / 10.7 / 11.7.  Parts are as fast above (4736 x 1090, 20,424 tiles, 12.1 both, and 4736 x 1500 13.4 -> 12.1),
+// and where windows are cut from the smallest matrices on (1040 x 1040 at 30 %, tf32, 40 columns 11.3 and 11.5; 1024 x 1700, 64
 // columns 12.4 and 12.4; 3000 x 3000 at 12 %, fp16 19.1 -> 13.2, tf32 24.7 -> 16.3; 2001 x 6167 at 28 %, 40 columns 33.2 -> 13.6).
 //
 // The tensor core cuts what it adds, so the error of a sum grows with the tiles it runs through: 1.4e-8 a tile here, and with 16
@@ -681,6 +682,7 @@ struct TallLaunch {
     double micros;
     uint32_t parts;
 };
+constexpr uint64_t kOneLaunchTiles = 20000;
 constexpr double kTallMaxSums = 128e6;  // bytes
 double short_micros(const b200spmm_plan *p, int64_t n) {  // (tiles over 148 SMs)
     return 14.0 + (double)p->info.total_tiles * (148.0 / p->n_sms) * (n <= 64 ? 0.28e-3 : 0.4e-3 * (double)((n + 127) / 128));
@@ -711,7 +713,7 @@ TallLaunch tall_launch(const b200spmm_plan *p, const TallFormat &f, int64_t n, u
     const double whole = tall_whole_micros(p, f, n);
     if (p->tall_forced) return {whole, 1};
     TallLaunch best{least > 1 ? 1e30 : whole, 1};
-    if (n <= 64 && p->sched.n_splits == 0) return best;
+    if (n <= 64 && p->sched.n_splits == 0 && p->info.total_tiles < kOneLaunchTiles) return best;
     const bool pair = tall_is_pair(f);
     const int64_t units = pair ? p->pair_clusters : p->n_sms, items = tall_items(f, n);
     const double longest = (double)f.max_window_tiles, alone = pair ? 0.088 : n > 128 ? 0.105 : 0.068;

@@ -233,7 +233,7 @@ def test_few_windows_are_cut_into_parts(dt, rows, n, window):
 
 
 @pytest.mark.parametrize("dt,rows,cols,n,window", [(np.float16, 1024, 1024, 64, 16), (np.float16, 1024, 1700, 64, 128), (np.float32, 1040, 1040, 40, 128),
-                                                   (np.float16, 3513, 3235, 32, 16), (np.float16, 3513, 3235, 40, 128)])
+                                                   (np.float16, 3513, 3235, 32, 16), (np.float16, 3513, 3235, 40, 128), (np.float16, 4736, 2200, 64, 128)])
 def test_up_to_64_columns_parts_are_for_schedules_that_cut_windows(dt, rows, cols, n, window):
     # where the 16-row kernel needs no second launch it is the faster one; 32 fp16 columns keep the exacter sums of the narrow kernel
     import torch
