@@ -580,11 +580,11 @@ int launch_rows_grid(b200spmm_plan *p, const RowsParams &prm, dim3 grid, void (*
 int launch_rows(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
                 cudaStream_t stream, int band) {
     const RowsFormat &f = p->rows_fmt;
-    if (band >= 0 && (size_t)band + 1 >= f.bands.size()) return B200SPMM_ERR_INVALID_ARG;
+    if (band >= 0 && ((size_t)band + 1 >= f.bands.size() || (f.bands.size() > 2 && !f.d_band_units))) return B200SPMM_ERR_INVALID_ARG;
     const RowBand &from = f.bands[band < 0 ? 0 : band], &to = band < 0 ? f.bands.back() : f.bands[band + 1];
     RowsParams prm{};
     prm.batches = f.d_batches;
-    prm.units = band >= 0 && f.d_band_units ? f.d_band_units : f.d_units;
+    prm.units = band >= 0 && f.bands.size() > 2 ? f.d_band_units : f.d_units;
     prm.unit_begin = from.unit;
     prm.unit_end = to.unit;
     prm.empty_begin = from.empty;
@@ -1725,12 +1725,18 @@ static int run_host(b200spmm_plan_t *p, const void *h_B, int64_t n, void *h_C, i
         p->d_C_bytes = c_bytes;
     }
     const bool rows = use_rows(p, n);
-    std::vector<uint64_t> band_row = p->sched.band_row;
-    if (rows) {
-        band_row.clear();
-        for (const RowBand &b : p->rows_fmt.bands) band_row.push_back(b.row);
+    std::vector<uint64_t> band_row;
+    if (!narrow_group_blocks(p, n)) {
+        if (rows) {
+            const int st = build_band_units(&p->rows_fmt, p->info.dtype == B200SPMM_TF32);
+            if (st != B200SPMM_OK) return st;
+            if (p->rows_fmt.d_band_units)
+                for (const RowBand &b : p->rows_fmt.bands) band_row.push_back(b.row);
+        } else if (!choose_tall(p, n).use) {
+            band_row = p->sched.band_row;
+        }
     }
-    const size_t bands = band_row.size() > 1 && !narrow_group_blocks(p, n) && (rows || !choose_tall(p, n).use) ? band_row.size() - 1 : 1;
+    const size_t bands = band_row.size() > 1 ? band_row.size() - 1 : 1;
     if (bands == 1 || p->info.eff_row_windows == 0) {
         B200_CUDA_TRY(cudaMemcpyAsync(p->d_B, h_B, b_bytes, cudaMemcpyHostToDevice, nullptr));
         int st = b200spmm_spmm(p, p->d_B, n, n, p->d_C, n, c_dtype, nullptr);

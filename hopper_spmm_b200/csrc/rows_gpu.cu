@@ -5,8 +5,7 @@
 //   2. per (window, row): running sums over the window's runs -> row lengths, and how many units there are of every length;
 //      one scan over the rows -> the units, slots and bands.  The longest come first, so the lengths alone say where every
 //      unit of a length lies and where its batches do: the host's one wait
-//   3. every row puts its units into the list; where there are bands, the list once more with the bands apart (CUB radix
-//      sort, four key bits)
+//   3. every row puts its units into the list
 //   4. the warps of step 1 write (column, value) to the place of their row's unit
 // Eight launches and one wait before the last.  With the units sorted (CUB), three scans and a launch for each small step there
 // were 26; the plan of a graph of 60,000 nodes and 700,000 entries took 232 us instead of 158, of 10,000 nodes 200 instead of 123.
@@ -292,8 +291,8 @@ row_totals_kernel(uint32_t rows, const RowSums *__restrict__ sums, LengthTables 
 // line of the split table.
 __global__ void __launch_bounds__(kBlock)
 place_units_kernel(const uint32_t *__restrict__ row_len, uint32_t rows, uint32_t cap, const RowSums *__restrict__ sums, LengthTables *__restrict__ tables,
-                   const RowTotals *__restrict__ totals, uint32_t bands, uint2 *__restrict__ units, uint32_t *__restrict__ unit_batch,
-                   RowSplit *__restrict__ splits, uint32_t *__restrict__ band_keys, uint32_t *__restrict__ batches, uint32_t batch_words) {
+                   const RowTotals *__restrict__ totals, uint2 *__restrict__ units, uint32_t *__restrict__ unit_batch,
+                   RowSplit *__restrict__ splits, uint32_t *__restrict__ batches, uint32_t batch_words) {
     __shared__ uint32_t base[kLengths + 1];
     for (uint32_t k = threadIdx.x; k <= kLengths; k += kBlock) base[k] = 0;
     __syncthreads();
@@ -316,8 +315,6 @@ place_units_kernel(const uint32_t *__restrict__ row_len, uint32_t rows, uint32_t
         batches[(uint64_t)totals->n_batches * batch_words + threadIdx.x] = batch_words == kBatchWords<true> ? (threadIdx.x == kTargetWord<true> ? kNoTarget : 0u)
                                                                                                  : (threadIdx.x == kTargetWord<false> ? kNoTarget : 0u);
     if (r >= rows) return;
-    uint32_t band = 0;
-    for (uint32_t k = 1; k < bands; ++k) band += r >= totals->band_row[k] ? 1u : 0u;
     const uint32_t first_unit = (uint32_t)sums[r].a - n;
     for (uint32_t q = 0; q < n; ++q) {
         const uint32_t key = q < full ? full_key : last_key, place = q < full ? base[full_key] + rank_full + q : base[last_key] + rank_last;
@@ -329,9 +326,38 @@ place_units_kernel(const uint32_t *__restrict__ row_len, uint32_t rows, uint32_t
             unit_batch[first_unit + q] = first;
         }
         units[place] = key != kEmpty ? make_uint2(first, batches_of_length(key)) : make_uint2(r, 0u);
-        if (bands > 1) band_keys[place] = (key != kEmpty ? 0u : kEmptyBandKey) | band;
     }
     if (n > 1) splits[(uint32_t)(sums[r].b >> 32) - 1] = RowSplit{r, (uint32_t)sums[r].b - n, (uint32_t)sums[r].b};
+}
+
+// The first rows of the bands.
+struct BandRows {
+    uint32_t row[kMaxBands];
+};
+
+// The band of every unit in the list, from the row that it adds to: its last batch names the row, or the slot of a cut one.
+__global__ void __launch_bounds__(kBlock)
+band_keys_kernel(const uint2 *__restrict__ units, uint32_t n_units, const uint32_t *__restrict__ batches, uint32_t batch_words, uint32_t target_word,
+                 const RowSplit *__restrict__ splits, uint32_t n_splits, BandRows first, uint32_t bands, uint32_t *__restrict__ keys) {
+    const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
+    if (i >= n_units) return;
+    const uint2 unit = units[i];
+    uint32_t row = unit.x;
+    if (unit.y) {
+        row = batches[(uint64_t)(unit.x + 4u * (unit.y - 1u)) * batch_words + target_word];
+        if (row & kSlotTarget) {
+            const uint32_t slot = row & ~kSlotTarget;
+            uint32_t lo = 0, hi = n_splits - 1;  // the last cut row that starts at or before the slot
+            while (lo < hi) {
+                const uint32_t mid = hi - (hi - lo) / 2;
+                if (splits[mid].slot_begin <= slot) lo = mid; else hi = mid - 1;
+            }
+            row = splits[lo].row;
+        }
+    }
+    uint32_t band = 0;
+    for (uint32_t k = 1; k < bands; ++k) band += row >= first.row[k] ? 1u : 0u;
+    keys[i] = (unit.y ? 0u : kEmptyBandKey) | band;
 }
 
 // band k <= bands: the places of its first unit and of its first row without entries in the list of the bands
@@ -625,6 +651,47 @@ int build_narrow(const b200spmm_btcf_info_t &info, uint64_t nnz, const uint32_t 
 
 }  // namespace
 
+int build_band_units(RowsFormat *f, bool tf32) {
+    if (f->d_band_units || f->bands.size() <= 2) return B200SPMM_OK;
+    const uint32_t bands = (uint32_t)f->bands.size() - 1, n = f->n_units;
+    struct Units {
+        uint2 *ptr = nullptr;
+        ~Units() { pool_free(ptr); }
+    } units;
+    PoolScratch tmp;
+    uint32_t *keys[2] = {}, *band_places = nullptr;
+    uint8_t *sort_tmp = nullptr;
+    size_t sort_bytes = 0;
+    B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, keys[0], keys[1], f->d_units, units.ptr, (int64_t)n, 0, kBandKeyBits));
+    cudaError_t e = pool_alloc(&units.ptr, n);
+    for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = tmp.alloc(&keys[k], n);
+    if (e == cudaSuccess) e = tmp.alloc(&band_places, 2 * bands + 2);
+    if (e == cudaSuccess) e = tmp.alloc(&sort_tmp, sort_bytes);
+    if (e == cudaErrorMemoryAllocation) {  // no room: one band
+        cudaGetLastError();
+        return B200SPMM_OK;
+    }
+    B200_CUDA_TRY(e);
+    BandRows first{};
+    for (uint32_t k = 0; k < bands; ++k) first.row[k] = (uint32_t)f->bands[k].row;
+    band_keys_kernel<<<(unsigned)((n + kBlock - 1) / kBlock), kBlock>>>(f->d_units, n, f->d_batches, tf32 ? kBatchWords<true> : kBatchWords<false>,
+                                                                      tf32 ? kTargetWord<true> : kTargetWord<false>, f->d_splits, f->n_splits, first, bands, keys[0]);
+    B200_CUDA_TRY(cudaGetLastError());
+    // (the units of a band keep their order)
+    B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, keys[0], keys[1], f->d_units, units.ptr, (int64_t)n, 0, kBandKeyBits));
+    band_units_kernel<<<1, 32>>>(keys[1], n, bands, band_places);
+    B200_CUDA_TRY(cudaGetLastError());
+    uint32_t places[2 * kMaxBands + 2];
+    B200_CUDA_TRY(cudaMemcpy(places, band_places, (2 * bands + 2) * 4, cudaMemcpyDeviceToHost));
+    for (uint32_t k = 0; k < bands; ++k) {
+        f->bands[k].unit = places[2 * k];
+        f->bands[k].empty = places[2 * k + 1];
+    }
+    f->d_band_units = units.ptr;
+    units.ptr = nullptr;
+    return B200SPMM_OK;
+}
+
 int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOffset, const uint32_t *d_tcA2B,
                       const void *d_data, const uint32_t *d_rowIdx, bool loose, int n_sms, double max_fill, bool force_rows,
                       RowsFormat *out, NarrowFormat *narrow) {
@@ -695,20 +762,17 @@ int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
     const uint64_t n_batches = (uint64_t)f.nnz / kUnitBatch + f.n_units + 6 * (kMaxUnitEntries / kUnitBatch) + 8;
     if (n_batches > 0xFFFFFFFFull || f.n_slots >= kSlotTarget - 1) return B200SPMM_OK;
     const uint32_t words = info.elt_size == 2 ? kBatchWords<false> : kBatchWords<true>;
-    uint32_t *unit_batch = nullptr, *band_keys[2] = {}, *band_places = nullptr;
+    uint32_t *unit_batch = nullptr;
     cudaError_t e = pool_alloc(&f.d_batches, ((uint64_t)f.n_batches + 1) * words);
     if (e == cudaSuccess) e = pool_alloc(&f.d_units, f.n_units);
-    if (e == cudaSuccess && bands > 1) e = pool_alloc(&f.d_band_units, f.n_units);
     if (e == cudaSuccess) e = pool_alloc(&f.d_splits, f.n_splits);
     if (e == cudaSuccess) e = tmp.alloc(&unit_batch, f.n_units);
-    for (int k = 0; k < 2 && e == cudaSuccess && bands > 1; ++k) e = tmp.alloc(&band_keys[k], f.n_units);
-    if (e == cudaSuccess && bands > 1) e = tmp.alloc(&band_places, 2 * bands + 2);
     if (e == cudaErrorMemoryAllocation) {  // no room: the tile kernels still work
         cudaGetLastError();
         return B200SPMM_OK;
     }
     B200_CUDA_TRY(e);
-    place_units_kernel<<<row_grid, kBlock>>>(row_len, rows, cap, sums, tables, totals, bands, f.d_units, unit_batch, f.d_splits, band_keys[0], f.d_batches, words);
+    place_units_kernel<<<row_grid, kBlock>>>(row_len, rows, cap, sums, tables, totals, f.d_units, unit_batch, f.d_splits, f.d_batches, words);
     if (f16)
         write_entries_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data16, d_rowIdx, run_window, n_runs, rows, cols, loose, cap, counts,
                                                              row_len, sums, unit_batch, f.d_batches);
@@ -716,21 +780,6 @@ int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
         write_entries_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data32, d_rowIdx, run_window, n_runs, rows, cols, loose, cap, counts,
                                                              row_len, sums, unit_batch, f.d_batches);
     B200_CUDA_TRY(cudaGetLastError());
-    if (bands > 1) {  // (the units of a band keep their order)
-        size_t sort_bytes = 0;
-        B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, band_keys[0], band_keys[1], f.d_units, f.d_band_units, (int64_t)f.n_units, 0, kBandKeyBits));
-        uint8_t *sort_tmp = nullptr;
-        B200_CUDA_TRY(tmp.alloc(&sort_tmp, sort_bytes));
-        B200_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, band_keys[0], band_keys[1], f.d_units, f.d_band_units, (int64_t)f.n_units, 0, kBandKeyBits));
-        band_units_kernel<<<1, 32>>>(band_keys[1], f.n_units, bands, band_places);
-        B200_CUDA_TRY(cudaGetLastError());
-        uint32_t places[2 * kMaxBands + 2];
-        B200_CUDA_TRY(cudaMemcpy(places, band_places, (2 * bands + 2) * 4, cudaMemcpyDeviceToHost));
-        for (uint32_t k = 0; k < bands; ++k) {
-            f.bands[k].unit = places[2 * k];
-            f.bands[k].empty = places[2 * k + 1];
-        }
-    }
     B200_CUDA_TRY(cudaDeviceSynchronize());
     if (!force_rows && narrow_pays(f.nnz, rows, info.cols, h.max_len, n_sms)) {
         const int st = build_narrow(info, f.nnz, d_rowOffset, d_tcA2B, d_data, d_rowIdx, n_sms, run_window, n_runs, run_grid, counts, sums, narrow);

@@ -28,7 +28,7 @@ struct RowSplit {
     uint32_t row, slot_begin, slot_end;
 };
 
-// A band of whole rows: where in the list of bands its units (longest first) and its rows without entries (behind
+// A band of whole rows: where in the list of the bands its units (longest first) and its rows without entries (behind
 // the units of all bands) begin, its cut rows and its rows.
 struct RowBand {
     uint32_t unit, empty, split;
@@ -38,7 +38,7 @@ struct RowBand {
 struct RowsFormat {
     uint32_t *d_batches = nullptr;    // [n_batches + 1][kBatchWords], the last one belongs to nobody
     uint2 *d_units = nullptr;         // [n_units] first batch and number of batches, longest first, then (row, 0) for rows without entries
-    uint2 *d_band_units = nullptr;    // the same band by band, or null where there is one band
+    uint2 *d_band_units = nullptr;    // the same band by band, once build_band_units has run
     RowSplit *d_splits = nullptr;     // [n_splits] by row
     uint64_t nnz = 0;
     uint32_t n_batches = 0, n_units = 0, n_splits = 0, n_slots = 0;
@@ -64,6 +64,9 @@ struct NarrowFormat {
 int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOffset, const uint32_t *d_tcA2B,
                       const void *d_data, const uint32_t *d_rowIdx, bool loose, int n_sms, double max_fill, bool force_rows,
                       RowsFormat *rows, NarrowFormat *narrow);
+// The list of the bands, where there are several and no list yet: only calls that copy C out band by band need it, and it is 8
+// bytes a row.  Waits for the device.  Stays empty when device memory is short; then everything is one band.
+int build_band_units(RowsFormat *f, bool tf32);
 void free_rows(RowsFormat *r);
 void free_narrow(NarrowFormat *f);
 

@@ -266,3 +266,33 @@ def test_tiles_of_consecutive_columns_read_b_in_boxes(dt, n):
         parity.check(dC.cpu().numpy(), 400, rp, ci, v, B)
     finally:
         plan.close()
+
+
+def test_the_list_of_the_bands_is_made_for_the_first_host_call():
+    # eight bytes a row that a plan of device products does not hold
+    import torch
+    from hopper_spmm_b200 import _capi as capi
+    rows, cols, n = 1 << 23, 1024, 8
+    ci = np.random.default_rng(3).integers(0, cols, rows).astype(np.uint32)
+    v = np.ones(rows, np.float16)
+    B = dense_b(cols, n, 3)
+    f = hs.DeviceBtcf(rows, cols, torch.arange(rows + 1, dtype=torch.int32, device="cuda"), torch.from_numpy(ci.view(np.int32)).cuda(), torch.from_numpy(v).cuda())
+    plan = hs.SpmmPlan(f)
+    try:
+        want = plan.spmm(torch.from_numpy(B).cuda(), c_half=True).cpu().numpy()
+        assert plan.launch_info().stages == 0 and np.array_equal(want, B[ci])
+
+        def free():
+            assert capi.lib().b200spmm_release_cached_memory(0) == 0
+            return torch.cuda.mem_get_info()[0]
+
+        before = free()
+        assert np.array_equal(plan.spmm_host(B, c_half=True), want)
+        assert plan.launch_info().kernel_launches > 2  # bands
+        taken = before - free()
+        assert taken >= rows * n * 2 + rows * 6  # C, and most of the list
+        assert np.array_equal(plan.spmm_host(B, c_half=True), want)
+        assert before - free() == taken
+    finally:
+        plan.close()
+        f.close()
