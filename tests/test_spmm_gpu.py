@@ -529,3 +529,22 @@ def test_the_result_is_made_where_torch_looks_for_it(c_half):
             assert torch.equal(plan.spmm(B, c_half=c_half), first)
     finally:
         plan.close()
+
+
+def test_a_profiler_lists_the_allocation_of_the_result():
+    # an observer of calls is no mode: it hears of what goes through the dispatcher, and the result does while one listens
+    import torch
+    rows, cols, rp, ci, v = random_csr(64, 40, 0.2, 3)
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    try:
+        B = torch.from_numpy(dense_b(cols, 24, 1)).cuda()
+        want = plan.spmm(B)
+        with torch.autograd.profiler.profile() as prof:
+            got = plan.spmm(B)
+        assert [e.key for e in prof.key_averages() if e.key == "aten::empty"]
+        assert torch.equal(got, want)
+        torch.use_deterministic_algorithms(True)
+        assert torch.equal(plan.spmm(B), want)
+    finally:
+        torch.use_deterministic_algorithms(False)
+        plan.close()
