@@ -683,7 +683,7 @@ struct TallLaunch {
     uint32_t parts;
 };
 constexpr uint64_t kOneLaunchTiles = 20000;
-constexpr double kTallMaxSums = 128e6;  // bytes
+constexpr double kTallMaxSums = 128e6;  // bytes of scratch that a plan may keep for them
 double short_micros(const b200spmm_plan *p, int64_t n) {  // (tiles over 148 SMs)
     return 14.0 + (double)p->info.total_tiles * (148.0 / p->n_sms) * (n <= 64 ? 0.28e-3 : 0.4e-3 * (double)((n + 127) / 128));
 }

@@ -5,10 +5,10 @@
 //   2. per (window, row): running sums over the window's runs -> row lengths, and how many units there are of every length;
 //      one scan over the rows -> the units, slots and bands.  The longest come first, so the lengths alone say where every
 //      unit of a length lies and where its batches do: the host's one wait
-//   3. every row puts its units into the list
+//   3. every row puts its units into the list (build_band_units makes the one with the bands apart, CUB radix sort, four key bits)
 //   4. the warps of step 1 write (column, value) to the place of their row's unit
 // Eight launches and one wait before the last.  With the units sorted (CUB), three scans and a launch for each small step there
-// were 26; the plan of a graph of 60,000 nodes and 700,000 entries took 232 us instead of 158, of 10,000 nodes 200 instead of 123.
+// were 26; the plan of a graph of 60,000 nodes and 700,000 entries took 232 us instead of 138, of 10,000 nodes 200 instead of 99.
 // A stored value is one whose bits are not all zero (an explicit zero adds nothing to a product), in a row and a column
 // of the matrix: the arrays may be a caller's, and what lies in a padded slot or below the last row multiplies nothing.
 #include <algorithm>

@@ -19,8 +19,9 @@
 // A work item is (super-window, feature slab, part of the window's tiles); items are numbered window-major, so the
 // CTAs that run at the same time work on the slabs of the same few windows and share their tiles in L2.  CTA b
 // starts with item b and claims further items from a global counter.  Where there are too few windows and slabs
-// for the SMs a window's tiles are cut into several parts (tall_launch in capi.cu has the rule); their sums go to
-// scratch and tall_sum_parts_kernel adds them up, always in the same order.
+// for the SMs, or a whole window's sums would be less exact than those of the 16-row kernel, a window's tiles are cut
+// into several parts (tall_launch in capi.cu has the rule); their sums go to scratch and tall_sum_parts_kernel adds
+// them up, always in the same order.
 //
 // Roles in a CTA of 416 threads, one CTA per SM:
 //   warps 0-7   epilogue: warp w drains TMEM lanes 32 (w % 4) .. +31 (32 window rows), columns half
@@ -594,8 +595,9 @@ spmm_tall_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
     }
 }
 
-// Adds the parts of the windows' rows up and writes them to C: four features a thread, the parts in order.  They lie in L2
-// (a launch has parts for one round of CTAs, 128 KB each).
+// Adds the parts of the windows' rows up and writes them to C: four features a thread, the parts in order.  Bound by reading
+// them: from L2 where they are parts for one round of CTAs (up to 128 KB each, 20 MB), in part from DRAM where sums that
+// have to be exact take several rounds (up to kTallMaxSums, 128 MB).
 __global__ void __launch_bounds__(256)
 tall_sum_parts_kernel(const float *partial, uint32_t parts, const uint32_t *__restrict__ rowIdx, uint32_t eff, uint32_t window_rows, void *C,
                       int64_t ldc, uint32_t rows, uint32_t n, uint32_t c_is_half) {

@@ -449,7 +449,8 @@ int b200spmm_spmm_noalloc_status(int device, void *stream);
  * is made when the plan is created (the merge must leave fewer than ~0.7 of the tiles, estimated on a
  * sample of windows; B200SPMM_WINDOW=16 or =128 in the environment overrides it) and per launch (the
  * expected time: rounds of windows x feature slabs against 16-row tiles spread evenly).  The format handed to
- * callers is unchanged.  b200spmm_plan_tall_info reports the merged format (row_window 128, or 0 when
+ * callers is unchanged.  A launch may share a window's tiles out in parts whose sums go to scratch of the plan, up to 128 MB
+ * of it, kept for the next launch.  b200spmm_plan_tall_info reports the merged format (row_window 128, or 0 when
  * the plan has none); b200spmm_plan_tall_copy_to_host copies its four arrays out (buffers sized from
  * that info) so that it can be compared with a conversion at 128 rows.  No counterpart in the
  * reference, which fixes ROW_WINDOW at 8 (src/common.h:17).
