@@ -366,7 +366,8 @@ int b200spmm_release_cached_memory(int device);
  * for both element types (the reference's tf32.cu has no kernel).
  * Rows of windows with no entries are written as zeros, so C needs no prior clearing.
  * The call may be captured into a CUDA graph, also as the plan's first one: the graph holds the kernels that the
- * call would run, and the plan must outlive it.  Scratch that a graph uses is kept until the plan is destroyed.
+ * call would run, and the plan must outlive it.  Scratch that a graph uses is kept until the plan is destroyed.  (One call
+ * has to come before the capture: rows of B 4 GiB apart or more, where the plan makes its tiles only then.)
  *   B, C 16-byte aligned; ldb*sizeof(b) and ldc*sizeof(c) multiples of 16; n a multiple of 8.
  */
 int b200spmm_spmm(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc,

@@ -203,7 +203,8 @@ def test_fewer_windows_than_sms_take_the_kernel_expected_to_be_faster(dt, n, win
 
 
 @pytest.mark.parametrize("dt,rows,n,window", [(np.float16, 1300, 72, 128), (np.float16, 1800, 128, 128), (np.float16, 1800, 328, 256),
-                                              (np.float32, 1300, 104, 128), (np.float32, 1800, 264, 256)])
+                                              (np.float32, 1300, 104, 128), (np.float32, 1800, 264, 256),
+                                              (np.float16, 1300, 40, 128), (np.float16, 1300, 64, 128), (np.float32, 1300, 24, 128)])
 def test_few_windows_are_cut_into_parts(dt, rows, n, window):
     # fewer windows than SMs or pairs, of unequal length and one gap: their tiles are shared out and the sums added up by a
     # launch of their own; every row written, nothing beside them, same bits again, in fp16 the rounded sums; in a graph
