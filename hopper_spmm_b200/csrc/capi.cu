@@ -21,6 +21,7 @@
 #include "spmm_pair_kernel.cuh"
 #include "spmm_rows_kernel.cuh"
 #include "spmm_tall_kernel.cuh"
+#include "spmm_window_kernel.cuh"
 #include "tall_gpu.hpp"
 #include "tensormap.hpp"
 
@@ -119,6 +120,9 @@ struct b200spmm_plan {
     Scratch b_packed;
     Scratch partial;  // fp32: pieces of windows or rows that are computed in parts, parts of super-windows
     std::vector<void *> outgrown;
+    // The kernel of single warps may take launches (windows_fit), or has to (windows_forced: B200SPMM_WINDOW=warps).
+    uint32_t max_short_tiles = 0;  // of a 16-row window
+    bool windows_fit = false, windows_forced = false;
     int n_sms = 0;
     // The tiles as the kernel's shared-memory image (spmm_kernel.cuh, SpmmParams::tiles_image): the plan's own
     // array swizzled in place when it owns the format, a swizzled copy when the arrays are the caller's.
@@ -636,6 +640,46 @@ int launch_rows(b200spmm_plan *p, const void *d_B, int64_t ldb, int64_t n, void 
                             from.split, to.split, stream);
 }
 
+// ---- windows of single warps
+int launch_windows(b200spmm_plan *p, uint32_t lines, const void *d_B, int64_t ldb, int64_t n, void *d_C, int64_t ldc, int c_dtype,
+                   cudaStream_t stream) {
+    const bool tf32 = p->info.dtype == B200SPMM_TF32;
+    WindowParams prm{};
+    prm.rowOffset = p->d_rowOffset;
+    prm.tcA2B = p->d_tcA2B;
+    prm.rowIdx = p->d_rowIdx;
+    prm.swizzled = p->d_tiles_image != nullptr;
+    prm.tiles = static_cast<const uint8_t *>(p->d_tiles_image ? p->d_tiles_image : p->d_data);
+    prm.B = d_B;
+    prm.C = d_C;
+    prm.ldc = ldc;
+    prm.pitch = (uint32_t)(ldb * p->info.elt_size);
+    prm.rows = (uint32_t)p->info.rows;
+    prm.cols = (uint32_t)p->info.cols;
+    prm.n = (uint32_t)n;
+    prm.eff = (uint32_t)p->info.eff_row_windows;
+    const uint32_t line = 128u / (uint32_t)p->info.elt_size;
+    prm.lines = (prm.n + line - 1) / line;
+    prm.c_is_half = c_dtype == B200SPMM_C_F16;
+    using Kernel = void (*)(const WindowParams);
+    static constexpr Kernel kernels[2][kWindowMaxLines] = {{spmm_window_kernel<false, 1>, spmm_window_kernel<false, 2>},
+                                                           {spmm_window_kernel<true, 1>, spmm_window_kernel<true, 2>}};
+    constexpr uint32_t threads = kWindowWarps * 32, smem = kWindowWarps * kWindowStages * kWindowStageBytes;
+    static_assert(smem <= 48 * 1024, "needs no attribute");
+    const uint32_t groups = (prm.lines + lines - 1) / lines;
+    const uint64_t blocks = ((uint64_t)prm.eff * groups + kWindowWarps - 1) / kWindowWarps;
+    B200_CUDA_TRY(launch_after(kernels[tf32][lines - 1], dim3((unsigned)blocks), threads, smem, 1, stream, prm));
+    p->last.n_ctas = (int)blocks;
+    p->last.threads = (int)threads;
+    p->last.stages = (int)kWindowStages;
+    p->last.feature_slab = (int)(line * lines);
+    p->last.n_slabs = (int)groups;
+    p->last.smem_bytes = (int64_t)smem;
+    p->last.kernel_launches = 1;
+    p->last.row_window = kRowWindow;
+    return B200SPMM_OK;
+}
+
 // ---- narrow B
 template <bool kTf32>
 int launch_narrow_vecs(const NarrowParams &prm, int vecs, unsigned n_ctas, size_t smem, cudaStream_t stream) {
@@ -770,6 +814,50 @@ TallChoice choose_tall(const b200spmm_plan *p, int64_t n) {
         c.packed_bytes = features * 32u * (size_t)((p->info.cols + p->info.col_window - 1) / p->info.col_window);
     }
     return c;
+}
+
+// Lines of 128 bytes that a warp of the kernel of single warps (spmm_window_kernel.cuh) multiplies, or 0 where the pipelined
+// 16-row kernel is expected to be faster, or would cut windows into pieces: here they are whole, and their sums have its bits.
+//
+// The estimates are least-squares fits to forced launches of block, uniform and pruned matrices of the ranges that the
+// benchmark draws, 8 to 2,000 columns (1,143 here, 15 % rms; 62 of the pipelined kernel on blocks, 7 %).  Here: a start, a step
+// for every stage of a long window, the copies of all tiles, and the warps to start.  There: a start, and per pass of 128
+// features a start of its own, the tiles and what it costs to hand a window over.  Us, pipelined / here, operands in L2:
+// blocks, tf32, 16384^2 at 0.5 %, 256 columns 16.2 / 13.0 (matrices in turn, from DRAM: 16.8 / 15.7); 13040 x 2960 at 0.9 %, 504
+// columns 15.5 / 11.2, 128 columns 7.3 / 4.9; 1648 x 5712 at 0.8 %, 512 columns 10.2 / 4.7; 1088 x 14304 at 0.3 %, 96 columns
+// 6.3 / 3.7; fp16, 16384^2 at 0.5 %, 64 columns 8.4 / 5.0, 256 columns 13.3 / 8.2.  Long windows stay: 1024^2 pruned to 10 %,
+// fp16, 64 columns 9.4 / 24.
+struct WindowCost {
+    double start, step, tile, warp;  // us; of a stage, of 1,000 tiles x groups of lines, of 1,000 warps
+};
+struct PipelinedCost {
+    double start, pass, tile, window;  // us; of 1,000 tiles and of 1,000 windows in a pass
+};
+constexpr WindowCost kWindowCost[2][kWindowMaxLines] = {{{2.4, 0.34, 0.174, 1.08}, {2.7, 0.33, 0.258, 1.61}}, {{1.8, 0.49, 0.085, 0.83}, {2.2, 0.345, 0.137, 1.02}}};
+constexpr PipelinedCost kPipelinedCost[2] = {{4.3, 1.71, 0.40, 0.17}, {4.9, 1.08, 0.36, 0.62}};
+uint32_t choose_window_lines(const b200spmm_plan *p, int64_t ldb, int64_t n) {
+    const bool tf32 = p->info.dtype == B200SPMM_TF32;
+    const uint64_t eff = p->info.eff_row_windows;
+    const uint32_t line = 128u / (uint32_t)p->info.elt_size, n_lines = (uint32_t)((n + line - 1) / line);
+    if (!p->windows_fit || (uint64_t)ldb * p->info.elt_size > 0xFFFFFFFFull || eff * n_lines > 0x7FFFFFFFull) return 0;  // 32-bit row pitch, grid
+    const double tiles = (double)p->info.total_tiles, scale = 1e-3 * (148.0 / p->n_sms);
+    double least = 1e30;
+    if (!p->windows_forced) {
+        const PipelinedCost &c = kPipelinedCost[tf32];
+        least = c.start + (double)((n + 127) / 128) * (c.pass + (c.tile * tiles + c.window * (double)eff) * scale);
+    }
+    const uint32_t longest = (uint32_t)((tiles / (double)eff + p->max_short_tiles) / 2);  // (of ten tiles on average: two standard deviations above)
+    uint32_t best = 0;
+    for (uint32_t lines = 1; lines <= kWindowMaxLines && lines <= n_lines; ++lines) {
+        const WindowCost &c = kWindowCost[tf32][lines - 1];
+        const uint32_t stage = kWindowStageBytes / (128u * (uint32_t)p->info.col_window * lines), steps = (longest + stage - 1) / stage;
+        const double micros = c.start + c.step * steps + (c.tile * tiles + c.warp * (double)eff) * scale * (double)((n_lines + lines - 1) / lines);
+        if (micros < least) {
+            least = micros;
+            best = lines;
+        }
+    }
+    return best;
 }
 
 // Column blocks per group for B of width n: as many as fit shared memory, 0 if the kernel does not take it.  Every
@@ -1050,6 +1138,12 @@ int plan_build_tile_path(b200spmm_plan *p, const uint32_t *h_rowOffset, const ui
         if (st != B200SPMM_OK) return st;
     }
     p->has_tile_path = true;
+    // An explicit CTA count, window height, form of the tiles or way to fetch rows asks for the pipelined kernels.  (A warp
+    // clears the rows of all windows that are missing behind its own.)
+    p->windows_forced = env_is("B200SPMM_WINDOW", "warps");
+    p->windows_fit = n_ctas <= 0 && !p->loose_lists && !p->gather_cpasync && !std::getenv("B200SPMM_TILES") &&
+                     (p->windows_forced || (!std::getenv("B200SPMM_WINDOW") && !p->sched.n_splits && info.total_row_windows <= 16 * info.eff_row_windows));
+    for (uint64_t w = 0; w < info.eff_row_windows; ++w) p->max_short_tiles = std::max(p->max_short_tiles, h_rowOffset[w + 1] - h_rowOffset[w]);
     return plan_build_tile_image(p);
 }
 
@@ -1605,8 +1699,10 @@ int spmm_launch(b200spmm_plan_t *p, const void *d_B, int64_t ldb, int64_t n, voi
         int st = plan_add_tile_path(p, 0);
         if (st != B200SPMM_OK) return st;
     }
-    note_bounded_waits(p, stream);
     TallChoice tall = band < 0 ? choose_tall(p, n) : TallChoice{};
+    if (const uint32_t lines = tall.use || band >= 0 || p->starve_gathers ? 0u : choose_window_lines(p, ldb, n))
+        return launch_windows(p, lines, d_B, ldb, n, d_C, ldc, c_dtype, stream);
+    note_bounded_waits(p, stream);
     if (tall.parts > 1 && tall.use && take_scratch(p, &p->partial, tall.partial_bytes, stream) != B200SPMM_OK) {
         // no room for the parts' sums: whole windows where they are as exact, else the 16-row kernel
         tall.use = tall.least_parts <= 1;
