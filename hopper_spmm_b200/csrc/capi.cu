@@ -16,6 +16,7 @@
 #include "device_pool.hpp"
 #include "format.hpp"
 #include "handles.hpp"
+#include "sparse24_gpu.hpp"
 #include "spmm_kernel.cuh"
 #include "spmm_narrow_kernel.cuh"
 #include "spmm_pair_kernel.cuh"
@@ -92,6 +93,7 @@ struct b200spmm_plan {
     // ... and in 256-row super-windows for the CTA-pair kernel (spmm_pair_kernel.cuh), which takes the
     // launches wider than 128 features when doubling the window height again halves the tile count.
     TallFormat pair;
+    Sparse24Format sparse;     // the same windows in the tensor core's 2:4 form (fp16), or empty
     int pair_clusters = 0;     // two-CTA clusters of that kernel the GPU runs at the same time
     // ... and as row units for the kernel that loads rows of B entry by entry (spmm_rows_kernel.cuh).  A matrix
     // whose tiles are nearly empty keeps nothing else (rows_only).
@@ -480,10 +482,10 @@ int launch_tall_one(b200spmm_plan *p, TallParams &prm, cudaStream_t stream) {
     return B200SPMM_OK;
 }
 
-template <bool kTf32>
+template <bool kTf32, bool kSparse>
 int launch_pair_one(b200spmm_plan *p, TallParams &prm, cudaStream_t stream) {
-    using Cfg = PairCfg<kTf32>;
-    auto kernel = spmm_pair_kernel<kTf32>;
+    using Cfg = PairCfg<kTf32, kSparse>;
+    auto kernel = spmm_pair_kernel<kTf32, kSparse>;
     prm.n_slabs = (prm.n + Cfg::kNs - 1) / Cfg::kNs;
     prm.n_items = prm.eff_row_windows * prm.n_slabs * prm.parts;
     const int n_pairs = (int)std::min<uint32_t>(prm.n_items, (uint32_t)p->pair_clusters);
@@ -502,10 +504,10 @@ int launch_pair_one(b200spmm_plan *p, TallParams &prm, cudaStream_t stream) {
 }
 
 // How many two-CTA clusters of the pair kernel the device runs at once (0: it cannot run it).
-template <bool kTf32>
+template <bool kTf32, bool kSparse = false>
 int pair_max_clusters(int *out) {
-    using Cfg = PairCfg<kTf32>;
-    auto kernel = spmm_pair_kernel<kTf32>;
+    using Cfg = PairCfg<kTf32, kSparse>;
+    auto kernel = spmm_pair_kernel<kTf32, kSparse>;
     B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmemBytes));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(2 * 148);
@@ -540,6 +542,7 @@ constexpr uint64_t kRowsWideMinTiles = 592, kRowsWideAnyTiles = 16384;  // (belo
 // 256 rows from the second number on: in parts the two heights take the same (1682 x 1536 at 11 %, 8,614 tiles, 816 columns
 // 21.5 and 22.5 us), and the plan takes 50 us less with one of them.
 constexpr uint64_t kTallMinShortTiles = 2048, kPairMinShortTiles = 16384;
+constexpr uint64_t kSparse24MinTiles = 20000;  // of 256 rows
 constexpr uint64_t kTallMaxCounted = 1 << 25, kTallMaxCountedCols = 393216;  // entries of lists; columns of one bit set
 
 bool use_rows(const b200spmm_plan *p, int64_t ldb) {
@@ -779,7 +782,7 @@ TallLaunch tall_launch(const b200spmm_plan *p, const TallFormat &f, int64_t n, u
 // Whether a launch goes to the super-window kernels, how, and what it needs of the plan's scratch.  Worked out once a launch.
 // Only with the TMA gathers, and - unless forced, for B at least one 128-byte box wide - only when it is expected to be faster.
 struct TallChoice {
-    bool use, pair;
+    bool use, pair, sparse;  // sparse: the pair kernel on 2:4 tiles
     uint32_t parts, least_parts;  // with fewer than the second the sums would be less exact than those of 16 rows
     size_t partial_bytes, packed_bytes;
 };
@@ -806,12 +809,15 @@ TallChoice choose_tall(const b200spmm_plan *p, int64_t n) {
         c.parts = l.parts;
     }
     const TallFormat &f = c.pair ? p->pair : p->tall;
+    // (2:4 windows in parts: 4096^2 at 10 %, 256 columns 24.8 us with dense tiles, 30.4 so)
+    c.sparse = c.pair && p->sparse.tiles && c.parts == 1;
     if (c.parts > 1) c.partial_bytes = (size_t)c.parts * (size_t)f.eff * f.rows * (size_t)n * 4;  // kTallMaxSums
     if (p->tall_pack_b) {
         // the pair kernel's CTAs fetch 128-feature halves of a 256-feature slab: both halves of the last slab must
         // exist in the packed copy (as zeros past n), so an even number of 128-feature blocks
         const size_t features = c.pair || n > 128 ? (size_t)(n + 255) / 256 * 256 : 128;
-        c.packed_bytes = features * 32u * (size_t)((p->info.cols + p->info.col_window - 1) / p->info.col_window);
+        const size_t group = c.sparse ? 32 : (size_t)p->info.col_window;  // rows of B
+        c.packed_bytes = features * (size_t)p->info.elt_size * group * (((size_t)p->info.cols + group - 1) / group);
     }
     return c;
 }
@@ -934,16 +940,27 @@ int launch_tall(b200spmm_plan *p, const TallChoice &choice, const void *d_B, int
     prm.tcA2B = fmt.d_tcA2B;
     prm.rowIdx = fmt.d_rowIdx;
     prm.data = static_cast<const uint8_t *>(fmt.d_data);
+    if (choice.sparse) {
+        prm.rowOffset = p->sparse.d_rowOffset;
+        prm.tcA2B = p->sparse.d_tcA2B;
+        prm.data = static_cast<const uint8_t *>(p->sparse.d_data);
+        prm.meta = static_cast<const uint8_t *>(p->sparse.d_meta);
+        prm.quads = p->sparse.d_quads;
+        prm.n_rest = p->sparse.d_n_rest;
+        prm.rest = p->sparse.d_rest;
+        prm.B = static_cast<const uint8_t *>(d_B);
+        prm.ldb_bytes = (uint64_t)ldb * 2u;
+    }
     if (p->tall_pack_b) {
-        const uint32_t cw = (uint32_t)p->info.col_window, esz = (uint32_t)p->info.elt_size;
+        const uint32_t cw = choice.sparse ? 32u : (uint32_t)p->info.col_window, esz = (uint32_t)p->info.elt_size;
         const uint32_t slab = (n <= 128 || pair) ? 128u : 256u;
         const uint32_t n_slabs = pair ? 2u * (uint32_t)((n + 255) / 256) : (uint32_t)((n + slab - 1) / slab);
         const uint32_t groups = (uint32_t)((p->info.cols + cw - 1) / cw);
-        const size_t need = choice.packed_bytes;  // n_slabs * groups * 32 * slab
+        const size_t need = choice.packed_bytes;  // n_slabs * groups * cw * esz * slab
         st = take_scratch(p, &p->b_packed, need, stream);
         if (st != B200SPMM_OK) return st;
         const int grid = (int)std::min<size_t>((need / 16 + 255) / 256, (size_t)p->n_sms * 16);
-        B200_CUDA_TRY(launch_after(tf32 ? pack_b_kernel<true> : pack_b_kernel<false>, dim3(grid), 256, 0, 1, stream, static_cast<const uint8_t *>(d_B),
+        B200_CUDA_TRY(launch_after(tf32 ? pack_b_kernel<true> : choice.sparse ? pack_b_kernel<false, 32> : pack_b_kernel<false>, dim3(grid), 256, 0, 1, stream, static_cast<const uint8_t *>(d_B),
                                    ldb * esz, (uint32_t)p->info.cols, (uint32_t)n, slab, n_slabs, groups, static_cast<uint8_t *>(p->b_packed.ptr)));
         prm.b_packed = static_cast<const uint8_t *>(p->b_packed.ptr);
         prm.b_groups = groups;
@@ -968,7 +985,7 @@ int launch_tall(b200spmm_plan *p, const TallChoice &choice, const void *d_B, int
     cudaMemsetAsync(g_prof, 0, 1024 * 32 * 8, stream);
     prm.prof = g_prof;
 #endif
-    if (pair) st = tf32 ? launch_pair_one<true>(p, prm, stream) : launch_pair_one<false>(p, prm, stream);
+    if (pair) st = tf32 ? launch_pair_one<true, false>(p, prm, stream) : choice.sparse ? launch_pair_one<false, true>(p, prm, stream) : launch_pair_one<false, false>(p, prm, stream);
     else if (n <= 128) st = tf32 ? launch_tall_one<true, 128>(p, prm, stream) : launch_tall_one<false, 128>(p, prm, stream);
     else st = tf32 ? launch_tall_one<true, 256>(p, prm, stream) : launch_tall_one<false, 256>(p, prm, stream);
     if (st != B200SPMM_OK || prm.parts == 1) return st;
@@ -1026,7 +1043,18 @@ int plan_build_tall(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_
     }
     uint32_t aligned = 0;
     B200_CUDA_TRY(cudaMemcpy(&aligned, p->tall.d_aligned, 4, cudaMemcpyDeviceToHost));
-    p->tall_pack_b = (uint64_t)aligned * 2 >= p->tall.tiles && !env_is("B200SPMM_PACK_B", "0");
+    const bool most_aligned = (uint64_t)aligned * 2 >= p->tall.tiles;
+    p->tall_pack_b = most_aligned && !env_is("B200SPMM_PACK_B", "0");
+    // The windows once more in 2:4 form, where most of their lists name neighbouring rows of B (the kernel has no room for gathers
+    // in every stage).  It takes 0.5 to 1 ms to make, which a small matrix does not get back: 14336 x 4096 at 8 % (14,336 tiles) 39.5 ->
+    // 31.3 us a product of 256 columns, plan 0.8 -> 1.3 ms.  B200SPMM_SPARSE24=0 keeps it out, =1 asks for it wherever it fits.
+    const bool always = env_is("B200SPMM_SPARSE24", "1");
+    if (p->pair.tiles && most_aligned && info.dtype == B200SPMM_F16 && (always || p->pair.tiles >= kSparse24MinTiles) && !env_is("B200SPMM_SPARSE24", "0")) {
+        int clusters = 0;
+        st = pair_max_clusters<false, true>(&clusters);
+        if (st == B200SPMM_OK && clusters >= p->pair_clusters) st = build_sparse24(p->pair, info.cols, always, &p->sparse);
+        if (st != B200SPMM_OK) return st;
+    }
     B200_CUDA_TRY(cudaDeviceSynchronize());
     return B200SPMM_OK;
 }
@@ -1484,6 +1512,7 @@ void b200spmm_plan_destroy(b200spmm_plan_t *p) {
     pool_free(p->d_tile_entries);
     free_tall(&p->tall);
     free_tall(&p->pair);
+    free_sparse24(&p->sparse);
     pool_free(p->b_packed.ptr);
     pool_free(p->partial.ptr);
     for (void *old : p->outgrown) pool_free(old);

@@ -39,6 +39,12 @@ B200_DEVICE uint4 ld_global_v4(const void *p) {
     return v;
 }
 
+// 32 bytes, 32-byte aligned.
+B200_DEVICE void ld_global_v8(const void *p, uint32_t *v) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "l"(p) : "memory");
+}
+
 // A load of a stream that nothing writes: what is not in L2 comes with the 256 bytes around it, the next of the stream.  (The
 // entries of row units, of which a lane group has one batch under way: 300,000 nodes, 64 / 128 features 77.6 / 141 -> 73.4 / 136
 // us, 2^20 nodes, 64 features 230 -> 220; an instruction of its own that fetches ahead costs 5 to 20 % instead.)
@@ -226,6 +232,18 @@ B200_DEVICE void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)[32]) {
         : "r"(taddr)
         : "memory");
 }
+// The other way: thread i's 32 words to lane taddr.lane + i.
+B200_DEVICE void tmem_st_32x32b_x32(uint32_t taddr, const float (&r)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+        ::"r"(taddr), "f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3]), "f"(r[4]), "f"(r[5]), "f"(r[6]), "f"(r[7]), "f"(r[8]), "f"(r[9]),
+          "f"(r[10]), "f"(r[11]), "f"(r[12]), "f"(r[13]), "f"(r[14]), "f"(r[15]), "f"(r[16]), "f"(r[17]), "f"(r[18]), "f"(r[19]),
+          "f"(r[20]), "f"(r[21]), "f"(r[22]), "f"(r[23]), "f"(r[24]), "f"(r[25]), "f"(r[26]), "f"(r[27]), "f"(r[28]), "f"(r[29]),
+          "f"(r[30]), "f"(r[31])
+        : "memory");
+}
+B200_DEVICE void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 B200_DEVICE void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // ------------------------------------------------------------------ CTA pairs (cta_group::2)
@@ -280,6 +298,22 @@ B200_DEVICE void umma_pair_ss_lohi_if(bool tf32, uint32_t on, uint32_t d_tmem, u
             "setp.ne.b32 p, %6, 0;\nsetp.ne.b32 q, %7, 0;\n"
             "@q tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n}\n"
             ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(on) : "memory");
+}
+// The same with a 2:4 sparse A: K is twice as large, and tensor memory column `meta` (an even one; the descriptor's lowest bit
+// adds one) says in both CTAs which two of four columns A's values belong to.
+enum : uint32_t { kSparseA = 1u << 2 };  // of the instruction descriptor
+B200_DEVICE void umma_pair_sparse_f16_if(uint32_t on, uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t meta,
+                                         uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p, q;\n.reg .b64 da, db;\nmov.b64 da, {%1, %2};\nmov.b64 db, {%3, %4};\n"
+        "setp.ne.b32 p, %7, 0;\nsetp.ne.b32 q, %8, 0;\n"
+        "@q tcgen05.mma.sp.cta_group::2.kind::f16 [%0], da, db, [%5], %6, p;\n}\n"
+        ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(meta), "r"(idesc), "r"(accumulate), "r"(on) : "memory");
+}
+// 128 lanes x 16 bytes from shared memory (core matrices of eight lanes) to four columns of tensor memory, in both CTAs; runs in
+// order with the MMAs that the thread issues.
+B200_DEVICE void tmem_copy_pair_128x128b(uint32_t taddr, uint64_t smem_desc) {
+    asm volatile("tcgen05.cp.cta_group::2.128x128b [%0], %1;" ::"r"(taddr), "l"(smem_desc) : "memory");
 }
 // One arrival on the barrier at offset `bar` in BOTH CTAs of the pair (mask 0b11) when every MMA this
 // thread issued so far has finished.

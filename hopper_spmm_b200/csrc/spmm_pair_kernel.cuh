@@ -19,10 +19,20 @@
 //               barriers); odd CTA: lane 0 forwards "my part of stage s has landed" to the even CTA's
 //               full barrier.  The warp owns the TMEM allocation (made by both CTAs together).
 //   warps 9-12  producers, as in the 128-row kernel, for this CTA's half of A and of B
+//
+// kSparse: tiles in the tensor core's 2:4 form (sparse24_gpu.hpp), 256 rows x 32 columns for the time and the bytes of A of a dense
+// tile of 16.  A stage brings 2 KB of metadata with its four tiles; the issuing thread copies it to four columns of tensor
+// memory (tcgen05.cp, which runs in order with the MMAs that follow), so there is one accumulator and an item's epilogue is not hidden
+// behind the next item's MMAs.  What rows have beyond two entries in a group of four is multiplied by the epilogue warps meanwhile.
+// Bound: L2 -> SM, 12.5 KB a tile step of 32 columns where dense tiles take 16 (52 bytes a clock and SM; two of its 240 clocks in
+// three are tensor-pipe clocks), and power.  28672 x 8192 at 10 %, us, dense and so: 192 columns, half results 118 and 95, 2,048
+// columns 788 and 672; without the rest 88 and 619.  Listing the rest's columns again as tiles instead was tried (18 % more tiles, any
+// column of B): with gathers 105 and 751, four warps issuing; with cp.async 119 and 784.
 // Every wait is bounded; both CTAs meet at a cluster barrier before either lets go of its shared or
 // tensor memory.
 #pragma once
 
+#include "sparse24_gpu.hpp"
 #include "spmm_tall_kernel.cuh"
 
 namespace b200spmm {
@@ -32,16 +42,20 @@ constexpr int kPairRows = 256;  // rows of a super-window of the pair kernel
 // TallParams as for the 128-row kernel, with: rowIdx a multiple of 256; data = per window the tiles of
 // the even CTA (rows 0-127, 4 KB images) followed by the tiles of the odd CTA (rows 128-255); b_packed
 // packed for 128-feature slabs (slab 2 S + r is CTA r's half of item slab S); n_slabs = ceil(n / 256).
-template <bool kTf32>
+template <bool kTf32, bool kSparse = false>
 struct PairCfg {
+    static_assert(!kSparse || !kTf32, "2:4 tiles hold fp16");
     static constexpr int kNs = 256;                         // features of an item
     static constexpr int kNc = 128;                         // ... of which one CTA fetches
-    static constexpr int kCW = kTf32 ? 8 : 16;
+    static constexpr int kCW = kSparse ? 32 : kTf32 ? 8 : 16;  // columns of a tile
     static constexpr int kEsz = kTf32 ? 4 : 2;
     static constexpr int kTps = kTallStageTiles;                          // tiles per ring stage (6 and 8 were slower: 711 / 729 us against 678)
-    static constexpr int kGatherBytes = 32 * kNc;           // CW rows x 128 features
-    static constexpr int kStageBytes = kTps * (kGatherBytes + kTallTileBytes);
-    static constexpr int kStages = 24 / kTps;               // 192 KB of operands in flight per CTA
+    static constexpr int kGatherBytes = kCW * kEsz * kNc;   // CW rows x 128 features
+    static constexpr int kMetaBytes = kSparse ? 2048 : 0;   // of a stage: four words for each of 128 lanes
+    static constexpr int kStageBytes = kTps * (kGatherBytes + kTallTileBytes) + kMetaBytes;
+    static constexpr int kStages = kSparse ? 4 : 24 / kTps;  // about 200 KB of operands in flight per CTA
+    static constexpr int kAccs = kSparse ? 1 : 2;           // accumulators of 256 columns of tensor memory
+    static constexpr uint32_t kMetaCols = kNs;              // the metadata of stage s lies behind the one accumulator, in columns + 4 s ..
     static constexpr int kProducerWarps = kStages < 4 ? kStages : 4;
     static constexpr int kEpilogueWarps = 8;
     static constexpr int kMmaWarp = 8;
@@ -51,7 +65,9 @@ struct PairCfg {
     static constexpr int kRowQuads = kCW / 4;
     static constexpr int kBoxes = kNc / kBoxFeatures;       // 128-byte column blocks of a CTA's half slab
     static constexpr int kGatherOps = kRowQuads * kBoxes;   // gather4 instructions per tile: 8
-    static constexpr int kBoxBytes = kCW * 128;
+    static constexpr int kBoxRows = kTf32 ? 8 : 16;         // of the tensor map for neighbouring rows
+    static constexpr int kBoxesPerBlock = kCW / kBoxRows;   // boxes of a tile one above the other
+    static constexpr int kBoxBytes = kBoxRows * 128;
     static_assert(kGatherOps <= 16 && kTps % 2 == 0 && kProducerWarps <= kStages, "see the 128-row kernel");
     static constexpr int kIdxSlots = 4;
     static constexpr int kIdxAhead = kIdxSlots - 1;
@@ -59,16 +75,67 @@ struct PairCfg {
     static constexpr int kIdxBytes = kProducerWarps * kIdxSlots * kSlotBytes;
     static constexpr int kBarriers = 2 * kStages + 5;       // full, empty, 2 x acc_full, 2 x acc_empty, drain
     static constexpr int kItemSlots = 64;
-    static constexpr uint32_t kTmemCols = 2 * kNs;          // two accumulators of 256 columns in each CTA
+    static constexpr uint32_t kTmemCols = 2 * kNs;          // two accumulators of 256 columns in each CTA, or one and metadata
     static constexpr size_t kSmemBytes =
         1024 + (size_t)kStages * kStageBytes + kIdxBytes + kBarriers * 8 + 16 + kItemSlots * 4 + 8;
+    static_assert(kSmemBytes <= 227 * 1024, "shared memory of a CTA");
 };
 
-template <bool kTf32>
-__global__ void __launch_bounds__((PairCfg<kTf32>::kThreads), 1)
+// sum[k] = the products of a row's rest with features feat0 + k of B, 32 of them, in fp32.  Every lane has a row of its own and reads
+// 64 bytes of other rows of B at a time, so the loads are as wide as they get; two entries ahead are as fast as three.
+B200_DEVICE void pair_sum_rest(const TallParams &p, const uint32_t *entries, uint32_t n, uint32_t feat0, float (&sum)[32]) {
+#pragma unroll
+    for (int k = 0; k < 32; ++k) sum[k] = 0.f;
+    if (feat0 >= p.n) return;
+    const uint32_t here = min(32u, p.n - feat0);  // a multiple of 8
+    const uint8_t *B = p.B + (uint64_t)feat0 * 2u;
+    const bool wide = here == 32u && ((reinterpret_cast<uintptr_t>(B) | p.ldb_bytes) & 31u) == 0;
+    auto add = [&](int at, uint32_t two, uint16_t a) {
+        asm("fma.rn.f32.f16 %0, %1, %2, %0;" : "+f"(sum[at]) : "h"(a), "h"((uint16_t)two));
+        asm("fma.rn.f32.f16 %0, %1, %2, %0;" : "+f"(sum[at + 1]) : "h"(a), "h"((uint16_t)(two >> 16)));
+    };
+    constexpr int kAhead = 2;  // entries whose rows of B are in flight
+    uint32_t next[kAhead];
+    auto fetch = [&](uint32_t i) {
+#pragma unroll
+        for (uint32_t k = 0; k < (uint32_t)kAhead; ++k) next[k] = i + k < n ? __ldg(entries + (uint64_t)(i + k) * kPairRows) : 0u;
+    };
+    fetch(0);
+    for (uint32_t i = 0; i < n; i += kAhead) {
+        uint32_t b[kAhead][16];
+        uint16_t a[kAhead];
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) {
+            const uint8_t *row = B + (uint64_t)(next[j] >> 16) * p.ldb_bytes;
+            a[j] = (uint16_t)next[j];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) b[j][k] = 0;
+            if (i + (uint32_t)j >= n) continue;
+            if (wide) {
+                ptx::ld_global_v8(row, b[j]);
+                ptx::ld_global_v8(row + 32, b[j] + 8);
+            } else {
+#pragma unroll
+                for (uint32_t v = 0; v < 4; ++v)
+                    if (v * 8u < here) {
+                        const uint4 x = ptx::ld_global_v4(row + v * 16u);
+                        b[j][4 * v] = x.x; b[j][4 * v + 1] = x.y; b[j][4 * v + 2] = x.z; b[j][4 * v + 3] = x.w;
+                    }
+            }
+        }
+        fetch(i + kAhead);
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j)
+#pragma unroll
+            for (int k = 0; k < 16; ++k) add(2 * k, b[j][k], a[j]);
+    }
+}
+
+template <bool kTf32, bool kSparse = false>
+__global__ void __launch_bounds__((PairCfg<kTf32, kSparse>::kThreads), 1)
 spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_bt,
                  const TallParams p) {
-    using Cfg = PairCfg<kTf32>;
+    using Cfg = PairCfg<kTf32, kSparse>;
     constexpr int kStages = Cfg::kStages;
     constexpr int kTps = Cfg::kTps;
     constexpr int kNs = Cfg::kNs;
@@ -82,7 +149,8 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
     const uint32_t gather_addr = raw_addr + pad;
     const uint32_t atile_addr = gather_addr + kStages * kTps * Cfg::kGatherBytes;
     uint32_t *idx_ring = reinterpret_cast<uint32_t *>(base + kStages * Cfg::kStageBytes);
-    const uint32_t idx_ring_addr = atile_addr + kStages * kTps * kTallTileBytes;
+    const uint32_t meta_addr = atile_addr + kStages * kTps * kTallTileBytes;
+    const uint32_t idx_ring_addr = meta_addr + kStages * Cfg::kMetaBytes;
     uint64_t *bars = reinterpret_cast<uint64_t *>(base + kStages * Cfg::kStageBytes + Cfg::kIdxBytes);
     const uint32_t bars_addr = idx_ring_addr + Cfg::kIdxBytes;
     auto full_bar = [&](uint32_t s) { return bars_addr + 8u * s; };
@@ -102,6 +170,10 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
     const uint64_t limit = p.wait_limit_ns;
     const uint32_t rank = ptx::cluster_cta_rank();  // 0: issues the MMAs and claims the items
     const uint32_t pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+
+    // round k uses accumulator k mod kAccs, for the (k / kAccs)-th time
+    auto acc_of = [](uint32_t round) { return Cfg::kAccs == 2 ? round & 1u : 0u; };
+    auto acc_phase = [](uint32_t round) { return (Cfg::kAccs == 2 ? round >> 1 : round) & 1u; };
 
     constexpr uint32_t kNoItem = 0xFFFFFFFFu;
     auto item_id = [&](uint32_t k) -> uint32_t {
@@ -165,9 +237,28 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
             const uint32_t w = t.w, slab = t.slab;
             const uint32_t row0 = p.rowIdx[w];
             const uint32_t gap_hi = w + 1 < p.eff_row_windows ? p.rowIdx[w + 1] : p.rows;
-            const uint32_t a = round & 1u;
+            const uint32_t a = acc_of(round);
+            // 2:4 tiles: this thread's row has a rest, entries that no tile holds.  Their products are summed while the tensor core
+            // works; three of the four 32-feature chunks wait in tensor memory, the last one in registers.
+            const uint32_t rest_cols = tmem_base + ((q * 32u) << 16) + Cfg::kMetaCols + 4u * kStages + hsel * 96u;
+            uint32_t most_rest = 0;
+            float rest[32] = {};
+            if constexpr (kSparse) {
+                const uint32_t in_window = rank * kTallRows + q * 32u + (uint32_t)lane;
+                const uint32_t n_rest = t.part == 0 ? p.n_rest[w * kPairRows + in_window] : 0u;
+                most_rest = __reduce_max_sync(0xffffffffu, n_rest);
+                const uint32_t *entries = p.rest + (uint64_t)w * (kSparse24MaxRest * kPairRows) + in_window;
+#pragma unroll 1
+                for (uint32_t c = 0; most_rest && c < kHalf / 32u; ++c) {
+                    const uint32_t feat0 = slab * kNs + hsel * kHalf + c * 32u;
+                    pair_sum_rest(p, entries, n_rest, feat0, rest);
+                    __syncwarp();
+                    if (c + 1 < kHalf / 32u) ptx::tmem_st_32x32b_x32(rest_cols + c * 32u, rest);
+                }
+                if (most_rest) ptx::tmem_st_wait();
+            }
             uint32_t ok = 1;
-            if (lane == 0) ok = ptx::mbar_wait(acc_full_bar(a), (round >> 1) & 1u, abort_flag, limit) ? 1u : 0u;
+            if (lane == 0) ok = ptx::mbar_wait(acc_full_bar(a), acc_phase(round), abort_flag, limit) ? 1u : 0u;
             ok = __shfl_sync(0xffffffffu, ok, 0);
             if (!ok) { epi_alive = false; break; }
             ptx::tcgen05_fence_after_sync();
@@ -185,6 +276,18 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
                     if (lane == 0) ptx::mbar_arrive_cluster(a ? leader_acc_empty1 : leader_acc_empty0);
                 }
                 const uint32_t feat0 = f_slab + col0;
+                if (kSparse && most_rest) {
+                    if (c + 1 < kHalf / 32u) {
+                        uint32_t v[32];
+                        ptx::tmem_ld_32x32b_x32(rest_cols + c * 32u, v);
+                        ptx::tmem_ld_wait();
+#pragma unroll
+                        for (int k = 0; k < 32; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) + __uint_as_float(v[k]));
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 32; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) + rest[k]);
+                    }
+                }
                 tall_store_row32(p, t.part, w * kPairRows + (row - row0), row, feat0, r);
             }
             // Rows of super-windows without entries are absent from the format: clear the gap after this
@@ -208,12 +311,13 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
         constexpr int kIdxLanes = Cfg::kCW * 4 / 16;
         const uint32_t g = hl % Cfg::kRowQuads, h = hl / Cfg::kRowQuads;
         const uint32_t op_quad = g, op_x = h * Cfg::kBoxFeatures;
-        const uint32_t op_dst = kTf32 ? (h * 2 + g) * 512u : (h * 2 + (g >> 1)) * 1024u + (g & 1u) * 512u;
+        const uint32_t op_dst = kTf32 ? (h * 2 + g) * 512u : (h * (Cfg::kCW / 8) + (g >> 1)) * 1024u + (g & 1u) * 512u;
         const uint32_t peer_list_addr = ptx::map_to_cta(item_list_addr, 1), peer_avail_addr = ptx::map_to_cta(item_avail_addr, 1);
 
         struct Cursor {
             uint32_t round, sp, tile_begin, n_tiles, stages, slab, done;
             uint64_t image;  // this CTA's first tile image of the item
+            uint64_t meta;   // ... and quad of metadata
         };
         uint32_t grabbed = 1;
         auto open_item = [&](Cursor &c) {
@@ -242,6 +346,10 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
             c.tile_begin = t0 + t.first;
             c.image = (uint64_t)t0 * 2u + (rank ? p.rowOffset[t.w + 1] - t0 : 0u) + t.first;
             c.stages = (c.n_tiles + kTps - 1) / kTps;
+            if constexpr (kSparse) {
+                const uint32_t q0 = p.quads[t.w];
+                c.meta = (uint64_t)q0 * 2u + (rank ? p.quads[t.w + 1] - q0 : 0u) + t.first / kTps;
+            }
         };
         auto normalise = [&](Cursor &c) {
             while (!c.done && c.sp >= c.stages) {
@@ -250,7 +358,7 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
                 open_item(c);
             }
         };
-        Cursor cur{0, pid, 0, 0, 0, 0, 0, 0};
+        Cursor cur{0, pid, 0, 0, 0, 0, 0, 0, 0};
         open_item(cur);
         normalise(cur);
         Cursor fc = cur;
@@ -297,7 +405,8 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
                     const uint32_t gather_bytes = (B200_DEBUG_BITS(p) & 1u) ? 0u : (uint32_t)Cfg::kGatherBytes;
                     const uint32_t tile_bytes = (B200_DEBUG_BITS(p) & 4u) ? 0u : (uint32_t)kTallTileBytes;
                     B200_PROF_T0();
-                    ptx::mbar_arrive_expect_tx(full_bar(s), here * (gather_bytes + tile_bytes) + p.starve_bytes);
+                    ptx::mbar_arrive_expect_tx(full_bar(s), here * (gather_bytes + tile_bytes) + Cfg::kMetaBytes + p.starve_bytes);
+                    if constexpr (kSparse) ptx::bulk_load(meta_addr + s * Cfg::kMetaBytes, p.meta + (cur.meta + cur.sp) * Cfg::kMetaBytes, Cfg::kMetaBytes, full_bar(s));
                     // this CTA's halves of the stage's tiles are neighbours in memory and in the ring: one copy
                     if (tile_bytes)
                         ptx::bulk_load(atile_addr + s * kTps * kTallTileBytes,
@@ -343,9 +452,9 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
                             if (hl == 0)
                                 ptx::bulk_load(dst, p.b_packed + ((uint64_t)my_slab * p.b_groups + first / (uint32_t)Cfg::kCW) * Cfg::kGatherBytes,
                                                (uint32_t)Cfg::kGatherBytes, full_bar(s));
-                        } else if (hl < (uint32_t)Cfg::kBoxes)
-                            ptx::tma_load_2d(dst + hl * Cfg::kBoxBytes, &tmap_bt, (int32_t)(my_slab * Cfg::kNc + hl * Cfg::kBoxFeatures),
-                                             (int32_t)first, full_bar(s));
+                        } else if (hl < (uint32_t)(Cfg::kBoxes * Cfg::kBoxesPerBlock))
+                            ptx::tma_load_2d(dst + hl * Cfg::kBoxBytes, &tmap_bt, (int32_t)(my_slab * Cfg::kNc + hl / Cfg::kBoxesPerBlock * Cfg::kBoxFeatures),
+                                             (int32_t)(first + hl % Cfg::kBoxesPerBlock * Cfg::kBoxRows), full_bar(s));
                     } else if (hl < (uint32_t)Cfg::kGatherOps) {
                         const uint4 rows4 = *reinterpret_cast<const uint4 *>(list + op_quad * 4);
                         ptx::tma_gather4_2d(dst + op_dst, &tmap_b, (int32_t)(my_slab * Cfg::kNc + op_x),
@@ -389,14 +498,15 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
     } else if (warp == Cfg::kMmaWarp && lane == 0 && rank == 0) {
         // =========================================================== MMA issuer (even CTA, warp 8, lane 0)
         constexpr uint32_t fmt = kTf32 ? ptx::kFmtTF32 : ptx::kFmtF16;
-        constexpr uint32_t idesc = ptx::make_instr_desc(fmt, kPairRows, kNs, false, true);
+        constexpr uint32_t idesc = ptx::make_instr_desc(fmt, kPairRows, kNs, false, true) | (kSparse ? ptx::kSparseA : 0u);
         const uint64_t a_desc0 = ptx::make_smem_desc(atile_addr, 16, 256, ptx::kSwizzle32B);
-        constexpr uint32_t b_lbo = kTf32 ? 1024u : 2048u, b_sbo = kTf32 ? 512u : 1024u;
+        constexpr uint32_t b_lbo = Cfg::kCW * 128u, b_sbo = kTf32 ? 512u : 1024u;
         const uint64_t b_desc0 =
             ptx::make_smem_desc(gather_addr, b_lbo, b_sbo, kTf32 ? ptx::kSwizzle128BBase32B : ptx::kSwizzle128B);
         const uint32_t a_hi = (uint32_t)(a_desc0 >> 32), b_hi = (uint32_t)(b_desc0 >> 32);
         const uint32_t a_lo0 = (uint32_t)a_desc0, b_lo0 = (uint32_t)b_desc0;
         constexpr uint32_t kATile16 = kTallTileBytes >> 4, kGather16 = Cfg::kGatherBytes >> 4;
+        const uint64_t meta_desc0 = ptx::make_smem_desc(meta_addr, 0, 128, ptx::kSwizzleNone);
         uint32_t s = 0, phase = 0;
         uint32_t alo = a_lo0, blo = b_lo0;
         bool alive = true;
@@ -413,10 +523,10 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
             const uint32_t item = item_id(round);
             if (item == kNoItem) break;
             uint32_t nt = tall_item<kTps>(p, item).n_tiles;
-            const uint32_t a = round & 1u;
+            const uint32_t a = acc_of(round);
             {
                 B200_PROF_T0();
-                alive = ptx::mbar_wait_cluster(acc_empty_bar(a), ((round >> 1) & 1u) ^ 1u, abort_flag, limit);
+                alive = ptx::mbar_wait_cluster(acc_empty_bar(a), acc_phase(round) ^ 1u, abort_flag, limit);
                 B200_PROF_ADD(prof_wait_acc);
             }
             ptx::tcgen05_fence_after_sync();
@@ -437,11 +547,16 @@ spmm_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_consta
 #ifdef B200SPMM_PROFILE
                 const long long prof_m0 = clock64();
 #endif
+                const uint32_t meta = tmem_base + Cfg::kMetaCols + s * 4u;
+                if constexpr (kSparse) ptx::tmem_copy_pair_128x128b(meta, meta_desc0 + (uint64_t)(s * (Cfg::kMetaBytes >> 4)));  // ahead of the MMAs, in order
 #pragma unroll
                 for (uint32_t q = 0; q < (uint32_t)kTps; ++q) {
                     const uint32_t on = q < here ? do_mma : 0u;
                     const uint32_t acc = q == 0 ? accumulate : 1u;
-                    ptx::umma_pair_ss_lohi_if(kTf32, on, d, alo + q * kATile16, a_hi, blo + q * kGather16, b_hi, idesc, acc);
+                    if constexpr (kSparse)  // (an odd column of metadata is named by the even one before it and a bit of the descriptor)
+                        ptx::umma_pair_sparse_f16_if(on, d, alo + q * kATile16, a_hi, blo + q * kGather16, b_hi, meta + (q & ~1u), idesc | (q & 1u), acc);
+                    else
+                        ptx::umma_pair_ss_lohi_if(kTf32, on, d, alo + q * kATile16, a_hi, blo + q * kGather16, b_hi, idesc, acc);
                 }
                 accumulate = 1;
                 nt -= here;

@@ -55,6 +55,12 @@ struct TallParams {
     // lies in shared memory, so a tile whose columns are that row group arrives by one bulk copy.
     const uint8_t *b_packed;
     uint32_t b_groups;          // row groups of B: ceil(cols / CW)
+    const uint8_t *B;           // 2:4 tiles only: [cols, n] row-major, rows of ldb_bytes
+    uint64_t ldb_bytes;
+    const uint8_t *meta;        // 2:4 tiles only (sparse24_gpu.hpp): which columns a row's values belong to
+    const uint32_t *quads;      // ... [eff+1] quads of tiles of the windows before
+    const uint32_t *n_rest;     // ... [eff][256] entries of every row's rest, and they themselves
+    const uint32_t *rest;
     uint32_t *sched_counter;    // [2] items handed out beyond the first gridDim.x, CTAs finished; zero at launch and at exit
     void *C;                    // [rows, n] row-major
     int64_t ldc;                // elements
@@ -634,12 +640,12 @@ tall_sum_parts_kernel(const float *partial, uint32_t parts, const uint32_t *__re
 // gathered tile down - fp16: 64-feature column blocks of 2 KB (16 rows x 128 B, the 16-byte pieces of a
 // row XORed with row % 8 inside each 8-row half); tf32: 32-feature column blocks of 1 KB (8 rows x 128 B,
 // the 32-byte units XORed with row % 4 inside each 4-row half).  Rows past `cols` and features past n are
-// zeros.  One thread per 16-byte piece.
-template <bool kTf32>
+// zeros.  One thread per 16-byte piece.  kCW = 32: groups of 32 rows for the 2:4 tiles, column blocks of 4 KB.
+template <bool kTf32, uint32_t kCW = kTf32 ? 8 : 16>
 __global__ void __launch_bounds__(256)
 pack_b_kernel(const uint8_t *B, int64_t ldb_bytes, uint32_t cols, uint32_t n, uint32_t kNs, uint32_t n_slabs,
               uint32_t n_groups, uint8_t *packed) {
-    constexpr uint32_t kCW = kTf32 ? 8 : 16, kEsz = kTf32 ? 4 : 2;
+    constexpr uint32_t kEsz = kTf32 ? 4 : 2;
     const uint32_t row_pieces = kNs * kEsz / 16;                       // 16-byte pieces of one row of a slab
     const uint64_t total = (uint64_t)n_slabs * n_groups * kCW * row_pieces;
     ptx::wait_for_grids_before();
@@ -660,9 +666,9 @@ pack_b_kernel(const uint8_t *B, int64_t ldb_bytes, uint32_t cols, uint32_t n, ui
             off = (h * 2 + (k >> 2)) * 512u + kr * 128u + ((((cc >> 1) ^ kr) << 5) | ((cc & 1u) << 4));
         } else {
             const uint32_t kr = k & 7u;
-            off = (h * 2 + (k >> 3)) * 1024u + kr * 128u + ((cc ^ kr) << 4);
+            off = (h * (kCW / 8) + (k >> 3)) * 1024u + kr * 128u + ((cc ^ kr) << 4);
         }
-        *reinterpret_cast<uint4 *>(packed + ((uint64_t)slab * n_groups + group) * (32u * kNs) + off) = v;
+        *reinterpret_cast<uint4 *>(packed + ((uint64_t)slab * n_groups + group) * (kCW * kEsz * kNs) + off) = v;
     }
 }
 

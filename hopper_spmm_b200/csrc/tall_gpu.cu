@@ -413,6 +413,7 @@ int build_tall_device(const b200spmm_btcf_info_t &info, const SuperCounts &count
         tiles_kernel<uint32_t><<<(unsigned)runs.size(), kTilesBlock>>>(d_runs, d_rowOffset, d_tcA2B, static_cast<const uint32_t *>(d_data), d_rowIdx,
                                                                        t.d_tcA2B, static_cast<uint8_t *>(t.d_data));
     B200_CUDA_TRY(cudaGetLastError());
+    t.h_rowOffset = std::move(rowOffset);
     *out = t;
     guard.t = nullptr;
     return B200SPMM_OK;

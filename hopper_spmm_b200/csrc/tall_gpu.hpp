@@ -13,6 +13,7 @@ struct TallFormat {
     uint32_t rows = 128;          // rows of a super-window: 128, or 256 for the CTA-pair kernel
     uint64_t eff = 0, tiles = 0;  // super-windows holding entries, their tiles (rows x CW each)
     uint64_t max_window_tiles = 0, min_window_tiles = 0;
+    std::vector<uint32_t> h_rowOffset;  // d_rowOffset on the host
     uint32_t *d_rowOffset = nullptr, *d_tcA2B = nullptr, *d_rowIdx = nullptr;
     uint32_t *d_aligned = nullptr;  // tiles whose columns are one aligned group of CW rows of B
     void *d_data = nullptr;  // tiles in the kernel's shared-memory image, 128 rows each: row r of an image has its
