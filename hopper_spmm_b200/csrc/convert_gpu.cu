@@ -5,10 +5,10 @@
 // benchmark matrix (5.2e8 entries) takes ten seconds on sixteen host cores and well under one on
 // the device.
 //
-// A matrix whose windows are not too empty for it (see window_bits_pay) is converted window by window: a block marks
-// the window's columns in a bit set in shared memory and lists them in order; after one scan over the windows the lists
-// move to their places.  60,000 nodes, 700,000 entries: 67 us with the values, where the sort took 101.  A block of 512 or 1024
-// threads is slower (conversion 140 us a call with 256, 164 with 512): most windows have a few hundred entries.
+// A matrix of up to 744,000 columns is converted window by window: a warp sorts the entries of a window in registers, or, where
+// they are more than kWarpEntries, a block marks their columns in a bit set in shared memory; either way an entry learns how many
+// distinct columns lie below its own, which is its place in the window's tiles.  One scan over the windows says where those
+// begin, and a pass over the entries writes column lists and values.
 //
 // Steps otherwise (all integer work, bound by HBM traffic):
 //   1. one key (window, column) per entry, in as few bits as the matrix needs - 32-bit keys where they fit - since
@@ -19,8 +19,8 @@
 //      rowOffset, rowIdx and all sizes.  The host waits for the device once on the way, for those sizes: a
 //      wait in each step (entries, distinct columns, windows, tiles) left the device idle for 80 of 290 us on
 //      a matrix of 700,000 entries.
-//   4. column lists scattered into tcA2B (pre-filled with 0xFFFFFFFF padding); every entry finds its slot by binary search in its window's column list and is written into
-//      the zero-filled tile array
+//   4. column lists scattered into tcA2B (pre-filled with 0xFFFFFFFF padding); every entry finds its slot by binary search in its
+//      window's column list and is written into the zero-filled tile array
 #include <algorithm>
 #include <cstdint>
 #include <cub/cub.cuh>
@@ -56,10 +56,22 @@ __device__ __forceinline__ uint32_t row_of_entry(const uint32_t *__restrict__ ro
     return lo;
 }
 
+// The last window whose first entry is p or one before it, found by a whole warp: 32 windows at a time.
+__device__ __forceinline__ uint32_t window_of_entry(const uint32_t *__restrict__ row_ptr, uint32_t n_windows, uint32_t row_window, uint32_t p) {
+    uint32_t lo = 0, hi = n_windows;  // row_ptr[lo * row_window] <= p, and behind hi - 1 none
+    while (hi - lo > 1) {
+        const uint32_t step = (hi - lo + 31) / 32, w = lo + (threadIdx.x & 31u) * step;
+        const uint32_t below = __ballot_sync(0xffffffffu, w < hi && (w == lo || row_ptr[w * row_window] <= p));
+        lo += (31u - (uint32_t)__clz((int)below)) * step;  // (lane 0 is always there)
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
+
 struct Totals {
     uint64_t n_unique;
     unsigned long long windows_tiles;  // windows that hold entries << 32 | their tiles
-    uint32_t bad;
+    uint32_t bad, hubs, long_windows;
 };
 
 // keys[p] = window(p) << col_bits | col[p]; flags row pointers that do not run from 0 to nnz, a column out
@@ -100,122 +112,271 @@ __global__ void window_bounds_kernel(const K *__restrict__ ukeys, const Totals *
     first[w] = lo;
 }
 
-constexpr int kBitsBlock = 256;
-constexpr size_t kBitsSmemMax = 100 * 1024;
+constexpr int kBitsBlock = 1024;
+constexpr size_t kBitsSmemMax = 125 * 1024, kSetsSmemMax = 220 * 1024;  // one set, the sets of a block
 constexpr uint32_t kGroupWords = 8;  // words of the bit set that share a rank
 
 inline uint32_t bit_words(uint64_t cols) { return (uint32_t)((cols + 32 * kGroupWords - 1) / (32 * kGroupWords)) * kGroupWords; }
-inline size_t bits_smem(uint64_t cols) { return (size_t)bit_words(cols) * 4 + (size_t)(bit_words(cols) / kGroupWords) * 4; }
+// the set, how many columns lie below a word in its group (a byte), and below a group
+inline size_t bits_smem(uint64_t cols) { return ((size_t)bit_words(cols) * 5 + (size_t)(bit_words(cols) / kGroupWords) * 4 + 15) / 16 * 16; }
 
-// A pass over the bit set costs a window its words, four at a time, where the sort costs an entry four or more passes
-// of ~20 bytes each.  Conversion of graphs in us, sets against sort, at words of the sets per entry: 133 / 212 at 10,
-// 151 / 218 at 23, 3,930 / 5,208 at 36, 272 / 268 at 58, 705 / 490 at 90.  The set has to leave room for two blocks an SM.
-inline bool window_bits_pay(uint64_t n_windows, uint64_t cols, uint64_t nnz) {
-    return bits_smem(cols) <= kBitsSmemMax && n_windows * bit_words(cols) <= 40 * nnz;
-}
+// What a column needs of a key beside the row (4 bits) and the entry (8 bits), see sort_window.
+constexpr uint32_t kKeyCols = (1u << 20) - 1u;
+static_assert(kBitsSmemMax / 11 * 2 * 32 < kKeyCols, "a column of the largest set fits a key");
 
-// The distinct columns of every window in order, at columns[first entry of the window ..], and how many they are.
-__global__ void __launch_bounds__(kBitsBlock)
-window_columns_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ col_idx, uint32_t rows, uint32_t cols, uint32_t nnz,
-                      uint32_t row_window, uint32_t n_windows, uint32_t words, uint32_t *__restrict__ columns, uint32_t *__restrict__ count,
-                      Totals *__restrict__ totals) {
-    constexpr int kUnroll = 8;  // columns of a thread in flight
-    extern __shared__ __align__(16) uint32_t bits[];
-    __shared__ uint32_t start[32], sums[kBitsBlock / 32];
-    const uint32_t groups = words / kGroupWords, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t *rank = bits + words;  // columns in the groups before
-    if (blockIdx.x == 0 && threadIdx.x == 0 && (row_ptr[0] != 0 || row_ptr[rows] != nnz)) atomicOr(&totals->bad, 1u);
-    for (uint32_t w = blockIdx.x; w < n_windows; w += gridDim.x) {
-        bool ok = true;
-        if (threadIdx.x <= row_window) {
-            const uint64_t r = (uint64_t)w * row_window + threadIdx.x;
-            const uint32_t s = row_ptr[min(r, (uint64_t)rows)], prev = threadIdx.x ? row_ptr[min(r - 1, (uint64_t)rows)] : 0u;
-            start[threadIdx.x] = s;
-            ok = s <= nnz && prev <= s;
-        }
-        for (uint32_t k = threadIdx.x; k < words / 4; k += kBitsBlock) reinterpret_cast<uint4 *>(bits)[k] = make_uint4(0, 0, 0, 0);
-        ok = __syncthreads_and(ok);
-        const uint32_t p0 = start[0], p1 = start[row_window];
-        if (!ok || p0 == p1) {
-            if (threadIdx.x == 0) {
-                count[w] = 0;
-                if (!ok) atomicOr(&totals->bad, 1u);
-            }
-            __syncthreads();
-            continue;
-        }
-        for (uint32_t q = p0 + threadIdx.x; q < p1; q += kUnroll * kBitsBlock) {  // (no overflow: p1 <= 2^32 - 1 is checked by the host)
-            uint32_t c[kUnroll], left[kUnroll];
+// The windows, where a block has room for a set.  Conversion of graphs in us, windows against the sort of all entries (four or
+// more passes of ~20 bytes an entry): 157 / 276 for 1.8e6 in 262,144, 960 / 1,560 for 10.4e6 in 524,288.
+inline bool by_windows_pays(uint64_t cols) { return bits_smem(cols) <= kBitsSmemMax; }
+
+// What the kernels of the windows read and write.
+struct WindowArgs {
+    const uint32_t *row_ptr, *col_idx;
+    uint32_t rows, cols, nnz, n_windows, row_window, log_cw, words;
+    uint32_t *places, *count;  // an entry's place in its window's tiles (tile, row, column), a window's distinct columns
+    uint32_t *listed;  // (the scan's output before it is written) windows for blocks: the longest from the front, others from the back
+    Totals *totals;
+    __device__ __forceinline__ uint32_t place(uint32_t column, uint32_t row) const {  // fewer than 2^24: 2^20 columns, 16 rows
+        return (((column >> log_cw) * row_window + row) << log_cw) | (column & ((1u << log_cw) - 1u));
+    }
+    // Lane k: the first entry of row k of window w, from row_window on the end of the last one.  False for all lanes if they are none.
+    __device__ __forceinline__ bool starts(uint32_t w, uint32_t lane, uint32_t *start) const {
+        *start = row_ptr[min((uint64_t)w * row_window + min(lane, row_window), (uint64_t)rows)];
+        const uint32_t prev = __shfl_up_sync(0xffffffffu, *start, 1);
+        return __all_sync(0xffffffffu, *start <= nnz && (lane == 0 || prev <= *start));
+    }
+    // the last row that starts at entry p or before it (for a whole warp)
+    __device__ __forceinline__ uint32_t row_of(uint64_t p, uint32_t start) const {
+        uint32_t r = 0;
 #pragma unroll
-            for (int k = 0; k < kUnroll; ++k) {
-                const uint64_t p = (uint64_t)q + (uint32_t)k * kBitsBlock;
-                c[k] = p < p1 ? col_idx[p] : 0u;
-                left[k] = p < p1 && p > p0 ? col_idx[p - 1] : 0u;
-            }
+        for (uint32_t step = 8; step; step /= 2) {
+            const uint32_t s = __shfl_sync(0xffffffffu, start, (int)(r + step));
+            if (r + step < row_window && s <= p) r += step;
+        }
+        return r;
+    }
+};
+
+constexpr uint32_t kWarpEntries = 256, kHubEntries = 4096;
+
+// A warp's window of up to 32 * kN entries, one key of column, row and entry each: a bitonic sort over the places lane * kN + k,
+// the strides below kN within a lane.
+template <int kN>
+__device__ __forceinline__ void sort_window(const WindowArgs &a, uint32_t w, uint32_t lane, uint32_t start, uint32_t p0, uint32_t n) {
+    uint32_t key[kN], before = 0, row_before = 0xFFFFFFFFu;  // column and row of the entry before the first one of a step
+    bool bad = false;
 #pragma unroll
-            for (int k = 0; k < kUnroll; ++k) {
-                const uint64_t p = (uint64_t)q + (uint32_t)k * kBitsBlock;
-                if (p >= p1) break;
-                if (p > p0 && left[k] >= c[k]) {  // only where a row starts
-                    bool row_start = false;
-                    for (uint32_t r = 1; r < row_window; ++r) row_start |= start[r] == p;
-                    if (!row_start) atomicOr(&totals->bad, 1u);
+    for (int k = 0; k < kN; ++k) key[k] = k * 32 + lane < n ? a.col_idx[p0 + k * 32 + lane] : 0xFFFFFFFFu;
+#pragma unroll
+    for (int k = 0; k < kN; ++k) {
+        const uint32_t i = k * 32 + lane, c = key[k], r = a.row_of((uint64_t)p0 + i, start);
+        uint32_t left = __shfl_up_sync(0xffffffffu, c, 1), left_row = __shfl_up_sync(0xffffffffu, r, 1);
+        if (lane == 0) left = before, left_row = row_before;
+        before = __shfl_sync(0xffffffffu, c, 31);
+        row_before = __shfl_sync(0xffffffffu, r, 31);
+        const bool live = i < n, fits = c < a.cols;
+        bad |= live && (!fits || (left_row == r && left >= c));
+        key[k] = live && fits ? c << 12 | r << 8 | i : 0xFFFFFFFFu;
+    }
+    if (__any_sync(0xffffffffu, bad)) {
+        if (lane == 0) {
+            a.count[w] = 0;
+            atomicOr(&a.totals->bad, 1u);
+        }
+        return;
+    }
+#pragma unroll
+    for (int size = 2; size <= 32 * kN; size *= 2) {
+#pragma unroll
+        for (int stride = size / 2; stride; stride /= 2) {
+            if (stride >= kN) {
+                // of two lanes, the one with the lower place keeps the smaller key in a rising run
+                const bool smaller = ((lane & (uint32_t)(stride / kN)) == 0) == ((lane & (uint32_t)(size / kN)) == 0);
+#pragma unroll
+                for (int k = 0; k < kN; ++k) {
+                    const uint32_t other = __shfl_xor_sync(0xffffffffu, key[k], stride / kN);
+                    key[k] = smaller ? min(key[k], other) : max(key[k], other);
                 }
-                if (c[k] < cols) atomicOr(bits + (c[k] >> 5), 1u << (c[k] & 31u));
-                else atomicOr(&totals->bad, 1u);
-            }
-            if (p1 - q <= kUnroll * kBitsBlock) break;
-        }
-        __syncthreads();
-        uint32_t base = 0;
-        for (uint32_t g0 = 0; g0 < groups; g0 += kBitsBlock) {  // one group a thread
-            const uint32_t g = g0 + threadIdx.x;
-            uint32_t mine = 0;
-            if (g < groups)
+            } else {
 #pragma unroll
-                for (uint32_t k = 0; k < kGroupWords; ++k) mine += __popc(bits[g * kGroupWords + k]);
-            uint32_t upto = mine;
+                for (int k = 0; k < kN; ++k) {
+                    if (k & stride) continue;
+                    const bool rising = size < kN ? (k & size) == 0 : (lane & (uint32_t)(size / kN)) == 0;
+                    const uint32_t lo = min(key[k], key[k + stride]), hi = max(key[k], key[k + stride]);
+                    key[k] = rising ? lo : hi;
+                    key[k + stride] = rising ? hi : lo;
+                }
+            }
+        }
+    }
+    uint32_t prev = __shfl_up_sync(0xffffffffu, key[kN - 1], 1), mine = 0;
+    if (lane == 0) prev = 0xFFFFFFFFu;  // (no entry's column)
+    bool first[kN];
 #pragma unroll
-            for (int d = 1; d < 32; d *= 2) {
-                const uint32_t x = __shfl_up_sync(0xffffffffu, upto, d);
-                if (lane >= (uint32_t)d) upto += x;
-            }
-            __syncthreads();  // `sums` of the round before has been read
-            if (lane == 31) sums[warp] = upto;
-            __syncthreads();
-            uint32_t before = base;
-            for (uint32_t k = 0; k < kBitsBlock / 32; ++k) {
-                if (k < warp) before += sums[k];
-                base += sums[k];
-            }
-            if (g < groups) rank[g] = before + upto - mine;
-        }
-        __syncthreads();
-        for (uint32_t k = threadIdx.x; k < words; k += kBitsBlock) {
-            uint32_t b = bits[k];
-            if (!b) continue;
-            uint32_t at = p0 + rank[k / kGroupWords];
-            for (uint32_t j = k / kGroupWords * kGroupWords; j < k; ++j) at += __popc(bits[j]);
-            for (; b; b &= b - 1u) columns[at++] = k * 32u + (uint32_t)__ffs((int)b) - 1u;
-        }
-        if (threadIdx.x == 0) count[w] = base;
-        __syncthreads();  // the next window clears the set
+    for (int k = 0; k < kN; ++k) {
+        first[k] = lane * kN + k < n && key[k] >> 12 != prev >> 12;
+        prev = key[k];
+        mine += first[k];
+    }
+    uint32_t upto = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, upto, d);
+        if (lane >= (uint32_t)d) upto += x;
+    }
+    if (lane == 31) a.count[w] = upto;
+    uint32_t at = upto - mine - 1;  // (of the column before: a column's first entry steps on)
+#pragma unroll
+    for (int k = 0; k < kN; ++k) {
+        at += first[k];
+        if (lane * kN + k < n) a.places[p0 + (key[k] & 255u)] = a.place(at, key[k] >> 8 & 15u);
     }
 }
 
-// The lists at their places, padded to whole tiles.
-__global__ void __launch_bounds__(kBitsBlock)
-place_columns_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ columns, const uint32_t *__restrict__ count,
-                     const uint32_t *__restrict__ tile_of, uint32_t n_windows, uint32_t row_window, uint32_t col_window,
-                     uint32_t *__restrict__ tcA2B) {
-    for (uint32_t w = blockIdx.x; w < n_windows; w += gridDim.x) {
-        const uint32_t n = count[w], padded = (n + col_window - 1) / col_window * col_window;
-        if (!n) continue;
-        const uint32_t *from = columns + row_ptr[w * row_window];
-        uint32_t *list = tcA2B + (uint64_t)tile_of[w] * col_window;
-#pragma unroll 4
-        for (uint32_t k = threadIdx.x; k < padded; k += kBitsBlock) list[k] = k < n ? from[k] : 0xFFFFFFFFu;
+// A window a warp.  `clear`: the tile array, zeroed on the way where it is there already.  A median window of a graph has a few
+// dozen entries: sorted by a warp that is some hundred instructions, marked in a set by a block of 256 threads it is 5,500,
+// most of them to clear and to count an empty set (60,000 nodes, 720,000 entries: 40 us; this kernel takes 9 with the zeroing of
+// 24 MB, the one for long windows 18 - 21).
+constexpr int kSortBlock = 256;
+__global__ void __launch_bounds__(kSortBlock)
+window_sort_kernel(const WindowArgs a, uint4 *__restrict__ clear, uint64_t n_clear) {
+    const uint32_t lane = threadIdx.x & 31u;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && (a.row_ptr[0] != 0 || a.row_ptr[a.rows] != a.nnz)) atomicOr(&a.totals->bad, 1u);
+    for (uint64_t w64 = (uint64_t)blockIdx.x * (kSortBlock / 32) + (threadIdx.x >> 5); w64 < a.n_windows; w64 += (uint64_t)gridDim.x * (kSortBlock / 32)) {
+        const uint32_t w = (uint32_t)w64;
+        uint32_t start;
+        const bool ok = a.starts(w, lane, &start);
+        const uint32_t p0 = __shfl_sync(0xffffffffu, start, 0), n = ok ? __shfl_sync(0xffffffffu, start, 31) - p0 : 0;
+        if (n == 0) {
+            if (lane == 0) {
+                a.count[w] = 0;
+                if (!ok) atomicOr(&a.totals->bad, 1u);
+            }
+        } else if (n <= 64) {
+            sort_window<2>(a, w, lane, start, p0, n);
+        } else if (n <= 128) {
+            sort_window<4>(a, w, lane, start, p0, n);
+        } else if (n <= kWarpEntries) {
+            sort_window<8>(a, w, lane, start, p0, n);
+        } else if (lane == 0) {
+            const bool hub = n > kHubEntries;
+            const uint32_t k = atomicAdd(hub ? &a.totals->hubs : &a.totals->long_windows, 1u);
+            a.listed[hub ? k : a.n_windows - 1 - k] = w;
+        }
     }
+    for (uint64_t k = (uint64_t)blockIdx.x * kSortBlock + threadIdx.x; k < n_clear; k += (uint64_t)gridDim.x * kSortBlock)
+        clear[k] = make_uint4(0, 0, 0, 0);
+}
+
+// A listed window by `threads` threads of the block (t of them this one), which have barrier `bar` and a set for themselves.
+__device__ __forceinline__ void mark_window(const WindowArgs &a, uint32_t w, uint32_t t, uint32_t threads, uint32_t bar, uint32_t *bits, uint32_t *sums) {
+    constexpr uint32_t kUnroll = 4;  // columns of a thread in flight
+    auto sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(threads) : "memory"); };
+    const uint32_t lane = t & 31u, warp = t >> 5, groups = a.words / kGroupWords;
+    uint32_t *rank = bits + a.words;  // columns in the groups before
+    uint8_t *in_group = reinterpret_cast<uint8_t *>(rank + groups);
+    uint32_t start;
+    a.starts(w, lane, &start);  // (every warp for itself; a window is listed if they are in order)
+    const uint32_t p0 = __shfl_sync(0xffffffffu, start, 0), n = __shfl_sync(0xffffffffu, start, 31) - p0;
+    const uint32_t *col = a.col_idx + p0;
+    start = lane < a.row_window ? start - p0 : 0xFFFFFFFFu;
+    for (uint32_t i = t; i < a.words / 4; i += threads) reinterpret_cast<uint4 *>(bits)[i] = make_uint4(0, 0, 0, 0);
+    sync();
+    for (uint32_t i0 = t & ~31u; i0 < n; i0 += kUnroll * threads) {  // of the warp's first lane
+        uint32_t c[kUnroll], left[kUnroll];
+#pragma unroll
+        for (uint32_t j = 0; j < kUnroll; ++j) {
+            const uint32_t i = i0 + j * threads + lane;
+            const bool live = j * threads < n - i0 && lane < n - i0 - j * threads;
+            c[j] = live ? col[i] : 0xFFFFFFFFu;
+            left[j] = live && lane == 0 && i ? col[i - 1] : 0u;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < kUnroll; ++j) {
+            if (j * threads >= n - i0) break;  // (the whole warp)
+            const uint32_t i = i0 + j * threads + lane, of_left = __shfl_up_sync(0xffffffffu, c[j], 1);
+            if (lane) left[j] = of_left;
+            if (c[j] < a.cols) atomicOr(bits + (c[j] >> 5), 1u << (c[j] & 31u));
+            if (i && left[j] >= c[j] && i < n) {  // only where a row starts
+                bool row_start = false;
+                for (uint32_t r = 1; r < a.row_window; ++r) row_start |= a.row_ptr[min((uint64_t)w * a.row_window + r, (uint64_t)a.rows)] == p0 + i;
+                if (!row_start) atomicOr(&a.totals->bad, 1u);
+            }
+            if (c[j] >= a.cols && lane < n - i0 - j * threads) atomicOr(&a.totals->bad, 1u);
+        }
+        if (n - i0 <= kUnroll * threads) break;  // (the sum may not fit)
+    }
+    sync();
+    uint32_t base = 0;
+    for (uint32_t g0 = 0; g0 < groups; g0 += threads) {  // one group a thread
+        const uint32_t g = g0 + t;
+        uint32_t mine = 0;
+        if (g < groups) {
+#pragma unroll
+            for (uint32_t h = 0; h < 2; ++h) {
+                const uint4 b = reinterpret_cast<const uint4 *>(bits)[2 * g + h];
+                const uint32_t word[4] = {b.x, b.y, b.z, b.w};
+                uint32_t below = 0;
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j) {
+                    below |= mine << (8 * j);  // (224 at most)
+                    mine += (uint32_t)__popc(word[j]);
+                }
+                reinterpret_cast<uint32_t *>(in_group)[2 * g + h] = below;
+            }
+        }
+        uint32_t upto = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, upto, d);
+            if (lane >= (uint32_t)d) upto += x;
+        }
+        if (g0) sync();  // `sums` of the round before has been read
+        if (lane == 31) sums[warp] = upto;
+        sync();
+        const uint32_t of_lane = lane < threads / 32 ? sums[lane] : 0u;
+        const uint32_t before = base + __reduce_add_sync(0xffffffffu, lane < warp ? of_lane : 0u);
+        base += __reduce_add_sync(0xffffffffu, of_lane);
+        if (g < groups) rank[g] = before + upto - mine;
+    }
+    sync();
+    for (uint32_t i0 = t & ~31u; i0 < n; i0 += kUnroll * threads) {
+        uint32_t c[kUnroll];
+#pragma unroll
+        for (uint32_t j = 0; j < kUnroll; ++j)
+            c[j] = j * threads < n - i0 && lane < n - i0 - j * threads ? col[i0 + j * threads + lane] : 0xFFFFFFFFu;
+#pragma unroll
+        for (uint32_t j = 0; j < kUnroll; ++j) {
+            if (j * threads >= n - i0) break;
+            // the rows that start at the warp's first entry or before it; most often all of its entries are of the last one
+            const uint32_t first = i0 + j * threads, rows = __ballot_sync(0xffffffffu, start <= first);
+            uint32_t r = 31u - (uint32_t)__clz((int)rows);
+            if (__any_sync(0xffffffffu, start > first && start - first < 32)) r = a.row_of(first + lane, start);
+            const uint32_t word = c[j] >> 5;
+            if (c[j] < a.cols)
+                a.places[p0 + first + lane] = a.place(rank[word / kGroupWords] + in_group[word] + (uint32_t)__popc(bits[word] & ((1u << (c[j] & 31u)) - 1u)), r);
+        }
+        if (n - i0 <= kUnroll * threads) break;
+    }
+    if (t == 0) a.count[w] = base;
+    sync();  // the next window clears the set
+}
+
+// The longest windows by a block each, of the others up to `most_parts` at a time.  Bound by the chain of a window - row
+// pointers, columns, marks, ranks, columns, places, a barrier after each - and by the longest one: 20,000 entries of a graph's
+// 720,000 take 20 us of one SM, where the others are done in 9.  Two blocks an SM, of 32 registers a thread, spill (23 us); lanes
+// that put the bits of one word together before the atomics cost more than the conflicts (23).
+__global__ void __launch_bounds__(kBitsBlock, 1)
+window_marks_kernel(const WindowArgs a, uint32_t most_parts, uint32_t set_words) {
+    extern __shared__ __align__(16) uint32_t sets[];
+    __shared__ uint32_t sums[4][32];
+    const uint32_t hubs = a.totals->hubs, n_long = a.totals->long_windows;
+    for (uint32_t k = blockIdx.x; k < hubs; k += gridDim.x) mark_window(a, a.listed[k], threadIdx.x, kBitsBlock, 0, sets, sums[0]);
+    uint32_t parts = most_parts;
+    while (parts > 1 && n_long <= gridDim.x * (parts / 2)) parts /= 2;
+    const uint32_t threads = kBitsBlock / parts, part = threadIdx.x / threads;
+    // from the last block on: the first ones have the longest windows
+    for (uint64_t k = (uint64_t)(gridDim.x - 1 - blockIdx.x) * parts + part; k < n_long; k += (uint64_t)gridDim.x * parts)
+        mark_window(a, a.listed[a.n_windows - 1 - (uint32_t)k], threadIdx.x % threads, threads, 1 + part, sets + part * set_words, sums[part]);
 }
 
 // The window's terms of the scan.  Fewer than 2^32 entries make fewer than 2^30 full tiles, 2^29 windows as many more.
@@ -245,6 +406,104 @@ __global__ void window_tables_kernel(const unsigned long long *__restrict__ befo
     if ((uint32_t)(before[w + 1] >> 32) == e) return;
     rowOffset[e] = tile;
     rowIdx[e] = w * row_window;
+}
+
+// The same scan and tables by one block, a load, a sum and a store for each 4,096 windows: 6 us for 3,750 of them, where the two
+// launches of the scan and the tables took 14.
+constexpr int kScanBlock = 1024;
+constexpr uint32_t kScanPer = 4, kOneBlockWindows = 16384;
+__global__ void __launch_bounds__(kScanBlock)
+scan_tables_kernel(const uint32_t *__restrict__ count, uint32_t n_windows, uint32_t row_window, uint32_t col_window,
+                   uint32_t *__restrict__ rowOffset, uint32_t *__restrict__ rowIdx, uint32_t *__restrict__ tile_of, Totals *__restrict__ totals) {
+    __shared__ unsigned long long warp_sums[kScanBlock / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    unsigned long long base = 0;
+    const WindowTerms terms{nullptr, count, n_windows, col_window};
+    for (uint32_t w0 = 0; w0 < n_windows; w0 += kScanBlock * kScanPer) {
+        const uint32_t w = w0 + threadIdx.x * kScanPer;
+        unsigned long long term[kScanPer], upto = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < kScanPer; ++k) {
+            term[k] = terms(w + k);
+            upto += term[k];
+        }
+        const unsigned long long mine = upto;
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+            const unsigned long long x = __shfl_up_sync(0xffffffffu, upto, d);
+            if (lane >= (uint32_t)d) upto += x;
+        }
+        if (w0) __syncthreads();  // the sums of the round before have been read
+        if (lane == 31) warp_sums[warp] = upto;
+        __syncthreads();
+        const unsigned long long of_lane = warp_sums[lane];  // (as many warps as lanes)
+        unsigned long long warps = of_lane;
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+            const unsigned long long x = __shfl_up_sync(0xffffffffu, warps, d);
+            if (lane >= (uint32_t)d) warps += x;
+        }
+        unsigned long long at = base + upto - mine + __shfl_sync(0xffffffffu, warps - of_lane, (int)warp);
+        base += __shfl_sync(0xffffffffu, warps, 31);
+#pragma unroll
+        for (uint32_t k = 0; k < kScanPer; ++k) {
+            if (w + k >= n_windows) break;
+            tile_of[w + k] = (uint32_t)at;
+            if (term[k]) {
+                rowOffset[at >> 32] = (uint32_t)at;
+                rowIdx[at >> 32] = (w + k) * row_window;
+            }
+            at += term[k];
+        }
+    }
+    if (threadIdx.x == 0) {
+        rowOffset[base >> 32] = (uint32_t)base;
+        totals->windows_tiles = base;
+    }
+}
+static_assert(kScanBlock / 32 == 32, "a lane for every warp's sum");
+
+// Entry p's column and value at its place; the list's slots without a column.  10 us for 720,000 entries; the columns listed
+// first, and every entry searching its column there, took 24.  A block takes kKeyEntries entries at a time
+// and looks for the windows of the first and the last of them.
+template <typename T>
+__global__ void __launch_bounds__(kBlock)
+place_entries_kernel(const uint32_t *__restrict__ row_ptr, const uint32_t *__restrict__ col_idx, const T *__restrict__ values,
+                     const uint32_t *__restrict__ places, const uint32_t *__restrict__ count, const uint32_t *__restrict__ tile_of,
+                     const Totals *__restrict__ totals, uint32_t nnz, uint32_t n_windows, uint32_t row_window, uint32_t log_cw,
+                     uint32_t *__restrict__ tcA2B, T *__restrict__ data) {
+    __shared__ uint32_t range[2];
+    if (totals->bad) return;  // (places are missing, and the windows need not hold the entries)
+    const uint32_t cw = 1u << log_cw, log_tile = log_cw + (row_window == 16 ? 4 : 3);
+    for (uint64_t w = (uint64_t)blockIdx.x * kBlock + threadIdx.x; w < n_windows; w += (uint64_t)gridDim.x * kBlock) {
+        const uint32_t n = count[w], padded = (n + cw - 1) & ~(cw - 1);
+        for (uint32_t k = n; k < padded; ++k) tcA2B[((uint64_t)tile_of[w] << log_cw) + k] = 0xFFFFFFFFu;
+    }
+    for (uint64_t p0 = (uint64_t)blockIdx.x * kKeyEntries; p0 < nnz; p0 += (uint64_t)gridDim.x * kKeyEntries) {
+        const uint32_t n = (uint32_t)min((uint64_t)kKeyEntries, nnz - p0);
+        __syncthreads();
+        if (threadIdx.x < 64) {
+            const uint32_t w = window_of_entry(row_ptr, n_windows, row_window, (uint32_t)p0 + (threadIdx.x < 32 ? 0u : n - 1));
+            if (threadIdx.x % 32 == 0) range[threadIdx.x / 32] = w;
+        }
+        __syncthreads();
+        const uint32_t first = range[0], end = range[1] + 1;
+#pragma unroll
+        for (uint32_t k = 0; k < kKeyEntries / kBlock; ++k) {
+            const uint32_t i = k * kBlock + threadIdx.x;
+            if (i >= n) break;
+            const uint32_t p = (uint32_t)p0 + i, place = places[p], c = col_idx[p];
+            const T v = values[p];
+            uint32_t lo = first, hi = end;
+            while (hi - lo > 1) {
+                const uint32_t mid = lo + (hi - lo) / 2;
+                if (row_ptr[mid * row_window] <= p) lo = mid; else hi = mid;
+            }
+            const uint64_t tile0 = tile_of[lo];
+            data[(tile0 << log_tile) + place] = v;
+            tcA2B[((tile0 + (place >> log_tile)) << log_cw) + (place & (cw - 1))] = c;  // (as every other entry of the column)
+        }
+    }
 }
 
 // distinct column j (sorted by window, column) -> its place in the window's padded column list
@@ -301,52 +560,92 @@ void scatter_values(const b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const ui
                                                                      (uint32_t)i.row_window, (uint32_t)i.col_window, static_cast<uint32_t *>(f->d_data));
 }
 
+// Up to this size the tile array is made ahead, as large as it can become (no column shared by two entries): it is cleared
+// while the places are found, and the host waits once instead of twice (about 12 us of 80).
+constexpr uint64_t kAheadBytes = (uint64_t)64 << 20;
+
+template <typename T>
+void place_entries(const b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const uint32_t *d_col_idx, const void *d_values, const uint32_t *places,
+                   const uint32_t *count, const uint32_t *tile_of, const Totals *totals, uint32_t log_cw, cudaStream_t stream) {
+    const auto &i = f->info;
+    const int grid = (int)std::min<uint64_t>((i.nnzs + kKeyEntries - 1) / kKeyEntries, 148 * 32);
+    place_entries_kernel<T><<<grid, kBlock, 0, stream>>>(d_row_ptr, d_col_idx, static_cast<const T *>(d_values), places, count, tile_of, totals,
+                                                         (uint32_t)i.nnzs, (uint32_t)i.total_row_windows, (uint32_t)i.row_window, log_cw,
+                                                         f->d_tcA2B, static_cast<T *>(f->d_data));
+}
+
 int convert_by_windows(b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const uint32_t *d_col_idx, const void *d_values, cudaStream_t stream) {
     const uint32_t rows = (uint32_t)f->info.rows, cols = (uint32_t)f->info.cols, nnz = (uint32_t)f->info.nnzs;
     const uint32_t n_windows = (uint32_t)f->info.total_row_windows, RW = (uint32_t)f->info.row_window, CW = (uint32_t)f->info.col_window;
-    const uint32_t words = bit_words(f->info.cols);
+    const uint32_t log_cw = CW == 16 ? 4 : CW == 8 ? 3 : 2;
     const size_t smem = bits_smem(f->info.cols);
-    const int esz = f->info.elt_size;
+    const uint64_t tile_bytes = (uint64_t)RW * CW * f->info.elt_size;
     PoolScratch tmp(stream);
     Totals *totals = nullptr;
-    uint32_t *columns = nullptr, *count = nullptr, *tile_of = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&columns, nnz));
-    unsigned long long *before = nullptr;
+    uint32_t *places = nullptr, *count = nullptr, *tile_of = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&places, nnz));
     B200_CUDA_TRY(tmp.alloc(&totals, 1));
     B200_CUDA_TRY(tmp.alloc(&count, n_windows));
     B200_CUDA_TRY(tmp.alloc(&tile_of, n_windows));
-    B200_CUDA_TRY(tmp.alloc(&before, (size_t)n_windows + 1));
-    const WindowTerms windows{nullptr, count, n_windows, CW};
-    auto terms = thrust::make_transform_iterator(thrust::make_counting_iterator<uint32_t>(0), windows);
-    size_t scan_bytes = 0;
-    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, terms, before, (int64_t)n_windows + 1, stream));
-    uint8_t *scan_tmp = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&scan_tmp, scan_bytes));
     B200_CUDA_TRY(pool_alloc(&f->d_rowOffset, (size_t)n_windows + 1, stream));
     B200_CUDA_TRY(pool_alloc(&f->d_rowIdx, n_windows, stream));
-    if (smem > 47 * 1024)  // (48 KB hold the kernel's own shared variables, too)
-        B200_CUDA_TRY(cudaFuncSetAttribute(window_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBitsSmemMax));
-    const unsigned grid = std::min<uint32_t>(n_windows, 148 * 64), table_grid = n_windows / kBlock + 1;
+    const uint64_t most_tiles = (uint64_t)nnz / CW + std::min(n_windows, nnz);
+    bool ahead = most_tiles * tile_bytes <= kAheadBytes;
+    auto alloc_tiles = [&](uint64_t tiles) {
+        const cudaError_t e = pool_alloc(&f->d_tcA2B, tiles * CW, stream);
+        return e == cudaSuccess ? pool_alloc_bytes(&f->d_data, std::max<uint64_t>(tiles * tile_bytes, 16), stream) : e;
+    };
+    if (ahead) {
+        const cudaError_t e = alloc_tiles(most_tiles);
+        if (e == cudaErrorMemoryAllocation) {  // what is needed may still fit
+            cudaGetLastError();
+            pool_free(f->d_tcA2B, stream);
+            f->d_tcA2B = nullptr;
+            ahead = false;
+        } else {
+            B200_CUDA_TRY(e);
+        }
+    }
+    const uint32_t parts = 4 * smem <= kSetsSmemMax ? 4 : 2 * smem <= kSetsSmemMax ? 2 : 1;
+    if (parts * smem > 47 * 1024)  // (48 KB hold the kernel's own shared variables, too)
+        B200_CUDA_TRY(cudaFuncSetAttribute(window_marks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSetsSmemMax));
     B200_CUDA_TRY(cudaMemsetAsync(totals, 0, sizeof(Totals), stream));
-    window_columns_kernel<<<grid, kBitsBlock, smem, stream>>>(d_row_ptr, d_col_idx, rows, cols, nnz, RW, n_windows, words, columns, count,
-                                                                 totals);
+    const WindowArgs args{d_row_ptr, d_col_idx, rows, cols, nnz, n_windows, RW, log_cw, bit_words(f->info.cols), places, count, tile_of, totals};
+    constexpr uint32_t kWarps = kSortBlock / 32;
+    window_sort_kernel<<<std::min<uint32_t>((n_windows + kWarps - 1) / kWarps, 148 * 64), kSortBlock, 0, stream>>>(
+        args, static_cast<uint4 *>(f->d_data), ahead ? most_tiles * tile_bytes / 16 : 0);
+    if (nnz > kWarpEntries) window_marks_kernel<<<std::min<uint32_t>(n_windows, 148), kBitsBlock, parts * smem, stream>>>(args, parts, (uint32_t)(smem / 4));
     B200_CUDA_TRY(cudaGetLastError());
-    B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, terms, before, (int64_t)n_windows + 1, stream));
-    window_tables_kernel<<<table_grid, kBlock, 0, stream>>>(before, n_windows, RW, f->d_rowOffset, f->d_rowIdx, tile_of, totals);
+    if (n_windows <= kOneBlockWindows) {
+        scan_tables_kernel<<<1, kScanBlock, 0, stream>>>(count, n_windows, RW, CW, f->d_rowOffset, f->d_rowIdx, tile_of, totals);
+    } else {
+        unsigned long long *before = nullptr;
+        uint8_t *scan_tmp = nullptr;
+        size_t scan_bytes = 0;
+        auto terms = thrust::make_transform_iterator(thrust::make_counting_iterator<uint32_t>(0), WindowTerms{nullptr, count, n_windows, CW});
+        B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, terms, before, (int64_t)n_windows + 1, stream));
+        B200_CUDA_TRY(tmp.alloc(&before, (size_t)n_windows + 1));
+        B200_CUDA_TRY(tmp.alloc(&scan_tmp, scan_bytes));
+        B200_CUDA_TRY(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, terms, before, (int64_t)n_windows + 1, stream));
+        window_tables_kernel<<<n_windows / kBlock + 1, kBlock, 0, stream>>>(before, n_windows, RW, f->d_rowOffset, f->d_rowIdx, tile_of, totals);
+    }
     B200_CUDA_TRY(cudaGetLastError());
+    auto place = [&]() {
+        if (f->info.elt_size == 2) place_entries<uint16_t>(f, d_row_ptr, d_col_idx, d_values, places, count, tile_of, totals, log_cw, stream);
+        else place_entries<uint32_t>(f, d_row_ptr, d_col_idx, d_values, places, count, tile_of, totals, log_cw, stream);
+        return cudaGetLastError();
+    };
+    if (ahead) B200_CUDA_TRY(place());
     Totals h;
     B200_CUDA_TRY(cudaMemcpyAsync(&h, totals, sizeof(h), cudaMemcpyDeviceToHost, stream));
     B200_CUDA_TRY(cudaStreamSynchronize(stream));
     if (h.bad) return B200SPMM_ERR_BAD_CSR;
     f->info.eff_row_windows = h.windows_tiles >> 32;
     f->info.total_tiles = (uint32_t)h.windows_tiles;
-    const uint64_t data_bytes = f->info.total_tiles * RW * CW * esz;
-    B200_CUDA_TRY(pool_alloc(&f->d_tcA2B, f->info.total_tiles * CW, stream));
-    B200_CUDA_TRY(pool_alloc_bytes(&f->d_data, std::max<uint64_t>(data_bytes, 16), stream));
-    B200_CUDA_TRY(cudaMemsetAsync(f->d_data, 0, data_bytes, stream));
-    place_columns_kernel<<<grid, kBitsBlock, 0, stream>>>(d_row_ptr, columns, count, tile_of, n_windows, RW, CW, f->d_tcA2B);
-    scatter_values(f, d_row_ptr, d_col_idx, d_values, windows, tile_of, stream);
-    B200_CUDA_TRY(cudaGetLastError());
+    if (ahead) return B200SPMM_OK;
+    B200_CUDA_TRY(alloc_tiles(f->info.total_tiles));
+    B200_CUDA_TRY(cudaMemsetAsync(f->d_data, 0, f->info.total_tiles * tile_bytes, stream));
+    B200_CUDA_TRY(place());
     B200_CUDA_TRY(cudaStreamSynchronize(stream));
     return B200SPMM_OK;
 }
@@ -512,7 +811,7 @@ int b200spmm_csr2btcf_nobitmap_device(uint64_t rows, uint64_t cols, uint64_t nnz
         return B200SPMM_OK;
     }
 
-    if (window_bits_pay(n_windows, cols, nnz)) {
+    if (by_windows_pays(cols)) {
         const int st = convert_by_windows(f, d_row_ptr, d_col_idx, d_values, stream);
         if (st != B200SPMM_OK) return st;
         guard.f = nullptr;

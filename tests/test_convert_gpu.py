@@ -115,3 +115,45 @@ def test_bit_set_that_just_fits_48_kb():
         assert np.array_equal(got[:ci.size], ci.view(np.uint32)) and (got[ci.size:] == 0xFFFFFFFF).all()
     """
     subprocess.run([sys.executable, "-c", code], check=True, timeout=300)
+
+
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+@pytest.mark.parametrize("rows,cols,nnz", [(100, 300, 1023), (100, 300, 1024), (100, 300, 1025), (65536, 64, 20000), (65552, 64, 20000),
+                                           (262144, 300, 300000), (262145, 300, 300000), (40000, 3000, 1100000), (40000, 3000, 2200000)])
+def test_entries_at_the_edges_of_the_window_passes(dt, rows, cols, nnz):
+    # entries a block places at a time; windows a round of the scan takes, the most that one block scans; a tile array made ahead
+    # and one that would be larger than that (tf32 from 1.04e6 entries on, fp16 from 2.08e6)
+    rng = np.random.default_rng(nnz + rows)
+    flat = np.sort(rng.choice(rows * cols, nnz, replace=False))
+    rp = np.searchsorted(flat, np.arange(rows + 1, dtype=np.int64) * cols).astype(np.uint32)
+    ci, v = (flat % cols).astype(np.uint32), rng.uniform(0.1, 1, nnz).astype(dt)
+    dev = device_convert(rows, cols, rp, ci, v)
+    assert_same(dev, hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    dev.close()
+
+
+@pytest.mark.parametrize("dt,rw,cw", [(np.float16, 16, 0), (np.float32, 16, 0), (np.float16, 8, 4)])
+def test_windows_at_the_edges_of_the_sorts_and_the_set(dt, rw, cw):
+    # entries of a window that a warp sorts with two, four and eight keys a lane, and that a block marks; among the last both lists
+    counts = [0, 1, 2, 63, 64, 65, 127, 128, 129, 0, 255, 256, 257, 4095, 4096, 4097, 9001, 1, 300, 64]
+    rng, cols = np.random.default_rng(7), 3001
+    lengths, ci = [], []
+    for n in counts:
+        cuts = np.sort(rng.integers(0, n + 1, rw - 1)) if n < 4000 else np.arange(1, rw) * n // rw  # (rows of up to `cols` entries)
+        lengths += list(np.diff(np.concatenate([[0], cuts, [n]])))
+    ci = np.concatenate([np.sort(rng.choice(cols if k % 3 else min(cols, 2 * n + 1), n, replace=False)) for k, n in enumerate(lengths)]).astype(np.uint32)
+    rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.uint32)
+    v, rows = rng.uniform(0.1, 1, ci.size).astype(dt), len(lengths)
+    dev = device_convert(rows, cols, rp, ci, v, rw, cw)
+    assert_same(dev, hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v), row_window=rw, **({"col_window": cw} if cw else {})))
+    dev.close()
+    for n in (2, 65, 129, 300, 4096):  # a column out of order, one twice, one out of range
+        for c in ([3, 1], [5, 5], [7, cols]):
+            bad, at = ci.copy(), int(rp[counts.index(n) * rw] if n != 300 else rp[18 * rw])
+            r = int(np.searchsorted(rp, at, side="right")) - 1
+            while lengths[r] < 2:
+                r += 1
+            bad[rp[r]:rp[r] + 2] = c
+            with pytest.raises(capi.SpmmError) as e:
+                device_convert(rows, cols, rp, bad, v, rw, cw)
+            assert e.value.status == capi.ERR_BAD_CSR
