@@ -207,15 +207,6 @@ tile_entries_kernel(const uint16_t *__restrict__ data, uint64_t tiles, uint32_t 
 
 }  // namespace tileimage
 
-namespace formatcheck {
-
-enum : uint32_t { kBadTables = 1u, kLooseLists = 2u };
-
-struct Found {
-    uint32_t flags;
-    int32_t falls;  // places where a column is not above the one before it, less those where a window starts
-};
-
 // Looks over the tables of a caller's format.  Bad tables: window offsets that do not rise from 0 to the number of tiles,
 // window rows that are past the end or closer than a window; nothing can run on them.  Loose lists: a window's columns are
 // not ascending and distinct with less than a tile of padding behind them, one is past the end, or a window starts off the
@@ -224,29 +215,29 @@ struct Found {
 // 60,000 nodes and 700,000 entries, now 5).  Reads inside [eff + 1], [eff] and [tiles * cw] whatever the tables hold.
 __global__ void __launch_bounds__(256)
 tables_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B, const uint32_t *__restrict__ rowIdx, uint32_t eff,
-              uint32_t tiles, uint64_t rows, uint64_t cols, uint32_t cw, Found *__restrict__ found) {
+              uint32_t tiles, uint64_t rows, uint64_t cols, uint32_t cw, formatcheck::Found *__restrict__ found) {
     uint32_t flags = 0;
     int32_t falls = 0;
     const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
-    if (first == 0 && (rowOffset[0] != 0 || rowOffset[eff] != tiles)) flags |= kBadTables;
+    if (first == 0 && (rowOffset[0] != 0 || rowOffset[eff] != tiles)) flags |= formatcheck::kBadTables;
     auto fall = [](uint32_t before, uint32_t c) { return c != kIdxMax && before >= c; };
     for (uint64_t w = first; w < eff; w += step) {
         const uint32_t t = rowOffset[w], row = rowIdx[w];
-        if (rowOffset[w + 1] <= t || row >= rows) flags |= kBadTables;
-        if (row % kRowWindow) flags |= kLooseLists;
+        if (rowOffset[w + 1] <= t || row >= rows) flags |= formatcheck::kBadTables;
+        if (row % kRowWindow) flags |= formatcheck::kLooseLists;
         if (!w) continue;
         const uint32_t row_before = rowIdx[w - 1];
-        if (row < row_before || row - row_before < (uint32_t)kRowWindow) flags |= kBadTables;
+        if (row < row_before || row - row_before < (uint32_t)kRowWindow) flags |= formatcheck::kBadTables;
         if (t && t < tiles && fall(tcA2B[(uint64_t)t * cw - 1], tcA2B[(uint64_t)t * cw])) --falls;
     }
     for (uint64_t q = first; q < (uint64_t)tiles * cw / 4; q += step) {
         const uint4 v = __ldg(reinterpret_cast<const uint4 *>(tcA2B) + q);
         const uint32_t c[4] = {v.x, v.y, v.z, v.w};
         uint32_t before = q ? __ldg(tcA2B + q * 4 - 1) : 0u;
-        if (q * 4 % cw == 0 && c[0] == kIdxMax) flags |= kLooseLists;
+        if (q * 4 % cw == 0 && c[0] == kIdxMax) flags |= formatcheck::kLooseLists;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            if (c[k] != kIdxMax && c[k] >= cols) flags |= kLooseLists;
+            if (c[k] != kIdxMax && c[k] >= cols) flags |= formatcheck::kLooseLists;
             if ((q || k) && fall(before, c[k])) ++falls;
             before = c[k];
         }
@@ -258,8 +249,6 @@ tables_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict
         if (flags) atomicOr(&found->flags, flags);
     }
 }
-
-}  // namespace formatcheck
 
 namespace {
 
@@ -1202,39 +1191,51 @@ int plan_start(b200spmm_plan *p) {
     B200_CUDA_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, p->device));
     if (major != 10) return B200SPMM_ERR_NO_DEVICE;
     B200_CUDA_TRY(cudaDeviceGetAttribute(&p->n_sms, cudaDevAttrMultiProcessorCount, p->device));
-    // status word, then the two counters of the chunk hand-out (the kernel leaves them at zero), then plan_check_tables' two
+    // status word, then the two counters of the chunk hand-out (the kernel leaves them at zero), then what tables_kernel finds
     B200_CUDA_TRY(pool_alloc(&p->d_status, 6));
     B200_CUDA_TRY(cudaMemset(p->d_status, 0, 6 * sizeof(uint32_t)));
     return B200SPMM_OK;
 }
 
-// A caller's device arrays: refused, or marked as loose (see formatcheck::tables_kernel).
-int plan_check_tables(b200spmm_plan *p) {
+formatcheck::Found *tables_found(const b200spmm_plan *p) { return reinterpret_cast<formatcheck::Found *>(p->d_status + 4); }
+
+// A caller's device arrays: looked over while the plan is made.
+int plan_start_table_check(b200spmm_plan *p) {
     const auto &info = p->info;
     if (info.eff_row_windows > info.total_tiles) return B200SPMM_ERR_INVALID_ARG;  // every window holds a tile
-    auto *d_found = reinterpret_cast<formatcheck::Found *>(p->d_status + 4);
-    formatcheck::Found found{};
     const uint64_t n = std::max<uint64_t>(info.eff_row_windows, info.total_tiles * (uint64_t)info.col_window / 4);
     const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)p->n_sms * 8));
-    formatcheck::tables_kernel<<<grid, 256>>>(p->d_rowOffset, p->d_tcA2B, p->d_rowIdx, (uint32_t)info.eff_row_windows, (uint32_t)info.total_tiles,
-                                              info.rows, info.cols, (uint32_t)info.col_window, d_found);
+    tables_kernel<<<grid, 256>>>(p->d_rowOffset, p->d_tcA2B, p->d_rowIdx, (uint32_t)info.eff_row_windows, (uint32_t)info.total_tiles,
+                                              info.rows, info.cols, (uint32_t)info.col_window, tables_found(p));
     B200_CUDA_TRY(cudaGetLastError());
-    B200_CUDA_TRY(cudaMemcpy(&found, d_found, sizeof(found), cudaMemcpyDeviceToHost));
-    if (found.flags & formatcheck::kBadTables) {
-        set_last_error_static("rowOffset or rowIdx does not describe windows of the matrix");
-        return B200SPMM_ERR_INVALID_ARG;
-    }
-    p->loose_lists = found.flags || found.falls;
     return B200SPMM_OK;
 }
 
-// h_rowOffset and h_rowIdx may be null: they are read back if the plan needs them.
-int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h_rowIdx, int n_ctas) {
+// Refused, or marked as loose (see tables_kernel).
+int plan_take_found(b200spmm_plan *p, const formatcheck::Found &found) {
+    if (found.bad()) {
+        set_last_error_static("rowOffset or rowIdx does not describe windows of the matrix");
+        return B200SPMM_ERR_INVALID_ARG;
+    }
+    p->loose_lists = found.loose();
+    p->row_boxes = !p->loose_lists;
+    return B200SPMM_OK;
+}
+
+// h_rowOffset and h_rowIdx may be null: they are read back if the plan needs them.  A caller's device arrays (checked) are being
+// looked over: what that finds comes with the sizes of the row units where those are asked for, or is waited for.
+int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h_rowIdx, int n_ctas, bool checked) {
     const auto &info = p->info;
+    formatcheck::Found found{};
+    bool found_known = !checked;
+    auto wait_for_check = [&]() -> int {
+        if (!found_known) B200_CUDA_TRY(cudaMemcpy(&found, tables_found(p), sizeof(found), cudaMemcpyDeviceToHost));
+        found_known = true;
+        return plan_take_found(p, found);
+    };
     const int cw = info.col_window;
     p->gather_cpasync = env_is("B200SPMM_GATHER", "cpasync");
     p->host_split = !env_is("B200SPMM_HOST_SPLIT", "0");
-    p->row_boxes = !p->loose_lists;
     // An explicit CTA count, a way to fetch tiles or rows, or a window height asks for a tile kernel.
     // B200SPMM_WINDOW=rows asks for the row units whatever the matrix.
     const bool force_rows = env_is("B200SPMM_WINDOW", "rows");
@@ -1242,25 +1243,30 @@ int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h
         const double fill = info.total_tiles ? (double)info.nnzs / ((double)info.total_tiles * kRowWindow * cw) : 0.0;
         double max_fill = kRowsMaxFill;
         if (fill > kRowsMaxFill && fill <= kRowsMaxFillWide && info.total_tiles >= kRowsWideMinTiles && !force_rows) {
+            int st = wait_for_check();
+            if (st != B200SPMM_OK) return st;
             std::vector<uint32_t> tables[2];
             if (!h_rowOffset) {
-                int st = read_window_tables(p, &tables[0], &tables[1]);
+                st = read_window_tables(p, &tables[0], &tables[1]);
                 if (st != B200SPMM_OK) return st;
             }
             double ratio = 1.0;
             uint64_t n_super = 0;
-            int st = estimate_tall_tile_ratio(info, h_rowOffset ? h_rowOffset : tables[0].data(), h_rowOffset ? h_rowIdx : tables[1].data(),
+            st = estimate_tall_tile_ratio(info, h_rowOffset ? h_rowOffset : tables[0].data(), h_rowOffset ? h_rowIdx : tables[1].data(),
                                               p->d_tcA2B, kTallRows, 48, &ratio, &n_super);
             if (st != B200SPMM_OK) return st;
             // (an eighth of the short tiles is the least that merging eight windows can leave)
             if (fill / (8.0 * ratio) < kTallMinFill || info.total_tiles < kRowsWideAnyTiles) max_fill = kRowsMaxFillWide;
         }
-        int st = build_row_formats(info, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, p->loose_lists, p->n_sms, max_fill, force_rows,
-                                   &p->rows_fmt, &p->narrow);
+        int st = build_row_formats(info, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, checked ? tables_found(p) : nullptr, &found, &found_known,
+                                   p->n_sms, max_fill, force_rows, &p->rows_fmt, &p->narrow);
+        if (st == B200SPMM_OK) st = wait_for_check();
         if (st != B200SPMM_OK) return st;
         p->rows_only = p->rows_fmt.n_units > 0;
         if (p->rows_only) return B200SPMM_OK;
     }
+    const int st = wait_for_check();
+    if (st != B200SPMM_OK) return st;
     return h_rowOffset ? plan_build_tile_path(p, h_rowOffset, h_rowIdx, n_ctas) : plan_add_tile_path(p, n_ctas);
 }
 
@@ -1561,7 +1567,7 @@ int b200spmm_plan_create(const b200spmm_btcf_t *h, int device, int n_ctas, b200s
     if (st == B200SPMM_OK) st = upload((void **)&p->d_rowIdx, f.rowIdx.data(), f.rowIdx.size() * 4);
     if (st == B200SPMM_OK) st = upload(&p->d_data, f.data.data(), f.data.size());
     if (st == B200SPMM_OK) st = plan_start(p);
-    if (st == B200SPMM_OK) st = guarded([&]() { return plan_finish(p, f.rowOffset.data(), f.rowIdx.data(), n_ctas); });
+    if (st == B200SPMM_OK) st = guarded([&]() { return plan_finish(p, f.rowOffset.data(), f.rowIdx.data(), n_ctas, false); });
     if (st != B200SPMM_OK) {
         b200spmm_plan_destroy(p);
         return st;
@@ -1594,8 +1600,8 @@ int b200spmm_plan_create_device(const b200spmm_btcf_info_t *info, const uint32_t
     p->d_data = const_cast<void *>(d_data);
     p->info.elt_size = info->dtype == B200SPMM_F16 ? 2 : 4;
     int st = plan_start(p);
-    if (st == B200SPMM_OK) st = plan_check_tables(p);
-    if (st == B200SPMM_OK) st = guarded([&]() { return plan_finish(p, nullptr, nullptr, n_ctas); });
+    if (st == B200SPMM_OK) st = plan_start_table_check(p);
+    if (st == B200SPMM_OK) st = guarded([&]() { return plan_finish(p, nullptr, nullptr, n_ctas, true); });
     if (st != B200SPMM_OK) {
         b200spmm_plan_destroy(p);
         return st;

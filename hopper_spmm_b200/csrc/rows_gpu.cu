@@ -3,12 +3,14 @@
 //   1. the tile stream in runs of kRunTiles, and a run cut where a window ends; a warp counts the stored values of each of
 //      the sixteen rows of its run (one 16-byte load per lane is half a tile row)
 //   2. per (window, row): running sums over the window's runs -> row lengths, and how many units there are of every length;
-//      one scan over the rows -> the units, slots and bands.  The longest come first, so the lengths alone say where every
-//      unit of a length lies and where its batches do: the host's one wait
+//      running sums over the rows -> the units, slots and bands.  The longest come first, so the lengths alone say where every
+//      unit of a length lies and where its batches do: the host's one wait, which brings what the look over a caller's tables
+//      has found as well
 //   3. every row puts its units into the list (build_band_units makes the one with the bands apart, CUB radix sort, four key bits)
 //   4. the warps of step 1 write (column, value) to the place of their row's unit
-// Eight launches and one wait before the last.  With the units sorted (CUB), three scans and a launch for each small step there
-// were 26; the plan of a graph of 60,000 nodes and 700,000 entries took 232 us instead of 138, of 10,000 nodes 200 instead of 99.
+// Seven launches and one wait before the last.  The plan of a graph of 60,000 nodes and 720,000 entries takes 95 us, of 10,000
+// nodes 80; with a wait for the tables, a scan in two launches, a hub row's pieces placed by one thread and values written as they
+// are found it was 138 and 99, with the units sorted, three scans and a launch for each small step (26 of them) 232 and 200.
 // A stored value is one whose bits are not all zero (an explicit zero adds nothing to a product), in a row and a column
 // of the matrix: the arrays may be a caller's, and what lies in a padded slot or below the last row multiplies nothing.
 #include <algorithm>
@@ -50,6 +52,9 @@ struct RowSums {
 struct AddSums {
     __host__ __device__ RowSums operator()(const RowSums &x, const RowSums &y) const { return {x.a + y.a, x.b + y.b}; }
 };
+// Rows a block of row_sums_kernel sums up, and how many such chunks one can have before it.
+constexpr uint32_t kChunkRows = 4 * kBlock, kMaxChunks = kBlock;
+
 struct RowTerms {
     const uint32_t *row_len;
     uint32_t cap;
@@ -65,6 +70,16 @@ struct RowTotals {
     uint32_t with_entries, n_batches, long_units[kLongUnits];  // units that have entries; and see RowsFormat
     uint32_t max_len;
     uint32_t band_row[kMaxBands + 1], band_cut[kMaxBands + 1];  // the bands' first rows and cut rows
+    formatcheck::Found found;
+    uint32_t blocks_done;  // of row_sums_kernel
+};
+
+// The look over the tables that runs ahead of the kernels here, if there is one, or what is known of them.
+struct Tables {
+    const formatcheck::Found *check;
+    bool known_loose;
+    __device__ __forceinline__ bool bad() const { return check && check->bad(); }
+    __device__ __forceinline__ bool loose() const { return check ? check->loose() : known_loose; }
 };
 
 // Where the units of a length lie in the list, and the four neighbours' batches (quads) in front of theirs.
@@ -80,15 +95,17 @@ struct LengthTables {
 __host__ __device__ __forceinline__ uint32_t first_run(uint32_t tile, uint32_t w) { return tile / kRunTiles + w; }
 
 // run -> window; clears what the kernels behind it count in
-__global__ void run_windows_kernel(const uint32_t *__restrict__ rowOffset, uint32_t eff, uint32_t rows, uint32_t *__restrict__ run_window,
-                                   uint32_t *__restrict__ row_len, LengthTables *__restrict__ tables, RowTotals *__restrict__ totals) {
+__global__ void run_windows_kernel(const uint32_t *__restrict__ rowOffset, uint32_t eff, uint32_t rows, Tables found, uint32_t *__restrict__ run_window,
+                                   uint32_t *__restrict__ row_len, LengthTables *__restrict__ tables, RowTotals *__restrict__ totals,
+                                   RowSums *__restrict__ chunks) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < eff)
+    if (i < kMaxChunks) chunks[i] = {0, 0};
+    if (i < eff && !found.bad())
         for (uint32_t r = first_run(rowOffset[i], i), end = first_run(rowOffset[i + 1], i + 1); r < end; ++r) run_window[r] = i;
     if (i < rows) row_len[i] = 0;
     if (blockIdx.x == 0) {
         for (uint32_t k = threadIdx.x; k < kLengths; k += blockDim.x) tables->count[k] = 0;
-        if (threadIdx.x == 0) totals->max_len = 0;
+        if (threadIdx.x == 0) totals->max_len = totals->blocks_done = 0;
     }
 }
 
@@ -104,32 +121,25 @@ struct RunTiles {
     }
 };
 
-// a[k] of registers, by halves: two predicates less a register than comparing k with every index
-template <int kN>
-__device__ __forceinline__ uint32_t pick(const uint32_t (&a)[kN], int k) {
-    const uint32_t lo = (k & 2) ? ((k & 1) ? a[3] : a[2]) : ((k & 1) ? a[1] : a[0]);
-    if (kN == 4) return lo;
-    const uint32_t hi = (k & 2) ? ((k & 1) ? a[kN - 1] : a[kN - 2]) : ((k & 1) ? a[kN - 3] : a[kN - 4]);
-    return (k & 4) ? hi : lo;
-}
-
 // The lane's share of a tile: row lane / 2, its left or right half of the columns.
 template <typename T>
 struct Piece {
     static constexpr int kPer = 16 / (int)sizeof(T);
     alignas(16) T v[kPer];
     uint32_t mask;
-    __device__ __forceinline__ T pick(int k) const {  // v[k]
-        const uint32_t *w = reinterpret_cast<const uint32_t *>(v);
-        const int i = sizeof(T) == 2 ? k >> 1 : k;
-        const uint32_t word = (i & 2) ? ((i & 1) ? w[3] : w[2]) : ((i & 1) ? w[1] : w[0]);
-        return sizeof(T) == 2 ? (T)(word >> ((k & 1) * 16)) : (T)word;
-    }
     __device__ __forceinline__ void load(const T *__restrict__ data, uint64_t tile, uint32_t lane) {
         *reinterpret_cast<uint4 *>(v) = __ldcs(reinterpret_cast<const uint4 *>(data + tile * (32 * kPer) + lane * kPer));
         mask = 0;
+        if (sizeof(T) == 2) {  // two values a word: a carry into the top bit of each half that is not zero
+            const uint32_t *w = reinterpret_cast<const uint32_t *>(v);
+            uint32_t m = 0;
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) mask |= v[k] != 0 ? 1u << k : 0u;
+            for (int k = 0; k < 4; ++k) m |= ((w[k] | ((w[k] & 0x7FFF7FFFu) + 0x7FFF7FFFu)) & 0x80008000u) >> (15 - 2 * k);
+            mask = (m | m >> 15) & 0xFFu;
+        } else {
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) mask |= v[k] != 0 ? 1u << k : 0u;
+        }
     }
     // Leaves the values that count.  `cols`: of the lane's half, `n_cols`: 0 for a row below the last one.  Unless the lists
     // are loose, only the last tile of a window has slots without a column.
@@ -152,8 +162,10 @@ template <typename T>
 __global__ void __launch_bounds__(kBlock)
 run_rows_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B, const T *__restrict__ data,
                 const uint32_t *__restrict__ rowIdx, const uint32_t *__restrict__ run_window,
-                uint32_t n_runs, uint32_t rows, uint32_t cols, bool loose, uint32_t *__restrict__ counts) {
+                uint32_t n_runs, uint32_t rows, uint32_t cols, Tables found, uint32_t *__restrict__ counts) {
     const uint32_t lane = threadIdx.x & 31u;
+    if (found.bad()) return;
+    const bool loose = found.loose();
     for (uint32_t run = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); run < n_runs; run += gridDim.x * (kBlock / 32)) {
         const RunTiles tiles(run, run_window, rowOffset);
         const uint32_t w = tiles.w, t0 = tiles.t0, t1 = tiles.t1, end = tiles.end;
@@ -192,15 +204,16 @@ run_rows_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restri
 
 // thread (window, row of it): counts of its runs become what the earlier runs hold; the sum is the row's length
 __global__ void __launch_bounds__(kBlock)
-row_lengths_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ rowIdx, uint32_t eff, uint32_t rows, uint32_t cap,
+row_lengths_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ rowIdx, uint32_t eff, uint32_t rows, uint32_t cap, Tables found,
                    uint32_t *__restrict__ counts, uint32_t *__restrict__ row_len, LengthTables *__restrict__ tables,
-                   RowTotals *__restrict__ totals) {
+                   RowTotals *__restrict__ totals, RowSums *__restrict__ chunks, uint32_t n_chunks) {
     __shared__ uint32_t here[kLengths];
+    if (found.bad()) return;
     for (uint32_t k = threadIdx.x; k < kLengths; k += kBlock) here[k] = 0;
     __syncthreads();
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t w = (uint32_t)(i >> 4), r = (uint32_t)i & 15u;
-    uint32_t sum = 0;
+    uint32_t sum = 0, chunk = 0;
     if (w < eff) {
         const uint32_t end = first_run(rowOffset[w + 1], w + 1);
         for (uint32_t run = first_run(rowOffset[w], w); run < end; run += 8) {
@@ -214,9 +227,21 @@ row_lengths_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__res
             }
         }
         if (rowIdx[w] + r < rows) row_len[rowIdx[w] + r] = sum;
+        chunk = (rowIdx[w] + r) / kChunkRows;
+    }
+    const uint32_t n = pieces_of(sum, cap);
+    if (n_chunks) {
+        // what the rows of a chunk add to the running sums, without the unit that every row has: a lane for each chunk of the warp
+        // (one or two, or a lane each where a caller's windows lie far apart)
+        const uint32_t same = __match_any_sync(0xffffffffu, chunk), lane = threadIdx.x & 31u;
+        const uint32_t len = __reduce_add_sync(same, sum), more = __reduce_add_sync(same, n - 1), slots = __reduce_add_sync(same, n > 1 ? n : 0u);
+        const uint32_t cut = __popc(__ballot_sync(0xffffffffu, n > 1) & same);
+        if (len && (uint32_t)__ffs((int)same) - 1u == lane) {
+            atomicAdd(&chunks[chunk].a, (unsigned long long)len << 32 | more);
+            if (cut) atomicAdd(&chunks[chunk].b, (unsigned long long)cut << 32 | slots);
+        }
     }
     if (sum) {  // (none below the last row)
-        const uint32_t n = pieces_of(sum, cap);
         if (n > 1) atomicAdd(&here[kMaxUnitEntries - cap], n - 1);
         atomicAdd(&here[kMaxUnitEntries - (sum - (n - 1) * cap)], 1u);
     }
@@ -251,9 +276,7 @@ __device__ __forceinline__ uint32_t block_exclusive_sum(uint32_t mine, uint32_t 
 // k of all four, then batch k + 1): the groups of a warp, which walk neighbours, read their entries from the same lines.  A
 // quad takes the steps of its first unit, which is its longest.
 static_assert(kLengths == kBlock, "a thread for every length");
-__global__ void __launch_bounds__(kBlock)
-row_totals_kernel(uint32_t rows, const RowSums *__restrict__ sums, LengthTables *__restrict__ tables, RowTotals *__restrict__ totals) {
-    __shared__ uint32_t warp_sums[kBlock / 32];
+__device__ __forceinline__ void row_totals(uint32_t rows, Tables found, const RowSums *sums, LengthTables *tables, RowTotals *totals, uint32_t *warp_sums) {
     const uint32_t k = threadIdx.x, count = tables->count[k], start = block_exclusive_sum(count, warp_sums);
     const uint32_t steps = (quads_before(start + count) - quads_before(start)) * batches_of_length(k);  // of the quads that begin here
     const uint32_t steps_before = block_exclusive_sum(steps, warp_sums);
@@ -266,12 +289,13 @@ row_totals_kernel(uint32_t rows, const RowSums *__restrict__ sums, LengthTables 
         tables->start[kEmpty] = tables->cursor[kEmpty] = totals->with_entries = start + count;
         totals->n_batches = 4 * (steps_before + steps);
     }
-    const RowSums all = sums[rows - 1];
+    const RowSums all = {__ldcg(&sums[rows - 1].a), __ldcg(&sums[rows - 1].b)};  // (other blocks may have written them just now)
     if (k == 0) {
         totals->entries = (uint32_t)(all.a >> 32);
         totals->units = (uint32_t)all.a;
         totals->cut_rows = (uint32_t)(all.b >> 32);
         totals->slots = (uint32_t)all.b;
+        totals->found = found.check ? *found.check : formatcheck::Found{};
     }
     if (k > kMaxBands) return;
     const uint64_t cost = (all.a >> 32) + kRowCost * rows;
@@ -280,11 +304,73 @@ row_totals_kernel(uint32_t rows, const RowSums *__restrict__ sums, LengthTables 
     const uint64_t want = cost * k / bands;
     while (k && k < bands && lo < hi) {
         const uint32_t mid = lo + (hi - lo) / 2;
-        if ((sums[mid].a >> 32) + kRowCost * (mid + 1) <= want) lo = mid + 1; else hi = mid;
+        if ((__ldcg(&sums[mid].a) >> 32) + kRowCost * (mid + 1) <= want) lo = mid + 1; else hi = mid;
     }
     if (!k || k >= bands) lo = k ? rows : 0u;
     totals->band_row[k] = lo;
-    totals->band_cut[k] = lo ? (uint32_t)(sums[lo - 1].b >> 32) : 0u;
+    totals->band_cut[k] = lo ? (uint32_t)(__ldcg(&sums[lo - 1].b) >> 32) : 0u;
+}
+
+__global__ void __launch_bounds__(kBlock)
+row_totals_kernel(uint32_t rows, Tables found, const RowSums *sums, LengthTables *tables, RowTotals *totals) {
+    __shared__ uint32_t warp_sums[kBlock / 32];
+    row_totals(rows, found, sums, tables, totals, warp_sums);
+}
+
+__device__ __forceinline__ unsigned long long shfl_up(unsigned long long x, int d) { return __shfl_up_sync(0xffffffffu, x, d); }
+
+// The running sums of up to kMaxChunks chunks of rows: a block adds up what row_lengths_kernel has summed of the chunks before its
+// own, and the last block to finish makes the totals.  60,000 rows: 8 us, where a scan in two launches and the totals took 15.
+__global__ void __launch_bounds__(kBlock)
+row_sums_kernel(const uint32_t *__restrict__ row_len, uint32_t rows, uint32_t cap, Tables found, const RowSums *__restrict__ chunks, RowSums *sums,
+                LengthTables *tables, RowTotals *totals) {
+    __shared__ RowSums warp_sums[kBlock / 32], warp_chunks[kBlock / 32];
+    __shared__ uint32_t totals_sums[kBlock / 32], last;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, r0 = blockIdx.x * kChunkRows + threadIdx.x * 4;
+    RowSums before = threadIdx.x < blockIdx.x ? chunks[threadIdx.x] : RowSums{0, 0};
+    uint32_t len[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) len[k] = r0 + k < rows ? row_len[r0 + k] : 0u;
+    RowSums of[4], upto{0, 0};
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+        const uint32_t n = pieces_of(len[k], cap);
+        upto.a += (unsigned long long)len[k] << 32 | n;
+        if (n > 1) upto.b += 1ull << 32 | n;
+        of[k] = upto;
+    }
+    const RowSums mine = upto;
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+        const RowSums x{shfl_up(upto.a, d), shfl_up(upto.b, d)};
+        if (lane >= (uint32_t)d) upto = AddSums{}(upto, x);
+    }
+#pragma unroll
+    for (int d = 16; d; d /= 2) {
+        before.a += __shfl_xor_sync(0xffffffffu, before.a, d);
+        before.b += __shfl_xor_sync(0xffffffffu, before.b, d);
+    }
+    if (lane == 31) {
+        warp_sums[warp] = upto;
+        warp_chunks[warp] = before;
+    }
+    __syncthreads();
+    RowSums base{(unsigned long long)blockIdx.x * kChunkRows + upto.a - mine.a, upto.b - mine.b};  // every row before has a unit
+#pragma unroll
+    for (uint32_t k = 0; k < kBlock / 32; ++k) {
+        base = AddSums{}(base, warp_chunks[k]);
+        if (k < warp) base = AddSums{}(base, warp_sums[k]);
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k)
+        if (r0 + k < rows) sums[r0 + k] = AddSums{}(base, of[k]);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&totals->blocks_done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    row_totals(rows, found, sums, tables, totals, totals_sums);
 }
 
 // Thread r: the units of row r take places among those of their length (in the order in which blocks of rows ask), and its
@@ -293,8 +379,12 @@ __global__ void __launch_bounds__(kBlock)
 place_units_kernel(const uint32_t *__restrict__ row_len, uint32_t rows, uint32_t cap, const RowSums *__restrict__ sums, LengthTables *__restrict__ tables,
                    const RowTotals *__restrict__ totals, uint2 *__restrict__ units, uint32_t *__restrict__ unit_batch,
                    RowSplit *__restrict__ splits, uint32_t *__restrict__ batches, uint32_t batch_words) {
-    __shared__ uint32_t base[kLengths + 1];
-    for (uint32_t k = threadIdx.x; k <= kLengths; k += kBlock) base[k] = 0;
+    __shared__ uint32_t base[kLengths + 1], start[kLengths + 1], quad_steps[kLengths];
+    for (uint32_t k = threadIdx.x; k <= kLengths; k += kBlock) {
+        base[k] = 0;
+        start[k] = tables->start[k];
+        if (k < kLengths) quad_steps[k] = tables->quad_steps[k];
+    }
     __syncthreads();
     const uint32_t r = blockIdx.x * kBlock + threadIdx.x;
     uint32_t n = 0, full = 0, last_key = 0, rank_full = 0, rank_last = 0;
@@ -314,20 +404,28 @@ place_units_kernel(const uint32_t *__restrict__ row_len, uint32_t rows, uint32_t
     if (blockIdx.x == 0 && threadIdx.x < batch_words)  // the batch that belongs to nobody
         batches[(uint64_t)totals->n_batches * batch_words + threadIdx.x] = batch_words == kBatchWords<true> ? (threadIdx.x == kTargetWord<true> ? kNoTarget : 0u)
                                                                                                  : (threadIdx.x == kTargetWord<false> ? kNoTarget : 0u);
-    if (r >= rows) return;
-    const uint32_t first_unit = (uint32_t)sums[r].a - n;
-    for (uint32_t q = 0; q < n; ++q) {
-        const uint32_t key = q < full ? full_key : last_key, place = q < full ? base[full_key] + rank_full + q : base[last_key] + rank_last;
-        uint32_t first = 0;
-        if (key != kEmpty) {
-            uint32_t of = key;  // the length of the quad's first unit
-            while (tables->start[of] > (place & ~3u)) --of;
-            first = 4 * (tables->quad_steps[of] + (place / 4 - quads_before(tables->start[of])) * batches_of_length(of)) + (place & 3u);
-            unit_batch[first_unit + q] = first;
-        }
-        units[place] = key != kEmpty ? make_uint2(first, batches_of_length(key)) : make_uint2(r, 0u);
+    const uint32_t lane = threadIdx.x & 31u;
+    const RowSums sum = r < rows ? sums[r] : RowSums{0, 0};
+    // a piece of `key` at `place` of the list, the unit_at-th unit of the rows' order
+    auto put = [&](uint32_t place, uint32_t key, uint32_t unit_at) {
+        uint32_t of = key;  // the length of the quad's first unit
+        while (start[of] > (place & ~3u)) --of;
+        const uint32_t first = 4 * (quad_steps[of] + (place / 4 - quads_before(start[of])) * batches_of_length(of)) + (place & 3u);
+        unit_batch[unit_at] = first;
+        units[place] = make_uint2(first, batches_of_length(key));
+    };
+    // the full pieces of a long row by the whole warp: a hub row has hundreds (60,000 nodes: by its own thread 16 us, now 9)
+    for (uint32_t cut = __ballot_sync(0xffffffffu, full != 0); cut; cut &= cut - 1u) {
+        const int from = __ffs((int)cut) - 1;
+        const uint32_t pieces = __shfl_sync(0xffffffffu, full, from), place = base[full_key] + __shfl_sync(0xffffffffu, rank_full, from);
+        const uint32_t unit_at = __shfl_sync(0xffffffffu, (uint32_t)sum.a - n, from);
+        for (uint32_t q = lane; q < pieces; q += 32) put(place + q, full_key, unit_at + q);
     }
-    if (n > 1) splits[(uint32_t)(sums[r].b >> 32) - 1] = RowSplit{r, (uint32_t)sums[r].b - n, (uint32_t)sums[r].b};
+    if (r >= rows) return;
+    const uint32_t place = base[last_key] + rank_last;
+    if (last_key != kEmpty) put(place, last_key, (uint32_t)sum.a - 1);
+    else units[place] = make_uint2(r, 0u);
+    if (n > 1) splits[(uint32_t)(sum.b >> 32) - 1] = RowSplit{r, (uint32_t)sum.b - n, (uint32_t)sum.b};
 }
 
 // The first rows of the bands.
@@ -394,78 +492,93 @@ __device__ __forceinline__ void split_value(T v, uint32_t n, T *first, T *unit) 
     *unit = (T)(sign | (exp > 10 ? (exp - 10) << (10 + kLow) : 1u << (max(exp, 1u) - 1 + kLow)));
 }
 
+// A warp lists the stored values of its run - tile, lane and place in the lane's half row - and then takes 32 of the list at a
+// time: written as they are found, lane by lane, a tile of a graph with 16 values kept 13 lanes of 32 busy in three rounds
+// (720,000 entries, 60,000 rows: 30 us, 330 instructions a tile; now 21, 210).  Bound by instructions: neither more of the list in
+// flight nor the list in the order of the rows' entries, which makes fewer and wider stores, is faster.
 template <typename T>
 __global__ void __launch_bounds__(kBlock)
 write_entries_kernel(const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ tcA2B, const T *__restrict__ data,
                      const uint32_t *__restrict__ rowIdx, const uint32_t *__restrict__ run_window, uint32_t n_runs, uint32_t rows, uint32_t n_cols,
-                     bool loose, uint32_t cap, const uint32_t *__restrict__ counts, const uint32_t *__restrict__ row_len,
+                     bool loose, uint32_t cap_bits, const uint32_t *__restrict__ counts, const uint32_t *__restrict__ row_len,
                      const RowSums *__restrict__ sums, const uint32_t *__restrict__ unit_batch, uint32_t *__restrict__ batches) {
-    constexpr int kPer = Piece<T>::kPer;
-    constexpr uint32_t kWords = kBatchWords<sizeof(T) == 4>, kTo = kTargetWord<sizeof(T) == 4>;
-    const uint32_t lane = threadIdx.x & 31u;
+    constexpr uint32_t kPer = Piece<T>::kPer, kWords = kBatchWords<sizeof(T) == 4>, kTo = kTargetWord<sizeof(T) == 4>;
+    __shared__ uint16_t lists[kBlock / 32][kRunTiles * 32 * kPer];
+    static_assert(kRunTiles * kPer <= 64, "a bit for each of a lane's values");
+    const uint32_t lane = threadIdx.x & 31u, cap = 1u << cap_bits;
+    uint16_t *list = lists[threadIdx.x >> 5];
     for (uint32_t run = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); run < n_runs; run += gridDim.x * (kBlock / 32)) {
         const RunTiles tiles(run, run_window, rowOffset);
-        const uint32_t w = tiles.w, t0 = tiles.t0, t1 = tiles.t1, w_end = tiles.end, row = min(rowIdx[w] + (lane >> 1), rows - 1);
-        if (t0 >= t1) continue;
-        const uint32_t len = row_len[row], limit = rowIdx[w] + (lane >> 1) < rows ? n_cols : 0u, n_pieces = pieces_of(len, cap);
+        const uint32_t w = tiles.w, t0 = tiles.t0, n_tiles = tiles.t1 - t0, first_row = rowIdx[w], row = min(first_row + (lane >> 1), rows - 1);
+        if (t0 >= tiles.t1) continue;
+        const uint32_t limit = first_row + (lane >> 1) < rows ? n_cols : 0u;
+        // of the lane's row
+        const uint32_t len = row_len[row], at = counts[(uint64_t)run * 16 + (lane >> 1)];  // its entries, those in front of the run
         const RowSums sum = sums[row];
-        const uint32_t *unit = unit_batch + ((uint32_t)sum.a - n_pieces);  // first batches of the row's units
-        uint32_t at = counts[(uint64_t)run * 16 + (lane >> 1)];  // entries of the row so far
-        // Everything a lane reads comes ahead of its stores and for all lanes at once - the unit it starts in, a tile's
-        // columns and values while the tile before is written: fetched at its first entry, one by one, they cost the warp
-        // a round trip to L2 per entry (43 us of a matrix of 700,000 entries, 60,000 rows; now 32).
-        uint32_t piece = min(at / cap, n_pieces - 1u), piece_end = (piece + 1) * cap;
-        uint32_t fill = (0u - min(len - piece * cap, cap)) % kUnitBatch;  // slots before the second entry of the unit
-        uint32_t *out = batches + (uint64_t)(len ? unit[piece] : 0u) * kWords;
-        // the unit's last batch holds its target, the others none; a batch's first entry writes it
-        auto target = [&](uint32_t e) {
-            const uint32_t entries = min(len - piece * cap, cap);
-            if (e / kUnitBatch + 1 < (entries + kUnitBatch - 1) / kUnitBatch) return kNoTarget;
-            return n_pieces > 1 ? kSlotTarget | ((uint32_t)sum.b - n_pieces + piece) : row;
-        };
-        auto put = [&](uint32_t e, uint32_t col, T v) {
-            uint32_t *words = out + (e / kUnitBatch) * (4 * kWords);
-            words[e % kUnitBatch] = col;
-            if (e % kUnitBatch == 0) words[kTo] = target(e);
-            reinterpret_cast<T *>(words + kUnitBatch)[e % kUnitBatch] = v;
-        };
-        Piece<T> next;
-        alignas(16) uint32_t next_cols[kPer];
-        auto fetch = [&](uint32_t t) {
-            next.load(data, t, lane);
-            load_columns(next_cols, tcA2B, t, lane);
-        };
-        fetch(t0);
-        for (uint32_t t = t0; t < t1; ++t) {
-            Piece<T> p = next;
-            uint32_t cols[kPer];
+        const uint32_t pieces = pieces_of(len, cap), unit = (uint32_t)sum.a - pieces, slot = (uint32_t)sum.b - pieces;
+        uint64_t found = 0;  // the lane's values, kPer bits a tile
 #pragma unroll
-            for (int k = 0; k < kPer; ++k) cols[k] = next_cols[k];
-            if (loose || t + 1 == w_end || limit == 0) p.keep(cols, limit);
-            if (t + 1 < t1) fetch(t + 1);
-            const uint32_t mine = (uint32_t)__popc(p.mask), other = __shfl_xor_sync(0xffffffffu, mine, 1);
-            uint32_t k_out = at + ((lane & 1u) ? other : 0u);
-            at += mine + other;
-            for (uint32_t m = p.mask; m; m &= m - 1u) {  // (two or three steps a warp; one per column would be eight)
-                const int k = __ffs((int)m) - 1;
-                const uint32_t col = pick(cols, k);
-                const T v = sizeof(T) == 2 ? p.pick(k) : (T)((uint32_t)p.pick(k) & 0xFFFFE000u);  // as the tensor core reads it
-                if (k_out >= piece_end) {
-                    piece = k_out / cap;
-                    piece_end = (piece + 1) * cap;
-                    out = batches + (uint64_t)unit[piece] * kWords;
-                    fill = (0u - min(len - piece * cap, cap)) % kUnitBatch;
-                }
-                const uint32_t e = k_out - piece * cap;
-                ++k_out;
-                T value = v, one;
-                if (!e && fill) {
-                    split_value(v, fill, &value, &one);
-                    for (uint32_t f = 1; f <= fill; ++f) put(f, col, one);
-                }
-                put(e ? e + fill : 0u, col, value);
+        for (uint32_t t = 0; t < kRunTiles; ++t) {
+            if (t >= n_tiles) break;
+            Piece<T> p;
+            p.load(data, t0 + t, lane);
+            if (loose || t0 + t + 1 == tiles.end || limit == 0) {
+                alignas(16) uint32_t cols[kPer];
+                load_columns(cols, tcA2B, t0 + t, lane);
+                p.keep(cols, limit);
             }
+            found |= (uint64_t)p.mask << (t * kPer);
         }
+        const uint32_t mine = (uint32_t)__popcll(found);
+        uint32_t upto = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, upto, d);
+            if (lane >= (uint32_t)d) upto += x;
+        }
+        const uint32_t n = __shfl_sync(0xffffffffu, upto, 31);
+        uint32_t to = upto - mine;
+        const uint32_t first_entry = at - to;  // of the lane's values, were there none in the other half
+        for (uint64_t m = found; m; m &= m - 1) list[to++] = (uint16_t)((uint32_t)(__ffsll((long long)m) - 1) << 5 | lane);
+        __syncwarp();
+        for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+            const uint32_t i = i0 + lane;
+            const uint32_t which = i < n ? list[i] : 0u, from = which & 31u, bit = which >> 5, tile = bit / kPer, k = bit % kPer;
+            uint32_t col = 0;
+            T v = 0;
+            if (i < n) {
+                col = tcA2B[(uint64_t)(t0 + tile) * (2 * kPer) + (from & 1u) * kPer + k];
+                v = data[(uint64_t)(t0 + tile) * (32 * kPer) + from * kPer + k];
+            }
+            // in front of it in the row, too: the other half's values up to this tile, or with it if that is the left one
+            const uint32_t other_bits = (tile + (from & 1u)) * kPer;
+            const uint64_t other = __shfl_sync(0xffffffffu, found, (int)(from ^ 1u)) & (other_bits == 64 ? ~0ull : (1ull << other_bits) - 1);
+            const uint32_t entry = i + __shfl_sync(0xffffffffu, first_entry, (int)from) + (uint32_t)__popcll(other);
+            const uint32_t row_entries = __shfl_sync(0xffffffffu, len, (int)from);
+            const uint32_t first_unit = __shfl_sync(0xffffffffu, unit, (int)from), first_slot = __shfl_sync(0xffffffffu, slot, (int)from);
+            if (i >= n) continue;
+            if (sizeof(T) == 4) v = (T)((uint32_t)v & 0xFFFFE000u);  // as the tensor core reads it
+            const uint32_t n_pieces = pieces_of(row_entries, cap), piece = min(entry >> cap_bits, n_pieces - 1), e = entry - (piece << cap_bits);
+            const uint32_t entries = min(row_entries - (piece << cap_bits), cap), fill = (0u - entries) % kUnitBatch;  // slots before the second entry
+            uint32_t *out = batches + (uint64_t)unit_batch[first_unit + piece] * kWords;
+            // the unit's last batch holds its target, the others none; a batch's first entry writes it
+            auto put = [&](uint32_t e, T value) {
+                uint32_t *words = out + (e / kUnitBatch) * (4 * kWords);
+                words[e % kUnitBatch] = col;
+                if (e % kUnitBatch == 0)
+                    words[kTo] = e / kUnitBatch + 1 < (entries + kUnitBatch - 1) / kUnitBatch ? kNoTarget
+                                 : n_pieces > 1                                              ? kSlotTarget | (first_slot + piece)
+                                                                                             : first_row + (from >> 1);
+                reinterpret_cast<T *>(words + kUnitBatch)[e % kUnitBatch] = value;
+            };
+            T value = v, one;
+            if (!e && fill) {
+                split_value(v, fill, &value, &one);
+                for (uint32_t f = 1; f <= fill; ++f) put(f, one);
+            }
+            put(e ? e + fill : 0u, value);
+        }
+        __syncwarp();
     }
 }
 
@@ -693,8 +806,8 @@ int build_band_units(RowsFormat *f, bool tf32) {
 }
 
 int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOffset, const uint32_t *d_tcA2B,
-                      const void *d_data, const uint32_t *d_rowIdx, bool loose, int n_sms, double max_fill, bool force_rows,
-                      RowsFormat *out, NarrowFormat *narrow) {
+                      const void *d_data, const uint32_t *d_rowIdx, const formatcheck::Found *d_found, formatcheck::Found *found, bool *found_known,
+                      int n_sms, double max_fill, bool force_rows, RowsFormat *out, NarrowFormat *narrow) {
     *out = RowsFormat();
     *narrow = NarrowFormat();
     const uint64_t tiles = info.total_tiles;
@@ -721,25 +834,40 @@ int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
     B200_CUDA_TRY(tmp.alloc(&sums, rows));
     B200_CUDA_TRY(tmp.alloc(&tables, 1));
     B200_CUDA_TRY(tmp.alloc(&totals, 1));
-    auto terms = thrust::make_transform_iterator(thrust::make_counting_iterator<uint32_t>(0), RowTerms{row_len, cap});
-    size_t scan_bytes = 0;
-    B200_CUDA_TRY(cub::DeviceScan::InclusiveScan(nullptr, scan_bytes, terms, sums, AddSums{}, (int64_t)rows));
-    uint8_t *scan_tmp = nullptr;
-    B200_CUDA_TRY(tmp.alloc(&scan_tmp, scan_bytes));
+    RowSums *chunks = nullptr;
+    B200_CUDA_TRY(tmp.alloc(&chunks, kMaxChunks));
+    const uint32_t n_chunks = rows <= kMaxChunks * kChunkRows ? (rows + kChunkRows - 1) / kChunkRows : 0;
+    const Tables look{*found_known ? nullptr : d_found, found->loose()};
 
     const bool f16 = info.elt_size == 2;
     const uint16_t *data16 = static_cast<const uint16_t *>(d_data);
     const uint32_t *data32 = static_cast<const uint32_t *>(d_data);
     const int run_grid = grid_for(n_runs64 * 32), row_grid = (int)(((uint64_t)rows + kBlock - 1) / kBlock);
-    run_windows_kernel<<<(unsigned)((std::max<uint64_t>(eff, rows) + kBlock - 1) / kBlock), kBlock>>>(d_rowOffset, eff, rows, run_window, row_len, tables, totals);
-    if (f16) run_rows_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data16, d_rowIdx, run_window, n_runs, rows, cols, loose, counts);
-    else run_rows_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data32, d_rowIdx, run_window, n_runs, rows, cols, loose, counts);
-    row_lengths_kernel<<<(unsigned)(((uint64_t)eff * 16 + kBlock - 1) / kBlock), kBlock>>>(d_rowOffset, d_rowIdx, eff, rows, cap, counts, row_len, tables, totals);
-    B200_CUDA_TRY(cub::DeviceScan::InclusiveScan(scan_tmp, scan_bytes, terms, sums, AddSums{}, (int64_t)rows));
-    row_totals_kernel<<<1, kBlock>>>(rows, sums, tables, totals);
+    run_windows_kernel<<<(unsigned)((std::max<uint64_t>(eff, rows) + kBlock - 1) / kBlock), kBlock>>>(d_rowOffset, eff, rows, look, run_window, row_len, tables, totals, chunks);
+    if (f16) run_rows_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data16, d_rowIdx, run_window, n_runs, rows, cols, look, counts);
+    else run_rows_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data32, d_rowIdx, run_window, n_runs, rows, cols, look, counts);
+    row_lengths_kernel<<<(unsigned)(((uint64_t)eff * 16 + kBlock - 1) / kBlock), kBlock>>>(d_rowOffset, d_rowIdx, eff, rows, cap, look, counts, row_len, tables, totals,
+                                                                                         chunks, n_chunks);
+    if (n_chunks) {
+        row_sums_kernel<<<n_chunks, kBlock>>>(row_len, rows, cap, look, chunks, sums, tables, totals);
+    } else {
+        auto terms = thrust::make_transform_iterator(thrust::make_counting_iterator<uint32_t>(0), RowTerms{row_len, cap});
+        size_t scan_bytes = 0;
+        B200_CUDA_TRY(cub::DeviceScan::InclusiveScan(nullptr, scan_bytes, terms, sums, AddSums{}, (int64_t)rows));
+        uint8_t *scan_tmp = nullptr;
+        B200_CUDA_TRY(tmp.alloc(&scan_tmp, scan_bytes));
+        B200_CUDA_TRY(cub::DeviceScan::InclusiveScan(scan_tmp, scan_bytes, terms, sums, AddSums{}, (int64_t)rows));
+        row_totals_kernel<<<1, kBlock>>>(rows, look, sums, tables, totals);
+    }
     B200_CUDA_TRY(cudaGetLastError());
     RowTotals h;
     B200_CUDA_TRY(cudaMemcpy(&h, totals, sizeof(h), cudaMemcpyDeviceToHost));
+    if (!*found_known) {
+        *found = h.found;
+        *found_known = true;
+        if (found->bad()) return B200SPMM_OK;  // (the caller refuses them)
+    }
+    const bool loose = found->loose();
     if (!force_rows && (double)h.entries > max_fill * (double)tiles * 16.0 * info.col_window) {
         if (narrow_pays(h.entries, rows, info.cols, h.max_len, n_sms))
             return build_narrow(info, h.entries, d_rowOffset, d_tcA2B, d_data, d_rowIdx, n_sms, run_window, n_runs, run_grid, counts, sums, narrow);
@@ -772,12 +900,14 @@ int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
         return B200SPMM_OK;
     }
     B200_CUDA_TRY(e);
+    uint32_t cap_bits = 0;  // (a power of two)
+    while ((1u << cap_bits) < cap) ++cap_bits;
     place_units_kernel<<<row_grid, kBlock>>>(row_len, rows, cap, sums, tables, totals, f.d_units, unit_batch, f.d_splits, f.d_batches, words);
     if (f16)
-        write_entries_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data16, d_rowIdx, run_window, n_runs, rows, cols, loose, cap, counts,
+        write_entries_kernel<uint16_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data16, d_rowIdx, run_window, n_runs, rows, cols, loose, cap_bits, counts,
                                                              row_len, sums, unit_batch, f.d_batches);
     else
-        write_entries_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data32, d_rowIdx, run_window, n_runs, rows, cols, loose, cap, counts,
+        write_entries_kernel<uint32_t><<<run_grid, kBlock>>>(d_rowOffset, d_tcA2B, data32, d_rowIdx, run_window, n_runs, rows, cols, loose, cap_bits, counts,
                                                              row_len, sums, unit_batch, f.d_batches);
     B200_CUDA_TRY(cudaGetLastError());
     B200_CUDA_TRY(cudaDeviceSynchronize());

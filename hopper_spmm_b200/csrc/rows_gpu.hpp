@@ -57,13 +57,30 @@ struct NarrowFormat {
     uint32_t n_blocks = 0, n_ctas = 0, max_rows = 0;  // max_rows: of one CTA
 };
 
+// What a look over the tables of a caller's format finds (tables_kernel in capi.cu).
+namespace formatcheck {
+
+enum : uint32_t { kBadTables = 1u, kLooseLists = 2u };
+
+struct Found {
+    uint32_t flags;
+    int32_t falls;  // places where a column is not above the one before it, less those where a window starts
+    __host__ __device__ bool bad() const { return (flags & kBadTables) != 0; }
+    __host__ __device__ bool loose() const { return flags || falls; }
+};
+
+}  // namespace formatcheck
+
 // Builds what the kernels outside the tile path want from a matrix: row units when `force_rows` or when at most
 // max_fill of the tiles' slots are in use, and the format for narrow B where it fits (at most 65,536 columns, rows
 // of some length, none so long that CTAs of whole rows could not be balanced).  The tiles must be in the reference's layout
-// (row-major 16 x CW); `loose`: slots without a column may lie anywhere in a window, and not only in its last tile.  A format stays empty when device memory is short.
+// (row-major 16 x CW).  `found`: of the tables; loose: slots without a column may lie anywhere in a window, and not only in its last
+// tile.  While a look over them is still under way it writes d_found, and *found is set from that unless *found_known says that it
+// already is: on return it does, if the host had to wait for the device.  Nothing is built from bad tables.  A format stays empty
+// when device memory is short.
 int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOffset, const uint32_t *d_tcA2B,
-                      const void *d_data, const uint32_t *d_rowIdx, bool loose, int n_sms, double max_fill, bool force_rows,
-                      RowsFormat *rows, NarrowFormat *narrow);
+                      const void *d_data, const uint32_t *d_rowIdx, const formatcheck::Found *d_found, formatcheck::Found *found, bool *found_known,
+                      int n_sms, double max_fill, bool force_rows, RowsFormat *rows, NarrowFormat *narrow);
 // The list of the bands, where there are several and no list yet: only calls that copy C out band by band need it, and it is 8
 // bytes a row.  Waits for the device.  Stays empty when device memory is short; then everything is one band.
 int build_band_units(RowsFormat *f, bool tf32);

@@ -136,3 +136,24 @@ def test_bad_tables_are_refused(what):
     with pytest.raises(capi.SpmmError) as e:
         make_plan(info, a)
     assert e.value.status == capi.ERR_INVALID_ARG
+
+
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+@pytest.mark.parametrize("shift", [8, 12, 15])
+def test_windows_across_the_chunks_of_the_row_sums(dt, shift):
+    # windows off the grid of 16 rows: some have rows on both sides of a multiple of 1,024, and far apart windows share a warp
+    rng, rows, cols = np.random.default_rng(shift), 6000, 900
+    lengths = rng.integers(0, 5, rows)
+    lengths[1500:4600] = 0
+    lengths[[1007, 1012, 1016]] = [300, 65, 900]
+    ci = np.concatenate([np.sort(rng.choice(cols, k, replace=False)) for k in lengths]).astype(np.uint32)
+    rp, v = np.concatenate([[0], np.cumsum(lengths)]).astype(np.uint32), rng.uniform(0.1, 1, ci.size).astype(dt)
+    f = hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v))
+    info = capi.BtcfInfo()
+    for k in ("cols", "nnzs", "total_row_windows", "eff_row_windows", "total_tiles", "row_window", "col_window"):
+        setattr(info, k, getattr(f, k))
+    info.rows = rows + shift
+    info.dtype, info.elt_size = (capi.F16, 2) if dt == np.float16 else (capi.TF32, 4)
+    a = {k: np.array(getattr(f, k)) for k in ("rowOffset", "tcA2B", "data", "rowIdx")}
+    a["rowIdx"] = a["rowIdx"] + np.uint32(shift)
+    check(info, a, np.concatenate([np.zeros(shift, np.uint32), rp]), ci, v, 40, True)

@@ -296,3 +296,34 @@ def test_the_list_of_the_bands_is_made_for_the_first_host_call():
     finally:
         plan.close()
         f.close()
+
+
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+@pytest.mark.parametrize("rows", [1023, 1024, 1025, 3000, 262144, 262145])
+def test_running_sums_at_the_edges_of_their_chunks(dt, rows, monkeypatch):
+    # chunks of 1,024 rows, as many of them as the one pass takes and one row more; rows of many pieces beside each other, at a
+    # chunk's edge and at the end, windows without rows, and a window whose runs are full: the most entries that a warp lists
+    import torch
+    monkeypatch.setenv("B200SPMM_WINDOW", "rows")
+    rng, cols = np.random.default_rng(rows), 5003
+    lengths = rng.integers(0, 4, rows)
+    lengths[100:180] = 0
+    lengths[[5, 6, 511, 1022, rows - 1]] = [5003, 4096, 4097, 65, 2049]
+    lengths[192:208] = 700
+    ci = np.concatenate([np.arange(k) + 3 if 192 <= r < 208 else np.sort(rng.choice(cols, k, replace=False)) if k > 3 else
+                         np.arange(k) * 1000 + r % 1000 for r, k in enumerate(lengths)]).astype(np.uint32)
+    rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.uint32)
+    v, B = rng.uniform(0.1, 1, ci.size).astype(dt), dense_b(cols, 8, 9, dt)
+    dB = torch.from_numpy(B).cuda()
+    plan = hs.SpmmPlan(hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    dev = hs.DeviceBtcf(rows, cols, *(torch.from_numpy(a).cuda() for a in (rp.view(np.int32), ci.view(np.int32), v)))
+    plan_dev = hs.SpmmPlan(dev)  # its tables are looked over while the units are made
+    try:
+        C_out = plan.spmm(dB)
+        assert plan.launch_info().stages == 0
+        parity.check(C_out.cpu().numpy(), rows, rp, ci, v, B)
+        assert torch.equal(plan_dev.spmm(dB), C_out)
+    finally:
+        plan.close()
+        plan_dev.close()
+        dev.close()
