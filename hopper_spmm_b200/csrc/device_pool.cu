@@ -45,50 +45,82 @@ cudaError_t pool_of(int device, cudaMemPool_t *out) {
 std::mutex g_large_lock;
 std::unordered_set<void *> g_large;  // the driver's own buffers: of kPoolMaxBytes and more, or allocated under a capture
 
+// What an upload uses; the next one finds it there.
+struct Staging {
+    char *pinned = nullptr;  // [kUploadThreads][2][kUploadChunk]
+    int device = -1;         // of the streams and events
+    cudaStream_t stream[kUploadThreads] = {};
+    cudaEvent_t done[kUploadThreads][2] = {};
+    void release_streams() {
+        for (int t = 0; t < kUploadThreads; ++t) {
+            for (cudaEvent_t &d : done[t]) {
+                if (d) cudaEventDestroy(d);
+                d = nullptr;
+            }
+            if (stream[t]) cudaStreamDestroy(stream[t]);
+            stream[t] = nullptr;
+        }
+        device = -1;
+    }
+    void release() {
+        release_streams();
+        if (pinned) cudaFreeHost(pinned);
+        pinned = nullptr;
+    }
+    // For the current device.  Leaves nothing behind when it fails.
+    cudaError_t open(int current) {
+        cudaError_t e = cudaSuccess;
+        if (!pinned) e = cudaHostAlloc(reinterpret_cast<void **>(&pinned), kUploadThreads * 2 * kUploadChunk, cudaHostAllocPortable);
+        if (e != cudaSuccess) pinned = nullptr;
+        if (e == cudaSuccess && device != current) {
+            release_streams();
+            for (int t = 0; t < kUploadThreads && e == cudaSuccess; ++t) {
+                e = cudaStreamCreateWithFlags(&stream[t], cudaStreamNonBlocking);
+                for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&done[t][k], cudaEventDisableTiming);
+            }
+            device = current;
+        }
+        if (e != cudaSuccess) release();
+        return e;
+    }
+};
 std::mutex g_staging_lock;
-void *g_staging = nullptr;  // [kUploadThreads][2][kUploadChunk] pinned bytes
+Staging g_staging;
 
 }  // namespace
 
 cudaError_t upload_pageable(void *dst, const void *src, size_t bytes) {
     std::unique_lock<std::mutex> guard(g_staging_lock, std::defer_lock);
     if (bytes < 4 * kUploadChunk || !guard.try_lock()) return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
-    if (!g_staging && cudaHostAlloc(&g_staging, kUploadThreads * 2 * kUploadChunk, cudaHostAllocPortable) != cudaSuccess) {
-        cudaGetLastError();
-        g_staging = nullptr;
-        return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
-    }
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // whatever was queued before the copy is done before it
+    if (e != cudaSuccess) return e;
+    if (g_staging.open(device) != cudaSuccess) {
+        cudaGetLastError();
+        return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    }
+    e = cudaStreamSynchronize(nullptr);  // whatever was queued before the copy is done before it
     if (e != cudaSuccess) return e;
     std::atomic<size_t> next{0};
     std::atomic<int> failed{(int)cudaSuccess};
     auto worker = [&](int t) {
-        cudaStream_t stream = nullptr;
-        cudaEvent_t done[2] = {nullptr, nullptr};
         auto ok = [&](cudaError_t r) {
             if (r != cudaSuccess) failed = (int)r;
             return r == cudaSuccess;
         };
-        if (ok(cudaSetDevice(device)) && ok(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking)) &&
-            ok(cudaEventCreateWithFlags(&done[0], cudaEventDisableTiming)) && ok(cudaEventCreateWithFlags(&done[1], cudaEventDisableTiming))) {
-            for (int k = 0; failed == (int)cudaSuccess; k ^= 1) {
-                const size_t at = next.fetch_add(kUploadChunk);
-                if (at >= bytes) break;
-                const size_t n = std::min(kUploadChunk, bytes - at);
-                char *buf = static_cast<char *>(g_staging) + (size_t)(2 * t + k) * kUploadChunk;
-                if (!ok(cudaEventSynchronize(done[k]))) break;  // (at once for an event never recorded)
-                std::memcpy(buf, static_cast<const char *>(src) + at, n);
-                if (!ok(cudaMemcpyAsync(static_cast<char *>(dst) + at, buf, n, cudaMemcpyHostToDevice, stream)) ||
-                    !ok(cudaEventRecord(done[k], stream)))
-                    break;
-            }
-            ok(cudaStreamSynchronize(stream));
+        if (!ok(cudaSetDevice(device))) return;
+        for (int k = 0; failed == (int)cudaSuccess; k ^= 1) {
+            const size_t at = next.fetch_add(kUploadChunk);
+            if (at >= bytes) break;
+            const size_t n = std::min(kUploadChunk, bytes - at);
+            char *buf = g_staging.pinned + (size_t)(2 * t + k) * kUploadChunk;
+            if (!ok(cudaEventSynchronize(g_staging.done[t][k]))) break;  // (at once for one not recorded since the last upload)
+            std::memcpy(buf, static_cast<const char *>(src) + at, n);
+            if (!ok(cudaMemcpyAsync(static_cast<char *>(dst) + at, buf, n, cudaMemcpyHostToDevice, g_staging.stream[t])) ||
+                !ok(cudaEventRecord(g_staging.done[t][k], g_staging.stream[t])))
+                break;
         }
-        for (cudaEvent_t d : done)
-            if (d) cudaEventDestroy(d);
-        if (stream) cudaStreamDestroy(stream);
+        ok(cudaStreamSynchronize(g_staging.stream[t]));
     };
     std::vector<std::thread> pool;
     pool.reserve(kUploadThreads);
@@ -151,8 +183,7 @@ void pool_free(void *ptr, cudaStream_t stream) {
 cudaError_t pool_release(int device) {
     {
         std::lock_guard<std::mutex> guard(g_staging_lock);
-        if (g_staging) cudaFreeHost(g_staging);
-        g_staging = nullptr;
+        g_staging.release();
     }
     cudaMemPool_t pool = nullptr;
     {

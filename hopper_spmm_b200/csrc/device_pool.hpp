@@ -39,7 +39,9 @@ cudaError_t pool_alloc(T **out, size_t count, cudaStream_t stream = nullptr) {
 
 // Copies `bytes` from pageable host memory to the current device and waits for it.  The driver's own copy moves 11
 // GB/s, one thread filling its staging buffer; here kUploadThreads threads fill pinned buffers of their own (16 MB
-// in all, kept for the next upload until b200spmm_release_cached_memory), which keeps the link at 40-50 GB/s.
+// in all) over streams of their own, which keeps the link at 40-50 GB/s.  Buffers, streams and events are kept for the next
+// upload until b200spmm_release_cached_memory, the latter for one device at a time: made anew they were 0.8 of the 5.0 ms that the
+// plan of a matrix of 108 MB took.  8 or 12 threads are no faster.
 // Small copies, and uploads while another one holds the buffers, go the driver's way.
 constexpr int kUploadThreads = 4;
 constexpr size_t kUploadChunk = (size_t)2 << 20;

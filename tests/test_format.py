@@ -316,3 +316,22 @@ def test_column_major_tiles_of_the_transposed_build(dt, rw):
     assert capi.lib().b200spmm_plan_create(f._h, 0, 0, C.byref(p)) == capi.ERR_UNSUPPORTED
     hs.transpose_tiles(f)
     assert not f.col_major_tiles and np.array_equal(np.asarray(f.data).view(bits), row_major.view(bits))
+
+
+@pytest.mark.parametrize("dt,rw,cw", [(np.float16, 16, 16), (np.float32, 8, 4)])
+@pytest.mark.parametrize("cols,per_row", [(64, 9), (65536, 700), (65537, 700), (65537, 3), (300000, 5)])
+def test_places_by_table_by_bits_and_by_search(dt, rw, cw, cols, per_row):
+    # the most columns that a table of places takes and one more; above that a window dense enough for a bit set and a sparse one
+    rng = np.random.default_rng(cols + per_row)
+    lengths = rng.integers(0, 2 * per_row, 70)
+    lengths[16:32] = 0
+    ci = np.concatenate([np.append(np.sort(rng.choice(cols - 1, max(k - 1, 0), replace=False)), [cols - 1] if k else []) for k in lengths]).astype(np.uint32)
+    rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.uint32)
+    v = rng.uniform(0.1, 1, ci.size).astype(dt)
+    assert same_format(convert(70, cols, rp, ci, v, rw, cw), oracle.csr2btcf_nobitmap(70, cols, rp, ci, v, rw, cw))
+    for at in (0, ci.size // 2, ci.size - 1):  # a column out of range in the first, a middle and the last window
+        bad = ci.copy()
+        bad[at] = cols
+        with pytest.raises(capi.SpmmError) as e:
+            convert(70, cols, rp, bad, v, rw, cw)
+        assert e.value.status == capi.ERR_BAD_CSR
