@@ -343,6 +343,8 @@ def run_other_workload(name, dev, steps, warmup, hbm_gbs, f16_tflops, tf32_tflop
         tinfo = capi_mod().BtcfInfo()
         getattr(lib, "b200spmm_plan_tall_info" if win == 128 else "b200spmm_plan_pair_info")(plan._p, ctypes.byref(tinfo))
         ex_tiles = int(tinfo.total_tiles)
+        if win == 256 and int(info.stages) == 4:  # the 2:4 form (dense tiles: six stages) leaves out two products of four
+            ex_tiles /= 2
     slab = int(info.feature_slab)
     rec["executed_mma_gflop"] = 2.0 * ex_tiles * win * btcf.col_window * (int(info.n_slabs) * slab) / 1e9
     rec["executed_mma_tflops"] = rec["executed_mma_gflop"] / ms

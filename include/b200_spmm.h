@@ -117,7 +117,7 @@ void b200spmm_btcf_destroy(b200spmm_btcf_t *f);
 
 /*
  * The same conversion on the GPU, for CSR arrays that already live on `device`; output arrays
- * stay on the device (hand them to b200spmm_plan_create_device).  Bit-identical to
+ * stay on the device (hand them to b200spmm_plan_create_device), up to 64 MB of them allocated ahead of their final size.  Bit-identical to
  * b200spmm_csr2btcf_nobitmap - and so to src/utils/convert.h:146-225 - for rows whose columns are
  * ascending and distinct, which is what the reference's loader produces (src/utils/load.h:137-145);
  * anything else is refused with B200SPMM_ERR_BAD_CSR.  Synchronous with respect to `stream`.
@@ -464,7 +464,8 @@ int b200spmm_plan_tall_copy_to_host(const b200spmm_plan_t *p, uint32_t *rowOffse
  * features: a pair of CTAs on neighbouring SMs (a cluster of two) then shares one MMA of 256 window rows x
  * 256 features, each CTA holding half of either operand, which halves what an SM fetches of B per tile.
  * Kept when the 256-row windows have at most 0.55 of the 128-row tiles (B200SPMM_WINDOW=256 forces it,
- * =128 keeps it out).  The two calls below are the counterparts of the two above for that copy
+ * =128 keeps it out).  fp16 plans of 20,000 and more such tiles keep them in the tensor core's 2:4 form as well and
+ * multiply whole windows in that (B200SPMM_SPARSE24=0 keeps it out, =1 asks for it wherever it fits).  The two calls below are the counterparts of the two above for that copy
  * (row_window 256, or 0 when the plan has none).
  */
 int b200spmm_plan_pair_info(const b200spmm_plan_t *p, b200spmm_btcf_info_t *info);
