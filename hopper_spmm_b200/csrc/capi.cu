@@ -1258,10 +1258,11 @@ int plan_finish(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_t *h
             // (an eighth of the short tiles is the least that merging eight windows can leave)
             if (fill / (8.0 * ratio) < kTallMinFill || info.total_tiles < kRowsWideAnyTiles) max_fill = kRowsMaxFillWide;
         }
-        int st = build_row_formats(info, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, checked ? tables_found(p) : nullptr, &found, &found_known,
-                                   p->n_sms, max_fill, force_rows, &p->rows_fmt, &p->narrow);
-        if (st == B200SPMM_OK) st = wait_for_check();
+        const int built = build_row_formats(info, p->d_rowOffset, p->d_tcA2B, p->d_data, p->d_rowIdx, checked ? tables_found(p) : nullptr, &found, &found_known,
+                                            p->n_sms, max_fill, force_rows, &p->rows_fmt, &p->narrow);
+        const int st = wait_for_check();  // (bad tables are refused as such, whatever became of the row units)
         if (st != B200SPMM_OK) return st;
+        if (built != B200SPMM_OK) return built;
         p->rows_only = p->rows_fmt.n_units > 0;
         if (p->rows_only) return B200SPMM_OK;
     }

@@ -811,8 +811,9 @@ int build_row_formats(const b200spmm_btcf_info_t &info, const uint32_t *d_rowOff
     *out = RowsFormat();
     *narrow = NarrowFormat();
     const uint64_t tiles = info.total_tiles;
-    // (the product is refused for more columns, and the running sums of entries are 32-bit)
-    if (!info.eff_row_windows || !tiles || info.rows >= kSlotTarget || info.cols > 0x7FFFFFFFull || info.nnzs > 0xFFFFFFFFull) return B200SPMM_OK;
+    // (the product is refused for more columns, and the running sums of entries are 32-bit; a caller's tables may name windows of a
+    // matrix without rows, which the look over them refuses)
+    if (!info.rows || !info.eff_row_windows || !tiles || info.rows >= kSlotTarget || info.cols > 0x7FFFFFFFull || info.nnzs > 0xFFFFFFFFull) return B200SPMM_OK;
     const uint32_t rows = (uint32_t)info.rows, cols = (uint32_t)info.cols, eff = (uint32_t)info.eff_row_windows;
     const uint32_t cap = unit_entries_for(info.nnzs, info.rows, n_sms);
     RowsFormat f;

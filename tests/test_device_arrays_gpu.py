@@ -138,6 +138,20 @@ def test_bad_tables_are_refused(what):
     assert e.value.status == capi.ERR_INVALID_ARG
 
 
+@pytest.mark.parametrize("kind", ["units", "tiles"])
+@pytest.mark.parametrize("window", [None, "rows", "16"])
+def test_windows_of_a_matrix_without_rows_are_refused(kind, window, monkeypatch):
+    # by the look over the tables alone: nothing is summed up over rows that are not there
+    if window:
+        monkeypatch.setenv("B200SPMM_WINDOW", window)
+    info, a = arrays(*matrix(kind, np.float16))
+    for rows in (0, 16):  # none, and as many as the first window has
+        info.rows = rows
+        with pytest.raises(capi.SpmmError) as e:
+            make_plan(info, a)
+        assert e.value.status == capi.ERR_INVALID_ARG
+
+
 @pytest.mark.parametrize("dt", [np.float16, np.float32])
 @pytest.mark.parametrize("shift", [8, 12, 15])
 def test_windows_across_the_chunks_of_the_row_sums(dt, shift):
