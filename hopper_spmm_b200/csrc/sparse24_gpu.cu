@@ -9,8 +9,11 @@
 // row that meets the infinity must keep it: idle places name columns that the row has no entry in, which the dense tile
 // multiplies by zero, too.  There are always enough of them.
 //
-//   1. tiles_kernel: a block takes kBlockTiles tiles of a window and a thread a row.  What goes to the rest is collected block by block
-//   2. rest_kernel: the blocks' entries of a row one after the other
+//   1. tiles_kernel: a block takes kBlockTiles tiles of a window and a thread a row.  It marks the entries that go to the rest in
+//      shared memory and, when it knows how many they are, asks for places in the row's list
+//   2. rest_kernel: blocks have asked in any order; every row's list is sorted by column
+// Only the length of a row's list is limited (kSparse24MaxRest).  With a limit of seven for every 16 tiles of a row as well,
+// one row-block of 2.5e-7 decided for the whole matrix: one 28672 x 8192 weight of ten at 10 %, 45 of a hundred at 10.9 %.
 // Bound by reading the dense tiles.
 #include <algorithm>
 #include <vector>
@@ -25,18 +28,12 @@ namespace {
 
 constexpr int kRows = 256;            // of a window, and threads of a block
 constexpr uint32_t kBlockTiles = 16;  // of 32 columns
-constexpr uint32_t kBlockRest = 7;    // entries of a row that a block may collect
 // Entries of the rest a row and dense tile, up to which the form pays: the epilogue warps get through 0.02 while the tensor core
 // does a tile.  28672 x 8192, us, dense and so: 10 % (0.015), 192 / 2,048 columns 105 / 772 and 89 / 661; 12 % (0.025) 113 / 690
 // and 111 / 678; 14 % (0.038) 113 / 692 and 137 / 882.
 constexpr double kMostRest = 0.02;
 
-struct Collected {
-    uint32_t *n;       // [blocks][256]
-    uint32_t *entry;   // [blocks][kBlockRest][256]
-    unsigned long long *total;  // entries, and whether some row has too many
-};
-constexpr unsigned long long kUnfit = 1ull << 63;
+constexpr unsigned long long kUnfit = 1ull << 63;  // in the number of all entries of the rest: some row has too many
 
 struct Row {
     uint32_t w[8];  // sixteen fp16
@@ -54,12 +51,12 @@ struct Row {
 
 __global__ void __launch_bounds__(kRows)
 tiles_kernel(const uint32_t *__restrict__ denseOffset, const uint32_t *__restrict__ dense_lists, const uint4 *__restrict__ dense,
-             const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ quads, uint32_t blocks, uint32_t *__restrict__ lists,
-             uint4 *__restrict__ data, uint16_t *__restrict__ meta, Collected rest) {
+             const uint32_t *__restrict__ rowOffset, const uint32_t *__restrict__ quads, uint32_t *__restrict__ lists, uint4 *__restrict__ data,
+             uint16_t *__restrict__ meta, uint32_t *__restrict__ n_rest, uint32_t *__restrict__ rest, unsigned long long *__restrict__ total) {
+    __shared__ uint32_t beyond[kBlockTiles][kRows];  // columns of a row and tile that go to the rest
     const uint32_t w = blockIdx.x, first = denseOffset[w], n = denseOffset[w + 1] - first, out = rowOffset[w], n_out = rowOffset[w + 1] - out;
     const uint32_t k0 = blockIdx.y * kBlockTiles, k1 = min(k0 + kBlockTiles, n_out), half = threadIdx.x >> 7, r = threadIdx.x & 127u, flip = (r >> 2) & 1u;
-    const uint64_t block = (uint64_t)w * blocks + blockIdx.y;
-    uint32_t n_rest = 0;
+    uint32_t n_mine = 0;
     const uint32_t *list = dense_lists + (uint64_t)first * 16u;
     if (k0 < k1) {
         for (uint32_t k = k0 * 32u + threadIdx.x; k < k1 * 32u; k += kRows) lists[(uint64_t)out * 32u + k] = k < n * 16u ? list[k] : kIdxMax;
@@ -69,7 +66,7 @@ tiles_kernel(const uint32_t *__restrict__ denseOffset, const uint32_t *__restric
         uint16_t *m_to = meta + ((uint64_t)quads[w] * 2 + half * (quads[w + 1] - quads[w])) * 1024u + ((r >> 4) * 16u + (r & 7u)) * 8u + (r >> 3 & 1u);
 #pragma unroll 2
         for (uint32_t k = k0; k < k1; ++k) {
-            uint32_t v[8] = {}, m[2] = {0x4444u, 0x4444u};
+            uint32_t v[8] = {}, m[2] = {0x4444u, 0x4444u}, over = 0;
 #pragma unroll
             for (uint32_t h = 0; h < 2; ++h) {
                 const uint32_t t = 2 * k + h;
@@ -81,13 +78,8 @@ tiles_kernel(const uint32_t *__restrict__ denseOffset, const uint32_t *__restric
                 for (int g = 0; g < 4; ++g) {
                     const uint32_t met = row.mask(g);
                     uint32_t have = met;
-                    while (__popc(have) > 2) {
-                        const uint32_t c = (uint32_t)__ffs((int)have) - 1u;
-                        have &= have - 1u;
-                        if (n_rest < kBlockRest)
-                            rest.entry[(block * kBlockRest + n_rest) * kRows + threadIdx.x] = list[t * 16u + g * 4u + c] << 16 | row.value(g, c);
-                        ++n_rest;
-                    }
+                    while (__popc(have) > 2) have &= have - 1u;
+                    over |= (met ^ have) << (16 * h + 4 * g);
                     uint32_t two = have, idle = ~met & 15u;
                     while (__popc(two) < 2) {
                         two |= idle & (0u - idle);
@@ -103,29 +95,42 @@ tiles_kernel(const uint32_t *__restrict__ denseOffset, const uint32_t *__restric
             uint16_t *mk = m_to + (uint64_t)(k / 4) * 1024u + (k & 3u) * 2u;
             mk[0] = (uint16_t)m[0];
             mk[64] = (uint16_t)m[1];
+            beyond[k - k0][threadIdx.x] = over;
+            n_mine += (uint32_t)__popc(over);
+        }
+        if (n_mine) {
+            uint32_t at = atomicAdd(n_rest + (uint64_t)w * kRows + threadIdx.x, n_mine);
+            const uint16_t *values = reinterpret_cast<const uint16_t *>(from + 2 * r);
+            for (uint32_t k = k0; k < k1; ++k)
+                for (uint32_t over = beyond[k - k0][threadIdx.x]; over; over &= over - 1u, ++at) {
+                    const uint32_t in_tile = (uint32_t)__ffs((int)over) - 1u, c = in_tile & 15u;
+                    const uint64_t t = 2 * k + (in_tile >> 4);
+                    if (at < kSparse24MaxRest)
+                        rest[((uint64_t)w * kSparse24MaxRest + at) * kRows + threadIdx.x] =
+                            list[t * 16u + c] << 16 | values[t * 2048 + ((c >> 3) ^ flip) * 8u + (c & 7u)];
+                }
         }
     }
-    rest.n[block * kRows + threadIdx.x] = n_rest;
-    const uint32_t sum = __reduce_add_sync(0xffffffffu, n_rest);
-    const bool unfit = __any_sync(0xffffffffu, n_rest > kBlockRest);
-    if ((threadIdx.x & 31u) == 0 && (sum || unfit)) {
-        if (unfit) atomicOr(rest.total, kUnfit);
-        else atomicAdd(rest.total, (unsigned long long)sum);
-    }
+    const uint32_t sum = __reduce_add_sync(0xffffffffu, n_mine);
+    if ((threadIdx.x & 31u) == 0 && sum) atomicAdd(total, (unsigned long long)sum);
 }
 
 __global__ void __launch_bounds__(kRows)
-rest_kernel(uint32_t blocks, Collected rest, uint32_t *__restrict__ n_rest, uint32_t *__restrict__ out) {
-    const uint32_t w = blockIdx.x;
-    uint32_t at = 0;
-    for (uint32_t b = 0; b < blocks; ++b) {
-        const uint64_t block = (uint64_t)w * blocks + b;
-        const uint32_t n = min(rest.n[block * kRows + threadIdx.x], kBlockRest);
-        for (uint32_t i = 0; i < n; ++i, ++at)
-            if (at < kSparse24MaxRest) out[((uint64_t)w * kSparse24MaxRest + at) * kRows + threadIdx.x] = rest.entry[(block * kBlockRest + i) * kRows + threadIdx.x];
+rest_kernel(const uint32_t *__restrict__ n_rest, uint32_t *__restrict__ rest, unsigned long long *__restrict__ total) {
+    __shared__ uint32_t sorted[kSparse24MaxRest][kRows];
+    const uint32_t r = threadIdx.x, n = n_rest[(uint64_t)blockIdx.x * kRows + r];
+    uint32_t *list = rest + (uint64_t)blockIdx.x * (kSparse24MaxRest * kRows) + r;
+    if (n > kSparse24MaxRest) {
+        atomicOr(total, kUnfit);
+        return;
     }
-    n_rest[(uint64_t)w * kRows + threadIdx.x] = min(at, kSparse24MaxRest);
-    if (at > kSparse24MaxRest) atomicOr(rest.total, kUnfit);
+    for (uint32_t i = 0; i < n; ++i) {
+        const uint32_t entry = list[i * kRows];
+        uint32_t at = i;
+        for (; at && sorted[at - 1][r] > entry; --at) sorted[at][r] = sorted[at - 1][r];
+        sorted[at][r] = entry;
+    }
+    for (uint32_t i = 0; i < n; ++i) list[i * kRows] = sorted[i][r];
 }
 
 }  // namespace
@@ -155,11 +160,6 @@ int build_sparse24(const TallFormat &pair, uint64_t cols, bool always, Sparse24F
     }
     f.tiles = rowOffset[n_windows];
     const uint32_t blocks = (longest + kBlockTiles - 1) / kBlockTiles;
-    PoolScratch tmp;
-    Collected rest{};
-    cudaError_t e = tmp.alloc(&rest.n, n_windows * blocks * kRows);
-    if (e == cudaSuccess) e = tmp.alloc(&rest.entry, n_windows * blocks * kRows * kBlockRest);
-    if (e == cudaSuccess) e = tmp.alloc(&rest.total, 1);
     // all in one buffer, which is the driver's own where it is large (new memory costs the pool more)
     size_t bytes = 0;
     auto place = [&](size_t n) {
@@ -168,8 +168,8 @@ int build_sparse24(const TallFormat &pair, uint64_t cols, bool always, Sparse24F
         return at;
     };
     const size_t data_at = place(f.tiles * 8192), meta_at = place((size_t)quads[n_windows] * 4096), lists_at = place(f.tiles * 128),
-                 n_rest_at = place(n_windows * kRows * 4), rest_at = place(n_windows * kRows * kSparse24MaxRest * 4), tables_at = place(tables.size() * 4);
-    if (e == cudaSuccess) e = pool_alloc_bytes(&f.d_data, bytes, nullptr);
+                 n_rest_at = place(n_windows * kRows * 4), total_at = place(8), rest_at = place(n_windows * kRows * kSparse24MaxRest * 4), tables_at = place(tables.size() * 4);
+    const cudaError_t e = pool_alloc_bytes(&f.d_data, bytes, nullptr);
     if (e == cudaErrorMemoryAllocation) {  // no room: the dense tiles still work
         cudaGetLastError();
         return B200SPMM_OK;
@@ -183,14 +183,15 @@ int build_sparse24(const TallFormat &pair, uint64_t cols, bool always, Sparse24F
     f.d_rowOffset = reinterpret_cast<uint32_t *>(base + tables_at);
     f.d_quads = f.d_rowOffset + n_windows + 1;
     B200_CUDA_TRY(cudaMemcpy(f.d_rowOffset, tables.data(), tables.size() * 4, cudaMemcpyHostToDevice));
-    B200_CUDA_TRY(cudaMemsetAsync(rest.total, 0, 8));
+    auto *d_total = reinterpret_cast<unsigned long long *>(base + total_at);
+    B200_CUDA_TRY(cudaMemsetAsync(base + n_rest_at, 0, total_at + 8 - n_rest_at));
     tiles_kernel<<<dim3((unsigned)n_windows, blocks), kRows>>>(pair.d_rowOffset, pair.d_tcA2B, static_cast<const uint4 *>(pair.d_data), f.d_rowOffset,
-                                                               f.d_quads, blocks, f.d_tcA2B, static_cast<uint4 *>(f.d_data),
-                                                               static_cast<uint16_t *>(f.d_meta), rest);
-    rest_kernel<<<(unsigned)n_windows, kRows>>>(blocks, rest, f.d_n_rest, f.d_rest);
+                                                               f.d_quads, f.d_tcA2B, static_cast<uint4 *>(f.d_data), static_cast<uint16_t *>(f.d_meta),
+                                                               f.d_n_rest, f.d_rest, d_total);
+    rest_kernel<<<(unsigned)n_windows, kRows>>>(f.d_n_rest, f.d_rest, d_total);
     B200_CUDA_TRY(cudaGetLastError());
     unsigned long long total = 0;
-    B200_CUDA_TRY(cudaMemcpy(&total, rest.total, 8, cudaMemcpyDeviceToHost));
+    B200_CUDA_TRY(cudaMemcpy(&total, d_total, 8, cudaMemcpyDeviceToHost));
     if ((total & kUnfit) || (!always && (double)total > kMostRest * (double)kRows * (double)pair.tiles)) return B200SPMM_OK;
     *out = f;
     guard.f = nullptr;

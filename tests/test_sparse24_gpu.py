@@ -158,3 +158,27 @@ def test_large_pruned_matrices_take_it_by_themselves(monkeypatch):
     assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
     rp, ci, v = csr.numpy()
     parity.check_rows(torch.cat([got[0][:300], got[0][-300:]]).cpu().numpy(), rp, ci, v, B.cpu().numpy(), [(0, 300), (csr.rows - 300, csr.rows)])
+
+
+@pytest.mark.parametrize("surplus,at", [(8, 64), (20, 64), (20, 484), (48, 0), (48, 496), (48, 1400)])
+def test_what_goes_to_the_rest_may_lie_close_together(surplus, at, monkeypatch):
+    # whole groups of four in some rows, two of each in the rest, in one block of 16 tiles (512 columns) or across two; every
+    # column in every window, so that groups of the lists are groups of columns
+    import torch
+    rows, cols, n = 300, 1500, 136
+    mask = np.random.default_rng(surplus).random((rows, cols)) < 0.02
+    mask[np.arange(cols) % 60, np.arange(cols)] = mask[260 + np.arange(cols) % 40, np.arange(cols)] = True
+    for r in (70, 133, 255):
+        mask[r] = False
+        mask[r, at:at + 2 * surplus] = True
+    rp = np.concatenate([[0], np.cumsum(mask.sum(1))]).astype(np.uint32)
+    ci = np.nonzero(mask)[1].astype(np.uint32)
+    rng = np.random.default_rng(3)
+    v = rng.choice(np.array([-3, -2, -1, 1, 2, 3], np.float16), ci.size)
+    B = torch.from_numpy(rng.integers(-4, 5, (cols, n)).astype(np.float16)).cuda()
+    f = hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v))
+    got = product(monkeypatch, f, B, True)
+    assert torch.equal(got, product(monkeypatch, f, B, False))
+    dense = np.zeros((rows, cols))
+    dense[np.repeat(np.arange(rows), np.diff(rp.astype(np.int64))), ci] = v
+    assert torch.equal(got.cpu().double(), torch.from_numpy(dense) @ B.cpu().double())
