@@ -124,6 +124,7 @@ struct b200spmm_plan {
     std::vector<void *> outgrown;
     // The kernel of single warps may take launches (windows_fit), or has to (windows_forced: B200SPMM_WINDOW=warps).
     uint32_t max_short_tiles = 0;  // of a 16-row window
+    uint32_t max_gap = 0;          // windows without entries one after the other, the ends of the matrix among them
     bool windows_fit = false, windows_forced = false;
     int n_sms = 0;
     // The tiles as the kernel's shared-memory image (spmm_kernel.cuh, SpmmParams::tiles_image): the plan's own
@@ -822,6 +823,12 @@ TallChoice choose_tall(const b200spmm_plan *p, int64_t n) {
 // columns 15.5 / 11.2, 128 columns 7.3 / 4.9; 1648 x 5712 at 0.8 %, 512 columns 10.2 / 4.7; 1088 x 14304 at 0.3 %, 96 columns
 // 6.3 / 3.7; fp16, 16384^2 at 0.5 %, 64 columns 8.4 / 5.0, 256 columns 13.3 / 8.2.  Long windows stay: 1024^2 pruned to 10 %,
 // fp16, 64 columns 9.4 / 24.
+//
+// Rows of missing windows are cleared by whoever has the window in front of them, and from five windows on the longest gap ends
+// last: 0.17 us a window and line of a warp (0.15 where a line of B is 256 bytes of C), 0.145 a window and pass of the pipelined
+// kernel's CTA (0.18 up to 96 columns, where half its lanes store).  16384 x 8192 of blocks at 0.5 %, 32 / 256 / 1,024 empty windows
+// behind: tf32, 128 columns, two lines 15 / 91 / 352, pipelined 12 / 45 / 156; 256 columns, two lines 18 / 95 / 356, one line 16 / 54
+// / 185, pipelined 20 / 86 / 311; fp16, 128 columns, one line 8.7 / 42 / 158, pipelined 12 / 44 / 156.
 struct WindowCost {
     double start, step, tile, warp;  // us; of a stage, of 1,000 tiles x groups of lines, of 1,000 warps
 };
@@ -830,23 +837,29 @@ struct PipelinedCost {
 };
 constexpr WindowCost kWindowCost[2][kWindowMaxLines] = {{{2.4, 0.34, 0.174, 1.08}, {2.7, 0.33, 0.258, 1.61}}, {{1.8, 0.49, 0.085, 0.83}, {2.2, 0.345, 0.137, 1.02}}};
 constexpr PipelinedCost kPipelinedCost[2] = {{4.3, 1.71, 0.40, 0.17}, {4.9, 1.08, 0.36, 0.62}};
+constexpr double kWindowGap[2] = {0.15, 0.17}, kPipelinedGap = 0.145, kPipelinedGapNarrow = 0.18;  // us
+constexpr uint32_t kHiddenGap = 5;
 uint32_t choose_window_lines(const b200spmm_plan *p, int64_t ldb, int64_t n) {
     const bool tf32 = p->info.dtype == B200SPMM_TF32;
     const uint64_t eff = p->info.eff_row_windows;
     const uint32_t line = 128u / (uint32_t)p->info.elt_size, n_lines = (uint32_t)((n + line - 1) / line);
     if (!p->windows_fit || (uint64_t)ldb * p->info.elt_size > 0xFFFFFFFFull || eff * n_lines > 0x7FFFFFFFull) return 0;  // 32-bit row pitch, grid
     const double tiles = (double)p->info.total_tiles, scale = 1e-3 * (148.0 / p->n_sms);
+    const double gap = p->max_gap > kHiddenGap ? (double)(p->max_gap - kHiddenGap) : 0.0;
     double least = 1e30;
     if (!p->windows_forced) {
         const PipelinedCost &c = kPipelinedCost[tf32];
-        least = c.start + (double)((n + 127) / 128) * (c.pass + (c.tile * tiles + c.window * (double)eff) * scale);
+        const double passes = (double)((n + 127) / 128);
+        least = c.start + passes * (c.pass + (c.tile * tiles + c.window * (double)eff) * scale) +
+                gap * (n <= 96 ? kPipelinedGapNarrow : passes * kPipelinedGap);
     }
     const uint32_t longest = (uint32_t)((tiles / (double)eff + p->max_short_tiles) / 2);  // (of ten tiles on average: two standard deviations above)
     uint32_t best = 0;
     for (uint32_t lines = 1; lines <= kWindowMaxLines && lines <= n_lines; ++lines) {
         const WindowCost &c = kWindowCost[tf32][lines - 1];
         const uint32_t stage = kWindowStageBytes / (128u * (uint32_t)p->info.col_window * lines), steps = (longest + stage - 1) / stage;
-        const double micros = c.start + c.step * steps + (c.tile * tiles + c.warp * (double)eff) * scale * (double)((n_lines + lines - 1) / lines);
+        const double micros = c.start + c.step * steps + (c.tile * tiles + c.warp * (double)eff) * scale * (double)((n_lines + lines - 1) / lines) +
+                              kWindowGap[tf32] * lines * gap;
         if (micros < least) {
             least = micros;
             best = lines;
@@ -1155,12 +1168,18 @@ int plan_build_tile_path(b200spmm_plan *p, const uint32_t *h_rowOffset, const ui
         if (st != B200SPMM_OK) return st;
     }
     p->has_tile_path = true;
-    // An explicit CTA count, window height, form of the tiles or way to fetch rows asks for the pipelined kernels.  (A warp
-    // clears the rows of all windows that are missing behind its own.)
+    // An explicit CTA count, window height, form of the tiles or way to fetch rows asks for the pipelined kernels, and so does a
+    // matrix of which less than one window in sixteen holds entries.  (How long its gaps may be: choose_window_lines.)
     p->windows_forced = env_is("B200SPMM_WINDOW", "warps");
     p->windows_fit = n_ctas <= 0 && !p->loose_lists && !p->gather_cpasync && !std::getenv("B200SPMM_TILES") &&
                      (p->windows_forced || (!std::getenv("B200SPMM_WINDOW") && !p->sched.n_splits && info.total_row_windows <= 16 * info.eff_row_windows));
-    for (uint64_t w = 0; w < info.eff_row_windows; ++w) p->max_short_tiles = std::max(p->max_short_tiles, h_rowOffset[w + 1] - h_rowOffset[w]);
+    uint64_t row = 0;  // behind the last window so far
+    for (uint64_t w = 0; w < info.eff_row_windows; ++w) {
+        p->max_short_tiles = std::max(p->max_short_tiles, h_rowOffset[w + 1] - h_rowOffset[w]);
+        p->max_gap = std::max(p->max_gap, (uint32_t)((h_rowIdx[w] - row) / kRowWindow));
+        row = (uint64_t)h_rowIdx[w] + kRowWindow;
+    }
+    if (info.rows > row) p->max_gap = std::max(p->max_gap, (uint32_t)((info.rows - row + kRowWindow - 1) / kRowWindow));
     return plan_build_tile_image(p);
 }
 

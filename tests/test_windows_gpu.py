@@ -97,3 +97,33 @@ def test_matrices_of_short_windows_choose_it_by_themselves():
             parity.check(C.cpu().numpy(), m.rows, rp, ci, v, B.cpu().numpy())
         finally:
             plan.close()
+
+
+@pytest.mark.parametrize("dt,n", [(np.float16, 256), (np.float32, 128)])
+@pytest.mark.parametrize("lead,tail", [(1, 1), (1024, 0), (2, 1024)])
+def test_long_gaps_are_not_cleared_by_warps_of_two_lines(dt, n, lead, tail, monkeypatch):
+    # a warp clears what is missing behind its window (and ahead of the first one), twice as slowly where it has two lines
+    import torch
+    m = synth.block_clustered_csr(16384, 8192, 0.005, seed=3, device="cuda")
+    ptr = m.row_ptr.to(torch.int32)
+    ptr = torch.cat([torch.zeros(16 * lead, dtype=torch.int32, device="cuda"), ptr, ptr[-1:].expand(16 * tail)])
+    rows, v = 16384 + 16 * (lead + tail), m.values.to(torch.float16 if dt == np.float16 else torch.float32)
+    f = hs.DeviceBtcf(rows, m.cols, ptr, m.col_idx, v)
+    B = synth.dense_normal(m.cols, n, 3, 3, "cuda", v.dtype)
+    plan = hs.SpmmPlan(f)
+    monkeypatch.setenv("B200SPMM_WINDOW", "16")
+    other = hs.SpmmPlan(f, n_ctas=1)
+    try:
+        got, want = (torch.full((rows, n), float("nan"), device="cuda") for _ in range(2))
+        plan.spmm(B, got)
+        info = plan.launch_info()
+        line = 64 if dt == np.float16 else 32
+        if lead + tail < 8:
+            assert (info.threads, info.feature_slab) == (128, 2 * line)
+        else:
+            assert info.threads != 128 or info.feature_slab == line
+        other.spmm(B, want)
+        assert torch.equal(got, want)
+    finally:
+        plan.close()
+        other.close()
