@@ -120,7 +120,7 @@ inline uint32_t bit_words(uint64_t cols) { return (uint32_t)((cols + 32 * kGroup
 // the set, how many columns lie below a word in its group (a byte), and below a group
 inline size_t bits_smem(uint64_t cols) { return ((size_t)bit_words(cols) * 5 + (size_t)(bit_words(cols) / kGroupWords) * 4 + 15) / 16 * 16; }
 
-// What a column needs of a key beside the row (4 bits) and the entry (8 bits), see sort_window.
+// What a column needs of a key beside the row (4 bits) and the entry (8 bits), or the entry alone (9 bits), see sort_window.
 constexpr uint32_t kKeyCols = (1u << 20) - 1u;
 static_assert(kBitsSmemMax / 11 * 2 * 32 < kKeyCols, "a column of the largest set fits a key");
 
@@ -156,12 +156,17 @@ struct WindowArgs {
     }
 };
 
-constexpr uint32_t kWarpEntries = 256, kHubEntries = 4096;
+constexpr uint32_t kHubEntries = 4096;
+// Entries of a window that a warp sorts.
+template <bool kWide>
+constexpr uint32_t kWarpEntries = kWide ? 512 : 256;
 
 // A warp's window of up to 32 * kN entries, one key of column, row and entry each: a bitonic sort over the places lane * kN + k,
-// the strides below kN within a lane.
+// the strides below kN within a lane.  (A key has no room for the row of one of 512 entries, which is looked up again.)
 template <int kN>
 __device__ __forceinline__ void sort_window(const WindowArgs &a, uint32_t w, uint32_t lane, uint32_t start, uint32_t p0, uint32_t n) {
+    constexpr bool kRowInKey = kN <= 8;
+    constexpr int kEntryBits = kRowInKey ? 8 : 9, kColumnAt = kRowInKey ? 12 : 9;
     uint32_t key[kN], before = 0, row_before = 0xFFFFFFFFu;  // column and row of the entry before the first one of a step
     bool bad = false;
 #pragma unroll
@@ -175,7 +180,7 @@ __device__ __forceinline__ void sort_window(const WindowArgs &a, uint32_t w, uin
         row_before = __shfl_sync(0xffffffffu, r, 31);
         const bool live = i < n, fits = c < a.cols;
         bad |= live && (!fits || (left_row == r && left >= c));
-        key[k] = live && fits ? c << 12 | r << 8 | i : 0xFFFFFFFFu;
+        key[k] = live && fits ? c << kColumnAt | (kRowInKey ? r << kEntryBits : 0u) | i : 0xFFFFFFFFu;
     }
     if (__any_sync(0xffffffffu, bad)) {
         if (lane == 0) {
@@ -213,7 +218,7 @@ __device__ __forceinline__ void sort_window(const WindowArgs &a, uint32_t w, uin
     bool first[kN];
 #pragma unroll
     for (int k = 0; k < kN; ++k) {
-        first[k] = lane * kN + k < n && key[k] >> 12 != prev >> 12;
+        first[k] = lane * kN + k < n && key[k] >> kColumnAt != prev >> kColumnAt;
         prev = key[k];
         mine += first[k];
     }
@@ -228,7 +233,9 @@ __device__ __forceinline__ void sort_window(const WindowArgs &a, uint32_t w, uin
 #pragma unroll
     for (int k = 0; k < kN; ++k) {
         at += first[k];
-        if (lane * kN + k < n) a.places[p0 + (key[k] & 255u)] = a.place(at, key[k] >> 8 & 15u);
+        const uint32_t entry = key[k] & ((1u << kEntryBits) - 1u);
+        const uint32_t r = kRowInKey ? key[k] >> kEntryBits & 15u : a.row_of((uint64_t)p0 + entry, start);
+        if (lane * kN + k < n) a.places[p0 + entry] = a.place(at, r);
     }
 }
 
@@ -236,8 +243,14 @@ __device__ __forceinline__ void sort_window(const WindowArgs &a, uint32_t w, uin
 // dozen entries: sorted by a warp that is some hundred instructions, marked in a set by a block of 256 threads it is 5,500,
 // most of them to clear and to count an empty set (60,000 nodes, 720,000 entries: 40 us; this kernel takes 9 with the zeroing of
 // 24 MB, the one for long windows 18 - 21).
+//
+// kWide: windows of up to 512 entries, for matrices of so many columns (655,361 and more) that a block has room for one set alone.
+// There a window of just over 256 entries waits for a set of 110 KB to be cleared and counted, 5.6 us of an SM: 660,000 nodes, 17 /
+// 20 / 30 entries a node 2,230 / 2,310 / 2,670 us, so 1,000 / 1,080 / 1,370 (through the sort of all entries 1,660 / 1,840 / 4,700).  Where
+// two sets and more fit, the wide kernel's code costs a small matrix more than that: a graph of 2,000 nodes 70 -> 80, of 60,000 96 -> 104.
 constexpr int kSortBlock = 256;
-__global__ void __launch_bounds__(kSortBlock)
+template <bool kWide>
+__global__ void __launch_bounds__(kSortBlock, 4)
 window_sort_kernel(const WindowArgs a, uint4 *__restrict__ clear, uint64_t n_clear) {
     const uint32_t lane = threadIdx.x & 31u;
     if (blockIdx.x == 0 && threadIdx.x == 0 && (a.row_ptr[0] != 0 || a.row_ptr[a.rows] != a.nnz)) atomicOr(&a.totals->bad, 1u);
@@ -255,8 +268,10 @@ window_sort_kernel(const WindowArgs a, uint4 *__restrict__ clear, uint64_t n_cle
             sort_window<2>(a, w, lane, start, p0, n);
         } else if (n <= 128) {
             sort_window<4>(a, w, lane, start, p0, n);
-        } else if (n <= kWarpEntries) {
+        } else if (n <= 256) {
             sort_window<8>(a, w, lane, start, p0, n);
+        } else if (n <= kWarpEntries<kWide>) {
+            if constexpr (kWide) sort_window<16>(a, w, lane, start, p0, n);
         } else if (lane == 0) {
             const bool hub = n > kHubEntries;
             const uint32_t k = atomicAdd(hub ? &a.totals->hubs : &a.totals->long_windows, 1u);
@@ -612,9 +627,10 @@ int convert_by_windows(b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const uint3
     B200_CUDA_TRY(cudaMemsetAsync(totals, 0, sizeof(Totals), stream));
     const WindowArgs args{d_row_ptr, d_col_idx, rows, cols, nnz, n_windows, RW, log_cw, bit_words(f->info.cols), places, count, tile_of, totals};
     constexpr uint32_t kWarps = kSortBlock / 32;
-    window_sort_kernel<<<std::min<uint32_t>((n_windows + kWarps - 1) / kWarps, 148 * 64), kSortBlock, 0, stream>>>(
+    const bool wide = parts == 1;
+    (wide ? window_sort_kernel<true> : window_sort_kernel<false>)<<<std::min<uint32_t>((n_windows + kWarps - 1) / kWarps, 148 * 64), kSortBlock, 0, stream>>>(
         args, static_cast<uint4 *>(f->d_data), ahead ? most_tiles * tile_bytes / 16 : 0);
-    if (nnz > kWarpEntries) window_marks_kernel<<<std::min<uint32_t>(n_windows, 148), kBitsBlock, parts * smem, stream>>>(args, parts, (uint32_t)(smem / 4));
+    if (nnz > (wide ? kWarpEntries<true> : kWarpEntries<false>)) window_marks_kernel<<<std::min<uint32_t>(n_windows, 148), kBitsBlock, parts * smem, stream>>>(args, parts, (uint32_t)(smem / 4));
     B200_CUDA_TRY(cudaGetLastError());
     if (n_windows <= kOneBlockWindows) {
         scan_tables_kernel<<<1, kScanBlock, 0, stream>>>(count, n_windows, RW, CW, f->d_rowOffset, f->d_rowIdx, tile_of, totals);

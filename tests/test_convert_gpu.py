@@ -157,3 +157,33 @@ def test_windows_at_the_edges_of_the_sorts_and_the_set(dt, rw, cw):
             with pytest.raises(capi.SpmmError) as e:
                 device_convert(rows, cols, rp, bad, v, rw, cw)
             assert e.value.status == capi.ERR_BAD_CSR
+
+
+@pytest.mark.parametrize("rw", [8, 16])
+@pytest.mark.parametrize("cols", [3001, 743000])
+def test_windows_of_up_to_512_entries_and_every_width_of_the_set(rw, cols):
+    # of 743,000 columns, where a block has one set, warps sort them with sixteen keys a lane; else blocks mark them
+    counts = [257, 511, 512, 513, 300, 0, 384, 512, 256, 4097]
+    rng, lengths, ci = np.random.default_rng(rw), [], []
+    for n in counts:
+        cuts = np.sort(rng.integers(0, n + 1, rw - 1)) if n < 4000 else np.arange(1, rw) * n // rw
+        lengths += list(np.diff(np.concatenate([[0], cuts, [n]])))
+    for k, n in enumerate(lengths):
+        row = np.sort(rng.choice(cols if k % 3 else min(cols, 2 * n + 1), n, replace=False))
+        if n > 1:
+            row[0], row[-1] = 0, cols - 1
+        ci.append(row)
+    ci = np.concatenate(ci).astype(np.uint32)
+    rp, v, rows = np.concatenate([[0], np.cumsum(lengths)]).astype(np.uint32), rng.uniform(0.1, 1, ci.size).astype(np.float16), len(lengths)
+    dev = device_convert(rows, cols, rp, ci, v, rw)
+    assert_same(dev, hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v), row_window=rw))
+    dev.close()
+    for w in (1, 2):  # a column out of order, one twice, one out of range
+        for c in ([3, 1], [5, 5], [7, cols]):
+            bad, r = ci.copy(), w * rw
+            while lengths[r] < 2:
+                r += 1
+            bad[rp[r]:rp[r] + 2] = c
+            with pytest.raises(capi.SpmmError) as e:
+                device_convert(rows, cols, rp, bad, v, rw)
+            assert e.value.status == capi.ERR_BAD_CSR
