@@ -575,8 +575,12 @@ void scatter_values(const b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const ui
                                                                      (uint32_t)i.row_window, (uint32_t)i.col_window, static_cast<uint32_t *>(f->d_data));
 }
 
-// Up to this size the tile array is made ahead, as large as it can become (no column shared by two entries): it is cleared
-// while the places are found, and the host waits once instead of twice (about 12 us of 80).
+// Up to this size the tile array is made ahead, as large as it can become (no column shared by two entries, or every column in
+// every window): it is cleared while the places are found, and the host waits once instead of twice (about 12 us of 80).  Without
+// the second bound, and cleared by the blocks of the windows alone, dense matrices had several times their tiles cleared and held:
+// pruned 1024 x 4096 / 2000 x 2000 at 30 % 166 / 118 us (113 / 105 with two waits), now 80 / 78.  Where windows share columns by
+// blocks the array stays too large; moving what is used to one of its size took 20 to 30 of 110 us and gave the pool, which maps 64
+// MB at a time, nothing to return.
 constexpr uint64_t kAheadBytes = (uint64_t)64 << 20;
 
 template <typename T>
@@ -604,7 +608,8 @@ int convert_by_windows(b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const uint3
     B200_CUDA_TRY(tmp.alloc(&tile_of, n_windows));
     B200_CUDA_TRY(pool_alloc(&f->d_rowOffset, (size_t)n_windows + 1, stream));
     B200_CUDA_TRY(pool_alloc(&f->d_rowIdx, n_windows, stream));
-    const uint64_t most_tiles = (uint64_t)nnz / CW + std::min(n_windows, nnz);
+    const uint64_t most_windows = std::min(n_windows, nnz);
+    const uint64_t most_tiles = std::min((uint64_t)nnz / CW + most_windows, most_windows * (((uint64_t)cols + CW - 1) / CW));
     bool ahead = most_tiles * tile_bytes <= kAheadBytes;
     auto alloc_tiles = [&](uint64_t tiles) {
         const cudaError_t e = pool_alloc(&f->d_tcA2B, tiles * CW, stream);
@@ -628,8 +633,12 @@ int convert_by_windows(b200spmm_dbtcf *f, const uint32_t *d_row_ptr, const uint3
     const WindowArgs args{d_row_ptr, d_col_idx, rows, cols, nnz, n_windows, RW, log_cw, bit_words(f->info.cols), places, count, tile_of, totals};
     constexpr uint32_t kWarps = kSortBlock / 32;
     const bool wide = parts == 1;
-    (wide ? window_sort_kernel<true> : window_sort_kernel<false>)<<<std::min<uint32_t>((n_windows + kWarps - 1) / kWarps, 148 * 64), kSortBlock, 0, stream>>>(
-        args, static_cast<uint4 *>(f->d_data), ahead ? most_tiles * tile_bytes / 16 : 0);
+    // as many blocks as there are windows, or as clear the tiles at the rate of the memory
+    const uint64_t n_clear = ahead ? most_tiles * tile_bytes / 16 : 0;
+    const uint32_t for_windows = std::min<uint32_t>((n_windows + kWarps - 1) / kWarps, 148 * 64);
+    const uint32_t for_clearing = (uint32_t)std::min<uint64_t>((n_clear + 8 * kSortBlock - 1) / (8 * kSortBlock), 148 * 4);
+    (wide ? window_sort_kernel<true> : window_sort_kernel<false>)<<<std::max(for_windows, for_clearing), kSortBlock, 0, stream>>>(
+        args, static_cast<uint4 *>(f->d_data), n_clear);
     if (nnz > (wide ? kWarpEntries<true> : kWarpEntries<false>)) window_marks_kernel<<<std::min<uint32_t>(n_windows, 148), kBitsBlock, parts * smem, stream>>>(args, parts, (uint32_t)(smem / 4));
     B200_CUDA_TRY(cudaGetLastError());
     if (n_windows <= kOneBlockWindows) {

@@ -187,3 +187,29 @@ def test_windows_of_up_to_512_entries_and_every_width_of_the_set(rw, cols):
             with pytest.raises(capi.SpmmError) as e:
                 device_convert(rows, cols, rp, bad, v, rw)
             assert e.value.status == capi.ERR_BAD_CSR
+
+
+def test_tiles_made_ahead_are_no_more_than_every_column_in_every_window():
+    # 1.9e6 entries, whose tiles could take 61 MB if they shared no column, and take 12
+    import torch
+    rng = np.random.default_rng(5)
+    rows = cols = 2400
+    mask = rng.random((rows, cols)) < 0.34
+    rp = np.concatenate([[0], np.cumsum(mask.sum(1))]).astype(np.uint32)
+    ci = np.nonzero(mask)[1].astype(np.uint32)
+    v = rng.uniform(0.1, 1, ci.size).astype(np.float16)
+    dev = [torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a).cuda() for a in (rp, ci, v)]
+
+    def free():
+        torch.cuda.synchronize()
+        assert capi.lib().b200spmm_release_cached_memory(0) == 0
+        return torch.cuda.mem_get_info()[0]
+
+    hs.DeviceBtcf(rows, cols, *dev).close()
+    before = free()
+    f = hs.DeviceBtcf(rows, cols, *dev)
+    assert_same(f, hs.CSR2BTCFNOBITMAP(hs.CSR_MTX(rows, cols, rp, ci, v)))
+    needed = f.total_tiles * (512 + 64)
+    assert before - free() <= needed + (34 << 20)  # (the pool takes 32 MB and more at a time; the tables)
+    f.close()
+    assert before - free() == 0
