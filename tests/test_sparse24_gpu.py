@@ -182,3 +182,53 @@ def test_what_goes_to_the_rest_may_lie_close_together(surplus, at, monkeypatch):
     dense = np.zeros((rows, cols))
     dense[np.repeat(np.arange(rows), np.diff(rp.astype(np.int64))), ci] = v
     assert torch.equal(got.cpu().double(), torch.from_numpy(dense) @ B.cpu().double())
+
+
+def test_matrices_beyond_the_limit_do_not_pay_for_the_form(monkeypatch):
+    # a twentieth of a row's groups has more than two entries: a sample says so in less than 0.1 ms, the form takes 0.6 ms and more
+    import time
+
+    import torch
+    csr = synth.pruned_weight_csr(20480, 8192, 0.22, seed=3, device="cuda")
+    f = hs.DeviceBtcf(csr.rows, csr.cols, csr.row_ptr.to(torch.int32), csr.col_idx, csr.values)
+    B = synth.dense_normal(csr.cols, 256, 3, 3, "cuda", torch.float16)
+    took = {}
+    for rounds in range(6):
+        for env in (None, "0"):
+            if env:
+                monkeypatch.setenv("B200SPMM_SPARSE24", env)
+            else:
+                monkeypatch.delenv("B200SPMM_SPARSE24", raising=False)
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            plan = hs.SpmmPlan(f)
+            torch.cuda.synchronize()
+            took.setdefault(env, []).append(time.perf_counter() - t0)
+            if not rounds:
+                plan.spmm(B)
+                assert plan.launch_info().row_window == 256 and plan.launch_info().stages == DENSE
+            plan.close()
+    assert min(took[None]) - min(took["0"]) < 0.35e-3
+    f.close()
+
+
+def test_weights_that_are_pruned_two_of_four_take_it(monkeypatch):
+    # half of all entries, and none in the rest
+    import torch
+    rows, cols, n = 12288, 8192, 256
+    g = torch.Generator(device="cuda").manual_seed(3)
+    pairs = torch.tensor([[0, 1], [0, 2], [0, 3], [1, 2], [1, 3], [2, 3]], device="cuda", dtype=torch.int32)
+    ci = pairs[torch.randint(0, 6, (rows * cols // 4,), generator=g, device="cuda")] + 4 * (torch.arange(rows * cols // 4, device="cuda", dtype=torch.int32) % (cols // 4))[:, None]
+    v = torch.randint(1, 4, (ci.numel(),), generator=g, device="cuda").half()
+    f = hs.DeviceBtcf(rows, cols, torch.arange(rows + 1, device="cuda", dtype=torch.int32) * (cols // 2), ci.reshape(-1), v)
+    B = torch.randint(-4, 5, (cols, n), generator=g, device="cuda").half()
+    plan = hs.SpmmPlan(f)
+    try:
+        C = plan.spmm(B)
+        assert plan.launch_info().row_window == 256 and plan.launch_info().stages == SPARSE
+        dense = torch.zeros((rows, cols), device="cuda", dtype=torch.float16)
+        dense.scatter_(1, ci.reshape(rows, -1).long(), v.reshape(rows, -1))
+        assert torch.equal(C, dense.float() @ B.float())
+    finally:
+        plan.close()
+        f.close()
