@@ -1048,8 +1048,11 @@ int plan_build_tall(b200spmm_plan *p, const uint32_t *h_rowOffset, const uint32_
     const bool most_aligned = (uint64_t)aligned * 2 >= p->tall.tiles;
     p->tall_pack_b = most_aligned && !env_is("B200SPMM_PACK_B", "0");
     // The windows once more in 2:4 form, where most of their lists name neighbouring rows of B (the kernel has no room for gathers
-    // in every stage).  It takes 0.5 to 1 ms to make, which a small matrix does not get back: 14336 x 4096 at 8 % (14,336 tiles) 39.5 ->
-    // 31.3 us a product of 256 columns, plan 0.8 -> 1.3 ms.  B200SPMM_SPARSE24=0 keeps it out, =1 asks for it wherever it fits.
+    // in every stage): 0.6 of their memory again, for launches of more than 128 columns in whole windows.  28672 x 8192 at 10 %
+    // (57,344 tiles): plan 3.3 -> 3.9 ms, 1,323 -> 1,598 MB, 738 -> 688 us a product of 2,048 columns.  14336 x 4096 at 8 % (14,336): plan 0.8
+    // -> 0.9 ms where the pool has room for its buffers, 1.1 -> 1.5 to 2.0 where it has not, 39 -> 31 us a product of 256 columns: up
+    // to a hundred products, more than a plan that is made anew has before it.  Sizes between were not measured.
+    // B200SPMM_SPARSE24=0 keeps it out, =1 asks for it wherever it fits.
     const bool always = env_is("B200SPMM_SPARSE24", "1");
     if (p->pair.tiles && most_aligned && info.dtype == B200SPMM_F16 && (always || p->pair.tiles >= kSparse24MinTiles) && !env_is("B200SPMM_SPARSE24", "0")) {
         int clusters = 0;

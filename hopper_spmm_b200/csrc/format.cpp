@@ -60,7 +60,7 @@ void parallel_chunks(uint64_t n_items, uint64_t chunk, int n_threads, Fn fn) {
 // The sorted distinct columns of a window, and the place of a column among them.  Where the window's entries are
 // dense in the columns (a pruned weight matrix: a sixth of them) a bit set does both in one step per entry;
 // otherwise the columns are sorted and searched.  The places of a matrix of few columns are kept column by column, in a table
-// that stays in the core's cache (14336 x 4096, a tenth of it kept: the conversion took 6.5 ms with bits counted for every entry, now 5.7).
+// that stays in the core's cache (14336 x 4096, a tenth of it kept: the conversion took 6.5 ms with bits counted for every entry, now 5.3).
 class WindowColumns {
 public:
     explicit WindowColumns(uint64_t cols) : words_((cols + 63) / 64), table_cols_(cols <= kTableCols ? cols : 0) {}

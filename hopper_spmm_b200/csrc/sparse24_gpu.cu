@@ -29,8 +29,10 @@ namespace {
 constexpr int kRows = 256;            // of a window, and threads of a block
 constexpr uint32_t kBlockTiles = 16;  // of 32 columns
 // Entries of the rest a row and dense tile, up to which the form pays: the epilogue warps get through 0.02 while the tensor core
-// does a tile.  28672 x 8192, us, dense and so: 10 % (0.015), 192 / 2,048 columns 105 / 772 and 89 / 661; 12 % (0.025) 113 / 690
-// and 111 / 678; 14 % (0.038) 113 / 692 and 137 / 882.
+// does a tile.  28672 x 8192, dense and so in turn, us of a loop of calls (and of single ones after 3 ms of rest): 192 columns, half
+// results, 10 % (0.015) 109 and 98 (117 and 102), 11 % (0.020) 107 and 104 (117 and 106), 12 % (0.026) 108 and 115 (118 and 117), 14 %
+// (0.040) 107 and 139; 2,048 columns, 10 % 738 and 688 at 1,635 MHz under the power cap (692 and 608), 11 % 735 and 731 (691 and 637),
+// 12 % 735 and 802 (695 and 703), 14 % 733 and 990.
 constexpr double kMostRest = 0.02;
 
 constexpr unsigned long long kUnfit = 1ull << 63;  // in the number of all entries of the rest: some row has too many

@@ -24,9 +24,10 @@
 // tile of 16.  A stage brings 2 KB of metadata with its four tiles; the issuing thread copies it to four columns of tensor
 // memory (tcgen05.cp, which runs in order with the MMAs that follow), so there is one accumulator and an item's epilogue is not hidden
 // behind the next item's MMAs.  What rows have beyond two entries in a group of four is multiplied by the epilogue warps meanwhile.
-// Bound: L2 -> SM, 12.5 KB a tile step of 32 columns where dense tiles take 16 (52 bytes a clock and SM; two of its 240 clocks in
-// three are tensor-pipe clocks), and power.  28672 x 8192 at 10 %, us, dense and so: 192 columns, half results 118 and 95, 2,048
-// columns 788 and 672; without the rest 88 and 619.  Listing the rest's columns again as tiles instead was tried (18 % more tiles, any
+// Bound: L2 -> SM, 12.5 KB a tile step of 32 columns where dense tiles take 16 (52 bytes a clock and SM, 240 clocks a step; the tensor
+// pipe is active for 40 % of a launch's cycles, with dense tiles for 72), and power.  28672 x 8192 at 10 %, us a call of a loop whose
+// matrices and operands change from call to call, dense and so: 192 columns, half results 118 and 95, 2,048 columns 788 and 672 under
+// the power cap; without the rest 88 and 619.  Listing the rest's columns again as tiles instead was tried (18 % more tiles, any
 // column of B): with gathers 105 and 751, four warps issuing; with cp.async 119 and 784.
 // Every wait is bounded; both CTAs meet at a cluster barrier before either lets go of its shared or
 // tensor memory.

@@ -464,8 +464,10 @@ int b200spmm_plan_tall_copy_to_host(const b200spmm_plan_t *p, uint32_t *rowOffse
  * features: a pair of CTAs on neighbouring SMs (a cluster of two) then shares one MMA of 256 window rows x
  * 256 features, each CTA holding half of either operand, which halves what an SM fetches of B per tile.
  * Kept when the 256-row windows have at most 0.55 of the 128-row tiles (B200SPMM_WINDOW=256 forces it,
- * =128 keeps it out).  fp16 plans of 20,000 and more such tiles keep them in the tensor core's 2:4 form as well and
- * multiply whole windows in that (B200SPMM_SPARSE24=0 keeps it out, =1 asks for it wherever it fits).  The two calls below are the counterparts of the two above for that copy
+ * =128 keeps it out).  fp16 plans of 20,000 and more such tiles keep them in the tensor core's 2:4 form as
+ * well (4.8 KB a tile beside its 8), where no more entries are left over than pays - about 11 % of the entries
+ * kept at random, or weights pruned two of four - and multiply whole windows in that (B200SPMM_SPARSE24=0 keeps
+ * it out, =1 asks for it wherever it fits).  The two calls below are the counterparts of the two above for that copy
  * (row_window 256, or 0 when the plan has none).
  */
 int b200spmm_plan_pair_info(const b200spmm_plan_t *p, b200spmm_btcf_info_t *info);
